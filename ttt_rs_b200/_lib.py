@@ -83,6 +83,7 @@ SYMBOLS = {
 NOALLOC_SCRATCH_BYTES = 32 << 20  # TTT_NOALLOC_SCRATCH_BYTES
 
 _lib: Optional[C.CDLL] = None
+_host = None
 
 
 def load() -> C.CDLL:
@@ -99,6 +100,21 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def host():
+    """The native host path (csrc/ttt_host.cpp)."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise RuntimeError("the native host path is missing or does not load: build it with "
+                               f"`python -m ttt_rs_b200.build` ({e})") from e
+        mod.init(TttError)
+        _host = mod
+    return _host
 
 
 def last_error() -> str:

@@ -1,4 +1,4 @@
-"""Builds the CUDA library (libttt_b200.so) for sm_100a with nvcc, in-tree.
+"""Builds the CUDA library (libttt_b200.so) for sm_100a with nvcc, in-tree, and the native host path (_host.so).
 
     python -m ttt_rs_b200.build            # rebuild if any source is newer than the library
     python -m ttt_rs_b200.build --force
@@ -18,6 +18,8 @@ LIB = PKG / "libttt_b200.so"
 PROBE_SRC = CSRC / "probe_chain_latency.cu"      # stand-alone measurement program (bench.py --workload chain-latency)
 PROBE_BIN = PKG / "build" / "probe_chain_latency"
 SOURCES = ["ttt_abi.cu", "ttt_linear_fwd.cu", "ttt_linear_bwd.cu", "ttt_mlp_fwd.cu", "ttt_layer.cu", "ttt_linear_partial.cu", "ttt_mlp_bwd.cu", "ttt_gemm.cu"]
+HOST_SRC = CSRC / "ttt_host.cpp"                 # native host path of the Python operator, linked against LIB
+HOST_LIB = PKG / "_host.so"
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
@@ -53,9 +55,32 @@ def build_probe(force: bool = False) -> Path:
     return PROBE_BIN
 
 
+def build_host(force: bool = False) -> Path:
+    """The CPython extension module `_host`, for the interpreter and the torch that run this."""
+    deps = [HOST_SRC, CSRC / "ttt_internal.h", PKG.parent / "include" / "ttt_b200.h"]
+    if not force and HOST_LIB.exists() and all(HOST_LIB.stat().st_mtime >= p.stat().st_mtime for p in deps):
+        return HOST_LIB
+    import sysconfig
+
+    import torch
+    tdir = Path(torch.__file__).resolve().parent
+    cuda = Path(find_nvcc()).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-Wno-attributes",
+           f"-I{tdir}/include", f"-I{tdir}/include/torch/csrc/api/include", f"-I{cuda}/include",
+           f"-I{sysconfig.get_paths()['include']}", str(HOST_SRC), "-o", str(HOST_LIB),
+           f"-L{tdir}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           f"-L{PKG}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SRC.name}:\n{r.stdout}")
+    return HOST_LIB
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     build_probe(force)
     if not force and not needs_build():
+        build_host(force)
         return LIB
     nvcc = find_nvcc()
     objs = []
@@ -78,6 +103,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}")
+    build_host(force)
     (build_dir / "ptxas.log").write_text("\n".join(log))
     if verbose:
         print("\n".join(log))

@@ -8,6 +8,7 @@
 #include <mutex>
 
 #include "../../include/ttt_b200.h"
+#include "ttt_internal.h"
 #include "ttt_kernels.h"
 
 namespace {
@@ -448,6 +449,21 @@ int ttt_linear_backward_state_grads(const ttt_dims* d, const void* xq, const voi
                                     void* grad_ttt_lr_eta, float* grad_token_eta, float* grad_ln_weight,
                                     float* grad_ln_bias, float* outer_grad_packed, void* workspace,
                                     size_t workspace_bytes, void* status, void* stream) {
+  return ttt_internal_linear_backward(d, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias,
+                                      weight_ckpt, bias_ckpt, grad_output, grad_weight_out, grad_bias_out, grad_xq,
+                                      grad_xk, grad_xv, grad_weight, grad_bias, grad_ttt_lr_eta, grad_token_eta,
+                                      grad_ln_weight, grad_ln_bias, TTT_F32, outer_grad_packed, workspace,
+                                      workspace_bytes, status, stream);
+}
+
+int ttt_internal_linear_backward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* weight,
+                                 const void* bias, const void* token_eta, const void* ttt_lr_eta, const void* ln_weight,
+                                 const void* ln_bias, const void* weight_ckpt, const void* bias_ckpt,
+                                 const void* grad_output, const void* grad_weight_out, const void* grad_bias_out,
+                                 void* grad_xq, void* grad_xk, void* grad_xv, void* grad_weight, void* grad_bias,
+                                 void* grad_ttt_lr_eta, void* grad_token_eta, void* grad_ln_weight, void* grad_ln_bias,
+                                 int reduced_dtype, float* outer_grad_packed, void* workspace, size_t workspace_bytes,
+                                 void* status, void* stream) {
   int rc = check_dims(d, true);
   if (rc != TTT_OK) return rc;
   const NamedPtr ptrs[] = {{"xq", xq},
@@ -536,13 +552,14 @@ int ttt_linear_backward_state_grads(const ttt_dims* d, const void* xq, const voi
   r.d_token_eta = grad_token_eta;
   r.d_ln_g = grad_ln_weight;
   r.d_ln_b = grad_ln_bias;
+  r.out_bf16 = reduced_dtype == TTT_BF16;
   r.packed = outer_grad_packed;
   r.B = d->batch;
   r.H = d->heads;
   r.F = d->head_dim;
   r.mb = d->mini_batch;
   r.T = d->seq_len;
-  r.NCH = wl.nch;
+  r.NCH = p.NCH;
   e = ttt::launch_linear_bwd_reduce(r, st);
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "backward reduction launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
@@ -977,6 +994,20 @@ extern "C" int ttt_mlp_backward(const ttt_dims* d, const void* xq, const void* x
                                 void* grad_b1, void* grad_w2, void* grad_b2, void* grad_ttt_lr_eta,
                                 float* grad_token_eta, float* grad_ln_weight, float* grad_ln_bias, void* workspace,
                                 size_t workspace_bytes, int workspace_from_forward, void* status, void* stream) {
+  return ttt_internal_mlp_backward(d, xq, xk, xv, w1, b1, w2, b2, token_eta, ttt_lr_eta, ln_weight, ln_bias, grad_output,
+                                   grad_xq, grad_xk, grad_xv, grad_w1, grad_b1, grad_w2, grad_b2, grad_ttt_lr_eta,
+                                   grad_token_eta, grad_ln_weight, grad_ln_bias, TTT_F32, workspace, workspace_bytes,
+                                   workspace_from_forward, status, stream);
+}
+
+extern "C" int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, const void* xk, const void* xv,
+                                         const void* w1, const void* b1, const void* w2, const void* b2,
+                                         const void* token_eta, const void* ttt_lr_eta, const void* ln_weight,
+                                         const void* ln_bias, const void* grad_output, void* grad_xq, void* grad_xk,
+                                         void* grad_xv, void* grad_w1, void* grad_b1, void* grad_w2, void* grad_b2,
+                                         void* grad_ttt_lr_eta, void* grad_token_eta, void* grad_ln_weight,
+                                         void* grad_ln_bias, int reduced_dtype, void* workspace, size_t workspace_bytes,
+                                         int workspace_from_forward, void* status, void* stream) {
   int rc = check_dims(d);
   if (rc != TTT_OK) return rc;
   if (d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "the TTT-MLP kernels are built for bf16 only");
@@ -1000,6 +1031,7 @@ extern "C" int ttt_mlp_backward(const ttt_dims* d, const void* xq, const void* x
   p.d_q = grad_xq; p.d_k = grad_xk; p.d_v = grad_xv; p.d_w1 = grad_w1; p.d_b1 = grad_b1; p.d_w2 = grad_w2;
   p.d_b2 = grad_b2; p.d_lr = grad_ttt_lr_eta; p.d_token_eta = grad_token_eta; p.d_ln_g = grad_ln_weight;
   p.d_ln_b = grad_ln_bias;
+  p.reduced_bf16 = reduced_dtype == TTT_BF16;
   p.workspace = ws;
   p.ws_stride = l.stride_floats;
   p.part_te = ws + l.off_te;

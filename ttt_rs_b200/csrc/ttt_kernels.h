@@ -41,7 +41,8 @@ struct LinBwdParams {
   void* d_lr;       // [B,H,T]
   int* sched;       // workspace: [0] next work item, [1 + stream] chunks of the stream finished so far (zeroed per launch)
   float* handoff;   // workspace: [B*H][2*F*F + F] W^T, dW^T (register layout) and db handed from chunk to chunk
-  int CH, NCH, nstreams;  // stages per chunk, chunks per stream, B*H
+  int CH, NCH, nstreams;  // stages per chunk, chunks per stream, B*H (the launcher sets CH = NS, NCH = 1, sched = null
+                          // where every stream has an SM of its own)
   uint32_t handoff_polls;  // iteration limit of the wait for another chunk's hand-off (each poll sleeps ~100 ns)
   int item_base;           // added to every work-item number (0 in normal use; the wait-limit test starts past the
                            // items that would publish the first hand-offs, so that a wait runs out)
@@ -55,12 +56,13 @@ struct LinBwdParams {
 
 struct ReduceParams {
   const float* part_ln;
-  const float* part_te;
+  float* part_te;  // (with `packed`, row 0 receives the sums)
   const float* part_w;
-  float* d_token_eta;  // [T] f32
-  float* d_ln_g;       // [H,F] f32
-  float* d_ln_b;       // [H,F] f32
-  float* packed;       // nullable: [H*F*F + 3*H*F + CS] f32
+  void* d_token_eta;  // [T], float32 or bf16
+  void* d_ln_g;       // [H,F]
+  void* d_ln_b;       // [H,F]
+  int out_bf16;       // element type of the three
+  float* packed;      // nullable: [H*F*F + 3*H*F + CS] f32
   int B, H, T, NCH;
   int F;   // features per head: 64, or 32 (two heads per 64-wide tile in part_ln)
   int mb;  // tokens per mini-batch (16 or 8): d_token_eta is folded to [mb]
@@ -232,10 +234,11 @@ struct MlpBwdParams {
   void* d_w2;
   void* d_b2;
   void* d_lr;
-  float* d_token_eta;  // [T] float32
-  float* d_ln_g;       // [H,F] float32
-  float* d_ln_b;
-  float* workspace;    // per stream `ws_stride` floats: state, state gradients, saved inner gradients
+  void* d_token_eta;  // [T], float32 or bf16
+  void* d_ln_g;       // [H,F]
+  void* d_ln_b;
+  int reduced_bf16;   // element type of the three
+  float* workspace;   // per stream `ws_stride` floats: state, state gradients, saved inner gradients
   size_t ws_stride;
   float* part_te;      // [B*H][T]
   float* part_ln;      // [B*H][2][F]
@@ -292,7 +295,7 @@ cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* map
                               const LinFwdParams& p, int nstreams, cudaStream_t st);
 // maps: q, k, v, d_out, d_q, d_k, d_v, gp; io: the plain pointers behind the first seven.
 cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, const void* const* io,
-                              const LinBwdParams& p, int nstreams, cudaStream_t st);
+                              LinBwdParams& p, int nstreams, cudaStream_t st);
 cudaError_t launch_linear_bwd_reduce(const ReduceParams& p, cudaStream_t st);
 
 }  // namespace ttt

@@ -225,11 +225,15 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
   // waits for an item with a smaller index (the later chunk of the same stream), which was taken by a block that runs
   // or has finished (a block takes an item only once it runs), so the wait graph has no cycle and the launch cannot
   // deadlock, whether or not every block of the grid is resident.
-  while (!failed) {
-    if (tid == 0) s_item = atomicAdd(&p.sched[0], 1);
-    __syncthreads();
-    const int item = s_item + p.item_base;
-    __syncthreads();
+  // (Without a scheduler -- every stream has an SM of its own -- block b takes stream b from end to end.)
+  for (int round = 0; !failed; ++round) {
+    int item = round == 0 ? (int)blockIdx.x : nitems;
+    if (p.sched != nullptr) {
+      if (tid == 0) s_item = atomicAdd(&p.sched[0], 1);
+      __syncthreads();
+      item = s_item + p.item_base;
+      __syncthreads();
+    }
     if (item >= nitems) break;
     const int crank = item / p.nstreams;  // 0 = last chunk of the sequence
     const int chunk = p.NCH - 1 - crank;
@@ -880,11 +884,16 @@ __global__ void __launch_bounds__(256) ttt_linear_bwd_reduce_kernel(const Reduce
       float sum = part[0][lane];
 #pragma unroll
       for (int w = 1; w < 8; ++w) sum += part[w][lane];
+      auto put = [&](void* dst, int at) {
+        if (p.out_bf16) st_from_float<__nv_bfloat16>(dst, (size_t)at, sum);
+        else st_from_float<float>(dst, (size_t)at, sum);
+      };
       if (i < n_te) {
-        p.d_token_eta[i] = sum;
+        put(p.d_token_eta, i);
+        if (p.packed != nullptr) p.part_te[i] = sum;  // for the fold below; no other block reads column i
       } else if (i < n_te + n_ln) {
         const int k = i - n_te;
-        (k < H * F ? p.d_ln_g : p.d_ln_b)[k % (H * F)] = sum;
+        put(k < H * F ? p.d_ln_g : p.d_ln_b, k % (H * F));
         if (p.packed != nullptr) p.packed[(size_t)H * F * F + H * F + k] = sum;
       } else {
         p.packed[i - n_te - n_ln] = sum;
@@ -899,14 +908,14 @@ __global__ void __launch_bounds__(256) ttt_linear_bwd_reduce_kernel(const Reduce
 __global__ void ttt_linear_bwd_fold_kernel(const ReduceParams p) {
   const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float acc = 0.f;
-  for (int s = lane; s < p.T / p.mb; s += 32) acc += p.d_token_eta[s * p.mb + c];
+  for (int s = lane; s < p.T / p.mb; s += 32) acc += p.part_te[s * p.mb + c];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) p.packed[(size_t)p.H * p.F * p.F + 3 * p.H * p.F + c] = acc;
 }
 
 template <typename T, int SEG, int MB>
-static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, const LinBwdParams& p, int nstreams,
+static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, LinBwdParams& p, int nstreams,
                                 cudaStream_t st) {
   using SM = BwdSmem<T, SEG>;
   auto kfn = ttt_linear_bwd_kernel<T, SEG, MB>;
@@ -933,9 +942,16 @@ static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, con
   if (per_sm > 512 / 64) per_sm = 512 / 64;  // tensor-memory columns
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   int grid = sms * per_sm;
+  if (nstreams <= sms && p.item_base == 0) {
+    // every stream alone on an SM: nothing to balance, so no chunks, no hand-offs of the state and no scheduler to clear
+    p.CH = p.NS;
+    p.NCH = 1;
+    p.sched = nullptr;
+  }
   const int nitems = nstreams * p.NCH;
   if (grid > nitems) grid = nitems;
-  if ((e = cudaMemsetAsync(p.sched, 0, sizeof(int) * (size_t)(1 + nstreams), st)) != cudaSuccess) return e;
+  if (p.sched != nullptr && (e = cudaMemsetAsync(p.sched, 0, sizeof(int) * (size_t)(1 + nstreams), st)) != cudaSuccess)
+    return e;
   LinBwdParams pp = p;
   RawTensor raw[7];
   void* args[9];
@@ -949,14 +965,14 @@ static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, con
 }
 
 template <typename T, int SEG>
-static cudaError_t launch_bwd_mb(int mb, const CUtensorMap* m, const void* const* io, const LinBwdParams& p,
+static cudaError_t launch_bwd_mb(int mb, const CUtensorMap* m, const void* const* io, LinBwdParams& p,
                                  int nstreams, cudaStream_t st) {
   return mb == 8 ? launch_bwd_t<T, SEG, 8>(m, io, p, nstreams, st) : launch_bwd_t<T, SEG, 16>(m, io, p, nstreams, st);
 }
 
 // mb: tokens per mini-batch, 16 or 8 (the maps' boxes then have 8 rows)
 cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, const void* const* io,
-                              const LinBwdParams& p, int nstreams, cudaStream_t st) {
+                              LinBwdParams& p, int nstreams, cudaStream_t st) {
   if (seg == 32) {
     if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 32>(mb, maps, io, p, nstreams, st);
     return launch_bwd_mb<float, 32>(mb, maps, io, p, nstreams, st);

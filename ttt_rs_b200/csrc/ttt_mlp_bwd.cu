@@ -1165,19 +1165,32 @@ __global__ void __launch_bounds__(MB_THREADS, 1) ttt_mlp_bwd_kernel(const MlpBwd
 #undef TRM
 }
 
-// grad_token_eta[t] = sum over streams, grad_ln_weight / grad_ln_bias [h][f] = sum over the batch; fixed order.
-__global__ void ttt_mlp_bwd_reduce_kernel(const float* part_te, const float* part_ln, int B, int H, int T, float* dte,
-                                          float* dg, float* db) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// grad_token_eta[t] = sum over streams, grad_ln_weight / grad_ln_bias [h][f] = sum over the batch; fixed order.  Block =
+// 32 consecutive outputs x 8 warps: warp w adds terms w, w + 8, ... (coalesced 128-byte reads), the eight sums are added
+// in warp order.  (One thread per output walking all streams took 14.5 us at 192 streams of 2048 tokens.)
+__global__ void __launch_bounds__(256) ttt_mlp_bwd_reduce_kernel(const float* part_te, const float* part_ln, int B, int H,
+                                                                 int T, int bf16, void* dte, void* dg, void* db) {
+  __shared__ float part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane, n_ln = 2 * H * HD;
+  float acc = 0.f;
   if (i < T) {
-    float s = 0.f;
-    for (int st = 0; st < B * H; ++st) s += part_te[(size_t)st * T + i];
-    dte[i] = s;
-  } else if (i < T + 2 * H * HD) {
+    for (int st = warp; st < B * H; st += 8) acc += part_te[(size_t)st * T + i];
+  } else if (i < T + n_ln) {
     const int j = i - T, which = j / (H * HD), hf = j % (H * HD), h = hf / HD, f = hf % HD;
-    float s = 0.f;
-    for (int b = 0; b < B; ++b) s += part_ln[((size_t)(b * H + h) * 2 + which) * HD + f];
-    (which ? db : dg)[hf] = s;
+    for (int b = warp; b < B; b += 8) acc += part_ln[((size_t)(b * H + h) * 2 + which) * HD + f];
+  }
+  part[warp][lane] = acc;
+  __syncthreads();
+  if (warp == 0 && i < T + n_ln) {
+    float sum = part[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) sum += part[w][lane];
+    const int j = i - T;
+    void* const dst = i < T ? dte : (j < H * HD ? dg : db);
+    const size_t at = i < T ? (size_t)i : (size_t)(j % (H * HD));
+    if (bf16) st_from_float<bf>(dst, at, sum);
+    else st_from_float<float>(dst, at, sum);
   }
 }
 
@@ -1211,8 +1224,8 @@ cudaError_t launch_mlp_bwd(const MlpBwdParams& p0, int B, cudaStream_t st) {
   e = cudaLaunchCooperativeKernel((const void*)ttt_mlp_bwd_kernel, dim3(grid), dim3(MB_THREADS), args, smem, st);
   if (e != cudaSuccess) return e;
   const int n = p.T + 2 * p.H * HD;
-  ttt_mlp_bwd_reduce_kernel<<<(n + 255) / 256, 256, 0, st>>>(p.part_te, p.part_ln, B, p.H, p.T, p.d_token_eta,
-                                                           p.d_ln_g, p.d_ln_b);
+  ttt_mlp_bwd_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(p.part_te, p.part_ln, B, p.H, p.T, p.reduced_bf16,
+                                                         p.d_token_eta, p.d_ln_g, p.d_ln_b);
   return cudaGetLastError();
 }
 

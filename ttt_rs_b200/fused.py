@@ -55,6 +55,7 @@ def device_status(device) -> torch.Tensor:
         if buf is None:
             buf = torch.zeros(_STATUS_WORDS, dtype=torch.int32, device=torch.device("cuda", idx))
             _status_buffers[key] = buf
+            _lib.host().set_status(idx, buf)
         return buf
 
 
@@ -208,6 +209,16 @@ class TttTileMultiKernel:
     def forward_launch(inputs: TttInputs, config: FusedTttConfig,
                        save_state: bool = True) -> Tuple[TttOutputs, Optional[TttSavedStateMulti]]:
         """`save_state=False` (inference): nothing is kept for a backward and the second return value is None."""
+        i, c = inputs, config
+        native = _lib.host().linear_forward(i.xq, i.xk, i.xv, i.weight, i.bias, i.token_eta, i.ttt_lr_eta, i.ln_weight,
+                                            i.ln_bias, c.mini_batch_len, c.head_dim, c.checkpoint_interval,
+                                            c.epsilon_scaled, save_state)
+        if native is not None:
+            outs = TttOutputs(*native[:3])
+            if not save_state:
+                return outs, None
+            return outs, TttSavedStateMulti(i.xq, i.xk, i.xv, i.weight, i.bias, i.token_eta, i.ttt_lr_eta, i.ln_weight,
+                                            i.ln_bias, native[3], native[4], device_status(i.xq.device))
         if config.mini_batch_len <= 0:
             raise TttError(_lib.TTT_ERR_SHAPE, "mini_batch_len must be set for TttTileMultiKernel")
         lib = _lib.load()
@@ -247,6 +258,12 @@ class TttTileMultiKernel:
     def forward_partial(inputs: TttInputs, config: FusedTttConfig, in_place: bool = False) -> TttOutputs:
         """One mini-batch of 1..16 tokens (sequence tail, decode step): `ttt_linear_forward_partial`.  Forward only.
         With `in_place` the state tensors of `inputs` are advanced and returned."""
+        i, c = inputs, config
+        native = _lib.host().linear_partial(i.xq, i.xk, i.xv, i.weight, i.bias, i.token_eta, i.ttt_lr_eta, i.ln_weight,
+                                            i.ln_bias, c.mini_batch_len, c.head_dim, c.checkpoint_interval,
+                                            c.epsilon_scaled, in_place)
+        if native is not None:
+            return TttOutputs(*native)
         lib = _lib.load()
         inputs = inputs.map(lambda t: t.contiguous())
         d = _dims(inputs.xq, config)
@@ -268,6 +285,14 @@ class TttTileMultiKernel:
         """Gradients w.r.t. the nine inputs, in input order.  By default only `grad_outputs.output` is used: upstream
         gradients of the returned final state are ignored, as in the reference.  With `use_state_grads=True`,
         `grad_outputs.weight` / `.bias` (when not None) are taken as the gradients flowing into the final state."""
+        s, c = saved, config
+        native = _lib.host().linear_backward(
+            s.xq, s.xk, s.xv, s.weight_init, s.bias, s.token_eta, s.ttt_lr_eta, s.ln_weight, s.ln_bias,
+            s.weight_checkpoints, s.bias_checkpoints, grad_outputs.output, c.mini_batch_len, c.head_dim,
+            c.checkpoint_interval, c.epsilon_scaled, outer_grad_packed, grad_outputs.weight if use_state_grads else None,
+            grad_outputs.bias if use_state_grads else None)
+        if native is not None:
+            return TttInputs(*native, status=device_status(s.xq.device))
         if config.mini_batch_len <= 0:
             raise TttError(_lib.TTT_ERR_SHAPE, "mini_batch_len must be set for TttTileMultiKernel backward")
         lib = _lib.load()
@@ -362,6 +387,11 @@ def fused_ttt_tile_forward_multi(xq, xk, xv, weight, bias, token_eta, ttt_lr_eta
         outs, _ = TttTileMultiKernel.forward_launch(
             TttInputs(xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias), config, save_state=False)
         return outs.output, outs.weight, outs.bias
+    native = _lib.host().linear_apply(xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias,
+                                      config.mini_batch_len, config.head_dim, config.checkpoint_interval,
+                                      config.epsilon_scaled)
+    if native is not None:
+        return native
     return _FusedTttTileMultiFn.apply(xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, config)
 
 
@@ -513,6 +543,12 @@ def fused_ttt_mlp_forward(xq, xk, xv, state: TTTMLPState, token_eta, ttt_lr_eta,
     `TTTMLP::forward_mini_batch`, rust/core/src/mlp.rs:127-208).  Returns (output, new TTTMLPState).
     bf16 only.  Its gradient is `fused_ttt_mlp_backward` (no autograd node is recorded here); a buffer from
     `mlp_backward_workspace` passed as `backward_workspace` is filled for it."""
+    st, c = state, config
+    native = _lib.host().mlp_forward(xq, xk, xv, st.w1, st.b1, st.w2, st.b2, token_eta, ttt_lr_eta, ln_weight, ln_bias,
+                                     c.mini_batch_len, c.head_dim, c.checkpoint_interval, c.epsilon_scaled,
+                                     backward_workspace)
+    if native is not None:
+        return native[0], TTTMLPState(*native[1:])
     lib = _lib.load()
     if not xq.is_cuda:
         raise TttError(_lib.TTT_ERR_CUDA, "inputs must be CUDA tensors: this operator has no CPU path")
@@ -626,8 +662,13 @@ class _FusedTttMlpFn(torch.autograd.Function):
 
 def fused_ttt_mlp(xq, xk, xv, state: TTTMLPState, token_eta, ttt_lr_eta, ln_weight, ln_bias, config: FusedTttConfig):
     """Differentiable whole-sequence TTT-MLP inner loop: returns (output, new TTTMLPState)."""
-    out, w1, b1, w2, b2 = _FusedTttMlpFn.apply(xq, xk, xv, state.w1, state.b1, state.w2, state.b2, token_eta,
-                                               ttt_lr_eta, ln_weight, ln_bias, config)
+    native = _lib.host().mlp_apply(xq, xk, xv, state.w1, state.b1, state.w2, state.b2, token_eta, ttt_lr_eta, ln_weight,
+                                   ln_bias, config.mini_batch_len, config.head_dim, config.checkpoint_interval,
+                                   config.epsilon_scaled)
+    if native is None:
+        native = _FusedTttMlpFn.apply(xq, xk, xv, state.w1, state.b1, state.w2, state.b2, token_eta, ttt_lr_eta,
+                                      ln_weight, ln_bias, config)
+    out, w1, b1, w2, b2 = native
     return out, TTTMLPState(w1, b1, w2, b2)
 
 
