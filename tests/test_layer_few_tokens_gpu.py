@@ -1,0 +1,30 @@
+"""The outer layer on few tokens (decode steps, short prompts: `ttt_layer_small_*`) and on lengths that leave a remainder
+(pitched inner loop and tail), against the CPU restatement."""
+
+import pytest
+import torch
+
+from conftest import assert_close
+from oracle import ttt_layer_oracle as LO
+from test_layer_gpu import _layer_from_params, _random_case
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T,H,F,use_gate,start", (
+    (1, 1, 1, 64, False, 0), (8, 1, 12, 64, True, 21), (17, 1, 12, 64, False, 3), (1, 1, 4, 32, True, 0),
+    (2, 16, 4, 32, False, 0), (1, 31, 3, 64, True, 0), (4, 7, 24, 32, False, 5), (32, 1, 32, 64, True, 9),
+    (33, 1, 12, 64, True, 9), (1, 41, 3, 64, True, 0), (2, 145, 4, 32, False, 0)))
+def test_short_and_ragged_calls_match_the_restatement(B, T, H, F, use_gate, start):
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    x, p = _random_case(B, T, H, 41 + B, False, use_gate, torch.bfloat16, F)
+    m, inner = _layer_from_params(tb, p, False, use_gate, torch.bfloat16, dev, H)
+    inner.allow_partial = True
+    with torch.no_grad():
+        state = inner.init_state(B)
+        y = m(x.to(torch.bfloat16).to(dev), inner, state, start)
+    tb.TttTileMultiKernel.check_status()
+    want, st = LO.ttt_layer_forward(x, p, num_heads=H, use_gate=use_gate, start_idx=start)
+    assert_close(y, want, 3e-2, "layer output", max_bad_frac=1e-3)
+    assert_close(state.weight, st["weight"], 2e-2, "state weight", max_bad_frac=1e-3)
+    assert_close(state.bias, st["bias"], 2e-2, "state bias", max_bad_frac=5e-3)

@@ -363,7 +363,7 @@ size_t ttt_linear_bias_ckpt_bytes(const ttt_dims* d) {
   return aux_layout(d).total_bytes;
 }
 
-int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* weight,
+static int linear_forward_impl(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk, const void* xv, const void* weight,
                        const void* bias, const void* token_eta, const void* ttt_lr_eta, const void* ln_weight,
                        const void* ln_bias, void* output, void* weight_out, void* bias_out, void* weight_ckpt,
                        void* bias_ckpt, void* status, void* stream) {
@@ -388,12 +388,14 @@ int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const 
   uint8_t* aux = static_cast<uint8_t*>(bias_ckpt);
   CUtensorMap maps[5];
   const void* bases[4] = {xq, xk, xv, output};
+  ttt_dims dm = *d;  // the tensors as they lie in memory
+  dm.seq_len = seq_pitch;
   for (int i = 0; i < 4; ++i) {
-    rc = make_io_map(&maps[i], bases[i], d);
+    rc = make_io_map(&maps[i], bases[i], &dm);
     if (rc != TTT_OK) return rc;
   }
   // the saved Gp tiles are always kept 64 wide; without saved state the map is never used, but must be a valid one
-  rc = save ? make_tile_map(&maps[4], aux + al.off_gp, pk.rows, d->dtype, d->mini_batch) : make_io_map(&maps[4], output, d);
+  rc = save ? make_tile_map(&maps[4], aux + al.off_gp, pk.rows, d->dtype, d->mini_batch) : make_io_map(&maps[4], output, &dm);
   if (rc != TTT_OK) return rc;
   ttt::LinFwdParams p;
   p.w0 = weight;
@@ -409,7 +411,8 @@ int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const 
   p.b_stage = save ? reinterpret_cast<float*>(aux + al.off_bias) : nullptr;
   p.status = static_cast<uint32_t*>(status);
   p.H = pk.heads;
-  p.T = d->seq_len;
+  p.T = seq_pitch;
+  p.lr_ld = lr_pitch;
   p.NS = d->seq_len / d->mini_batch;
   p.K = d->checkpoint_interval;
   p.NCK = (int)num_ckpt(d);
@@ -419,6 +422,28 @@ int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const 
                              static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
+}
+
+int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* weight,
+                       const void* bias, const void* token_eta, const void* ttt_lr_eta, const void* ln_weight,
+                       const void* ln_bias, void* output, void* weight_out, void* bias_out, void* weight_ckpt,
+                       void* bias_ckpt, void* status, void* stream) {
+  const int T = d != nullptr ? d->seq_len : 0;
+  return linear_forward_impl(d, T, T, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, output,
+                             weight_out, bias_out, weight_ckpt, bias_ckpt, status, stream);
+}
+
+int ttt_internal_linear_infer(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk,
+                              const void* xv, const void* weight, const void* bias, const void* token_eta,
+                              const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
+                              void* weight_out, void* bias_out, void* status, void* stream) {
+  if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
+  if (seq_pitch < d->seq_len || lr_pitch < d->seq_len || (int64_t)lr_pitch * (d->dtype == TTT_BF16 ? 2 : 4) % 16 != 0)
+    return fail(TTT_ERR_SHAPE, "pitches must cover the sequence, learning-rate rows start on 16 bytes");
+  if ((int64_t)d->batch * d->heads * seq_pitch >= (int64_t)1 << 31)
+    return fail(TTT_ERR_SHAPE, "batch*heads*seq_pitch must be below 2^31");
+  return linear_forward_impl(d, seq_pitch, lr_pitch, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias,
+                             output, weight_out, bias_out, nullptr, nullptr, status, stream);
 }
 
 size_t ttt_linear_backward_workspace_bytes(const ttt_dims* d) {
@@ -693,12 +718,12 @@ int check_layer_dims(const ttt_dims* d) {
 }
 }  // namespace
 
-extern "C" int ttt_layer_prologue(const ttt_dims* d, const void* q_src, const void* k_src, const void* v_src,
+extern "C" int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src, const void* k_src, const void* v_src,
                                   int64_t src_ld, const void* lr_logits, int64_t lr_ld, const void* lr_bias,
                                   const void* conv_q_weight, const void* conv_q_bias, const void* conv_k_weight,
                                   const void* conv_k_bias, int conv_kernel, int start_idx, int rope_mode,
                                   float rope_theta, float base_lr, void* xq, void* xk, void* xv, void* ttt_lr_eta,
-                                  void* stream) {
+                                  int lr_pitch, void* stream) {
   int rc = check_layer_dims(d);
   if (rc != TTT_OK) return rc;
   const bool conv = conv_q_weight != nullptr;
@@ -711,6 +736,7 @@ extern "C" int ttt_layer_prologue(const ttt_dims* d, const void* q_src, const vo
     return fail(TTT_ERR_UNSUPPORTED, "wrapped rotary positions need 1 <= mini_batch <= 64 (got %d)", d->mini_batch);
   if (rope_mode != 0 && !(rope_theta > 0.f)) return fail(TTT_ERR_SHAPE, "rope_theta must be positive");
   if (start_idx < 0) return fail(TTT_ERR_SHAPE, "start_idx must be >= 0");
+  if (lr_pitch < d->seq_len) return fail(TTT_ERR_SHAPE, "lr_pitch must be >= seq_len");
   const int64_t cols = (int64_t)d->heads * d->head_dim;
   if (src_ld < cols || (src_ld & 7) != 0)
     return fail(TTT_ERR_SHAPE, "src_ld (%lld) must be >= heads*head_dim and a multiple of 8", (long long)src_ld);
@@ -737,6 +763,7 @@ extern "C" int ttt_layer_prologue(const ttt_dims* d, const void* q_src, const vo
   p.xk = xk;
   p.xv = xv;
   p.lr_out = ttt_lr_eta;
+  p.lr_ld_out = lr_pitch;
   p.B = d->batch;
   p.H = d->heads;
   p.T = d->seq_len;
@@ -748,6 +775,17 @@ extern "C" int ttt_layer_prologue(const ttt_dims* d, const void* q_src, const vo
   cudaError_t e = ttt::launch_layer_prologue(d->dtype, d->head_dim, p, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "layer prologue launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
+}
+
+extern "C" int ttt_layer_prologue(const ttt_dims* d, const void* q_src, const void* k_src, const void* v_src,
+                                  int64_t src_ld, const void* lr_logits, int64_t lr_ld, const void* lr_bias,
+                                  const void* conv_q_weight, const void* conv_q_bias, const void* conv_k_weight,
+                                  const void* conv_k_bias, int conv_kernel, int start_idx, int rope_mode,
+                                  float rope_theta, float base_lr, void* xq, void* xk, void* xv, void* ttt_lr_eta,
+                                  void* stream) {
+  return ttt_internal_layer_prologue(d, q_src, k_src, v_src, src_ld, lr_logits, lr_ld, lr_bias, conv_q_weight,
+                                     conv_q_bias, conv_k_weight, conv_k_bias, conv_kernel, start_idx, rope_mode,
+                                     rope_theta, base_lr, xq, xk, xv, ttt_lr_eta, d != nullptr ? d->seq_len : 0, stream);
 }
 
 extern "C" int ttt_layer_epilogue(const ttt_dims* d, const void* inner_out, const void* gate, int64_t gate_ld,
@@ -783,7 +821,7 @@ extern "C" int ttt_layer_epilogue(const ttt_dims* d, const void* inner_out, cons
   return TTT_OK;
 }
 
-extern "C" int ttt_linear_forward_partial(const ttt_dims* d, const void* xq, const void* xk, const void* xv,
+extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled, const void* xq, const void* xk, const void* xv,
                                           const void* weight, const void* bias, const void* token_eta,
                                           const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
                                           void* output, void* weight_out, void* bias_out, void* stream) {
@@ -816,9 +854,64 @@ extern "C" int ttt_linear_forward_partial(const ttt_dims* d, const void* xq, con
   p.b_out = bias_out;
   p.H = d->heads;
   p.R = d->seq_len;
+  p.row_ld = seq_pitch;
+  p.row_off = first;
+  p.lr_ld = lr_pitch;
+  p.state_settled = state_settled;
   p.eps = d->epsilon;
   cudaError_t e = ttt::launch_linear_partial(d->dtype, d->head_dim, p, d->batch * d->heads, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "partial forward launch failed: %s", cudaGetErrorString(e));
+  return TTT_OK;
+}
+
+extern "C" int ttt_linear_forward_partial(const ttt_dims* d, const void* xq, const void* xk, const void* xv,
+                                          const void* weight, const void* bias, const void* token_eta,
+                                          const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
+                                          void* output, void* weight_out, void* bias_out, void* stream) {
+  const int T = d != nullptr ? d->seq_len : 0;
+  return ttt_internal_linear_tail(d, T, 0, T, 0, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, output,
+                                  weight_out, bias_out, stream);
+}
+
+extern "C" int ttt_internal_layer_small_fits(const ttt_dims* d) {
+  const int64_t C = (int64_t)d->heads * d->head_dim, M = (int64_t)d->batch * d->seq_len;
+  return d->dtype == TTT_BF16 && (d->head_dim == 64 || d->head_dim == 32) && C <= 2048 && C % 32 == 0 && M <= ttt::SMALL_M;
+}
+
+extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, int64_t x_ld, const void* weights,
+                                             int64_t w_ld, int w_rows, int lr_col, const void* lr_bias, int start_idx,
+                                             int rope_mode, float rope_theta, float base_lr, void* xq, void* xk,
+                                             void* xv, void* gate, void* ttt_lr_eta, int lr_pitch, void* stream) {
+  if (!ttt_internal_layer_small_fits(d)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
+  if (x_ld % 8 != 0 || w_ld % 8 != 0) return fail(TTT_ERR_ALIGN, "row pitches must be multiples of 8 elements");
+  const NamedPtr ptrs[] = {{"x", x}, {"weights", weights}, {"xq", xq}, {"xk", xk}, {"xv", xv}};
+  if (const int rc = check_ptrs(ptrs, 5); rc != TTT_OK) return rc;
+  ttt::SmallProjParams p;
+  p.x = x; p.w = weights; p.lr_bias = lr_bias;
+  p.xq = xq; p.xk = xk; p.xv = xv; p.gate = gate; p.lr_out = ttt_lr_eta;
+  p.M = d->batch * d->seq_len; p.N = w_rows; p.K = d->heads * d->head_dim; p.ldx = (int)x_ld; p.ldw = (int)w_ld;
+  p.H = d->heads; p.F = d->head_dim; p.T = d->seq_len; p.lr_col = lr_col; p.lr_ld = lr_pitch;
+  p.start_idx = start_idx; p.pos_mod = rope_mode == 1 ? d->mini_batch : 1; p.rope_mode = rope_mode;
+  p.rope_theta = rope_mode != 0 ? rope_theta : 1.f; p.base_lr = base_lr;
+  cudaError_t e = ttt::launch_layer_small_proj(p, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "few-token projection launch failed: %s", cudaGetErrorString(e));
+  return TTT_OK;
+}
+
+extern "C" int ttt_internal_layer_small_out(const ttt_dims* d, const void* inner_out, const void* gate, int gate_ld,
+                                            const void* post_norm_weight, const void* post_norm_bias, float eps,
+                                            const void* o_proj, int64_t o_ld, void* y, void* stream) {
+  if (!ttt_internal_layer_small_fits(d)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
+  if (gate_ld % 8 != 0 || o_ld % 8 != 0) return fail(TTT_ERR_ALIGN, "row pitches must be multiples of 8 elements");
+  const NamedPtr ptrs[] = {{"inner_out", inner_out}, {"post_norm_weight", post_norm_weight},
+                           {"post_norm_bias", post_norm_bias}, {"o_proj", o_proj}, {"y", y}};
+  if (const int rc = check_ptrs(ptrs, 5); rc != TTT_OK) return rc;
+  ttt::SmallOutParams p;
+  p.inner_out = inner_out; p.gate = gate; p.ln_w = post_norm_weight; p.ln_b = post_norm_bias; p.w = o_proj; p.y = y;
+  p.M = d->batch * d->seq_len; p.H = d->heads; p.F = d->head_dim; p.T = d->seq_len; p.ldw = (int)o_ld;
+  p.ld_gate = gate_ld; p.eps = eps;
+  cudaError_t e = ttt::launch_layer_small_out(p, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "few-token output launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
 }
 

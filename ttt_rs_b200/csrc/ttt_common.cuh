@@ -340,4 +340,26 @@ __device__ __forceinline__ void tmem_st_8x4(uint32_t taddr, const float (&r)[8][
       : "memory");
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------------------------------
+// A kernel launched with launch_dependent may begin while the kernel before it on the stream drains: its launch and
+// prologue (and loads of data that neither the kernel before nor an unfinished one writes) are off the chain.
+// pdl_wait: everything before on the stream is complete and visible.  pdl_go: the next kernel may begin; called after
+// pdl_wait, so that at most one kernel is unfinished when a later one starts.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 }  // namespace ttt

@@ -395,6 +395,164 @@ PyObject* py_mlp_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- the outer layer, inference ------------------------------------------------------------------------------------
+// param_key(tensors...) -> bytes that change with any tensor's storage, version, dtype or device (None entries allowed)
+PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  PyObject* r = PyBytes_FromStringAndSize(nullptr, n * 16);
+  if (!r) return nullptr;
+  uint64_t* k = reinterpret_cast<uint64_t*>(PyBytes_AS_STRING(r));
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    k[2 * i] = k[2 * i + 1] = 0;
+    if (!THPVariable_Check(args[i])) continue;
+    const Tensor& t = THPVariable_Unpack(args[i]);
+    k[2 * i] = reinterpret_cast<uint64_t>(t.const_data_ptr());
+    k[2 * i + 1] = ((uint64_t)t._version() << 16) | ((uint64_t)t.scalar_type() << 8) | (uint64_t)(uint8_t)t.device().index();
+  }
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// layer_infer(x, stacked weights, token_eta of one mini-batch, lr_bias, conv q weight / bias, conv k weight / bias (or four
+//             None), state weight, state bias, ln weight, ln bias, post norm weight, bias, o_proj, gate 0/1, heads,
+//             mini_batch, rope_mode, rope_theta, base_lr, lr_col, eps_scaled, allow_partial, in_place, start_idx)
+//   -> (y, state weight, state bias) | None
+// One call of TTT.forward without gradients, bf16: projections + prologue, inner loop (whole mini-batches, then the
+// remainder as a mini-batch of its own), post norm (+ gate), output projection.
+PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 26)) return nullptr;
+  Tensor t[15];
+  for (int i = 0; i < 15; ++i) {
+    if (args[i] == Py_None && i >= 4 && i < 8) continue;
+    NONE_IF(!THPVariable_Check(args[i]));
+    t[i] = THPVariable_Unpack(args[i]);
+  }
+  const Tensor &x = t[0], &wcat = t[1], &te = t[2], &lr_bias = t[3], &sw = t[8], &sb = t[9];
+  const bool use_gate = as_int(args[15]) != 0, conv = t[4].defined();
+  const int64_t H = as_int(args[16]), mb = as_int(args[17]), rope = as_int(args[18]), lr_col = as_int(args[21]);
+  const float theta = (float)PyFloat_AsDouble(args[19]), base_lr = (float)PyFloat_AsDouble(args[20]);
+  const int64_t eps_scaled = as_int(args[22]), start = as_int(args[25]);
+  const bool allow_partial = args[23] == Py_True, in_place = args[24] == Py_True;
+  if (PyErr_Occurred()) return nullptr;
+
+  NONE_IF(!x.is_cuda() || x.dim() != 3 || x.scalar_type() != at::kBFloat16 || H <= 0);
+  const c10::Device dev = x.device();
+  const at::ScalarType bf = at::kBFloat16;
+  const int64_t B = x.size(0), T = x.size(1), C = x.size(2), F = C / H, M = B * T;
+  // rows of x: one pitch for all tokens
+  NONE_IF(M <= 0 || F * H != C || (F != 64 && F != 32) || C > 2048 || C % 8 != 0 || x.stride(2) != 1);
+  const int64_t x_ld = T > 1 ? x.stride(1) : x.stride(0);
+  NONE_IF((T > 1 && B > 1 && x.stride(0) != T * x_ld) || x_ld < C || x_ld % 8 != 0);
+  const int64_t N = wcat.size(0);
+  NONE_IF(!is(wcat, bf, dev, {N, C}) || te.dim() != 1 || te.size(0) < mb || !is(te, bf, dev, {te.size(0)}));
+  NONE_IF(lr_bias.numel() != H || lr_bias.scalar_type() != bf || !lr_bias.is_contiguous() || lr_bias.device() != dev);
+  NONE_IF(!is(sw, bf, dev, {B, H, F, F}) || !is(sb, bf, dev, {B, H, F}) || !is(t[10], bf, dev, {H, F}) ||
+          !is(t[11], bf, dev, {H, F}) || !is(t[12], bf, dev, {C}) || !is(t[13], bf, dev, {C}) || !is(t[14], bf, dev, {C, C}));
+  int conv_k = 0;
+  if (conv) {
+    for (int i = 4; i < 8; ++i)
+      NONE_IF(!t[i].defined() || t[i].scalar_type() != bf || !t[i].is_contiguous() || t[i].device() != dev || t[i].size(0) != C);
+    conv_k = (int)(t[4].numel() / C);
+    NONE_IF(t[5].numel() != C || t[7].numel() != C || t[6].numel() != t[4].numel());
+  }
+  const int64_t L = T / mb * mb, R = T - L;
+  NONE_IF(R != 0 && !allow_partial);
+  Dims m;
+  m.dt = bf;
+  m.dev = dev;
+  m.status = g_status[dev.index()];
+  NONE_IF(!m.status.defined() || M > INT32_MAX || H > 64);
+  ttt_dims d{(int32_t)B, (int32_t)H, (int32_t)T, (int32_t)F, (int32_t)mb, 1, (float)eps_scaled * 1e-9f, TTT_BF16};
+
+  c10::cuda::CUDAGuard guard(dev);
+  void* const st = m.stream();
+  void* const status = m.status.data_ptr();
+  const bool small = !conv && ttt_internal_layer_small_fits(&d);
+  const bool fused = !small && !conv && T % 128 == 0 && F == 64 && rope != 2 && mb <= 16 && lr_col % 64 == 0;
+  // temporaries from one allocation, each on a 256-byte boundary
+  int64_t at_ = 0;
+  auto room = [&](int64_t elements) {
+    const int64_t o = at_;
+    at_ += (elements * 2 + 255) & ~(int64_t)255;
+    return o;
+  };
+  const int64_t lr_pitch = (T + 7) & ~(int64_t)7;
+  const int64_t o_q = room(M * C), o_k = room(M * C), o_v = room(M * C), o_lr = room(B * H * lr_pitch), o_in = room(M * C);
+  const int64_t o_proj = small || fused ? 0 : room(M * N);
+  const int64_t o_gate = use_gate && (small || fused) ? room(M * C) : 0;
+  const int64_t o_y = small ? 0 : room(M * C);
+  Tensor tmp = at::empty({at_}, m.opt(at::kByte));
+  uint8_t* const base = static_cast<uint8_t*>(tmp.data_ptr());
+  Tensor y = at::empty({B, T, C}, m.opt());
+  const uint8_t* gate = nullptr;
+  int64_t gate_ld = C;
+  const int64_t g_col = lr_col - C;
+  // ---- projections, head split, rotary embedding, learning rates
+  if (small) {
+    NONE_IF(ttt_internal_layer_small_proj(&d, x.const_data_ptr(), x_ld, wcat.const_data_ptr(), C, (int)N, (int)lr_col,
+                                          lr_bias.const_data_ptr(), (int)start, (int)rope, theta, base_lr, base + o_q,
+                                          base + o_k, base + o_v, use_gate ? base + o_gate : nullptr, base + o_lr,
+                                          (int)lr_pitch, st) != TTT_OK);
+    if (use_gate) gate = base + o_gate;
+  } else if (fused) {
+    NONE_IF(ttt_layer_projections(&d, x.const_data_ptr(), x_ld, C, wcat.const_data_ptr(), C, N, 0, C, 2 * C,
+                                  use_gate ? g_col : -1, lr_col, lr_bias.const_data_ptr(), (int)start, (int)rope, theta,
+                                  base_lr, base + o_q, base + o_k, base + o_v, use_gate ? base + o_gate : nullptr,
+                                  base + o_lr, status, st) != TTT_OK);
+    if (use_gate) gate = base + o_gate;
+  } else {
+    uint8_t* const proj = base + o_proj;
+    NONE_IF(N % 8 != 0);
+    NONE_IF(ttt_gemm_bf16_tn(M, N, C, x.const_data_ptr(), x_ld, wcat.const_data_ptr(), C, proj, N, status, st) != TTT_OK);
+    const int64_t k_col = conv ? 0 : C, v_col = conv ? C : 2 * C;
+    NONE_IF(ttt_internal_layer_prologue(&d, proj, proj + 2 * k_col, proj + 2 * v_col, N, proj + 2 * lr_col, N,
+                                        lr_bias.const_data_ptr(), conv ? t[4].const_data_ptr() : nullptr,
+                                        conv ? t[5].const_data_ptr() : nullptr, conv ? t[6].const_data_ptr() : nullptr,
+                                        conv ? t[7].const_data_ptr() : nullptr, conv_k, (int)start, (int)rope, theta,
+                                        base_lr, base + o_q, base + o_k, base + o_v, base + o_lr, (int)lr_pitch,
+                                        st) != TTT_OK);
+    if (use_gate) gate = proj + 2 * g_col, gate_ld = N;
+  }
+  // ---- inner loop
+  Tensor w = sw, b = sb;
+  if (L > 0) {
+    w = at::empty({B, H, F, F}, m.opt());
+    b = at::empty({B, H, F}, m.opt());
+    ttt_dims di = d;
+    di.seq_len = (int32_t)L;
+    NONE_IF(ttt_internal_linear_infer(&di, (int)T, (int)lr_pitch, base + o_q, base + o_k, base + o_v,
+                                      sw.const_data_ptr(), sb.const_data_ptr(), te.const_data_ptr(), base + o_lr,
+                                      t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in, w.data_ptr(),
+                                      b.data_ptr(), status, st) != TTT_OK);
+  }
+  if (R > 0) {
+    const Tensor w_in = w, b_in = b;
+    if (L == 0 && !in_place) {
+      w = at::empty({B, H, F, F}, m.opt());
+      b = at::empty({B, H, F}, m.opt());
+    }
+    ttt_dims dt = d;
+    dt.seq_len = (int32_t)R;
+    NONE_IF(ttt_internal_linear_tail(&dt, (int)T, (int)L, (int)lr_pitch, small && L == 0, base + o_q, base + o_k, base + o_v,
+                                     w_in.const_data_ptr(), b_in.const_data_ptr(), te.const_data_ptr(), base + o_lr,
+                                     t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in,
+                                     const_cast<void*>(w.const_data_ptr()), const_cast<void*>(b.const_data_ptr()),
+                                     st) != TTT_OK);
+  }
+  // ---- post norm, gate, output projection
+  if (small) {
+    NONE_IF(ttt_internal_layer_small_out(&d, base + o_in, gate, (int)gate_ld, t[12].const_data_ptr(),
+                                         t[13].const_data_ptr(), 1e-6f, t[14].const_data_ptr(), C, y.data_ptr(), st) != TTT_OK);
+  } else {
+    NONE_IF(ttt_layer_epilogue(&d, base + o_in, gate, gate != nullptr ? gate_ld : 0, t[12].const_data_ptr(),
+                               t[13].const_data_ptr(), 1e-6f, base + o_y, st) != TTT_OK);
+    NONE_IF(ttt_gemm_bf16_tn(M, C, C, base + o_y, C, t[14].const_data_ptr(), C, y.data_ptr(), C, status, st) != TTT_OK);
+  }
+  return wrap({y, w, b});
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST(set_status),
@@ -404,6 +562,8 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST(linear_apply),
                          FAST(mlp_forward),
                          FAST(mlp_apply),
+                         FAST(param_key),
+                         FAST(layer_infer),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

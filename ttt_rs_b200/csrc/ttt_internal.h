@@ -27,4 +27,34 @@ int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, const void* xk,
                               void* grad_ln_weight, void* grad_ln_bias, int reduced_dtype, void* workspace,
                               size_t workspace_bytes, int workspace_from_forward, void* status, void* stream);
 
+// Inference forward over the first `d->seq_len` tokens (whole mini-batches) of sequences whose rows are `seq_pitch` tokens
+// apart in xq, xk, xv, output and `lr_pitch` elements apart in ttt_lr_eta; token_eta: the first mini-batch's.
+int ttt_internal_linear_infer(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk,
+                              const void* xv, const void* weight, const void* bias, const void* token_eta,
+                              const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
+                              void* weight_out, void* bias_out, void* status, void* stream);
+// ttt_linear_forward_partial on tokens [first, first + d->seq_len) of such sequences.  state_settled: the launch before
+// this one on the stream was ttt_internal_layer_small_proj (the state may be read before that has finished).
+int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled, const void* xq, const void* xk,
+                             const void* xv, const void* weight, const void* bias, const void* token_eta,
+                             const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
+                             void* weight_out, void* bias_out, void* stream);
+// ttt_layer_prologue with rows of lr_pitch elements in ttt_lr_eta
+int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src, const void* k_src, const void* v_src,
+                                int64_t src_ld, const void* lr_logits, int64_t lr_ld, const void* lr_bias,
+                                const void* conv_q_weight, const void* conv_q_bias, const void* conv_k_weight,
+                                const void* conv_k_bias, int conv_kernel, int start_idx, int rope_mode,
+                                float rope_theta, float base_lr, void* xq, void* xk, void* xv, void* ttt_lr_eta,
+                                int lr_pitch, void* stream);
+// Few-token forms (bf16): projections with the prologue, and post norm (+ gate) with the output projection; 0 from
+// _fits: not for this shape.  weights: q | k | v | (gate) blocks of heads * head_dim rows, learning-rate rows from lr_col.
+int ttt_internal_layer_small_fits(const ttt_dims* d);
+int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, int64_t x_ld, const void* weights, int64_t w_ld,
+                                  int w_rows, int lr_col, const void* lr_bias, int start_idx, int rope_mode,
+                                  float rope_theta, float base_lr, void* xq, void* xk, void* xv, void* gate,
+                                  void* ttt_lr_eta, int lr_pitch, void* stream);
+int ttt_internal_layer_small_out(const ttt_dims* d, const void* inner_out, const void* gate, int gate_ld,
+                                 const void* post_norm_weight, const void* post_norm_bias, float eps, const void* o_proj,
+                                 int64_t o_ld, void* y, void* stream);
+
 }  // extern "C"

@@ -11,7 +11,7 @@ struct LinFwdParams {
   const void* w0;         // [B,H,F,F] element type T
   const void* b0;         // [B,H,F]
   const void* token_eta;  // [T], first 16 entries read
-  const void* lr;         // [B,H,T]
+  const void* lr;         // [B,H,lr_ld], lr_ld elements per (batch, head): T, or more where the caller pads the rows
   const void* ln_g;       // [H,F]
   const void* ln_b;       // [H,F]
   void* w_out;            // [B,H,F,F]
@@ -20,7 +20,8 @@ struct LinFwdParams {
   float4* stats;          // [B*H*T][2]: (mean1, rstd1, A, Bv), (mean2, rstd2, 0, 0) per token
   float* b_stage;         // [B*H*(NS+1), F] float32: bias at the start of every stage, final bias last
   uint32_t* status;       // device uint32[4] or null
-  int H, T, NS, K, NCK;
+  int H, T, NS, K, NCK;   // T: tokens per stream in memory (NS mini-batches of them are walked)
+  int lr_ld;
   float eps;
 };
 
@@ -108,7 +109,9 @@ struct LayerProParams {
   void* xq;            // [B,H,T,F]
   void* xk;
   void* xv;
-  void* lr_out;        // [B,H,T]
+  void* lr_out;        // [B,H,lr_ld_out] (lr_ld_out >= T)
+  int lr_ld_out;
+  int tchunk;          // tokens per warp task, set by the launcher
   int B, H, T;
   int start_idx, pos_mod, rope_mode;  // rope_mode: 0 none, 1 positions modulo pos_mod, 2 global positions
   float rope_theta, base_lr;
@@ -123,6 +126,28 @@ struct LayerEpiParams {
   int B, H, T;
   float eps;
 };
+// Few-token forms of the layer's two sides (ttt_layer_small.cu): up to SMALL_M rows, bf16, head_dim 64 or 32, at most 2048
+// features, hidden a multiple of 32
+constexpr int SMALL_M = 32;
+struct SmallProjParams {
+  const void* x;  // [M, ldx], rows b * T + t
+  const void* w;  // [N, ldw]: q | k | v | (gate) blocks of H F rows, then H learning-rate rows from lr_col on
+  const void* lr_bias;
+  void *xq, *xk, *xv, *gate, *lr_out;  // [B,H,T,F] x 3, [M, H F] or null, [B,H,lr_ld]
+  int M, N, K, ldx, ldw, H, F, T, lr_col, lr_ld;
+  int start_idx, pos_mod, rope_mode;
+  float rope_theta, base_lr;
+};
+struct SmallOutParams {
+  const void* inner_out;  // [B,H,T,F]
+  const void* gate;       // [M, ld_gate] or null
+  const void *ln_w, *ln_b, *w;  // w [H F, ldw]
+  void* y;                // [M, H F]
+  int M, H, F, T, ldw, ld_gate;
+  float eps;
+};
+cudaError_t launch_layer_small_proj(const SmallProjParams& p, cudaStream_t st);
+cudaError_t launch_layer_small_out(const SmallOutParams& p, cudaStream_t st);
 struct LayerProBwdParams {
   const void* dxq;  // [B,H,T,F] gradients of the prologue's outputs
   const void* dxk;
@@ -137,6 +162,7 @@ struct LayerProBwdParams {
   long ld_dlr;
   int lr_cols;
   int B, H, T;
+  int tchunk;  // set by the launcher
   int start_idx, pos_mod, rope_mode;
   float rope_theta, base_lr;
 };
@@ -194,21 +220,26 @@ size_t layer_epilogue_bwd_workspace_bytes(int B, int H, int T, int head_dim);
 cudaError_t launch_layer_epilogue(int dtype, int head_dim, const LayerEpiParams& p, cudaStream_t st);
 
 // One mini-batch of R <= 16 tokens per stream (decode step, sequence tail): ttt_linear_partial.cu.
+// One mini-batch of R rows per stream; row i of stream s is row s * row_ld + row_off + i of xq, xk, xv, out, and element
+// s * lr_ld + row_off + i of lr (a mini-batch of its own: row_ld = lr_ld = R, row_off = 0; the tail of a longer sequence:
+// the sequence's pitch and the tail's first token).
 struct LinPartialParams {
-  const void* xq;  // [B,H,R,F]
+  const void* xq;  // [B,H,row_ld,F]
   const void* xk;
   const void* xv;
   const void* w0;         // [B,H,F,F]
   const void* b0;         // [B,H,F]
   const void* token_eta;  // [R]
-  const void* lr;         // [B,H,R]
+  const void* lr;         // [B,H,lr_ld]
   const void* ln_g;       // [H,F]
   const void* ln_b;
-  void* out;              // [B,H,R,F]
+  void* out;              // [B,H,row_ld,F]
   void* w_out;            // may alias w0
   void* b_out;            // may alias b0
   int H, R;
+  int row_ld, row_off, lr_ld;
   float eps;
+  int state_settled;  // the kernel before this one on the stream does not write the state (see launch_dependent)
 };
 cudaError_t launch_linear_partial(int dtype, int head_dim, const LinPartialParams& p, int nstreams, cudaStream_t st);
 

@@ -60,7 +60,7 @@ struct Vec8<float> {
 };
 
 constexpr int PRO_THREADS = 256;
-constexpr int PRO_TCHUNK = 32;   // tokens per warp task
+constexpr int PRO_TCHUNK = 32;   // tokens per warp task, at most
 constexpr int PRO_MAXK = 4;      // causal convolution taps supported
 constexpr int PRO_MAXPOS = 64;   // rotary table rows (positions modulo the mini-batch length)
 
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
   __syncthreads();
 
   const int hq = lane / SUBS, sub = lane % SUBS;
-  const int hgroups = (H + HPW - 1) / HPW, tchunks = (NT + PRO_TCHUNK - 1) / PRO_TCHUNK;
+  const int hgroups = (H + HPW - 1) / HPW, tchunks = (NT + p.tchunk - 1) / p.tchunk;
   const long ntasks = (long)p.B * hgroups * tchunks;
   const int KC = p.conv_k;
 
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
     const int h = HPW * hg + hq;
     if (h >= H) continue;
     const int col = h * F + 8 * sub;  // first of this lane's 8 columns inside a projection block
-    const int t0 = tc * PRO_TCHUNK, t1 = min(NT, t0 + PRO_TCHUNK);
+    const int t0 = tc * p.tchunk, t1 = min(NT, t0 + p.tchunk);
 
     // convolution taps and biases of this lane's 8 channels (loop-invariant); window slot j holds token
     // t-(PRO_MAXK-1)+j and taps are right-aligned (the last tap multiplies token t), so slots older than the kernel
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
     const int b = (int)(e / ((long)NT * H));
     float z = ld_as_float<T>(p.lr_logits, ((size_t)b * NT + t) * p.ld_lr + h);
     if (p.lr_bias != nullptr) z += ld_as_float<T>(p.lr_bias, (size_t)h);
-    st_from_float<T>(p.lr_out, (size_t)e, p.base_lr / F / (1.f + expf(-z)));
+    st_from_float<T>(p.lr_out, ((size_t)b * H + h) * p.lr_ld_out + t, p.base_lr / F / (1.f + expf(-z)));
   }
 }
 
@@ -379,12 +379,17 @@ static int sm_count() {
   return n;
 }
 
-// grid of the two prologue kernels: one warp per (batch, group of 256 / head_dim heads, token chunk), capped
-static int prologue_grid(int B, int H, int T, int head_dim) {
+// Grid of the two prologue kernels: one warp per (batch, group of 256 / head_dim heads, token chunk), capped.  The chunk
+// is halved down to one group of PRO_TG tokens while the tasks leave schedulers without a second warp: a chunk is a chain
+// of loads and stores, and a short prompt's time is that chain (1 x 1001 tokens, 12 heads: 20.4 us with chunks of 32).
+static int prologue_grid(int B, int H, int T, int head_dim, int* tchunk) {
   const int hpw = 256 / head_dim;
-  const long ntasks = (long)B * ((H + hpw - 1) / hpw) * ((T + PRO_TCHUNK - 1) / PRO_TCHUNK);
-  const long want = (ntasks + PRO_THREADS / 32 - 1) / (PRO_THREADS / 32);
   const long cap = (long)sm_count() * 8;
+  int ch = PRO_TCHUNK;
+  auto tasks = [&](int c) { return (long)B * ((H + hpw - 1) / hpw) * ((T + c - 1) / c); };
+  while (ch > PRO_TG && tasks(ch) < (long)sm_count() * 8) ch /= 2;
+  *tchunk = ch;
+  const long want = (tasks(ch) + PRO_THREADS / 32 - 1) / (PRO_THREADS / 32);
   return (int)(want < 1 ? 1 : (want > cap ? cap : want));
 }
 
@@ -396,8 +401,9 @@ static void launch_pro_t(const LayerProParams& p, int grid, cudaStream_t st) {
     ttt_layer_prologue_kernel<T, false, FD><<<grid, PRO_THREADS, 0, st>>>(p);
 }
 
-cudaError_t launch_layer_prologue(int dtype, int head_dim, const LayerProParams& p, cudaStream_t st) {
-  const int grid = prologue_grid(p.B, p.H, p.T, head_dim);
+cudaError_t launch_layer_prologue(int dtype, int head_dim, const LayerProParams& p0, cudaStream_t st) {
+  LayerProParams p = p0;
+  const int grid = prologue_grid(p.B, p.H, p.T, head_dim, &p.tchunk);
   if (head_dim == 32) {
     if (dtype == 1) launch_pro_t<__nv_bfloat16, 32>(p, grid, st);
     else launch_pro_t<float, 32>(p, grid, st);
@@ -469,7 +475,7 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
   }
   __syncthreads();
   const int hq = lane / SUBS, sub = lane % SUBS;
-  const int hgroups = (H + HPW - 1) / HPW, tchunks = (NT + PRO_TCHUNK - 1) / PRO_TCHUNK;
+  const int hgroups = (H + HPW - 1) / HPW, tchunks = (NT + p.tchunk - 1) / p.tchunk;
   const long ntasks = (long)p.B * hgroups * tchunks;
   for (long task = (long)blockIdx.x * (PRO_THREADS / 32) + warp; task < ntasks; task += (long)gridDim.x * (PRO_THREADS / 32)) {
     const int tc = (int)(task % tchunks);
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
     const int h = HPW * hg + hq;
     if (h >= H) continue;
     const int col = h * F + 8 * sub;
-    const int t0 = tc * PRO_TCHUNK, t1 = min(NT, t0 + PRO_TCHUNK);
+    const int t0 = tc * p.tchunk, t1 = min(NT, t0 + p.tchunk);
     for (int tb = t0; tb < t1; tb += PRO_TG) {
       Vec8<T> vq[PRO_TG], vk[PRO_TG], vv[PRO_TG];
 #pragma unroll
@@ -814,8 +820,9 @@ __global__ void __launch_bounds__(256) ttt_layer_epilogue_bwd_reduce_kernel(cons
   }
 }
 
-cudaError_t launch_layer_prologue_bwd(int dtype, int head_dim, const LayerProBwdParams& p, cudaStream_t st) {
-  const int grid = prologue_grid(p.B, p.H, p.T, head_dim);
+cudaError_t launch_layer_prologue_bwd(int dtype, int head_dim, const LayerProBwdParams& p0, cudaStream_t st) {
+  LayerProBwdParams p = p0;
+  const int grid = prologue_grid(p.B, p.H, p.T, head_dim, &p.tchunk);
   if (head_dim == 32) {
     if (dtype == 1) ttt_layer_prologue_bwd_kernel<__nv_bfloat16, 32><<<grid, PRO_THREADS, 0, st>>>(p);
     else ttt_layer_prologue_bwd_kernel<float, 32><<<grid, PRO_THREADS, 0, st>>>(p);

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
       tma_load_tile<T>(tq + TF::BYTES, &tm_k, r0, bar);
       tma_load_tile<T>(tq + 2 * TF::BYTES, &tm_v, r0, bar);
       bulk_load_1d(base + SM::OFF_LR + slot * 64,
-                   static_cast<const uint8_t*>(p.lr) + (size_t)(row_base + s * MB) * TF::ELT, MB * TF::ELT, bar);
+                   static_cast<const uint8_t*>(p.lr) + ((size_t)stream * p.lr_ld + s * MB) * TF::ELT, MB * TF::ELT, bar);
     } else {
       mbar_expect_tx(bar, ((GATHER ? 0 : 3 * TF::RAW_BYTES) + 2 * CS * TF::ELT) * MB / CS);
       if constexpr (!GATHER) {
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
 #pragma unroll
       for (int j = 0; j < 2; ++j)  // ttt_lr_eta is [B, H, T]: the two heads of the pair are T elements apart
         bulk_load_1d(base + SM::OFF_LR + slot * SM::LR_SLOT + j * CS * TF::ELT,
-                     static_cast<const uint8_t*>(p.lr) + ((size_t)(2 * stream + j) * p.T + s * MB) * TF::ELT,
+                     static_cast<const uint8_t*>(p.lr) + ((size_t)(2 * stream + j) * p.lr_ld + s * MB) * TF::ELT,
                      MB * TF::ELT, bar);
     }
   };

@@ -7,203 +7,278 @@
 // r = 1 (rust/layer/src/ttt.rs:253-256).  The reference's fused kernels refuse these shapes
 // (rust/fused/src/linear_fused_tile/wrapper.rs:152-172); only its unfused tensor-op path covers them.
 //
-// Work per stream is tiny (r <= 16 rows against an F x F state, F = 64 or 32), so this is a CUDA-core kernel: one
-// F-thread CTA per (batch, head) stream, thread n owns column n of W (F float registers) and column n of every 16 x F
-// tile; the stream's state is read and written exactly once (the HBM traffic that bounds a decode step).
+// Work per stream is tiny (r <= 16 rows against an F x F state, F = 64 or 32): CUDA cores, and the time is the chain of
+// dependent steps -- load the state, z = x W + b, LayerNorm statistics, gradient, second LayerNorm, update.  So:
+//   * one 4-warp CTA per stream; warp w holds rows [w F/4, (w + 1) F/4) of W (lane: F/32 adjacent columns, coalesced 64- or
+//     128-byte rows), so z is a partial sum per warp, met in shared memory: one barrier;
+//   * from there on a row belongs to one warp (row i to warp i % 4): every row sum is a warp shuffle, no barrier; the
+//     gradients of all rows meet in shared memory once more for the output and the update.
+// The state is read and written exactly once, three barriers in all.  (One thread per column with the row sums crossing
+// warps ten times: 22 us for 9 rows of 12 streams, 4.1 us for one row of 96.)
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
 
 namespace ttt {
 
-template <int FD>
+constexpr int PT_WARPS = 4;
+
+// N adjacent columns; VEC: as one access (the pointers are aligned to it), else element by element
+template <typename T, bool VEC, int N>
+__device__ __forceinline__ void ld_cols(const void* base, size_t idx, float (&v)[N]) {
+  if constexpr (N == 1 || !VEC) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = ld_as_float<T>(base, idx + i);
+  } else if constexpr (sizeof(T) == 2) {
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(static_cast<const T*>(base) + idx);
+    v[0] = bf16_lo(u);
+    v[1] = bf16_hi(u);
+  } else {
+    const float2 u = *reinterpret_cast<const float2*>(static_cast<const T*>(base) + idx);
+    v[0] = u.x;
+    v[1] = u.y;
+  }
+}
+template <typename T, bool VEC, int N>
+__device__ __forceinline__ void st_cols(void* base, size_t idx, const float (&v)[N]) {
+  if constexpr (N == 1 || !VEC) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) st_from_float<T>(base, idx + i, v[i]);
+  } else if constexpr (sizeof(T) == 2) *reinterpret_cast<uint32_t*>(static_cast<T*>(base) + idx) = pack_bf16(v[0], v[1]);
+  else *reinterpret_cast<float2*>(static_cast<T*>(base) + idx) = make_float2(v[0], v[1]);
+}
+// sums of N values over the warp, all of them in every lane
+template <int N>
+__device__ __forceinline__ void warp_sums(float (&v)[N]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+}
+
+template <int RM, int FD>
 struct PartialSmem {
-  float q[CS][FD], k[CS][FD], v[CS][FD];
-  float attn[CS][CS];
-  float lr[CS], te[CS];
-  float red[2][CS][2];  // cross-warp partial sums
+  float q[RM][FD], k[RM][FD], g[RM][FD];  // g: the rows' gradients
+  float z[PT_WARPS][2][RM][FD];           // the warps' partial K W and Q W
+  float attn[RM][RM];
+  float lr[RM], te[RM];
 };
 
-// Sums over the F columns (threads) of two values per row, for rows < r.  Every thread gets the totals.
-template <int RM, int FD>
-__device__ __forceinline__ void row_sums(PartialSmem<FD>& sm, int r, int tid, float (&a)[RM], float (&b)[RM]) {
-  const int warp = tid >> 5, lane = tid & 31;
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    if (i < r) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
-        b[i] += __shfl_xor_sync(0xffffffffu, b[i], o);
-      }
-      if (lane == 0) {
-        sm.red[warp][i][0] = a[i];
-        sm.red[warp][i][1] = b[i];
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    if (i < r) {
-      a[i] = (FD == 64) ? sm.red[0][i][0] + sm.red[1][i][0] : sm.red[0][i][0];
-      b[i] = (FD == 64) ? sm.red[0][i][1] + sm.red[1][i][1] : sm.red[0][i][1];
-    }
-  }
-  __syncthreads();  // red may be reused
-}
-
-// RM: compile-time bound on the number of rows (1 for the decode step, 4, or 16), so that short mini-batches do not
-// pay for sixteen rows of predicated-off arithmetic.
-template <typename T, int RM, int FD>
-__global__ void __launch_bounds__(FD) ttt_linear_partial_kernel(const LinPartialParams p) {
-  constexpr int HD = FD;  // features per head in this instantiation (shadows the 64 of the tiled kernels)
-  constexpr int PT_THREADS = FD;
-  __shared__ PartialSmem<FD> sm;
-  const int n = threadIdx.x;
+// RM: compile-time bound on the number of rows (1 for the decode step, 4, or 16).
+template <typename T, int RM, int FD, bool VEC>
+__global__ void __launch_bounds__(32 * PT_WARPS) ttt_linear_partial_kernel(const LinPartialParams p) {
+  constexpr int NC = FD / 32, KR = FD / PT_WARPS;            // columns per lane, rows of W per warp
+  constexpr int RW = (RM + PT_WARPS - 1) / PT_WARPS;         // rows of the mini-batch per warp
+  constexpr int NT = 32 * PT_WARPS;
+  constexpr float INV_F = 1.f / FD;
+  __shared__ __align__(16) PartialSmem<RM, FD> sm;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int stream = blockIdx.x, head = stream % p.H, r = p.R;
-  const size_t row0 = (size_t)stream * r;
+  const size_t row0 = (size_t)stream * p.row_ld + p.row_off;
+  const int c0 = NC * lane, k0 = KR * warp;
 
-  // tiles (converted to float), learning rates, token coefficients
-  for (int e = n; e < r * HD; e += PT_THREADS) {
-    const int i = e / HD, c = e % HD;
-    sm.q[i][c] = ld_as_float<T>(p.xq, (row0 + i) * HD + c);
-    sm.k[i][c] = ld_as_float<T>(p.xk, (row0 + i) * HD + c);
-    sm.v[i][c] = ld_as_float<T>(p.xv, (row0 + i) * HD + c);
-  }
-  if (n < r) {
-    sm.lr[n] = ld_as_float<T>(p.lr, row0 + n);
-    sm.te[n] = ld_as_float<T>(p.token_eta, (size_t)n);
-  }
-  float w[HD];
+  float w[KR][NC];
+  if (!p.state_settled) pdl_wait();
 #pragma unroll
-  for (int k = 0; k < HD; ++k) w[k] = ld_as_float<T>(p.w0, (size_t)stream * HD * HD + (size_t)k * HD + n);
-  float bias = ld_as_float<T>(p.b0, (size_t)stream * HD + n);
-  const float gam = ld_as_float<T>(p.ln_g, (size_t)head * HD + n), bet = ld_as_float<T>(p.ln_b, (size_t)head * HD + n);
+  for (int k = 0; k < KR; ++k) ld_cols<T, VEC>(p.w0, (size_t)stream * FD * FD + (size_t)(k0 + k) * FD + c0, w[k]);
+  if (p.state_settled) pdl_wait();
+  pdl_go();
+  for (int e = tid; e < r * FD; e += NT) {
+    sm.q[0][e] = ld_as_float<T>(p.xq, row0 * FD + e);
+    sm.k[0][e] = ld_as_float<T>(p.xk, row0 * FD + e);
+  }
+  if (tid < r) {
+    sm.lr[tid] = ld_as_float<T>(p.lr, (size_t)stream * p.lr_ld + p.row_off + tid);
+    sm.te[tid] = ld_as_float<T>(p.token_eta, (size_t)tid);
+  }
+  float bias[NC], gam[NC], bet[NC], v[RW][NC];
+  ld_cols<T, VEC>(p.b0, (size_t)stream * FD + c0, bias);
+  ld_cols<T, VEC>(p.ln_g, (size_t)head * FD + c0, gam);
+  ld_cols<T, VEC>(p.ln_b, (size_t)head * FD + c0, bet);
+#pragma unroll
+  for (int j = 0; j < RW; ++j)
+    if (warp + PT_WARPS * j < r) ld_cols<T, VEC>(p.xv, (row0 + warp + PT_WARPS * j) * FD + c0, v[j]);
   __syncthreads();
 
-  // Attn[i][j] = Q[i] . K[j] for j <= i
-  for (int e = n; e < r * r; e += PT_THREADS) {
-    const int i = e / r, j = e % r;
-    float s = 0.f;
-    if (j <= i) {
-#pragma unroll
-      for (int k = 0; k < HD; ++k) s = fmaf(sm.q[i][k], sm.k[j][k], s);
-    }
-    sm.attn[i][j] = s;
-  }
-
-  // Z1 = K W + b and Zq = Q W + b, column n
-  float z1[RM], zq[RM];
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    z1[i] = zq[i] = bias;
-    if (i < r) {
-#pragma unroll
-      for (int k = 0; k < HD; ++k) {
-        z1[i] = fmaf(sm.k[i][k], w[k], z1[i]);
-        zq[i] = fmaf(sm.q[i][k], w[k], zq[i]);
-      }
-    }
-  }
-
-  // LayerNorm statistics of Z1 (two-pass variance), then G = dL/dZ1
-  float a[RM], b2[RM], mean[RM], rstd[RM];
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    a[i] = z1[i];
-    b2[i] = 0.f;
-  }
-  row_sums<RM, FD>(sm, r, n, a, b2);
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    mean[i] = a[i] * (1.f / HD);
-    const float d = z1[i] - mean[i];
-    a[i] = d * d;
-    b2[i] = 0.f;
-  }
-  row_sums<RM, FD>(sm, r, n, a, b2);
-  float xh[RM], gx[RM], g[RM];
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    rstd[i] = 1.f / sqrtf(a[i] * (1.f / HD) + p.eps);
-    xh[i] = (z1[i] - mean[i]) * rstd[i];
-    const float tgt = (i < r) ? sm.v[i][n] - sm.k[i][n] : 0.f;
-    gx[i] = (gam * xh[i] + bet - tgt) * gam;
-    a[i] = gx[i];
-    b2[i] = gx[i] * xh[i];
-  }
-  row_sums<RM, FD>(sm, r, n, a, b2);
+  // ---- this warp's share of Z1 = K W and Zq = Q W; Attn[i][j] = Q[i] . K[j] for j <= i
 #pragma unroll
   for (int i = 0; i < RM; ++i)
-    g[i] = (i < r) ? (gx[i] - a[i] * (1.f / HD) - xh[i] * b2[i] * (1.f / HD)) * rstd[i] : 0.f;
-
-  // Zbar = Zq - sum_{j<=i} te[i] lr[j] (1 + Attn[i][j]) G[j];  out = Q + LN(Zbar)
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
     if (i < r) {
-      float s = 0.f;
+      float a[NC] = {}, b[NC] = {};
 #pragma unroll
-      for (int j = 0; j < RM; ++j)
-        if (j <= i && j < r) s = fmaf(sm.lr[j] * (1.f + sm.attn[i][j]), g[j], s);
-      zq[i] -= sm.te[i] * s;
+      for (int k = 0; k < KR; k += 4) {
+        const float4 kk = *reinterpret_cast<const float4*>(&sm.k[i][k0 + k]), qq = *reinterpret_cast<const float4*>(&sm.q[i][k0 + k]);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          a[c] = fmaf(kk.w, w[k + 3][c], fmaf(kk.z, w[k + 2][c], fmaf(kk.y, w[k + 1][c], fmaf(kk.x, w[k][c], a[c]))));
+          b[c] = fmaf(qq.w, w[k + 3][c], fmaf(qq.z, w[k + 2][c], fmaf(qq.y, w[k + 1][c], fmaf(qq.x, w[k][c], b[c]))));
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        sm.z[warp][0][i][c0 + c] = a[c];
+        sm.z[warp][1][i][c0 + c] = b[c];
+      }
     }
-    a[i] = zq[i];
-    b2[i] = 0.f;
-  }
-  row_sums<RM, FD>(sm, r, n, a, b2);
+  for (int e = tid; e < r * r; e += NT) {
+    const int i = e / r, j = e - i * r;
+    if (j > i) continue;
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    mean[i] = a[i] * (1.f / HD);
-    const float d = zq[i] - mean[i];
-    a[i] = d * d;
-    b2[i] = 0.f;
-  }
-  row_sums<RM, FD>(sm, r, n, a, b2);
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    if (i < r) {
-      const float rs = 1.f / sqrtf(a[i] * (1.f / HD) + p.eps);
-      st_from_float<T>(p.out, (row0 + i) * HD + n, sm.q[i][n] + gam * (zq[i] - mean[i]) * rs + bet);
+    for (int k = 0; k < FD; k += 8) {
+      const float4 qa = *reinterpret_cast<const float4*>(&sm.q[i][k]), ka = *reinterpret_cast<const float4*>(&sm.k[j][k]);
+      const float4 qb = *reinterpret_cast<const float4*>(&sm.q[i][k + 4]), kb = *reinterpret_cast<const float4*>(&sm.k[j][k + 4]);
+      s0 = fmaf(qa.w, ka.w, fmaf(qa.z, ka.z, fmaf(qa.y, ka.y, fmaf(qa.x, ka.x, s0))));
+      s1 = fmaf(qb.w, kb.w, fmaf(qb.z, kb.z, fmaf(qb.y, kb.y, fmaf(qb.x, kb.x, s1))));
     }
+    sm.attn[i][j] = s0 + s1;
   }
+  __syncthreads();
 
-  // state update with the last row of eta: W -= (te[r-1] lr o K)^T G,  b -= sum_j te[r-1] lr[j] G[j]
+  // ---- per row (i = warp + 4 j): LayerNorm statistics of Z1 (two-pass variance), G = dL/dZ1
+  float z[RW][NC], st[RW], mean[RW];
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    const int i = min(warp + PT_WARPS * j, r - 1);  // (rows beyond the last: computed on the last one's values, not kept)
+    st[j] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      z[j][c] = bias[c] + ((sm.z[0][0][i][c0 + c] + sm.z[1][0][i][c0 + c]) + (sm.z[2][0][i][c0 + c] + sm.z[3][0][i][c0 + c]));
+      st[j] += z[j][c];
+    }
+  }
+  warp_sums(st);
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    mean[j] = st[j] * INV_F;
+    st[j] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      z[j][c] -= mean[j];
+      st[j] = fmaf(z[j][c], z[j][c], st[j]);
+    }
+  }
+  warp_sums(st);
+  float gx[RW][NC], sums[2 * RW], rstd[RW];
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    rstd[j] = 1.f / sqrtf(st[j] * INV_F + p.eps);
+    sums[2 * j] = sums[2 * j + 1] = 0.f;
+    const int i = min(warp + PT_WARPS * j, r - 1);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      z[j][c] *= rstd[j];  // x_hat
+      const float tgt = (warp + PT_WARPS * j < r) ? v[j][c] - sm.k[i][c0 + c] : 0.f;
+      gx[j][c] = (gam[c] * z[j][c] + bet[c] - tgt) * gam[c];
+      sums[2 * j] += gx[j][c];
+      sums[2 * j + 1] = fmaf(gx[j][c], z[j][c], sums[2 * j + 1]);
+    }
+  }
+  warp_sums(sums);
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    const int i = warp + PT_WARPS * j;
+    if (i < r) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        sm.g[i][c0 + c] = (gx[j][c] - sums[2 * j] * INV_F - z[j][c] * sums[2 * j + 1] * INV_F) * rstd[j];
+    }
+  }
+  __syncthreads();
+
+  // ---- state update with the last row of eta: W -= (te[r-1] lr o K)^T G, b -= sum_j te[r-1] lr[j] G[j]
   const float te_last = sm.te[r - 1];
-  float gl[RM];
+  float b_in[NC];
 #pragma unroll
-  for (int j = 0; j < RM; ++j) gl[j] = (j < r) ? te_last * sm.lr[j] * g[j] : 0.f;
+  for (int c = 0; c < NC; ++c) b_in[c] = bias[c];
+  for (int j = 0; j < r; ++j) {
+    const float e = te_last * sm.lr[j];
+    float gl[NC];
 #pragma unroll
-  for (int j = 0; j < RM; ++j) {
-    if (j < r) {
-      bias -= gl[j];
+    for (int c = 0; c < NC; ++c) {
+      gl[c] = e * sm.g[j][c0 + c];
+      bias[c] -= gl[c];
+    }
 #pragma unroll
-      for (int k = 0; k < HD; ++k) w[k] = fmaf(-sm.k[j][k], gl[j], w[k]);
+    for (int k = 0; k < KR; k += 4) {
+      const float4 kk = *reinterpret_cast<const float4*>(&sm.k[j][k0 + k]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        w[k][c] = fmaf(-kk.x, gl[c], w[k][c]);
+        w[k + 1][c] = fmaf(-kk.y, gl[c], w[k + 1][c]);
+        w[k + 2][c] = fmaf(-kk.z, gl[c], w[k + 2][c]);
+        w[k + 3][c] = fmaf(-kk.w, gl[c], w[k + 3][c]);
+      }
     }
   }
 #pragma unroll
-  for (int k = 0; k < HD; ++k) st_from_float<T>(p.w_out, (size_t)stream * HD * HD + (size_t)k * HD + n, w[k]);
-  st_from_float<T>(p.b_out, (size_t)stream * HD + n, bias);
+  for (int k = 0; k < KR; ++k) st_cols<T, VEC>(p.w_out, (size_t)stream * FD * FD + (size_t)(k0 + k) * FD + c0, w[k]);
+
+  // ---- Zbar = Zq - sum_{j<=i} te[i] lr[j] (1 + Attn[i][j]) G[j];  out = Q + LN(Zbar)
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    const int i = min(warp + PT_WARPS * j, r - 1);
+    float s[NC] = {};
+    for (int l = 0; l <= i; ++l) {
+      const float m = sm.lr[l] * (1.f + sm.attn[i][l]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) s[c] = fmaf(m, sm.g[l][c0 + c], s[c]);
+    }
+    st[j] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const float zq = b_in[c] + ((sm.z[0][1][i][c0 + c] + sm.z[1][1][i][c0 + c]) + (sm.z[2][1][i][c0 + c] + sm.z[3][1][i][c0 + c]));
+      z[j][c] = zq - sm.te[i] * s[c];
+      st[j] += z[j][c];
+    }
+  }
+  warp_sums(st);
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    mean[j] = st[j] * INV_F;
+    st[j] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      z[j][c] -= mean[j];
+      st[j] = fmaf(z[j][c], z[j][c], st[j]);
+    }
+  }
+  warp_sums(st);
+#pragma unroll
+  for (int j = 0; j < RW; ++j) {
+    const int i = warp + PT_WARPS * j;
+    if (i < r) {
+      const float rs = 1.f / sqrtf(st[j] * INV_F + p.eps);
+      float o[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) o[c] = sm.q[i][c0 + c] + gam[c] * z[j][c] * rs + bet[c];
+      st_cols<T, VEC>(p.out, (row0 + i) * FD + c0, o);
+    }
+  }
+  // (in place or not: every warp read the old state before the first barrier)
+  if (warp == 0) st_cols<T, VEC>(p.b_out, (size_t)stream * FD + c0, bias);
 }
 
-template <typename T, int FD>
-static void launch_partial_t(const LinPartialParams& p, int nstreams, cudaStream_t st) {
-  if (p.R == 1)
-    ttt_linear_partial_kernel<T, 1, FD><<<nstreams, FD, 0, st>>>(p);
-  else if (p.R <= 4)
-    ttt_linear_partial_kernel<T, 4, FD><<<nstreams, FD, 0, st>>>(p);
-  else
-    ttt_linear_partial_kernel<T, 16, FD><<<nstreams, FD, 0, st>>>(p);
+template <typename T, int FD, bool VEC>
+static cudaError_t launch_partial_t(const LinPartialParams& p, int nstreams, cudaStream_t st) {
+  auto kfn = p.R == 1   ? ttt_linear_partial_kernel<T, 1, FD, VEC>
+             : p.R <= 4 ? ttt_linear_partial_kernel<T, 4, FD, VEC>
+                        : ttt_linear_partial_kernel<T, 16, FD, VEC>;
+  return launch_dependent(kfn, nstreams, 32 * PT_WARPS, 0, st, p);
+}
+template <typename T>
+static cudaError_t launch_partial_d(int head_dim, const LinPartialParams& p, int nstreams, cudaStream_t st) {
+  if (head_dim == 32) return launch_partial_t<T, 32, false>(p, nstreams, st);
+  // column pairs as one access where every tensor starts on one (any tensor of its own does; a view may not)
+  uintptr_t all = 0;
+  for (const void* q : {p.w0, p.b0, p.ln_g, p.ln_b, p.xv, (const void*)p.out, (const void*)p.w_out, (const void*)p.b_out})
+    all |= reinterpret_cast<uintptr_t>(q);
+  return all % (2 * sizeof(T)) == 0 ? launch_partial_t<T, 64, true>(p, nstreams, st)
+                                    : launch_partial_t<T, 64, false>(p, nstreams, st);
 }
 
 cudaError_t launch_linear_partial(int dtype, int head_dim, const LinPartialParams& p, int nstreams, cudaStream_t st) {
-  if (head_dim == 32) {
-    if (dtype == 1) launch_partial_t<__nv_bfloat16, 32>(p, nstreams, st);
-    else launch_partial_t<float, 32>(p, nstreams, st);
-  } else {
-    if (dtype == 1) launch_partial_t<__nv_bfloat16, 64>(p, nstreams, st);
-    else launch_partial_t<float, 64>(p, nstreams, st);
-  }
-  return cudaGetLastError();
+  return dtype == 1 ? launch_partial_d<__nv_bfloat16>(head_dim, p, nstreams, st)
+                    : launch_partial_d<float>(head_dim, p, nstreams, st);
 }
 
 }  // namespace ttt

@@ -20,6 +20,7 @@ There is no PyTorch fallback for the layer kernels: without the CUDA library the
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from dataclasses import dataclass
 from typing import Optional
 
@@ -27,9 +28,10 @@ import torch
 
 from . import _lib
 from ._lib import TttDims
-from .fused import FusedTileMultiTTTLinear, Qkv, TTTInputsInner, TTTLinear, TTTLinearState
+from .fused import FusedTileMultiTTTLinear, FusedTttConfig, Qkv, TTTInputsInner, TTTLinear, TTTLinearState
 
 ROPE_NONE, ROPE_WRAPPED, ROPE_GLOBAL = 0, 1, 2
+_NO_CONV = (None, None, None, None)
 _POS = {"none": ROPE_NONE, "rope": ROPE_WRAPPED, "rope_global": ROPE_GLOBAL}
 
 
@@ -50,6 +52,11 @@ class TTTLayerConfig:
     @property
     def head_dim(self) -> int:
         return self.hidden_size // self.num_heads
+
+
+@functools.lru_cache(maxsize=64)
+def _eps_scaled(eps: float) -> int:
+    return FusedTttConfig.new(1, 1, eps).epsilon_scaled
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -341,6 +348,7 @@ class TTT(torch.nn.Module):
         self.post_norm_weight = torch.nn.Parameter(torch.ones(hs, **kw))
         self.post_norm_bias = torch.nn.Parameter(torch.zeros(hs, **kw))
         self._wcat, self._wcat_key = None, None
+        self._te, self._te_key = None, None
 
     # ---- one GEMM for every projection of x ----------------------------------------------------------------
     def _fused_weight(self):
@@ -350,7 +358,7 @@ class TTT(torch.nn.Module):
         dtype cast all invalidate it."""
         srcs = [w for w in (self.q_proj, self.k_proj, self.v_proj, self.g_proj) if w is not None]
         srcs.append(self.learnable_ttt_lr_weight)
-        key = tuple((w.data_ptr(), w._version, w.dtype, w.device) for w in srcs)
+        key = _lib.host().param_key(*srcs)
         if self._wcat is None or self._wcat_key != key:
             self._wcat_key = key
             c = self.config
@@ -372,7 +380,15 @@ class TTT(torch.nn.Module):
         return self._wcat
 
     def invalidate_fused_weight(self):
-        self._wcat = None
+        self._wcat = self._te = None
+
+    def _token_eta(self, dtype):
+        """token_eta of one mini-batch (the kernels read no further), in `dtype`; kept like the stacked weights."""
+        key = _lib.host().param_key(self.token_idx, self.learnable_token_idx), dtype
+        if self._te is None or self._te_key != key:
+            self._te_key = key
+            self._te = torch.clamp_min(self.token_idx + self.learnable_token_idx.detach(), 0.0).to(dtype)
+        return self._te
 
     @staticmethod
     def _project(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -412,11 +428,34 @@ class TTT(torch.nn.Module):
         gate = proj.reshape(B * T, -1)[:, cols["g"]:] if c.use_gate else None
         return TTTInputsInner(Qkv(xq, xk, xv), token_eta, lr, start_idx), gate, proj.shape[-1]
 
+    def _infer_native(self, x: torch.Tensor, inner, state, start_idx: int) -> Optional[torch.Tensor]:
+        """The whole inference forward as one native call (bf16; None: not a case it takes, nothing was done)."""
+        c = self.config
+        if type(inner) is not FusedTileMultiTTTLinear or not x.is_cuda:
+            return None
+        i = inner.inner
+        if i.mini_batch_size != c.mini_batch_size:
+            return None
+        wcat, cols = self._fused_weight()
+        conv = (self.q_conv_weight, self.q_conv_bias, self.k_conv_weight, self.k_conv_bias) if c.share_qk else _NO_CONV
+        r = _lib.host().layer_infer(
+            x, wcat, self._token_eta(x.dtype), self.learnable_ttt_lr_bias, *conv, state.weight, state.bias, i.ln_weight,
+            i.ln_bias, self.post_norm_weight, self.post_norm_bias, self.o_proj, c.use_gate, c.num_heads,
+            c.mini_batch_size, _POS[c.pos_encoding], c.rope_theta, c.base_lr, cols["lr"], _eps_scaled(i.epsilon),
+            inner.allow_partial, inner.partial_in_place, start_idx)
+        if r is None:
+            return None
+        y, state.weight, state.bias = r
+        return y
+
     def forward(self, x: torch.Tensor, inner: FusedTileMultiTTTLinear, state: TTTLinearState,
                 start_idx: int = 0) -> torch.Tensor:
         """x [B, T, hidden] -> [B, T, hidden]; `state` is advanced in place (rust/layer/src/ttt.rs:269-299)."""
         if torch.is_grad_enabled():
             return self._forward_train(x, inner, state, start_idx)
+        y = self._infer_native(x, inner, state, start_idx)
+        if y is not None:
+            return y
         inputs, gate, gate_ld = self.get_inner_loop_inputs(x, start_idx)
         out = inner.forward(state, inputs)  # [B, H, T, F]
         y = layer_epilogue(out.contiguous(), self.post_norm_weight, self.post_norm_bias, 1e-6, gate,
@@ -476,13 +515,15 @@ def new_inner(config: TTTLayerConfig, checkpoint_interval: int = 1, device=None,
 
 
 class DecodeGraphs:
-    """Token-by-token generation through one layer with the whole step (projection GEMM, prologue, decode kernel,
-    epilogue, output GEMM: five launches, launch-bound at small batch) captured once per rotary phase as a CUDA graph.
+    """Token-by-token generation through one layer, the state advanced in place.
 
-    The rotary position enters the prologue as a scalar argument, so with positions wrapped at the mini-batch there
-    are `mini_batch_size` distinct steps; each is captured on first use.  The state is advanced in place, the input
-    is read from `self.x` [B, 1, hidden] and the result lands in the tensor `step` returns (overwritten by the next
-    step of the same phase)."""
+    Where the native path covers the layer (bf16, see `TTT.forward`), a step is its launches issued directly: three for
+    few sequences, overlapped through programmatic dependent launch, which leaves nothing for a graph to save and
+    spares the copy of the input into a captured buffer.  Otherwise the step (projection GEMM, prologue, decode kernel,
+    epilogue, output GEMM) is captured once per rotary phase as a CUDA graph: the rotary position enters the prologue
+    as a scalar argument, so with positions wrapped at the mini-batch there are `mini_batch_size` distinct steps, each
+    captured on first use; the input is copied to `self.x` [B, 1, hidden] and the result lands in the tensor `step`
+    returns (overwritten by the next step of the same phase)."""
 
     def __init__(self, layer: "TTT", inner: FusedTileMultiTTTLinear, state: TTTLinearState, batch: int):
         c = layer.config
@@ -498,8 +539,12 @@ class DecodeGraphs:
 
     def step(self, x: torch.Tensor, start_idx: int) -> torch.Tensor:
         """One token per sequence: x [B, 1, hidden] at position `start_idx`."""
-        self.x.copy_(x)
         ph = start_idx % self.period
+        if not self._graphs and x.shape == self.x.shape and x.dtype == self.x.dtype:
+            y = self.layer._infer_native(x, self.inner, self.state, ph)
+            if y is not None:
+                return y
+        self.x.copy_(x)
         g = self._graphs.get(ph)
         if g is None:
             # warm-up run on a side stream (lazy initialisation of the libraries must happen outside the capture);
