@@ -535,11 +535,13 @@ template <bool FUSED>
 static cudaError_t launch_gemm_t(const CUtensorMap* m, const GemmParams& p, cudaStream_t st) {
   using SM = GemmSmem<FUSED, false>;
   auto kfn = ttt_gemm_bf16_tn_kernel<FUSED, false>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
+  static DeviceValue ready;
+  int sms = 0;
+  const cudaError_t e = ready.get(0, &sms, [&](int* n) {
+    const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
+    return a != cudaSuccess ? a : device_sms(n);
+  });
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   const long ntiles = (long)((p.N + GEMM_BN - 1) / GEMM_BN) * ((p.M + GEMM_BM - 1) / GEMM_BM);
   const int grid = (int)(ntiles < sms ? ntiles : sms);  // persistent: one CTA per SM walks the tiles
   kfn<<<grid, GEMM_THREADS, SM::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
@@ -551,11 +553,6 @@ template <bool FUSED>
 static cudaError_t launch_gemm_pair_t(const CUtensorMap* m, const GemmParams& p, cudaStream_t st) {
   using SM = GemmSmem<FUSED, true>;
   auto kfn = ttt_gemm_bf16_tn_kernel<FUSED, true>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
-  if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -567,12 +564,20 @@ static cudaError_t launch_gemm_pair_t(const CUtensorMap* m, const GemmParams& p,
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cfg.gridDim = dim3(2 * (sms / 2));
+  static DeviceValue resident;
   int nclusters = 0;
-  if ((e = cudaOccupancyMaxActiveClusters(&nclusters, kfn, &cfg)) != cudaSuccess) return e;
+  const cudaError_t e = resident.get(0, &nclusters, [&](int* n) {
+    int sms = 0;
+    cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
+    if (a != cudaSuccess || (a = device_sms(&sms)) != cudaSuccess) return a;
+    cfg.gridDim = dim3(2 * (sms / 2));
+    if ((a = cudaOccupancyMaxActiveClusters(n, kfn, &cfg)) != cudaSuccess) return a;
+    if (*n > sms / 2) *n = sms / 2;
+    return cudaSuccess;
+  });
+  if (e != cudaSuccess) return e;
   if (nclusters < 1) return cudaErrorLaunchOutOfResources;
   const long ntiles = (long)((p.N + GEMM_BN - 1) / GEMM_BN) * ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM));
-  if (nclusters > sms / 2) nclusters = sms / 2;
   if (nclusters > ntiles) nclusters = (int)ntiles;
   cfg.gridDim = dim3(2 * nclusters);
   return cudaLaunchKernelEx(&cfg, kfn, m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);

@@ -5,7 +5,39 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace ttt {
+
+// A launch parameter that depends on the device (and at most on `key`), computed on first use: the queries behind it
+// (function attributes, occupancy) cost a microsecond or more each, and a launch makes several.  `fn(int* value)` is
+// idempotent.
+struct DeviceValue {
+  static constexpr int N = 64;
+  std::atomic<uint64_t> slot[N] = {};
+  template <class Fn>
+  cudaError_t get(uint32_t key, int* value, Fn fn) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t have = dev < N ? slot[dev].load(std::memory_order_acquire) : 0;
+    if (have != 0 && (uint32_t)(have >> 32) == key + 1) {
+      *value = (int)(uint32_t)have;
+      return cudaSuccess;
+    }
+    if ((e = fn(value)) != cudaSuccess) return e;
+    if (dev < N) slot[dev].store(((uint64_t)(key + 1) << 32) | (uint32_t)*value, std::memory_order_release);
+    return cudaSuccess;
+  }
+};
+inline cudaError_t device_sms(int* sms) {
+  static DeviceValue v;
+  return v.get(0, sms, [](int* n) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e != cudaSuccess ? e : cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev);
+  });
+}
 
 struct LinFwdParams {
   const void* w0;         // [B,H,F,F] element type T

@@ -374,9 +374,8 @@ __global__ void __launch_bounds__(EPI_THREADS, (MAXCH <= 4 ? 4 : 2)) ttt_layer_e
 }
 
 static int sm_count() {
-  int dev = 0, n = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n;
+  int n = 148;
+  return device_sms(&n) == cudaSuccess ? n : 148;
 }
 
 // Grid of the two prologue kernels: one warp per (batch, group of 256 / head_dim heads, token chunk), capped.  The chunk
@@ -420,12 +419,16 @@ static cudaError_t launch_epi_t(const LayerEpiParams& p, cudaStream_t st) {
   constexpr int TT = 64 / MAXCH;
   const size_t smem = 2 * (size_t)TT * C * sizeof(T) + 2 * (size_t)C * sizeof(float);
   auto kfn = ttt_layer_epilogue_kernel<T, MAXCH, FD>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static DeviceValue resident;
+  int per_sm = 1;
+  cudaError_t e = resident.get((uint32_t)C, &per_sm, [&](int* n) {
+    constexpr int CMAX = 512 * MAXCH / (int)sizeof(T);  // the widest row of this instantiation
+    const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               2 * TT * CMAX * (int)sizeof(T) + 2 * CMAX * (int)sizeof(float));
+    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, EPI_THREADS, smem);
+  });
   if (e != cudaSuccess) return e;
   const long ntiles = (long)p.B * ((p.T + TT - 1) / TT);
-  int per_sm = 1;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, EPI_THREADS, smem);
-  if (e != cudaSuccess) return e;
   const long cap = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
   const int grid = (int)(ntiles < cap ? ntiles : cap);
   kfn<<<grid < 1 ? 1 : grid, EPI_THREADS, smem, st>>>(p);
@@ -844,12 +847,16 @@ static cudaError_t launch_epi_bwd_t(LayerEpiBwdParams p, cudaStream_t st) {
   constexpr int TT = 64 / MAXCH;
   const size_t smem = 2 * (size_t)TT * C * sizeof(T) + 2 * (size_t)C * sizeof(float);
   auto kfn = ttt_layer_epilogue_bwd_kernel<T, MAXCH, FD>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static DeviceValue resident;
+  int per_sm = 1;
+  cudaError_t e = resident.get((uint32_t)C, &per_sm, [&](int* n) {
+    constexpr int CMAX = 512 * MAXCH / (int)sizeof(T);  // the widest row of this instantiation
+    const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               2 * TT * CMAX * (int)sizeof(T) + 2 * CMAX * (int)sizeof(float));
+    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, EPI_THREADS, smem);
+  });
   if (e != cudaSuccess) return e;
   const long ntiles = (long)p.B * ((p.T + TT - 1) / TT);
-  int per_sm = 1;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, EPI_THREADS, smem);
-  if (e != cudaSuccess) return e;
   if (per_sm > 2) per_sm = 2;
   const long cap = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
   const int grid = (int)(ntiles < cap ? ntiles : cap);

@@ -239,7 +239,12 @@ cudaError_t launch_layer_small_proj(const SmallProjParams& p, cudaStream_t st) {
 template <int MT>
 static cudaError_t launch_out_t(const SmallOutParams& p, cudaStream_t st) {
   const int C = p.H * p.F, smem = 16 * MT * (C + 32) * 2;
-  cudaError_t e = cudaFuncSetAttribute(ttt_layer_small_out_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static DeviceValue ready;
+  int most = 0;
+  const cudaError_t e = ready.get(0, &most, [](int* n) {
+    *n = 16 * MT * (2048 + 32) * 2;
+    return cudaFuncSetAttribute(ttt_layer_small_out_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, *n);
+  });
   if (e != cudaSuccess) return e;
   return launch_dependent(ttt_layer_small_out_kernel<MT>, C / 8, SM_THREADS, smem, st, p);
 }

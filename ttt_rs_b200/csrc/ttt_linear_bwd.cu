@@ -919,27 +919,31 @@ static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, Lin
                                 cudaStream_t st) {
   using SM = BwdSmem<T, SEG>;
   auto kfn = ttt_linear_bwd_kernel<T, SEG, MB>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
-  if (e != cudaSuccess) return e;
   // Persistent grid: as many blocks as fit on the device at once, never more than there are work items.  The count
   // comes from the kernel's registers and shared memory: the occupancy calculator answers one block per SM for any
   // kernel that allocates tensor memory, whatever it allocates (which also rules out a cooperative launch of more).
   // Co-residency is not needed for progress: a block takes an item only once it runs, and the item it may wait for
   // has a smaller index, so it was taken by a block that runs or has finished; a block that is not resident yet holds
   // nothing anybody waits for.
-  int dev = 0, sms = 0, regs_sm = 0, smem_sm = 0, smem_rsv = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess) return e;
-  cudaFuncAttributes fa;
-  if ((e = cudaFuncGetAttributes(&fa, kfn)) != cudaSuccess) return e;
-  const int regs_block = ((fa.numRegs + 7) & ~7) * NTHREADS;  // registers are allocated in units of 8 per thread
-  const int smem_block = (int)SM::DYN_BYTES + (int)fa.sharedSizeBytes + smem_rsv;
-  int per_sm = regs_sm / regs_block;
-  if (smem_sm / smem_block < per_sm) per_sm = smem_sm / smem_block;
-  if (per_sm > 512 / 64) per_sm = 512 / 64;  // tensor-memory columns
+  static DeviceValue resident;
+  int sms = 0, per_sm = 0;
+  cudaError_t e = resident.get(0, &per_sm, [&](int* n) {
+    int dev = 0, regs_sm = 0, smem_sm = 0, smem_rsv = 0;
+    cudaFuncAttributes fa;
+    cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
+    if (a != cudaSuccess || (a = cudaGetDevice(&dev)) != cudaSuccess) return a;
+    if ((a = cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev)) != cudaSuccess) return a;
+    if ((a = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return a;
+    if ((a = cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess) return a;
+    if ((a = cudaFuncGetAttributes(&fa, kfn)) != cudaSuccess) return a;
+    const int regs_block = ((fa.numRegs + 7) & ~7) * NTHREADS;  // registers are allocated in units of 8 per thread
+    const int smem_block = (int)SM::DYN_BYTES + (int)fa.sharedSizeBytes + smem_rsv;
+    *n = regs_sm / regs_block;
+    if (smem_sm / smem_block < *n) *n = smem_sm / smem_block;
+    if (*n > 512 / 64) *n = 512 / 64;  // tensor-memory columns
+    return cudaSuccess;
+  });
+  if (e != cudaSuccess || (e = device_sms(&sms)) != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   int grid = sms * per_sm;
   if (nstreams <= sms && p.item_base == 0) {

@@ -461,7 +461,12 @@ static cudaError_t launch_fwd_t(const CUtensorMap* m, const void* const* io, con
                                 cudaStream_t st) {
   using SM = FwdSmem<T, SEG>;
   auto kfn = ttt_linear_fwd_kernel<T, SEG, MB>;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::DYN_BYTES);
+  static DeviceValue ready;
+  int bytes = 0;
+  const cudaError_t e = ready.get(0, &bytes, [&](int* n) {
+    *n = (int)SM::DYN_BYTES;
+    return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, *n);
+  });
   if (e != cudaSuccess) return e;
   if constexpr (PairIo<T, SEG>::GATHER) {
     kfn<<<nstreams, NTHREADS, SM::DYN_BYTES, st>>>(RawTensor{const_cast<void*>(io[0])}, RawTensor{const_cast<void*>(io[1])},

@@ -1207,15 +1207,15 @@ cudaError_t launch_mlp_bwd(const MlpBwdParams& p0, int B, cudaStream_t st) {
   p.CH = MLP_BWD_CHUNK;
   p.NCH = (p.NS + p.CH - 1) / p.CH;
   const size_t smem = sizeof(MlpBwdSmem);
-  cudaError_t e = cudaFuncSetAttribute(ttt_mlp_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  static DeviceValue resident;
+  int sms = 0, per_sm = 0;
+  cudaError_t e = resident.get(0, &per_sm, [&](int* n) {
+    const cudaError_t a = cudaFuncSetAttribute(ttt_mlp_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, ttt_mlp_bwd_kernel, MB_THREADS, smem);
+  });
+  if (e != cudaSuccess || (e = device_sms(&sms)) != cudaSuccess) return e;
   // persistent grid: blocks wait on one another's hand-offs, so all of them must be resident (cooperative launch);
   // more blocks than streams would only wait (a stream's items run one after the other)
-  int dev = 0, sms = 0, per_sm = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ttt_mlp_bwd_kernel, MB_THREADS, smem)) != cudaSuccess)
-    return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   int grid = sms * per_sm;
   if (grid > p.nstreams) grid = p.nstreams;

@@ -662,18 +662,19 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 
 cudaError_t launch_mlp_fwd(const CUtensorMap* m, const MlpFwdParams& p, int nstreams, cudaStream_t st) {
   auto kfn = ttt_mlp_fwd_kernel;
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MlpSmem::DYN_BYTES);
+  static DeviceValue resident;
+  int sms = 0, per_sm = 0;
+  cudaError_t e = resident.get(0, &per_sm, [&](int* n) {
+    const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MlpSmem::DYN_BYTES);
+    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, MLP_THREADS, MlpSmem::DYN_BYTES);
+  });
   if (e != cudaSuccess) return e;
   if (p.sched == nullptr) {  // no workspace to park state in: one block per stream
     kfn<<<nstreams, MLP_THREADS, MlpSmem::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], p);
     return cudaGetLastError();
   }
   // persistent: as many blocks as are co-resident (they wait on one another's hand-offs), never more than items
-  int dev = 0, sms = 0, per_sm = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, MLP_THREADS, MlpSmem::DYN_BYTES)) != cudaSuccess)
-    return e;
+  if ((e = device_sms(&sms)) != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   MlpFwdParams pp = p;
   pp.nstreams = nstreams;

@@ -349,6 +349,7 @@ class TTT(torch.nn.Module):
         self.post_norm_bias = torch.nn.Parameter(torch.zeros(hs, **kw))
         self._wcat, self._wcat_key = None, None
         self._te, self._te_key = None, None
+        self._native_key = None
 
     # ---- one GEMM for every projection of x ----------------------------------------------------------------
     def _fused_weight(self):
@@ -436,13 +437,22 @@ class TTT(torch.nn.Module):
         i = inner.inner
         if i.mini_batch_size != c.mini_batch_size:
             return None
-        wcat, cols = self._fused_weight()
-        conv = (self.q_conv_weight, self.q_conv_bias, self.k_conv_weight, self.k_conv_bias) if c.share_qk else _NO_CONV
-        r = _lib.host().layer_infer(
-            x, wcat, self._token_eta(x.dtype), self.learnable_ttt_lr_bias, *conv, state.weight, state.bias, i.ln_weight,
-            i.ln_bias, self.post_norm_weight, self.post_norm_bias, self.o_proj, c.use_gate, c.num_heads,
-            c.mini_batch_size, _POS[c.pos_encoding], c.rope_theta, c.base_lr, cols["lr"], _eps_scaled(i.epsilon),
-            inner.allow_partial, inner.partial_in_place, start_idx)
+        # (parameters through the dictionary: attribute access on a module costs a multiple of it, and this call runs
+        # once per generated token and layer)
+        P, I, native = self._parameters.get, i._parameters.get, _lib.host()
+        key = native.param_key(P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj"), P("learnable_ttt_lr_weight"),
+                               self._buffers.get("token_idx"), P("learnable_token_idx"))
+        if self._native_key != key or self._wcat is None or self._te is None or self._te.dtype != x.dtype:
+            self._fused_weight()
+            self._token_eta(x.dtype)
+            self._native_key = key
+        wcat, cols = self._wcat
+        conv = (P("q_conv_weight"), P("q_conv_bias"), P("k_conv_weight"), P("k_conv_bias")) if c.share_qk else _NO_CONV
+        r = native.layer_infer(
+            x, wcat, self._te, P("learnable_ttt_lr_bias"), *conv, state.weight, state.bias, I("ln_weight"), I("ln_bias"),
+            P("post_norm_weight"), P("post_norm_bias"), P("o_proj"), c.use_gate, c.num_heads, c.mini_batch_size,
+            _POS[c.pos_encoding], c.rope_theta, c.base_lr, cols["lr"], _eps_scaled(i.epsilon), inner.allow_partial,
+            inner.partial_in_place, start_idx)
         if r is None:
             return None
         y, state.weight, state.bias = r
@@ -540,7 +550,7 @@ class DecodeGraphs:
     def step(self, x: torch.Tensor, start_idx: int) -> torch.Tensor:
         """One token per sequence: x [B, 1, hidden] at position `start_idx`."""
         ph = start_idx % self.period
-        if not self._graphs and x.shape == self.x.shape and x.dtype == self.x.dtype:
+        if not self._graphs and x.size(1) == 1:
             y = self.layer._infer_native(x, self.inner, self.state, ph)
             if y is not None:
                 return y
