@@ -419,15 +419,13 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       ldsm_np<NP>(aq, pq + lane_off_A(lane, 16 * ks), PL, false);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
-        mma_np<NP>(z1[nt], ak, bw[nt]);
-        mma_np<NP>(zq[nt], aq, bw[nt]);
+        mma_np2<NP>(z1[nt], ak, bw[nt], zq[nt], aq, bw[nt]);
         mma_np<NP>(kdw[nt], ak, bdw[nt]);
       }
       // the A fragments of K are also the B fragments of Q K^T (the same four 8x8 blocks in another order)
       const Pk<NP> bj0[2] = {ak[0], ak[2]}, bj1[2] = {ak[1], ak[3]};
       if (SEG == 64 || (ks >> 1) == hsel) {  // Q K^T contracts over the head's own features only
-        mma_np<NP>(at[0], aq, bj0);
-        mma_np<NP>(at[1], aq, bj1);
+        mma_np2<NP>(at[0], aq, bj0, at[1], aq, bj1);
       }
     }
     tmem_st_8x4(tm_w, wt);  // W_s^T: next used by the stage below (dW^T is unchanged so far: nothing to store)
@@ -470,8 +468,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       Pk<NP> bg[4];
       ldsm_np<NP>(bg, pg + lane_off_B_kn(lane, nb), PL, true);
       const Pk<NP> b0[2] = {bg[0], bg[1]}, b1[2] = {bg[2], bg[3]};
-      mma_np<NP>(zq[0], am, b0);
-      mma_np<NP>(zq[1], am, b1);
+      mma_np2<NP>(zq[0], am, b0, zq[1], am, b1);
     }
     // ---- 6/7. LN backward of the output (row statistics of Zbar saved by the forward) -> dZbar
     F2 dzb[2][2], dzsum[2];
@@ -545,18 +542,15 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         // P' = dZbar Gp^T (16x16, over the head's own columns); the A fragments of Gp serve as its B fragments (same
         // 8x8 blocks, other order)
         const Pk<NP> b0[2] = {ags[0], ags[2]}, b1[2] = {ags[1], ags[3]};
-        mma_np<NP>(pp[0], adz, b0);
-        mma_np<NP>(pp[1], adz, b1);
+        mma_np2<NP>(pp[0], adz, b0, pp[1], adz, b1);
       }
       {  // dq += dZbar W^T (columns nb..nb+15)
         const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
-        mma_np<NP>(dq[0], adz, b0);
-        mma_np<NP>(dq[1], adz, b1);
+        mma_np2<NP>(dq[0], adz, b0, dq[1], adz, b1);
       }
       {  // Gl' = Gp dW^T (columns nb..nb+15)
         const Pk<NP> b0[2] = {bdw[0], bdw[1]}, b1[2] = {bdw[2], bdw[3]};
-        mma_np<NP>(gl[0], ags, b0);
-        mma_np<NP>(gl[1], ags, b1);
+        mma_np2<NP>(gl[0], ags, b0, gl[1], ags, b1);
       }
     }
     // dM' = -tril(P');  dA = dM' o te[i];  d te[i] = sum_j dM'[i,j] (1 + Attn[i,j])
@@ -587,12 +581,9 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       const Pk<NP> k0[2] = {bkt[0], bkt[1]}, k1[2] = {bkt[2], bkt[3]};
       const Pk<NP> q0[2] = {bqt[0], bqt[1]}, q1[2] = {bqt[2], bqt[3]};
       const Pk<NP> z0[2] = {bdz[0], bdz[1]}, zz1[2] = {bdz[2], bdz[3]};
-      mma_np<NP>(dq[0], ada, k0);  // dq += dA K
-      mma_np<NP>(dq[1], ada, k1);
-      mma_np<NP>(dk[0], adat, q0);  // dk = dA^T Q
-      mma_np<NP>(dk[1], adat, q1);
-      mma_np<NP>(dgp[0], amt, z0);  // dGp = -M'^T dZbar
-      mma_np<NP>(dgp[1], amt, zz1);
+      mma_np2<NP>(dq[0], ada, k0, dq[1], ada, k1);  // dq += dA K
+      mma_np2<NP>(dk[0], adat, q0, dk[1], adat, q1);  // dk = dA^T Q
+      mma_np2<NP>(dgp[0], amt, z0, dgp[1], amt, zz1);  // dGp = -M'^T dZbar
     }
     // ---- 10. gradient reaching Gp, the lr / token_eta terms, and the first pair of second-derivative sums
     F2 u[2][2], v[2][2];
@@ -691,8 +682,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         ldsm_np<NP>(bwt, tW + ks * SM::PLANES + lane_off_B_kn(lane, nb), PL, true);
       }
       const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
-      mma_np<NP>(dk[0], adz1, b0);
-      mma_np<NP>(dk[1], adz1, b1);
+      mma_np2<NP>(dk[0], adz1, b0, dk[1], adz1, b1);
     }
     // dW^T += dZbar^T Q, then dW^T += dZ1^T K: both here (the dZbar tile and this stage's Q tile are still in place), so
     // that dW^T is in registers for this one stretch of the stage
@@ -706,8 +696,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         Pk<NP> bq[4];
         ldsm_np<NP>(bq, pq + lane_off_B_kn(lane, 16 * kp), PL, true);
         const Pk<NP> b0[2] = {bq[0], bq[1]}, b1[2] = {bq[2], bq[3]};
-        mma_np<NP>(dwt[2 * kp], adzt, b0);
-        mma_np<NP>(dwt[2 * kp + 1], adzt, b1);
+        mma_np2<NP>(dwt[2 * kp], adzt, b0, dwt[2 * kp + 1], adzt, b1);
       }
     }
     {
@@ -719,8 +708,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         Pk<NP> bk[4];
         ldsm_np<NP>(bk, pk + lane_off_B_kn(lane, 16 * kp), PL, true);
         const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]};
-        mma_np<NP>(dwt[2 * kp], adzt, b0);
-        mma_np<NP>(dwt[2 * kp + 1], adzt, b1);
+        mma_np2<NP>(dwt[2 * kp], adzt, b0, dwt[2 * kp + 1], adzt, b1);
       }
     }
     tmem_st_8x4(tm_dw, dwt);

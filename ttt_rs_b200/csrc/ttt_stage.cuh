@@ -189,29 +189,8 @@ __device__ __forceinline__ void g_from_pieces(const F2 (&gx)[2][2], const F2 (&x
       G[nt][r] = f2mul(f2fma(xh[nt][r], f2(-Bv[r]), f2sub(gx[nt][r], f2(A[r]))), f2(rs[r]));
 }
 
-// State update of one stage from Gp = lr o G held as transposed A fragments (agt = {n-lo/tok-lo, n-hi/tok-lo,
-// n-lo/tok-hi, n-hi/tok-hi}):   tmp = Gp^T K  (16 n x 64 k per warp),   W^T += coef * tmp.
-// Forward uses coef = -te15; the backward's reverse walk undoes a stage with coef = +te15 and the same tmp.
-template <int NP>
-__device__ __forceinline__ void state_update(float (&wt)[8][4], const Pk<NP> (&agt)[4], uint32_t k_planes, int lane,
-                                             float coef) {
-#pragma unroll
-  for (int kp = 0; kp < 4; ++kp) {
-    Pk<NP> bk[4];
-    ldsm_np<NP>(bk, k_planes + lane_off_B_kn(lane, 16 * kp), TILE_BF16_BYTES, true);
-    const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]};
-    float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f};
-    mma_np<NP>(t0, agt, b0);
-    mma_np<NP>(t1, agt, b1);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      wt[2 * kp][i] = fmaf(coef, t0[i], wt[2 * kp][i]);
-      wt[2 * kp + 1][i] = fmaf(coef, t1[i], wt[2 * kp + 1][i]);
-    }
-  }
-}
-
-// Same rank-16 update accumulated straight into the state registers: S^T += A^T-fragments x K.  Used with the state
+// Rank-16 state update of one stage from Gp = lr o G held as transposed A fragments (agt = {n-lo/tok-lo, n-hi/tok-lo,
+// n-lo/tok-hi, n-hi/tok-hi}), accumulated straight into the state registers: S^T += A^T-fragments x K.  Used with the state
 // kept as W / (-te15), so neither temporaries nor a scaling pass are needed; the backward's reversal passes the
 // fragments with their sign bits flipped.
 // `khalf`: -1 = all 64 k-columns; 0 / 1 = only k in [0,32) / [32,64) (a 32-wide head's own block when two heads share
@@ -225,8 +204,7 @@ __device__ __forceinline__ void state_update_direct(float (&wt)[8][4], const Pk<
     Pk<NP> bk[4];
     ldsm_np<NP>(bk, k_planes + lane_off_B_kn(lane, 16 * kp), TILE_BF16_BYTES, true);
     const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]};
-    mma_np<NP>(wt[2 * kp], agt, b0);
-    mma_np<NP>(wt[2 * kp + 1], agt, b1);
+    mma_np2<NP>(wt[2 * kp], agt, b0, wt[2 * kp + 1], agt, b1);
   }
 }
 template <int NP>
