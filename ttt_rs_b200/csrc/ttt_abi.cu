@@ -78,10 +78,9 @@ int make_gemm_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, 
   return TTT_OK;
 }
 
-// View of a float32 [B,H,T,32] tensor for the kernels that take a PAIR of 32-wide heads per 64-wide tile: 2-D
-// [B*H*T, 32], box = 16 tokens x 32 features = 16 rows of 128 bytes = one half tile.  (In bf16 a half tile is 64 bytes
-// wide, narrower than the swizzle span; those tiles are gathered by the kernel from the plain pointer and the map is a
-// placeholder over the same memory.)
+// View of a [B,H,T,32] tensor for the kernels that take a PAIR of 32-wide heads per 64-wide tile: 2-D
+// [B*H*T, 32], box = 16 tokens x 32 features = one half tile, swizzled over its 128-byte (float32) or
+// 64-byte (bfloat16) rows.
 int make_pair_map(CUtensorMap* m, const void* base, int64_t pairs, int64_t T, int dtype, int box_rows = 16) {
   EncodeFn enc = get_encode_fn();
   if (enc == nullptr) return fail(TTT_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
@@ -418,7 +417,7 @@ static int linear_forward_impl(const ttt_dims* d, int seq_pitch, int lr_pitch, c
   p.NCK = (int)num_ckpt(d);
   p.eps = d->epsilon;
   cudaError_t e =
-      ttt::launch_linear_fwd(d->dtype, pk.seg, d->mini_batch, maps, bases, p, (int)pk.streams,
+      ttt::launch_linear_fwd(d->dtype, pk.seg, d->mini_batch, maps, p, (int)pk.streams,
                              static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
@@ -568,7 +567,7 @@ int ttt_internal_linear_backward(const ttt_dims* d, const void* xq, const void* 
   p.NCK = (int)num_ckpt(d);
   p.eps = d->epsilon;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = ttt::launch_linear_bwd(d->dtype, pk.seg, d->mini_batch, maps, bases, p, (int)pk.streams, st);
+  cudaError_t e = ttt::launch_linear_bwd(d->dtype, pk.seg, d->mini_batch, maps, p, (int)pk.streams, st);
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "backward launch failed: %s", cudaGetErrorString(e));
   ttt::ReduceParams r;
   r.part_ln = p.part_ln;

@@ -352,13 +352,12 @@ cudaError_t launch_mlp_fwd(const CUtensorMap* maps, const MlpFwdParams& p, int n
 
 // dtype: 0 = float32, 1 = bfloat16.  seg: features per head, 64 or 32 (two heads per tile).  mb: tokens per
 // mini-batch, 16 or 8 (the tile maps then have boxes of 8 rows).
-// maps: q, k, v, out, gp (saved lr-scaled LN gradient, [B*H*T, 64] of T); io: the plain pointers behind the first
-// four maps, in the same order (used by the instantiation that gathers its tiles: seg 32 in bf16).
-cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* maps, const void* const* io,
-                              const LinFwdParams& p, int nstreams, cudaStream_t st);
-// maps: q, k, v, d_out, d_q, d_k, d_v, gp; io: the plain pointers behind the first seven.
-cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, const void* const* io,
-                              LinBwdParams& p, int nstreams, cudaStream_t st);
+// maps: q, k, v, out, gp (saved lr-scaled LN gradient, [B*H*T, 64] of T)
+cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* maps, const LinFwdParams& p, int nstreams,
+                              cudaStream_t st);
+// maps: q, k, v, d_out, d_q, d_k, d_v, gp
+cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, LinBwdParams& p, int nstreams,
+                              cudaStream_t st);
 cudaError_t launch_linear_bwd_reduce(const ReduceParams& p, cudaStream_t st);
 
 }  // namespace ttt

@@ -63,13 +63,13 @@ struct BwdSmem {
 
 template <typename T, int SEG, int MB>
 __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 : 1))
-    ttt_linear_bwd_kernel(const __grid_constant__ typename PairIo<T, SEG>::Ref tm_q,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_k,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_v,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_do,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_dq,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_dk,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_dv,
+    ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
+                          const __grid_constant__ CUtensorMap tm_k,
+                          const __grid_constant__ CUtensorMap tm_v,
+                          const __grid_constant__ CUtensorMap tm_do,
+                          const __grid_constant__ CUtensorMap tm_dq,
+                          const __grid_constant__ CUtensorMap tm_dk,
+                          const __grid_constant__ CUtensorMap tm_dv,
                           const __grid_constant__ CUtensorMap tm_g, const LinBwdParams p) {
   using TF = TileFmt<T>;
   using SM = BwdSmem<T, SEG>;
@@ -77,11 +77,6 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
   constexpr uint32_t PL = TILE_BF16_BYTES;  // plane stride
   constexpr float INV_F = 1.f / SEG;        // features per head (LayerNorm row length)
   constexpr int NH = (SEG == 32) ? 2 : 1;   // heads per tile
-  // The loads of the next stage are issued by the first thread of warp 1, the stores (and their bulk groups) by thread
-  // 0: one warp doing both arrives at the stage's barriers that much later than the other three.
-  constexpr int LOADER = 32;
-  constexpr bool GATHER = PairIo<T, SEG>::GATHER;  // q, k, v, d_out, d_q, d_k, d_v tiles moved by the threads, not TMA
-
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = smem_u32(smem_raw);
   const uint32_t base = (raw_u32 + 1023u) & ~1023u;
@@ -92,6 +87,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
 
   const Lane L;
   const int tid = L.tid, lane = L.lane, g = L.g, t = L.t, nb = L.nb, warp = L.warp;
+  const int uw = __shfl_sync(0xffffffffu, warp, 0);  // (known to be the same in all lanes)
   const int hsel = warp >> 1;                 // SEG = 32: which head of the pair this warp's columns belong to
   const int khalf = (SEG == 32) ? hsel : -1;  // and the k-range of W^T / dW^T that is its own block
   const int NS = p.NS;
@@ -109,20 +105,15 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
   const uint32_t tm_w = s_tmem + ((32u * (uint32_t)warp) << 16), tm_dw = tm_w + 32u;
 
   if (tid == 0) {
-    if constexpr (!GATHER) {
-      prefetch_tmap(&tm_q);
-      prefetch_tmap(&tm_k);
-      prefetch_tmap(&tm_v);
-      prefetch_tmap(&tm_do);
-    }
+    prefetch_tmap(&tm_q);
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
+    prefetch_tmap(&tm_do);
     prefetch_tmap(&tm_g);
-    if constexpr (!GATHER) {
-      prefetch_tmap(&tm_dq);
-      prefetch_tmap(&tm_dk);
-      prefetch_tmap(&tm_dv);
-    }
-    // arrivals per phase: thread 0's expect_tx, plus every thread's cp.async arrival where tiles are gathered
-    for (int i = 0; i < SM::NSLOT; ++i) mbar_init(bar0 + 8 * i, GATHER ? 1 + NTHREADS : 1);
+    prefetch_tmap(&tm_dq);
+    prefetch_tmap(&tm_dk);
+    prefetch_tmap(&tm_dv);
+    for (int i = 0; i < SM::NSLOT; ++i) mbar_init(bar0 + 8 * i, 4);  // each warp counts the bytes of its own copies
     fence_mbar_init();
   }
   if constexpr (MB < CS) {
@@ -131,11 +122,12 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     for (uint32_t e = tid * 4; e < SM::NSLOT * SM::SLOT; e += NTHREADS * 4) {
       const uint32_t o = e % SM::SLOT;
       bool pad = false;
-      if (o < 3 * TF::BYTES) {  // q, k, gp: raw tile, then operand planes derived from it
-        const uint32_t in_tile = o % TF::BYTES;
-        pad = in_tile >= TF::RAW_BYTES || (in_tile % 2048) >= MB * 128;
+      if (o < 2 * TF::BYTES) {  // q, k: raw tile, then operand planes derived from it
+        pad = io_pad<T, SEG, MB>(o % TF::BYTES);
+      } else if (o < SM::OFF_V) {  // gp: always in the 64-wide form
+        pad = io_pad<T, 64, MB>(o - SM::OFF_G);
       } else if (o < SM::OFF_STAT) {  // v, d_out: raw tiles
-        pad = ((o - 3 * TF::BYTES) % 2048) >= MB * 128;
+        pad = io_pad<T, SEG, MB>((o - SM::OFF_V) % TF::RAW_BYTES);
       } else if (o < SM::OFF_BS) {
         pad = (o - SM::OFF_STAT) >= MB * 32 * NH;
       } else if (o >= SM::OFF_LR) {
@@ -146,50 +138,64 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
   }
   __syncthreads();
 
-  // everything stage s needs, into slot n % NSLOT (thread 0: TMA / bulk copies)
+  // Everything stage s needs, into slot n % NSLOT, and the output tiles of a stage from their staging buffers.  Issuing a copy
+  // takes its thread some 100 cycles, on the way of the stage's next barrier whichever warp does it: they are spread over
+  // the four warps, and a stage's stores share the next stage's first barrier (bf16, 64 stages: 146 -> 134 us at 12 streams,
+  // 291 -> 278 us at 384; float32: 453 -> 442 us at 96).  Pairs of 32-wide heads come as two 64-byte-swizzled boxes per tile
+  // (gathered by the threads they cost 162 us at 72 heads, 150 us this way).
   auto issue_loads = [&](int n, int s) {
     const int slot = n % SM::NSLOT;
     const uint32_t bar = bar0 + 8 * slot;
     const uint32_t sl = base + slot * SM::SLOT;
     const int r0 = row_base + s * MB;
-    if constexpr (SEG == 64) {
-      mbar_expect_tx(bar, (5u * TF::RAW_BYTES + 512u + CS * TF::ELT) * MB / CS + 256u);
-      tma_load_tile<T>(sl + SM::OFF_K, &tm_k, r0, bar);
-      tma_load_tile<T>(sl + SM::OFF_G, &tm_g, r0, bar);
-      tma_load_tile<T>(sl + SM::OFF_Q, &tm_q, r0, bar);
-      tma_load_tile<T>(sl + SM::OFF_V, &tm_v, r0, bar);
-      tma_load_tile<T>(sl + SM::OFF_DO, &tm_do, r0, bar);
-      bulk_load_1d(sl + SM::OFF_STAT, p.stats + (size_t)r0 * 2, 512u * MB / CS, bar);
-      bulk_load_1d(sl + SM::OFF_BS, p.b_stage + ((size_t)stream * (NS + 1) + s) * HD, 256u, bar);
-      bulk_load_1d(sl + SM::OFF_LR, static_cast<const uint8_t*>(p.lr) + (size_t)r0 * TF::ELT, MB * TF::ELT, bar);
-    } else {
-      mbar_expect_tx(bar, ((GATHER ? 1u : 5u) * TF::RAW_BYTES + 1024u + 2 * CS * TF::ELT) * MB / CS + 256u);
-      tma_load_tile<T>(sl + SM::OFF_G, &tm_g, r0, bar);  // saved tiles are kept in the packed 64-wide form
-      if constexpr (!GATHER) {
-        tma_load_pair<T>(sl + SM::OFF_K, &tm_k, stream, s * MB, p.T, bar);
-        tma_load_pair<T>(sl + SM::OFF_Q, &tm_q, stream, s * MB, p.T, bar);
-        tma_load_pair<T>(sl + SM::OFF_V, &tm_v, stream, s * MB, p.T, bar);
-        tma_load_pair<T>(sl + SM::OFF_DO, &tm_do, stream, s * MB, p.T, bar);
-      }
-      bulk_load_1d(sl + SM::OFF_STAT, p.stats + (size_t)r0 * 4, 1024u * MB / CS, bar);
-      bulk_load_1d(sl + SM::OFF_BS, p.b_stage + ((size_t)stream * (NS + 1) + s) * HD, 256u, bar);
+    constexpr uint32_t TILE = TF::RAW_BYTES * MB / CS;
+    if (uw == 0) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, TILE + NH * MB * TF::ELT);
+        tma_load_tile<T>(sl + SM::OFF_G, &tm_g, r0, bar);  // saved tiles are kept in the packed 64-wide form
 #pragma unroll
-      for (int j = 0; j < 2; ++j)  // ttt_lr_eta is [B, H, T]: the two heads of the pair are T elements apart
-        bulk_load_1d(sl + SM::OFF_LR + j * CS * TF::ELT,
-                     static_cast<const uint8_t*>(p.lr) + ((size_t)(2 * stream + j) * p.T + s * MB) * TF::ELT,
-                     MB * TF::ELT, bar);
+        for (int j = 0; j < NH; ++j)  // ttt_lr_eta is [B, H, T]: the two heads of a pair are T elements apart
+          bulk_load_1d(sl + SM::OFF_LR + j * CS * TF::ELT,
+                       static_cast<const uint8_t*>(p.lr) + ((size_t)(NH * stream + j) * p.T + s * MB) * TF::ELT,
+                       MB * TF::ELT, bar);
+      }
+    } else if (uw == 1) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, TILE + 512u * NH * MB / CS);
+        tma_load_io<T, SEG>(sl + SM::OFF_K, &tm_k, stream, s * MB, p.T, bar);
+        bulk_load_1d(sl + SM::OFF_STAT, p.stats + (size_t)r0 * 2 * NH, 512u * NH * MB / CS, bar);
+      }
+    } else if (uw == 2) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, TILE + 256u);
+        tma_load_io<T, SEG>(sl + SM::OFF_DO, &tm_do, stream, s * MB, p.T, bar);
+        bulk_load_1d(sl + SM::OFF_BS, p.b_stage + ((size_t)stream * (NS + 1) + s) * HD, 256u, bar);
+      }
+    } else {
+      if (elect_one()) {
+        mbar_expect_tx(bar, 2 * TILE);
+        tma_load_io<T, SEG>(sl + SM::OFF_Q, &tm_q, stream, s * MB, p.T, bar);
+        tma_load_io<T, SEG>(sl + SM::OFF_V, &tm_v, stream, s * MB, p.T, bar);
+      }
     }
   };
-  // every thread, where tiles are gathered: its 16-byte chunk of the k, q, v, d_out tiles, then its arrival
-  auto issue_gather = [&](int n, int s) {
-    if constexpr (GATHER) {
-      const int slot = n % SM::NSLOT;
-      const uint32_t sl = base + slot * SM::SLOT;
-      gather_pair_tile_bf16<MB>(sl + SM::OFF_K, tm_k.ptr, stream, s * MB, p.T, tid);
-      gather_pair_tile_bf16<MB>(sl + SM::OFF_Q, tm_q.ptr, stream, s * MB, p.T, tid);
-      gather_pair_tile_bf16<MB>(sl + SM::OFF_V, tm_v.ptr, stream, s * MB, p.T, tid);
-      gather_pair_tile_bf16<MB>(sl + SM::OFF_DO, tm_do.ptr, stream, s * MB, p.T, tid);
-      cp_async_mbar_arrive_noinc(bar0 + 8 * slot);
+  auto issue_stores = [&](int s) {
+    const uint32_t so = base + SM::OFF_OUT + uw * TF::RAW_BYTES;
+    if (uw == 0) {
+      if (elect_one()) {
+        tma_store_io<T, SEG>(&tm_dq, stream, s * MB, p.T, so);
+        bulk_commit();
+      }
+    } else if (uw == 1) {
+      if (elect_one()) {
+        tma_store_io<T, SEG>(&tm_dk, stream, s * MB, p.T, so);
+        bulk_commit();
+      }
+    } else if (uw == 2) {
+      if (elect_one()) {
+        tma_store_io<T, SEG>(&tm_dv, stream, s * MB, p.T, so);
+        bulk_commit();
+      }
     }
   };
 
@@ -241,8 +247,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     row_base = stream * p.T;
     const int head = stream % p.H;
     const int s_lo = chunk * p.CH, s_hi = min(s_lo + p.CH, NS) - 1;
-    if (tid == LOADER) issue_loads(n, s_hi);
-    issue_gather(n, s_hi);
+    issue_loads(n, s_hi);
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
       const int c = nb + 8 * nt + 2 * t;
@@ -351,12 +356,12 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     int fail = mbar_wait_bounded(bar0 + 8 * slot, (n / SM::NSLOT) & 1) ? 0 : 1;
     bool next_issued = false;
     auto issue_next = [&]() {
-      // runs right after the first CTA barrier of this stage: every thread has left the previous stage,
-      // so the other slot may be overwritten
+      // right behind the first CTA barrier of this stage: every thread has left the previous stage, so its output tiles
+      // are complete and the other slot may be overwritten
       if (!next_issued) {
         next_issued = true;
-        if (tid == LOADER && s > s_lo) issue_loads(n + 1, s - 1);
-        if (GATHER && s > s_lo) issue_gather(n + 1, s - 1);
+        if (s < s_hi) issue_stores(s + 1);
+        if (s > s_lo) issue_loads(n + 1, s - 1);
       }
     };
     if constexpr (NP == 3) {
@@ -371,7 +376,6 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         if (tid == 0) report_timeout(p.status, 11, s);
         break;
       }
-      issue_next();
     }
     // (SEG = 32: the pair's second head has its 16 values right after the first head's)
     const float lr_row[2] = {ld_as_float<T>(gsl + SM::OFF_LR, (SEG == 32 ? hsel * CS : 0) + g),
@@ -386,7 +390,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       if (w_moves) {
         ldsm_np<NP>(agt, pg + lane_off_B_nk(lane, nb), PL, true);
         const Pk<NP> ngt[4] = {neg_pk<NP>(agt[0]), neg_pk<NP>(agt[1]), neg_pk<NP>(agt[2]), neg_pk<NP>(agt[3])};
-        state_update_direct<NP>(wt, ngt, pk, lane, khalf);
+        state_update_direct<NP, SEG>(wt, ngt, pk, lane, khalf);
       }
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
@@ -415,8 +419,8 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       Pk<NP> bw[2][2], bdw[2][2], ak[4], aq[4];
       bfrag_from_state<NP>(wt, ks, bw);
       bfrag_from_state<NP>(dwt, ks, bdw);
-      ldsm_np<NP>(ak, pk + lane_off_A(lane, 16 * ks), PL, false);
-      ldsm_np<NP>(aq, pq + lane_off_A(lane, 16 * ks), PL, false);
+      ldsm_np<NP>(ak, pk + lane_off_io<T, SEG>(lane, 16 * ks), PL, false);
+      ldsm_np<NP>(aq, pq + lane_off_io<T, SEG>(lane, 16 * ks), PL, false);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
         mma_np2<NP>(z1[nt], ak, bw[nt], zq[nt], aq, bw[nt]);
@@ -451,7 +455,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       F2 z1p[2][2];
       slab_pairs(z1, z1p);
       float sa[2], sb[2];
-      ln_l2_pieces<T>(z1p, mean1, rstd1, gam, bet, tk, tv, L, xh, gy, gx, sa, sb);
+      ln_l2_pieces<T, SEG>(z1p, mean1, rstd1, gam, bet, tk, tv, L, xh, gy, gx, sa, sb);
       g_from_pieces(gx, xh, A, Bv1, rstd1, G);
     }
     // ---- 5. Zbar = Zq - M' Gp   (am holds -M')
@@ -480,7 +484,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const F2 d = ld_pair<T>(tdo, g + 8 * r, nb + 8 * nt + 2 * t);
+          const F2 d = ld_io<T, SEG>(tdo, g + 8 * r, nb + 8 * nt + 2 * t);
           const F2 x = f2mul(f2sub(pr(zq[nt], r), f2(mean2[r])), f2(rstd2[r]));
           xz[nt][r] = x;
           dq[nt][2 * r] = d.x;
@@ -573,8 +577,8 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     }
     {
       Pk<NP> bkt[4], bqt[4], bdz[4];
-      ldsm_np<NP>(bkt, pk + lane_off_B_kn(lane, nb), PL, true);
-      ldsm_np<NP>(bqt, pq + lane_off_B_kn(lane, nb), PL, true);
+      ldsm_np<NP>(bkt, pk + lane_off_io<T, SEG>(lane, nb), PL, true);
+      ldsm_np<NP>(bqt, pq + lane_off_io<T, SEG>(lane, nb), PL, true);
       ldsm_np<NP>(bdz, tDZ + lane_off_B_kn(lane, nb), PL, true);
       const Pk<NP> adat[4] = {movm_t_np<NP>(ada[0]), movm_t_np<NP>(ada[2]), movm_t_np<NP>(ada[1]), movm_t_np<NP>(ada[3])};
       const Pk<NP> amt[4] = {movm_t_np<NP>(am[0]), movm_t_np<NP>(am[2]), movm_t_np<NP>(am[1]), movm_t_np<NP>(am[3])};
@@ -594,7 +598,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const F2 kk = ld_pair<T>(tk, g + 8 * r, nb + 8 * nt + 2 * t);
+          const F2 kk = ld_io<T, SEG>(tk, g + 8 * r, nb + 8 * nt + 2 * t);
           const F2 glp = pr(gl[nt], r);
           // dL/dGp = -M'^T dZbar - te15 (K dW + db)
           const F2 dg = f2fma(f2add(pr(kdw[nt], r), dbias[nt]), f2(-te15), pr(dgp[nt], r));
@@ -668,7 +672,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
       for (int r = 0; r < 2; ++r) st_pair_planes<NP>(tDZ1, g + 8 * r, nb + 8 * nt + 2 * t, dz1[nt][r].x, dz1[nt][r].y);
-    if (tid == 0) bulk_wait_read<0>();  // the previous stage's output tiles have left the staging buffers
+    if (elect_one()) bulk_wait_read<0>();  // the previous stage's output tiles have left the staging buffers
     __syncthreads();
     // ---- 13. dk += dZ1 W^T ; dW^T += dZ1^T K ; bias gradient
 #pragma unroll
@@ -694,7 +698,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       for (int kp = 0; kp < 4; ++kp) {
         if (khalf >= 0 && (kp >> 1) != khalf) continue;  // paired heads: only the head's own block of dW^T
         Pk<NP> bq[4];
-        ldsm_np<NP>(bq, pq + lane_off_B_kn(lane, 16 * kp), PL, true);
+        ldsm_np<NP>(bq, pq + lane_off_io<T, SEG>(lane, 16 * kp), PL, true);
         const Pk<NP> b0[2] = {bq[0], bq[1]}, b1[2] = {bq[2], bq[3]};
         mma_np2<NP>(dwt[2 * kp], adzt, b0, dwt[2 * kp + 1], adzt, b1);
       }
@@ -706,7 +710,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       for (int kp = 0; kp < 4; ++kp) {
         if (khalf >= 0 && (kp >> 1) != khalf) continue;
         Pk<NP> bk[4];
-        ldsm_np<NP>(bk, pk + lane_off_B_kn(lane, 16 * kp), PL, true);
+        ldsm_np<NP>(bk, pk + lane_off_io<T, SEG>(lane, 16 * kp), PL, true);
         const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]};
         mma_np2<NP>(dwt[2 * kp], adzt, b0, dwt[2 * kp + 1], adzt, b1);
       }
@@ -726,33 +730,17 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         for (int r = 0; r < 2; ++r) {
           const int row = g + 8 * r, col = nb + 8 * nt + 2 * t;
           const F2 dkk = f2sub(pr(dk[nt], r), dT[nt][r]);
-          st_pair<T>(so_q, row, col, dq[nt][2 * r], dq[nt][2 * r + 1]);
-          st_pair<T>(so_k, row, col, dkk.x, dkk.y);
-          st_pair<T>(so_v, row, col, dT[nt][r].x, dT[nt][r].y);
+          st_io<T, SEG>(so_q, row, col, dq[nt][2 * r], dq[nt][2 * r + 1]);
+          st_io<T, SEG>(so_k, row, col, dkk.x, dkk.y);
+          st_io<T, SEG>(so_v, row, col, dT[nt][r].x, dT[nt][r].y);
         }
-      fence_proxy_async_smem();
-      __syncthreads();
-      if constexpr (GATHER) {
-        scatter_pair_tile_bf16<MB>(tm_dq.ptr, stream, s * MB, p.T, so_q, tid);
-        scatter_pair_tile_bf16<MB>(tm_dk.ptr, stream, s * MB, p.T, so_k, tid);
-        scatter_pair_tile_bf16<MB>(tm_dv.ptr, stream, s * MB, p.T, so_v, tid);
-      } else if (tid == 0) {
-        if constexpr (SEG == 64) {
-          const int r0 = row_base + s * MB;
-          tma_store_tile<T>(&tm_dq, r0, so_q);
-          tma_store_tile<T>(&tm_dk, r0, so_k);
-          tma_store_tile<T>(&tm_dv, r0, so_v);
-        } else {
-          tma_store_pair<T>(&tm_dq, stream, s * MB, p.T, so_q);
-          tma_store_pair<T>(&tm_dk, stream, s * MB, p.T, so_k);
-          tma_store_pair<T>(&tm_dv, stream, s * MB, p.T, so_v);
-        }
-        bulk_commit();
-      }
+      fence_proxy_async_smem();  // (stored behind the next stage's first barrier)
     }
   }
 
     if (failed) break;
+    __syncthreads();
+    issue_stores(s_lo);
     tmem_wait_st();
     tmem_ld_8x4(tm_w, wt);
     tmem_ld_8x4(tm_dw, dwt);
@@ -821,8 +809,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       }
     }
   }  // item loop
-  if (tid == 0) bulk_wait_all<0>();
-  if constexpr (GATHER) cp_async_wait_all();  // (an item that gave up may leave gathers in flight)
+  if (elect_one()) bulk_wait_all<0>();
   tmem_wait_st();
   tmem_fence_before_sync();
   __syncthreads();
@@ -903,7 +890,7 @@ __global__ void ttt_linear_bwd_fold_kernel(const ReduceParams p) {
 }
 
 template <typename T, int SEG, int MB>
-static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, LinBwdParams& p, int nstreams,
+static cudaError_t launch_bwd_t(const CUtensorMap* m, LinBwdParams& p, int nstreams,
                                 cudaStream_t st) {
   using SM = BwdSmem<T, SEG>;
   auto kfn = ttt_linear_bwd_kernel<T, SEG, MB>;
@@ -944,33 +931,25 @@ static cudaError_t launch_bwd_t(const CUtensorMap* m, const void* const* io, Lin
   if (grid > nitems) grid = nitems;
   if (p.sched != nullptr && (e = cudaMemsetAsync(p.sched, 0, sizeof(int) * (size_t)(1 + nstreams), st)) != cudaSuccess)
     return e;
-  LinBwdParams pp = p;
-  RawTensor raw[7];
-  void* args[9];
-  for (int i = 0; i < 7; ++i) {
-    raw[i].ptr = const_cast<void*>(io[i]);
-    args[i] = PairIo<T, SEG>::GATHER ? (void*)&raw[i] : (void*)&m[i];
-  }
-  args[7] = (void*)&m[7];
-  args[8] = (void*)&pp;
-  return cudaLaunchKernel((const void*)kfn, dim3(grid), dim3(NTHREADS), args, SM::DYN_BYTES, st);
+  kfn<<<grid, NTHREADS, SM::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], p);
+  return cudaGetLastError();
 }
 
 template <typename T, int SEG>
-static cudaError_t launch_bwd_mb(int mb, const CUtensorMap* m, const void* const* io, LinBwdParams& p,
+static cudaError_t launch_bwd_mb(int mb, const CUtensorMap* m, LinBwdParams& p,
                                  int nstreams, cudaStream_t st) {
-  return mb == 8 ? launch_bwd_t<T, SEG, 8>(m, io, p, nstreams, st) : launch_bwd_t<T, SEG, 16>(m, io, p, nstreams, st);
+  return mb == 8 ? launch_bwd_t<T, SEG, 8>(m, p, nstreams, st) : launch_bwd_t<T, SEG, 16>(m, p, nstreams, st);
 }
 
 // mb: tokens per mini-batch, 16 or 8 (the maps' boxes then have 8 rows)
-cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, const void* const* io,
+cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps,
                               LinBwdParams& p, int nstreams, cudaStream_t st) {
   if (seg == 32) {
-    if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 32>(mb, maps, io, p, nstreams, st);
-    return launch_bwd_mb<float, 32>(mb, maps, io, p, nstreams, st);
+    if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 32>(mb, maps, p, nstreams, st);
+    return launch_bwd_mb<float, 32>(mb, maps, p, nstreams, st);
   }
-  if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 64>(mb, maps, io, p, nstreams, st);
-  return launch_bwd_mb<float, 64>(mb, maps, io, p, nstreams, st);
+  if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 64>(mb, maps, p, nstreams, st);
+  return launch_bwd_mb<float, 64>(mb, maps, p, nstreams, st);
 }
 
 cudaError_t launch_linear_bwd_reduce(const ReduceParams& p, cudaStream_t st) {

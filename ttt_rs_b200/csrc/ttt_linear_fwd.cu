@@ -50,17 +50,16 @@ struct FwdSmem {
 
 template <typename T, int SEG, int MB>
 __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
-    ttt_linear_fwd_kernel(const __grid_constant__ typename PairIo<T, SEG>::Ref tm_q,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_k,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_v,
-                          const __grid_constant__ typename PairIo<T, SEG>::Ref tm_o,
+    ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
+                          const __grid_constant__ CUtensorMap tm_k,
+                          const __grid_constant__ CUtensorMap tm_v,
+                          const __grid_constant__ CUtensorMap tm_o,
                           const __grid_constant__ CUtensorMap tm_g, const LinFwdParams p) {
   using TF = TileFmt<T>;
   using SM = FwdSmem<T, SEG>;
   constexpr int NP = TF::NP;
   constexpr bool TWO_PASS = (sizeof(T) == 4);
   constexpr float INV_F = 1.f / SEG;  // features per head (LayerNorm row length)
-  constexpr bool GATHER = PairIo<T, SEG>::GATHER;  // q, k, v, out tiles moved by the threads instead of TMA
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = smem_u32(smem_raw);
@@ -71,6 +70,8 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
 
   const Lane L;
   const int tid = L.tid, lane = L.lane, g = L.g, t = L.t, nb = L.nb;
+  const int warp = __shfl_sync(0xffffffffu, L.warp, 0);  // (known to be the same in all lanes)
+  constexpr int HPT = HD / SEG;              // heads per tile
   const int hsel = L.warp >> 1;              // SEG = 32: which head of the pair this warp's columns belong to
   const int khalf = (SEG == 32) ? hsel : -1; // and the k-range of the state that is its own block
   const int stream = blockIdx.x;             // (batch, head) stream, or (batch, pair of heads) when SEG = 32
@@ -82,24 +83,18 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
   const bool save = (p.w_ckpt != nullptr);
 
   if (tid == 0) {
-    if constexpr (!GATHER) {
-      prefetch_tmap(&tm_q);
-      prefetch_tmap(&tm_k);
-      prefetch_tmap(&tm_v);
-      prefetch_tmap(&tm_o);
-    }
+    prefetch_tmap(&tm_q);
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
+    prefetch_tmap(&tm_o);
     prefetch_tmap(&tm_g);
-    // arrivals per phase: thread 0's expect_tx, plus every thread's cp.async arrival where tiles are gathered
-    for (int i = 0; i < FWD_NST; ++i) mbar_init(bar0 + 8 * i, GATHER ? 1 + NTHREADS : 1);
+    for (int i = 0; i < FWD_NST; ++i) mbar_init(bar0 + 8 * i, 3);  // the three warps that load count their own bytes
     fence_mbar_init();
   }
   if constexpr (MB < CS) {
     // padding rows of every tile of the ring, and the lr slots: zero once; the copies only ever write the first MB rows
     for (uint32_t e = tid * 16; e < FWD_NST * SM::SLOT; e += NTHREADS * 16) {
-      const uint32_t in_tile = e % TF::BYTES;
-      // raw tile: 16 rows of 128 bytes (bf16) or two halves of 16 rows of 128 bytes (f32); planes are derived from it
-      const bool raw = in_tile < TF::RAW_BYTES;
-      if (!raw || (in_tile % 2048) >= MB * 128)
+      if (io_pad<T, SEG, MB>(e % TF::BYTES))
         asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(base + e), "r"(0u) : "memory");
     }
     for (uint32_t e = tid * 4; e < FWD_NST * SM::LR_SLOT; e += NTHREADS * 4)
@@ -107,49 +102,52 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
   }
   __syncthreads();
 
-  // thread 0: TMA / bulk copies of one stage into its ring slot
-  auto issue_loads = [&](int s) {
-    const int slot = s % FWD_NST;
-    const uint32_t bar = bar0 + 8 * slot;
-    const uint32_t tq = base + slot * SM::SLOT;
-    if constexpr (SEG == 64) {
-      mbar_expect_tx(bar, (3 * TF::RAW_BYTES + CS * TF::ELT) * MB / CS);
-      const int r0 = row_base + s * MB;
-      tma_load_tile<T>(tq, &tm_q, r0, bar);
-      tma_load_tile<T>(tq + TF::BYTES, &tm_k, r0, bar);
-      tma_load_tile<T>(tq + 2 * TF::BYTES, &tm_v, r0, bar);
-      bulk_load_1d(base + SM::OFF_LR + slot * 64,
-                   static_cast<const uint8_t*>(p.lr) + ((size_t)stream * p.lr_ld + s * MB) * TF::ELT, MB * TF::ELT, bar);
-    } else {
-      mbar_expect_tx(bar, ((GATHER ? 0 : 3 * TF::RAW_BYTES) + 2 * CS * TF::ELT) * MB / CS);
-      if constexpr (!GATHER) {
-        tma_load_pair<T>(tq, &tm_q, stream, s * MB, p.T, bar);
-        tma_load_pair<T>(tq + TF::BYTES, &tm_k, stream, s * MB, p.T, bar);
-        tma_load_pair<T>(tq + 2 * TF::BYTES, &tm_v, stream, s * MB, p.T, bar);
-      }
+  // The copies of a stage, in and out.  Issuing one takes its thread some 100 cycles, on the way of the stage's next barrier
+  // whichever warp does it, so they are spread: warp 1 loads v and lr, warp 2 q, warp 3 k; warp 0 stores the output, warp 2
+  // the saved Gp tile.  (64 stages of float32: 204 -> 196 us at 96 streams; bf16 heads of 32, which were gathered by the
+  // threads: 129 -> 121 us at 768 heads; bf16 heads of 64 as before.)
+  auto issue_loads = [&](int s, int slot) {
+    const uint32_t bar = bar0 + 8 * slot, tq = base + slot * SM::SLOT;
+    constexpr uint32_t TILE = TF::RAW_BYTES * MB / CS;
+    if (warp == 1) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, TILE + HPT * MB * TF::ELT);
+        tma_load_io<T, SEG>(tq + 2 * TF::BYTES, &tm_v, stream, s * MB, p.T, bar);
 #pragma unroll
-      for (int j = 0; j < 2; ++j)  // ttt_lr_eta is [B, H, T]: the two heads of the pair are T elements apart
-        bulk_load_1d(base + SM::OFF_LR + slot * SM::LR_SLOT + j * CS * TF::ELT,
-                     static_cast<const uint8_t*>(p.lr) + ((size_t)(2 * stream + j) * p.lr_ld + s * MB) * TF::ELT,
-                     MB * TF::ELT, bar);
+        for (int j = 0; j < HPT; ++j)  // ttt_lr_eta is [B, H, T]: the two heads of a pair are lr_ld elements apart
+          bulk_load_1d(base + SM::OFF_LR + slot * SM::LR_SLOT + j * CS * TF::ELT,
+                       static_cast<const uint8_t*>(p.lr) + ((size_t)(HPT * stream + j) * p.lr_ld + s * MB) * TF::ELT,
+                       MB * TF::ELT, bar);
+      }
+    } else if (warp == 2) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, TILE);
+        tma_load_io<T, SEG>(tq, &tm_q, stream, s * MB, p.T, bar);
+      }
+    } else if (warp == 3) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, TILE);
+        tma_load_io<T, SEG>(tq + TF::BYTES, &tm_k, stream, s * MB, p.T, bar);
+      }
     }
   };
-  // every thread, where tiles are gathered: its 16-byte chunk of the q, k, v tiles, then its arrival on the barrier
-  auto issue_gather = [&](int s) {
-    if constexpr (GATHER) {
-      const int slot = s % FWD_NST;
-      const uint32_t tq = base + slot * SM::SLOT;
-      gather_pair_tile_bf16<MB>(tq, tm_q.ptr, stream, s * MB, p.T, tid);
-      gather_pair_tile_bf16<MB>(tq + TF::BYTES, tm_k.ptr, stream, s * MB, p.T, tid);
-      gather_pair_tile_bf16<MB>(tq + 2 * TF::BYTES, tm_v.ptr, stream, s * MB, p.T, tid);
-      cp_async_mbar_arrive_noinc(bar0 + 8 * slot);
+  auto issue_stores = [&](int s) {
+    if (warp == 0) {
+      if (elect_one()) {
+        tma_store_io<T, SEG>(&tm_o, stream, s * MB, p.T, base + SM::OFF_OUT + (s & 1) * TF::RAW_BYTES);
+        bulk_commit();
+        bulk_wait_read<1>();
+      }
+    } else if (warp == 2 && save) {
+      if (elect_one()) {
+        // saved tiles are kept in the packed 64-wide form
+        tma_store_tile<T>(&tm_g, row_base + s * MB, base + SM::OFF_OUT + (2 + (s & 1)) * TF::RAW_BYTES);
+        bulk_commit();
+        bulk_wait_read<1>();
+      }
     }
   };
-  if (tid == 0) {
-    for (int s = 0; s < FWD_NST && s < NS; ++s) issue_loads(s);
-  }
-  if constexpr (GATHER)
-    for (int s = 0; s < FWD_NST && s < NS; ++s) issue_gather(s);
+  for (int s = 0; s < FWD_NST && s < NS; ++s) issue_loads(s, s);
 
   // ---- per-thread constants: 4 owned columns c(nt,e) = nb + 8nt + 2t + e, rows g and g+8
   F2 gam[2], bet[2];
@@ -231,8 +229,8 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
       Pk<NP> bw[2][2];
       bfrag_from_state<NP>(wt, ks, bw);
       Pk<NP> ak[4], aq[4];
-      ldsm_np<NP>(ak, pk + lane_off_A(lane, 16 * ks), TILE_BF16_BYTES, false);
-      ldsm_np<NP>(aq, pq + lane_off_A(lane, 16 * ks), TILE_BF16_BYTES, false);
+      ldsm_np<NP>(ak, pk + lane_off_io<T, SEG>(lane, 16 * ks), TILE_BF16_BYTES, false);
+      ldsm_np<NP>(aq, pq + lane_off_io<T, SEG>(lane, 16 * ks), TILE_BF16_BYTES, false);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
         mma_np2<NP>(z1[nt], ak, bw[nt], zq[nt], aq, bw[nt]);
@@ -288,12 +286,17 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
       if (tid == 0) report_timeout(p.status, 2, s);
       return false;
     }
+    // behind this barrier every thread has left the previous stage: its outputs are complete, its ring slot is free
+    if (s > 0) {
+      issue_stores(s - 1);
+      if (s + FWD_NST - 1 < NS) issue_loads(s + FWD_NST - 1, slot == 0 ? FWD_NST - 1 : slot - 1);
+    }
     F2 gp[2][2];
     float4 st1[2];  // saved row statistics of Z1: (mean, rstd, mean(gx), mean(gx * x_hat))
     {
       F2 xh[2][2], gy[2][2], gx[2][2];
       float sa[2], sb[2];
-      ln_l2_pieces<T>(z1p, mean, rstd, gam, bet, tk, tv, L, xh, gy, gx, sa, sb);
+      ln_l2_pieces<T, SEG>(z1p, mean, rstd, gam, bet, tk, tv, L, xh, gy, gx, sa, sb);
       float2 a0, a1;
       int f2_ = 0;
       xch_rows2<SEG, false>(&xch[xsel], L, sa[0], sb[0], sa[1], sb[1], a0, a1, f2_);
@@ -345,7 +348,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
     // ---- state update: W^T[nb.., :] -= te15 * Gp^T K ; b -= te15 * colsum(Gp)
     {
       const Pk<NP> agt[4] = {gt[0][0], gt[1][0], gt[0][1], gt[1][1]};
-      if (w_moves) state_update_direct<NP>(wt, agt, pk, lane, khalf);
+      if (w_moves) state_update_direct<NP, SEG>(wt, agt, pk, lane, khalf);
       if constexpr (NP == 1) {
         // column sums of the bf16 Gp tile as a product with a tile of ones (every row of the result is the sum)
         constexpr uint32_t ONES = 0x3F803F80u;
@@ -398,24 +401,10 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
       for (int r = 0; r < 2; ++r) {
         const int row = g + 8 * r, col = nb + 8 * nt + 2 * t;
         const F2 x = f2mul(f2sub(zb[nt][r], f2(mean[r])), f2(rstd[r]));
-        const F2 o = f2add(ld_pair<T>(tq, row, col), f2fma(gam[nt], x, bet[nt]));
-        st_pair<T>(so, row, col, o.x, o.y);
+        const F2 o = f2add(ld_io<T, SEG>(tq, row, col), f2fma(gam[nt], x, bet[nt]));
+        st_io<T, SEG>(so, row, col, o.x, o.y);
       }
-    fence_proxy_async_smem();
-    __syncthreads();
-    if constexpr (GATHER) scatter_pair_tile_bf16<MB>(tm_o.ptr, stream, s * MB, p.T, so, tid);
-    if (tid == 0) {
-      if constexpr (SEG == 64) tma_store_tile<T>(&tm_o, row_base + s * MB, so);
-      else if constexpr (!GATHER) tma_store_pair<T>(&tm_o, stream, s * MB, p.T, so);
-      if (save) tma_store_tile<T>(&tm_g, row_base + s * MB, sg);  // saved tiles are kept in the packed 64-wide form
-      bulk_commit();
-      bulk_wait_read<1>();
-    }
-    // (the next loads by the first thread of warp 1: thread 0 is busy with the stores, and a warp that does both
-    // arrives at the next stage's first barrier that much later than the other three)
-    if (tid == 32 && s + FWD_NST < NS) issue_loads(s + FWD_NST);
-    if constexpr (GATHER)
-      if (s + FWD_NST < NS) issue_gather(s + FWD_NST);
+    fence_proxy_async_smem();  // (stored behind the next stage's first barrier)
     return true;
   };
   // bf16: the stage loop unrolled over the ring slots.  float32: a stage is too long for that, three copies of it leave the
@@ -462,12 +451,13 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
       }
     }
   }
-  if (tid == 0) bulk_wait_all<0>();
-  if constexpr (GATHER) cp_async_wait_all();  // (a stage that gave up may leave gathers in flight)
+  __syncthreads();
+  if (!failed) issue_stores(NS - 1);
+  if (elect_one()) bulk_wait_all<0>();
 }
 
 template <typename T, int SEG, int MB>
-static cudaError_t launch_fwd_t(const CUtensorMap* m, const void* const* io, const LinFwdParams& p, int nstreams,
+static cudaError_t launch_fwd_t(const CUtensorMap* m, const LinFwdParams& p, int nstreams,
                                 cudaStream_t st) {
   using SM = FwdSmem<T, SEG>;
   auto kfn = ttt_linear_fwd_kernel<T, SEG, MB>;
@@ -478,31 +468,25 @@ static cudaError_t launch_fwd_t(const CUtensorMap* m, const void* const* io, con
     return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, *n);
   });
   if (e != cudaSuccess) return e;
-  if constexpr (PairIo<T, SEG>::GATHER) {
-    kfn<<<nstreams, NTHREADS, SM::DYN_BYTES, st>>>(RawTensor{const_cast<void*>(io[0])}, RawTensor{const_cast<void*>(io[1])},
-                                                   RawTensor{const_cast<void*>(io[2])},
-                                                   RawTensor{const_cast<void*>(io[3])}, m[4], p);
-  } else {
-    kfn<<<nstreams, NTHREADS, SM::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], p);
-  }
+  kfn<<<nstreams, NTHREADS, SM::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], p);
   return cudaGetLastError();
 }
 
 template <typename T, int SEG>
-static cudaError_t launch_fwd_mb(int mb, const CUtensorMap* m, const void* const* io, const LinFwdParams& p,
+static cudaError_t launch_fwd_mb(int mb, const CUtensorMap* m, const LinFwdParams& p,
                                  int nstreams, cudaStream_t st) {
-  return mb == 8 ? launch_fwd_t<T, SEG, 8>(m, io, p, nstreams, st) : launch_fwd_t<T, SEG, 16>(m, io, p, nstreams, st);
+  return mb == 8 ? launch_fwd_t<T, SEG, 8>(m, p, nstreams, st) : launch_fwd_t<T, SEG, 16>(m, p, nstreams, st);
 }
 
 // mb: tokens per mini-batch, 16 or 8 (the maps' boxes then have 8 rows)
-cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* maps, const void* const* io,
+cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* maps,
                               const LinFwdParams& p, int nstreams, cudaStream_t st) {
   if (seg == 32) {
-    if (dtype == 1) return launch_fwd_mb<__nv_bfloat16, 32>(mb, maps, io, p, nstreams, st);
-    return launch_fwd_mb<float, 32>(mb, maps, io, p, nstreams, st);
+    if (dtype == 1) return launch_fwd_mb<__nv_bfloat16, 32>(mb, maps, p, nstreams, st);
+    return launch_fwd_mb<float, 32>(mb, maps, p, nstreams, st);
   }
-  if (dtype == 1) return launch_fwd_mb<__nv_bfloat16, 64>(mb, maps, io, p, nstreams, st);
-  return launch_fwd_mb<float, 64>(mb, maps, io, p, nstreams, st);
+  if (dtype == 1) return launch_fwd_mb<__nv_bfloat16, 64>(mb, maps, p, nstreams, st);
+  return launch_fwd_mb<float, 64>(mb, maps, p, nstreams, st);
 }
 
 }  // namespace ttt

@@ -152,7 +152,7 @@ __device__ __forceinline__ void bfrag_from_state(const float (&m)[8][4], int ks,
 // LN + L2 gradient pieces for one slab of Z1 given its row statistics.
 // Outputs x_hat, gy = gamma*x_hat + beta - (v - k), gx = gy*gamma and the per-thread partial row sums of gx, gx*x_hat.
 // gam / bet: the thread's column pairs, index nt.
-template <typename T>
+template <typename T, int SEG>
 __device__ __forceinline__ void ln_l2_pieces(const F2 (&z1)[2][2], const float (&mean)[2], const float (&rstd)[2],
                                              const F2 (&gam)[2], const F2 (&bet)[2], uint32_t tk, uint32_t tv,
                                              const Lane& L, F2 (&xh)[2][2], F2 (&gy)[2][2], F2 (&gx)[2][2],
@@ -163,7 +163,7 @@ __device__ __forceinline__ void ln_l2_pieces(const F2 (&z1)[2][2], const float (
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int row = L.g + 8 * r, col = L.nb + 8 * nt + 2 * L.t;
-      const F2 tg = f2sub(ld_pair<T>(tv, row, col), ld_pair<T>(tk, row, col));
+      const F2 tg = f2sub(ld_io<T, SEG>(tv, row, col), ld_io<T, SEG>(tk, row, col));
       const F2 x = f2mul(f2sub(z1[nt][r], f2(mean[r])), f2(rstd[r]));
       const F2 y = f2fma(gam[nt], x, f2sub(bet[nt], tg));
       const F2 gg = f2mul(y, gam[nt]);
@@ -195,14 +195,14 @@ __device__ __forceinline__ void g_from_pieces(const F2 (&gx)[2][2], const F2 (&x
 // fragments with their sign bits flipped.
 // `khalf`: -1 = all 64 k-columns; 0 / 1 = only k in [0,32) / [32,64) (a 32-wide head's own block when two heads share
 // the tile: the other block of the state stays zero).
-template <int NP>
+template <int NP, int SEG = 64>
 __device__ __forceinline__ void state_update_direct(float (&wt)[8][4], const Pk<NP> (&agt)[4], uint32_t k_planes,
                                                     int lane, int khalf = -1) {
 #pragma unroll
   for (int kp = 0; kp < 4; ++kp) {
     if (khalf >= 0 && (kp >> 1) != khalf) continue;
     Pk<NP> bk[4];
-    ldsm_np<NP>(bk, k_planes + lane_off_B_kn(lane, 16 * kp), TILE_BF16_BYTES, true);
+    ldsm_np<NP>(bk, k_planes + lane_off_io<std::conditional_t<NP == 1, __nv_bfloat16, float>, SEG>(lane, 16 * kp), TILE_BF16_BYTES, true);
     const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]};
     mma_np2<NP>(wt[2 * kp], agt, b0, wt[2 * kp + 1], agt, b1);
   }

@@ -117,56 +117,65 @@ __device__ __forceinline__ void tma_store_tile(const CUtensorMap* tm, int row0, 
   }
 }
 
-// Tile of a PAIR of 32-wide heads (head_dim 32): the two heads' 16 x 32 blocks side by side in one 16 x 64 tile, so
-// that the 64-wide kernels serve two such streams at once.  `pair` = index of the head pair (packed stream), `t0` =
-// first token, `seq` = tokens per sequence; the caller's tensor is [B*H, seq, 32], heads 2 pair and 2 pair + 1.
-//
-// float32: a half tile is 16 rows of 128 bytes, exactly one 128-byte-swizzled TMA box of the 2-D view [B*H*seq, 32].
-// bf16: a half tile is only 64 bytes wide, and a swizzled TMA box row narrower than the swizzle span still occupies a
-// whole 128-byte row of shared memory, so TMA cannot put the two halves side by side.  The tile is gathered instead:
-// 128 chunks of 16 bytes, one cp.async per thread, written at the swizzled position TMA would have used; results leave
-// the same way (ld.shared + st.global per thread).
-// How a kernel is handed one of the caller's [B,H,T,F] tensors: a TMA descriptor, or a plain pointer where the tiles
-// are gathered (the kernel's parameter list is unchanged for every other instantiation).
-struct alignas(64) RawTensor {
-  void* ptr;
-};
+// One of the caller's tiles, as the TTT-Linear kernels hold it.  SEG = 64: the tile above.  SEG = 32: the tiles of a PAIR of
+// 32-wide heads side by side, so that the 64-wide kernels serve two such streams at once: two boxes of 16 rows x 32 columns
+// of the 2-D view [B*H*seq, 32], one per head, the second behind the first.  In float32 a box row is 128 bytes and the pair
+// has the layout of the 64-wide tile (two 128-byte-swizzled halves); in bf16 it is 64 bytes, swizzled over 64 bytes.
 template <typename T, int SEG>
-struct PairIo {
-  static constexpr bool GATHER = (SEG == 32 && sizeof(T) == 2);
-  using Ref = std::conditional_t<GATHER, RawTensor, CUtensorMap>;
-};
-template <int ROWS = 16>  // rows of the tile that exist (a mini-batch of 8 fills the first 8)
-__device__ __forceinline__ void gather_pair_tile_bf16(uint32_t tile, const void* base, int pair, int t0, int seq, int tid) {
-  const int row = tid >> 3, c = tid & 7;  // chunk c of the 128-byte row: head c >> 2, features 8 (c & 3) ..
-  if (ROWS < 16 && row >= ROWS) return;
-  const uint8_t* src = static_cast<const uint8_t*>(base) +
-                       (((size_t)(2 * pair + (c >> 2)) * seq + t0 + row) * 32 + (c & 3) * 8) * 2;
-  cp_async_16(tile + row * 128 + ((c ^ (row & 7)) << 4), src);
+__device__ __forceinline__ uint32_t off_io(int row, int col) {
+  if constexpr (sizeof(T) == 4) return off_f32(row, col);
+  else if constexpr (SEG == 64) return off_bf16(row, col);
+  else return static_cast<uint32_t>(((col >> 5) << 10) + row * 64 + (((((col & 31) >> 3) ^ (row >> 1)) & 3) << 4) + ((col & 7) << 1));
 }
-template <int ROWS = 16>
-__device__ __forceinline__ void scatter_pair_tile_bf16(void* base, int pair, int t0, int seq, uint32_t tile, int tid) {
-  const int row = tid >> 3, c = tid & 7;
-  if (ROWS < 16 && row >= ROWS) return;
-  uint4 v;
-  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(tile + row * 128 + ((c ^ (row & 7)) << 4)));
-  uint8_t* dst = static_cast<uint8_t*>(base) + (((size_t)(2 * pair + (c >> 2)) * seq + t0 + row) * 32 + (c & 3) * 8) * 2;
-  *reinterpret_cast<uint4*>(dst) = v;
+template <typename T, int SEG>
+__device__ __forceinline__ float2 ld_io(uint32_t tile, int row, int col) {
+  const uint32_t a = tile + off_io<T, SEG>(row, col);
+  if constexpr (sizeof(T) == 4) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+  } else {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+    return make_float2(bf16_lo(v), bf16_hi(v));
+  }
 }
-// float32 pair tile by TMA: two boxes of the [B*H*seq, 32] view, one per head.
-template <typename T>
-__device__ __forceinline__ void tma_load_pair(uint32_t tile, const CUtensorMap* tm, int pair, int t0, int seq, uint32_t bar) {
-  static_assert(sizeof(T) == 4, "bf16 pair tiles are gathered, not loaded by TMA");
-  tma_load_2d(tile, tm, 0, (2 * pair) * seq + t0, bar);
-  tma_load_2d(tile + 2048, tm, 0, (2 * pair + 1) * seq + t0, bar);
+template <typename T, int SEG>
+__device__ __forceinline__ void st_io(uint32_t tile, int row, int col, float x, float y) {
+  const uint32_t a = tile + off_io<T, SEG>(row, col);
+  if constexpr (sizeof(T) == 4) asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(a), "f"(x), "f"(y) : "memory");
+  else asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(pack_bf16(x, y)) : "memory");
 }
-template <typename T>
-__device__ __forceinline__ void tma_store_pair(const CUtensorMap* tm, int pair, int t0, int seq, uint32_t tile) {
-  static_assert(sizeof(T) == 4, "bf16 pair tiles are scattered, not stored by TMA");
-  tma_store_2d(tm, 0, (2 * pair) * seq + t0, tile);
-  tma_store_2d(tm, 0, (2 * pair + 1) * seq + t0, tile + 2048);
+// ldmatrix.x4 lane offset into the tile's operand planes, columns kc..kc+15 (lane_off_A, which is also lane_off_B_kn)
+template <typename T, int SEG>
+__device__ __forceinline__ uint32_t lane_off_io(int lane, int kc) {
+  if constexpr (sizeof(T) == 2 && SEG == 32) return off_io<T, SEG>((lane & 7) + (((lane >> 3) & 1) << 3), kc + ((lane >> 4) << 3));
+  else return lane_off_A(lane, kc);
+}
+// `stream` (SEG = 32: pair) and first token of the tile; `seq` tokens per stream
+template <typename T, int SEG>
+__device__ __forceinline__ void tma_load_io(uint32_t tile, const CUtensorMap* tm, int stream, int t0, int seq, uint32_t bar) {
+  if constexpr (SEG == 64) {
+    tma_load_tile<T>(tile, tm, stream * seq + t0, bar);
+  } else {
+    tma_load_2d(tile, tm, 0, (2 * stream) * seq + t0, bar);
+    tma_load_2d(tile + TileFmt<T>::RAW_BYTES / 2, tm, 0, (2 * stream + 1) * seq + t0, bar);
+  }
+}
+template <typename T, int SEG>
+__device__ __forceinline__ void tma_store_io(const CUtensorMap* tm, int stream, int t0, int seq, uint32_t tile) {
+  if constexpr (SEG == 64) {
+    tma_store_tile<T>(tm, stream * seq + t0, tile);
+  } else {
+    tma_store_2d(tm, 0, (2 * stream) * seq + t0, tile);
+    tma_store_2d(tm, 0, (2 * stream + 1) * seq + t0, tile + TileFmt<T>::RAW_BYTES / 2);
+  }
+}
+// Byte `o` of such a tile (operand planes included) belongs to a row that a mini-batch of MB tokens does not fill.
+template <typename T, int SEG, int MB>
+__device__ __forceinline__ bool io_pad(uint32_t o) {
+  constexpr uint32_t BOX = (SEG == 32) ? TileFmt<T>::RAW_BYTES / 2 : 2048, ROW = BOX / CS;
+  return o >= TileFmt<T>::RAW_BYTES || (o % BOX) >= MB * ROW;
 }
 
 }  // namespace ttt
