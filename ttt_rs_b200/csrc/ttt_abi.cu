@@ -1063,7 +1063,6 @@ extern "C" int ttt_layer_epilogue_backward(const ttt_dims* d, const void* grad_y
   p.d_ln_w = grad_post_norm_weight;
   p.d_ln_b = grad_post_norm_bias;
   p.partials = static_cast<float*>(workspace);
-  p.row_stats = nullptr;
   p.B = d->batch;
   p.H = d->heads;
   p.T = d->seq_len;

@@ -210,8 +210,8 @@ struct LayerEpiBwdParams {
   long ld_dgate;
   float* d_ln_w;          // [H*F] float32
   float* d_ln_b;
-  float* partials;        // workspace (float32): [B*T][2] row statistics, then [slabs][2][H*F] partial sums
-  float2* row_stats;      // set by the launcher (start of the workspace)
+  float* partials;        // workspace (float32): [CTAs][2][H*F] partial sums
+  int row_groups;         // set by the launcher: rows of a tile that a CTA's threads work on at once
   int B, H, T;
   float eps;
 };

@@ -550,256 +550,219 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
   }
 }
 
-// Epilogue backward.  Same tiling as the forward kernel: the inner-output tile is fetched into shared memory, each
-// warp takes whole rows, recomputes the row statistics, forms
-//   dn = dy * gelu(g),  dg = dy * n * gelu'(g)   (n = gamma x_hat + beta; without a gate dn = dy),
-//   dz = rstd * (dx - mean(dx) - x_hat * mean(dx * x_hat)),  dx = dn * gamma,
-// writes dz back into the tile (then scattered to [B,H,T,F] per head segment) and leaves (mean, rstd) of every row in
-// `row_stats` for the parameter-gradient kernel below.
-template <typename T, int MAXCH, int FD>
-__global__ void __launch_bounds__(EPI_THREADS, (MAXCH <= 4 ? 2 : 1)) ttt_layer_epilogue_bwd_kernel(const LayerEpiBwdParams p) {
+// Epilogue backward, one pass over the token tiles: with dn = dy * gelu(g) and n = gamma x_hat + beta (without a gate dn = dy)
+//   dg = dy * n * gelu'(g),  dz = rstd * (dx - mean(dx) - x_hat * mean(dx * x_hat)),  dx = dn * gamma,
+//   d weight[c] = sum over tokens of dn * x_hat,  d bias[c] = sum of dn.
+// Bound by memory (dy and the inner output read once, dz written once), so everything happens while a tile of TT tokens is
+// in shared memory, both operands double-buffered with asynchronous copies.  Row phase: a warp per row, two rounds of
+// shuffles (the mean; then the variance and both sums of dx together).  Column phase: a thread per 16-byte chunk of columns
+// and row group, which writes dz straight to [B,H,T,F] and keeps its columns' parameter sums in registers over all of the
+// CTA's tiles; the row groups meet in shared memory at the end and leave one [2][C] row of `partials` per CTA.
+// 65536 tokens x 768, bf16: 187 -> 86 us without a gate, 359 -> 208 us with one; float32 409 -> 104 us (the parameter sums
+// were a kernel of their own that read both operands again).  TT: with a gate (whose row phase is bound by tanh) half, so
+// that the tanh values that the column phase uses again fit beside two CTAs' tiles.
+constexpr int EPI_BWD_THREADS = 384;
+template <typename T, int MAXCH, int FD, bool GATE>
+__global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T) == 2 || MAXCH == 16) ? 2 : 3)
+    ttt_layer_epilogue_bwd_kernel(const LayerEpiBwdParams p) {
   constexpr int HD = FD;  // features per head in this instantiation
-  constexpr int TT = 64 / MAXCH;
+  constexpr int TT = (GATE ? 32 : 64) / MAXCH;
   constexpr int EPC = 16 / sizeof(T);
   constexpr int CPR = HD / EPC;
   extern __shared__ __align__(16) uint8_t epi_smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int H = p.H, NT = p.T, C = H * HD;
+  const int nch = C / EPC, ngroups = p.row_groups;
   const size_t tile_bytes = (size_t)TT * C * sizeof(T);
-  float* gam = reinterpret_cast<float*>(epi_smem + 2 * tile_bytes);
-  float* bet = gam + C;
-  for (int c = tid; c < C; c += EPI_THREADS) {
-    gam[c] = ld_as_float<T>(p.ln_w, (size_t)c);
-    bet[c] = ld_as_float<T>(p.ln_b, (size_t)c);
-  }
+  float4* stat = reinterpret_cast<float4*>(epi_smem + 4 * tile_bytes);  // per row: mean, rstd, mean(dx), mean(dx x_hat)
+  float* gam = reinterpret_cast<float*>(stat + TT);
+  float* th_tile = gam + C;  // with a gate: the row phase's tanh values [TT][C], for the column phase
+  for (int c = tid; c < C; c += blockDim.x) gam[c] = ld_as_float<T>(p.ln_w, (size_t)c);
   const int tiles_per_b = (NT + TT - 1) / TT;
   const long ntiles = (long)p.B * tiles_per_b;
-  const int nch = C / EPC;
-  constexpr int seg = TT * CPR;
+  const int my_ch = tid % nch, my_grp = tid / nch, c_own = my_ch * EPC;
+  const int h_own = c_own / HD, f_own = c_own - h_own * HD;
 
+  // tile `tile_id`: the inner output to buffer `buf`, dy to buffer 2 + buf (both [TT][C])
   auto fetch = [&](long tile_id, int buf) {
     if (tile_id < ntiles) {
-      const int b = (int)(tile_id / tiles_per_b);
-      const int t0 = (int)(tile_id % tiles_per_b) * TT;
+      const int b = (int)(tile_id / tiles_per_b), t0 = (int)(tile_id - (long)b * tiles_per_b) * TT;
       const int rows = min(TT, NT - t0);
-      const uint32_t dst0 = smem_u32(epi_smem + buf * tile_bytes);
-      for (int idx = tid; idx < H * seg; idx += EPI_THREADS) {
-        const int h = idx / seg, i = idx - h * seg, r = i / CPR, cc = i - r * CPR;
-        if (r < rows) {
-          const T* src = static_cast<const T*>(p.inner_out) + (((size_t)b * H + h) * NT + t0) * HD + (size_t)i * EPC;
-          const uint32_t dst = dst0 + (uint32_t)(((size_t)r * C + h * HD + cc * EPC) * sizeof(T));
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+      if (my_grp < ngroups) {
+        const uint32_t dst = smem_u32(epi_smem + buf * tile_bytes) + (uint32_t)(c_own * sizeof(T));
+        const T* z = static_cast<const T*>(p.inner_out) + (((size_t)b * H + h_own) * NT + t0) * HD + f_own;
+        const T* y = static_cast<const T*>(p.dy) + ((size_t)b * NT + t0) * C + c_own;
+        for (int r = my_grp; r < rows; r += ngroups) {
+          const uint32_t d = dst + (uint32_t)(r * C * sizeof(T));
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(z + (size_t)r * HD) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 2 * (uint32_t)tile_bytes), "l"(y + (size_t)r * C)
+                       : "memory");
         }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  auto chunk = [](const void* src, float (&f)[EPC]) {
+    if constexpr (sizeof(T) == 2) {
+      Vec8<T> raw;
+      raw.load(static_cast<const T*>(src));
+      raw.unpack(f);
+    } else {
+      const float4 v = *reinterpret_cast<const float4*>(src);
+      f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+    }
+  };
+  auto gate_chunk = [&](size_t tok, int c0, float (&g)[EPC]) {  // (rows of the gate buffer are aligned to 8 bytes only)
+    const uint2* src = reinterpret_cast<const uint2*>(static_cast<const T*>(p.gate) + tok * p.ld_gate + c0);
+    const uint2 a = src[0], b = src[1];
+    if constexpr (sizeof(T) == 2) {
+      g[0] = bf16_lo(a.x); g[1] = bf16_hi(a.x); g[2] = bf16_lo(a.y); g[3] = bf16_hi(a.y);
+      g[4] = bf16_lo(b.x); g[5] = bf16_hi(b.x); g[6] = bf16_lo(b.y); g[7] = bf16_hi(b.y);
+    } else {
+      g[0] = __uint_as_float(a.x); g[1] = __uint_as_float(a.y); g[2] = __uint_as_float(b.x); g[3] = __uint_as_float(b.y);
+    }
+  };
+  auto gelu_tanh = [](float g) { return tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)); };
 
+  float ag[EPC], ab[EPC], gam_own[EPC], bet_own[EPC];
+#pragma unroll
+  for (int e = 0; e < EPC; ++e) {
+    ag[e] = ab[e] = 0.f;
+    gam_own[e] = ld_as_float<T>(p.ln_w, (size_t)(c_own + e));
+    bet_own[e] = GATE ? ld_as_float<T>(p.ln_b, (size_t)(c_own + e)) : 0.f;
+  }
   int buf = 0;
   fetch(blockIdx.x, 0);
   for (long tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, buf ^= 1) {
-    const int b = (int)(tile_id / tiles_per_b);
-    const int t0 = (int)(tile_id % tiles_per_b) * TT;
+    const int b = (int)(tile_id / tiles_per_b), t0 = (int)(tile_id - (long)b * tiles_per_b) * TT;
     const int rows = min(TT, NT - t0);
     fetch(tile_id + gridDim.x, buf ^ 1);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    T* tile = reinterpret_cast<T*>(epi_smem + buf * tile_bytes);
-    for (int r = warp; r < rows; r += EPI_THREADS / 32) {
-      T* row = tile + (size_t)r * C;
-      const size_t tok = (size_t)b * NT + t0 + r;
-      float v[MAXCH][EPC];
+    const uint8_t* zt = epi_smem + buf * tile_bytes;
+    const uint8_t* yt = zt + 2 * tile_bytes;
+    for (int r = warp; r < rows; r += nwarps) {
+      const T* zr = reinterpret_cast<const T*>(zt) + (size_t)r * C;
+      const T* yr = reinterpret_cast<const T*>(yt) + (size_t)r * C;
       float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < MAXCH; ++j) {
-        const int ch = j * 32 + lane;
-        if (ch < nch) {
-          if constexpr (sizeof(T) == 2) {
-            Vec8<T> raw;
-            raw.load(row + ch * EPC);
-            raw.unpack(v[j]);
-          } else {
-            const float4 f = *reinterpret_cast<const float4*>(row + ch * EPC);
-            v[j][0] = f.x; v[j][1] = f.y; v[j][2] = f.z; v[j][3] = f.w;
-          }
-#pragma unroll
-          for (int e = 0; e < EPC; ++e) s += v[j][e];
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      const float mean = s / C;
-      float q = 0.f;
 #pragma unroll
       for (int j = 0; j < MAXCH; ++j)
         if (j * 32 + lane < nch) {
+          float v[EPC];
+          chunk(zr + (j * 32 + lane) * EPC, v);
 #pragma unroll
-          for (int e = 0; e < EPC; ++e) {
-            v[j][e] -= mean;
-            q = fmaf(v[j][e], v[j][e], q);
-          }
+          for (int e = 0; e < EPC; ++e) s += v[e];
         }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-      const float rstd = 1.f / sqrtf(q / C + p.eps);
-      if (lane == 0) p.row_stats[tok] = make_float2(mean, rstd);
-      // pass 1: x_hat, dn (and dg), dx = dn * gamma and its two row sums
-      float dxv[MAXCH][EPC];
-      float m1 = 0.f, m2 = 0.f;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const float mean = s / C;
+      float q = 0.f, m1 = 0.f, m2 = 0.f;
 #pragma unroll
-      for (int j = 0; j < MAXCH; ++j) {
-        const int ch = j * 32 + lane;
-        if (ch < nch) {
-          const int c0 = ch * EPC;
-          float dy[EPC];
-          const T* dyp = static_cast<const T*>(p.dy) + tok * C + c0;
-          if constexpr (sizeof(T) == 2) {
-            Vec8<T> raw;
-            raw.load(dyp);
-            raw.unpack(dy);
-          } else {
-            const float4 f = *reinterpret_cast<const float4*>(dyp);
-            dy[0] = f.x; dy[1] = f.y; dy[2] = f.z; dy[3] = f.w;
-          }
-          float gt[EPC], dg[EPC];
-          if (p.gate != nullptr) {
-            const T* gp = static_cast<const T*>(p.gate) + tok * p.ld_gate + c0;
-            if constexpr (sizeof(T) == 2) {
-              const uint2 g0 = reinterpret_cast<const uint2*>(gp)[0], g1 = reinterpret_cast<const uint2*>(gp)[1];
-              gt[0] = bf16_lo(g0.x); gt[1] = bf16_hi(g0.x); gt[2] = bf16_lo(g0.y); gt[3] = bf16_hi(g0.y);
-              gt[4] = bf16_lo(g1.x); gt[5] = bf16_hi(g1.x); gt[6] = bf16_lo(g1.y); gt[7] = bf16_hi(g1.y);
-            } else {
-              const float2 g0 = reinterpret_cast<const float2*>(gp)[0], g1 = reinterpret_cast<const float2*>(gp)[1];
-              gt[0] = g0.x; gt[1] = g0.y; gt[2] = g1.x; gt[3] = g1.y;
-            }
+      for (int j = 0; j < MAXCH; ++j)
+        if (j * 32 + lane < nch) {
+          const int c0 = (j * 32 + lane) * EPC;
+          float v[EPC], dn[EPC], g[EPC];
+          chunk(zr + c0, v);
+          chunk(yr + c0, dn);
+          float th[EPC];
+          if constexpr (GATE) {
+            gate_chunk((size_t)b * NT + t0 + r, c0, g);
+#pragma unroll
+            for (int e = 0; e < EPC; ++e) th[e] = gelu_tanh(g[e]);
+#pragma unroll
+            for (int e = 0; e < EPC; e += 4)
+              *reinterpret_cast<float4*>(&th_tile[(size_t)r * C + c0 + e]) = make_float4(th[e], th[e + 1], th[e + 2], th[e + 3]);
           }
 #pragma unroll
           for (int e = 0; e < EPC; ++e) {
-            const float xh = v[j][e] * rstd;
-            float dn = dy[e];
-            if (p.gate != nullptr) {
-              const float g = gt[e], g2 = g * g;
-              const float u = 0.7978845608028654f * (g + 0.044715f * g * g2);
-              const float th = tanhf(u);
-              const float gelu = 0.5f * g * (1.f + th);
-              const float dgelu = 0.5f * (1.f + th) + 0.5f * g * (1.f - th * th) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * g2);
-              dg[e] = dy[e] * (gam[c0 + e] * xh + bet[c0 + e]) * dgelu;
-              dn = dy[e] * gelu;
-            }
-            const float dx = dn * gam[c0 + e];
-            dxv[j][e] = dx;
+            if constexpr (GATE) dn[e] *= 0.5f * g[e] * (1.f + th[e]);
+            const float x = v[e] - mean, dx = dn[e] * gam[c0 + e];
+            q = fmaf(x, x, q);
             m1 += dx;
-            m2 = fmaf(dx, xh, m2);
-          }
-          if (p.gate != nullptr) {
-            T* dgp = static_cast<T*>(p.dgate) + tok * p.ld_dgate + c0;
-            if constexpr (sizeof(T) == 2) {
-              uint2 o0, o1;
-              o0.x = pack_bf16(dg[0], dg[1]); o0.y = pack_bf16(dg[2], dg[3]);
-              o1.x = pack_bf16(dg[4], dg[5]); o1.y = pack_bf16(dg[6], dg[7]);
-              reinterpret_cast<uint2*>(dgp)[0] = o0;
-              reinterpret_cast<uint2*>(dgp)[1] = o1;
-            } else {
-              reinterpret_cast<float2*>(dgp)[0] = make_float2(dg[0], dg[1]);
-              reinterpret_cast<float2*>(dgp)[1] = make_float2(dg[2], dg[3]);
-            }
+            m2 = fmaf(dx, x, m2);
           }
         }
-      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
+        q += __shfl_xor_sync(0xffffffffu, q, o);
         m1 += __shfl_xor_sync(0xffffffffu, m1, o);
         m2 += __shfl_xor_sync(0xffffffffu, m2, o);
       }
-      m1 /= C;
-      m2 /= C;
-      // pass 2: dz back into the tile, in place
+      const float rstd = 1.f / sqrtf(q / C + p.eps);
+      if (lane == 0) stat[r] = make_float4(mean, rstd, m1 / C, m2 * rstd / C);
+    }
+    __syncthreads();
+    if (my_grp < ngroups) {
+      T* out = static_cast<T*>(p.d_inner) + (((size_t)b * H + h_own) * NT + t0) * HD + f_own;
+      for (int r = my_grp; r < rows; r += ngroups) {
+        const float4 st = stat[r];
+        const size_t tok = (size_t)b * NT + t0 + r;
+        float z[EPC], dn[EPC];
+        chunk(reinterpret_cast<const T*>(zt) + (size_t)r * C + c_own, z);
+        chunk(reinterpret_cast<const T*>(yt) + (size_t)r * C + c_own, dn);
+        if constexpr (GATE) {
+          float g[EPC], dg[EPC];
+          gate_chunk(tok, c_own, g);
+          float th[EPC];
 #pragma unroll
-      for (int j = 0; j < MAXCH; ++j) {
-        const int ch = j * 32 + lane;
-        if (ch < nch) {
-          float dz[EPC];
+          for (int e = 0; e < EPC; e += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(&th_tile[(size_t)r * C + c_own + e]);
+            th[e] = v.x; th[e + 1] = v.y; th[e + 2] = v.z; th[e + 3] = v.w;
+          }
 #pragma unroll
-          for (int e = 0; e < EPC; ++e) dz[e] = rstd * (dxv[j][e] - m1 - v[j][e] * rstd * m2);
+          for (int e = 0; e < EPC; ++e) {
+            const float g2 = g[e] * g[e];
+            const float dgelu = 0.5f * (1.f + th[e]) + 0.5f * g[e] * (1.f - th[e] * th[e]) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * g2);
+            dg[e] = dn[e] * (gam_own[e] * ((z[e] - st.x) * st.y) + bet_own[e]) * dgelu;
+            dn[e] *= 0.5f * g[e] * (1.f + th[e]);
+          }
+          uint2* dst = reinterpret_cast<uint2*>(static_cast<T*>(p.dgate) + tok * p.ld_dgate + c_own);
           if constexpr (sizeof(T) == 2) {
-            Vec8<T> o;
-            o.pack(dz);
-            o.store(row + ch * EPC);
+            dst[0] = make_uint2(pack_bf16(dg[0], dg[1]), pack_bf16(dg[2], dg[3]));
+            dst[1] = make_uint2(pack_bf16(dg[4], dg[5]), pack_bf16(dg[6], dg[7]));
           } else {
-            *reinterpret_cast<float4*>(row + ch * EPC) = make_float4(dz[0], dz[1], dz[2], dz[3]);
+            dst[0] = make_uint2(__float_as_uint(dg[0]), __float_as_uint(dg[1]));
+            dst[1] = make_uint2(__float_as_uint(dg[2]), __float_as_uint(dg[3]));
           }
         }
-      }
-    }
-    __syncthreads();  // the tile now holds dz for every row
-    for (int idx = tid; idx < H * seg; idx += EPI_THREADS) {
-      const int h = idx / seg, i = idx - h * seg, r = i / CPR, cc = i - r * CPR;
-      if (r < rows) {
-        T* dst = static_cast<T*>(p.d_inner) + (((size_t)b * H + h) * NT + t0) * HD + (size_t)i * EPC;
-        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(tile + (size_t)r * C + h * HD + cc * EPC);
+#pragma unroll
+        for (int e = 0; e < EPC; ++e) {
+          const float xh = (z[e] - st.x) * st.y;
+          ag[e] = fmaf(dn[e], xh, ag[e]);
+          ab[e] += dn[e];
+          z[e] = st.y * (dn[e] * gam_own[e] - st.z - xh * st.w);
+        }
+        if constexpr (sizeof(T) == 2) {
+          Vec8<T> o;
+          o.pack(z);
+          o.store(out + (size_t)r * HD);
+        } else {
+          *reinterpret_cast<float4*>(out + (size_t)r * HD) = make_float4(z[0], z[1], z[2], z[3]);
+        }
       }
     }
     __syncthreads();  // done with this buffer before the next iteration refills it
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-
-}
-
-// Parameter gradients of the post norm: d weight[c] = sum over tokens of dn * x_hat, d bias[c] = sum of dn.  One CTA
-// per slab of PARAM_SLAB tokens, one thread per column pair, rows walked in order; the slab's sums go to `partials`.
-constexpr int PARAM_SLAB = 128;
-template <typename T, int FD>
-__global__ void ttt_layer_epilogue_bwd_param_kernel(const LayerEpiBwdParams p) {
-  constexpr int HD = FD;  // features per head in this instantiation
-  const int H = p.H, NT = p.T, C = H * HD;
-  const int pair = threadIdx.x;          // columns 2*pair, 2*pair+1
-  const int c = 2 * pair, h = c / HD, f = c % HD;
-  const long ntok = (long)p.B * NT;
-  const long row0 = (long)blockIdx.x * PARAM_SLAB;
-  const long row1 = row0 + PARAM_SLAB < ntok ? row0 + PARAM_SLAB : ntok;
-  auto ld2 = [](const void* base, size_t idx) -> float2 {
-    if constexpr (sizeof(T) == 2) {
-      const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const T*>(base) + idx);
-      return make_float2(bf16_lo(w), bf16_hi(w));
-    } else {
-      return *reinterpret_cast<const float2*>(static_cast<const T*>(base) + idx);
-    }
-  };
-  float2 ag = make_float2(0.f, 0.f), ab = make_float2(0.f, 0.f);
-  int t = (int)(row0 % NT), b = (int)(row0 / NT);
-  size_t zoff = (((size_t)b * H + h) * NT + t) * HD + f;  // advances by one row per token, re-based at a batch boundary
-  size_t doff = (size_t)row0 * C + c, goff = (size_t)row0 * p.ld_gate + c;
-#pragma unroll 4
-  for (long tok = row0; tok < row1; ++tok) {
-    const float2 st = p.row_stats[tok];
-    const float2 z = ld2(p.inner_out, zoff);
-    float2 dn = ld2(p.dy, doff);
-    if (p.gate != nullptr) {
-      const float2 g = ld2(p.gate, goff);
-      const float u0 = 0.7978845608028654f * (g.x + 0.044715f * g.x * g.x * g.x);
-      const float u1 = 0.7978845608028654f * (g.y + 0.044715f * g.y * g.y * g.y);
-      dn.x *= 0.5f * g.x * (1.f + tanhf(u0));
-      dn.y *= 0.5f * g.y * (1.f + tanhf(u1));
-    }
-    ag.x = fmaf(dn.x, (z.x - st.x) * st.y, ag.x);
-    ag.y = fmaf(dn.y, (z.y - st.x) * st.y, ag.y);
-    ab.x += dn.x;
-    ab.y += dn.y;
-    doff += C;
-    goff += p.ld_gate;
-    zoff += HD;
-    if (++t == NT) {
-      t = 0;
-      ++b;
-      zoff = ((size_t)b * H + h) * NT * HD + f;
+  __syncthreads();
+  // row groups to shared memory ([group][2][C] float32, over the tile buffers), summed in group order
+  float* red = reinterpret_cast<float*>(epi_smem);
+  if (my_grp < ngroups) {
+#pragma unroll
+    for (int e = 0; e < EPC; ++e) {
+      red[(size_t)my_grp * 2 * C + c_own + e] = ag[e];
+      red[(size_t)my_grp * 2 * C + C + c_own + e] = ab[e];
     }
   }
-  float* out = p.partials + (size_t)blockIdx.x * 2 * C;
-  *reinterpret_cast<float2*>(out + c) = ag;
-  *reinterpret_cast<float2*>(out + C + c) = ab;
+  __syncthreads();
+  for (int c = tid; c < 2 * C; c += blockDim.x) {
+    float sum = red[c];
+    for (int g = 1; g < ngroups; ++g) sum += red[(size_t)g * 2 * C + c];
+    p.partials[(size_t)blockIdx.x * 2 * C + c] = sum;
+  }
 }
 
-// d post_norm_weight / d post_norm_bias: the slabs' partial rows added in a fixed order.  A CTA owns 32 columns;
+// d post_norm_weight / d post_norm_bias: the CTAs' partial rows added in a fixed order.  A CTA owns 32 columns;
 // its 8 warps each add an interleaved eighth of the parts (lanes = columns, so every load is one coalesced 128-byte
 // row segment), and the eight sums are combined in warp order through shared memory.
 __global__ void __launch_bounds__(256) ttt_layer_epilogue_bwd_reduce_kernel(const float* partials, int nparts, int C,
@@ -836,42 +799,45 @@ cudaError_t launch_layer_prologue_bwd(int dtype, int head_dim, const LayerProBwd
   return cudaGetLastError();
 }
 
+// CTAs of the epilogue backward, at most: each leaves one row of partial sums
+constexpr int EPI_BWD_MAX_CTAS = 148 * 4;
 size_t layer_epilogue_bwd_workspace_bytes(int B, int H, int T, int head_dim) {
-  const size_t ntok = (size_t)B * T, nslab = (ntok + PARAM_SLAB - 1) / PARAM_SLAB;
-  return ntok * sizeof(float2) + nslab * 2 * (size_t)H * head_dim * sizeof(float);
+  const size_t ntok = (size_t)B * T;  // (a tile holds at least one token)
+  return (ntok < EPI_BWD_MAX_CTAS ? ntok : EPI_BWD_MAX_CTAS) * 2 * (size_t)H * head_dim * sizeof(float);
 }
 
-template <typename T, int MAXCH, int FD>
-static cudaError_t launch_epi_bwd_t(LayerEpiBwdParams p, cudaStream_t st) {
-  const int C = p.H * FD;
-  constexpr int TT = 64 / MAXCH;
-  const size_t smem = 2 * (size_t)TT * C * sizeof(T) + 2 * (size_t)C * sizeof(float);
-  auto kfn = ttt_layer_epilogue_bwd_kernel<T, MAXCH, FD>;
+template <typename T, int MAXCH, int FD, bool GATE>
+static cudaError_t launch_epi_bwd_g(LayerEpiBwdParams p, cudaStream_t st) {
+  const int C = p.H * FD, nch = C / (16 / (int)sizeof(T));
+  constexpr int TT = (GATE ? 32 : 64) / MAXCH, MAXT = MAXCH == 16 ? 512 : EPI_BWD_THREADS;
+  auto kfn = ttt_layer_epilogue_bwd_kernel<T, MAXCH, FD, GATE>;
+  // as many row groups as fit a CTA, but no more than a tile has rows
+  p.row_groups = MAXT / nch < TT ? MAXT / nch : TT;
+  const int threads = (p.row_groups * nch + 31) & ~31;
+  const size_t smem = 4 * (size_t)TT * C * sizeof(T) + TT * sizeof(float4) + (size_t)(GATE ? TT + 1 : 1) * C * sizeof(float);
   static DeviceValue resident;
   int per_sm = 1;
   cudaError_t e = resident.get((uint32_t)C, &per_sm, [&](int* n) {
     constexpr int CMAX = 512 * MAXCH / (int)sizeof(T);  // the widest row of this instantiation
     const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               2 * TT * CMAX * (int)sizeof(T) + 2 * CMAX * (int)sizeof(float));
-    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, EPI_THREADS, smem);
+                                               4 * TT * CMAX * (int)sizeof(T) + TT * 16 + (GATE ? TT + 1 : 1) * CMAX * 4);
+    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, threads, smem);
   });
   if (e != cudaSuccess) return e;
   const long ntiles = (long)p.B * ((p.T + TT - 1) / TT);
-  if (per_sm > 2) per_sm = 2;
-  const long cap = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
-  const int grid = (int)(ntiles < cap ? ntiles : cap);
-  kfn<<<grid < 1 ? 1 : grid, EPI_THREADS, smem, st>>>(p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const long ntok = (long)p.B * p.T;
-  const int nslab = (int)((ntok + PARAM_SLAB - 1) / PARAM_SLAB);
-  ttt_layer_epilogue_bwd_param_kernel<T, FD><<<nslab, C / 2, 0, st>>>(p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  ttt_layer_epilogue_bwd_reduce_kernel<<<(2 * C + 31) / 32, 256, 0, st>>>(p.partials, nslab, C, p.d_ln_w, p.d_ln_b);
+  long grid = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
+  if (grid > EPI_BWD_MAX_CTAS) grid = EPI_BWD_MAX_CTAS;
+  if (grid > ntiles) grid = ntiles;
+  kfn<<<(int)grid, threads, smem, st>>>(p);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  ttt_layer_epilogue_bwd_reduce_kernel<<<(2 * C + 31) / 32, 256, 0, st>>>(p.partials, (int)grid, C, p.d_ln_w, p.d_ln_b);
   return cudaGetLastError();
 }
 
+template <typename T, int MAXCH, int FD>
+static cudaError_t launch_epi_bwd_t(const LayerEpiBwdParams& p, cudaStream_t st) {
+  return p.gate != nullptr ? launch_epi_bwd_g<T, MAXCH, FD, true>(p, st) : launch_epi_bwd_g<T, MAXCH, FD, false>(p, st);
+}
 template <int FD>
 static cudaError_t launch_epi_bwd_f(int dtype, const LayerEpiBwdParams& p, cudaStream_t st) {
   const int C = p.H * FD;
@@ -880,11 +846,7 @@ static cudaError_t launch_epi_bwd_f(int dtype, const LayerEpiBwdParams& p, cudaS
   return C <= 1024 ? launch_epi_bwd_t<float, 8, FD>(p, st) : launch_epi_bwd_t<float, 16, FD>(p, st);
 }
 
-cudaError_t launch_layer_epilogue_bwd(int dtype, int head_dim, const LayerEpiBwdParams& p0, cudaStream_t st) {
-  // workspace: (mean, rstd) per token, then the slabs' partial parameter gradients
-  LayerEpiBwdParams p = p0;
-  p.row_stats = reinterpret_cast<float2*>(p0.partials);
-  p.partials = p0.partials + 2 * (size_t)p0.B * p0.T;
+cudaError_t launch_layer_epilogue_bwd(int dtype, int head_dim, const LayerEpiBwdParams& p, cudaStream_t st) {
   return head_dim == 32 ? launch_epi_bwd_f<32>(dtype, p, st) : launch_epi_bwd_f<64>(dtype, p, st);
 }
 
