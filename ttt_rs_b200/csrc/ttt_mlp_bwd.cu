@@ -294,7 +294,8 @@ __device__ __forceinline__ void tile_mma(const MC C, const float alpha, EPI epi,
   for (int tile0 = warp; tile0 < total; tile0 += NW * TG) {
     int i0[TG], j0[TG];
     bool on[TG];
-    float acc[TG][4];
+    constexpr int NC = TG == 1 ? 2 : 1;  // a lone output tile: two accumulators take turns, halving the chain of products
+    float acc[TG * NC][4];
     float2 cin[TG][2];
 #pragma unroll
     for (int u = 0; u < TG; ++u) {
@@ -304,7 +305,7 @@ __device__ __forceinline__ void tile_mma(const MC C, const float alpha, EPI epi,
       i0[u] = 16 * mt;
       j0[u] = 8 * (tl - mt * ntn);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[u][q] = 0.f;
+      for (int q = 0; q < 4; ++q) acc[u][q] = acc[u + (NC - 1) * TG][q] = 0.f;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         cin[u][h] = make_float2(0.f, 0.f);
@@ -316,8 +317,11 @@ __device__ __forceinline__ void tile_mma(const MC C, const float alpha, EPI epi,
       typedef typename std::remove_cv<typename std::remove_reference<decltype(P)>::type>::type PT;
       constexpr int K = PT::K;
       // operands in the workspace: the whole contraction unrolled, so that the loads of all steps are in flight
+      // (shared-memory operands: four steps; at 48 to 192 streams that and the second accumulator of a lone tile take 2.7 %
+      // off the kernel, 946 -> 918 us at 192 streams of 32 stages; more steps, or the operands of two tiles or steps by one
+      // ldmatrix.x4, give nothing)
       constexpr bool GLOBAL = is_global_operand<decltype(PT::A)>::value || is_global_operand<decltype(PT::B)>::value;
-#pragma unroll(GLOBAL ? 16 : (K >= 64 ? 2 : 1))
+#pragma unroll(GLOBAL ? 16 : (K >= 64 ? 4 : 1))
       for (int k0 = 0; k0 < K; k0 += 16) {
         uint32_t pa[NA][4], pb[NB][2];
 #pragma unroll
@@ -329,11 +333,14 @@ __device__ __forceinline__ void tile_mma(const MC C, const float alpha, EPI epi,
         for (int u = 0; u < TG; ++u) {
           const uint32_t(&a)[4] = pa[u / GA];
           const uint32_t(&b_)[2] = pb[SHARE_B ? 0 : u];
-          mma_bf16(acc[u], a[0], a[1], a[2], a[3], b_[0], b_[1]);
+          mma_bf16(acc[NC == 2 && (k0 & 16) ? u + TG : u], a[0], a[1], a[2], a[3], b_[0], b_[1]);
         }
       }
     };
     (run(pr), ...);
+    if constexpr (NC == 2)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[0][q] += acc[1][q];
 #pragma unroll
     for (int u = 0; u < TG; ++u)
       if (on[u]) {
