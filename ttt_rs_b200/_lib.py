@@ -79,6 +79,12 @@ SYMBOLS = {
     "ttt_layer_qk_conv_backward_workspace_bytes": (C.c_size_t, [_DP]),
     "ttt_layer_qk_conv_backward": (C.c_int, [_DP, _P, _P, _P, C.c_int64, _P, _P, _P, _P, _P, _P, C.c_size_t, _P]),
 }
+# entry points of this package alone (csrc/ttt_internal.h)
+INTERNAL = {
+    "ttt_internal_layer_projections": (C.c_int, [_DP, _P, C.c_int64, C.c_int64, _P, C.c_int64, C.c_int64, C.c_int64,
+                                                 C.c_int64, C.c_int64, C.c_int64, C.c_int64, _P, C.c_int, C.c_int,
+                                                 C.c_float, C.c_float, C.c_int, _P, _P, _P, _P, _P, _P, _P]),
+}
 
 NOALLOC_SCRATCH_BYTES = 32 << 20  # TTT_NOALLOC_SCRATCH_BYTES
 
@@ -94,7 +100,7 @@ def load() -> C.CDLL:
                 f"{LIB_PATH} is missing: build it with `python -m ttt_rs_b200.build` "
                 "(nvcc, sm_100a). There is no CPU or PyTorch fallback for this operator.")
         lib = C.CDLL(str(LIB_PATH))
-        for name, (res, args) in SYMBOLS.items():
+        for name, (res, args) in {**SYMBOLS, **INTERNAL}.items():
             fn = getattr(lib, name)
             fn.restype = res
             fn.argtypes = args

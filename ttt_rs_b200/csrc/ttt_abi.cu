@@ -281,11 +281,11 @@ int ttt_gemm_bf16_tn(int64_t m, int64_t n, int64_t k, const void* a, int64_t lda
   return TTT_OK;
 }
 
-int ttt_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_t hidden, const void* weights,
-                          int64_t w_ld, int64_t w_rows, int64_t q_col, int64_t k_col, int64_t v_col, int64_t g_col,
-                          int64_t lr_col, const void* lr_bias, int start_idx, int rope_mode, float rope_theta,
-                          float base_lr, void* xq, void* xk, void* xv, void* gate, void* ttt_lr_eta, void* status,
-                          void* stream) {
+int ttt_internal_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_t hidden, const void* weights,
+                                   int64_t w_ld, int64_t w_rows, int64_t q_col, int64_t k_col, int64_t v_col, int64_t g_col,
+                                   int64_t lr_col, const void* lr_bias, int start_idx, int rope_mode, float rope_theta,
+                                   float base_lr, int round_proj, void* xq, void* xk, void* xv, void* gate,
+                                   void* ttt_lr_eta, void* status, void* stream) {
   if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
   if (d->batch <= 0 || d->heads <= 0 || d->seq_len <= 0) return fail(TTT_ERR_SHAPE, "batch, heads, seq_len must be positive");
   if (d->dtype != TTT_BF16 || d->head_dim != 64)
@@ -338,10 +338,19 @@ int ttt_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_
   p.f.H = d->heads; p.f.T = d->seq_len;
   p.f.start_idx = start_idx; p.f.pos_mod = rope_mode == 1 ? d->mini_batch : 1; p.f.rope_mode = rope_mode;
   p.f.rope_theta = rope_mode == 1 ? rope_theta : 1.f; p.f.base_lr = base_lr;
-  p.f.lr_bias = lr_bias; p.f.lr_out = ttt_lr_eta;
+  p.f.lr_bias = lr_bias; p.f.lr_out = ttt_lr_eta; p.f.round_proj = round_proj;
   cudaError_t e = ttt::launch_gemm_bf16_tn(maps, p, true, pair, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "fused projection launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
+}
+int ttt_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_t hidden, const void* weights,
+                          int64_t w_ld, int64_t w_rows, int64_t q_col, int64_t k_col, int64_t v_col, int64_t g_col,
+                          int64_t lr_col, const void* lr_bias, int start_idx, int rope_mode, float rope_theta,
+                          float base_lr, void* xq, void* xk, void* xv, void* gate, void* ttt_lr_eta, void* status,
+                          void* stream) {
+  return ttt_internal_layer_projections(d, x, x_ld, hidden, weights, w_ld, w_rows, q_col, k_col, v_col, g_col, lr_col,
+                                        lr_bias, start_idx, rope_mode, rope_theta, base_lr, 0, xq, xk, xv, gate, ttt_lr_eta,
+                                        status, stream);
 }
 
 void ttt_b200_debug_handoff(uint32_t poll_limit, int32_t first_item) {

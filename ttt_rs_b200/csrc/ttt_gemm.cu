@@ -453,6 +453,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             uint32_t r[32];
             tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + buf * GEMM_BN + 32 * c, r);
             if (FUSED) {
+              if (p.f.round_proj && kd != 2) {  // (v is rounded once either way)
+#pragma unroll
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__bfloat162float(__float2bfloat16_rn(__uint_as_float(r[i]))));
+              }
               if (kd == 4) {
                 // learning-rate logits: column i of this group is head i
 #pragma unroll

@@ -46,6 +46,13 @@ int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src, const void
                                 const void* conv_k_bias, int conv_kernel, int start_idx, int rope_mode,
                                 float rope_theta, float base_lr, void* xq, void* xk, void* xv, void* ttt_lr_eta,
                                 int lr_pitch, void* stream);
+// ttt_layer_projections; round_proj: the projections are rounded to bf16 before the rotation and the learning-rate gate, as
+// they are when a product and ttt_layer_prologue compute them one after the other (training).
+int ttt_internal_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_t hidden, const void* weights,
+                                   int64_t w_ld, int64_t w_rows, int64_t q_col, int64_t k_col, int64_t v_col, int64_t g_col,
+                                   int64_t lr_col, const void* lr_bias, int start_idx, int rope_mode, float rope_theta,
+                                   float base_lr, int round_proj, void* xq, void* xk, void* xv, void* gate,
+                                   void* ttt_lr_eta, void* status, void* stream);
 // Few-token forms (bf16): projections with the prologue, and post norm (+ gate) with the output projection; 0 from
 // _fits: not for this shape.  weights: q | k | v | (gate) blocks of heads * head_dim rows, learning-rate rows from lr_col.
 int ttt_internal_layer_small_fits(const ttt_dims* d);

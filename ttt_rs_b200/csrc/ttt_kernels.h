@@ -336,6 +336,7 @@ struct GemmFuse {
   int q_col, k_col, v_col, g_col, lr_col;
   int H, T;                 // heads, tokens per sequence (T % 128 == 0)
   int start_idx, pos_mod, rope_mode;  // rope_mode 0 none, 1 positions (start_idx + t) mod pos_mod, pos_mod <= 16
+  int round_proj;  // round the projections to bf16 first, as a product followed by the prologue would (training)
   float rope_theta, base_lr;
   const void* lr_bias;      // [H] bf16 or null
   void* lr_out;             // ttt_lr_eta [B,H,T] bf16

@@ -147,11 +147,12 @@ def gemm_bf16_tn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 
 
 def layer_projections(x: torch.Tensor, wcat: torch.Tensor, cols, cfg: TTTLayerConfig, lr_bias: Optional[torch.Tensor],
-                      start_idx: int = 0):
+                      start_idx: int = 0, round_proj: bool = False):
     """All projections of the layer plus the prologue in ONE launch (`ttt_layer_projections`: the tcgen05 GEMM with the
     head split, rotary rotation and learning-rate gate in its epilogue).  x [B, T, hidden] bf16, wcat the stacked
     q | k | v | (g) | lr weight rows with their starts in `cols`.  Returns xq, xk, xv [B,H,T,F], ttt_lr_eta [B,H,T] and
-    the gate buffer [B*T, H*F] (None without a gate)."""
+    the gate buffer [B*T, H*F] (None without a gate).  `round_proj`: the projections rounded to bf16 before the rotation
+    and the gate, the values a separate product and prologue would give (training)."""
     from .fused import device_status
     lib = _lib.load()
     B, T, hidden = x.shape
@@ -167,10 +168,11 @@ def layer_projections(x: torch.Tensor, wcat: torch.Tensor, cols, cfg: TTTLayerCo
     bias = None if lr_bias is None else lr_bias.detach().reshape(-1).to(x.dtype).contiguous()
     stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
     with torch.cuda.device(dev):
-        _lib.check(lib.ttt_layer_projections(
+        _lib.check(lib.ttt_internal_layer_projections(
             C.byref(d), _ptr(x2), x2.stride(0), hidden, _ptr(wcat), wcat.stride(0), wcat.shape[0], cols["q"], cols["k"],
             cols["v"], cols.get("g", -1), cols["lr"], _ptr(bias), start_idx, _POS[cfg.pos_encoding], cfg.rope_theta,
-            cfg.base_lr, _ptr(xq), _ptr(xk), _ptr(xv), _ptr(gate), _ptr(lr), _ptr(device_status(dev)), stream))
+            cfg.base_lr, int(round_proj), _ptr(xq), _ptr(xk), _ptr(xv), _ptr(gate), _ptr(lr), _ptr(device_status(dev)),
+            stream))
     return xq, xk, xv, lr, gate
 
 
@@ -189,24 +191,65 @@ class _PrologueFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dxq, dxk, dxv, dlr):
         (lr,) = ctx.saved_tensors
-        cfg, cols, start_idx, (B, T, N) = ctx.meta
-        lib = _lib.load()
-        H, F = cfg.num_heads, cfg.head_dim
-        dt = lr.dtype
-        esz = lr.element_size()
-        dproj = torch.empty(B, T, N, dtype=dt, device=lr.device)
-        d = TttDims(B, H, T, F, cfg.mini_batch_size, 1, 0.0, _dtype_code(dt))
-        base = dproj.data_ptr()
-        col = lambda c: C.c_void_p(base + c * esz)  # noqa: E731
-        stream = C.c_void_p(torch.cuda.current_stream(lr.device).cuda_stream)
-        dxq, dxk, dxv, dlr = (t.contiguous() for t in (dxq, dxk, dxv, dlr))  # named: copies must outlive the launch
-        with torch.cuda.device(lr.device):
-            _lib.check(lib.ttt_layer_prologue_backward(
-                C.byref(d), _ptr(dxq), _ptr(dxk), _ptr(dxv),
-                _ptr(dlr), _ptr(lr), start_idx, _POS[cfg.pos_encoding], cfg.rope_theta, cfg.base_lr,
-                col(cols["q"]), col(cols["k"]), col(cols["v"]), N, col(cols["lr"]), N, N - cols["lr"], stream))
-        dbias = dproj[..., cols["lr"]:cols["lr"] + H].float().sum(dim=(0, 1)).to(dt).reshape(H, 1)
+        cfg, cols, start_idx, shape = ctx.meta
+        dproj = torch.empty(shape, dtype=lr.dtype, device=lr.device)
+        dbias = _prologue_backward(dproj, cols, cfg, start_idx, lr, dxq, dxk, dxv, dlr)
         return dproj, dbias, None, None, None
+
+
+def _prologue_backward(dproj, cols, cfg, start_idx, lr, dxq, dxk, dxv, dlr):
+    """Gradients of the inner-loop inputs -> the q, k, v and lr-logit columns (and the padding behind them) of `dproj`
+    [B, T, N]; returns the gradient of the lr bias [H, 1]."""
+    lib = _lib.load()
+    B, T, N = dproj.shape
+    H, F = cfg.num_heads, cfg.head_dim
+    dt = lr.dtype
+    esz = lr.element_size()
+    d = TttDims(B, H, T, F, cfg.mini_batch_size, 1, 0.0, _dtype_code(dt))
+    base = dproj.data_ptr()
+    col = lambda c: C.c_void_p(base + c * esz)  # noqa: E731
+    stream = C.c_void_p(torch.cuda.current_stream(lr.device).cuda_stream)
+    dxq, dxk, dxv, dlr = (t.contiguous() for t in (dxq, dxk, dxv, dlr))  # named: copies must outlive the launch
+    with torch.cuda.device(lr.device):
+        _lib.check(lib.ttt_layer_prologue_backward(
+            C.byref(d), _ptr(dxq), _ptr(dxk), _ptr(dxv),
+            _ptr(dlr), _ptr(lr), start_idx, _POS[cfg.pos_encoding], cfg.rope_theta, cfg.base_lr,
+            col(cols["q"]), col(cols["k"]), col(cols["v"]), N, col(cols["lr"]), N, N - cols["lr"], stream))
+    return dproj[..., cols["lr"]:cols["lr"] + H].sum(dim=(0, 1), dtype=torch.float32).to(dt).reshape(H, 1)
+
+
+class _ProjectionsFn(torch.autograd.Function):
+    """`layer_projections` with its gradients.  The column gradients of every projection are one [B, T, N] buffer, so the
+    weights' and the input's gradients are one product each; the gate's columns of it are written by the epilogue's
+    gradient kernel (`grads` hands the buffer over; see `_EpilogueFn`)."""
+
+    @staticmethod
+    def forward(ctx, x, q, k, v, g, lr_weight, lr_bias, wcat, cols, cfg, start_idx, grads):
+        xq, xk, xv, lr, gate = layer_projections(x, wcat, cols, cfg, lr_bias, start_idx, round_proj=True)
+        ctx.save_for_backward(x, wcat, lr)
+        ctx.meta = (cols, cfg, start_idx, grads, lr_weight.shape)
+        return xq, xk, xv, lr, None if gate is None else gate.reshape(*x.shape[:2], -1)
+
+    @staticmethod
+    def backward(ctx, dxq, dxk, dxv, dlr, dgate):
+        x, wcat, lr = ctx.saved_tensors
+        cols, cfg, start_idx, grads, lr_shape = ctx.meta
+        B, T, hs = x.shape
+        N, C_ = wcat.shape[0], cfg.num_heads * cfg.head_dim
+        dproj = grads.pop("dproj", None)
+        if dproj is None:
+            dproj = torch.empty(B, T, N, dtype=x.dtype, device=x.device)
+        if "g" in cols:
+            cg = dproj[..., cols["g"]:cols["g"] + C_]
+            if dgate.data_ptr() != cg.data_ptr() or dgate.stride() != cg.stride():
+                cg.copy_(dgate)  # (the gradient did not come straight from the epilogue)
+        dbias = _prologue_backward(dproj, cols, cfg, start_idx, lr, dxq, dxk, dxv, dlr)
+        d2 = dproj.reshape(B * T, N)
+        dx = torch.matmul(d2, wcat).reshape(B, T, hs) if ctx.needs_input_grad[0] else None
+        dw = torch.matmul(d2.t(), x.reshape(B * T, hs))
+        rows = lambda n, cnt: dw[cols[n]:cols[n] + cnt]  # noqa: E731
+        return (dx, rows("q", hs), rows("k", hs), rows("v", hs), rows("g", hs) if "g" in cols else None,
+                rows("lr", cfg.num_heads).reshape(lr_shape), dbias, None, None, None, None, None)
 
 
 def _taps4(w: torch.Tensor, dt) -> torch.Tensor:
@@ -278,16 +321,18 @@ class _QkConvFn(torch.autograd.Function):
 
 
 class _EpilogueFn(torch.autograd.Function):
-    """`ttt_layer_epilogue` with its gradient `ttt_layer_epilogue_backward`."""
+    """`ttt_layer_epilogue` with its gradient `ttt_layer_epilogue_backward`.  `grads` (optional): a dict for the
+    projections' gradient step, which receives the [B, T, width] buffer whose columns `col`.. hold the gate's gradient."""
 
     @staticmethod
-    def forward(ctx, inner_out, gate, ln_weight, ln_bias, eps):
+    def forward(ctx, inner_out, gate, ln_weight, ln_bias, eps, grads=None, width=0, col=0):
         inner_out = inner_out.contiguous()
         g2d, ld = (None, 0) if gate is None else (gate.contiguous().reshape(-1, gate.shape[-1]), gate.shape[-1])
         y = layer_epilogue(inner_out, ln_weight, ln_bias, eps, g2d, ld)
         ctx.save_for_backward(inner_out, g2d, ln_weight, ln_bias)
         ctx.eps = eps
         ctx.gate_shape = None if gate is None else gate.shape
+        ctx.grads = (grads, width, col)
         return y
 
     @staticmethod
@@ -298,7 +343,13 @@ class _EpilogueFn(torch.autograd.Function):
         dt, dev = inner_out.dtype, inner_out.device
         d = TttDims(B, H, T, F, 16, 1, 0.0, _dtype_code(dt))
         d_inner = torch.empty_like(inner_out)
-        d_gate = None if g2d is None else torch.empty_like(g2d)
+        d_gate = None
+        grads, width, col0 = getattr(ctx, "grads", (None, 0, 0))
+        if g2d is not None and grads is not None:
+            grads["dproj"] = torch.empty(B, T, width, dtype=dt, device=dev)
+            d_gate = grads["dproj"].reshape(B * T, width)[:, col0:col0 + H * F]
+        elif g2d is not None:
+            d_gate = torch.empty_like(g2d)
         dw = torch.empty(H * F, dtype=torch.float32, device=dev)
         db = torch.empty(H * F, dtype=torch.float32, device=dev)
         ws_bytes = lib.ttt_layer_epilogue_backward_workspace_bytes(C.byref(d))
@@ -309,10 +360,10 @@ class _EpilogueFn(torch.autograd.Function):
         with torch.cuda.device(dev):
             _lib.check(lib.ttt_layer_epilogue_backward(
                 C.byref(d), _ptr(dy), _ptr(inner_out), _ptr(g2d), 0 if g2d is None else g2d.shape[1],
-                _ptr(w), _ptr(b), ctx.eps, _ptr(d_inner), _ptr(d_gate), 0 if d_gate is None else d_gate.shape[1],
+                _ptr(w), _ptr(b), ctx.eps, _ptr(d_inner), _ptr(d_gate), 0 if d_gate is None else d_gate.stride(0),
                 _ptr(dw), _ptr(db), _ptr(ws), ws_bytes, stream))
         dg = None if d_gate is None else d_gate.reshape(ctx.gate_shape)
-        return d_inner, dg, dw.to(ln_weight.dtype), db.to(ln_bias.dtype), None
+        return d_inner, dg, dw.to(ln_weight.dtype), db.to(ln_bias.dtype), None, None, None, None
 
 
 class TTT(torch.nn.Module):
@@ -362,23 +413,26 @@ class TTT(torch.nn.Module):
         key = _lib.host().param_key(*srcs)
         if self._wcat is None or self._wcat_key != key:
             self._wcat_key = key
-            c = self.config
-            blocks, cols, off = [], {}, 0
-            for name, w in (("q", self.q_proj), ("k", self.k_proj), ("v", self.v_proj), ("g", self.g_proj)):
-                if w is not None:
-                    blocks.append(w)
-                    cols[name] = off
-                    off += w.shape[0]
-            blocks.append(self.learnable_ttt_lr_weight.reshape(c.num_heads, c.hidden_size))
-            cols["lr"] = off
-            off += c.num_heads
-            pad = (-off) % 8
-            if pad:
-                blocks.append(torch.zeros(pad, c.hidden_size, dtype=self.q_proj.dtype, device=self.q_proj.device))
-            if "k" not in cols:
-                cols["k"] = cols["q"]
-            self._wcat = (torch.cat([b.detach() for b in blocks], dim=0).contiguous(), cols)
+            self._wcat = self._stack_weights()
         return self._wcat
+
+    def _stack_weights(self):
+        c = self.config
+        blocks, cols, off = [], {}, 0
+        for name, w in (("q", self.q_proj), ("k", self.k_proj), ("v", self.v_proj), ("g", self.g_proj)):
+            if w is not None:
+                blocks.append(w)
+                cols[name] = off
+                off += w.shape[0]
+        blocks.append(self.learnable_ttt_lr_weight.reshape(c.num_heads, c.hidden_size))
+        cols["lr"] = off
+        off += c.num_heads
+        pad = (-off) % 8
+        if pad:
+            blocks.append(torch.zeros(pad, c.hidden_size, dtype=self.q_proj.dtype, device=self.q_proj.device))
+        if "k" not in cols:
+            cols["k"] = cols["q"]
+        return torch.cat([b.detach() for b in blocks], dim=0).contiguous(), cols
 
     def invalidate_fused_weight(self):
         self._wcat = self._te = None
@@ -474,12 +528,26 @@ class TTT(torch.nn.Module):
 
 
 def _train_forward(self, x, inner, state, start_idx):
-    """Training path: the same kernels, each with its gradient kernel, joined by torch autograd (which also supplies
-    the gradients of the library GEMMs).  The gate projection is a GEMM of its own here, so that every column of the
-    fused projection's gradient is written by exactly one kernel."""
+    """Training path: the same kernels, each with its gradient kernel, joined by torch autograd.  Where the one-launch
+    projections apply (bf16, no shared q / k) they run here as in inference; elsewhere the projection is a library
+    product, and the gate's a product of its own, so that every column of the fused projection's gradient is written by
+    exactly one kernel.  (65536 tokens of 768 features: one launch instead of product + prologue 300 -> 186 us.)"""
     c = self.config
     B, T, _ = x.shape
     H, hs = c.num_heads, c.hidden_size
+    te = torch.clamp_min(self.token_idx + self.learnable_token_idx, 0.0)
+    token_eta = te.repeat((T + c.mini_batch_size - 1) // c.mini_batch_size)[:T].to(x.dtype)
+    if not c.share_qk and x.dtype == torch.bfloat16 == self.q_proj.dtype:
+        wcat, cols = self._stack_weights()  # (not kept: the weights change with every step)
+        if self._can_fuse_projections(x, cols):
+            grads = {}
+            xq, xk, xv, lr, gate = _ProjectionsFn.apply(
+                x, self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.learnable_ttt_lr_weight,
+                self.learnable_ttt_lr_bias, wcat, cols, c, start_idx, grads)
+            out = inner.forward(state, TTTInputsInner(Qkv(xq, xk, xv), token_eta, lr, start_idx))
+            y = _EpilogueFn.apply(out, gate, self.post_norm_weight, self.post_norm_bias, 1e-6,
+                                  grads if gate is not None else None, wcat.shape[0], cols.get("g", 0))
+            return torch.matmul(y, self.o_proj.t())
     if c.share_qk:
         # shared projection | v | lr logits, then the two convolutions as a step of their own (with its gradient
         # kernel); the prologue sees the usual q | k | v | lr layout
@@ -504,8 +572,6 @@ def _train_forward(self, x, inner, state, start_idx):
         proj = torch.matmul(x, torch.cat(blocks, dim=0).t())
     cols = {"q": 0, "k": hs, "v": 2 * hs, "lr": 3 * hs}
     xq, xk, xv, lr = _PrologueFn.apply(proj, self.learnable_ttt_lr_bias, c, cols, start_idx)
-    te = torch.clamp_min(self.token_idx + self.learnable_token_idx, 0.0)
-    token_eta = te.repeat((T + c.mini_batch_size - 1) // c.mini_batch_size)[:T].to(x.dtype)
     out = inner.forward(state, TTTInputsInner(Qkv(xq, xk, xv), token_eta, lr, start_idx))
     gate = torch.matmul(x, self.g_proj.t()) if c.use_gate else None
     y = _EpilogueFn.apply(out, gate, self.post_norm_weight, self.post_norm_bias, 1e-6)
