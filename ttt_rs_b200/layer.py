@@ -252,6 +252,27 @@ class _ProjectionsFn(torch.autograd.Function):
                 rows("lr", cfg.num_heads).reshape(lr_shape), dbias, None, None, None, None, None)
 
 
+class _TokenEtaFn(torch.autograd.Function):
+    """max(token_idx + learnable_token_idx, 0) repeated over the sequence's mini-batches, in `dtype` (autograd's own gradient
+    of the same expression is six launches of a few hundred elements)."""
+
+    @staticmethod
+    def forward(ctx, token_idx, learnable, T, dtype):
+        te = token_idx + learnable
+        ctx.save_for_backward(te)
+        ctx.dtype = learnable.dtype
+        return torch.clamp_min(te, 0.0).to(dtype).repeat((T + te.shape[0] - 1) // te.shape[0])[:T]
+
+    @staticmethod
+    def backward(ctx, d):
+        (te,) = ctx.saved_tensors
+        mb = te.shape[0]
+        if d.shape[0] % mb:
+            d = torch.nn.functional.pad(d, (0, -d.shape[0] % mb))
+        s = d.reshape(-1, mb).sum(dim=0, dtype=ctx.dtype)
+        return None, torch.where(te >= 0, s, 0.0), None, None
+
+
 def _taps4(w: torch.Tensor, dt) -> torch.Tensor:
     """Depthwise convolution weight [C,1,K] or [C,K] (K <= 4) -> [C,4], taps aligned to the end (tap j multiplies
     token t - 3 + j)."""
@@ -535,8 +556,7 @@ def _train_forward(self, x, inner, state, start_idx):
     c = self.config
     B, T, _ = x.shape
     H, hs = c.num_heads, c.hidden_size
-    te = torch.clamp_min(self.token_idx + self.learnable_token_idx, 0.0)
-    token_eta = te.repeat((T + c.mini_batch_size - 1) // c.mini_batch_size)[:T].to(x.dtype)
+    token_eta = _TokenEtaFn.apply(self.token_idx, self.learnable_token_idx, T, x.dtype)
     if not c.share_qk and x.dtype == torch.bfloat16 == self.q_proj.dtype:
         wcat, cols = self._stack_weights()  # (not kept: the weights change with every step)
         if self._can_fuse_projections(x, cols):
