@@ -455,7 +455,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             if (FUSED) {
               if (p.f.round_proj && kd != 2) {  // (v is rounded once either way)
 #pragma unroll
-                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__bfloat162float(__float2bfloat16_rn(__uint_as_float(r[i]))));
+                for (int i = 0; i < 32; i += 2) {
+                  const uint32_t v = pack_bf16(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                  r[i] = __float_as_uint(bf16_lo(v));
+                  r[i + 1] = __float_as_uint(bf16_hi(v));
+                }
               }
               if (kd == 4) {
                 // learning-rate logits: column i of this group is head i
