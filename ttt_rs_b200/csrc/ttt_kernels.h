@@ -155,6 +155,7 @@ struct LayerEpiParams {
   const void* ln_w;       // [H*F]
   const void* ln_b;
   void* y;                // [B,T,H*F]
+  int row_groups;         // set by the launcher: rows of a tile that a CTA's threads work on at once
   int B, H, T;
   float eps;
 };
