@@ -394,8 +394,9 @@ static cudaError_t launch_epi_g(LayerEpiParams p, cudaStream_t st) {
   const int C = p.H * FD, nch = C / (16 / (int)sizeof(T));
   constexpr int TT = 64 / MAXCH, MAXT = MAXCH == 16 ? 512 : EPI_THREADS;
   auto kfn = ttt_layer_epilogue_kernel<T, MAXCH, FD, GATE>;
-  // as many row groups as fit a CTA, but no more than a tile has rows
+  // as many row groups as fit a CTA and divide the rows of a tile evenly (65536 x 512, bf16: 39.8 us with 6 groups, 35.8 with 4)
   p.row_groups = MAXT / nch < TT ? MAXT / nch : TT;
+  while (TT % p.row_groups) --p.row_groups;
   const int threads = (p.row_groups * nch + 31) & ~31;
   const size_t smem = 2 * (size_t)TT * C * sizeof(T) + TT * sizeof(float2);
   static DeviceValue resident;
