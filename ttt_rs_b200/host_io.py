@@ -46,13 +46,20 @@ def chunk_bounds(batch: int, chunks: int, taper: bool = True):
 def auto_chunks(batch: int, heads: int, seq_len: int, head_dim: int, elem_size: int, mini_batch: int,
                 backward: bool = True) -> int:
     """Number of equal chunks for a link-bound step.  A chunk's kernels are a chain of seq_len / mini_batch dependent
-    stages whose time does not shrink with the chunk (about 1.5 us per forward stage and 3.3 us per backward stage on
+    stages whose time does not shrink with the chunk (about 1.2 us per forward stage and 2.1 us per backward stage on
     a B200), so a chunk must carry enough rows that copying it takes longer than that chain -- else the compute
     stream, not the link, paces the pipeline -- and no more, because the first copy-in and the last copy-out are not
     overlapped.  The link moves about 45 GB/s per direction with both directions busy."""
-    chain_ms = (seq_len / mini_batch) * (4.8e-3 if backward else 1.5e-3)
+    chain_ms = (seq_len / mini_batch) * (3.3e-3 if backward else 1.2e-3)
     row_ms = heads * seq_len * head_dim * elem_size * (4 if backward else 3) / 45e6
     rows = max(1, -int(-1.3 * chain_ms // row_ms))
+    # Rows that cut the batch into equal chunks, if there are such up to twice as many (behind a chunk larger than the one
+    # before it the copy-out waits), and then no more than a dozen chunks, each of which costs its events and launches:
+    # 12 x 2048 x 64 bf16, forward + backward, 32 rows: 8 chunks 9.6 ms, 16 chunks 9.8, 11 unequal ones 10.4; 16 rows: 8
+    # chunks 5.2 ms, 6 unequal ones 5.8; 8 rows: 4 chunks 3.13 ms, 3 unequal ones 3.39.
+    even = [r for r in range(rows, 2 * rows + 1) if batch % r == 0]
+    if even:
+        rows = next((r for r in even if batch // r <= 12), even[-1])
     return max(1, -(-batch // rows))
 
 
