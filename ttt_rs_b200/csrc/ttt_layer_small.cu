@@ -17,6 +17,11 @@ namespace ttt {
 
 constexpr int SM_THREADS = 256, SM_WARPS = 8;
 
+// These kernels begin while the kernel before them runs (launch_dependent).  What that one may be writing -- activations,
+// for the first of them weights too -- is read by ordinary loads behind pdl_wait: the non-coherent path promises data that
+// nobody writes while the kernel runs, and such a load may be moved above the wait.  It is left to the output kernel's
+// weights: its predecessor, the inner step, writes none, and everything before that has finished when it starts.
+__device__ __forceinline__ uint4 ld4(const void* p) { return *static_cast<const uint4*>(p); }
 __device__ __forceinline__ uint4 ldg4(const void* p) { return __ldg(static_cast<const uint4*>(p)); }
 
 // acc[mt][nt] += A . B^T over one 32-wide slice: a[mt][half] rows 16 mt + g + 8 half, b[nt] rows 8 nt + g
@@ -76,14 +81,14 @@ __global__ void __launch_bounds__(SM_THREADS) ttt_layer_small_proj_kernel(const 
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       const int n = n0 + 8 * nt + g;
-      b[nt] = n < p.N ? ldg4(w + (size_t)n * p.ldw + k) : zero;
+      b[nt] = n < p.N ? ld4(w + (size_t)n * p.ldw + k) : zero;
     }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int m = 16 * mt + g + 8 * r;
-        a[mt][r] = m < p.M ? ldg4(x + (size_t)m * p.ldx + k) : zero;
+        a[mt][r] = m < p.M ? ld4(x + (size_t)m * p.ldx + k) : zero;
       }
     slice_mma(acc, a, b);
   }
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(SM_THREADS) ttt_layer_small_out_kernel(const S
       const int c = 8 * lane + 256 * i;
       if (c < C) {
         const int h = c / p.F, f = c - h * p.F;
-        const uint4 q = ldg4(static_cast<const __nv_bfloat16*>(p.inner_out) + (((size_t)b * p.H + h) * p.T + tok) * p.F + f);
+        const uint4 q = ld4(static_cast<const __nv_bfloat16*>(p.inner_out) + (((size_t)b * p.H + h) * p.T + tok) * p.F + f);
         const uint32_t u[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(SM_THREADS) ttt_layer_small_out_kernel(const S
           y[2 * j + 1] = fmaf(v[i][2 * j + 1] * rstd, bf16_hi(gu[j]), bf16_hi(bu[j]));
         }
         if (p.gate != nullptr) {
-          const uint4 tq = ldg4(static_cast<const __nv_bfloat16*>(p.gate) + (size_t)m * p.ld_gate + c);
+          const uint4 tq = ld4(static_cast<const __nv_bfloat16*>(p.gate) + (size_t)m * p.ld_gate + c);
           const uint32_t tu[4] = {tq.x, tq.y, tq.z, tq.w};
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
