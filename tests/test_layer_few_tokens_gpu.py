@@ -28,3 +28,19 @@ def test_short_and_ragged_calls_match_the_restatement(B, T, H, F, use_gate, star
     assert_close(y, want, 3e-2, "layer output", max_bad_frac=1e-3)
     assert_close(state.weight, st["weight"], 2e-2, "state weight", max_bad_frac=1e-3)
     assert_close(state.bias, st["bias"], 2e-2, "state bias", max_bad_frac=5e-3)
+
+
+@pytest.mark.gpu
+def test_one_token_of_sequences_in_a_buffer_beyond_32_bit_offsets():
+    """A decode step on a slice of a [2, T, C] buffer with T C = 2^31: the rows' pitch does not fit 32 bits."""
+    import ttt_rs_b200 as tb
+    H, C, far = 2, 128, 1 << 31
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H)
+    torch.manual_seed(5)
+    m = tb.TTT(cfg, device="cuda", dtype=torch.bfloat16)
+    inner = tb.new_inner(cfg, device="cuda", dtype=torch.bfloat16, allow_partial=True)
+    rows = (torch.randn(2, 1, C, device="cuda") * 0.5).bfloat16()
+    x = torch.empty(far + C, dtype=torch.bfloat16, device="cuda").as_strided((2, 1, C), (far, C, 1))
+    x.copy_(rows)
+    with torch.no_grad():
+        assert torch.equal(m(x, inner, inner.init_state(2)), m(rows, inner, inner.init_state(2)))

@@ -897,7 +897,7 @@ extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, i
   ttt::SmallProjParams p;
   p.x = x; p.w = weights; p.lr_bias = lr_bias;
   p.xq = xq; p.xk = xk; p.xv = xv; p.gate = gate; p.lr_out = ttt_lr_eta;
-  p.M = d->batch * d->seq_len; p.N = w_rows; p.K = d->heads * d->head_dim; p.ldx = (int)x_ld; p.ldw = (int)w_ld;
+  p.M = d->batch * d->seq_len; p.N = w_rows; p.K = d->heads * d->head_dim; p.ldx = (long)x_ld; p.ldw = (int)w_ld;
   p.H = d->heads; p.F = d->head_dim; p.T = d->seq_len; p.lr_col = lr_col; p.lr_ld = lr_pitch;
   p.start_idx = start_idx; p.pos_mod = rope_mode == 1 ? d->mini_batch : 1; p.rope_mode = rope_mode;
   p.rope_theta = rope_mode != 0 ? rope_theta : 1.f; p.base_lr = base_lr;

@@ -167,7 +167,8 @@ struct SmallProjParams {
   const void* w;  // [N, ldw]: q | k | v | (gate) blocks of H F rows, then H learning-rate rows from lr_col on
   const void* lr_bias;
   void *xq, *xk, *xv, *gate, *lr_out;  // [B,H,T,F] x 3, [M, H F] or null, [B,H,lr_ld]
-  int M, N, K, ldx, ldw, H, F, T, lr_col, lr_ld;
+  long ldx;  // (one-token calls on a slice of a [B, T, C] buffer: T C elements)
+  int M, N, K, ldw, H, F, T, lr_col, lr_ld;
   int start_idx, pos_mod, rope_mode;
   float rope_theta, base_lr;
 };
