@@ -187,6 +187,23 @@ def test_partial_and_layer_entry_points_validate_their_arguments(lib):
     assert epi(eps=-1.0) == _lib.TTT_ERR_SHAPE
 
 
+def test_few_token_projections_refuse_what_the_prologue_refuses(lib):
+    """The few-token form takes over calls of the prologue: positions, rotation modes and angles refused there stay refused."""
+    fake, d = C.c_void_p(0x1000), _dims(seq_len=1)
+
+    def proj(start=0, mode=1, theta=10000.0, dims=d):
+        f = lib.ttt_internal_layer_small_proj
+        f.restype, f.argtypes = C.c_int, [_lib._DP, _lib._P, C.c_int64, _lib._P, C.c_int64, C.c_int, C.c_int, _lib._P, C.c_int,
+                                          C.c_int, C.c_float, C.c_float] + [_lib._P] * 5 + [C.c_int, _lib._P]
+        return f(C.byref(dims), fake, 128, fake, 128, 392, 384, None, start, mode, theta, 1.0, fake, fake, fake, None, fake, 8,
+                 None)
+
+    assert proj(start=-1) == _lib.TTT_ERR_SHAPE
+    assert proj(mode=3) == proj(mode=-1) == _lib.TTT_ERR_UNSUPPORTED
+    assert proj(theta=0.0) == proj(theta=float("nan")) == _lib.TTT_ERR_SHAPE
+    assert proj(dims=_dims(seq_len=1, mini_batch=65)) == proj(dims=_dims(seq_len=1, mini_batch=0)) == _lib.TTT_ERR_UNSUPPORTED
+
+
 def test_rust_declarations_in_the_integration_guide_match_the_header():
     """The integration guide carries the Rust `extern "C"` block a maintainer would paste; it is generated from the header.
     The committed text must equal a fresh generation, and every declaration must have as many arguments as the

@@ -724,6 +724,14 @@ int check_layer_dims(const ttt_dims* d) {
     return fail(TTT_ERR_SHAPE, "batch*heads*seq_len must be below 2^31");
   return TTT_OK;
 }
+int check_rotation(const ttt_dims* d, int start_idx, int rope_mode, float rope_theta) {
+  if (rope_mode < 0 || rope_mode > 2) return fail(TTT_ERR_UNSUPPORTED, "rope_mode=%d (0 none, 1 wrapped, 2 global)", rope_mode);
+  if (rope_mode == 1 && (d->mini_batch < 1 || d->mini_batch > 64))
+    return fail(TTT_ERR_UNSUPPORTED, "wrapped rotary positions need 1 <= mini_batch <= 64 (got %d)", d->mini_batch);
+  if (rope_mode != 0 && !(rope_theta > 0.f)) return fail(TTT_ERR_SHAPE, "rope_theta must be positive");
+  if (start_idx < 0) return fail(TTT_ERR_SHAPE, "start_idx must be >= 0");
+  return TTT_OK;
+}
 }  // namespace
 
 extern "C" int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src, const void* k_src, const void* v_src,
@@ -739,11 +747,7 @@ extern "C" int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src,
     return fail(TTT_ERR_NULL, "conv_q_weight, conv_q_bias, conv_k_weight and conv_k_bias must be given together");
   if (conv && (conv_kernel < 1 || conv_kernel > 4))
     return fail(TTT_ERR_UNSUPPORTED, "conv_kernel=%d (supported: 1..4)", conv_kernel);
-  if (rope_mode < 0 || rope_mode > 2) return fail(TTT_ERR_UNSUPPORTED, "rope_mode=%d (0 none, 1 wrapped, 2 global)", rope_mode);
-  if (rope_mode == 1 && (d->mini_batch < 1 || d->mini_batch > 64))
-    return fail(TTT_ERR_UNSUPPORTED, "wrapped rotary positions need 1 <= mini_batch <= 64 (got %d)", d->mini_batch);
-  if (rope_mode != 0 && !(rope_theta > 0.f)) return fail(TTT_ERR_SHAPE, "rope_theta must be positive");
-  if (start_idx < 0) return fail(TTT_ERR_SHAPE, "start_idx must be >= 0");
+  if ((rc = check_rotation(d, start_idx, rope_mode, rope_theta)) != TTT_OK) return rc;
   if (lr_pitch < d->seq_len) return fail(TTT_ERR_SHAPE, "lr_pitch must be >= seq_len");
   const int64_t cols = (int64_t)d->heads * d->head_dim;
   if (src_ld < cols || (src_ld & 7) != 0)
@@ -891,6 +895,7 @@ extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, i
                                              int rope_mode, float rope_theta, float base_lr, void* xq, void* xk,
                                              void* xv, void* gate, void* ttt_lr_eta, int lr_pitch, void* stream) {
   if (!ttt_internal_layer_small_fits(d)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
+  if (const int rc = check_rotation(d, start_idx, rope_mode, rope_theta); rc != TTT_OK) return rc;
   if (x_ld % 8 != 0 || w_ld % 8 != 0) return fail(TTT_ERR_ALIGN, "row pitches must be multiples of 8 elements");
   const NamedPtr ptrs[] = {{"x", x}, {"weights", weights}, {"xq", xq}, {"xk", xk}, {"xv", xv}};
   if (const int rc = check_ptrs(ptrs, 5); rc != TTT_OK) return rc;
@@ -930,11 +935,7 @@ extern "C" int ttt_layer_prologue_backward(const ttt_dims* d, const void* grad_x
                                            void* grad_lr_logits, int64_t lr_ld, int lr_cols, void* stream) {
   int rc = check_layer_dims(d);
   if (rc != TTT_OK) return rc;
-  if (rope_mode < 0 || rope_mode > 2) return fail(TTT_ERR_UNSUPPORTED, "rope_mode=%d (0 none, 1 wrapped, 2 global)", rope_mode);
-  if (rope_mode == 1 && (d->mini_batch < 1 || d->mini_batch > 64))
-    return fail(TTT_ERR_UNSUPPORTED, "wrapped rotary positions need 1 <= mini_batch <= 64 (got %d)", d->mini_batch);
-  if (rope_mode != 0 && !(rope_theta > 0.f)) return fail(TTT_ERR_SHAPE, "rope_theta must be positive");
-  if (start_idx < 0) return fail(TTT_ERR_SHAPE, "start_idx must be >= 0");
+  if ((rc = check_rotation(d, start_idx, rope_mode, rope_theta)) != TTT_OK) return rc;
   if (!(base_lr != 0.f)) return fail(TTT_ERR_SHAPE, "base_lr must be non-zero");
   if (dst_ld < (int64_t)d->heads * d->head_dim || (dst_ld & 7) != 0)
     return fail(TTT_ERR_SHAPE, "dst_ld (%lld) must be >= heads*head_dim and a multiple of 8", (long long)dst_ld);
