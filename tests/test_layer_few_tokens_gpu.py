@@ -44,3 +44,27 @@ def test_one_token_of_sequences_in_a_buffer_beyond_32_bit_offsets():
     x.copy_(rows)
     with torch.no_grad():
         assert torch.equal(m(x, inner, inner.init_state(2)), m(rows, inner, inner.init_state(2)))
+
+
+@pytest.mark.gpu
+def test_a_call_that_goes_another_way_advances_the_state_once(monkeypatch):
+    """Post-norm parameters off the 16-byte grid: the native layer call declines them, and has touched nothing by then."""
+    import ttt_rs_b200 as tb
+    H, C = 2, 128
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H)
+    torch.manual_seed(6)
+    m = tb.TTT(cfg, device="cuda", dtype=torch.bfloat16)
+    inner = tb.new_inner(cfg, device="cuda", dtype=torch.bfloat16, allow_partial=True, partial_in_place=True)
+    x = (torch.randn(3, 1, C, device="cuda") * 0.5).bfloat16()
+
+    def step():
+        with torch.no_grad():
+            state = inner.init_state(3)
+            return m(x, inner, state), state.weight, state.bias
+
+    step()
+    m.post_norm_weight = torch.nn.Parameter(torch.ones(C + 1, device="cuda", dtype=torch.bfloat16)[1:])
+    got = step()
+    monkeypatch.setattr(m, "_infer_native", lambda *a: None)
+    for a, b in zip(got, step()):
+        assert torch.equal(a, b)

@@ -42,6 +42,7 @@ PyObject* g_error_type = nullptr;  // TttError(code, message)
   throw python_error();
 }
 
+bool on_16_bytes(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0; }
 bool is(const Tensor& t, at::ScalarType dt, const c10::Device& dev, c10::IntArrayRef sizes) {
   return t.defined() && t.is_cuda() && t.device() == dev && t.scalar_type() == dt && t.sizes() == sizes &&
          t.is_contiguous() && t.layout() == c10::kStrided;
@@ -419,6 +420,8 @@ PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
 //   -> (y, state weight, state bias) | None
 // One call of TTT.forward without gradients, bf16: projections + prologue, inner loop (whole mini-batches, then the
 // remainder as a mini-batch of its own), post norm (+ gate), output projection.
+// None comes before the first launch only (what a later launch would refuse is looked at up front): the caller then takes
+// another way from the same state.  An error after that is raised.
 PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 26)) return nullptr;
@@ -436,7 +439,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const bool allow_partial = args[23] == Py_True, in_place = args[24] == Py_True;
   if (PyErr_Occurred()) return nullptr;
 
-  NONE_IF(!x.is_cuda() || x.dim() != 3 || x.scalar_type() != at::kBFloat16 || H <= 0);
+  NONE_IF(!x.is_cuda() || x.dim() != 3 || x.scalar_type() != at::kBFloat16 || H <= 0 || mb <= 0);
   const c10::Device dev = x.device();
   const at::ScalarType bf = at::kBFloat16;
   const int64_t B = x.size(0), T = x.size(1), C = x.size(2), F = C / H, M = B * T;
@@ -457,7 +460,10 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     NONE_IF(t[5].numel() != C || t[7].numel() != C || t[6].numel() != t[4].numel());
   }
   const int64_t L = T / mb * mb, R = T - L;
-  NONE_IF(R != 0 && !allow_partial);
+  NONE_IF(R > 16 || (R != 0 && !allow_partial));
+  NONE_IF(L > 0 && ((mb != 16 && mb != 8) || (F == 32 && H % 2 != 0)));
+  for (int i : {0, 1, 14}) NONE_IF(!on_16_bytes(t[i]));
+  for (int i : {8, 9, 10, 11}) NONE_IF(L > 0 && !on_16_bytes(t[i]));  // (the remainder's kernel takes any alignment)
   Dims m;
   m.dt = bf;
   m.dev = dev;
@@ -469,6 +475,11 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   void* const st = m.stream();
   void* const status = m.status.data_ptr();
   const bool small = !conv && ttt_internal_layer_small_fits(&d);
+  NONE_IF(small && (!on_16_bytes(t[12]) || !on_16_bytes(t[13])));
+  NONE_IF(!small && N % 8 != 0);
+  auto must = [](int rc) {
+    if (rc != TTT_OK) throw_error(rc);
+  };
   const bool fused = !small && !conv && T % 128 == 0 && F == 64 && rope != 2 && mb <= 16 && lr_col % 64 == 0;
   // temporaries from one allocation, each on a 256-byte boundary
   int64_t at_ = 0;
@@ -503,15 +514,14 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (use_gate) gate = base + o_gate;
   } else {
     uint8_t* const proj = base + o_proj;
-    NONE_IF(N % 8 != 0);
     NONE_IF(ttt_gemm_bf16_tn(M, N, C, x.const_data_ptr(), x_ld, wcat.const_data_ptr(), C, proj, N, status, st) != TTT_OK);
     const int64_t k_col = conv ? 0 : C, v_col = conv ? C : 2 * C;
-    NONE_IF(ttt_internal_layer_prologue(&d, proj, proj + 2 * k_col, proj + 2 * v_col, N, proj + 2 * lr_col, N,
-                                        lr_bias.const_data_ptr(), conv ? t[4].const_data_ptr() : nullptr,
-                                        conv ? t[5].const_data_ptr() : nullptr, conv ? t[6].const_data_ptr() : nullptr,
-                                        conv ? t[7].const_data_ptr() : nullptr, conv_k, (int)start, (int)rope, theta,
-                                        base_lr, base + o_q, base + o_k, base + o_v, base + o_lr, (int)lr_pitch,
-                                        st) != TTT_OK);
+    must(ttt_internal_layer_prologue(&d, proj, proj + 2 * k_col, proj + 2 * v_col, N, proj + 2 * lr_col, N,
+                                     lr_bias.const_data_ptr(), conv ? t[4].const_data_ptr() : nullptr,
+                                     conv ? t[5].const_data_ptr() : nullptr, conv ? t[6].const_data_ptr() : nullptr,
+                                     conv ? t[7].const_data_ptr() : nullptr, conv_k, (int)start, (int)rope, theta,
+                                     base_lr, base + o_q, base + o_k, base + o_v, base + o_lr, (int)lr_pitch,
+                                     st));
     if (use_gate) gate = proj + 2 * g_col, gate_ld = N;
   }
   // ---- inner loop
@@ -521,10 +531,10 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     b = at::empty({B, H, F}, m.opt());
     ttt_dims di = d;
     di.seq_len = (int32_t)L;
-    NONE_IF(ttt_internal_linear_infer(&di, (int)T, (int)lr_pitch, base + o_q, base + o_k, base + o_v,
-                                      sw.const_data_ptr(), sb.const_data_ptr(), te.const_data_ptr(), base + o_lr,
-                                      t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in, w.data_ptr(),
-                                      b.data_ptr(), status, st) != TTT_OK);
+    must(ttt_internal_linear_infer(&di, (int)T, (int)lr_pitch, base + o_q, base + o_k, base + o_v,
+                                   sw.const_data_ptr(), sb.const_data_ptr(), te.const_data_ptr(), base + o_lr,
+                                   t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in, w.data_ptr(),
+                                   b.data_ptr(), status, st));
   }
   if (R > 0) {
     const Tensor w_in = w, b_in = b;
@@ -534,20 +544,20 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     ttt_dims dt = d;
     dt.seq_len = (int32_t)R;
-    NONE_IF(ttt_internal_linear_tail(&dt, (int)T, (int)L, (int)lr_pitch, small && L == 0, base + o_q, base + o_k, base + o_v,
-                                     w_in.const_data_ptr(), b_in.const_data_ptr(), te.const_data_ptr(), base + o_lr,
-                                     t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in,
-                                     const_cast<void*>(w.const_data_ptr()), const_cast<void*>(b.const_data_ptr()),
-                                     st) != TTT_OK);
+    must(ttt_internal_linear_tail(&dt, (int)T, (int)L, (int)lr_pitch, small && L == 0, base + o_q, base + o_k, base + o_v,
+                                  w_in.const_data_ptr(), b_in.const_data_ptr(), te.const_data_ptr(), base + o_lr,
+                                  t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in,
+                                  const_cast<void*>(w.const_data_ptr()), const_cast<void*>(b.const_data_ptr()),
+                                  st));
   }
   // ---- post norm, gate, output projection
   if (small) {
-    NONE_IF(ttt_internal_layer_small_out(&d, base + o_in, gate, (int)gate_ld, t[12].const_data_ptr(),
-                                         t[13].const_data_ptr(), 1e-6f, t[14].const_data_ptr(), C, y.data_ptr(), st) != TTT_OK);
+    must(ttt_internal_layer_small_out(&d, base + o_in, gate, (int)gate_ld, t[12].const_data_ptr(),
+                                      t[13].const_data_ptr(), 1e-6f, t[14].const_data_ptr(), C, y.data_ptr(), st));
   } else {
-    NONE_IF(ttt_layer_epilogue(&d, base + o_in, gate, gate != nullptr ? gate_ld : 0, t[12].const_data_ptr(),
-                               t[13].const_data_ptr(), 1e-6f, base + o_y, st) != TTT_OK);
-    NONE_IF(ttt_gemm_bf16_tn(M, C, C, base + o_y, C, t[14].const_data_ptr(), C, y.data_ptr(), C, status, st) != TTT_OK);
+    must(ttt_layer_epilogue(&d, base + o_in, gate, gate != nullptr ? gate_ld : 0, t[12].const_data_ptr(),
+                            t[13].const_data_ptr(), 1e-6f, base + o_y, st));
+    must(ttt_gemm_bf16_tn(M, C, C, base + o_y, C, t[14].const_data_ptr(), C, y.data_ptr(), C, status, st));
   }
   return wrap({y, w, b});
   END_HANDLE_TH_ERRORS
