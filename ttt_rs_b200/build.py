@@ -20,6 +20,7 @@ PROBE_BIN = PKG / "build" / "probe_chain_latency"
 SOURCES = ["ttt_abi.cu", "ttt_linear_fwd.cu", "ttt_linear_bwd.cu", "ttt_mlp_fwd.cu", "ttt_layer.cu", "ttt_layer_small.cu", "ttt_linear_partial.cu", "ttt_mlp_bwd.cu", "ttt_gemm.cu"]
 HOST_SRC = CSRC / "ttt_host.cpp"                 # native host path of the Python operator, linked against LIB
 HOST_LIB = PKG / "_host.so"
+HOST_TAG = PKG / "build" / "_host.tag"           # what HOST_LIB was built against
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
@@ -55,10 +56,21 @@ def build_probe(force: bool = False) -> Path:
     return PROBE_BIN
 
 
+def host_tag() -> str:
+    """The interpreter and the torch that run this: `_host` uses the C++ interfaces of both, which change from one version
+    to the next."""
+    import sysconfig
+
+    import torch
+    return f"{sysconfig.get_config_var('EXT_SUFFIX')} torch {torch.__version__} {torch.version.git_version}\n"
+
+
 def build_host(force: bool = False) -> Path:
     """The CPython extension module `_host`, for the interpreter and the torch that run this."""
     deps = [HOST_SRC, CSRC / "ttt_internal.h", PKG.parent / "include" / "ttt_b200.h"]
-    if not force and HOST_LIB.exists() and all(HOST_LIB.stat().st_mtime >= p.stat().st_mtime for p in deps):
+    tag = host_tag()
+    if not force and HOST_LIB.exists() and all(HOST_LIB.stat().st_mtime >= p.stat().st_mtime for p in deps) \
+            and HOST_TAG.exists() and HOST_TAG.read_text() == tag:
         return HOST_LIB
     import sysconfig
 
@@ -74,6 +86,8 @@ def build_host(force: bool = False) -> Path:
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {HOST_SRC.name}:\n{r.stdout}")
+    HOST_TAG.parent.mkdir(exist_ok=True)
+    HOST_TAG.write_text(tag)
     return HOST_LIB
 
 
