@@ -68,3 +68,35 @@ def test_a_call_that_goes_another_way_advances_the_state_once(monkeypatch):
     monkeypatch.setattr(m, "_infer_native", lambda *a: None)
     for a, b in zip(got, step()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", (1, 40, 128))  # few-token form; general form with a remainder; one-launch projections
+def test_token_eta_follows_its_parameters_at_every_call(T):
+    """Also through `.data`, which leaves the parameter's version as it was; the kernels form the values that tensor
+    operations give (negative sums clamped, sums rounded to bf16)."""
+    import ttt_rs_b200 as tb
+    H, C = 2, 128
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H)
+    torch.manual_seed(8)
+    m = tb.TTT(cfg, device="cuda", dtype=torch.bfloat16)
+    inner = tb.new_inner(cfg, device="cuda", dtype=torch.bfloat16, allow_partial=True)
+    x = (torch.randn(3, T, C, device="cuda") * 0.5).bfloat16()
+
+    def run():
+        with torch.no_grad():
+            state = inner.init_state(3)
+            return [m(x, inner, state), state.weight, state.bias]
+
+    run()
+    seen = []
+    for shift in (0.37, -0.4):
+        m.learnable_token_idx.data.add_(shift)
+        seen.append(run())
+        te = torch.clamp_min(m.token_idx + m.learnable_token_idx, 0.0)
+        idx, learnable = m.token_idx, m.learnable_token_idx
+        m.token_idx, m.learnable_token_idx = te.detach(), torch.nn.Parameter(torch.zeros_like(te))
+        for a, b in zip(seen[-1], run()):
+            assert torch.equal(a, b)
+        m.token_idx, m.learnable_token_idx = idx, learnable
+    assert not torch.equal(seen[0][1], seen[1][1])

@@ -372,9 +372,9 @@ size_t ttt_linear_bias_ckpt_bytes(const ttt_dims* d) {
 }
 
 static int linear_forward_impl(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk, const void* xv, const void* weight,
-                       const void* bias, const void* token_eta, const void* ttt_lr_eta, const void* ln_weight,
-                       const void* ln_bias, void* output, void* weight_out, void* bias_out, void* weight_ckpt,
-                       void* bias_ckpt, void* status, void* stream) {
+                       const void* bias, const void* token_eta, const void* token_eta_add, const void* ttt_lr_eta,
+                       const void* ln_weight, const void* ln_bias, void* output, void* weight_out, void* bias_out,
+                       void* weight_ckpt, void* bias_ckpt, void* status, void* stream) {
   int rc = check_dims(d, true);
   if (rc != TTT_OK) return rc;
   const NamedPtr ptrs[] = {{"xq", xq},           {"xk", xk},
@@ -409,6 +409,7 @@ static int linear_forward_impl(const ttt_dims* d, int seq_pitch, int lr_pitch, c
   p.w0 = weight;
   p.b0 = bias;
   p.token_eta = token_eta;
+  p.token_eta_add = token_eta_add;
   p.lr = ttt_lr_eta;
   p.ln_g = ln_weight;
   p.ln_b = ln_bias;
@@ -437,21 +438,23 @@ int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const 
                        const void* ln_bias, void* output, void* weight_out, void* bias_out, void* weight_ckpt,
                        void* bias_ckpt, void* status, void* stream) {
   const int T = d != nullptr ? d->seq_len : 0;
-  return linear_forward_impl(d, T, T, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, output,
+  return linear_forward_impl(d, T, T, xq, xk, xv, weight, bias, token_eta, nullptr, ttt_lr_eta, ln_weight, ln_bias, output,
                              weight_out, bias_out, weight_ckpt, bias_ckpt, status, stream);
 }
 
 int ttt_internal_linear_infer(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk,
                               const void* xv, const void* weight, const void* bias, const void* token_eta,
-                              const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
-                              void* weight_out, void* bias_out, void* status, void* stream) {
+                              const void* token_eta_add, const void* ttt_lr_eta, const void* ln_weight,
+                              const void* ln_bias, void* output, void* weight_out, void* bias_out, void* status,
+                              void* stream) {
   if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
+  if (token_eta_add != nullptr && d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "token_eta_add is bf16 only");
   if (seq_pitch < d->seq_len || lr_pitch < d->seq_len || (int64_t)lr_pitch * (d->dtype == TTT_BF16 ? 2 : 4) % 16 != 0)
     return fail(TTT_ERR_SHAPE, "pitches must cover the sequence, learning-rate rows start on 16 bytes");
   if ((int64_t)d->batch * d->heads * seq_pitch >= (int64_t)1 << 31)
     return fail(TTT_ERR_SHAPE, "batch*heads*seq_pitch must be below 2^31");
-  return linear_forward_impl(d, seq_pitch, lr_pitch, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias,
-                             output, weight_out, bias_out, nullptr, nullptr, status, stream);
+  return linear_forward_impl(d, seq_pitch, lr_pitch, xq, xk, xv, weight, bias, token_eta, token_eta_add, ttt_lr_eta,
+                             ln_weight, ln_bias, output, weight_out, bias_out, nullptr, nullptr, status, stream);
 }
 
 size_t ttt_linear_backward_workspace_bytes(const ttt_dims* d) {
@@ -833,11 +836,13 @@ extern "C" int ttt_layer_epilogue(const ttt_dims* d, const void* inner_out, cons
   return TTT_OK;
 }
 
-extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled, const void* xq, const void* xk, const void* xv,
-                                          const void* weight, const void* bias, const void* token_eta,
-                                          const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
-                                          void* output, void* weight_out, void* bias_out, void* stream) {
+extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled,
+                                        const void* xq, const void* xk, const void* xv, const void* weight,
+                                        const void* bias, const void* token_eta, const void* token_eta_add,
+                                        const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
+                                        void* output, void* weight_out, void* bias_out, void* stream) {
   if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
+  if (token_eta_add != nullptr && d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "token_eta_add is bf16 only");
   if (d->batch <= 0 || d->heads <= 0) return fail(TTT_ERR_SHAPE, "batch and heads must be positive");
   if (d->dtype != TTT_F32 && d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "unknown dtype %d", d->dtype);
   if (d->head_dim != 64 && d->head_dim != 32)
@@ -858,6 +863,7 @@ extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int fi
   p.w0 = weight;
   p.b0 = bias;
   p.token_eta = token_eta;
+  p.token_eta_add = token_eta_add;
   p.lr = ttt_lr_eta;
   p.ln_g = ln_weight;
   p.ln_b = ln_bias;
@@ -881,8 +887,8 @@ extern "C" int ttt_linear_forward_partial(const ttt_dims* d, const void* xq, con
                                           const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
                                           void* output, void* weight_out, void* bias_out, void* stream) {
   const int T = d != nullptr ? d->seq_len : 0;
-  return ttt_internal_linear_tail(d, T, 0, T, 0, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, output,
-                                  weight_out, bias_out, stream);
+  return ttt_internal_linear_tail(d, T, 0, T, 0, xq, xk, xv, weight, bias, token_eta, nullptr, ttt_lr_eta, ln_weight,
+                                  ln_bias, output, weight_out, bias_out, stream);
 }
 
 extern "C" int ttt_internal_layer_small_fits(const ttt_dims* d) {

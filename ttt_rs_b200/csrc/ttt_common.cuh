@@ -319,6 +319,18 @@ template <>
 __device__ __forceinline__ float ld_as_float<__nv_bfloat16>(const void* base, size_t idx) {
   return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[idx]);
 }
+// token_eta of position i in the mini-batch: te[i], or with `add` (bf16 only) max(te[i] + add[i], 0), the sum rounded to T
+// as an addition of its own would leave it
+template <typename T>
+__device__ __forceinline__ float ld_token_eta(const void* te, const void* add, int i) {
+  float v = ld_as_float<T>(te, (size_t)i);
+  if constexpr (sizeof(T) == 2)
+    if (add != nullptr) {
+      v = __bfloat162float(__float2bfloat16_rn(v + ld_as_float<T>(add, (size_t)i)));
+      if (v < 0.f) v = 0.f;  // (a NaN stays one)
+    }
+  return v;
+}
 template <typename T>
 __device__ __forceinline__ void st_from_float(void* base, size_t idx, float v);
 template <>

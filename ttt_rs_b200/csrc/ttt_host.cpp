@@ -416,7 +416,8 @@ PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // layer_infer(x, stacked weights, token_eta of one mini-batch, lr_bias, conv q weight / bias, conv k weight / bias (or four
 //             None), state weight, state bias, ln weight, ln bias, post norm weight, bias, o_proj, gate 0/1, heads,
-//             mini_batch, rope_mode, rope_theta, base_lr, lr_col, eps_scaled, allow_partial, in_place, start_idx)
+//             mini_batch, rope_mode, rope_theta, base_lr, lr_col, eps_scaled, allow_partial, in_place, start_idx,
+//             what is added to token_eta before it is clamped at zero, or None)
 //   -> (y, state weight, state bias) | None
 // One call of TTT.forward without gradients, bf16: projections + prologue, inner loop (whole mini-batches, then the
 // remainder as a mini-batch of its own), post norm (+ gate), output projection.
@@ -424,12 +425,16 @@ PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // another way from the same state.  An error after that is raised.
 PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (!arity(n, 26)) return nullptr;
-  Tensor t[15];
+  if (!arity(n, 27)) return nullptr;
+  Tensor t[15], te_add;
   for (int i = 0; i < 15; ++i) {
     if (args[i] == Py_None && i >= 4 && i < 8) continue;
     NONE_IF(!THPVariable_Check(args[i]));
     t[i] = THPVariable_Unpack(args[i]);
+  }
+  if (args[26] != Py_None) {
+    NONE_IF(!THPVariable_Check(args[26]));
+    te_add = THPVariable_Unpack(args[26]);
   }
   const Tensor &x = t[0], &wcat = t[1], &te = t[2], &lr_bias = t[3], &sw = t[8], &sb = t[9];
   const bool use_gate = as_int(args[15]) != 0, conv = t[4].defined();
@@ -449,6 +454,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   NONE_IF((T > 1 && B > 1 && x.stride(0) != T * x_ld) || x_ld < C || x_ld % 8 != 0);
   const int64_t N = wcat.size(0);
   NONE_IF(!is(wcat, bf, dev, {N, C}) || te.dim() != 1 || te.size(0) < mb || !is(te, bf, dev, {te.size(0)}));
+  NONE_IF(te_add.defined() && !is(te_add, bf, dev, {te.size(0)}));
   NONE_IF(lr_bias.numel() != H || lr_bias.scalar_type() != bf || !lr_bias.is_contiguous() || lr_bias.device() != dev);
   NONE_IF(!is(sw, bf, dev, {B, H, F, F}) || !is(sb, bf, dev, {B, H, F}) || !is(t[10], bf, dev, {H, F}) ||
           !is(t[11], bf, dev, {H, F}) || !is(t[12], bf, dev, {C}) || !is(t[13], bf, dev, {C}) || !is(t[14], bf, dev, {C, C}));
@@ -463,7 +469,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   NONE_IF(R > 16 || (R != 0 && !allow_partial));
   NONE_IF(L > 0 && ((mb != 16 && mb != 8) || (F == 32 && H % 2 != 0)));
   for (int i : {0, 1, 14}) NONE_IF(!on_16_bytes(t[i]));
-  for (int i : {8, 9, 10, 11}) NONE_IF(L > 0 && !on_16_bytes(t[i]));  // (the remainder's kernel takes any alignment)
+  for (int i : {2, 8, 9, 10, 11}) NONE_IF(L > 0 && !on_16_bytes(t[i]));  // (the remainder's kernel takes any alignment)
   Dims m;
   m.dt = bf;
   m.dev = dev;
@@ -480,6 +486,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   auto must = [](int rc) {
     if (rc != TTT_OK) throw_error(rc);
   };
+  const void* const add = te_add.defined() ? te_add.const_data_ptr() : nullptr;
   const bool fused = !small && !conv && T % 128 == 0 && F == 64 && rope != 2 && mb <= 16 && lr_col % 64 == 0;
   // temporaries from one allocation, each on a 256-byte boundary
   int64_t at_ = 0;
@@ -532,7 +539,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     ttt_dims di = d;
     di.seq_len = (int32_t)L;
     must(ttt_internal_linear_infer(&di, (int)T, (int)lr_pitch, base + o_q, base + o_k, base + o_v,
-                                   sw.const_data_ptr(), sb.const_data_ptr(), te.const_data_ptr(), base + o_lr,
+                                   sw.const_data_ptr(), sb.const_data_ptr(), te.const_data_ptr(), add, base + o_lr,
                                    t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in, w.data_ptr(),
                                    b.data_ptr(), status, st));
   }
@@ -545,7 +552,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     ttt_dims dt = d;
     dt.seq_len = (int32_t)R;
     must(ttt_internal_linear_tail(&dt, (int)T, (int)L, (int)lr_pitch, small && L == 0, base + o_q, base + o_k, base + o_v,
-                                  w_in.const_data_ptr(), b_in.const_data_ptr(), te.const_data_ptr(), base + o_lr,
+                                  w_in.const_data_ptr(), b_in.const_data_ptr(), te.const_data_ptr(), add, base + o_lr,
                                   t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in,
                                   const_cast<void*>(w.const_data_ptr()), const_cast<void*>(b.const_data_ptr()),
                                   st));

@@ -29,15 +29,16 @@ int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, const void* xk,
 
 // Inference forward over the first `d->seq_len` tokens (whole mini-batches) of sequences whose rows are `seq_pitch` tokens
 // apart in xq, xk, xv, output and `lr_pitch` elements apart in ttt_lr_eta; token_eta: the first mini-batch's.
+// token_eta_add (bf16, or null): token_eta is max(token_eta + token_eta_add, 0), as the layer forms it from its parameters.
 int ttt_internal_linear_infer(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk,
                               const void* xv, const void* weight, const void* bias, const void* token_eta,
-                              const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
+                              const void* token_eta_add, const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
                               void* weight_out, void* bias_out, void* status, void* stream);
 // ttt_linear_forward_partial on tokens [first, first + d->seq_len) of such sequences.  state_settled: the launch before
 // this one on the stream was ttt_internal_layer_small_proj (the state may be read before that has finished).
 int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled, const void* xq, const void* xk,
                              const void* xv, const void* weight, const void* bias, const void* token_eta,
-                             const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
+                             const void* token_eta_add, const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
                              void* weight_out, void* bias_out, void* stream);
 // ttt_layer_prologue with rows of lr_pitch elements in ttt_lr_eta
 int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src, const void* k_src, const void* v_src,

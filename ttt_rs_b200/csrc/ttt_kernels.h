@@ -43,6 +43,7 @@ struct LinFwdParams {
   const void* w0;         // [B,H,F,F] element type T
   const void* b0;         // [B,H,F]
   const void* token_eta;  // [T], first 16 entries read
+  const void* token_eta_add;  // or null: see ld_token_eta
   const void* lr;         // [B,H,lr_ld], lr_ld elements per (batch, head): T, or more where the caller pads the rows
   const void* ln_g;       // [H,F]
   const void* ln_b;       // [H,F]
@@ -264,6 +265,7 @@ struct LinPartialParams {
   const void* w0;         // [B,H,F,F]
   const void* b0;         // [B,H,F]
   const void* token_eta;  // [R]
+  const void* token_eta_add;  // or null: see ld_token_eta
   const void* lr;         // [B,H,lr_ld]
   const void* ln_g;       // [H,F]
   const void* ln_b;

@@ -420,7 +420,6 @@ class TTT(torch.nn.Module):
         self.post_norm_weight = torch.nn.Parameter(torch.ones(hs, **kw))
         self.post_norm_bias = torch.nn.Parameter(torch.zeros(hs, **kw))
         self._wcat, self._wcat_key = None, None
-        self._te, self._te_key = None, None
         self._native_key = None
 
     # ---- one GEMM for every projection of x ----------------------------------------------------------------
@@ -456,15 +455,7 @@ class TTT(torch.nn.Module):
         return torch.cat([b.detach() for b in blocks], dim=0).contiguous(), cols
 
     def invalidate_fused_weight(self):
-        self._wcat = self._te = None
-
-    def _token_eta(self, dtype):
-        """token_eta of one mini-batch (the kernels read no further), in `dtype`; kept like the stacked weights."""
-        key = _lib.host().param_key(self.token_idx, self.learnable_token_idx), dtype
-        if self._te is None or self._te_key != key:
-            self._te_key = key
-            self._te = torch.clamp_min(self.token_idx + self.learnable_token_idx.detach(), 0.0).to(dtype)
-        return self._te
+        self._wcat = None
 
     @staticmethod
     def _project(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -515,19 +506,21 @@ class TTT(torch.nn.Module):
         # (parameters through the dictionary: attribute access on a module costs a multiple of it, and this call runs
         # once per generated token and layer)
         P, I, native = self._parameters.get, i._parameters.get, _lib.host()
-        key = native.param_key(P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj"), P("learnable_ttt_lr_weight"),
-                               self._buffers.get("token_idx"), P("learnable_token_idx"))
-        if self._native_key != key or self._wcat is None or self._te is None or self._te.dtype != x.dtype:
+        key = native.param_key(P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj"), P("learnable_ttt_lr_weight"))
+        if self._native_key != key or self._wcat is None:
             self._fused_weight()
-            self._token_eta(x.dtype)
             self._native_key = key
+        # token_eta is formed in the kernels that use it (its first mini-batch: they read no further)
+        te, te_add = self._buffers.get("token_idx"), P("learnable_token_idx")
+        if te is None or te_add is None or te.dtype != x.dtype or te_add.dtype != x.dtype:
+            te, te_add = torch.clamp_min(self.token_idx + self.learnable_token_idx, 0.0).to(x.dtype), None
         wcat, cols = self._wcat
         conv = (P("q_conv_weight"), P("q_conv_bias"), P("k_conv_weight"), P("k_conv_bias")) if c.share_qk else _NO_CONV
         r = native.layer_infer(
-            x, wcat, self._te, P("learnable_ttt_lr_bias"), *conv, state.weight, state.bias, I("ln_weight"), I("ln_bias"),
+            x, wcat, te, P("learnable_ttt_lr_bias"), *conv, state.weight, state.bias, I("ln_weight"), I("ln_bias"),
             P("post_norm_weight"), P("post_norm_bias"), P("o_proj"), c.use_gate, c.num_heads, c.mini_batch_size,
             _POS[c.pos_encoding], c.rope_theta, c.base_lr, cols["lr"], _eps_scaled(i.epsilon), inner.allow_partial,
-            inner.partial_in_place, start_idx)
+            inner.partial_in_place, start_idx, te_add)
         if r is None:
             return None
         y, state.weight, state.bias = r
