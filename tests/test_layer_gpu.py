@@ -301,3 +301,40 @@ def test_inference_forward_follows_in_place_parameter_updates(golden_dir):
     want = LO.ttt_layer_forward(p["input"], p, num_heads=2)[0]
     assert_close(y1, want, 2e-4, "layer output after in-place parameter update")
     assert (y1 - y0).abs().max().item() > 1e-3, "the update must change the output"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ("functional_call", "parametrization"))
+def test_inference_follows_weights_that_are_computed_for_the_call(how):
+    """Weights that live for one call only (another storage each time, or the same address again with other values)."""
+    import ttt_rs_b200 as tb
+    H, C = 2, 128
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H)
+    torch.manual_seed(9)
+    m = tb.TTT(cfg, device="cuda", dtype=torch.bfloat16)
+    inner = tb.new_inner(cfg, device="cuda", dtype=torch.bfloat16)
+    x = (torch.randn(2, 32, C, device="cuda") * 0.5).bfloat16()
+    base = m.q_proj.detach().clone()
+
+    class Scale(torch.nn.Module):
+        by = 1.0
+
+        def forward(self, w):
+            return w * self.by
+
+    with torch.no_grad():
+        m(x, inner, inner.init_state(2))
+        want = []
+        for by in (2.0, 4.0):
+            m.q_proj.copy_(base * by)
+            want.append(m(x, inner, inner.init_state(2)))
+        m.q_proj.copy_(base)
+        if how == "parametrization":
+            torch.nn.utils.parametrize.register_parametrization(m, "q_proj", Scale())
+        for by, w in zip((2.0, 4.0), want):
+            if how == "parametrization":
+                m.parametrizations.q_proj[0].by = by
+                y = m(x, inner, inner.init_state(2))
+            else:
+                y = torch.func.functional_call(m, {"q_proj": base * by}, (x, inner, inner.init_state(2)))
+            assert torch.equal(y, w)

@@ -419,7 +419,7 @@ class TTT(torch.nn.Module):
         self.learnable_token_idx = torch.nn.Parameter(torch.zeros(c.mini_batch_size, **kw))
         self.post_norm_weight = torch.nn.Parameter(torch.ones(hs, **kw))
         self.post_norm_bias = torch.nn.Parameter(torch.zeros(hs, **kw))
-        self._wcat, self._wcat_key = None, None
+        self._wcat, self._wcat_key, self._wcat_held = None, None, None
         self._native_key = None
 
     # ---- one GEMM for every projection of x ----------------------------------------------------------------
@@ -427,13 +427,15 @@ class TTT(torch.nn.Module):
         """Rows: q | (k) | v | (g) | lr logits (H rows), padded to a multiple of 8 rows.  The concatenation is cached
         and rebuilt whenever one of its source parameters has changed: the cache key holds each parameter's storage
         address, in-place version counter, dtype and device, so an optimizer step, `load_state_dict`, `.to()` or a
-        dtype cast all invalidate it."""
+        dtype cast all invalidate it.  The storage it was built from is held, so that no other tensor can take its
+        address.  (In-place writes through `.data` leave the version as it was: `invalidate_fused_weight`.)"""
         srcs = [w for w in (self.q_proj, self.k_proj, self.v_proj, self.g_proj) if w is not None]
         srcs.append(self.learnable_ttt_lr_weight)
         key = _lib.host().param_key(*srcs)
         if self._wcat is None or self._wcat_key != key:
             self._wcat_key = key
             self._wcat = self._stack_weights()
+            self._wcat_held = [w.detach() for w in srcs]
         return self._wcat
 
     def _stack_weights(self):
@@ -455,7 +457,7 @@ class TTT(torch.nn.Module):
         return torch.cat([b.detach() for b in blocks], dim=0).contiguous(), cols
 
     def invalidate_fused_weight(self):
-        self._wcat = None
+        self._wcat = self._wcat_held = None
 
     @staticmethod
     def _project(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -508,6 +510,10 @@ class TTT(torch.nn.Module):
         P, I, native = self._parameters.get, i._parameters.get, _lib.host()
         key = native.param_key(P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj"), P("learnable_ttt_lr_weight"))
         if self._native_key != key or self._wcat is None:
+            if any(w is not None and P(n) is not w for n, w in (
+                    ("q_proj", self.q_proj), ("k_proj", self.k_proj), ("v_proj", self.v_proj), ("g_proj", self.g_proj),
+                    ("learnable_ttt_lr_weight", self.learnable_ttt_lr_weight))):
+                return None  # (a weight that is computed at every access)
             self._fused_weight()
             self._native_key = key
         # token_eta is formed in the kernels that use it (its first mini-batch: they read no further)
