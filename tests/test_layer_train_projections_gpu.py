@@ -38,3 +38,34 @@ def test_training_step_matches_the_unfused_projections(monkeypatch, B, T, H, mb,
     for got in (fused, apart):
         for a, r in zip(got, want):
             assert (a.float() - r.float()).norm() <= 2e-2 * r.float().norm() + 1e-5
+
+
+def test_frozen_projections_cost_no_weight_product(monkeypatch):
+    import ttt_rs_b200 as tb
+    H, T, C = 3, 128, 192
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H, use_gate=True)
+    torch.manual_seed(2)
+    m = tb.TTT(cfg, device="cuda", dtype=torch.bfloat16)
+    inner = tb.new_inner(cfg, device="cuda", dtype=torch.bfloat16)
+    x = (torch.randn(2, T, C, device="cuda") * 0.5).bfloat16().requires_grad_()
+    gy = (torch.randn(2, T, C, device="cuda") * 0.1).bfloat16()
+    shapes, matmul = [], torch.matmul
+
+    def counted(a, b):
+        shapes.append((a.shape[0], b.shape[-1]))
+        return matmul(a, b)
+
+    def step():
+        shapes.clear()
+        m(x, inner, inner.init_state(2)).backward(gy)
+        g, x.grad = x.grad, None
+        return g
+
+    monkeypatch.setattr(torch, "matmul", counted)
+    N = m._stack_weights()[0].shape[0]
+    want = step()
+    assert (N, C) in shapes
+    for p in (m.q_proj, m.k_proj, m.v_proj, m.g_proj, m.learnable_ttt_lr_weight):
+        p.requires_grad_(False)
+    assert torch.equal(step(), want)
+    assert (N, C) not in shapes

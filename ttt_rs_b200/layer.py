@@ -246,6 +246,8 @@ class _ProjectionsFn(torch.autograd.Function):
         dbias = _prologue_backward(dproj, cols, cfg, start_idx, lr, dxq, dxk, dxv, dlr)
         d2 = dproj.reshape(B * T, N)
         dx = torch.matmul(d2, wcat).reshape(B, T, hs) if ctx.needs_input_grad[0] else None
+        if not any(ctx.needs_input_grad[1:6]):  # frozen projections
+            return dx, None, None, None, None, None, dbias, None, None, None, None, None
         dw = torch.matmul(d2.t(), x.reshape(B * T, hs))
         rows = lambda n, cnt: dw[cols[n]:cols[n] + cnt]  # noqa: E731
         return (dx, rows("q", hs), rows("k", hs), rows("v", hs), rows("g", hs) if "g" in cols else None,
