@@ -69,3 +69,16 @@ def test_frozen_projections_cost_no_weight_product(monkeypatch):
         p.requires_grad_(False)
     assert torch.equal(step(), want)
     assert (N, C) not in shapes
+
+
+def test_lengths_without_the_one_launch_form_stack_no_weights(monkeypatch):
+    import ttt_rs_b200 as tb
+    H, C = 2, 128
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H)
+    m = tb.TTT(cfg, device="cuda", dtype=torch.bfloat16)
+    inner = tb.new_inner(cfg, device="cuda", dtype=torch.bfloat16)
+    calls, stack = [], m._stack_weights
+    monkeypatch.setattr(m, "_stack_weights", lambda: calls.append(1) or stack())
+    for T, n in ((144, 0), (256, 1)):
+        m(torch.randn(1, T, C, device="cuda").bfloat16(), inner, inner.init_state(1)).sum().backward()
+        assert len(calls) == n

@@ -440,22 +440,21 @@ class TTT(torch.nn.Module):
             self._wcat_held = [w.detach() for w in srcs]
         return self._wcat
 
-    def _stack_weights(self):
+    def _columns(self):
+        """First row of each projection in the stacked weights = first column of it in their product."""
         c = self.config
-        blocks, cols, off = [], {}, 0
-        for name, w in (("q", self.q_proj), ("k", self.k_proj), ("v", self.v_proj), ("g", self.g_proj)):
-            if w is not None:
-                blocks.append(w)
-                cols[name] = off
-                off += w.shape[0]
+        names = ("q",) + (() if c.share_qk else ("k",)) + ("v",) + (("g",) if c.use_gate else ()) + ("lr",)
+        cols = {n: i * c.hidden_size for i, n in enumerate(names)}
+        cols.setdefault("k", cols["q"])
+        return cols
+
+    def _stack_weights(self):
+        c, cols = self.config, self._columns()
+        blocks = [w for w in (self.q_proj, self.k_proj, self.v_proj, self.g_proj) if w is not None]
         blocks.append(self.learnable_ttt_lr_weight.reshape(c.num_heads, c.hidden_size))
-        cols["lr"] = off
-        off += c.num_heads
-        pad = (-off) % 8
+        pad = (-(cols["lr"] + c.num_heads)) % 8
         if pad:
             blocks.append(torch.zeros(pad, c.hidden_size, dtype=self.q_proj.dtype, device=self.q_proj.device))
-        if "k" not in cols:
-            cols["k"] = cols["q"]
         return torch.cat([b.detach() for b in blocks], dim=0).contiguous(), cols
 
     def invalidate_fused_weight(self):
@@ -558,17 +557,16 @@ def _train_forward(self, x, inner, state, start_idx):
     B, T, _ = x.shape
     H, hs = c.num_heads, c.hidden_size
     token_eta = _TokenEtaFn.apply(self.token_idx, self.learnable_token_idx, T, x.dtype)
-    if not c.share_qk and x.dtype == torch.bfloat16 == self.q_proj.dtype:
+    if self.q_proj.dtype == torch.bfloat16 and self._can_fuse_projections(x, self._columns()):
         wcat, cols = self._stack_weights()  # (not kept: the weights change with every step)
-        if self._can_fuse_projections(x, cols):
-            grads = {}
-            xq, xk, xv, lr, gate = _ProjectionsFn.apply(
-                x, self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.learnable_ttt_lr_weight,
-                self.learnable_ttt_lr_bias, wcat, cols, c, start_idx, grads)
-            out = inner.forward(state, TTTInputsInner(Qkv(xq, xk, xv), token_eta, lr, start_idx))
-            y = _EpilogueFn.apply(out, gate, self.post_norm_weight, self.post_norm_bias, 1e-6,
-                                  grads if gate is not None else None, wcat.shape[0], cols.get("g", 0))
-            return torch.matmul(y, self.o_proj.t())
+        grads = {}
+        xq, xk, xv, lr, gate = _ProjectionsFn.apply(
+            x, self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.learnable_ttt_lr_weight,
+            self.learnable_ttt_lr_bias, wcat, cols, c, start_idx, grads)
+        out = inner.forward(state, TTTInputsInner(Qkv(xq, xk, xv), token_eta, lr, start_idx))
+        y = _EpilogueFn.apply(out, gate, self.post_norm_weight, self.post_norm_bias, 1e-6,
+                              grads if gate is not None else None, wcat.shape[0], cols.get("g", 0))
+        return torch.matmul(y, self.o_proj.t())
     if c.share_qk:
         # shared projection | v | lr logits, then the two convolutions as a step of their own (with its gradient
         # kernel); the prologue sees the usual q | k | v | lr layout
