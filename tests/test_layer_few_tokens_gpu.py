@@ -100,3 +100,19 @@ def test_token_eta_follows_its_parameters_at_every_call(T):
             assert torch.equal(a, b)
         m.token_idx, m.learnable_token_idx = idx, learnable
     assert not torch.equal(seen[0][1], seen[1][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,use_gate", ((16, 32, True), (17, 32, False), (32, 24, False), (21, 24, True), (22, 24, True),
+                                          (32, 16, True), (32, 17, True)))
+def test_either_side_of_where_the_general_form_takes_over(B, H, use_gate):
+    import ttt_rs_b200 as tb
+    x, p = _random_case(B, 1, H, 7 + H, False, use_gate, torch.bfloat16)
+    m, inner = _layer_from_params(tb, p, False, use_gate, torch.bfloat16, torch.device("cuda:0"), H)
+    inner.allow_partial = True
+    with torch.no_grad():
+        state = inner.init_state(B)
+        y = m(x.bfloat16().cuda(), inner, state, 3)
+    want, st = LO.ttt_layer_forward(x, p, num_heads=H, use_gate=use_gate, start_idx=3)
+    assert_close(y, want, 3e-2, "layer output", max_bad_frac=1e-3)
+    assert_close(state.weight, st["weight"], 2e-2, "state weight", max_bad_frac=1e-3)

@@ -480,7 +480,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   c10::cuda::CUDAGuard guard(dev);
   void* const st = m.stream();
   void* const status = m.status.data_ptr();
-  const bool small = !conv && ttt_internal_layer_small_fits(&d);
+  const bool small = !conv && ttt_internal_layer_small_fits(&d, use_gate);
   NONE_IF(small && (!on_16_bytes(t[12]) || !on_16_bytes(t[13])));
   NONE_IF(!small && N % 8 != 0);
   auto must = [](int rc) {
