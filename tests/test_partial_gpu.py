@@ -112,19 +112,23 @@ def test_layer_prefill_then_token_by_token_decode():
 
 
 @pytest.mark.gpu
-def test_decode_through_cuda_graphs_equals_eager_decode():
-    """The captured decode step (one CUDA graph per rotary phase, state advanced in place) gives the same bits as
-    calling the layer token by token, across two wraps of the rotary positions."""
+@pytest.mark.parametrize("dtype,native", ((torch.float32, False), (torch.bfloat16, False), (torch.bfloat16, True)))
+def test_decode_through_cuda_graphs_equals_eager_decode(monkeypatch, dtype, native):
+    """`DecodeGraphs` gives the same bits as calling the layer token by token, across two wraps of the rotary positions:
+    by its captured steps (one CUDA graph per rotary phase, state advanced in place), and where the native call takes
+    the layer by that call with the position reduced to its phase."""
     import ttt_rs_b200 as tb
     dev = torch.device("cuda:0")
     B, H, T0, steps = 2, 2, 16, 35
     cfg = tb.TTTLayerConfig(hidden_size=H * 64, num_heads=H, use_gate=True)
     torch.manual_seed(3)
-    layer = tb.TTT(cfg, device=dev, dtype=torch.bfloat16)
-    x = (torch.randn(B, T0 + steps, H * 64, device=dev) * 0.5).to(torch.bfloat16)
+    layer = tb.TTT(cfg, device=dev, dtype=dtype)
+    if not native:
+        monkeypatch.setattr(layer, "_infer_native", lambda *a: None)
+    x = (torch.randn(B, T0 + steps, H * 64, device=dev) * 0.5).to(dtype)
 
     def run(use_graphs):
-        inner = tb.new_inner(cfg, device=dev, dtype=torch.bfloat16, allow_partial=True, partial_in_place=True)
+        inner = tb.new_inner(cfg, device=dev, dtype=dtype, allow_partial=True, partial_in_place=True)
         with torch.no_grad():
             inner.inner.weight_init.copy_(torch.randn(H, 64, 64, generator=torch.Generator().manual_seed(1)) * 0.02)
             state = inner.init_state(B)
@@ -137,6 +141,8 @@ def test_decode_through_cuda_graphs_equals_eager_decode():
                 y = dec.step(xi, T0 + i) if use_graphs else layer(xi.contiguous(), inner, state, T0 + i)
                 outs.append(y.clone())
         torch.cuda.synchronize()
+        if use_graphs:
+            assert len(dec._graphs) == (0 if native else 16)
         return torch.cat(outs, dim=1), state.weight.clone()
 
     ye, we = run(False)
