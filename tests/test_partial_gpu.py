@@ -149,3 +149,36 @@ def test_decode_through_cuda_graphs_equals_eager_decode(monkeypatch, dtype, nati
     yg, wg = run(True)
     assert torch.equal(ye, yg), "outputs differ between eager and graph decode"
     assert torch.equal(we, wg), "state differs between eager and graph decode"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", ("in place", "replaced", "through .data"))
+def test_captured_steps_follow_the_parameters(change):
+    import ttt_rs_b200 as tb
+    B, H = 2, 2
+    C = H * 64
+    cfg = tb.TTTLayerConfig(hidden_size=C, num_heads=H)
+    torch.manual_seed(4)
+    layer = tb.TTT(cfg, device="cuda")
+    inner = tb.new_inner(cfg, device="cuda", allow_partial=True, partial_in_place=True)
+    x = torch.randn(B, 2, C, device="cuda") * 0.5
+    new = {n: torch.randn(C, C, device="cuda") * 0.02 for n in ("q_proj", "o_proj")}
+    with torch.no_grad():
+        state = inner.init_state(B)
+        dec = tb.DecodeGraphs(layer, inner, state, B)
+        dec.step(x[:, :1], 0)
+        dec.step(x[:, :1], 16)  # the captured step again
+        assert dec._graphs
+        for n, w in new.items():
+            if change == "in place":
+                getattr(layer, n).copy_(w)
+            elif change == "replaced":
+                setattr(layer, n, torch.nn.Parameter(w))
+            else:
+                getattr(layer, n).data.copy_(w)
+        if change == "through .data":
+            layer.invalidate_fused_weight()
+        other = tb.TTTLinearState(state.weight.clone(), state.bias.clone())
+        got = dec.step(x[:, 1:], 32).clone()
+        want = layer(x[:, 1:].contiguous(), inner, other, 32)
+    assert torch.equal(got, want) and torch.equal(state.weight, other.weight)

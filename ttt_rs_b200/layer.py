@@ -618,7 +618,8 @@ class DecodeGraphs:
     epilogue, output GEMM) is captured once per rotary phase as a CUDA graph: the rotary position enters the prologue
     as a scalar argument, so with positions wrapped at the mini-batch there are `mini_batch_size` distinct steps, each
     captured on first use; the input is copied to `self.x` [B, 1, hidden] and the result lands in the tensor `step`
-    returns (overwritten by the next step of the same phase)."""
+    returns (overwritten by the next step of the same phase).  The graphs read the parameters (and the stacked weights)
+    where they lay at the capture: they are captured anew once a parameter has changed or the state is another one."""
 
     def __init__(self, layer: "TTT", inner: FusedTileMultiTTTLinear, state: TTTLinearState, batch: int):
         c = layer.config
@@ -631,6 +632,7 @@ class DecodeGraphs:
         self.x = torch.zeros(batch, 1, c.hidden_size, dtype=p.dtype, device=p.device)
         self.period = c.mini_batch_size if c.pos_encoding == "rope" else 1
         self._graphs, self._outs = {}, {}
+        self._key, self._wcat = None, None
 
     def step(self, x: torch.Tensor, start_idx: int) -> torch.Tensor:
         """One token per sequence: x [B, 1, hidden] at position `start_idx`."""
@@ -640,6 +642,11 @@ class DecodeGraphs:
             if y is not None:
                 return y
         self.x.copy_(x)
+        key = (_lib.host().param_key(*self.layer._parameters.values(), *self.layer._buffers.values(),
+                                     *self.inner.inner._parameters.values()),
+               self.state.weight.data_ptr(), self.state.bias.data_ptr())
+        if key != self._key or self.layer._wcat is not self._wcat:
+            self._graphs, self._outs, self._key = {}, {}, key
         g = self._graphs.get(ph)
         if g is None:
             # warm-up run on a side stream (lazy initialisation of the libraries must happen outside the capture);
@@ -655,7 +662,7 @@ class DecodeGraphs:
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g), torch.no_grad():
                 self._outs[ph] = self.layer(self.x, self.inner, self.state, ph)
-            self._graphs[ph] = g
+            self._graphs[ph], self._wcat = g, self.layer._wcat
             # the capture itself does not execute: the state is still w0, b0 and the replay below does the step
         g.replay()
         return self._outs[ph]
