@@ -338,3 +338,58 @@ def test_inference_follows_weights_that_are_computed_for_the_call(how):
             else:
                 y = torch.func.functional_call(m, {"q_proj": base * by}, (x, inner, inner.init_state(2)))
             assert torch.equal(y, w)
+
+
+def _plain_layer(H=2, dtype=torch.bfloat16):
+    import ttt_rs_b200 as tb
+    cfg = tb.TTTLayerConfig(hidden_size=64 * H, num_heads=H)
+    torch.manual_seed(12)
+    m = tb.TTT(cfg, device="cuda", dtype=dtype)
+    inner = tb.new_inner(cfg, device="cuda", dtype=dtype)
+    x = (torch.randn(2, 32, 64 * H, device="cuda") * 0.5).to(dtype)
+    return m, lambda: m(x, inner, inner.init_state(2))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", (True, False))
+def test_another_stream_waits_for_the_stacked_weights(monkeypatch, native):
+    m, call = _plain_layer()
+    if not native:
+        monkeypatch.setattr(m, "_infer_native", lambda *a: None)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.no_grad():
+        want = call()
+        torch.cuda.synchronize()
+        m.invalidate_fused_weight()
+        with torch.cuda.stream(a):
+            torch.cuda._sleep(50_000_000)  # the weights are stacked behind about 25 ms of other work
+            call()
+        with torch.cuda.stream(b):
+            got = call()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+        assert len(m._stack.on_streams) == 2
+
+
+@pytest.mark.gpu
+def test_weights_stacked_during_a_capture_are_not_kept():
+    m, call = _plain_layer()
+    with torch.no_grad():
+        want = call()
+        m.invalidate_fused_weight()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out = call()
+        assert m._stack is None
+        g.replay()
+        assert torch.equal(out, want) and torch.equal(call(), want)
+
+
+@pytest.mark.gpu
+def test_a_layer_that_has_run_can_be_copied():
+    import copy
+    m, call = _plain_layer()
+    with torch.no_grad():
+        call()
+    c = copy.deepcopy(m)
+    assert c._stack is None and m._stack is not None and torch.equal(c.q_proj, m.q_proj)

@@ -397,12 +397,8 @@ PyObject* py_mlp_apply(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---- the outer layer, inference ------------------------------------------------------------------------------------
-// param_key(tensors...) -> bytes that change with any tensor's storage, version, dtype or device (None entries allowed)
-PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
-  PyObject* r = PyBytes_FromStringAndSize(nullptr, n * 16);
-  if (!r) return nullptr;
-  uint64_t* k = reinterpret_cast<uint64_t*>(PyBytes_AS_STRING(r));
+// tensors (None entries allowed) -> 16 bytes each that change with its storage, version, dtype or device
+void fill_key(PyObject* const* args, Py_ssize_t n, uint64_t* k) {
   for (Py_ssize_t i = 0; i < n; ++i) {
     k[2 * i] = k[2 * i + 1] = 0;
     if (!THPVariable_Check(args[i])) continue;
@@ -410,14 +406,35 @@ PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
     k[2 * i] = reinterpret_cast<uint64_t>(t.const_data_ptr());
     k[2 * i + 1] = ((uint64_t)t._version() << 16) | ((uint64_t)t.scalar_type() << 8) | (uint64_t)(uint8_t)t.device().index();
   }
+}
+// param_key(tensors...) -> their key
+PyObject* py_param_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  PyObject* r = PyBytes_FromStringAndSize(nullptr, n * 16);
+  if (r) fill_key(args, n, reinterpret_cast<uint64_t*>(PyBytes_AS_STRING(r)));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+// stream_key(device index, tensors...) -> the current stream of that device, then their key
+PyObject* py_stream_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n < 1) return arity(n, 1), nullptr;
+  const int64_t dev = as_int(args[0]);
+  if (PyErr_Occurred()) return nullptr;
+  const uint64_t st = reinterpret_cast<uint64_t>(c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  PyObject* r = PyBytes_FromStringAndSize(nullptr, 8 + (n - 1) * 16);
+  if (!r) return nullptr;
+  uint64_t* const k = reinterpret_cast<uint64_t*>(PyBytes_AS_STRING(r));
+  k[0] = st;
+  fill_key(args + 1, n - 1, k + 1);
   return r;
   END_HANDLE_TH_ERRORS
 }
 
-// layer_infer(x, stacked weights, token_eta of one mini-batch, lr_bias, conv q weight / bias, conv k weight / bias (or four
+// layer_infer(x, stacked weights, token_idx of one mini-batch, lr_bias, conv q weight / bias, conv k weight / bias (or four
 //             None), state weight, state bias, ln weight, ln bias, post norm weight, bias, o_proj, gate 0/1, heads,
 //             mini_batch, rope_mode, rope_theta, base_lr, lr_col, eps_scaled, allow_partial, in_place, start_idx,
-//             what is added to token_eta before it is clamped at zero, or None)
+//             learnable_token_idx)
 //   -> (y, state weight, state bias) | None
 // One call of TTT.forward without gradients, bf16: projections + prologue, inner loop (whole mini-batches, then the
 // remainder as a mini-batch of its own), post norm (+ gate), output projection.
@@ -432,10 +449,8 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     NONE_IF(!THPVariable_Check(args[i]));
     t[i] = THPVariable_Unpack(args[i]);
   }
-  if (args[26] != Py_None) {
-    NONE_IF(!THPVariable_Check(args[26]));
-    te_add = THPVariable_Unpack(args[26]);
-  }
+  NONE_IF(!THPVariable_Check(args[26]));
+  te_add = THPVariable_Unpack(args[26]);
   const Tensor &x = t[0], &wcat = t[1], &te = t[2], &lr_bias = t[3], &sw = t[8], &sb = t[9];
   const bool use_gate = as_int(args[15]) != 0, conv = t[4].defined();
   const int64_t H = as_int(args[16]), mb = as_int(args[17]), rope = as_int(args[18]), lr_col = as_int(args[21]);
@@ -454,7 +469,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   NONE_IF((T > 1 && B > 1 && x.stride(0) != T * x_ld) || x_ld < C || x_ld % 8 != 0);
   const int64_t N = wcat.size(0);
   NONE_IF(!is(wcat, bf, dev, {N, C}) || te.dim() != 1 || te.size(0) < mb || !is(te, bf, dev, {te.size(0)}));
-  NONE_IF(te_add.defined() && !is(te_add, bf, dev, {te.size(0)}));
+  NONE_IF(!is(te_add, bf, dev, {te.size(0)}));
   NONE_IF(lr_bias.numel() != H || lr_bias.scalar_type() != bf || !lr_bias.is_contiguous() || lr_bias.device() != dev);
   NONE_IF(!is(sw, bf, dev, {B, H, F, F}) || !is(sb, bf, dev, {B, H, F}) || !is(t[10], bf, dev, {H, F}) ||
           !is(t[11], bf, dev, {H, F}) || !is(t[12], bf, dev, {C}) || !is(t[13], bf, dev, {C}) || !is(t[14], bf, dev, {C, C}));
@@ -486,7 +501,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   auto must = [](int rc) {
     if (rc != TTT_OK) throw_error(rc);
   };
-  const void* const add = te_add.defined() ? te_add.const_data_ptr() : nullptr;
+  const void* const add = te_add.const_data_ptr();
   const bool fused = !small && !conv && T % 128 == 0 && F == 64 && rope != 2 && mb <= 16 && lr_col % 64 == 0;
   // temporaries from one allocation, each on a 256-byte boundary
   int64_t at_ = 0;
@@ -580,6 +595,7 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST(mlp_forward),
                          FAST(mlp_apply),
                          FAST(param_key),
+                         FAST(stream_key),
                          FAST(layer_infer),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

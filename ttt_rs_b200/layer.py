@@ -389,6 +389,15 @@ class _EpilogueFn(torch.autograd.Function):
         return d_inner, dg, dw.to(ln_weight.dtype), db.to(ln_bias.dtype), None, None, None, None
 
 
+class _Stack:
+    """Stacked projection weights of a layer: the key and the storage of what they were built from, the event behind the
+    building, and the key with each stream whose work is known to come behind that event."""
+    __slots__ = ("key", "wcat", "cols", "held", "ready", "on_streams")
+
+    def __init__(self, key, wcat, cols, held):
+        self.key, self.wcat, self.cols, self.held, self.ready, self.on_streams = key, wcat, cols, held, None, set()
+
+
 class TTT(torch.nn.Module):
     """Outer TTT layer.  Parameter names follow the reference (`q_proj`, `k_proj`, `v_proj`, `g_proj`, `o_proj`,
     `q_conv` / `k_conv`, `learnable_ttt_lr_weight` [H, hidden, 1], `learnable_ttt_lr_bias` [H, 1], `token_idx`,
@@ -421,24 +430,42 @@ class TTT(torch.nn.Module):
         self.learnable_token_idx = torch.nn.Parameter(torch.zeros(c.mini_batch_size, **kw))
         self.post_norm_weight = torch.nn.Parameter(torch.ones(hs, **kw))
         self.post_norm_bias = torch.nn.Parameter(torch.zeros(hs, **kw))
-        self._wcat, self._wcat_key, self._wcat_held = None, None, None
-        self._native_key = None
+        self._stack = None
+
+    def __getstate__(self):  # (copies and pickles stack their own)
+        return {**self.__dict__, "_stack": None}
 
     # ---- one GEMM for every projection of x ----------------------------------------------------------------
+    def _sources(self):
+        return self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.learnable_ttt_lr_weight
+
     def _fused_weight(self):
-        """Rows: q | (k) | v | (g) | lr logits (H rows), padded to a multiple of 8 rows.  The concatenation is cached
-        and rebuilt whenever one of its source parameters has changed: the cache key holds each parameter's storage
-        address, in-place version counter, dtype and device, so an optimizer step, `load_state_dict`, `.to()` or a
-        dtype cast all invalidate it.  The storage it was built from is held, so that no other tensor can take its
-        address.  (In-place writes through `.data` leave the version as it was: `invalidate_fused_weight`.)"""
-        srcs = [w for w in (self.q_proj, self.k_proj, self.v_proj, self.g_proj) if w is not None]
-        srcs.append(self.learnable_ttt_lr_weight)
-        key = _lib.host().param_key(*srcs)
-        if self._wcat is None or self._wcat_key != key:
-            self._wcat_key = key
-            self._wcat = self._stack_weights()
-            self._wcat_held = [w.detach() for w in srcs]
-        return self._wcat
+        """(stacked weights, their columns).  Rows: q | (k) | v | (g) | lr logits (H rows), padded to a multiple of 8 rows.
+        The concatenation is kept and rebuilt whenever one of its source parameters has changed: the key holds each
+        parameter's storage address, in-place version counter, dtype and device, so an optimizer step,
+        `load_state_dict`, `.to()` or a dtype cast all invalidate it.  The storage it was built from is held, so that no
+        other tensor can take its address.  (In-place writes through `.data` leave the version as it was:
+        `invalidate_fused_weight`.)"""
+        srcs, native = self._sources(), _lib.host()
+        key, dev = native.param_key(*srcs), self.q_proj.device
+        capturing = dev.type == "cuda" and torch.cuda.is_current_stream_capturing()
+        s = self._stack
+        if s is None or s.key != key:
+            wcat, cols = self._stack_weights()
+            if capturing:  # nothing has been computed: a part of the graph, not of this layer
+                return wcat, cols
+            s = _Stack(key, wcat, cols, [w.detach() for w in srcs if w is not None])
+            if dev.type == "cuda":
+                s.ready = torch.cuda.current_stream(dev).record_event()
+            self._stack = s
+        if dev.type == "cuda" and not capturing:  # (a capture begins behind everything that was queued)
+            here = native.stream_key(dev.index, *srcs)
+            if here not in s.on_streams:
+                cur = torch.cuda.current_stream(dev)
+                cur.wait_event(s.ready)
+                s.wcat.record_stream(cur)
+                s.on_streams.add(here)
+        return s.wcat, s.cols
 
     def _columns(self):
         """First row of each projection in the stacked weights = first column of it in their product."""
@@ -458,7 +485,7 @@ class TTT(torch.nn.Module):
         return torch.cat([b.detach() for b in blocks], dim=0).contiguous(), cols
 
     def invalidate_fused_weight(self):
-        self._wcat = self._wcat_held = None
+        self._stack = None
 
     @staticmethod
     def _project(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -503,31 +530,26 @@ class TTT(torch.nn.Module):
         c = self.config
         if type(inner) is not FusedTileMultiTTTLinear or not x.is_cuda:
             return None
-        i = inner.inner
+        # (modules and parameters through the dictionaries: attribute access on a module costs a multiple of it, and this
+        # call runs once per generated token and layer)
+        i = inner._modules["inner"]
         if i.mini_batch_size != c.mini_batch_size:
             return None
-        # (parameters through the dictionary: attribute access on a module costs a multiple of it, and this call runs
-        # once per generated token and layer)
         P, I, native = self._parameters.get, i._parameters.get, _lib.host()
-        key = native.param_key(P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj"), P("learnable_ttt_lr_weight"))
-        if self._native_key != key or self._wcat is None:
-            if any(w is not None and P(n) is not w for n, w in (
-                    ("q_proj", self.q_proj), ("k_proj", self.k_proj), ("v_proj", self.v_proj), ("g_proj", self.g_proj),
-                    ("learnable_ttt_lr_weight", self.learnable_ttt_lr_weight))):
-                return None  # (a weight that is computed at every access)
-            self._fused_weight()
-            self._native_key = key
-        # token_eta is formed in the kernels that use it (its first mini-batch: they read no further)
-        te, te_add = self._buffers.get("token_idx"), P("learnable_token_idx")
-        if te is None or te_add is None or te.dtype != x.dtype or te_add.dtype != x.dtype:
-            te, te_add = torch.clamp_min(self.token_idx + self.learnable_token_idx, 0.0).to(x.dtype), None
-        wcat, cols = self._wcat
+        srcs = P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj"), P("learnable_ttt_lr_weight")
+        s = self._stack
+        if s is not None and native.stream_key(x.get_device(), *srcs) in s.on_streams:
+            wcat, cols = s.wcat, s.cols
+        elif all(a is b for a, b in zip(srcs, self._sources())):
+            wcat, cols = self._fused_weight()
+        else:
+            return None  # (a weight that is computed at every access)
         conv = (P("q_conv_weight"), P("q_conv_bias"), P("k_conv_weight"), P("k_conv_bias")) if c.share_qk else _NO_CONV
         r = native.layer_infer(
-            x, wcat, te, P("learnable_ttt_lr_bias"), *conv, state.weight, state.bias, I("ln_weight"), I("ln_bias"),
-            P("post_norm_weight"), P("post_norm_bias"), P("o_proj"), c.use_gate, c.num_heads, c.mini_batch_size,
+            x, wcat, self._buffers.get("token_idx"), P("learnable_ttt_lr_bias"), *conv, state.weight, state.bias,
+            I("ln_weight"), I("ln_bias"), P("post_norm_weight"), P("post_norm_bias"), P("o_proj"), c.use_gate, c.num_heads, c.mini_batch_size,
             _POS[c.pos_encoding], c.rope_theta, c.base_lr, cols["lr"], _eps_scaled(i.epsilon), inner.allow_partial,
-            inner.partial_in_place, start_idx, te_add)
+            inner.partial_in_place, start_idx, P("learnable_token_idx"))
         if r is None:
             return None
         y, state.weight, state.bias = r
@@ -632,7 +654,7 @@ class DecodeGraphs:
         self.x = torch.zeros(batch, 1, c.hidden_size, dtype=p.dtype, device=p.device)
         self.period = c.mini_batch_size if c.pos_encoding == "rope" else 1
         self._graphs, self._outs = {}, {}
-        self._key, self._wcat = None, None
+        self._key, self._stack = None, None
 
     def step(self, x: torch.Tensor, start_idx: int) -> torch.Tensor:
         """One token per sequence: x [B, 1, hidden] at position `start_idx`."""
@@ -645,7 +667,7 @@ class DecodeGraphs:
         key = (_lib.host().param_key(*self.layer._parameters.values(), *self.layer._buffers.values(),
                                      *self.inner.inner._parameters.values()),
                self.state.weight.data_ptr(), self.state.bias.data_ptr())
-        if key != self._key or self.layer._wcat is not self._wcat:
+        if key != self._key or self.layer._stack is not self._stack:
             self._graphs, self._outs, self._key = {}, {}, key
         g = self._graphs.get(ph)
         if g is None:
@@ -662,7 +684,7 @@ class DecodeGraphs:
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g), torch.no_grad():
                 self._outs[ph] = self.layer(self.x, self.inner, self.state, ph)
-            self._graphs[ph], self._wcat = g, self.layer._wcat
+            self._graphs[ph], self._stack = g, self.layer._stack
             # the capture itself does not execute: the state is still w0, b0 and the replay below does the step
         g.replay()
         return self._outs[ph]
