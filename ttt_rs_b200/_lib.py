@@ -83,7 +83,7 @@ SYMBOLS = {
 INTERNAL = {
     "ttt_internal_layer_projections": (C.c_int, [_DP, _P, C.c_int64, C.c_int64, _P, C.c_int64, C.c_int64, C.c_int64,
                                                  C.c_int64, C.c_int64, C.c_int64, C.c_int64, _P, C.c_int, C.c_int,
-                                                 C.c_float, C.c_float, C.c_int, _P, _P, _P, _P, _P, _P, _P]),
+                                                 C.c_float, C.c_float, C.c_int] + [_P] * 10),
 }
 
 NOALLOC_SCRATCH_BYTES = 32 << 20  # TTT_NOALLOC_SCRATCH_BYTES

@@ -170,6 +170,12 @@ int check_ptrs(const NamedPtr* ptrs, int n) {
   return TTT_OK;
 }
 
+ttt::TokenEtaParams token_eta_params(const ttt_dims* d, const void* idx, const void* learnable, void* out) {
+  ttt::TokenEtaParams e{idx, learnable, out, 0};
+  if (idx != nullptr && learnable != nullptr && out != nullptr && d->dtype == TTT_BF16) e.n = d->mini_batch < 16 ? d->mini_batch : 16;
+  return e;
+}
+
 int64_t num_ckpt(const ttt_dims* d) {
   const int64_t ns = d->seq_len / d->mini_batch;
   return (ns + d->checkpoint_interval - 1) / d->checkpoint_interval;
@@ -284,8 +290,9 @@ int ttt_gemm_bf16_tn(int64_t m, int64_t n, int64_t k, const void* a, int64_t lda
 int ttt_internal_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_t hidden, const void* weights,
                                    int64_t w_ld, int64_t w_rows, int64_t q_col, int64_t k_col, int64_t v_col, int64_t g_col,
                                    int64_t lr_col, const void* lr_bias, int start_idx, int rope_mode, float rope_theta,
-                                   float base_lr, int round_proj, void* xq, void* xk, void* xv, void* gate,
-                                   void* ttt_lr_eta, void* status, void* stream) {
+                                   float base_lr, int round_proj, const void* token_idx, const void* learnable_token_idx,
+                                   void* token_eta_out, void* xq, void* xk, void* xv, void* gate, void* ttt_lr_eta,
+                                   void* status, void* stream) {
   if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
   if (d->batch <= 0 || d->heads <= 0 || d->seq_len <= 0) return fail(TTT_ERR_SHAPE, "batch, heads, seq_len must be positive");
   if (d->dtype != TTT_BF16 || d->head_dim != 64)
@@ -339,6 +346,7 @@ int ttt_internal_layer_projections(const ttt_dims* d, const void* x, int64_t x_l
   p.f.start_idx = start_idx; p.f.pos_mod = rope_mode == 1 ? d->mini_batch : 1; p.f.rope_mode = rope_mode;
   p.f.rope_theta = rope_mode == 1 ? rope_theta : 1.f; p.f.base_lr = base_lr;
   p.f.lr_bias = lr_bias; p.f.lr_out = ttt_lr_eta; p.f.round_proj = round_proj;
+  p.f.te = token_eta_params(d, token_idx, learnable_token_idx, token_eta_out);
   cudaError_t e = ttt::launch_gemm_bf16_tn(maps, p, true, pair, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "fused projection launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
@@ -349,8 +357,8 @@ int ttt_layer_projections(const ttt_dims* d, const void* x, int64_t x_ld, int64_
                           float base_lr, void* xq, void* xk, void* xv, void* gate, void* ttt_lr_eta, void* status,
                           void* stream) {
   return ttt_internal_layer_projections(d, x, x_ld, hidden, weights, w_ld, w_rows, q_col, k_col, v_col, g_col, lr_col,
-                                        lr_bias, start_idx, rope_mode, rope_theta, base_lr, 0, xq, xk, xv, gate, ttt_lr_eta,
-                                        status, stream);
+                                        lr_bias, start_idx, rope_mode, rope_theta, base_lr, 0, nullptr, nullptr, nullptr, xq, xk,
+                                        xv, gate, ttt_lr_eta, status, stream);
 }
 
 void ttt_b200_debug_handoff(uint32_t poll_limit, int32_t first_item) {
@@ -372,9 +380,9 @@ size_t ttt_linear_bias_ckpt_bytes(const ttt_dims* d) {
 }
 
 static int linear_forward_impl(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk, const void* xv, const void* weight,
-                       const void* bias, const void* token_eta, const void* token_eta_add, const void* ttt_lr_eta,
-                       const void* ln_weight, const void* ln_bias, void* output, void* weight_out, void* bias_out,
-                       void* weight_ckpt, void* bias_ckpt, void* status, void* stream) {
+                       const void* bias, const void* token_eta, const void* ttt_lr_eta, const void* ln_weight,
+                       const void* ln_bias, void* output, void* weight_out, void* bias_out, void* weight_ckpt,
+                       void* bias_ckpt, void* status, void* stream) {
   int rc = check_dims(d, true);
   if (rc != TTT_OK) return rc;
   const NamedPtr ptrs[] = {{"xq", xq},           {"xk", xk},
@@ -409,7 +417,6 @@ static int linear_forward_impl(const ttt_dims* d, int seq_pitch, int lr_pitch, c
   p.w0 = weight;
   p.b0 = bias;
   p.token_eta = token_eta;
-  p.token_eta_add = token_eta_add;
   p.lr = ttt_lr_eta;
   p.ln_g = ln_weight;
   p.ln_b = ln_bias;
@@ -438,23 +445,21 @@ int ttt_linear_forward(const ttt_dims* d, const void* xq, const void* xk, const 
                        const void* ln_bias, void* output, void* weight_out, void* bias_out, void* weight_ckpt,
                        void* bias_ckpt, void* status, void* stream) {
   const int T = d != nullptr ? d->seq_len : 0;
-  return linear_forward_impl(d, T, T, xq, xk, xv, weight, bias, token_eta, nullptr, ttt_lr_eta, ln_weight, ln_bias, output,
+  return linear_forward_impl(d, T, T, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, output,
                              weight_out, bias_out, weight_ckpt, bias_ckpt, status, stream);
 }
 
 int ttt_internal_linear_infer(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk,
                               const void* xv, const void* weight, const void* bias, const void* token_eta,
-                              const void* token_eta_add, const void* ttt_lr_eta, const void* ln_weight,
-                              const void* ln_bias, void* output, void* weight_out, void* bias_out, void* status,
-                              void* stream) {
+                              const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias, void* output,
+                              void* weight_out, void* bias_out, void* status, void* stream) {
   if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
-  if (token_eta_add != nullptr && d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "token_eta_add is bf16 only");
   if (seq_pitch < d->seq_len || lr_pitch < d->seq_len || (int64_t)lr_pitch * (d->dtype == TTT_BF16 ? 2 : 4) % 16 != 0)
     return fail(TTT_ERR_SHAPE, "pitches must cover the sequence, learning-rate rows start on 16 bytes");
   if ((int64_t)d->batch * d->heads * seq_pitch >= (int64_t)1 << 31)
     return fail(TTT_ERR_SHAPE, "batch*heads*seq_pitch must be below 2^31");
-  return linear_forward_impl(d, seq_pitch, lr_pitch, xq, xk, xv, weight, bias, token_eta, token_eta_add, ttt_lr_eta,
-                             ln_weight, ln_bias, output, weight_out, bias_out, nullptr, nullptr, status, stream);
+  return linear_forward_impl(d, seq_pitch, lr_pitch, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias,
+                             output, weight_out, bias_out, nullptr, nullptr, status, stream);
 }
 
 size_t ttt_linear_backward_workspace_bytes(const ttt_dims* d) {
@@ -741,8 +746,9 @@ extern "C" int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src,
                                   int64_t src_ld, const void* lr_logits, int64_t lr_ld, const void* lr_bias,
                                   const void* conv_q_weight, const void* conv_q_bias, const void* conv_k_weight,
                                   const void* conv_k_bias, int conv_kernel, int start_idx, int rope_mode,
-                                  float rope_theta, float base_lr, void* xq, void* xk, void* xv, void* ttt_lr_eta,
-                                  int lr_pitch, void* stream) {
+                                  float rope_theta, float base_lr, const void* token_idx,
+                                  const void* learnable_token_idx, void* token_eta_out, void* xq, void* xk, void* xv,
+                                  void* ttt_lr_eta, int lr_pitch, void* stream) {
   int rc = check_layer_dims(d);
   if (rc != TTT_OK) return rc;
   const bool conv = conv_q_weight != nullptr;
@@ -787,6 +793,7 @@ extern "C" int ttt_internal_layer_prologue(const ttt_dims* d, const void* q_src,
   p.rope_mode = rope_mode;
   p.rope_theta = rope_mode != 0 ? rope_theta : 1.f;
   p.base_lr = base_lr;
+  p.te = token_eta_params(d, token_idx, learnable_token_idx, token_eta_out);
   cudaError_t e = ttt::launch_layer_prologue(d->dtype, d->head_dim, p, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "layer prologue launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
@@ -800,7 +807,8 @@ extern "C" int ttt_layer_prologue(const ttt_dims* d, const void* q_src, const vo
                                   void* stream) {
   return ttt_internal_layer_prologue(d, q_src, k_src, v_src, src_ld, lr_logits, lr_ld, lr_bias, conv_q_weight,
                                      conv_q_bias, conv_k_weight, conv_k_bias, conv_kernel, start_idx, rope_mode,
-                                     rope_theta, base_lr, xq, xk, xv, ttt_lr_eta, d != nullptr ? d->seq_len : 0, stream);
+                                     rope_theta, base_lr, nullptr, nullptr, nullptr, xq, xk, xv, ttt_lr_eta,
+                                     d != nullptr ? d->seq_len : 0, stream);
 }
 
 extern "C" int ttt_layer_epilogue(const ttt_dims* d, const void* inner_out, const void* gate, int64_t gate_ld,
@@ -836,13 +844,11 @@ extern "C" int ttt_layer_epilogue(const ttt_dims* d, const void* inner_out, cons
   return TTT_OK;
 }
 
-extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled,
-                                        const void* xq, const void* xk, const void* xv, const void* weight,
-                                        const void* bias, const void* token_eta, const void* token_eta_add,
-                                        const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
-                                        void* output, void* weight_out, void* bias_out, void* stream) {
+extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int first, int lr_pitch, int state_settled, const void* xq, const void* xk, const void* xv,
+                                          const void* weight, const void* bias, const void* token_eta,
+                                          const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
+                                          void* output, void* weight_out, void* bias_out, void* stream) {
   if (d == nullptr) return fail(TTT_ERR_NULL, "dims is null");
-  if (token_eta_add != nullptr && d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "token_eta_add is bf16 only");
   if (d->batch <= 0 || d->heads <= 0) return fail(TTT_ERR_SHAPE, "batch and heads must be positive");
   if (d->dtype != TTT_F32 && d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "unknown dtype %d", d->dtype);
   if (d->head_dim != 64 && d->head_dim != 32)
@@ -863,7 +869,6 @@ extern "C" int ttt_internal_linear_tail(const ttt_dims* d, int seq_pitch, int fi
   p.w0 = weight;
   p.b0 = bias;
   p.token_eta = token_eta;
-  p.token_eta_add = token_eta_add;
   p.lr = ttt_lr_eta;
   p.ln_g = ln_weight;
   p.ln_b = ln_bias;
@@ -887,8 +892,8 @@ extern "C" int ttt_linear_forward_partial(const ttt_dims* d, const void* xq, con
                                           const void* ttt_lr_eta, const void* ln_weight, const void* ln_bias,
                                           void* output, void* weight_out, void* bias_out, void* stream) {
   const int T = d != nullptr ? d->seq_len : 0;
-  return ttt_internal_linear_tail(d, T, 0, T, 0, xq, xk, xv, weight, bias, token_eta, nullptr, ttt_lr_eta, ln_weight,
-                                  ln_bias, output, weight_out, bias_out, stream);
+  return ttt_internal_linear_tail(d, T, 0, T, 0, xq, xk, xv, weight, bias, token_eta, ttt_lr_eta, ln_weight, ln_bias, output,
+                                  weight_out, bias_out, stream);
 }
 
 extern "C" int ttt_internal_layer_small_fits(const ttt_dims* d, int gate) {
@@ -899,7 +904,8 @@ extern "C" int ttt_internal_layer_small_fits(const ttt_dims* d, int gate) {
 
 extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, int64_t x_ld, const void* weights,
                                              int64_t w_ld, int w_rows, int lr_col, const void* lr_bias, int start_idx,
-                                             int rope_mode, float rope_theta, float base_lr, void* xq, void* xk,
+                                             int rope_mode, float rope_theta, float base_lr, const void* token_idx,
+                                             const void* learnable_token_idx, void* token_eta_out, void* xq, void* xk,
                                              void* xv, void* gate, void* ttt_lr_eta, int lr_pitch, void* stream) {
   if (!ttt_internal_layer_small_fits(d, gate != nullptr)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
   if (const int rc = check_rotation(d, start_idx, rope_mode, rope_theta); rc != TTT_OK) return rc;
@@ -913,6 +919,7 @@ extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, i
   p.H = d->heads; p.F = d->head_dim; p.T = d->seq_len; p.lr_col = lr_col; p.lr_ld = lr_pitch;
   p.start_idx = start_idx; p.pos_mod = rope_mode == 1 ? d->mini_batch : 1; p.rope_mode = rope_mode;
   p.rope_theta = rope_mode != 0 ? rope_theta : 1.f; p.base_lr = base_lr;
+  p.te = token_eta_params(d, token_idx, learnable_token_idx, token_eta_out);
   cudaError_t e = ttt::launch_layer_small_proj(p, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "few-token projection launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;

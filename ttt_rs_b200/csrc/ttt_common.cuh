@@ -319,18 +319,6 @@ template <>
 __device__ __forceinline__ float ld_as_float<__nv_bfloat16>(const void* base, size_t idx) {
   return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[idx]);
 }
-// token_eta of position i in the mini-batch: te[i], or with `add` (bf16 only) max(te[i] + add[i], 0), the sum rounded to T
-// as an addition of its own would leave it
-template <typename T>
-__device__ __forceinline__ float ld_token_eta(const void* te, const void* add, int i) {
-  float v = ld_as_float<T>(te, (size_t)i);
-  if constexpr (sizeof(T) == 2)
-    if (add != nullptr) {
-      v = __bfloat162float(__float2bfloat16_rn(v + ld_as_float<T>(add, (size_t)i)));
-      if (v < 0.f) v = 0.f;  // (a NaN stays one)
-    }
-  return v;
-}
 template <typename T>
 __device__ __forceinline__ void st_from_float(void* base, size_t idx, float v);
 template <>
@@ -377,6 +365,25 @@ __device__ __forceinline__ void tmem_st_8x4(uint32_t taddr, const float (&r)[8][
 }
 
 // ---- programmatic dependent launch ------------------------------------------------------------------------------
+// One element of TokenEtaParams, in two halves with the kernel's own work between them (the loads are on their way during it)
+struct TokenEtaElement {
+  __nv_bfloat16 a, b;
+  template <class P>
+  __device__ __forceinline__ void load(const P& p, int i) {
+    if (i < p.n) {
+      a = static_cast<const __nv_bfloat16*>(p.idx)[i];
+      b = static_cast<const __nv_bfloat16*>(p.learnable)[i];
+    }
+  }
+  template <class P>
+  __device__ __forceinline__ void store(const P& p, int i) const {
+    if (i < p.n) {  // the sum rounded as an addition of its own would leave it; a NaN stays one
+      const float s = __bfloat162float(__float2bfloat16_rn(__bfloat162float(a) + __bfloat162float(b)));
+      static_cast<__nv_bfloat16*>(p.out)[i] = __float2bfloat16_rn(s < 0.f ? 0.f : s);
+    }
+  }
+};
+
 // A kernel launched with launch_dependent may begin while the kernel before it on the stream drains: its launch and
 // prologue (and loads of data that neither the kernel before nor an unfinished one writes) are off the chain.
 // pdl_wait: everything before on the stream is complete and visible.  pdl_go: the next kernel may begin; called after

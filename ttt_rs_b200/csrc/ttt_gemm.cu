@@ -374,6 +374,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int q = warp & 3;
     const int row = 32 * q + lane;
     const float2* rope_tab = reinterpret_cast<const float2*>(gbase + SM::OFF_ROPE);
+    if (FUSED && blockIdx.x == 0) {  // (while the first tile's products run)
+      TokenEtaElement te;
+      te.load(p.f.te, tid - 64);
+      te.store(p.f.te, tid - 64);
+    }
     if (FUSED && p.f.rope_mode == 1) {
       // (cos, sin) of position x pair, positions taken modulo the mini-batch length (at most 16 here)
       const float log2_theta = log2f(p.f.rope_theta);

@@ -451,7 +451,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   NONE_IF(!THPVariable_Check(args[26]));
   te_add = THPVariable_Unpack(args[26]);
-  const Tensor &x = t[0], &wcat = t[1], &te = t[2], &lr_bias = t[3], &sw = t[8], &sb = t[9];
+  const Tensor &x = t[0], &wcat = t[1], &te_idx = t[2], &lr_bias = t[3], &sw = t[8], &sb = t[9];
   const bool use_gate = as_int(args[15]) != 0, conv = t[4].defined();
   const int64_t H = as_int(args[16]), mb = as_int(args[17]), rope = as_int(args[18]), lr_col = as_int(args[21]);
   const float theta = (float)PyFloat_AsDouble(args[19]), base_lr = (float)PyFloat_AsDouble(args[20]);
@@ -468,8 +468,8 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int64_t x_ld = T > 1 ? x.stride(1) : x.stride(0);
   NONE_IF((T > 1 && B > 1 && x.stride(0) != T * x_ld) || x_ld < C || x_ld % 8 != 0);
   const int64_t N = wcat.size(0);
-  NONE_IF(!is(wcat, bf, dev, {N, C}) || te.dim() != 1 || te.size(0) < mb || !is(te, bf, dev, {te.size(0)}));
-  NONE_IF(!is(te_add, bf, dev, {te.size(0)}));
+  NONE_IF(!is(wcat, bf, dev, {N, C}) || te_idx.dim() != 1 || te_idx.size(0) < mb ||
+          !is(te_idx, bf, dev, {te_idx.size(0)}) || !is(te_add, bf, dev, {te_idx.size(0)}));
   NONE_IF(lr_bias.numel() != H || lr_bias.scalar_type() != bf || !lr_bias.is_contiguous() || lr_bias.device() != dev);
   NONE_IF(!is(sw, bf, dev, {B, H, F, F}) || !is(sb, bf, dev, {B, H, F}) || !is(t[10], bf, dev, {H, F}) ||
           !is(t[11], bf, dev, {H, F}) || !is(t[12], bf, dev, {C}) || !is(t[13], bf, dev, {C}) || !is(t[14], bf, dev, {C, C}));
@@ -484,7 +484,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   NONE_IF(R > 16 || (R != 0 && !allow_partial));
   NONE_IF(L > 0 && ((mb != 16 && mb != 8) || (F == 32 && H % 2 != 0)));
   for (int i : {0, 1, 14}) NONE_IF(!on_16_bytes(t[i]));
-  for (int i : {2, 8, 9, 10, 11}) NONE_IF(L > 0 && !on_16_bytes(t[i]));  // (the remainder's kernel takes any alignment)
+  for (int i : {8, 9, 10, 11}) NONE_IF(L > 0 && !on_16_bytes(t[i]));  // (the remainder's kernel takes any alignment)
   Dims m;
   m.dt = bf;
   m.dev = dev;
@@ -501,7 +501,6 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   auto must = [](int rc) {
     if (rc != TTT_OK) throw_error(rc);
   };
-  const void* const add = te_add.const_data_ptr();
   const bool fused = !small && !conv && T % 128 == 0 && F == 64 && rope != 2 && mb <= 16 && lr_col % 64 == 0;
   // temporaries from one allocation, each on a 256-byte boundary
   int64_t at_ = 0;
@@ -511,28 +510,33 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return o;
   };
   const int64_t lr_pitch = (T + 7) & ~(int64_t)7;
-  const int64_t o_q = room(M * C), o_k = room(M * C), o_v = room(M * C), o_lr = room(B * H * lr_pitch), o_in = room(M * C);
+  const int64_t o_q = room(M * C), o_k = room(M * C), o_v = room(M * C), o_lr = room(B * H * lr_pitch), o_in = room(M * C),
+                o_te = room(16);
   const int64_t o_proj = small || fused ? 0 : room(M * N);
   const int64_t o_gate = use_gate && (small || fused) ? room(M * C) : 0;
   const int64_t o_y = small ? 0 : room(M * C);
   Tensor tmp = at::empty({at_}, m.opt(at::kByte));
   uint8_t* const base = static_cast<uint8_t*>(tmp.data_ptr());
   Tensor y = at::empty({B, T, C}, m.opt());
+  const void* const idx = te_idx.const_data_ptr();
+  const void* const learnable = te_add.const_data_ptr();
+  void* const te = base + o_te;
   const uint8_t* gate = nullptr;
   int64_t gate_ld = C;
   const int64_t g_col = lr_col - C;
-  // ---- projections, head split, rotary embedding, learning rates
+  // ---- projections, head split, rotary embedding, learning rates, token_eta
   if (small) {
     NONE_IF(ttt_internal_layer_small_proj(&d, x.const_data_ptr(), x_ld, wcat.const_data_ptr(), C, (int)N, (int)lr_col,
-                                          lr_bias.const_data_ptr(), (int)start, (int)rope, theta, base_lr, base + o_q,
-                                          base + o_k, base + o_v, use_gate ? base + o_gate : nullptr, base + o_lr,
+                                          lr_bias.const_data_ptr(), (int)start, (int)rope, theta, base_lr, idx, learnable, te,
+                                          base + o_q, base + o_k, base + o_v, use_gate ? base + o_gate : nullptr, base + o_lr,
                                           (int)lr_pitch, st) != TTT_OK);
     if (use_gate) gate = base + o_gate;
   } else if (fused) {
-    NONE_IF(ttt_layer_projections(&d, x.const_data_ptr(), x_ld, C, wcat.const_data_ptr(), C, N, 0, C, 2 * C,
-                                  use_gate ? g_col : -1, lr_col, lr_bias.const_data_ptr(), (int)start, (int)rope, theta,
-                                  base_lr, base + o_q, base + o_k, base + o_v, use_gate ? base + o_gate : nullptr,
-                                  base + o_lr, status, st) != TTT_OK);
+    NONE_IF(ttt_internal_layer_projections(&d, x.const_data_ptr(), x_ld, C, wcat.const_data_ptr(), C, N, 0, C, 2 * C,
+                                           use_gate ? g_col : -1, lr_col, lr_bias.const_data_ptr(), (int)start,
+                                           (int)rope, theta, base_lr, 0, idx, learnable, te, base + o_q, base + o_k,
+                                           base + o_v, use_gate ? base + o_gate : nullptr, base + o_lr, status,
+                                           st) != TTT_OK);
     if (use_gate) gate = base + o_gate;
   } else {
     uint8_t* const proj = base + o_proj;
@@ -542,8 +546,8 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
                                      lr_bias.const_data_ptr(), conv ? t[4].const_data_ptr() : nullptr,
                                      conv ? t[5].const_data_ptr() : nullptr, conv ? t[6].const_data_ptr() : nullptr,
                                      conv ? t[7].const_data_ptr() : nullptr, conv_k, (int)start, (int)rope, theta,
-                                     base_lr, base + o_q, base + o_k, base + o_v, base + o_lr, (int)lr_pitch,
-                                     st));
+                                     base_lr, idx, learnable, te, base + o_q, base + o_k, base + o_v, base + o_lr,
+                                     (int)lr_pitch, st));
     if (use_gate) gate = proj + 2 * g_col, gate_ld = N;
   }
   // ---- inner loop
@@ -554,7 +558,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     ttt_dims di = d;
     di.seq_len = (int32_t)L;
     must(ttt_internal_linear_infer(&di, (int)T, (int)lr_pitch, base + o_q, base + o_k, base + o_v,
-                                   sw.const_data_ptr(), sb.const_data_ptr(), te.const_data_ptr(), add, base + o_lr,
+                                   sw.const_data_ptr(), sb.const_data_ptr(), te, base + o_lr,
                                    t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in, w.data_ptr(),
                                    b.data_ptr(), status, st));
   }
@@ -567,7 +571,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     ttt_dims dt = d;
     dt.seq_len = (int32_t)R;
     must(ttt_internal_linear_tail(&dt, (int)T, (int)L, (int)lr_pitch, small && L == 0, base + o_q, base + o_k, base + o_v,
-                                  w_in.const_data_ptr(), b_in.const_data_ptr(), te.const_data_ptr(), add, base + o_lr,
+                                  w_in.const_data_ptr(), b_in.const_data_ptr(), te, base + o_lr,
                                   t[10].const_data_ptr(), t[11].const_data_ptr(), base + o_in,
                                   const_cast<void*>(w.const_data_ptr()), const_cast<void*>(b.const_data_ptr()),
                                   st));

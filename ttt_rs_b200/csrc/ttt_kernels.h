@@ -43,7 +43,6 @@ struct LinFwdParams {
   const void* w0;         // [B,H,F,F] element type T
   const void* b0;         // [B,H,F]
   const void* token_eta;  // [T], first 16 entries read
-  const void* token_eta_add;  // or null: see ld_token_eta
   const void* lr;         // [B,H,lr_ld], lr_ld elements per (batch, head): T, or more where the caller pads the rows
   const void* ln_g;       // [H,F]
   const void* ln_b;       // [H,F]
@@ -125,6 +124,13 @@ struct MlpFwdParams {
   int H, T, NS;
   float eps;
 };
+// token_eta of one mini-batch as the layer forms it from its parameters (bf16), written by the kernel that writes the
+// learning rates: out[i] = max(idx[i] + learnable[i], 0).  n = 0: not asked for.
+struct TokenEtaParams {
+  const void *idx, *learnable;
+  void* out;
+  int n;
+};
 // Outer-layer steps either side of the inner loop (ttt_layer.cu).
 struct LayerProParams {
   const void* q_src;   // projection outputs, rows = tokens (b*T + t), this head-major column block of H*F columns;
@@ -145,6 +151,7 @@ struct LayerProParams {
   void* lr_out;        // [B,H,lr_ld_out] (lr_ld_out >= T)
   int lr_ld_out;
   int tchunk;          // tokens per warp task, set by the launcher
+  TokenEtaParams te;   // (bf16)
   int B, H, T;
   int start_idx, pos_mod, rope_mode;  // rope_mode: 0 none, 1 positions modulo pos_mod, 2 global positions
   float rope_theta, base_lr;
@@ -179,6 +186,7 @@ struct SmallProjParams {
   int M, N, K, ldw, H, F, T, lr_col, lr_ld;
   int start_idx, pos_mod, rope_mode;
   float rope_theta, base_lr;
+  TokenEtaParams te;
 };
 struct SmallOutParams {
   const void* inner_out;  // [B,H,T,F]
@@ -272,7 +280,6 @@ struct LinPartialParams {
   const void* w0;         // [B,H,F,F]
   const void* b0;         // [B,H,F]
   const void* token_eta;  // [R]
-  const void* token_eta_add;  // or null: see ld_token_eta
   const void* lr;         // [B,H,lr_ld]
   const void* ln_g;       // [H,F]
   const void* ln_b;
@@ -351,6 +358,7 @@ struct GemmFuse {
   float rope_theta, base_lr;
   const void* lr_bias;      // [H] bf16 or null
   void* lr_out;             // ttt_lr_eta [B,H,T] bf16
+  TokenEtaParams te;
 };
 struct GemmParams {
   int M, N, K;

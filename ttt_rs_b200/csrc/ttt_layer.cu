@@ -79,6 +79,8 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
   const bool rope = p.rope_mode != 0;
   const bool rope_wrap = p.rope_mode == 1;
   const float log2_theta = log2f(p.rope_theta);
+  TokenEtaElement te;
+  if (sizeof(T) == 2 && blockIdx.x == 0) te.load(p.te, tid);
   if (rope && rope_wrap) {
     for (int e = tid; e < p.pos_mod * 32; e += PRO_THREADS) {
       const int pos = e >> 5, i = e & 31;
@@ -88,6 +90,7 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
       rope_tab[pos][i] = make_float2(c, s);
     }
   }
+  if (sizeof(T) == 2 && blockIdx.x == 0) te.store(p.te, tid);
   __syncthreads();
 
   const int hq = lane / SUBS, sub = lane % SUBS;

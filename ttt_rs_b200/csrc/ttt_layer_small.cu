@@ -62,7 +62,8 @@ __device__ __forceinline__ float2 tile_sum(float* red, const float (&acc)[MT][NT
   return s;
 }
 
-// Projections: x [M, K] . w[N, K]^T with the head split, the rotary rotation and the learning-rate gate on the way out.
+// Projections: x [M, K] . w[N, K]^T with the head split, the rotary rotation and the learning-rate gate on the way out;
+// token_eta by the first block.
 template <int MT>
 __global__ void __launch_bounds__(SM_THREADS) ttt_layer_small_proj_kernel(const SmallProjParams p) {
   constexpr int NT = 2;
@@ -75,6 +76,8 @@ __global__ void __launch_bounds__(SM_THREADS) ttt_layer_small_proj_kernel(const 
   float acc[MT][NT][4] = {};
   pdl_wait();
   pdl_go();
+  TokenEtaElement te;
+  if (blockIdx.x == 0) te.load(p.te, tid);
 #pragma unroll 4
   for (int k = warp * 32 + 8 * t; k < p.K; k += SM_WARPS * 32) {
     uint4 a[MT][2], b[NT];
@@ -92,6 +95,7 @@ __global__ void __launch_bounds__(SM_THREADS) ttt_layer_small_proj_kernel(const 
       }
     slice_mma(acc, a, b);
   }
+  if (blockIdx.x == 0) te.store(p.te, tid);
   const int C = p.H * p.F;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) {

@@ -162,9 +162,8 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
   }
   // (MB = 8: rows 8..15 of every tile are padding -- zero K, Q, V, lr and token_eta, so they neither move the state
   // nor reach the output, and nothing of them is stored)
-  const float te_row[2] = {ld_token_eta<T>(p.token_eta, p.token_eta_add, g),
-                           MB == CS ? ld_token_eta<T>(p.token_eta, p.token_eta_add, g + 8) : 0.f};
-  const float te15 = ld_token_eta<T>(p.token_eta, p.token_eta_add, MB - 1);
+  const float te_row[2] = {ld_as_float<T>(p.token_eta, g), MB == CS ? ld_as_float<T>(p.token_eta, g + 8) : 0.f};
+  const float te15 = ld_as_float<T>(p.token_eta, MB - 1);
   // The state is carried as What = W / wscale with wscale = -te15, so that the update W -= te15 Gp^T K becomes
   // What += Gp^T K, accumulated by the tensor cores straight into the registers.  (te15 == 0: W never changes.)
   const bool w_moves = (te15 != 0.f);

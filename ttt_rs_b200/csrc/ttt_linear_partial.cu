@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(32 * PT_WARPS) ttt_linear_partial_kernel(const
   }
   if (tid < r) {
     sm.lr[tid] = ld_as_float<T>(p.lr, (size_t)stream * p.lr_ld + p.row_off + tid);
-    sm.te[tid] = ld_token_eta<T>(p.token_eta, p.token_eta_add, tid);
+    sm.te[tid] = ld_as_float<T>(p.token_eta, (size_t)tid);
   }
   float bias[NC], gam[NC], bet[NC], v[RW][NC];
   ld_cols<T, VEC>(p.b0, (size_t)stream * FD + c0, bias);

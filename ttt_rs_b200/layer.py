@@ -171,8 +171,8 @@ def layer_projections(x: torch.Tensor, wcat: torch.Tensor, cols, cfg: TTTLayerCo
         _lib.check(lib.ttt_internal_layer_projections(
             C.byref(d), _ptr(x2), x2.stride(0), hidden, _ptr(wcat), wcat.stride(0), wcat.shape[0], cols["q"], cols["k"],
             cols["v"], cols.get("g", -1), cols["lr"], _ptr(bias), start_idx, _POS[cfg.pos_encoding], cfg.rope_theta,
-            cfg.base_lr, int(round_proj), _ptr(xq), _ptr(xk), _ptr(xv), _ptr(gate), _ptr(lr), _ptr(device_status(dev)),
-            stream))
+            cfg.base_lr, int(round_proj), None, None, None, _ptr(xq), _ptr(xk), _ptr(xv), _ptr(gate), _ptr(lr),
+            _ptr(device_status(dev)), stream))
     return xq, xk, xv, lr, gate
 
 
