@@ -457,7 +457,9 @@ class TTT(torch.nn.Module):
             s = _Stack(key, wcat, cols, [w.detach() for w in srcs if w is not None])
             if dev.type == "cuda":
                 s.ready = torch.cuda.current_stream(dev).record_event()
+                s.on_streams.add(native.stream_key(dev.index, *srcs))
             self._stack = s
+            return wcat, cols
         if dev.type == "cuda" and not capturing:  # (a capture begins behind everything that was queued)
             here = native.stream_key(dev.index, *srcs)
             if here not in s.on_streams:
