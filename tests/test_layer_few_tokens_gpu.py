@@ -103,8 +103,8 @@ def test_token_eta_follows_its_parameters_at_every_call(T):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B,H,use_gate", ((16, 32, True), (17, 32, False), (32, 24, False), (21, 24, True), (22, 24, True),
-                                          (32, 16, True), (32, 17, True)))
+@pytest.mark.parametrize("B,H,use_gate", ((16, 32, True), (17, 32, False), (32, 32, True), (17, 12, True), (24, 16, False),
+                                          (25, 16, False), (32, 12, False), (17, 22, False)))
 def test_either_side_of_where_the_general_form_takes_over(B, H, use_gate):
     import ttt_rs_b200 as tb
     x, p = _random_case(B, 1, H, 7 + H, False, use_gate, torch.bfloat16)

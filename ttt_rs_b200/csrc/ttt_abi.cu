@@ -896,10 +896,13 @@ extern "C" int ttt_linear_forward_partial(const ttt_dims* d, const void* xq, con
                                   weight_out, bias_out, stream);
 }
 
-extern "C" int ttt_internal_layer_small_fits(const ttt_dims* d, int gate) {
+extern "C" int ttt_internal_layer_small_fits(const ttt_dims* d) {
   const int64_t C = (int64_t)d->heads * d->head_dim, M = (int64_t)d->batch * d->seq_len;
-  return d->dtype == TTT_BF16 && (d->head_dim == 64 || d->head_dim == 32) && C <= 2048 && C % 32 == 0 &&
-         ttt::layer_small_rows(M, C, gate != 0);
+  return d->dtype == TTT_BF16 && (d->head_dim == 64 || d->head_dim == 32) && C <= 2048 && C % 32 == 0 && M <= ttt::SMALL_M;
+}
+extern "C" int ttt_internal_layer_small_out_fits(const ttt_dims* d, int gate) {
+  return ttt_internal_layer_small_fits(d) &&
+         ttt::layer_small_out_rows((int64_t)d->batch * d->seq_len, (int64_t)d->heads * d->head_dim, gate != 0);
 }
 
 extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, int64_t x_ld, const void* weights,
@@ -907,7 +910,7 @@ extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, i
                                              int rope_mode, float rope_theta, float base_lr, const void* token_idx,
                                              const void* learnable_token_idx, void* token_eta_out, void* xq, void* xk,
                                              void* xv, void* gate, void* ttt_lr_eta, int lr_pitch, void* stream) {
-  if (!ttt_internal_layer_small_fits(d, gate != nullptr)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
+  if (!ttt_internal_layer_small_fits(d)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
   if (const int rc = check_rotation(d, start_idx, rope_mode, rope_theta); rc != TTT_OK) return rc;
   if (x_ld % 8 != 0 || w_ld % 8 != 0) return fail(TTT_ERR_ALIGN, "row pitches must be multiples of 8 elements");
   const NamedPtr ptrs[] = {{"x", x}, {"weights", weights}, {"xq", xq}, {"xk", xk}, {"xv", xv}};
@@ -928,7 +931,7 @@ extern "C" int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, i
 extern "C" int ttt_internal_layer_small_out(const ttt_dims* d, const void* inner_out, const void* gate, int gate_ld,
                                             const void* post_norm_weight, const void* post_norm_bias, float eps,
                                             const void* o_proj, int64_t o_ld, void* y, void* stream) {
-  if (!ttt_internal_layer_small_fits(d, gate != nullptr)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
+  if (!ttt_internal_layer_small_out_fits(d, gate != nullptr)) return fail(TTT_ERR_UNSUPPORTED, "too many tokens or features for the few-token form");
   if (gate_ld % 8 != 0 || o_ld % 8 != 0) return fail(TTT_ERR_ALIGN, "row pitches must be multiples of 8 elements");
   const NamedPtr ptrs[] = {{"inner_out", inner_out}, {"post_norm_weight", post_norm_weight},
                            {"post_norm_bias", post_norm_bias}, {"o_proj", o_proj}, {"y", y}};

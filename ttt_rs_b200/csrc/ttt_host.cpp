@@ -495,8 +495,9 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   c10::cuda::CUDAGuard guard(dev);
   void* const st = m.stream();
   void* const status = m.status.data_ptr();
-  const bool small = !conv && ttt_internal_layer_small_fits(&d, use_gate);
-  NONE_IF(small && (!on_16_bytes(t[12]) || !on_16_bytes(t[13])));
+  const bool small = !conv && ttt_internal_layer_small_fits(&d);  // few-token form of the projections,
+  const bool small_out = small && ttt_internal_layer_small_out_fits(&d, use_gate);  // of the output side
+  NONE_IF(small_out && (!on_16_bytes(t[12]) || !on_16_bytes(t[13])));
   NONE_IF(!small && N % 8 != 0);
   auto must = [](int rc) {
     if (rc != TTT_OK) throw_error(rc);
@@ -514,7 +515,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 o_te = room(16);
   const int64_t o_proj = small || fused ? 0 : room(M * N);
   const int64_t o_gate = use_gate && (small || fused) ? room(M * C) : 0;
-  const int64_t o_y = small ? 0 : room(M * C);
+  const int64_t o_y = small_out ? 0 : room(M * C);
   Tensor tmp = at::empty({at_}, m.opt(at::kByte));
   uint8_t* const base = static_cast<uint8_t*>(tmp.data_ptr());
   Tensor y = at::empty({B, T, C}, m.opt());
@@ -577,7 +578,7 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
                                   st));
   }
   // ---- post norm, gate, output projection
-  if (small) {
+  if (small_out) {
     must(ttt_internal_layer_small_out(&d, base + o_in, gate, (int)gate_ld, t[12].const_data_ptr(),
                                       t[13].const_data_ptr(), 1e-6f, t[14].const_data_ptr(), C, y.data_ptr(), st));
   } else {

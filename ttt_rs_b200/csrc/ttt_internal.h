@@ -57,8 +57,9 @@ int ttt_internal_layer_projections(const ttt_dims* d, const void* x, int64_t x_l
                                    void* token_eta_out, void* xq, void* xk, void* xv, void* gate,
                                    void* ttt_lr_eta, void* status, void* stream);
 // Few-token forms (bf16): projections with the prologue, and post norm (+ gate) with the output projection; 0 from
-// _fits: not for this shape.  weights: q | k | v | (gate) blocks of heads * head_dim rows, learning-rate rows from lr_col.
-int ttt_internal_layer_small_fits(const ttt_dims* d, int gate);
+// _fits and _out_fits: not for this shape.  weights: q | k | v | (gate) blocks of heads * head_dim rows, learning-rate rows from lr_col.
+int ttt_internal_layer_small_fits(const ttt_dims* d);
+int ttt_internal_layer_small_out_fits(const ttt_dims* d, int gate);
 int ttt_internal_layer_small_proj(const ttt_dims* d, const void* x, int64_t x_ld, const void* weights, int64_t w_ld,
                                   int w_rows, int lr_col, const void* lr_bias, int start_idx, int rope_mode,
                                   float rope_theta, float base_lr, const void* token_idx,

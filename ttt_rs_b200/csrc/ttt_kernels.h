@@ -167,15 +167,19 @@ struct LayerEpiParams {
   int B, H, T;
   float eps;
 };
-// Few-token forms of the layer's two sides (ttt_layer_small.cu): bf16, head_dim 64 or 32, at most 2048 features, hidden a
-// multiple of 32, and rows up to where the general form (tensor-core GEMMs, prologue, epilogue) is the faster one.  Up to 16
-// rows that is nowhere.  From 17 on every CTA of the output kernel holds 32 rows (64 C bytes: from 1700 features on one CTA
-// per SM and two waves) and gates all of them for itself.  Whole decode step, few-token / general form, us:
-//   rows x features   16 x 2048   32 x 768    32 x 1024   24 x 1280   32 x 1280   24 x 1536   32 x 1536   17 x 2048
-//   no gate           27.4/44.1   23.4/31.7   26.8/34.9   27.5/39.1   31.3/39.2   32.3/40.0   38.1/40.0   47.4/44.0
-//   gate              37.3/46.7   29.5/34.9   36.4/36.8   36.2/41.0   42.5/41.0   43.0/41.0   51.1/41.1   69.6/46.6
-inline bool layer_small_rows(int64_t rows, int64_t features, bool gate) {
-  return rows <= 16 || (rows <= 32 && features <= 1536 && (!gate || rows * features <= 32768));
+// Few-token forms of the layer's two sides (ttt_layer_small.cu): up to SMALL_M rows, bf16, head_dim 64 or 32, at most 2048
+// features, hidden a multiple of 32.
+constexpr int SMALL_M = 32;
+// The output side only where it is faster than epilogue + tensor-core GEMM.  Up to 16 rows that is everywhere.  From 17 on
+// every CTA normalises (and gates) up to 32 rows for itself and holds them in 64 C bytes of shared memory (from 1700 features
+// on one CTA per SM and two waves).  Decode step of a layer, output side few-token / general, us (all general: 31 to 47):
+//   features          768               1024              1280              1536              2048
+//   17 rows       20.2 / 22.7       22.5 / 24.6       25.8 / 26.7       30.8 / 29.8       47.7 / 33.8
+//   24 rows       20.5 / 22.6       23.5 / 24.7       27.5 / 27.7       32.8 / 29.9       50.2 / 34.0
+//   32 rows       23.0 / 22.6       26.6 / 25.8       31.7 / 28.8       38.4 / 31.7       59.3 / 35.9
+//   24, gated     25.2 / 24.6       30.1 / 26.7       35.8 / 29.5       43.1 / 32.0       72.4 / 41.0
+inline bool layer_small_out_rows(int64_t rows, int64_t features, bool gate) {
+  return rows <= 16 || (rows <= SMALL_M && !gate && rows * features <= 24576);
 }
 struct SmallProjParams {
   const void* x;  // [M, ldx], rows b * T + t
