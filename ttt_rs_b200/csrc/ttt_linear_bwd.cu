@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       s1t[0] = o0.x * INV_F; s2t[0] = o0.y * INV_F;
       s1t[1] = o1.x * INV_F; s2t[1] = o1.y * INV_F;
       const float rt_all = col_sum(o0.w + o1.w);  // sum over the 16 rows
-      // (every warp holds these row values; warp 2 writes them: warps 0 and 1 issue the stage's stores and loads)
+      // (every warp holds these row values; warp 2 writes them, of a pair of heads the first warp of each)
       if ((SEG == 32 ? (warp & 1) == 0 : warp == 2) && t == 0) {
         // per (batch, head) stream of the caller's tensors: the pair's heads are streams 2 * stream and 2 * stream + 1
         const size_t o = (SEG == 32 ? (size_t)(2 * stream + hsel) * p.T : (size_t)row_base) + (size_t)s * MB;

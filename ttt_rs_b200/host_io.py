@@ -55,8 +55,10 @@ def auto_chunks(batch: int, heads: int, seq_len: int, head_dim: int, elem_size: 
     rows = max(1, -int(-1.3 * chain_ms // row_ms))
     # Rows that cut the batch into equal chunks, if there are such up to twice as many (behind a chunk larger than the one
     # before it the copy-out waits), and then no more than a dozen chunks, each of which costs its events and launches:
-    # 12 x 2048 x 64 bf16, forward + backward, 32 rows: 8 chunks 9.6 ms, 16 chunks 9.8, 11 unequal ones 10.4; 16 rows: 8
-    # chunks 5.2 ms, 6 unequal ones 5.8; 8 rows: 4 chunks 3.13 ms, 3 unequal ones 3.39.
+    # 12 x 2048 x 64 bf16, forward + backward, in turn with the bare copies of the same bytes (time over theirs, two hosts):
+    # 32 rows: 8 chunks 1.17, 16 chunks 1.17 and 1.19, 4 chunks 1.25, 11 unequal ones 1.24 and 1.26, 6 to 14 other unequal
+    # ones 1.26 to 1.30; 20 rows: 10 chunks 1.22, 5 chunks 1.25, 7 unequal ones 1.31; 16 rows: 8 chunks 1.28, 4 chunks
+    # 1.31, 6 unequal ones 1.38; 8 rows: 4 chunks 1.45, 3 unequal ones 1.58.
     even = [r for r in range(rows, 2 * rows + 1) if batch % r == 0]
     if even:
         rows = next((r for r in even if batch // r <= 12), even[-1])

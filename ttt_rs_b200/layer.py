@@ -3,17 +3,19 @@
 state, start_idx)`.
 
 What runs where:
-  * q/k/v(/gate) projections and the per-head learning-rate logits: ONE library GEMM over the concatenated weights
-    (the reference issues one GEMM per projection plus a batched matmul for the gate logits);
-  * head split + permute to [B,H,T,F], shared-QK causal convolutions, rotary embedding, sigmoid learning-rate gate:
-    `ttt_layer_prologue` (one pass over the projection output);
+  * q/k/v(/gate) projections and the per-head learning-rate logits: one product over the stacked weights, on the tcgen05
+    GEMM `ttt_gemm_bf16_tn` in bf16 (float32: a library product; the reference issues one GEMM per projection plus a
+    batched matmul for the gate logits);
+  * head split + permute to [B,H,T,F], shared-QK causal convolutions, rotary embedding, sigmoid learning-rate gate: in
+    the product's epilogue where `TTT._can_fuse_projections` says so, else `ttt_layer_prologue` (one pass over the
+    projection output); few tokens: all of it in one kernel without tensor-core tiles;
   * inner loop: the fused kernel behind `FusedTileMultiTTTLinear`;
   * permute back + post LayerNorm + gelu gate: `ttt_layer_epilogue` (one pass);
-  * output projection: library GEMM.
+  * output projection: `ttt_gemm_bf16_tn` in bf16 (few tokens: together with the norm), else a library product.
 Under autograd the same kernels run with their gradient kernels (`ttt_layer_prologue_backward`,
-`ttt_layer_epilogue_backward`) joined by torch autograd, so the layer trains end to end; with the shared-QK layout the
-two convolutions are a step of their own there (`ttt_layer_qk_conv`, `ttt_layer_qk_conv_backward`) instead of being
-applied inside the prologue kernel.
+`ttt_layer_epilogue_backward`) joined by torch autograd, so the layer trains end to end; the output projection and the
+products of the gradients are library GEMMs there.  With the shared-QK layout the two convolutions are a step of their own
+(`ttt_layer_qk_conv`, `ttt_layer_qk_conv_backward`) instead of being applied inside the prologue kernel.
 There is no PyTorch fallback for the layer kernels: without the CUDA library the calls raise.
 """
 
@@ -152,7 +154,7 @@ def layer_projections(x: torch.Tensor, wcat: torch.Tensor, cols, cfg: TTTLayerCo
     head split, rotary rotation and learning-rate gate in its epilogue).  x [B, T, hidden] bf16, wcat the stacked
     q | k | v | (g) | lr weight rows with their starts in `cols`.  Returns xq, xk, xv [B,H,T,F], ttt_lr_eta [B,H,T] and
     the gate buffer [B*T, H*F] (None without a gate).  `round_proj`: the projections rounded to bf16 before the rotation
-    and the gate, the values a separate product and prologue would give (training)."""
+    and the gate, where a separate product and prologue round them (training)."""
     from .fused import device_status
     lib = _lib.load()
     B, T, hidden = x.shape
@@ -576,7 +578,7 @@ def _train_forward(self, x, inner, state, start_idx):
     """Training path: the same kernels, each with its gradient kernel, joined by torch autograd.  Where the one-launch
     projections apply (bf16, no shared q / k) they run here as in inference; elsewhere the projection is a library
     product, and the gate's a product of its own, so that every column of the fused projection's gradient is written by
-    exactly one kernel.  (65536 tokens of 768 features: one launch instead of product + prologue 300 -> 186 us.)"""
+    exactly one kernel.  (65536 tokens of 768 features: one launch instead of product + prologue 300 -> 219 us.)"""
     c = self.config
     B, T, _ = x.shape
     H, hs = c.num_heads, c.hidden_size
@@ -636,9 +638,12 @@ def new_inner(config: TTTLayerConfig, checkpoint_interval: int = 1, device=None,
 class DecodeGraphs:
     """Token-by-token generation through one layer, the state advanced in place.
 
-    Where the native path covers the layer (bf16, see `TTT.forward`), a step is its launches issued directly: three for
-    few sequences, overlapped through programmatic dependent launch, which leaves nothing for a graph to save and
-    spares the copy of the input into a captured buffer.  Otherwise the step (projection GEMM, prologue, decode kernel,
+    Where the native path covers the layer (bf16, see `TTT.forward`), a step is its launches issued directly: three or
+    four for few sequences, overlapped through programmatic dependent launch, five for more.  A graph would save up to 5 us of
+    host time and lose most or all of them to the copy of the input into the captured buffer; steps in sequence, direct /
+    copy + replay / replay alone, us: 8 sequences x 768 features 14.4 / 18.5 / 15.2, 16 x 2048 27.4 / 31.7 / 28.3, 33 x
+    768 31.7 / 32.0 / 29.0, 64 x 2048 52.3 / 53.8 / 48.4, 128 x 768 38.2 / 38.0 / 33.9, 128 x 2048 63.6 / 65.6 / 60.0;
+    gated 33 x 768 34.9 / 32.8 / 29.7.  Otherwise the step (projection GEMM, prologue, decode kernel,
     epilogue, output GEMM) is captured once per rotary phase as a CUDA graph: the rotary position enters the prologue
     as a scalar argument, so with positions wrapped at the mini-batch there are `mini_batch_size` distinct steps, each
     captured on first use; the input is copied to `self.x` [B, 1, hidden] and the result lands in the tensor `step`
