@@ -22,7 +22,7 @@
  *    reference panics (unsupported tile config, seq_len not a multiple of the mini-batch:
  *    linear_fused_tile/mod.rs:143, forward/launch.rs:209-213) these functions return an error and launch
  *    nothing.
- *  - `status`, when non-null, points to 4 device uint32 words (16 for ttt_mlp_backward) that the caller zeroed
+ *  - `status`, when non-null, points to 4 device uint32 words that the caller zeroed
  *    once; a kernel whose bounded wait (on a TMA completion barrier, or on another block's hand-off) expires
  *    writes {TTT_ERR_TIMEOUT, where, block, stage} there by compare-and-swap from zero and returns early, leaving
  *    its outputs unwritten.  Launches never clear the words, so one buffer per device can serve every launch and
@@ -173,8 +173,8 @@ int ttt_linear_backward_state_grads(const ttt_dims* d, const void* xq, const voi
  *   token_eta [T], ttt_lr_eta [B,H,T], ln_weight / ln_bias [H,F]   bf16
  *   output          bf16 [B,H,T,F] (out);  w1_out, b1_out, w2_out, b2_out (out) final state, same shapes
  *   backward_workspace (optional, out): ttt_mlp_backward_workspace_bytes(d) bytes, 16-byte aligned.  When given, the
- *                   forward leaves there the float32 final state and the bf16 operands of every state update, which
- *                   is all the backward's own first pass would compute: pass the buffer on to ttt_mlp_backward
+ *                   forward leaves there the float32 final state and a record of every mini-batch (the bf16 operands of its
+ *                   state updates, the inputs of its two LayerNorms): pass the buffer on to ttt_mlp_backward
  *                   with workspace_from_forward = 1.  NULL (with 0 bytes) for inference.
  * One block per SM; a block holds 256 columns of the SM's tensor memory (the float32 state between its uses) while it
  * runs.
@@ -188,20 +188,18 @@ int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const voi
 /* TTT-MLP backward (bf16): gradient of ttt_mlp_forward for loss = <grad_output, output>; gradients w.r.t. the returned
  * final state are taken as zero, as for the TTT-Linear operator.  The reference has no fused counterpart: it
  * differentiates the tensor ops of rust/core/src/mlp.rs:127-208 with Burn autodiff.  Inputs are the forward's inputs
- * (nothing saved by the forward is needed: the kernel re-walks the sequence; with `workspace_from_forward` != 0 the
- * workspace is the one a ttt_mlp_forward call on the same inputs filled, and the re-walk is skipped), outputs:
+ * (nothing saved by the forward is needed: the forward kernel is then run first, to fill the workspace; with
+ * `workspace_from_forward` != 0 the workspace is the one a ttt_mlp_forward call on the same inputs filled), outputs:
  *   grad_xq, grad_xk, grad_xv [B,H,T,F]; grad_w1 [B,H,F,4F], grad_b1 [B,H,4F], grad_w2 [B,H,4F,F], grad_b2 [B,H,F]
  *   (per batch element); grad_ttt_lr_eta [B,H,T]; float32 grad_token_eta [T] (per stage position, summed over B, H),
  *   float32 grad_ln_weight / grad_ln_bias [H,F] (summed over B).  All written, never accumulated into.
- * `workspace`: ttt_mlp_backward_workspace_bytes(d) bytes, 16-byte aligned (float32 state and state gradients, a bf16
- * copy of the state gradients, the hand-off records and the saved bf16 per-stage inner gradients of every stream:
- * about B*H*(323 KB + 11 KB per mini-batch), plus the scheduler words).  The kernel is persistent: blocks take (stream,
- * chunk of 8 mini-batches) work items and hand a stream's state to one another through the workspace; it is launched
- * cooperatively (all blocks co-resident), one block per SM, and every hand-off wait is bounded.  A block allocates the
- * SM's whole tensor memory (512 columns) for the float32 state while it runs and frees it before it exits, so a kernel
- * of another stream that wants tensor memory on the same SM waits for it.  `status` (optional, 16 device words, zeroed by the
- * caller): {TTT_ERR_TIMEOUT, 1, block, item} if such a wait ran out; builds instrumented for tuning write per-phase
- * cycle counts of one block to the 16 words instead.
+ * `workspace`: ttt_mlp_backward_workspace_bytes(d) bytes, 16-byte aligned (the float32 state and state gradients, a
+ * hand-off record and one record per mini-batch of every stream: about B*H*(259 KB + 27.5 KB per mini-batch), plus the
+ * scheduler words).  The kernel is persistent: blocks take (stream, chunk of mini-batches) work items and hand a stream's
+ * state to one another through the workspace; it is launched cooperatively (all blocks co-resident), one block per SM, and
+ * every hand-off wait is bounded.  A block allocates the SM's whole tensor memory (512 columns) for the float32 state while
+ * it runs and frees it before it exits, so a kernel of another stream that wants tensor memory on the same SM waits for it.
+ * `status` (optional, 4 device words, zeroed by the caller): {TTT_ERR_TIMEOUT, where, block, item} if a wait ran out.
  */
 size_t ttt_mlp_backward_workspace_bytes(const ttt_dims* d);
 int ttt_mlp_backward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* w1, const void* b1,

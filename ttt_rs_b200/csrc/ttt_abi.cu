@@ -45,6 +45,19 @@ EncodeFn get_encode_fn() {
   return fn;
 }
 
+// cuTensorMapEncodeTiled with the device's context current to this thread.  It is a driver call: on a thread that has made
+// no runtime call yet (an autograd worker whose allocations are served from the cache) there is none, and the runtime
+// only binds one by the calls that need it.
+template <class... A>
+CUresult encode_tiled(EncodeFn enc, A... args) {
+  CUresult r = enc(args...);
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = enc(args...);
+  }
+  return r;
+}
+
 // 2-D view [rows, 64] of a [B,H,T,64] tensor, box = one 16-token tile (or half of it for float32),
 // 128-byte swizzle so that ldmatrix / element-wise shared-memory reads are bank-conflict free.
 int make_tile_map(CUtensorMap* m, const void* base, int64_t rows, int dtype, int box_rows = 16) {
@@ -55,7 +68,7 @@ int make_tile_map(CUtensorMap* m, const void* base, int64_t rows, int dtype, int
   const cuuint64_t strides[1] = {(cuuint64_t)(64 * (bf ? 2 : 4))};
   const cuuint32_t box[2] = {(cuuint32_t)(bf ? 64 : 32), (cuuint32_t)box_rows};  // (8 rows: mini-batches of 8 tokens)
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+  CUresult r = encode_tiled(enc, m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TTT_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
@@ -71,7 +84,7 @@ int make_gemm_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, 
   const cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
   const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_tiled(enc, m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TTT_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
@@ -89,7 +102,7 @@ int make_pair_map(CUtensorMap* m, const void* base, int64_t pairs, int64_t T, in
   const cuuint64_t strides[1] = {(cuuint64_t)(32 * (bf ? 2 : 4))};
   const cuuint32_t box[2] = {32, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+  CUresult r = encode_tiled(enc, m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    bf ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -642,6 +655,7 @@ int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const voi
   p.status = static_cast<uint32_t*>(status);
   p.bwd_ws = static_cast<float*>(backward_workspace);
   p.bwd_ws_stride = wl.stride_floats;
+  p.walk_only = 0;
   // with a workspace the launch is persistent and uses the workspace's scheduler words (the backward re-zeroes them)
   p.sched = backward_workspace != nullptr ? reinterpret_cast<int*>(static_cast<float*>(backward_workspace) + wl.off_sched)
                                           : nullptr;
@@ -1143,9 +1157,29 @@ extern "C" int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, cons
     return fail(TTT_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", l.total_bytes, workspace_bytes);
   if ((reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return fail(TTT_ERR_ALIGN, "workspace is not 16-byte aligned");
   float* ws = static_cast<float*>(workspace);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  CUtensorMap maps[4];
+  const void* bases[4] = {xq, xk, xv, grad_output};
+  for (int i = 0; i < 4; ++i) {
+    rc = make_tile_map(&maps[i], bases[i], (int64_t)d->batch * d->heads * d->seq_len, d->dtype);
+    if (rc != TTT_OK) return rc;
+  }
+  if (workspace_from_forward == 0) {  // the stages' records and the final state, by the forward kernel itself
+    ttt::MlpFwdParams f{};
+    f.w1 = w1; f.b1 = b1; f.w2 = w2; f.b2 = b2;
+    f.token_eta = token_eta; f.lr = ttt_lr_eta; f.ln_g = ln_weight; f.ln_b = ln_bias;
+    f.status = static_cast<uint32_t*>(status);
+    f.bwd_ws = ws;
+    f.bwd_ws_stride = l.stride_floats;
+    f.walk_only = 1;
+    f.sched = reinterpret_cast<int*>(ws + l.off_sched);
+    f.handoff_polls = g_handoff_polls.load();
+    f.H = d->heads; f.T = d->seq_len; f.NS = d->seq_len / d->mini_batch; f.eps = d->epsilon;
+    const cudaError_t e = ttt::launch_mlp_fwd(maps, f, d->batch * d->heads, st);  // (the output's map is not used)
+    if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "MLP forward walk launch failed: %s", cudaGetErrorString(e));
+  }
   ttt::MlpBwdParams p;
-  p.xq = xq; p.xk = xk; p.xv = xv; p.w1 = w1; p.b1 = b1; p.w2 = w2; p.b2 = b2;
-  p.token_eta = token_eta; p.lr = ttt_lr_eta; p.ln_g = ln_weight; p.ln_b = ln_bias; p.d_out = grad_output;
+  p.token_eta = token_eta; p.lr = ttt_lr_eta; p.ln_g = ln_weight; p.ln_b = ln_bias;
   p.d_q = grad_xq; p.d_k = grad_xk; p.d_v = grad_xv; p.d_w1 = grad_w1; p.d_b1 = grad_b1; p.d_w2 = grad_w2;
   p.d_b2 = grad_b2; p.d_lr = grad_ttt_lr_eta; p.d_token_eta = grad_token_eta; p.d_ln_g = grad_ln_weight;
   p.d_ln_b = grad_ln_bias;
@@ -1155,11 +1189,9 @@ extern "C" int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, cons
   p.part_te = ws + l.off_te;
   p.part_ln = ws + l.off_ln;
   p.sched = reinterpret_cast<int*>(ws + l.off_sched);
-  p.pass1_done = workspace_from_forward != 0;
   p.status = static_cast<uint32_t*>(status);
-  p.trace = static_cast<unsigned int*>(status);  // instrumented builds write 16 words of cycle counts here instead
   p.H = d->heads; p.T = d->seq_len; p.NS = d->seq_len / d->mini_batch; p.eps = d->epsilon;
-  cudaError_t e = ttt::launch_mlp_bwd(p, d->batch, static_cast<cudaStream_t>(stream));
+  cudaError_t e = ttt::launch_mlp_bwd(maps, p, d->batch, st);
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "MLP backward launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
 }

@@ -115,10 +115,11 @@ struct MlpFwdParams {
   void* w2_out;
   void* b2_out;
   uint32_t* status;
-  float* bwd_ws;         // optional: the backward's workspace; the forward then leaves there what the backward's own
-  size_t bwd_ws_stride;  // first pass would compute (final state, final biases, lr-scaled inner gradients per stage)
-  int* sched;            // with bwd_ws: [1 + B*H] work-item counter and per-stream count of finished chunks (the
-                         // persistent launch; zeroed by the launcher), else null
+  float* bwd_ws;         // optional: the backward's workspace; the forward then leaves there the final state and a record
+  size_t bwd_ws_stride;  // of every stage
+  int walk_only;         // only that: no output and no final state for the caller
+  int* sched;            // with bwd_ws (null otherwise): [1 + B*H] work-item counter and per-stream count of finished chunks (the
+                         // persistent launch; zeroed by the launcher)
   int nstreams, CH, NCH; // set by the launcher: streams, stages per work item, items per stream
   uint32_t handoff_polls;  // iteration limit of the wait for the previous chunk's state
   int H, T, NS;
@@ -299,19 +300,11 @@ cudaError_t launch_linear_partial(int dtype, int head_dim, const LinPartialParam
 
 // TTT-MLP backward (ttt_mlp_bwd.cu), bf16 I/O.
 struct MlpBwdParams {
-  const void* xq;  // [B,H,T,F]
-  const void* xk;
-  const void* xv;
-  const void* w1;  // [B,H,F,E]
-  const void* b1;  // [B,H,E]
-  const void* w2;  // [B,H,E,F]
-  const void* b2;  // [B,H,F]
   const void* token_eta;
   const void* lr;
   const void* ln_g;
   const void* ln_b;
-  const void* d_out;  // [B,H,T,F]
-  void* d_q;
+  void* d_q;  // [B,H,T,F]
   void* d_k;
   void* d_v;
   void* d_w1;
@@ -323,33 +316,49 @@ struct MlpBwdParams {
   void* d_ln_g;       // [H,F]
   void* d_ln_b;
   int reduced_bf16;   // element type of the three
-  float* workspace;   // per stream `ws_stride` floats: state, state gradients, saved inner gradients
+  float* workspace;   // per stream `ws_stride` floats, filled by the forward
   size_t ws_stride;
   float* part_te;      // [B*H][T]
   float* part_ln;      // [B*H][2][F]
-  unsigned int* trace;  // optional 16 words (per-phase cycle counts of block 0 in instrumented builds), else null
   int* sched;           // [1 + B*H] work-item counter and per-stream count of finished items (zeroed by the launcher)
   uint32_t* status;     // optional 4 words: {TTT_ERR_TIMEOUT, where, block, item} if a hand-off wait ran out
   int H, T, NS;
-  int nstreams, CH, NCH;  // set by the launcher: streams, stages per work item, items per pass
-  int pass1_done;         // the forward already filled the workspace (ttt_mlp_forward with backward_workspace)
+  int nstreams, CH, NCH;  // set by the launcher: streams, stages per work item, items per stream
   float eps;
 };
-// Per-stream block of the TTT-MLP backward's workspace, in floats: W1 [64][256], W2 [256][64], dW1, dW2 (float32, each
-// stored tile by tile in accumulator-fragment order, see mlp_state_at), the hand-off record between work items
-// (b1, b2, db1, db2, d ln_weight, d ln_bias), then per stage the bf16 tiles lr o g1 [NS][16][256] and lr o g2
-// [NS][16][64], then the float32 biases b1 | b2 at the start of every stage [NS][256 + 64], then bf16 copies of dW1 and
-// dW2 (64 KB) that the backward reads as product operands.
+// Per-stream block of the TTT-MLP backward's workspace: the float32 masters of W1^T, W2, dW1^T, dW2, each [256 hidden][64]
+// (order: mlp_master_at; W1 and W2 divided by -token_eta[15], as the kernels carry them, unless that is zero), the hand-off
+// record between work items, then one record per stage, written by the forward.
 constexpr int MLP_BWD_HANDOFF_FLOATS = 2 * 256 + 4 * 64;
-constexpr int MLP_HO_B1 = 0, MLP_HO_B2 = 256, MLP_HO_DB1 = 320, MLP_HO_DB2 = 576, MLP_HO_DG = 640, MLP_HO_DB = 704;
-// element (r, c) of a float32 matrix with C columns stored in accumulator-fragment order: the 16 x 8 tile
-// (r / 16, c / 8) occupies 128 consecutive floats, its rows 0..7 before its rows 8..15, and inside a half the
-// element (r % 8, c % 8) sits at 8 * (r % 8) + (c % 8)
-__host__ __device__ inline int mlp_state_at(int r, int c, int C) {
-  return (((r >> 4) * (C / 8) + (c >> 3)) << 7) + (((r >> 3) & 1) << 6) + ((r & 7) << 3) + (c & 7);
+constexpr int MLP_HO_B1 = 0, MLP_HO_B2 = 256, MLP_HO_DB1 = 320, MLP_HO_DB2 = 576, MLP_HO_DG = 640;  // DG: weight, bias [2][64]
+// element (hidden feature e, feature f) of a master, as a float index: 16-byte pieces of 32 consecutive hidden features
+// (the lanes of a warp) side by side
+__host__ __device__ inline int mlp_master_at(int e, int f) { return ((((e >> 5) * 16 + (f >> 2)) * 32 + (e & 31)) << 2) + (f & 3); }
+// A stage's record, in bytes.  X2 [16][256] and G1p [16][256] (four tiles of 64 columns) and G2p [16][64]: bf16, in the
+// swizzled form that shared memory holds them in (off_bf16); float32: Z2, Zb2 [16][64], b1 [256] at the start of the stage, and
+// per token (8 floats) mean and 1 / std of Z2, the two row means of its LayerNorm gradient, mean and 1 / std of Zb2
+constexpr int MLP_REC_X2 = 0, MLP_REC_G1P = 8192, MLP_REC_G2P = 16384, MLP_REC_Z2 = 18432, MLP_REC_ZB2 = 22528,
+              MLP_REC_B1 = 26624, MLP_REC_STAT = 27648, MLP_REC_BYTES = 28160;
+// Stages per work item of the persistent launches: a stream that has a block to itself is one item; otherwise the length
+// for which the busiest block has least to do, a hand-over of a stream counted as one stage and a half (the backward: 512 KB
+// through L2 against a stage of 4 us)
+inline int mlp_chunk_stages(int NS, int nstreams, int blocks) {
+  if (nstreams <= blocks) return NS;
+  int best = NS;
+  long long least = -1;
+  for (int ch = 8; ch <= 64; ch += 4) {
+    const long long nch = (NS + ch - 1) / ch, rounds = (nch * nstreams + blocks - 1) / blocks;
+    const long long cost = rounds * (2 * (ch < NS ? ch : NS) + 3);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = ch;
+    }
+  }
+  return best < NS ? best : NS;
 }
 size_t mlp_bwd_ws_stride_floats(int T);
-cudaError_t launch_mlp_bwd(const MlpBwdParams& p, int B, cudaStream_t st);
+// maps: q, k, v, d_out
+cudaError_t launch_mlp_bwd(const CUtensorMap* maps, const MlpBwdParams& p, int B, cudaStream_t st);
 
 // bf16 projection GEMM C[M,N] = A[M,K] . B[N,K]^T on tcgen05 (ttt_gemm.cu).  maps: A, B (loads, box 64 x 128), C (store).
 // Fused epilogue of the layer's stacked projection (ttt_layer_projections): where the column blocks of the product

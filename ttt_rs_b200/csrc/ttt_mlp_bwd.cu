@@ -5,1171 +5,933 @@
 // grad_xq/xk/xv, grad_w1/b1/w2/b2 (per batch element), grad_ttt_lr_eta, and per-stream partials of grad_token_eta and
 // of the LayerNorm parameter gradients (summed over streams in a fixed order by ttt_mlp_bwd_reduce_kernel).
 //
-// How: the stage-by-stage analytic backward (reverse walk over the mini-batches carrying dW1, db1, dW2, db2; GELU
-// and LayerNorm second derivatives).
-//   pass 1 walks forward once and saves the lr-scaled inner gradients g1p = lr o g1, g2p = lr o g2 of every stage
-//          (bf16: exactly the operand values of the state update, so that pass 2 can undo the update); the forward
-//          kernel can do this instead while it runs (it then also leaves the final state in the workspace);
-//   pass 2 walks backward: W1_s = W1_{s+1} + K^T g1p, W2_s = W2_{s+1} + X2^T g2p recover the state of the stage,
-//          the stage's forward intermediates are recomputed from it, and the gradient steps follow.
-// Where things live: the float32 masters of W1, W2, dW1, dW2 (256 KB per stream) sit in the SM's tensor memory while a
-// work item runs (each thread owns the 128 floats its accumulator fragments update, see MatM) and in the workspace
-// between work items; every matrix that is an operand of a product sits in shared memory as a padded row-major bf16
-// tile that ldmatrix reads directly (the 16 x 256 and 16 x 64 working tiles, and bf16 shadows of W1 and W2 refreshed
-// by the same epilogue that updates the masters) -- except dW1 and dW2, for whose bf16 copies shared memory has no
-// room: those are in the workspace (MatH).  Tiles that only accumulate or feed a LayerNorm (z2, z2b, dg2, dk, ...)
-// are float32.  Operand precision is the forward kernel's: bf16 operands, float32 accumulation.
-#include <type_traits>
-
+// How: the stage-by-stage analytic backward (reverse walk over the mini-batches carrying dW1, db1, dW2, db2; GELU and
+// LayerNorm second derivatives).  The forward kernel leaves one record per stage (MlpStage: X2, the lr-scaled inner
+// gradients G1p and G2p, Z2, Zb2, b1): W1_s = W1_{s+1} + te15 K^T G1p, W2_s = W2_{s+1} + te15 X2^T G2p undo the stage's
+// update, and both LayerNorms of the stage are differentiated straight from the saved Z2 and Zb2.
+//
+// Where things live, and who does what:
+//  * The float32 masters of W1^T, W2, dW1^T, dW2 fill the SM's tensor memory, each as [256 hidden][64 features] = two
+//    128-lane accumulators of 64 columns.  Undoing the two updates and adding the five rank-16 terms of dW1, dW2 are
+//    fourteen tcgen05.mma (M = 128, N = 64, K = 16) that accumulate into them in place; their operands are the token tiles
+//    as they are, read MN-major (hidden or features contiguous, tokens the contraction).
+//  * After every stage each warp reads its quarter of one matrix back (tcgen05.ld) and refreshes that matrix's bf16 copy
+//    in shared memory ([256][64], 128-byte rows, swizzled): the operand of all products that involve the state.
+//  * A warp owns 16 hidden features of every 16 x 256 tile, in mma.sync accumulator layout, from Z1 to dZ1: GELU and its
+//    derivatives, the small causal matrices (each warp forms Q K^T and dZb2 G2^T for itself, 16 products that would
+//    otherwise cost a barrier and a trip through shared memory) and their products with its own columns (operands through
+//    movmatrix) never leave its registers.  Only what is contracted over all 256 hidden features is written out.
+//  * A warp also owns one token row of the 16 x 64 tiles for the two LayerNorms.
+// A stage is six barrier intervals (I1..I6 below).  Before, 25 phases passed every intermediate tile through shared
+// memory as bf16, undid the updates through registers and read dW from L2: 43 k cycles a stage; 192 streams of 128 stages
+// forward and backward 4.11 ms, now 2.68 ms.
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
+#include "ttt_stage.cuh"
 
 namespace ttt {
 
 constexpr int MB_THREADS = 512;
-constexpr int MB_NW = MB_THREADS / 32;  // warps of the CTA
-constexpr int MB_E = 256;               // hidden width of the inner MLP (4 * head_dim)
-constexpr int MLP_BWD_CHUNK = 8;        // stages per work item
-static_assert(MB_NW == CS, "the row-wise (LayerNorm) steps give one tile row to each warp");
-// Row lengths of the shared-memory tiles: width + 8 elements.  For bf16 tiles the row stride is then an odd multiple
-// of 16 bytes, so the eight 16-byte rows of an ldmatrix 8x8 block fall in distinct banks; for float32 tiles a stride
-// of 8 (mod 32) words makes the 64-bit accesses of a half-warp (4 rows x 4 column pairs) conflict-free.
-constexpr int EB = MB_E + 8, FB = HD + 8, CB = CS + 8;  // bf16 tiles
-constexpr int FP = HD + 8, CP = CS + 8;                 // float32 tiles
+constexpr int MB_E = 256;  // hidden width of the inner MLP (4 * head_dim)
 constexpr float GELU_C0 = 0.7978845608028654f, GELU_C1 = 0.044715f;
 typedef __nv_bfloat16 bf;
 
-// ---- matrix views ----------------------------------------------------------------------------------------------
-// float32 matrix with compile-time strides: element (i, j) at p[i * RS + j * CS_] (global or shared memory)
-template <int RS, int CS_>
-struct MatT {
-  float* p;
-  static constexpr int rs = RS, cs = CS_;
+// Shared memory: offsets from a 1024-byte aligned base.  Token tiles are [16][64] bf16 with the 128-byte swizzle; the
+// 16 x 256 ones are four of those (64 hidden features each).
+struct MlpBwdSmem {
+  static constexpr uint32_t TL = TILE_BF16_BYTES, ET = 4 * TILE_BF16_BYTES, WM = MB_E * HD * 2;
+  static constexpr uint32_t W1 = 0, W2 = W1 + WM, DW1 = W2 + WM, DW2 = DW1 + WM;  // [256 hidden][64] bf16
+  static constexpr uint32_t X2 = DW2 + WM;          // two: this stage's and the next one's
+  static constexpr uint32_t X2B = X2 + 2 * ET, G1 = X2B + ET, DZ1B = G1 + ET, DH = DZ1B + ET;
+  static constexpr uint32_t DZ1 = DH + ET, G1P = DZ1 + ET;
+  static constexpr uint32_t PART = DZ1;             // float [4][16][64], I3..I4 only: dZ1 is written in I5, G1p (with the next V) lands after I4
+  static constexpr uint32_t IN = G1P + ET;          // two x (q, k, dO)
+  static constexpr uint32_t V = IN + 6 * TL, G2P = V + TL, G2 = G2P + TL, DZ2B = G2 + TL, DZ2 = DZ2B + TL;
+  static constexpr uint32_t EXD = DZ2 + TL;         // float [16][64]: dk products; in I3..I4 partials of A2
+  static constexpr uint32_t EXG = EXD + 4096;       // float [16][64]: -l o gl1; in I3..I4 partials of dM1
+  static constexpr uint32_t AD = EXG + 4096;        // float [16][17]: A1[i][j] at [i][j], dM2[i][j] at [j][i + 1]  (j <= i)
+  static constexpr uint32_t DET = AD + 16 * 17 * 4; // float [16][17]: dEta o lr; before I4 the row sums of 16 warps [16][16]
+  static constexpr uint32_t DA1 = DET + 16 * 17 * 4;  // bf16 [16][24]
+  static constexpr uint32_t DB2 = DA1 + 16 * 24 * 2;  // float [64]
+  static constexpr uint32_t LR = DB2 + HD * 4;      // float [2][16], then ell = te15 lr [2][16]
+  static constexpr uint32_t TE = LR + 4 * CS * 4;   // float [16]
+  static constexpr uint32_t DLG = TE + CS * 4;      // float [8][16]
+  static constexpr uint32_t DLP = DLG + 8 * CS * 4; // float [16] sum over i of dEta te, then [16] the rest of dell
+  static constexpr uint32_t LN = DLP + 2 * CS * 4;  // float [2][64]: LayerNorm weight, bias
+  static constexpr uint32_t BAR = LN + 2 * HD * 4; // mbarriers: stage inputs, G1p, products; then item, tensor-memory base
+  static constexpr uint32_t TOTAL = BAR + 3 * 8 + 8;
 };
-template <int RS, int CS_>
-__device__ __forceinline__ MatT<CS_, RS> tr(const MatT<RS, CS_> m) { return MatT<CS_, RS>{m.p}; }
-// bf16 tile in shared memory, rows of LD elements, given by the shared-space byte address of element (0, 0).
-// TR = true: the operand is the transpose of the stored tile.
-template <int LD, bool TR>
-struct SB {
-  uint32_t a;
-};
-template <int LD, bool TR>
-__device__ __forceinline__ SB<LD, !TR> tr(const SB<LD, TR> m) { return SB<LD, !TR>{m.a}; }
+static_assert(MlpBwdSmem::TOTAL <= 227 * 1024, "shared-memory tiles exceed one SM");
+static_assert(MlpBwdSmem::DA1 % 16 == 0 && MlpBwdSmem::BAR % 8 == 0, "alignment");
 
-// float32 matrix [R][C] in the workspace, stored tile by tile in accumulator-fragment order: the 16 x 8 tile
-// (r / 16, c / 8) occupies 128 consecutive floats, its rows 0..7 before its rows 8..15, and inside a half the
-// element (r % 8, c % 8) sits at 8 * (r % 8) + (c % 8).  A warp's read-modify-write of an output tile is then two
-// contiguous 256-byte accesses instead of sixteen 32-byte row pieces, and so are the operand fetches along a row.
-// TR = true: the operand is the transpose of the stored matrix.  Successive work items of a stream may run on
-// different SMs, so every read of these matrices bypasses L1 (ld.global.cg).
-template <int R, int C, bool TR>
-struct MatG {
-  float* p;
-  static __device__ __forceinline__ int at(int r, int c) { return mlp_state_at(r, c, C); }
-};
-template <int R, int C, bool TR>
-__device__ __forceinline__ MatG<R, C, !TR> tr(const MatG<R, C, TR> m) { return MatG<R, C, !TR>{m.p}; }
-
-// bf16 copy of a float32 matrix [R][C] of the workspace, read as the B operand of a product in either orientation
-// (the state gradients dW1, dW2 enter four products per stage, two of them transposed).  Stored in 8 x 8 supertiles
-// of 128 bytes; inside a supertile in 2 x 2 blocks of 8 bytes, rows of a block one after the other: element (r, c)
-// sits at mlp_shadow_at(r, c, C).  A B-fragment register is then one 32-bit load (pair along a row) or one 64-bit
-// load and a byte permute (pair along a column), every warp-wide load is one 128-byte line in both orientations, and
-// the writer's accumulator pair (r, c), (r, c + 1) is one 32-bit store (a warp's half tile = one line).
-__host__ __device__ inline int mlp_shadow_at(int r, int c, int C) {
-  return (((r >> 3) * (C >> 3) + (c >> 3)) << 6) + (((((r >> 1) & 3) << 2) + ((c >> 1) & 3)) << 2) + ((r & 1) << 1) + (c & 1);
+// ---- tcgen05 ---------------------------------------------------------------------------------------------------
+// operand descriptor of token tiles read MN-major: 64 contiguous elements (128 bytes, swizzled) x 8 tokens per atom, the
+// other 8 tokens 1024 bytes on, the next 64 elements (A: M = 128) one tile on
+__device__ __forceinline__ uint64_t token_desc(uint32_t tile) {
+  return (uint64_t)((tile >> 4) & 0x3fff) | ((uint64_t)(TILE_BF16_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
 }
-template <int R, int C, bool TR>
-struct MatH {
-  bf* p;
-};
-template <int R, int C, bool TR>
-__device__ __forceinline__ MatH<R, C, !TR> tr(const MatH<R, C, TR> m) { return MatH<R, C, !TR>{m.p}; }
-
-// float32 master of a state matrix in tensor memory, used as a scratchpad that no tensor-core instruction touches:
-// rank16_update gives the 16 x 8 output tiles of a 64 x 256 (or 256 x 64) matrix to the 16 warps, eight tiles each,
-// always the same ones, so a thread only ever reads and writes its own 32 floats of a matrix -- and a warp can only
-// address its own quarter of the 128 tensor-memory lanes anyway.  Thread (warp w, lane l) owns lane 32 (w % 4) + l; the four
-// warps that share a lane quarter take 128 of the 512 columns each (w / 4), 32 columns per matrix (W1, W2, dW1, dW2):
-// 4 matrices x 64 KB = the SM's whole 256 KB.  Column 4 u + 2 h + e of a matrix holds element (g + 8 h, 2 t + e) of the
-// warp's u-th tile (g = l / 4, t = l % 4): the order of the accumulator registers.  A read-modify-write of a matrix is
-// one tcgen05.ld and one tcgen05.st of 32 columns per thread instead of a round trip to L2.
-template <int R, int C>
-struct MatM {
-  uint32_t taddr;  // lane quarter and first column of this warp's 32 columns of the matrix
-};
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
-      "%30,%31}, [%32];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
-        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]), "=f"(r[16]),
-        "=f"(r[17]), "=f"(r[18]), "=f"(r[19]), "=f"(r[20]), "=f"(r[21]), "=f"(r[22]), "=f"(r[23]), "=f"(r[24]),
-        "=f"(r[25]), "=f"(r[26]), "=f"(r[27]), "=f"(r[28]), "=f"(r[29]), "=f"(r[30]), "=f"(r[31])
-      : "r"(taddr)
-      : "memory");
+// D[128 x 64] (float32) += (-)A . B over 16 tokens; A and B bf16, MN-major
+constexpr uint32_t UPD_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t UPD_NEGATE = 1u << 13;
+__device__ __forceinline__ void umma_update(uint32_t d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 1, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+               "l"(token_desc(a_tile)), "l"(token_desc(b_tile)), "r"(idesc)
+               : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
-      "%30,%31};\n\t"
-      "tcgen05.wait::st.sync.aligned;"
-      ::"f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]),
-        "f"(r[10]), "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "f"(r[16]), "f"(r[17]), "f"(r[18]),
-        "f"(r[19]), "f"(r[20]), "f"(r[21]), "f"(r[22]), "f"(r[23]), "f"(r[24]), "f"(r[25]), "f"(r[26]), "f"(r[27]),
-        "f"(r[28]), "f"(r[29]), "f"(r[30]), "f"(r[31]), "r"(taddr)
-      : "memory");
+__device__ __forceinline__ void umma_commit_to(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2_t(uint32_t (&r)[2], uint32_t addr) {
+__device__ __forceinline__ void ldsm_x2_trans(uint32_t (&r)[2], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
-
-// ---- fragment loads: A fragment of rows i0..i0+15, contraction indices k0..k0+15 -------------------------------
-template <int LD, bool TR>
-__device__ __forceinline__ void load_A(const SB<LD, TR> A, int i0, int k0, int lane, uint32_t (&r)[4]) {
-  if constexpr (!TR) {  // stored [i][k]
-    ldsm_x4(r, A.a + ((i0 + (lane & 15)) * LD + k0 + 8 * (lane >> 4)) * 2);
-  } else {  // stored [k][i]: the four 8x8 blocks are read transposed
-    ldsm_x4_t(r, A.a + ((k0 + (lane & 7) + 8 * (lane >> 4)) * LD + i0 + 8 * ((lane >> 3) & 1)) * 2);
-  }
+__device__ __forceinline__ void mma4(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  mma_bf16(c, a[0], a[1], a[2], a[3], b0, b1);
 }
-template <int RS, int CS_>
-__device__ __forceinline__ void load_A(const MatT<RS, CS_> A, int i0, int k0, int lane, uint32_t (&r)[4]) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const float* s = A.p + (i0 + g + 8 * (q & 1)) * RS + (k0 + 2 * t + 8 * (q >> 1)) * CS_;
-    if constexpr (CS_ == 1) {
-      const float2 f = *reinterpret_cast<const float2*>(s);
-      r[q] = pack_bf16(f.x, f.y);
-    } else {
-      r[q] = pack_bf16(s[0], s[CS_]);
-    }
-  }
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_f(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ float lds_f(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
 }
-// B fragment of contraction indices k0..k0+15, columns j0..j0+7
-template <int LD, bool TR>
-__device__ __forceinline__ void load_B(const SB<LD, TR> B, int k0, int j0, int lane, uint32_t (&r)[2]) {
-  if constexpr (!TR) {  // stored [k][n]
-    ldsm_x2_t(r, B.a + ((k0 + (lane & 15)) * LD + j0) * 2);
-  } else {  // stored [n][k]
-    ldsm_x2(r, B.a + ((j0 + (lane & 7)) * LD + k0 + 8 * ((lane >> 3) & 1)) * 2);
-  }
+__device__ __forceinline__ F2 lds_f2(uint32_t a) {
+  F2 v;
+  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
 }
-template <int RS, int CS_>
-__device__ __forceinline__ void load_B(const MatT<RS, CS_> B, int k0, int j0, int lane, uint32_t (&r)[2]) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const float* s = B.p + (k0 + 2 * t + 8 * q) * RS + (j0 + g) * CS_;
-    if constexpr (RS == 1) {
-      const float2 f = *reinterpret_cast<const float2*>(s);
-      r[q] = pack_bf16(f.x, f.y);
-    } else {
-      r[q] = pack_bf16(s[0], s[RS]);
-    }
-  }
+__device__ __forceinline__ void sts_f2(uint32_t a, F2 v) { asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory"); }
+// loads that stay where they are written (an ordinary one is sunk to its first use, behind the barrier it was to overlap)
+__device__ __forceinline__ F2 ldg_now2(const void* p) {
+  F2 v;
+  asm volatile("ld.global.cg.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
 }
-template <int R, int C, bool TR>
-__device__ __forceinline__ void load_A(const MatG<R, C, TR> A, int i0, int k0, int lane, uint32_t (&r)[4]) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = i0 + g + 8 * (q & 1), k = k0 + 2 * t + 8 * (q >> 1);
-    if constexpr (!TR) {  // stored [i][k]: the pair (k, k + 1) is adjacent
-      const float2 f = __ldcg(reinterpret_cast<const float2*>(A.p + A.at(i, k)));
-      r[q] = pack_bf16(f.x, f.y);
-    } else {
-      r[q] = pack_bf16(__ldcg(A.p + A.at(k, i)), __ldcg(A.p + A.at(k + 1, i)));
-    }
-  }
+__device__ __forceinline__ float4 ldg_now4(const void* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
 }
-template <int R, int C, bool TR>
-__device__ __forceinline__ void load_B(const MatG<R, C, TR> B, int k0, int j0, int lane, uint32_t (&r)[2]) {
-  const int g = lane >> 2, t = lane & 3;
-  // k0 is a multiple of 16 and j0 of 8, so the tile index and the place inside the tile separate
-  if constexpr (TR) {  // stored [j][k]: the pair (k, k + 1) is adjacent; the two registers lie in neighbouring tiles
-    const float* s = B.p + ((((j0 >> 4) * (C / 8) + (k0 >> 3)) << 7) + (((j0 >> 3) & 1) << 6) + (g << 3) + 2 * t);
-    const float2 f0 = __ldcg(reinterpret_cast<const float2*>(s)), f1 = __ldcg(reinterpret_cast<const float2*>(s + 128));
-    r[0] = pack_bf16(f0.x, f0.y);
-    r[1] = pack_bf16(f1.x, f1.y);
-  } else {  // stored [k][j]: rows 2t, 2t + 1 of the upper and of the lower half of one tile
-    const float* s = B.p + ((((k0 >> 4) * (C / 8) + (j0 >> 3)) << 7) + (t << 4) + g);
-    r[0] = pack_bf16(__ldcg(s), __ldcg(s + 8));
-    r[1] = pack_bf16(__ldcg(s + 64), __ldcg(s + 72));
-  }
+__device__ __forceinline__ F2 unpack_bf16(uint32_t v) { return make_float2(bf16_lo(v), bf16_hi(v)); }
+// sums over the warp of two (four) values: the halves of the warp (quarters) reduce one value each
+__device__ __forceinline__ F2 warp_sum2(float a, float b) {
+  const bool hi = threadIdx.x & 16;
+  float v = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const float w = __shfl_xor_sync(0xffffffffu, v, 16);
+  return hi ? f2(w, v) : f2(v, w);
 }
-template <int R, int C, bool TR>
-__device__ __forceinline__ void load_B(const MatH<R, C, TR> B, int k0, int j0, int lane, uint32_t (&r)[2]) {
-  const int g = lane >> 2, t = lane & 3;
-  if constexpr (TR) {  // stored [j][k]: the pair (k, k + 1) is adjacent
+__device__ __forceinline__ float warp_sum4_spread(float a, float b, float c, float d) {  // lanes 8 i ..: the i-th sum
+  const bool hi = threadIdx.x & 16, mid = threadIdx.x & 8;
+  const float x = (hi ? c : a) + __shfl_xor_sync(0xffffffffu, hi ? a : c, 16);
+  const float y = (hi ? d : b) + __shfl_xor_sync(0xffffffffu, hi ? b : d, 16);
+  float v = (mid ? y : x) + __shfl_xor_sync(0xffffffffu, mid ? x : y, 8);
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
-      r[q] = __ldcg(reinterpret_cast<const uint32_t*>(B.p + mlp_shadow_at(j0 + g, k0 + 2 * t + 8 * q, C)));
-  } else {  // stored [k][j]: rows k, k + 1 of the 2 x 2 block that holds column j
-    const uint32_t sel = (g & 1) ? 0x7632u : 0x5410u;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const uint2 w = __ldcg(reinterpret_cast<const uint2*>(B.p + mlp_shadow_at(k0 + 2 * t + 8 * q, (j0 + g) & ~1, C)));
-      r[q] = __byte_perm(w.x, w.y, sel);
-    }
-  }
-}
-template <int R, int C>
-__device__ __forceinline__ float2 c_load(const MatG<R, C, false> M, int i, int j) {
-  return __ldcg(reinterpret_cast<const float2*>(M.p + M.at(i, j)));
-}
-template <int R, int C>
-__device__ __forceinline__ void c_store(const MatG<R, C, false> M, int i, int j, float x, float y) {
-  *reinterpret_cast<float2*>(M.p + M.at(i, j)) = make_float2(x, y);
-}
-// the output pair (i, j), (i, j + 1)
-template <int RS>
-__device__ __forceinline__ float2 c_load(const MatT<RS, 1> C, int i, int j) {
-  return *reinterpret_cast<const float2*>(C.p + i * RS + j);
-}
-template <int RS>
-__device__ __forceinline__ void c_store(const MatT<RS, 1> C, int i, int j, float x, float y) {
-  *reinterpret_cast<float2*>(C.p + i * RS + j) = make_float2(x, y);
-}
-template <int LD>
-__device__ __forceinline__ float2 c_load(const SB<LD, false> C, int i, int j) {
-  uint32_t v;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(C.a + (i * LD + j) * 2));
-  return make_float2(bf16_lo(v), bf16_hi(v));
-}
-template <int LD>
-__device__ __forceinline__ void c_store(const SB<LD, false> C, int i, int j, float x, float y) {
-  asm volatile("st.shared.b32 [%0], %1;" ::"r"(C.a + (i * LD + j) * 2), "r"(pack_bf16(x, y)) : "memory");
-}
-
-struct NoEpi {};
-template <int K_, class MA_, class MB_>
-struct Prod {
-  MA_ A;
-  MB_ B;
-  static constexpr int K = K_;
-};
-template <int K, class MA, class MB>
-__device__ __forceinline__ Prod<K, MA, MB> prod(const MA a, const MB b) { return Prod<K, MA, MB>{a, b}; }
-
-template <class X>
-struct is_global_operand : std::false_type {};
-template <int R, int C, bool TR>
-struct is_global_operand<MatG<R, C, TR>> : std::true_type {};
-template <int R, int C, bool TR>
-struct is_global_operand<MatH<R, C, TR>> : std::true_type {};
-
-// C[M x N] = (ACC ? C : 0) + alpha * sum over the given products of A[M x K] . B[K x N];  M % 16 == 0, N % 8 == 0,
-// K % 16 == 0; every extent and stride is a compile-time constant.  With an epilogue functor the finished pair
-// (i, j), (i, j + 1) goes to epi(i, j, x, y) instead of being stored to C.
-// Output tiles of 16 x 8 are dealt to the warps round-robin (for one WOFF the same tile always goes to the same warp,
-// so successive accumulations into one matrix with the same WOFF need no barrier between them).  A warp works on up to TGMAX of its tiles
-// at a time: tile0 + u * NW, u < TG, so that their loads (for an accumulation into the float32 state in the
-// workspace: a round trip to L2) are in flight together.  When a row of output tiles goes round the warps GA times,
-// GA consecutive tiles of a warp share their rows (one A fragment serves them); when NW is a multiple of the tiles
-// per row all tiles of a warp share their columns (one B fragment).
-template <bool ACC, int M, int N, int TGMAX = 4, int WOFF = 0, class MC, class EPI, class... PR>
-__device__ __forceinline__ void tile_mma(const MC C, const float alpha, EPI epi, const PR... pr) {
-  constexpr int NW = MB_NW, ntn = N / 8, total = (M / 16) * ntn, per_warp = (total + NW - 1) / NW;
-  constexpr int GA = (ntn % NW == 0) ? ntn / NW : 1;
-  constexpr bool SHARE_B = (NW % ntn == 0) && per_warp > 1;
-  constexpr int TG1 = per_warp < TGMAX ? per_warp : TGMAX;
-  constexpr int TG = TG1 < GA ? GA : TG1 / GA * GA;
-  constexpr int NA = TG / GA, NB = SHARE_B ? 1 : TG;
-  static_assert(TG % GA == 0 && GA <= 4, "tile grouping");
-  // WOFF: the tiles go round the warps starting at warp WOFF -- a product of 8 tiles that shares its phase with
-  // another one is given to the upper eight warps, so that no warp walks both contractions one after the other
-  const int warp = ((threadIdx.x >> 5) + (NW - WOFF)) & (NW - 1), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll 1
-  for (int tile0 = warp; tile0 < total; tile0 += NW * TG) {
-    int i0[TG], j0[TG];
-    bool on[TG];
-    constexpr int NC = TG == 1 ? 2 : 1;  // a lone output tile: two accumulators take turns, halving the chain of products
-    float acc[TG * NC][4];
-    float2 cin[TG][2];
-#pragma unroll
-    for (int u = 0; u < TG; ++u) {
-      const int tile = tile0 + u * NW;
-      on[u] = tile < total;
-      const int tl = on[u] ? tile : tile0, mt = tl / ntn;
-      i0[u] = 16 * mt;
-      j0[u] = 8 * (tl - mt * ntn);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[u][q] = acc[u + (NC - 1) * TG][q] = 0.f;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        cin[u][h] = make_float2(0.f, 0.f);
-        if constexpr (ACC)
-          if (on[u]) cin[u][h] = c_load(C, i0[u] + g + 8 * h, j0[u] + 2 * t);
-      }
-    }
-    auto run = [&](const auto P) {
-      typedef typename std::remove_cv<typename std::remove_reference<decltype(P)>::type>::type PT;
-      constexpr int K = PT::K;
-      // operands in the workspace: the whole contraction unrolled, so that the loads of all steps are in flight
-      // (shared-memory operands: four steps; at 48 to 192 streams that and the second accumulator of a lone tile take 2.7 %
-      // off the kernel, 946 -> 918 us at 192 streams of 32 stages; more steps, or the operands of two tiles or steps by one
-      // ldmatrix.x4, give nothing)
-      constexpr bool GLOBAL = is_global_operand<decltype(PT::A)>::value || is_global_operand<decltype(PT::B)>::value;
-#pragma unroll(GLOBAL ? 16 : (K >= 64 ? 4 : 1))
-      for (int k0 = 0; k0 < K; k0 += 16) {
-        uint32_t pa[NA][4], pb[NB][2];
-#pragma unroll
-        for (int u = 0; u < TG; ++u) {
-          if (u % GA == 0) load_A(P.A, i0[u], k0, lane, pa[u / GA]);
-          if (u == 0 || !SHARE_B) load_B(P.B, k0, j0[u], lane, pb[SHARE_B ? 0 : u]);
-        }
-#pragma unroll
-        for (int u = 0; u < TG; ++u) {
-          const uint32_t(&a)[4] = pa[u / GA];
-          const uint32_t(&b_)[2] = pb[SHARE_B ? 0 : u];
-          mma_bf16(acc[NC == 2 && (k0 & 16) ? u + TG : u], a[0], a[1], a[2], a[3], b_[0], b_[1]);
-        }
-      }
-    };
-    (run(pr), ...);
-    if constexpr (NC == 2)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[0][q] += acc[1][q];
-#pragma unroll
-    for (int u = 0; u < TG; ++u)
-      if (on[u]) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int i = i0[u] + g + 8 * h, j = j0[u] + 2 * t;
-          const float x = cin[u][h].x + alpha * acc[u][2 * h], y = cin[u][h].y + alpha * acc[u][2 * h + 1];
-          if constexpr (std::is_same<EPI, NoEpi>::value) c_store(C, i, j, x, y);
-          else epi(i, j, x, y);
-        }
-      }
-  }
-}
-
-// M[R][C] (float32 master in tensor memory) += alpha * sum over p of A_p^T B_p for token tiles A_p [16][R] and
-// B_p [16][C] (bf16, shared memory, rows of LDA / LDB elements): the rank-16 updates of the state and of its gradient.
-// The warp's eight output tiles are the ones tile_mma would deal it (tile w + 16 u: for the 64 x 256 matrices row tile
-// u / 2 and column tile w + 16 (u % 2), for the 256 x 64 ones row tile 2 u + w / 8 and column tile w % 8), so that the
-// operand copies written by the epilogue line up with what the other products read; every shared-memory address is a
-// per-thread base plus a compile-time offset.  epi(u, h, x, y) receives the finished pair (row g + 8 h of tile u,
-// columns 2 t, 2 t + 1) for the copies it keeps (u and h are compile-time constants after unrolling).
-template <int R, int C, int LDA, int LDB, int NP, class EPI>
-__device__ __forceinline__ void rank16_update(const MatM<R, C> M, const float alpha, EPI epi,
-                                              const uint32_t (&a_tiles)[NP], const uint32_t (&b_tiles)[NP]) {
-  static_assert((R == HD && C == MB_E) || (R == MB_E && C == HD), "the two shapes of the state matrices");
-  constexpr bool WIDE = C == MB_E;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // A^T fragment of rows i0 .. i0 + 15: the four 8 x 8 blocks of the stored [token][row] tile, read transposed
-  const uint32_t a_off = ((((lane & 7) + 8 * (lane >> 4)) * LDA + 8 * ((lane >> 3) & 1) + (WIDE ? 0 : 16 * (warp >> 3))) * 2);
-  const uint32_t b_off = (((lane & 15) * LDB + (WIDE ? 8 * warp : 8 * (warp & 7))) * 2);
-  float acc[8][4];
-#pragma unroll
-  for (int u = 0; u < 8; ++u)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[u][q] = 0.f;
-#pragma unroll
-  for (int pi = 0; pi < NP; ++pi) {
-    if constexpr (WIDE) {
-      uint32_t fa[4][4], fb[2][2];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) ldsm_x4_t(fa[m], a_tiles[pi] + a_off + 16 * m * 2);
-#pragma unroll
-      for (int n = 0; n < 2; ++n) ldsm_x2_t(fb[n], b_tiles[pi] + b_off + 128 * n * 2);
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        mma_bf16(acc[u], fa[u >> 1][0], fa[u >> 1][1], fa[u >> 1][2], fa[u >> 1][3], fb[u & 1][0], fb[u & 1][1]);
-    } else {
-      uint32_t fa[8][4], fb[2];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) ldsm_x4_t(fa[u], a_tiles[pi] + a_off + 32 * u * 2);
-      ldsm_x2_t(fb, b_tiles[pi] + b_off);
-#pragma unroll
-      for (int u = 0; u < 8; ++u) mma_bf16(acc[u], fa[u][0], fa[u][1], fa[u][2], fa[u][3], fb[0], fb[1]);
-    }
-  }
-  float tm[32];
-  tmem_ld32(M.taddr, tm);
-#pragma unroll
-  for (int u = 0; u < 8; ++u)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float x = tm[4 * u + 2 * h] + alpha * acc[u][2 * h], y = tm[4 * u + 2 * h + 1] + alpha * acc[u][2 * h + 1];
-      tm[4 * u + 2 * h] = x;
-      tm[4 * u + 2 * h + 1] = y;
-      epi(u, h, x, y);
-    }
-  tmem_st32(M.taddr, tm);
-}
-
-// ---- element-wise helpers --------------------------------------------------------------------------------------
-// tanh(x) = 1 - 2 / (1 + e^{2x}) with the fast exponential and division (relative error ~1e-6, as in the forward kernel)
-__device__ __forceinline__ float tanh_fast(float x) { return 1.f - __fdividef(2.f, 1.f + __expf(2.f * x)); }
-// gelu(x), gelu'(x) and (D2) gelu''(x) from one tanh
-template <bool D2>
-__device__ __forceinline__ void gelu_all(float x, float& f, float& d1, float& d2) {
-  const float x2 = x * x, th = tanh_fast(GELU_C0 * x * (1.f + GELU_C1 * x2));
-  const float hs = 0.5f * x * (1.f - th * th), du = GELU_C0 * (1.f + 3.f * GELU_C1 * x2);
-  f = 0.5f * x * (1.f + th);
-  d1 = hs * du + 0.5f * (1.f + th);
-  if constexpr (D2) d2 = (1.f - th * th) * du + hs * (6.f * GELU_C0 * GELU_C1 * x - 2.f * th * du * du);
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// a pair of adjacent bf16 elements of a tile (even column)
-__device__ __forceinline__ float2 ldb2(const bf* p) {
-  const uint32_t v = *reinterpret_cast<const uint32_t*>(p);
-  return make_float2(bf16_lo(v), bf16_hi(v));
-}
-__device__ __forceinline__ void stb2(bf* p, float x, float y) { *reinterpret_cast<uint32_t*>(p) = pack_bf16(x, y); }
-__device__ __forceinline__ float ldb(const bf* p) { return __bfloat162float(*p); }
+// float [16][64] exchange tile: column groups of 8 permuted by the row, so that the 64-bit accesses of an accumulator
+// fragment (4 rows x 4 column pairs per half-warp) fall in distinct banks
+__device__ __forceinline__ uint32_t off_x(int row, int col) { return (uint32_t)(row * 256 + ((col ^ ((row & 3) << 3)) << 2)); }
 
-// visit the column pairs of a [16][E] tile / of a [16][F] tile (one pair per thread) / the elements of a [16][16] tile
-template <class Fn>
-__device__ __forceinline__ void for_e2(Fn f) {
-#pragma unroll
-  for (int it = 0; it < CS * MB_E / 2 / MB_THREADS; ++it) {
-    const int e = threadIdx.x + it * MB_THREADS;
-    f(e / (MB_E / 2), 2 * (e % (MB_E / 2)));
+// gelu(z), gelu'(z) and (D2) gelu''(z) of a pair from one tanh.  tanh(x) = 1 - 2 / (1 + e^{2x}) with the fast exponential and
+// division (relative error ~1e-6, as in the forward kernel)
+template <bool D2>
+__device__ __forceinline__ F2 gelu_pair(F2 z, F2& d1, F2& d2) {
+  const F2 z2 = f2mul(z, z);
+  const F2 inner = f2mul(f2mul(z, f2(GELU_C0)), f2fma(z2, f2(GELU_C1), f2(1.f)));
+  const F2 th = f2(1.f - __fdividef(2.f, 1.f + __expf(2.f * inner.x)), 1.f - __fdividef(2.f, 1.f + __expf(2.f * inner.y)));
+  const F2 hz = f2mul(z, f2(0.5f)), sech2 = f2fma(f2neg(th), th, f2(1.f));
+  const F2 du = f2fma(z2, f2(3.f * GELU_C0 * GELU_C1), f2(GELU_C0)), hs = f2mul(hz, sech2);
+  d1 = f2fma(hs, du, f2fma(th, f2(0.5f), f2(0.5f)));
+  if constexpr (D2) {
+    const F2 e = f2fma(f2mul(f2mul(th, du), du), f2(-2.f), f2mul(z, f2(6.f * GELU_C0 * GELU_C1)));
+    d2 = f2fma(sech2, du, f2mul(hs, e));
   }
-}
-template <class Fn>
-__device__ __forceinline__ void for_f2(Fn f) {
-  static_assert(CS * HD / 2 == MB_THREADS, "one pair per thread");
-  f((int)threadIdx.x / (HD / 2), 2 * ((int)threadIdx.x % (HD / 2)));
-}
-template <class Fn>
-__device__ __forceinline__ void for_c(Fn f) {
-  if (threadIdx.x < CS * CS) f((int)threadIdx.x / CS, (int)threadIdx.x % CS);
+  return f2fma(hz, th, hz);
 }
 
-struct __align__(16) MlpBwdSmem {
-  // bf16 operand tiles
-  bf gd1[CS][EB], gd2[CS][EB], x2[CS][EB], g1[CS][EB];  // gelu'(z1), gelu''(z1), gelu(z1), g1
-  bf z1b[CS][EB], x2b[CS][EB];  // gelu'(z1b) (then scratch: l o x2, column partials), gelu(z1b)
-  bf t1[CS][EB], t2[CS][EB], t3[CS][EB], t4[CS][EB];  // g1p | dz1b;  dg1, dh;  gl2;  dz1 (and column partials)
-  bf q[CS][FB], k[CS][FB], v[CS][FB], dO[CS][FB], g2[CS][FB], g2p[CS][FB], dz2b[CS][FB], dz2[CS][FB];
-  bf m1[CS][CB], m2[CS][CB], m1n[CS][CB], m2n[CS][CB], da1[CS][CB], da2[CS][CB];  // m*n = -m*
-  bf w1[HD][EB], w2[MB_E][FB];  // bf16 shadows of the float32 state in the workspace
-  // float32 tiles
-  float z2[CS][FP], z2b[CS][FP], dg2[CS][FP], dk[CS][FP], gl1[CS][FP];
-  float eta[CS][CP], a1[CS][CP], a2[CS][CP], dm[CS][CP], deta[CS][CP];
-  float lr[CS], te[CS], ell[CS], dell[CS];
-  float b1[MB_E], db1[MB_E], b2[HD], db2[HD];  // biases and their gradients stay on chip for the whole walk
-  float dgam[HD], dbet[HD], gam[HD], bet[HD];  // this stream's LayerNorm parameter gradients; the parameters
+// The thread's place, read anew in every interval of a stage: what follows from it (a dozen addresses) is then formed where
+// it is used instead of being kept across the loop, which would push the tiles' values into local memory.
+struct Place {
+  int tid, warp, lane, g, t;
+  __device__ __forceinline__ Place() {
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    warp = tid >> 5;
+    lane = tid & 31;
+    g = lane >> 2;
+    t = lane & 3;
+  }
+  // ldmatrix address of an A fragment in a token tile; k-step ks: ^ (ks << 5)
+  __device__ __forceinline__ uint32_t a_off() const { return lane_off_A(lane, 0); }
+  // of a B fragment (both n-tiles) in a [256][64] matrix whose rows are this warp's 16 hidden features; k-step ks: ^ (ks << 5)
+  __device__ __forceinline__ uint32_t bn_off() const {
+    return (16 * warp + (lane & 7) + ((lane >> 4) << 3)) * 128 + ((((lane >> 3) & 1) ^ (lane & 7)) << 4);
+  }
+  // pair (row g, this warp's hidden column 2 t) of a 16 x 256 tile; n-tile: ^ 16, row g + 8: + 1024
+  __device__ __forceinline__ uint32_t e_off() const {
+    return (warp >> 2) * TILE_BF16_BYTES + g * 128 + (((2 * (warp & 3)) ^ g) << 4) + 4 * t;
+  }
+  // this warp's share of the masters: matrix warp / 4 (W1, W2, dW1, dW2), lane quarter warp % 4 = hidden features
+  // 32 (warp % 4) + lane and, 64 columns on, those + 128
+  __device__ __forceinline__ int mi() const { return warp >> 2; }
+  __device__ __forceinline__ uint32_t tm(uint32_t tmem) const { return tmem + ((32u * (uint32_t)(warp & 3)) << 16) + 128u * (uint32_t)mi(); }
+  __device__ __forceinline__ int rc() const { return 2 * lane; }  // row-wise steps: row = warp, columns rc, rc + 1
 };
-static_assert(sizeof(MlpBwdSmem) + 1024 <= 227 * 1024, "shared-memory tiles exceed one SM");
-static_assert(sizeof(bf) * CS * EB >= sizeof(float) * MB_NW * 2 * HD, "column partials alias a [16][E] tile");
+#define TTT_PLACE \
+  const Place P;  \
+  [[maybe_unused]] const int tid = P.tid, warp = P.warp, lane = P.lane, g = P.g, t = P.t, rc = P.rc();
 
-// G = d/dz of 0.5 |LN(z) - (v - k)|^2 for a [16][64] tile (rust/core/src/util.rs:155-182); one row per warp, the
-// lane owns columns 2 lane, 2 lane + 1
-template <bool SAVE>
-__device__ __forceinline__ void ln_l2_grad_tile(MlpBwdSmem& S, const float (*z)[FP], bf (*G)[FB], float eps,
-                                                uint32_t* g2p_global) {
-  const int r = threadIdx.x >> 5, c = 2 * (threadIdx.x & 31);
-  const float2 zz = *reinterpret_cast<const float2*>(&z[r][c]);
-  const float mu = warp_sum(zz.x + zz.y) * (1.f / HD);
-  const float var = warp_sum((zz.x - mu) * (zz.x - mu) + (zz.y - mu) * (zz.y - mu)) * (1.f / HD);
-  const float rs = 1.f / sqrtf(var + eps);
-  const float2 vv = ldb2(&S.v[r][c]), kk = ldb2(&S.k[r][c]);
-  const float x0 = (zz.x - mu) * rs, x1 = (zz.y - mu) * rs;
-  const float gx0 = (S.gam[c] * x0 + S.bet[c] - (vv.x - kk.x)) * S.gam[c];
-  const float gx1 = (S.gam[c + 1] * x1 + S.bet[c + 1] - (vv.y - kk.y)) * S.gam[c + 1];
-  const float s1 = warp_sum(gx0 + gx1) * (1.f / HD);
-  const float s2 = warp_sum(gx0 * x0 + gx1 * x1) * (1.f / HD);
-  const float G0 = (gx0 - s1 - x0 * s2) * rs, G1 = (gx1 - s1 - x1 * s2) * rs;
-  stb2(&G[r][c], G0, G1);
-  if constexpr (SAVE) {  // lr o G, rounded once from the float32 value
-    const uint32_t v = pack_bf16(S.lr[r] * G0, S.lr[r] * G1);
-    g2p_global[(r * HD + c) >> 1] = v;
-    *reinterpret_cast<uint32_t*>(&S.g2p[r][c]) = v;
-  }
-}
-
-// column sums of a [16][N] bf16 tile (rows of ld elements) added, with sign, to dst[N]
-__device__ __forceinline__ void add_colsum(float* dst, const bf* tile, int N, int ld, float sign) {
-  for (int c = threadIdx.x; c < N; c += MB_THREADS) {
-    float s = 0.f;
-#pragma unroll
-    for (int r = 0; r < CS; ++r) s += ldb(tile + r * ld + c);
-    dst[c] += sign * s;
-  }
-}
-
-__global__ void __launch_bounds__(MB_THREADS, 1) ttt_mlp_bwd_kernel(const MlpBwdParams p) {
-  extern __shared__ __align__(16) uint8_t mlp_bwd_smem[];
-  MlpBwdSmem& S = *reinterpret_cast<MlpBwdSmem*>(mlp_bwd_smem);
+__global__ void __launch_bounds__(MB_THREADS, 1)
+    ttt_mlp_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                       const MlpBwdParams p) {
+  using SM = MlpBwdSmem;
   typedef __nv_bfloat16 T;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr uint32_t TL = SM::TL, ET = SM::ET;
+  extern __shared__ __align__(1024) uint8_t mlp_bwd_smem[];
+  const uint32_t base0 = smem_u32(mlp_bwd_smem);
   const int NS = p.NS;
-  constexpr int F = HD, E = MB_E;
-  constexpr int HO_B1 = MLP_HO_B1, HO_B2 = MLP_HO_B2, HO_DB1 = MLP_HO_DB1, HO_DB2 = MLP_HO_DB2, HO_DG = MLP_HO_DG,
-                HO_DB = MLP_HO_DB;
-  static_assert(HO_B2 == E && HO_DB1 == E + F && HO_DB2 == 2 * E + F && HO_DG == 2 * E + 2 * F &&
-                    HO_DB == 2 * E + 3 * F && HO_DB + F == MLP_BWD_HANDOFF_FLOATS, "hand-off record");
-  float* const b1 = S.b1;
-  float* const b2 = S.b2;
-  float* const db1 = S.db1;
-  float* const db2 = S.db2;
-  __shared__ int s_item;
-  __shared__ uint32_t s_tmem;
-  // Tensor memory, all 512 columns (shared memory keeps the block alone on its SM): the float32 masters of the state
-  // and of its gradient while a work item runs (see MatM).  The warp that allocates frees it at the end of the kernel;
-  // every way out of the item loop below leads there.
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  const uint32_t barL = base0 + SM::BAR, barG = barL + 8, barM = barL + 16;
+  int* const s_item = reinterpret_cast<int*>(mlp_bwd_smem + SM::BAR + 24);
+  const uint32_t* const s_tmem = reinterpret_cast<const uint32_t*>(mlp_bwd_smem + SM::BAR + 28);
+  if ((base0 & 1023u) != 0) {  // (the tiles need it; dynamic shared memory starts there when there is no static one)
+    if (threadIdx.x == 0) report_timeout(p.status, 2, 0);
+    return;
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  // Tensor memory, all 512 columns (shared memory keeps the block alone on its SM).  The warp that allocates frees it at
+  // the end of the kernel; every way out of the item loop leads there.
+  if (threadIdx.x < 32) tmem_alloc(base0 + SM::BAR + 28, 512);
+  if (threadIdx.x == 32) {
+    mbar_init(barL, 1);
+    mbar_init(barG, 1);
+    mbar_init(barM, 1);
+    fence_mbar_init();
+    prefetch_tmap(&tm_q);
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
+    prefetch_tmap(&tm_do);
+  }
+  tmem_fence_before_sync();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_mine = s_tmem + ((32u * (uint32_t)(warp & 3)) << 16) + 128u * (uint32_t)(warp >> 2);
-  // workspace <-> tensor memory, this thread's 32 floats of one matrix (MatG stores a 16 x 8 tile as 128 consecutive
-  // floats in the order of the accumulator registers: tile index = the index rank16_update deals by)
-  auto master_in = [&](const float* M, const uint32_t taddr) {
-    float v[32];
-    const float* src = M + warp * 128 + 8 * (lane >> 2) + 2 * (lane & 3);
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float2 f = __ldcg(reinterpret_cast<const float2*>(src + u * (MB_NW * 128) + 64 * h));
-        v[4 * u + 2 * h] = f.x;
-        v[4 * u + 2 * h + 1] = f.y;
-      }
-    tmem_st32(taddr, v);
-  };
-  auto master_out = [&](float* M, const uint32_t taddr) {
-    float v[32];
-    tmem_ld32(taddr, v);
-    float* dst = M + warp * 128 + 8 * (lane >> 2) + 2 * (lane & 3);
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        *reinterpret_cast<float2*>(dst + u * (MB_NW * 128) + 64 * h) = make_float2(v[4 * u + 2 * h], v[4 * u + 2 * h + 1]);
-  };
+  tmem_fence_after_sync();
+  const uint32_t tmem = *s_tmem;
+  const float te_last = ld_as_float<T>(p.token_eta, CS - 1);
+  // the masters of W1, W2 are carried divided by wscale = -te15, so that a stage's update accumulates directly (te15 = 0:
+  // they never move)
+  const bool w_moves = te_last != 0.f;
+  const float wscale = w_moves ? -te_last : 1.f;
+  if (threadIdx.x < CS) sts_f(base0 + SM::TE + 4 * threadIdx.x, ld_as_float<T>(p.token_eta, threadIdx.x));
 
-  // Persistent block.  A stream is a chain of 2 NCH work items: its chunks of CH stages in pass 1 (ranks 0 ..
-  // NCH-1, forward), then in pass 2 (ranks NCH .. 2 NCH-1, backward).  Items are handed out rank by rank over all
-  // streams, so an item only waits for an item with a smaller index (its predecessor in the chain), which is done or
-  // held by a resident block: the launch cannot deadlock while all blocks are co-resident (cooperative launch).
-  // Between items the stream's state lives in the workspace: the four float32 matrices anyway, the biases, their
-  // gradients and the LayerNorm parameter gradients in a small hand-off record.
-  // When the forward has already filled the workspace (pass1_done) the chains start at rank NCH.
-  const int rank0 = p.pass1_done ? p.NCH : 0;
-  const int nitems = p.nstreams * (2 * p.NCH - rank0);
-#ifdef TTT_MLP_TRACE
-  unsigned long long tr_acc[16] = {0}, tr_last = 0;
-#endif
+  const int nitems = p.nstreams * p.NCH;
+  uint32_t nload = 0, nmma = 0;  // stages whose inputs have been asked for / batches of products issued (barrier parities)
+  int failed = 0;
   while (true) {
-    if (tid == 0) s_item = atomicAdd(&p.sched[0], 1);
+    // Persistent block.  A stream is a chain of NCH work items, its chunks of CH stages from the last to the first.  Items
+    // are handed out rank by rank over all streams, so an item only waits for an item with a smaller index, which is
+    // done or held by a resident block.  Between items a stream's masters, bias gradients and LayerNorm parameter
+    // gradients are in the workspace.
+    if (threadIdx.x == 0) *s_item = atomicAdd(&p.sched[0], 1);
     __syncthreads();
-    const int item = s_item;
+    const int item = *s_item;
     __syncthreads();
     if (item >= nitems) break;
-    const int rel = item / p.nstreams, rank = rank0 + rel, stream = item - rel * p.nstreams, head = stream % p.H;
-    const bool pass1 = rank < p.NCH;
-    const int chunk = pass1 ? rank : 2 * p.NCH - 1 - rank;
-    const int s_lo = chunk * p.CH, s_hi = min(s_lo + p.CH, NS);
-    const size_t row_base = (size_t)stream * p.T;
-
-  // per-stream workspace: W1 [F][E], W2 [E][F], dW1, dW2 (float32, in the tile order of MatG), the hand-off record,
-  // then g1p [NS][16][E], g2p [NS][16][F] (bf16), then b1 | b2 at the start of every stage [NS][E + F] (float32),
-  // then the bf16 operand copies of dW1 and dW2
-  float* ws = p.workspace + (size_t)stream * p.ws_stride;
-  float* W1 = ws;
-  float* W2 = W1 + F * E;
-  float* dW1 = W2 + E * F;
-  float* dW2 = dW1 + F * E;
-  float* ho = dW2 + E * F;
-  bf* g1p_all = reinterpret_cast<bf*>(ho + MLP_BWD_HANDOFF_FLOATS);
-  bf* g2p_all = g1p_all + (size_t)NS * CS * E;
-  float* bst = reinterpret_cast<float*>(g2p_all + (size_t)NS * CS * F);  // [NS][E + F]: b1, b2 at the start of a stage
-  bf* dW1h = reinterpret_cast<bf*>(bst + (size_t)NS * (E + F));            // bf16 operand copies of dW1, dW2 (MatH)
-  bf* dW2h = dW1h + F * E;
-
-  if (rel > 0) {
-    // wait (bounded) until the previous item of this stream has published its state
-    int ok = 1;
-    if (tid == 0) {
-      ok = 0;
-      const volatile int* flag = p.sched + 1 + stream;
-      for (uint32_t it = 0; it < (1u << 24); ++it) {
-        if (*flag >= rel) {
-          ok = 1;
-          break;
+    const int rank = item / p.nstreams, stream = item - rank * p.nstreams, head = stream % p.H;
+    const int chunk = p.NCH - 1 - rank, s_lo = chunk * p.CH, s_hi = min(s_lo + p.CH, NS) - 1;
+    const int row_base = stream * p.T;
+    float* const ws = p.workspace + (size_t)stream * p.ws_stride;
+    float* const ho = ws + 4 * HD * MB_E;
+    const uint8_t* const rec0 = reinterpret_cast<const uint8_t*>(ho + MLP_BWD_HANDOFF_FLOATS);
+    if (rank > 0) {
+      // wait (bounded) until the previous item of this stream has published its state
+      int ok = 1;
+      if (threadIdx.x == 0) {
+        ok = 0;
+        const volatile int* flag = p.sched + 1 + stream;
+        for (uint32_t it = 0; it < (1u << 24); ++it) {
+          if (*flag >= rank) {
+            ok = 1;
+            break;
+          }
+          __nanosleep(100);
         }
-        __nanosleep(100);
+        __threadfence();
       }
-      __threadfence();
+      if (__syncthreads_or(ok ? 0 : 1)) {
+        if (threadIdx.x == 0) report_timeout(p.status, 1, item);
+        break;
+      }
     }
-    if (__syncthreads_or(ok ? 0 : 1)) {
-      if (tid == 0 && p.status != nullptr && atomicCAS(p.status, 0u, (uint32_t)KST_TIMEOUT) == 0u) {
-        p.status[1] = 1u;
-        p.status[2] = blockIdx.x;
-        p.status[3] = (uint32_t)item;
+    auto issue_inputs = [&](int s, int buf) {
+      const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
+      const int r0 = row_base + s * CS;
+      const uint32_t in = base0 + SM::IN + buf * 3 * TL;
+      mbar_expect_tx(barL, 4 * TL + ET);
+      tma_load_2d(in, &tm_q, 0, r0, barL);
+      tma_load_2d(in + TL, &tm_k, 0, r0, barL);
+      tma_load_2d(in + 2 * TL, &tm_do, 0, r0, barL);
+      bulk_load_1d(base0 + SM::X2 + buf * ET, rec + MLP_REC_X2, ET, barL);
+      bulk_load_1d(base0 + SM::G2P, rec + MLP_REC_G2P, TL, barL);
+    };
+    auto issue_late = [&](int s) {  // what is read until I4: V, and G1p where the partial sums of I3 are
+      mbar_expect_tx(barG, ET + TL);
+      tma_load_2d(base0 + SM::V, &tm_v, 0, row_base + s * CS, barG);
+      bulk_load_1d(base0 + SM::G1P, rec0 + (size_t)s * MLP_REC_BYTES + MLP_REC_G1P, ET, barG);
+    };
+    // the lines of a stage's record that are read late (G1p) or by ordinary loads, asked into L2
+    auto prefetch_record = [&](int s) {
+      const int tid = threadIdx.x;
+      const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
+      if (tid < 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_G1P + 128 * tid));
+      else if (tid < 64 + 76) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_Z2 + 128 * (tid - 64)));
+    };
+    // what a thread reads of a stage by itself: its pair of Z2 and Zb2 and the row's statistics, its hidden columns of b1
+    F2 zz, zzb, b1v[2], st2;
+    float4 st1;
+    auto load_first = [&](int s) {
+      TTT_PLACE
+      const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
+      zz = ldg_now2(rec + MLP_REC_Z2 + 8 * tid);
+      st1 = ldg_now4(rec + MLP_REC_STAT + 32 * warp);
+    };
+    auto load_own = [&](int s) {
+      load_first(s);
+      TTT_PLACE
+      const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
+      zzb = ldg_now2(rec + MLP_REC_ZB2 + 8 * tid);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) b1v[nt] = ldg_now2(rec + MLP_REC_B1 + 8 * (8 * warp + 4 * nt + t));
+      st2 = ldg_now2(rec + MLP_REC_STAT + 32 * warp + 16);
+    };
+    auto put_rates = [&](int buf, float lr) {  // 16 lanes
+      const int lane = threadIdx.x & 31;
+      sts_f(base0 + SM::LR + buf * CS * 4 + 4 * lane, lr);
+      sts_f(base0 + SM::LR + (2 + buf) * CS * 4 + 4 * lane, te_last * lr);
+    };
+    // W1_s, W2_s from W1_{s+1}, W2_{s+1} (inputs of stage s in buffer `buf`): one thread
+    auto undo_updates = [&](int buf) {
+      if (!w_moves) return;
+      const uint32_t k = base0 + SM::IN + buf * 3 * TL + TL;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        umma_update(tmem + 64 * h, base0 + SM::G1P + h * 2 * TL, k, UPD_IDESC | UPD_NEGATE);
+        umma_update(tmem + 128 + 64 * h, base0 + SM::X2 + buf * ET + h * 2 * TL, base0 + SM::G2P, UPD_IDESC | UPD_NEGATE);
       }
+    };
+
+    // ---- item begins: masters into tensor memory, gradients carried from the later chunk, the inputs of its last stage
+    int s = s_hi;
+    uint32_t buf = nload & 1;
+    if (threadIdx.x == 0) {
+      issue_inputs(s, buf);
+      issue_late(s);
+    }
+    load_own(s);
+    if (threadIdx.x < CS) put_rates(buf, ld_as_float<T>(p.lr, row_base + (size_t)s * CS + threadIdx.x));
+    const bool fresh = rank == 0;  // the gradients w.r.t. the final state are zero
+    F2 db1v[2], dgam = f2(0.f), dbet = f2(0.f);
+    {
+      TTT_PLACE
+      const float4* src = reinterpret_cast<const float4*>(ws + P.mi() * HD * MB_E) + lane;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          float v[8][4];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (P.mi() < 2 || !fresh) f = __ldcg(src + ((h * 4 + (warp & 3)) * 16 + cc * 8 + j) * 32);
+            v[j][0] = f.x; v[j][1] = f.y; v[j][2] = f.z; v[j][3] = f.w;
+          }
+          tmem_st_8x4(P.tm(tmem) + 64 * h + 32 * cc, v);
+        }
+      tmem_wait_st();
+      if (tid < 2 * HD) sts_f(base0 + SM::LN + 4 * tid, ld_as_float<T>(tid < HD ? p.ln_g : p.ln_b, (size_t)head * HD + (tid & (HD - 1))));
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+        db1v[nt] = fresh ? f2(0.f) : __ldcg(reinterpret_cast<const float2*>(ho + MLP_HO_DB1) + 8 * warp + 4 * nt + t);
+      if (tid < HD) sts_f(base0 + SM::DB2 + 4 * tid, fresh ? 0.f : __ldcg(ho + MLP_HO_DB2 + tid));
+    }
+    tmem_fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x >> 5 == 15 && elect_one()) {
+      tmem_fence_after_sync();
+      if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+      undo_updates(buf);
+      umma_commit_to(barM);
+    }
+
+    while (true) {
+      // (addresses formed anew in every stage: kept across the loop they would push the tiles' values into local memory)
+      uint32_t base = base0;
+      asm volatile("" : "+r"(base));
+      const uint32_t sAD = base + SM::AD, sDET = base + SM::DET, sDB2 = base + SM::DB2, sTE = base + SM::TE, sLN = base + SM::LN;
+      // ---- I1. The stage's operands: bf16 copies of the four masters; both LayerNorms, a row per warp
+      const uint32_t tq = base + SM::IN + buf * 3 * TL, tk = tq + TL, tdo = tk + TL, tx2 = base + SM::X2 + buf * ET;
+      const uint32_t sLR = base + SM::LR + buf * CS * 4, sELL = sLR + 2 * CS * 4;
+      if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+      ++nload;
+      {
+        TTT_PLACE
+        const uint32_t r_off = off_bf16(warp, rc);
+        const F2 gam = lds_f2(sLN + 4 * rc), bet = lds_f2(sLN + 4 * (HD + rc));
+        const F2 vv = ld_pair<T>(base + SM::V, warp, rc), kk = ld_pair<T>(tk, warp, rc), dd = ld_pair<T>(tdo, warp, rc);
+        const F2 xh = f2mul(f2add(zz, f2(-st1.x)), f2(st1.y));
+        const F2 xb = f2mul(f2add(zzb, f2(-st2.x)), f2(st2.y)), tt = f2mul(dd, gam);
+        const F2 gy = f2sub(f2fma(gam, xh, bet), f2sub(vv, kk));
+        const F2 sums = warp_sum2(f2hsum(tt), f2hsum(f2mul(tt, xb)));
+        const F2 G = f2mul(f2fma(xh, f2(-st1.w), f2fma(gy, gam, f2(-st1.z))), f2(st1.y));
+        const F2 dzb = f2mul(f2fma(xb, f2(sums.y * (-1.f / HD)), f2add(tt, f2(sums.x * (-1.f / HD)))), f2(st2.y));
+        dgam = f2fma(dd, xb, dgam);
+        dbet = f2add(dbet, dd);
+        // (the products of the stage before may still be reading the two tiles)
+        if (!mbar_wait_bounded(barM, nmma & 1)) failed = 1;
+        ++nmma;
+        tmem_fence_after_sync();
+        sts32(base + SM::G2 + r_off, pack_bf16(G.x, G.y));
+        sts32(base + SM::DZ2B + r_off, pack_bf16(dzb.x, dzb.y));
+      }
+      {
+        TTT_PLACE
+        const float sc = P.mi() < 2 ? wscale : 1.f;
+        const uint32_t dst = base + SM::W1 + P.mi() * SM::WM + (32 * (warp & 3) + lane) * 128;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int cc = 0; cc < 2; ++cc) {
+            float v[8][4];
+            tmem_ld_8x4(P.tm(tmem) + 64 * h + 32 * cc, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint32_t w[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const F2 x = f2mul(f2(v[2 * i + (j >> 1)][2 * (j & 1)], v[2 * i + (j >> 1)][2 * (j & 1) + 1]), f2(sc));
+                w[j] = pack_bf16(x.x, x.y);
+              }
+              asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + h * 128 * 128 + (((4 * cc + i) ^ (lane & 7)) << 4)),
+                           "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                           : "memory");
+            }
+          }
+      }
+      tmem_fence_before_sync();
+      failed = __syncthreads_or(failed);  // 1
+      if (failed) break;
+      if (s > s_lo) {
+        if (threadIdx.x == 0) issue_inputs(s - 1, buf ^ 1);
+        prefetch_record(s - 1);
+      }
+
+      // ---- I2. From Z1 to dH, this warp's 16 hidden features
+      F2 gd1[2][2], dz1a[2][2];  // gelu'(Z1); dG1 o H o gelu''(Z1)
+      float dx[2][4];            // dX2 so far: dA2^T X2b - l o gl2
+      {
+        TTT_PLACE
+        const uint32_t a_off = P.a_off(), bn_off = P.bn_off(), e_st = P.e_off();
+        const float te_row[2] = {lds_f(sTE + 4 * g), lds_f(sTE + 4 * (g + 8))};
+        const float ell[2] = {lds_f(sELL + 4 * g), lds_f(sELL + 4 * (g + 8))};
+        const F2 lrc[2] = {lds_f2(sLR + 8 * t), lds_f2(sLR + 32 + 8 * t)};
+        float z1[2][4] = {}, zq[2][4] = {}, at[2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          uint32_t ak[4], aq[4], bw[4];
+          ldsm_x4(ak, (tk + a_off) ^ (ks << 5));
+          ldsm_x4(aq, (tq + a_off) ^ (ks << 5));
+          ldsm_x4(bw, (base + SM::W1 + bn_off) ^ (ks << 5));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            mma4(z1[nt], ak, bw[2 * nt], bw[2 * nt + 1]);
+            mma4(zq[nt], aq, bw[2 * nt], bw[2 * nt + 1]);
+            mma4(at[nt], aq, ak[nt], ak[nt + 2]);           // Q K^T (the blocks of an A fragment are those of a B fragment)
+          }
+        }
+        uint32_t x2[2][2], gd2[2][2];  // bf16 pairs
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            F2 d2;
+            const F2 x = gelu_pair<true>(f2add(pr(z1[nt], r), b1v[nt]), gd1[nt][r], d2);
+            x2[nt][r] = pack_bf16(x.x, x.y);
+            gd2[nt][r] = pack_bf16(d2.x, d2.y);
+            zq[nt][2 * r] += b1v[nt].x;
+            zq[nt][2 * r + 1] += b1v[nt].y;
+          }
+        // -M1 = -eta o (1 + A1), as an A operand
+        uint32_t am1[4];
+#pragma unroll
+        for (int jt = 0; jt < 2; ++jt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int i = g + 8 * r, j = 8 * jt + 2 * t;
+            const F2 e = f2mul(lrc[jt], f2(-te_row[r])), m = f2fma(pr(at[jt], r), e, e);
+            am1[2 * jt + r] = pack_bf16(j <= i ? m.x : 0.f, j + 1 <= i ? m.y : 0.f);
+            if (warp == 0) {
+              if (j <= i) sts_f(sAD + 4 * (17 * i + j), at[jt][2 * r]);
+              if (j + 1 <= i) sts_f(sAD + 4 * (17 * i + j + 1), at[jt][2 * r + 1]);
+            }
+          }
+        float h[2][4] = {}, dzw[2][4] = {}, gl2[2][4] = {}, dm[2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          uint32_t ag[4], az[4], bw[4], bd[4];
+          ldsm_x4(ag, (base + SM::G2 + a_off) ^ (ks << 5));
+          ldsm_x4(az, (base + SM::DZ2B + a_off) ^ (ks << 5));
+          ldsm_x4(bw, (base + SM::W2 + bn_off) ^ (ks << 5));
+          ldsm_x4(bd, (base + SM::DW2 + bn_off) ^ (ks << 5));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            mma4(h[nt], ag, bw[2 * nt], bw[2 * nt + 1]);     // H = G2 W2^T
+            mma4(dzw[nt], az, bw[2 * nt], bw[2 * nt + 1]);   // dZb2 W2^T
+            mma4(gl2[nt], ag, bd[2 * nt], bd[2 * nt + 1]);   // G2 dW2^T
+            mma4(dm[nt], az, ag[nt], ag[nt + 2]);            // dZb2 G2^T = -dM2
+          }
+        }
+        uint32_t ad2[4];  // dA2 = dM2 o eta, as an A operand
+#pragma unroll
+        for (int jt = 0; jt < 2; ++jt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int i = g + 8 * r, j = 8 * jt + 2 * t;
+            const F2 m = f2mul(pr(dm[jt], r), f2mul(lrc[jt], f2(-te_row[r])));
+            ad2[2 * jt + r] = pack_bf16(j <= i ? m.x : 0.f, j + 1 <= i ? m.y : 0.f);
+            if (warp == 1) {
+              if (j <= i) sts_f(sAD + 4 * (17 * j + i + 1), -dm[jt][2 * r]);
+              if (j + 1 <= i) sts_f(sAD + 4 * (17 * (j + 1) + i + 1), -dm[jt][2 * r + 1]);
+            }
+          }
+        uint32_t tb[2][2];  // a tile's own columns as a B operand (contraction over the tokens)
+        float del[2] = {0.f, 0.f};
+        // G1 = H o gelu'(Z1);  Zb1 = Q W1 + b1 - M1 G1
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 g1 = f2mul(pr(h[nt], r), gd1[nt][r]);
+            const uint32_t v = pack_bf16(g1.x, g1.y);
+            sts32(base + SM::G1 + (e_st ^ (nt << 4)) + r * 1024, v);
+            tb[nt][r] = movm_t(v);
+            const F2 q = f2fma(g1, db1v[nt], f2mul(pr(gl2[nt], r), unpack_bf16(x2[nt][r])));
+            del[r] += f2hsum(q);
+          }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) mma4(zq[nt], am1, tb[nt][0], tb[nt][1]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          del[r] = quad_sum(del[r]);
+          if (t == 0) sts_f(sDET + 4 * (16 * warp + g + 8 * r), del[r]);
+        }
+        // dZb2 W2^T + dA2 X2
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+          mma4(dzw[nt], ad2, movm_t(x2[nt][0]), movm_t(x2[nt][1]));
+        // X2b = gelu(Zb1);  dZ1b = (dZb2 W2^T + dA2 X2) o gelu'(Zb1);  dX2 = dA2^T X2b - l o gl2 + ..
+        const uint32_t ad2t[4] = {movm_t(ad2[0]), movm_t(ad2[2]), movm_t(ad2[1]), movm_t(ad2[3])};
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          uint32_t xb[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            F2 d1, unused;
+            const F2 x = gelu_pair<false>(pr(zq[nt], r), d1, unused), d = f2mul(pr(dzw[nt], r), d1);
+            const uint32_t v = pack_bf16(x.x, x.y), w = pack_bf16(d.x, d.y);
+            sts32(base + SM::X2B + (e_st ^ (nt << 4)) + r * 1024, v);
+            sts32(base + SM::DZ1B + (e_st ^ (nt << 4)) + r * 1024, w);
+            xb[r] = movm_t(v);
+            tb[nt][r] = movm_t(w);
+            dx[nt][2 * r] = -ell[r] * gl2[nt][2 * r];
+            dx[nt][2 * r + 1] = -ell[r] * gl2[nt][2 * r + 1];
+          }
+          mma4(dx[nt], ad2t, xb[0], xb[1]);
+        }
+        // dG1 = -M1^T dZ1b - l o (K dW1 + db1);  dH = dG1 o gelu'(Z1)
+        const uint32_t am1t[4] = {movm_t(am1[0]), movm_t(am1[2]), movm_t(am1[1]), movm_t(am1[3])};
+        float u1[2][4] = {};  // K dW1
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          uint32_t ak[4], bd[4];
+          ldsm_x4(ak, (tk + a_off) ^ (ks << 5));
+          ldsm_x4(bd, (base + SM::DW1 + bn_off) ^ (ks << 5));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(u1[nt], ak, bd[2 * nt], bd[2 * nt + 1]);
+        }
+        constexpr uint32_t ONES = 0x3f803f80u;
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          float d[4] = {}, cs[4] = {};
+          mma4(d, am1t, tb[nt][0], tb[nt][1]);
+          mma_bf16(cs, ONES, ONES, ONES, ONES, tb[nt][0], tb[nt][1]);  // column sums
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 dg = f2fma(f2add(pr(u1[nt], r), db1v[nt]), f2(-ell[r]), pr(d, r));
+            const F2 dh = f2mul(dg, gd1[nt][r]);
+            dz1a[nt][r] = f2mul(f2mul(dg, pr(h[nt], r)), unpack_bf16(gd2[nt][r]));
+            sts32(base + SM::DH + (e_st ^ (nt << 4)) + r * 1024, pack_bf16(dh.x, dh.y));
+          }
+          db1v[nt] = f2add(db1v[nt], f2(cs[0], cs[1]));
+        }
+      }
+      __syncthreads();  // 2
+
+      // ---- I3. Contractions over the hidden features that the chain waits for: dH W2 - l o (X2 dW2) (four partial sums), and
+      //      the causal matrices A2 = X2b X2^T, dZ1b G1^T (eight warps, a quarter of one of them each)
+      float dell_row;
+      load_first(s);  // Z2's LayerNorm once more, for I4
+      {
+        TTT_PLACE
+        const uint32_t a_off = P.a_off();
+        const int np = warp & 3, kq = warp >> 2;
+        const uint32_t b_off = (64 * kq + (lane & 15)) * 128 + (((2 * np + (lane >> 4)) ^ (lane & 7)) << 4);
+        float p1[2][4] = {}, p2[2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          uint32_t ax[4], ah[4], bd[4], bw[4];
+          ldsm_x4(ax, (tx2 + kq * TL + a_off) ^ (ks << 5));
+          ldsm_x4(ah, (base + SM::DH + kq * TL + a_off) ^ (ks << 5));
+          ldsm_x4_t(bd, base + SM::DW2 + b_off + ks * 2048);
+          ldsm_x4_t(bw, base + SM::W2 + b_off + ks * 2048);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            mma4(p1[nt], ax, bd[2 * nt], bd[2 * nt + 1]);
+            mma4(p2[nt], ah, bw[2 * nt], bw[2 * nt + 1]);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float l = lds_f(sELL + 4 * (g + 8 * r));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+            sts_f2(base + SM::PART + kq * 4096 + off_x(g + 8 * r, 16 * np + 8 * nt + 2 * t), f2fma(pr(p1[nt], r), f2(-l), pr(p2[nt], r)));
+        }
+        if (warp < 8) {
+          const int q = warp & 3;
+          const uint32_t ta = (warp < 4 ? base + SM::X2B : base + SM::DZ1B) + q * TL + a_off;
+          const uint32_t tb_ = (warp < 4 ? tx2 : base + SM::G1) + q * TL + a_off;
+          float c[2][4] = {};
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            uint32_t a[4], b[4];
+            ldsm_x4(a, ta ^ (ks << 5));
+            ldsm_x4(b, tb_ ^ (ks << 5));
+            mma4(c[0], a, b[0], b[2]);
+            mma4(c[1], a, b[1], b[3]);
+          }
+          const uint32_t dst = (warp < 4 ? base + SM::EXD : base + SM::EXG) + q * 1024;
+#pragma unroll
+          for (int jt = 0; jt < 2; ++jt)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {  // transposed, [j][i], rows of 16: the reader takes a column of the matrix
+              sts_f(dst + 4 * (16 * (8 * jt + 2 * t) + g + 8 * r), c[jt][2 * r]);
+              sts_f(dst + 4 * (16 * (8 * jt + 2 * t + 1) + g + 8 * r), c[jt][2 * r + 1]);
+            }
+        }
+        dell_row = lane < 16 ? lds_f(sDET + 4 * (16 * lane + warp)) : 0.f;  // row sums of the 16 warps (finished in I4)
+      }
+      __syncthreads();  // 3
+
+      // ---- I4. Token row j = warp: dG2, the second derivative of the LayerNorm (dZ2, d target), the row's eta gradients
+      F2 dT;
+      {
+        TTT_PLACE
+        const uint32_t r_off = off_bf16(warp, rc), x_off = off_x(warp, rc);
+        const F2 bet = lds_f2(sLN + 4 * (HD + rc)), vk = f2sub(ld_pair<T>(base + SM::V, warp, rc), ld_pair<T>(tk, warp, rc));
+        const float lr_j = lds_f(sLR + 4 * warp), ell_j = lds_f(sELL + 4 * warp);
+        const F2 db2v = lds_f2(sDB2 + 4 * rc), gam = lds_f2(sLN + 4 * rc);
+        const float rs = st1.y, sg = st1.z, sgx = st1.w;
+        const F2 xh = f2mul(f2add(zz, f2(-st1.x)), f2(rs)), gy = f2sub(f2fma(gam, xh, bet), vk);  // its output minus the target
+        const F2 gxh = f2mul(gy, gam), G = f2mul(f2fma(xh, f2(-sgx), f2add(gxh, f2(-sg))), f2(rs));
+        F2 dg2 = f2mul(db2v, f2(-ell_j));
+#pragma unroll
+        for (int kq = 0; kq < 4; ++kq) dg2 = f2add(dg2, lds_f2(base + SM::PART + kq * 4096 + x_off));
+        // lane i < 16: column j of the causal matrices
+        const uint32_t sM2 = base + SM::EXG + 3 * 1024 + 64 * warp;  // (each lane has read the partial sum there)
+        float m2 = 0.f, dlr = 0.f;
+        if (lane < 16) {
+          float a2 = 0.f, d1 = 0.f;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            a2 += lds_f(base + SM::EXD + q * 1024 + 4 * (16 * warp + lane));
+            d1 -= lds_f(base + SM::EXG + q * 1024 + 4 * (16 * warp + lane));
+          }
+          const float te_i = lds_f(sTE + 4 * lane);
+          float deta = 0.f, da1 = 0.f;
+          if (lane >= warp) {
+            m2 = te_i * lr_j * (1.f + a2);
+            deta = lds_f(sAD + 4 * (17 * warp + lane + 1)) * (1.f + a2) + d1 * (1.f + lds_f(sAD + 4 * (17 * lane + warp)));
+            da1 = d1 * te_i * lr_j;
+          }
+          dlr = deta * te_i;
+          sts_f(sM2 + 4 * lane, m2);
+          sts_f(sDET + 4 * (17 * lane + warp), deta * lr_j);
+          *reinterpret_cast<bf*>(mlp_bwd_smem + SM::DA1 + 2 * (24 * lane + warp)) = __float2bfloat16_rn(da1);
+        }
+        // dG2 = dH W2 - l o (X2 dW2) - l (x) db2 - M2^T dZb2
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < CS; i += 4) {
+          float m[4];
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(m[0]), "=f"(m[1]), "=f"(m[2]), "=f"(m[3]) : "r"(sM2 + 4 * i) : "memory");
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dg2 = f2fma(ld_pair<T>(base + SM::DZ2B, i + j, rc), f2(-m[j]), dg2);
+        }
+        const F2 vv = f2mul(dg2, f2(-rs));
+        const float sums = warp_sum4_spread(f2hsum(vv), dlr, f2hsum(f2mul(vv, xh)), dell_row + f2hsum(f2mul(G, db2v)));
+        const float sv = __shfl_sync(0xffffffffu, sums, 0) * (1.f / HD), svx = __shfl_sync(0xffffffffu, sums, 16) * (1.f / HD);
+        const F2 dgxh = f2fma(xh, f2(svx), f2fma(dg2, f2(rs), f2(sv))), dy = f2mul(gam, dgxh);
+        dgam = f2add(dgam, f2fma(gy, dgxh, f2mul(dy, xh)));
+        dbet = f2add(dbet, dy);
+        dT = f2neg(dy);
+        const F2 dxh = f2fma(dy, gam, f2fma(gxh, f2(svx), f2mul(vv, f2(sgx))));
+        const F2 sd = warp_sum2(f2hsum(dxh), f2hsum(f2fma(dxh, xh, f2mul(dg2, G))));
+        const F2 dz2 = f2fma(xh, f2(sd.y * (-1.f / HD) * rs), f2mul(f2add(dxh, f2(sd.x * (-1.f / HD))), f2(rs)));
+        sts32(base + SM::DZ2 + r_off, pack_bf16(dz2.x, dz2.y));
+        if (lane == 8) sts_f(base + SM::DLP + 4 * warp, sums);
+        if (lane == 24) sts_f(base + SM::DLP + 4 * (CS + warp), sums);
+        fence_proxy_async_smem();  // (G1p lands where the partial sums were)
+      }
+      __syncthreads();  // 4
+      if (s > s_lo && threadIdx.x == 0) issue_late(s - 1);
+
+      // ---- I5. dX2 += dZ2 W2^T;  dZ1 = dG1 o H o gelu''(Z1) + dX2 o gelu'(Z1)
+      {
+        TTT_PLACE
+        const uint32_t a_off = P.a_off(), bn_off = P.bn_off(), e_st = P.e_off();
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          uint32_t az[4], bw[4];
+          ldsm_x4(az, (base + SM::DZ2 + a_off) ^ (ks << 5));
+          ldsm_x4(bw, (base + SM::W2 + bn_off) ^ (ks << 5));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(dx[nt], az, bw[2 * nt], bw[2 * nt + 1]);
+        }
+        constexpr uint32_t ONES = 0x3f803f80u;
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          uint32_t tb[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 d = f2fma(pr(dx[nt], r), gd1[nt][r], dz1a[nt][r]);
+            const uint32_t v = pack_bf16(d.x, d.y);
+            sts32(base + SM::DZ1 + (e_st ^ (nt << 4)) + r * 1024, v);
+            tb[r] = movm_t(v);
+          }
+          float cs[4] = {};
+          mma_bf16(cs, ONES, ONES, ONES, ONES, tb[0], tb[1]);
+          db1v[nt] = f2add(db1v[nt], f2(cs[0], cs[1]));
+        }
+        fence_proxy_async_smem();  // every operand tile of the products below has been written by now
+      }
+      __syncthreads();  // 5
+
+      // ---- I6. dW1 += Q^T dZ1b + K^T dZ1, dW2 += X2^T dZ2 + X2b^T dZb2 + dH^T G2, and W1, W2 one stage back: tcgen05, in
+      //      the background of dq = dZ1b W1^T + dA1 K, dk = dZ1 W1^T + dA1^T Q (warps 0..7, eight features each) and
+      //      gl1 = G1 dW1^T (warps 8..15)
+      if (threadIdx.x >> 5 == 15 && elect_one()) {
+        tmem_fence_after_sync();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t d1 = tmem + 256 + 64 * h, d2 = d1 + 128, o = h * 2 * TL;
+          umma_update(d1, base + SM::DZ1B + o, tq, UPD_IDESC);
+          umma_update(d1, base + SM::DZ1 + o, tk, UPD_IDESC);
+          umma_update(d2, tx2 + o, base + SM::DZ2, UPD_IDESC);
+          umma_update(d2, base + SM::X2B + o, base + SM::DZ2B, UPD_IDESC);
+          umma_update(d2, base + SM::DH + o, base + SM::G2, UPD_IDESC);
+        }
+      }
+      __syncwarp();
+      if (s > s_lo) load_own(s - 1);
+      const size_t r0 = (size_t)(row_base + s * CS) * HD;
+      {
+        TTT_PLACE
+        const uint32_t a_off = P.a_off();
+        const int nt = warp & 7, col = 8 * nt + 2 * t;
+        const uint32_t b_off = lane * 128 + ((nt ^ (lane & 7)) << 4);
+        const uint32_t f_off = (lane & 15) * 128 + ((nt ^ (lane & 7)) << 4);  // the tile's 16 tokens as k, columns 8 nt.. as n
+        if (warp < 8) {
+          float aq[2][4] = {}, ak[2][4] = {};
+#pragma unroll
+          for (int kp = 0; kp < 8; ++kp) {
+            uint32_t a0[4], a1[4], c0[4], c1[4], b[4];
+            const uint32_t o = (kp >> 1) * TL + a_off, x = (kp & 1) << 6;
+            ldsm_x4_t(b, base + SM::W1 + b_off + kp * 4096);
+            ldsm_x4(a0, (base + SM::DZ1B + o) ^ x);
+            ldsm_x4(a1, (base + SM::DZ1B + o) ^ (x + 32));
+            ldsm_x4(c0, (base + SM::DZ1 + o) ^ x);
+            ldsm_x4(c1, (base + SM::DZ1 + o) ^ (x + 32));
+            mma4(aq[0], a0, b[0], b[1]);
+            mma4(ak[0], c0, b[0], b[1]);
+            mma4(aq[1], a1, b[2], b[3]);
+            mma4(ak[1], c1, b[2], b[3]);
+          }
+          uint32_t da[4], dat[4], bk[2], bq[2], bz[2], by[2];
+          ldsm_x4(da, base + SM::DA1 + (lane & 15) * 48 + (lane >> 4) * 16);                                // dA1
+          ldsm_x4_t(dat, base + SM::DA1 + ((lane & 7) + ((lane >> 4) << 3)) * 48 + ((lane >> 3) & 1) * 16);  // dA1^T
+          ldsm_x2_trans(bk, tk + f_off);
+          ldsm_x2_trans(bq, tq + f_off);
+          ldsm_x2_trans(bz, base + SM::DZ2B + f_off);
+          ldsm_x2_trans(by, base + SM::DZ2 + f_off);
+          mma4(aq[0], da, bk[0], bk[1]);
+          mma4(ak[0], dat, bq[0], bq[1]);
+          constexpr uint32_t ONES = 0x3f803f80u;
+          float cs[4] = {}, ct[4] = {};
+          mma_bf16(cs, ONES, ONES, ONES, ONES, bz[0], bz[1]);
+          mma_bf16(ct, ONES, ONES, ONES, ONES, by[0], by[1]);
+          if (g == 0) sts_f2(sDB2 + 4 * col, f2add(lds_f2(sDB2 + 4 * col), f2(cs[0] + ct[0], cs[1] + ct[1])));
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 o = f2add(f2add(pr(aq[0], r), pr(aq[1], r)), ld_pair<T>(tdo, g + 8 * r, col));
+            static_cast<uint32_t*>(p.d_q)[(r0 + (g + 8 * r) * HD + col) >> 1] = pack_bf16(o.x, o.y);
+            sts_f2(base + SM::EXD + off_x(g + 8 * r, col), f2add(pr(ak[0], r), pr(ak[1], r)));
+          }
+        } else {
+          float c[2][4] = {};
+#pragma unroll
+          for (int kp = 0; kp < 8; ++kp) {
+            uint32_t a0[4], a1[4], b[4];
+            const uint32_t o = (kp >> 1) * TL + a_off, x = (kp & 1) << 6;
+            ldsm_x4_t(b, base + SM::DW1 + b_off + kp * 4096);
+            ldsm_x4(a0, (base + SM::G1 + o) ^ x);
+            ldsm_x4(a1, (base + SM::G1 + o) ^ (x + 32));
+            mma4(c[0], a0, b[0], b[1]);
+            mma4(c[1], a1, b[2], b[3]);
+          }
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 gl = f2add(pr(c[0], r), pr(c[1], r)), kk = ld_pair<T>(tk, g + 8 * r, col);
+            const float l = lds_f(sELL + 4 * (g + 8 * r)), d = quad_sum(f2hsum(f2mul(gl, kk)));
+            if (t == 0) sts_f(base + SM::DLG + 4 * (CS * nt + g + 8 * r), d);
+            sts_f2(base + SM::EXG + off_x(g + 8 * r, col), f2mul(gl, f2(-l)));
+          }
+          if (warp == 14 && s > s_lo && lane < CS) put_rates(buf ^ 1, ld_as_float<T>(p.lr, row_base + (size_t)(s - 1) * CS + lane));
+          if (warp == 15 && elect_one()) {
+            if (s > s_lo) {
+              if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+              undo_updates(buf ^ 1);
+            }
+            umma_commit_to(barM);
+          }
+          __syncwarp();
+        }
+      }
+      __syncthreads();  // 6
+      // ---- outputs of the stage: dk = (products) - l o gl1 - dT, dv = dT; the eta factors
+      {
+        TTT_PLACE
+        const uint32_t x_off = off_x(warp, rc);
+        const F2 dk = f2sub(f2add(lds_f2(base + SM::EXD + x_off), lds_f2(base + SM::EXG + x_off)), dT);
+        const size_t at = (r0 >> 1) + tid;
+        static_cast<uint32_t*>(p.d_k)[at] = pack_bf16(dk.x, dk.y);
+        static_cast<uint32_t*>(p.d_v)[at] = pack_bf16(dT.x, dT.y);
+      }
+      if (threadIdx.x >> 5 == 13) {
+        const int lane = threadIdx.x & 31;
+        // dell[j] = -(gl1[j].K[j] + G1[j].db1 + gl2[j].X2[j] + G2[j].db2)
+        float dell = 0.f, dte = 0.f, lr = 0.f;
+        if (lane < CS) {
+          dell = lds_f(base + SM::DLP + 4 * (CS + lane));
+#pragma unroll
+          for (int w = 0; w < 8; ++w) dell += lds_f(base + SM::DLG + 4 * (CS * w + lane));
+          dell = -dell;
+          lr = lds_f(sLR + 4 * lane);
+#pragma unroll
+          for (int j = 0; j < CS; ++j) dte += lds_f(sDET + 4 * (17 * lane + j));
+          st_from_float<T>(p.d_lr, row_base + (size_t)s * CS + lane, lds_f(base + SM::DLP + 4 * lane) + dell * te_last);
+        }
+        const float sum = warp_sum(dell * lr);
+        if (lane < CS) p.part_te[(size_t)row_base + (size_t)s * CS + lane] = lane == CS - 1 ? dte + sum : dte;
+      }
+      if (s == s_lo) break;
+      --s;
+      buf ^= 1;
+    }
+    if (!failed) {
+      if (!mbar_wait_bounded(barM, nmma & 1)) failed = 1;
+      ++nmma;
+      tmem_fence_after_sync();
+    }
+    failed = __syncthreads_or(failed);
+    if (failed) {
+      if (threadIdx.x == 0) report_timeout(p.status, 3, item);
       break;
     }
-  }
-  if (tid < HD) {
-    S.gam[tid] = ld_as_float<T>(p.ln_g, (size_t)head * HD + tid);
-    S.bet[tid] = ld_as_float<T>(p.ln_b, (size_t)head * HD + tid);
-    const bool fresh = rank <= p.NCH;  // the LayerNorm parameter gradients start with pass 2
-    S.dgam[tid] = fresh ? 0.f : __ldcg(ho + HO_DG + tid);
-    S.dbet[tid] = fresh ? 0.f : __ldcg(ho + HO_DB + tid);
-  }
-  if (tid < CS) S.te[tid] = ld_as_float<T>(p.token_eta, (size_t)tid);
-  if (rank == 0) {
-    for (int e = tid; e < F * E; e += MB_THREADS) {
-      const bf a = static_cast<const bf*>(p.w1)[(size_t)stream * F * E + e];
-      const bf b = static_cast<const bf*>(p.w2)[(size_t)stream * F * E + e];
-      W1[MatG<F, E, false>::at(e / E, e % E)] = __bfloat162float(a);
-      W2[MatG<E, F, false>::at(e / F, e % F)] = __bfloat162float(b);
-      S.w1[e / E][e % E] = a;
-      S.w2[e / F][e % F] = b;
-    }
-    for (int e = tid; e < E; e += MB_THREADS) b1[e] = ld_as_float<T>(p.b1, (size_t)stream * E + e);
-    if (tid < F) b2[tid] = ld_as_float<T>(p.b2, (size_t)stream * F + tid);
-  } else {
-    // bf16 shadows from the float32 state the previous item left in the workspace
-    for (int e = 2 * tid; e < F * E; e += 2 * MB_THREADS) {
-      const float2 a = __ldcg(reinterpret_cast<const float2*>(W1 + MatG<F, E, false>::at(e / E, e % E)));
-      const float2 b = __ldcg(reinterpret_cast<const float2*>(W2 + MatG<E, F, false>::at(e / F, e % F)));
-      stb2(&S.w1[e / E][e % E], a.x, a.y);
-      stb2(&S.w2[e / F][e % F], b.x, b.y);
-    }
-    for (int e = tid; e < E; e += MB_THREADS) b1[e] = __ldcg(ho + HO_B1 + e);
-    if (tid < F) b2[tid] = __ldcg(ho + HO_B2 + tid);
-  }
-  if (!pass1) {
-    const bool fresh = rank == p.NCH;  // first item of pass 2: the gradients w.r.t. the final state are zero
-    if (fresh)
-      for (int e = tid; e < F * E; e += MB_THREADS) {
-        dW1[e] = 0.f;
-        dW2[e] = 0.f;
-        reinterpret_cast<uint32_t*>(dW1h)[e] = 0u;  // both bf16 copies: 2 F E elements = F E words
-      }
-    for (int e = tid; e < E; e += MB_THREADS) db1[e] = fresh ? 0.f : __ldcg(ho + HO_DB1 + e);
-    if (tid < F) db2[tid] = fresh ? 0.f : __ldcg(ho + HO_DB2 + tid);
-  }
-  __syncthreads();
-  // the masters of this item: W1, W2 (and in pass 2 dW1, dW2) from the workspace, where the previous item of the
-  // stream (or the forward kernel, or the lines above) left them
-  const uint32_t tW1a = tmem_mine, tW2a = tmem_mine + 32, tdW1a = tmem_mine + 64, tdW2a = tmem_mine + 96;
-  master_in(W1, tW1a);
-  master_in(W2, tW2a);
-  if (!pass1) {
-    master_in(dW1, tdW1a);
-    master_in(dW2, tdW2a);
-  }
-  const float te_last = S.te[CS - 1];
-// per-phase cycle counts of block 0 (instrumented builds only; written to the status words after the walk)
-#ifdef TTT_MLP_TRACE
-  tr_last = clock64();
-#define TRM(i) { __syncthreads(); const unsigned long long n_ = clock64(); tr_acc[i] += n_ - tr_last; tr_last = n_; }
-#else
-#define TRM(i)
-#endif
-
-  // ---- operand / output views
-  const MatM<F, E> mW1{tW1a}, mdW1{tdW1a};
-  const MatM<E, F> mW2{tW2a}, mdW2{tdW2a};
-  const MatH<F, E, false> hdW1{dW1h};
-  const MatH<E, F, false> hdW2{dW2h};
-  const MatT<1, 1> none{nullptr};
-  typedef SB<EB, false> TE;
-  typedef SB<FB, false> TF_;
-  typedef SB<CB, false> TC;
-  const TE sx2{smem_u32(S.x2)}, sg1{smem_u32(S.g1)}, sz1b{smem_u32(S.z1b)}, sx2b{smem_u32(S.x2b)};
-  const TE st1{smem_u32(S.t1)}, st2{smem_u32(S.t2)}, st3{smem_u32(S.t3)}, st4{smem_u32(S.t4)}, sw1{smem_u32(S.w1)};
-  const TF_ sq{smem_u32(S.q)}, sk{smem_u32(S.k)}, sg2{smem_u32(S.g2)}, sg2p{smem_u32(S.g2p)}, sdz2b{smem_u32(S.dz2b)};
-  const TF_ sdz2{smem_u32(S.dz2)}, sw2{smem_u32(S.w2)};
-  const TC sm1{smem_u32(S.m1)}, sm2{smem_u32(S.m2)}, sm1n{smem_u32(S.m1n)}, sm2n{smem_u32(S.m2n)};
-  const TC sda1{smem_u32(S.da1)}, sda2{smem_u32(S.da2)};
-  const MatT<FP, 1> mdq{&S.z2b[0][0]}, mdg2{&S.dg2[0][0]}, mdk{&S.dk[0][0]}, mgl1{&S.gl1[0][0]};
-  float(*const dq)[FP] = S.z2b;  // z2b is dead once the output LayerNorm has been differentiated: its tile then holds dq
-  const MatT<CP, 1> ma1{&S.a1[0][0]}, ma2{&S.a2[0][0]}, mdm{&S.dm[0][0]};
-  const NoEpi noepi;
-
-  // W += sign * A^T B with the float32 master in tensor memory and its bf16 shadow refreshed together
-  // (t1 / g2p hold lr o g1 / lr o g2, the operands of the forward's update; its scale te[15] is applied here)
-  // where this thread's pairs of a 64 x 256 / 256 x 64 matrix go (see rank16_update for the tiles of a warp): in the
-  // bf16 shadows in shared memory and in the bf16 operand copies in the workspace (MatH), as element offsets of the
-  // pair (tile u = 0, half h = 0); the other pairs follow at compile-time distances
-  const int fg = lane >> 2, ft = lane & 3;
-  const uint32_t w1_at = smem_u32(S.w1) + 2 * (fg * EB + 8 * warp + 2 * ft);
-  const uint32_t w2_at = smem_u32(S.w2) + 2 * ((16 * (warp >> 3) + fg) * FB + 8 * (warp & 7) + 2 * ft);
-  const int h_sub = ((((fg >> 1) & 3) * 4 + ft) * 4) + (fg & 1) * 2;
-  bf* const dW1h_at = dW1h + warp * 64 + h_sub;
-  bf* const dW2h_at = dW2h + (16 * (warp >> 3) + (warp & 7)) * 64 + h_sub;
-  auto update_w1 = [&](const float sign) {  // W1 += sign * te[15] * K^T t1
-    const uint32_t a[1] = {sk.a}, b[1] = {st1.a};
-    rank16_update<F, E, FB, EB, 1>(mW1, sign * te_last, [&](int u, int h, float x, float y) {
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(w1_at + 2 * ((16 * (u >> 1) + 8 * h) * EB + 128 * (u & 1))), "r"(pack_bf16(x, y)) : "memory");
-    }, a, b);
-  };
-  auto update_w2 = [&](const float sign) {  // W2 += sign * te[15] * X2^T g2p
-    const uint32_t a[1] = {sx2.a}, b[1] = {sg2p.a};
-    rank16_update<E, F, EB, FB, 1>(mW2, sign * te_last, [&](int u, int h, float x, float y) {
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(w2_at + 2 * ((32 * u + 8 * h) * FB)), "r"(pack_bf16(x, y)) : "memory");
-    }, a, b);
-  };
-  // z1 = K W1 + b1, x2 = gelu(z1); z1 itself is only needed through gelu'(z1) and (pass 2) gelu''(z1)
-  auto forward_first_layer = [&](auto d2_tag) {
-    constexpr bool D2 = decltype(d2_tag)::value;
-    tile_mma<false, CS, E>(none, 1.f, [&](int i, int j, float x, float y) {
-      float f0, f1, a0, a1, c0 = 0.f, c1 = 0.f;
-      gelu_all<D2>(x + b1[j], f0, a0, c0);
-      gelu_all<D2>(y + b1[j + 1], f1, a1, c1);
-      stb2(&S.x2[i][j], f0, f1);
-      stb2(&S.gd1[i][j], a0, a1);
-      if constexpr (D2) stb2(&S.gd2[i][j], c0, c1);
-    }, prod<F>(sk, sw1));
-    __syncthreads();
-  };
-  // z2 = x2 W2 + b2, g2 = ln_l2_grad(z2, v - k), g1 = (g2 W2^T) o gelu'(z1)
-  // In pass 1 (save_tag true) l o g1 and l o g2 also go to t1 / g2p and to the workspace.
-  auto forward_second_layer = [&](auto save_tag, uint32_t* g1p, uint32_t* g2p) {
-    constexpr bool SAVE = decltype(save_tag)::value;
-    tile_mma<false, CS, F>(none, 1.f, [&](int i, int j, float x, float y) {
-      *reinterpret_cast<float2*>(&S.z2[i][j]) = make_float2(x + b2[j], y + b2[j + 1]);
-    }, prod<E>(sx2, sw2));
-    __syncthreads();
-    ln_l2_grad_tile<SAVE>(S, S.z2, S.g2, p.eps, g2p);
-    __syncthreads();
-    tile_mma<false, CS, E>(none, 1.f, [&](int i, int j, float x, float y) {
-      const float2 d1 = ldb2(&S.gd1[i][j]);
-      x *= d1.x;
-      y *= d1.y;
-      stb2(&S.g1[i][j], x, y);
-      if constexpr (SAVE) {
-        const uint32_t v = pack_bf16(S.lr[i] * x, S.lr[i] * y);
-        g1p[(i * E + j) >> 1] = v;
-        *reinterpret_cast<uint32_t*>(&S.t1[i][j]) = v;
-      }
-    }, prod<F>(sg2, tr(sw2)));
-    __syncthreads();
-  };
-  // one 16-byte piece per thread: [16][64] bf16 tiles from global memory (128 threads per tile)
-  auto tile_piece = [&](int idx, int& r, int& c) {
-    r = idx >> 3;
-    c = 8 * (idx & 7);
-  };
-
-  // ============================== pass 1: forward walk, saving g1p and g2p ==============================
-  if (pass1)
-  for (int s = s_lo; s < s_hi; ++s) {
-    const size_t r0 = (row_base + (size_t)s * CS) * HD;
-    if (tid < 256) {
-      int r, c;
-      tile_piece(tid & 127, r, c);
-      const T* src = static_cast<const T*>(tid < 128 ? p.xk : p.xv) + r0;
-      bf(*dst)[FB] = tid < 128 ? S.k : S.v;
-      *reinterpret_cast<uint4*>(&dst[r][c]) = *reinterpret_cast<const uint4*>(src + r * HD + c);
-    } else if (tid < 256 + CS) {
-      S.lr[tid - 256] = ld_as_float<T>(p.lr, row_base + (size_t)s * CS + (tid - 256));
-    }
-    for (int e = tid; e < E + F; e += MB_THREADS) bst[(size_t)s * (E + F) + e] = e < E ? b1[e] : b2[e - E];
-    __syncthreads();
-    TRM(0)
-    forward_first_layer(std::false_type{});
-    forward_second_layer(std::true_type{}, reinterpret_cast<uint32_t*>(g1p_all + (size_t)s * CS * E),
-                         reinterpret_cast<uint32_t*>(g2p_all + (size_t)s * CS * F));
-    TRM(1)
-    update_w1(-1.f);
-    update_w2(-1.f);
-    add_colsum(b1, &S.t1[0][0], E, EB, -te_last);
-    add_colsum(b2, &S.g2p[0][0], F, FB, -te_last);
-    __syncthreads();
-    TRM(2)
-  }
-
-  // ============================== pass 2: backward walk ==============================
-  float(*const colpart)[2 * HD] = reinterpret_cast<float(*)[2 * HD]>(&S.z1b[0][0]);  // only while z1b is not live
-  // The inputs of a stage (one 16-byte piece per thread and tile, the lr row, the biases at the start of the stage:
-  // those were saved on the way forward, they are not recovered by undoing the update, since the forward takes its
-  // column sums in float32 and the operand tiles are bf16) are fetched into registers while the previous stage
-  // writes its outputs, and put in place when the stage begins.
-  struct StageIn {
-    uint4 g1v, in, g2v;
-    float bias, lr;
-  };
-  auto fetch = [&](const int s) {
-    StageIn v;
-    const size_t r0 = (row_base + (size_t)s * CS) * HD;
-    v.g1v = __ldcg(reinterpret_cast<const uint4*>(g1p_all + (size_t)s * CS * E) + tid);
-    int r, c;
-    tile_piece(tid & 127, r, c);
-    const int which = tid >> 7;
-    const T* src = static_cast<const T*>(which == 0 ? p.xq : which == 1 ? p.xk : which == 2 ? p.xv : p.d_out) + r0;
-    v.in = *reinterpret_cast<const uint4*>(src + r * HD + c);
-    v.g2v = make_uint4(0u, 0u, 0u, 0u);
-    if (tid < 128) v.g2v = __ldcg(reinterpret_cast<const uint4*>(g2p_all + (size_t)s * CS * F) + tid);
-    v.bias = tid < E + F ? __ldcg(bst + (size_t)s * (E + F) + tid) : 0.f;
-    v.lr = tid < CS ? ld_as_float<T>(p.lr, row_base + (size_t)s * CS + tid) : 0.f;
-    return v;
-  };
-  // the lines fetch(s) will read, asked into L2 a whole stage ahead (the q / k / v / d_out rows come from HBM, and
-  // the fetch sits at the end of a stage with only the output stores between it and the commit that needs its data)
-  auto prefetch_l2 = [&](const int s) {
-    const size_t r0 = (row_base + (size_t)s * CS) * HD;
-    int r, c;
-    tile_piece(tid & 127, r, c);
-    const int which = tid >> 7;
-    const T* src = static_cast<const T*>(which == 0 ? p.xq : which == 1 ? p.xk : which == 2 ? p.xv : p.d_out) + r0;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(src + r * HD + c));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(g1p_all + (size_t)s * CS * E) + tid));
-    if (tid < 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(g2p_all + (size_t)s * CS * F) + tid));
-    if (tid < E + F) asm volatile("prefetch.global.L2 [%0];" ::"l"(bst + (size_t)s * (E + F) + tid));
-  };
-  auto commit = [&](const StageIn& v) {
-    int r, c;
-    tile_piece(tid & 127, r, c);
-    const int which = tid >> 7;
-    bf(*dst)[FB] = which == 0 ? S.q : which == 1 ? S.k : which == 2 ? S.v : S.dO;
-    *reinterpret_cast<uint4*>(&dst[r][c]) = v.in;
-    *reinterpret_cast<uint4*>(&S.t1[tid >> 5][8 * (tid & 31)]) = v.g1v;
-    if (tid < 128) *reinterpret_cast<uint4*>(&S.g2p[r][c]) = v.g2v;
-    if (tid < E) b1[tid] = v.bias;
-    else if (tid < E + F) b2[tid - E] = v.bias;
-    if (tid < CS) {
-      S.lr[tid] = v.lr;
-      S.ell[tid] = te_last * v.lr;
-    }
-  };
-  StageIn nxt;
-  if (!pass1) nxt = fetch(s_hi - 1);
-  if (!pass1)
-  for (int s = s_hi - 1; s >= s_lo; --s) {
-    const size_t r0 = (row_base + (size_t)s * CS) * HD;
-    commit(nxt);
-    if (s > s_lo) prefetch_l2(s - 1);
-    __syncthreads();
-    TRM(3)
-    // ---- state at the start of this stage: undo the stage's updates (W1 first: X2 depends on it)
-    update_w1(1.f);
-    // (in the same phase, since neither depends on the state: the eta matrix and a1 = Q K^T)
-    for_c([&](int i, int j) { S.eta[i][j] = (j <= i) ? S.te[i] * S.lr[j] : 0.f; });
-    tile_mma<false, CS, CS>(ma1, 1.f, noepi, prod<F>(sq, tr(sk)));
-    __syncthreads();
-    for_c([&](int i, int j) {
-      const float a = (j <= i) ? S.a1[i][j] : 0.f, m = S.eta[i][j] * (1.f + a);
-      S.a1[i][j] = a;
-      S.m1[i][j] = __float2bfloat16_rn(m);
-      S.m1n[i][j] = __float2bfloat16_rn(-m);
-    });
-    forward_first_layer(std::true_type{});  // x2 (and the GELU derivatives) of this stage, needed to undo the second layer's update
-    update_w2(1.f);
-    __syncthreads();
-    TRM(4)
-    // ---- forward intermediates of the stage
-    forward_second_layer(std::false_type{}, nullptr, nullptr);
-    TRM(5)
-    tile_mma<false, CS, E>(none, 1.f, [&](int i, int j, float x, float y) {          // z1b = Q W1 - M1 g1 + b1; x2b = gelu
-      float f0, f1, a0, a1, c0, c1;
-      gelu_all<false>(x + b1[j], f0, a0, c0);
-      gelu_all<false>(y + b1[j + 1], f1, a1, c1);
-      stb2(&S.z1b[i][j], a0, a1);  // gelu'(z1b), all that step 3 needs of z1b
-      stb2(&S.x2b[i][j], f0, f1);
-    }, prod<F>(sq, sw1), prod<CS>(sm1n, sg1));
-    __syncthreads();
-    tile_mma<false, CS, CS>(ma2, 1.f, noepi, prod<E>(sx2b, tr(sx2)));              // a2 = x2b x2^T
-    tile_mma<false, CS, F, 4, 8>(mdq, 1.f, noepi, prod<E>(sx2b, sw2));             // z2b = x2b W2 ... (float32 tile)
-    __syncthreads();
-    for_c([&](int i, int j) {
-      const float a = (j <= i) ? S.a2[i][j] : 0.f, m = S.eta[i][j] * (1.f + a);
-      S.a2[i][j] = a;
-      S.m2[i][j] = __float2bfloat16_rn(m);
-      S.m2n[i][j] = __float2bfloat16_rn(-m);
-    });
-    __syncthreads();
-    tile_mma<true, CS, F>(mdq, 1.f, [&](int i, int j, float x, float y) {           // ... - M2 g2 + b2
-      *reinterpret_cast<float2*>(&S.z2b[i][j]) = make_float2(x + b2[j], y + b2[j + 1]);
-    }, prod<CS>(sm2n, sg2));
-    __syncthreads();
-
-    TRM(6)
-    // ---- 1. output LayerNorm: dz2b, LN parameter gradients (one row per warp, columns 2 lane, 2 lane + 1)
+    // ---- item ends: LayerNorm parameter gradients over the 16 rows; the masters and gradients go to the workspace for the
+    //      stream's next item, or (last item) the state gradients to the caller
+    const bool last = rank == p.NCH - 1;
+    TTT_PLACE
     {
-      const int r = warp, c = 2 * lane;
-      const float2 zz = *reinterpret_cast<const float2*>(&S.z2b[r][c]);
-      const float mu = warp_sum(zz.x + zz.y) * (1.f / HD);
-      const float var = warp_sum((zz.x - mu) * (zz.x - mu) + (zz.y - mu) * (zz.y - mu)) * (1.f / HD);
-      const float rs = 1.f / sqrtf(var + p.eps);
-      const float x0 = (zz.x - mu) * rs, x1 = (zz.y - mu) * rs;
-      const float2 d = ldb2(&S.dO[r][c]);
-      const float t0 = d.x * S.gam[c], t1_ = d.y * S.gam[c + 1];
-      const float s1 = warp_sum(t0 + t1_) * (1.f / HD);
-      const float s2 = warp_sum(t0 * x0 + t1_ * x1) * (1.f / HD);
-      stb2(&S.dz2b[r][c], (t0 - s1 - x0 * s2) * rs, (t1_ - s1 - x1 * s2) * rs);
-      // z1b's tile is still live: the partials of this step go through t4, which is free until step 5
-      float(*cp)[2 * HD] = reinterpret_cast<float(*)[2 * HD]>(&S.t4[0][0]);
-      *reinterpret_cast<float2*>(&cp[warp][c]) = make_float2(d.x * x0, d.y * x1);
-      *reinterpret_cast<float2*>(&cp[warp][HD + c]) = make_float2(d.x, d.y);
+      sts_f2(base0 + SM::PART + 4 * (128 * warp + rc), dgam);
+      sts_f2(base0 + SM::PART + 4 * (128 * warp + HD + rc), dbet);
     }
+    if (!last || P.mi() >= 2) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          float v[8][4];
+          tmem_ld_8x4(P.tm(tmem) + 64 * h + 32 * cc, v);
+          const int e = 128 * h + 32 * (warp & 3) + lane;
+          if (!last) {
+            float4* dst = reinterpret_cast<float4*>(ws + P.mi() * HD * MB_E) + lane;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              dst[((h * 4 + (warp & 3)) * 16 + cc * 8 + j) * 32] = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+          } else if (P.mi() == 2) {  // dW1^T [e][k] -> grad_w1 [k][e]
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              st_from_float<T>(p.d_w1, ((size_t)stream * HD + 32 * cc + j) * MB_E + e, v[j >> 2][j & 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              st_from_float<T>(p.d_w2, ((size_t)stream * MB_E + e) * HD + 32 * cc + j, v[j >> 2][j & 3]);
+          }
+        }
+    }
+    if (g == 0) {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const int e = 16 * warp + 8 * nt + 2 * t;
+        if (!last) *reinterpret_cast<float2*>(ho + MLP_HO_DB1 + e) = db1v[nt];
+        else {
+          st_from_float<T>(p.d_b1, (size_t)stream * MB_E + e, db1v[nt].x);
+          st_from_float<T>(p.d_b1, (size_t)stream * MB_E + e + 1, db1v[nt].y);
+        }
+      }
+    }
+    tmem_fence_before_sync();
     __syncthreads();
     if (tid < 2 * HD) {
-      const float(*cp)[2 * HD] = reinterpret_cast<const float(*)[2 * HD]>(&S.t4[0][0]);
-      float s_ = 0.f;
+      float sum = fresh ? 0.f : __ldcg(ho + MLP_HO_DG + tid);
 #pragma unroll
-      for (int w = 0; w < MB_NW; ++w) s_ += cp[w][tid];
-      if (tid < HD) S.dgam[tid] += s_; else S.dbet[tid - HD] += s_;
+      for (int w = 0; w < CS; ++w) sum += lds_f(base0 + SM::PART + 4 * (128 * w + tid));
+      if (!last) ho[MLP_HO_DG + tid] = sum;
+      else p.part_ln[(size_t)stream * 2 * HD + tid] = sum;
+    } else if (tid < 3 * HD) {
+      const int f = tid - 2 * HD;
+      if (!last) ho[MLP_HO_DB2 + f] = lds_f((base0 + SM::DB2) + 4 * f);
+      else st_from_float<T>(p.d_b2, (size_t)stream * HD + f, lds_f((base0 + SM::DB2) + 4 * f));
     }
-    TRM(7)
-    // ---- 2. z2b = x2b W2 + b2 - M2 g2
-    tile_mma<false, CS, CS>(mdm, -1.f, noepi, prod<F>(sdz2b, tr(sg2)));            // dM2 = -tril(dz2b g2^T)
-    tile_mma<false, CS, F, 4, 8>(mdg2, 1.f, noepi, prod<CS>(tr(sm2n), sdz2b));     // dg2 = -M2^T dz2b
-    __syncthreads();
-    for_c([&](int i, int j) {
-      const float d = (j <= i) ? S.dm[i][j] : 0.f;
-      S.da2[i][j] = __float2bfloat16_rn(d * S.eta[i][j]);
-      S.deta[i][j] = d * (1.f + S.a2[i][j]);
-    });
-    __syncthreads();
-    TRM(8)
-    // ---- 3. dz1b = (dz2b W2^T + dA2 x2) o gelu'(z1b)  (kept in t1)
-    tile_mma<false, CS, E>(none, 1.f, [&](int i, int j, float x, float y) {
-      const float2 d1 = ldb2(&S.z1b[i][j]);
-      stb2(&S.t1[i][j], x * d1.x, y * d1.y);
-    }, prod<F>(sdz2b, tr(sw2)), prod<CS>(sda2, sx2));
-    __syncthreads();
-    // ---- 4. z1b = Q W1 + b1 - M1 g1
-    tile_mma<false, CS, CS>(mdm, -1.f, noepi, prod<E>(st1, tr(sg1)));              // dM1 = -tril(dz1b g1^T)
-    // l o K goes to dz2 (free until step 7), l o x2 to z1b (dead after step 3)
-    for_f2([&](int r, int c) {
-      const float2 k_ = ldb2(&S.k[r][c]);
-      stb2(&S.dz2[r][c], S.ell[r] * k_.x, S.ell[r] * k_.y);
-    });
-    for_e2([&](int r, int c) {
-      const float2 x = ldb2(&S.x2[r][c]);
-      stb2(&S.z1b[r][c], S.ell[r] * x.x, S.ell[r] * x.y);
-    });
-    __syncthreads();
-    for_c([&](int i, int j) {
-      const float d = (j <= i) ? S.dm[i][j] : 0.f;
-      S.da1[i][j] = __float2bfloat16_rn(d * S.eta[i][j]);
-      S.deta[i][j] += d * (1.f + S.a1[i][j]);
-    });
-    __syncthreads();
-    tile_mma<false, CS, F>(mdq, 1.f, noepi, prod<E>(st1, tr(sw1)), prod<CS>(sda1, sk));   // dq = dz1b W1^T + dA1 K
-    tile_mma<false, CS, F, 4, 8>(mdk, 1.f, noepi, prod<CS>(tr(sda1), sq));         // dk = dA1^T Q
-    TRM(9)
-    // ---- 5. the four state updates; dW1, db1, dW2, db2 still hold the gradients w.r.t. the next stage's state
-    tile_mma<false, CS, F>(mgl1, 1.f, noepi, prod<E>(sg1, tr(hdW1)));              // gl1 = g1 dW1^T
-    tile_mma<false, CS, E>(st3, 1.f, noepi, prod<F>(sg2, tr(hdW2)));               // gl2 = g2 dW2^T
-    tile_mma<false, CS, E>(none, -1.f, [&](int i, int j, float x, float y) {         // dg1 = -M1^T dz1b - (l o K) dW1 - l (x) db1
-      stb2(&S.t2[i][j], x - S.ell[i] * db1[j], y - S.ell[i] * db1[j + 1]);
-    }, prod<CS>(tr(sm1), st1), prod<F>(sdz2, hdW1));
-    tile_mma<true, CS, F, 4, 8>(mdg2, -1.f, [&](int i, int j, float x, float y) {   // dg2 -= (l o x2) dW2 + l (x) db2
-      *reinterpret_cast<float2*>(&S.dg2[i][j]) = make_float2(x - S.ell[i] * db2[j], y - S.ell[i] * db2[j + 1]);
-    }, prod<E>(sz1b, hdW2));
-    __syncthreads();
-    // dell[j] = -( gl1[j].K[j] + g1[j].db1 + gl2[j].x2[j] + g2[j].db2 )   (one row per warp)
-    {
-      const int r = warp;
-      float acc = 0.f;
-      {
-        const int c = 2 * lane;
-        const float2 gl = *reinterpret_cast<const float2*>(&S.gl1[r][c]), k_ = ldb2(&S.k[r][c]), g_ = ldb2(&S.g2[r][c]);
-        acc += gl.x * k_.x + gl.y * k_.y + g_.x * db2[c] + g_.y * db2[c + 1];
-      }
-#pragma unroll
-      for (int c = 2 * lane; c < E; c += 64) {
-        const float2 g_ = ldb2(&S.g1[r][c]), l2 = ldb2(&S.t3[r][c]), x = ldb2(&S.x2[r][c]);
-        acc += g_.x * db1[c] + g_.y * db1[c + 1] + l2.x * x.x + l2.y * x.y;
-      }
-      acc = warp_sum(acc);
-      if (lane == 0) S.dell[r] = -acc;
+    fence_proxy_async_smem();  // (the next item's G1p lands where the row sums were)
+    if (!last) {
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) *reinterpret_cast<volatile int*>(p.sched + 1 + stream) = rank + 1;
     }
-    for_f2([&](int r, int c) {                                                     // dk -= l o gl1
-      float2* d = reinterpret_cast<float2*>(&S.dk[r][c]);
-      const float2 gl = *reinterpret_cast<const float2*>(&S.gl1[r][c]);
-      *d = make_float2(d->x - S.ell[r] * gl.x, d->y - S.ell[r] * gl.y);
-    });
-    // (no barrier: step 6 reads and writes none of what the two loops above touch)
-    TRM(10)
-    // ---- 6. g1 = h o gelu'(z1), h = g2 W2^T (recomputed):  dz1 = dg1 o h o gelu''(z1) (t4),  dh = dg1 o gelu'(z1) (t2)
-    tile_mma<false, CS, E>(none, 1.f, [&](int i, int j, float hx, float hy) {
-      const float2 d = ldb2(&S.t2[i][j]), d1 = ldb2(&S.gd1[i][j]), d2 = ldb2(&S.gd2[i][j]);
-      stb2(&S.t4[i][j], d.x * hx * d2.x, d.y * hy * d2.y);
-      stb2(&S.t2[i][j], d.x * d1.x, d.y * d1.y);
-    }, prod<F>(sg2, tr(sw2)));
-    __syncthreads();
-    tile_mma<true, CS, F>(mdg2, 1.f, noepi, prod<E>(st2, sw2));                    // dg2 += dh W2
-    __syncthreads();
-    TRM(11)
-    // ---- 7. second derivative through g2 = ln_l2_grad(z2, v - k): dz2, d target (into gl1, which is dead by now),
-    //         LN parameter gradients (column partials in z1b's tile, whose scratch use is over)
-    {
-      const int r = warp, c = 2 * lane;
-      const float2 zz = *reinterpret_cast<const float2*>(&S.z2[r][c]);
-      const float mu = warp_sum(zz.x + zz.y) * (1.f / HD);
-      const float var = warp_sum((zz.x - mu) * (zz.x - mu) + (zz.y - mu) * (zz.y - mu)) * (1.f / HD);
-      const float rs = 1.f / sqrtf(var + p.eps);
-      const float2 vv_ = ldb2(&S.v[r][c]), kk = ldb2(&S.k[r][c]);
-      const float2 uu = *reinterpret_cast<const float2*>(&S.dg2[r][c]);
-      const float xh[2] = {(zz.x - mu) * rs, (zz.y - mu) * rs}, tg[2] = {vv_.x - kk.x, vv_.y - kk.y}, u[2] = {uu.x, uu.y};
-      float gy[2], gxh[2], vv[2], sg = 0.f, sgx = 0.f, sv = 0.f, svx = 0.f;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        gy[e] = S.gam[c + e] * xh[e] + S.bet[c + e] - tg[e];
-        gxh[e] = gy[e] * S.gam[c + e];
-        vv[e] = -u[e] * rs;
-        sg += gxh[e];
-        sgx += gxh[e] * xh[e];
-        sv += vv[e];
-        svx += vv[e] * xh[e];
-      }
-      sg = warp_sum(sg) * (1.f / HD);
-      sgx = warp_sum(sgx) * (1.f / HD);
-      sv = warp_sum(sv) * (1.f / HD);
-      svx = warp_sum(svx) * (1.f / HD);
-      float dxh[2], pg[2], pb[2], dt[2], sd = 0.f, sS = 0.f;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float G = (gxh[e] - sg - xh[e] * sgx) * rs;
-        const float dgxh = u[e] * rs + sv + xh[e] * svx;
-        const float dy = S.gam[c + e] * dgxh;
-        pg[e] = gy[e] * dgxh + dy * xh[e];
-        pb[e] = dy;
-        dxh[e] = dy * S.gam[c + e] + gxh[e] * svx + vv[e] * sgx;
-        sd += dxh[e];
-        sS += -(dxh[e] * xh[e] + u[e] * G) * rs;
-        dt[e] = -S.gam[c + e] * dgxh;  // d target
-      }
-      sd = warp_sum(sd) * (1.f / HD);
-      sS = warp_sum(sS) * (1.f / HD);
-      *reinterpret_cast<float2*>(&S.gl1[r][c]) = make_float2(dt[0], dt[1]);
-      stb2(&S.dz2[r][c], dxh[0] * rs - sd * rs + xh[0] * sS, dxh[1] * rs - sd * rs + xh[1] * sS);
-      *reinterpret_cast<float2*>(&colpart[warp][c]) = make_float2(pg[0], pg[1]);
-      *reinterpret_cast<float2*>(&colpart[warp][HD + c]) = make_float2(pb[0], pb[1]);
-    }
-    __syncthreads();
-    if (tid < 2 * HD) {
-      float s_ = 0.f;
-#pragma unroll
-      for (int w = 0; w < MB_NW; ++w) s_ += colpart[w][tid];
-      if (tid < HD) S.dgam[tid] += s_; else S.dbet[tid - HD] += s_;
-    }
-    TRM(12)
-    // ---- 8./9./10. z2 = x2 W2 + b2, x2 = gelu(z1), z1 = K W1 + b1:
-    //      dx2 = dA2^T x2b + dz2 W2^T - l o gl2  (never stored);  dz1 += dx2 o gelu'(z1) (t4);  dk += dz1 W1^T
-    tile_mma<false, CS, E>(none, 1.f, [&](int i, int j, float x, float y) {
-      const float2 d1 = ldb2(&S.gd1[i][j]), d = ldb2(&S.t4[i][j]), gl2 = ldb2(&S.t3[i][j]);
-      x -= S.ell[i] * gl2.x;
-      y -= S.ell[i] * gl2.y;
-      stb2(&S.t4[i][j], d.x + x * d1.x, d.y + y * d1.y);
-    }, prod<CS>(tr(sda2), sx2b), prod<F>(sdz2, tr(sw2)));
-    __syncthreads();
-    tile_mma<true, CS, F>(mdk, 1.f, noepi, prod<E>(st4, tr(sw1)));
-    TRM(13)
-    // ---- gradients w.r.t. this stage's state (all reads of the next-stage gradients are done): one pass over each
-    //      float32 master, the contraction running over the tokens of all the tile pairs
-    {
-      const uint32_t a[3] = {st2.a, sx2b.a, sx2.a}, b[3] = {sg2.a, sdz2b.a, sdz2.a};
-      rank16_update<E, F, EB, FB, 3>(mdW2, 1.f, [&](int u, int h, float x, float y) {
-        *reinterpret_cast<uint32_t*>(dW2h_at + (4 * u + h) * 512) = pack_bf16(x, y);
-      }, a, b);
-    }
-    {
-      const uint32_t a[2] = {sq.a, sk.a}, b[2] = {st1.a, st4.a};
-      rank16_update<F, E, FB, EB, 2>(mdW1, 1.f, [&](int u, int h, float x, float y) {
-        *reinterpret_cast<uint32_t*>(dW1h_at + ((2 * (u >> 1) + h) * 32 + 16 * (u & 1)) * 64) = pack_bf16(x, y);
-      }, a, b);
-    }
-    add_colsum(db2, &S.dz2b[0][0], F, FB, 1.f);
-    add_colsum(db1, &S.t1[0][0], E, EB, 1.f);
-    TRM(14)
-    // ---- 11. eta factors and outputs of the stage
-    if (tid >= MB_THREADS - CS) {
-      const int i = tid - (MB_THREADS - CS);
-      float dte = 0.f, dlr = 0.f;
-      for (int j = 0; j < CS; ++j) {
-        dte += S.deta[i][j] * S.lr[j];
-        dlr += S.deta[j][i] * S.te[j];
-      }
-      if (i == CS - 1)
-        for (int j = 0; j < CS; ++j) dte += S.dell[j] * S.lr[j];
-      dlr += S.dell[i] * te_last;
-      p.part_te[(size_t)stream * p.T + (size_t)s * CS + i] = dte;
-      st_from_float<T>(p.d_lr, row_base + (size_t)s * CS + i, dlr);
-    }
-    __syncthreads();
-    add_colsum(db2, &S.dz2[0][0], F, FB, 1.f);
-    add_colsum(db1, &S.t4[0][0], E, EB, 1.f);
-    if (s > s_lo) nxt = fetch(s - 1);
-    for_f2([&](int r, int c) {  // dq += dO;  dk -= dT;  dv = dT  (gl1 holds d target)
-      const float2 a = *reinterpret_cast<const float2*>(&dq[r][c]), o = ldb2(&S.dO[r][c]);
-      const float2 b = *reinterpret_cast<const float2*>(&S.dk[r][c]), dT = *reinterpret_cast<const float2*>(&S.gl1[r][c]);
-      const size_t at = (r0 + (size_t)r * HD + c) >> 1;
-      static_cast<uint32_t*>(p.d_q)[at] = pack_bf16(a.x + o.x, a.y + o.y);
-      static_cast<uint32_t*>(p.d_k)[at] = pack_bf16(b.x - dT.x, b.y - dT.y);
-      static_cast<uint32_t*>(p.d_v)[at] = pack_bf16(dT.x, dT.y);
-    });
-    __syncthreads();
-    TRM(15)
-  }
-  __syncthreads();
-  // the masters go back to the workspace: for the stream's next item, or (last item) for the output loop below
-  if (rank < 2 * p.NCH - 1) {
-    master_out(W1, tW1a);
-    master_out(W2, tW2a);
-  }
-  if (!pass1) {
-    master_out(dW1, tdW1a);
-    master_out(dW2, tdW2a);
-  }
-  if (rank < 2 * p.NCH - 1) {
-    // hand the stream to its next item
-    for (int e = tid; e < E; e += MB_THREADS) {
-      ho[HO_B1 + e] = b1[e];
-      ho[HO_DB1 + e] = db1[e];
-    }
-    if (tid < F) {
-      ho[HO_B2 + tid] = b2[tid];
-      ho[HO_DB2 + tid] = db2[tid];
-      ho[HO_DG + tid] = S.dgam[tid];
-      ho[HO_DB + tid] = S.dbet[tid];
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) *reinterpret_cast<volatile int*>(p.sched + 1 + stream) = rel + 1;
-  } else {
-    // ---- gradients w.r.t. the initial state, per-stream LayerNorm parameter gradients
-    __syncthreads();  // dW1, dW2 are in the workspace for every thread
-    for (int e = tid; e < F * E; e += MB_THREADS) {
-      st_from_float<T>(p.d_w1, (size_t)stream * F * E + e, __ldcg(dW1 + MatG<F, E, false>::at(e / E, e % E)));
-      st_from_float<T>(p.d_w2, (size_t)stream * F * E + e, __ldcg(dW2 + MatG<E, F, false>::at(e / F, e % F)));
-    }
-    for (int e = tid; e < E; e += MB_THREADS) st_from_float<T>(p.d_b1, (size_t)stream * E + e, db1[e]);
-    if (tid < F) {
-      st_from_float<T>(p.d_b2, (size_t)stream * F + tid, db2[tid]);
-      p.part_ln[(size_t)stream * 2 * HD + tid] = S.dgam[tid];
-      p.part_ln[(size_t)stream * 2 * HD + HD + tid] = S.dbet[tid];
-    }
-  }
   }  // item loop
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (failed && threadIdx.x == 0)  // copies and products in flight land before the block leaves
+    for (int i = 0; i < 4096; ++i)
+      if (mbar_try_wait(barL, nload & 1) && mbar_try_wait(barG, nload & 1) && mbar_try_wait(barM, nmma & 1)) break;
+  tmem_fence_before_sync();
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_tmem) : "memory");
-#ifdef TTT_MLP_TRACE
-  if (tid == 0 && blockIdx.x == 0 && p.trace != nullptr)
-    for (int i = 0; i < 16; ++i) p.trace[i] = (unsigned int)(tr_acc[i] / NS);
-#endif
-#undef TRM
+  if (threadIdx.x < 32) tmem_dealloc(tmem, 512);
 }
 
 // grad_token_eta[t] = sum over streams, grad_ln_weight / grad_ln_bias [h][f] = sum over the batch; fixed order.  Block =
@@ -1201,24 +963,19 @@ __global__ void __launch_bounds__(256) ttt_mlp_bwd_reduce_kernel(const float* pa
   }
 }
 
-// floats of workspace per stream: the four float32 state matrices, the hand-off record, the bf16 g1p / g2p tiles of
-// every stage, the float32 biases at the start of every stage, the bf16 operand copies of dW1 and dW2
+// floats of workspace per stream: the four float32 masters, the hand-off record, one record per stage
 size_t mlp_bwd_ws_stride_floats(int T) {
-  const size_t ns = (size_t)T / CS;
-  return 4 * (size_t)HD * MB_E + MLP_BWD_HANDOFF_FLOATS + ns * CS * (MB_E + HD) / 2 + ns * (MB_E + HD) + (size_t)HD * MB_E;
+  return 4 * (size_t)HD * MB_E + MLP_BWD_HANDOFF_FLOATS + (size_t)T / CS * (MLP_REC_BYTES / 4);
 }
 
-cudaError_t launch_mlp_bwd(const MlpBwdParams& p0, int B, cudaStream_t st) {
+cudaError_t launch_mlp_bwd(const CUtensorMap* m, const MlpBwdParams& p0, int B, cudaStream_t st) {
   MlpBwdParams p = p0;
   p.nstreams = B * p.H;
-  p.CH = MLP_BWD_CHUNK;
-  p.NCH = (p.NS + p.CH - 1) / p.CH;
-  const size_t smem = sizeof(MlpBwdSmem);
   static DeviceValue resident;
   int sms = 0, per_sm = 0;
   cudaError_t e = resident.get(0, &per_sm, [&](int* n) {
-    const cudaError_t a = cudaFuncSetAttribute(ttt_mlp_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, ttt_mlp_bwd_kernel, MB_THREADS, smem);
+    const cudaError_t a = cudaFuncSetAttribute(ttt_mlp_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MlpBwdSmem::TOTAL);
+    return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, ttt_mlp_bwd_kernel, MB_THREADS, MlpBwdSmem::TOTAL);
   });
   if (e != cudaSuccess || (e = device_sms(&sms)) != cudaSuccess) return e;
   // persistent grid: blocks wait on one another's hand-offs, so all of them must be resident (cooperative launch);
@@ -1226,9 +983,11 @@ cudaError_t launch_mlp_bwd(const MlpBwdParams& p0, int B, cudaStream_t st) {
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   int grid = sms * per_sm;
   if (grid > p.nstreams) grid = p.nstreams;
+  p.CH = mlp_chunk_stages(p.NS, p.nstreams, grid);
+  p.NCH = (p.NS + p.CH - 1) / p.CH;
   if ((e = cudaMemsetAsync(p.sched, 0, sizeof(int) * (size_t)(1 + p.nstreams), st)) != cudaSuccess) return e;
-  void* args[] = {(void*)&p};
-  e = cudaLaunchCooperativeKernel((const void*)ttt_mlp_bwd_kernel, dim3(grid), dim3(MB_THREADS), args, smem, st);
+  void* args[] = {(void*)&m[0], (void*)&m[1], (void*)&m[2], (void*)&m[3], (void*)&p};
+  e = cudaLaunchCooperativeKernel((const void*)ttt_mlp_bwd_kernel, dim3(grid), dim3(MB_THREADS), args, MlpBwdSmem::TOTAL, st);
   if (e != cudaSuccess) return e;
   const int n = p.T + 2 * p.H * HD;
   ttt_mlp_bwd_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(p.part_te, p.part_ln, B, p.H, p.T, p.reduced_bf16,

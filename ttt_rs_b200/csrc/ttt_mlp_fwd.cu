@@ -17,7 +17,7 @@
 //
 // Scheduling.  One CTA fills an SM (255 registers x 256 threads), so a launch of one CTA per stream runs in whole
 // waves: 192 streams on 148 SMs cost two stream-times.  When the caller passes the backward's workspace (training),
-// the kernel is launched persistently instead: blocks take work items (stream, chunk of MLP_FWD_CHUNK stages), first
+// the kernel is launched persistently instead: blocks take work items (stream, chunk of stages: mlp_chunk_stages), first
 // chunks of all streams first; a chunk leaves the float32 state and biases in the stream's workspace block (where
 // the final state is due anyway) and the next chunk of that stream -- on whichever block takes it -- picks them up.
 // An item waits only for an item of smaller index, which a resident block already holds (cooperative launch), and
@@ -31,7 +31,6 @@ namespace ttt {
 constexpr int MLP_THREADS = 256;
 constexpr int MLP_E = 256;
 constexpr int MLP_NST = 2;
-constexpr int MLP_FWD_CHUNK = 16;  // stages per work item of the persistent launch
 
 struct MlpSmem {
   static constexpr uint32_t TILE = TILE_BF16_BYTES;                   // [16][64] bf16
@@ -100,6 +99,9 @@ __device__ __forceinline__ void ldsm_x2_t(uint32_t (&r)[2], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
 
+// SAVE: persistent, with the backward's workspace (the tests of a record pointer in the stage loop cost inference 1.5 %: 48
+// streams of 31 stages 161.8 against 159.4 us).
+template <bool SAVE>
 __global__ void __launch_bounds__(MLP_THREADS, 1)
     ttt_mlp_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   const int tid = L.tid, lane = L.lane, g = L.g, t = L.t, warp = L.warp;
   const int eb = 32 * warp, fb = 8 * warp;
   const int NS = p.NS;
-  const bool persistent = (p.sched != nullptr);
+  constexpr bool persistent = SAVE;
   const int CH = persistent ? p.CH : NS, NCH = persistent ? p.NCH : 1;
   const int nitems = persistent ? p.nstreams * NCH : (int)gridDim.x;
   __shared__ int s_item;
@@ -150,9 +152,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   // every stage (the bf16 operands of the state updates) and the final state go there, so that the backward can
   // start its reverse walk at once.  Set per work item.
   float* bws = nullptr;
-  uint32_t* sv_g1p = nullptr;
-  uint32_t* sv_g2p = nullptr;
-  float* sv_bst = nullptr;
+  uint8_t* rec0 = nullptr;
 
   // stage s of the current stream into ring slot n % MLP_NST (n counts the stages this block has visited)
   auto issue_loads = [&](int n, int s) {
@@ -213,10 +213,10 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     head = stream % p.H;
     row_base = stream * p.T;
     const int s_lo = chunk * CH, s_hi = min(s_lo + CH, NS) - 1;
-    bws = p.bwd_ws != nullptr ? p.bwd_ws + (size_t)stream * p.bwd_ws_stride : nullptr;
-    sv_g1p = bws != nullptr ? reinterpret_cast<uint32_t*>(bws + 4 * HD * MLP_E + MLP_BWD_HANDOFF_FLOATS) : nullptr;
-    sv_g2p = bws != nullptr ? sv_g1p + (size_t)NS * CS * MLP_E / 2 : nullptr;
-    sv_bst = bws != nullptr ? reinterpret_cast<float*>(sv_g2p + (size_t)NS * CS * HD / 2) : nullptr;
+    if constexpr (SAVE) {
+      bws = p.bwd_ws + (size_t)stream * p.bwd_ws_stride;
+      rec0 = reinterpret_cast<uint8_t*>(bws + 4 * HD * MLP_E + MLP_BWD_HANDOFF_FLOATS);
+    }
     gam = f2(ld_as_float<T>(p.ln_g, (size_t)head * HD + fc), ld_as_float<T>(p.ln_g, (size_t)head * HD + fc + 1));
     bet = f2(ld_as_float<T>(p.ln_b, (size_t)head * HD + fc), ld_as_float<T>(p.ln_b, (size_t)head * HD + fc + 1));
     if (chunk == 0) {
@@ -287,11 +287,10 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     const int slot = n % MLP_NST;
     const uint32_t tq = base + slot * SM::SLOT, tk = tq + TL, tv = tk + TL;
     int fail = mbar_wait_bounded(bar0 + 8 * slot, (n / MLP_NST) & 1) ? 0 : 1;
-    if (sv_bst != nullptr && g == 0) {  // biases at the start of the stage, for the backward
-      float* const bs = sv_bst + (size_t)s * (MLP_E + HD);
+    uint8_t* const rec = rec0 + (size_t)s * MLP_REC_BYTES;  // the backward's record of the stage
+    if (SAVE && g == 0) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(bs + eb + 8 * j + 2 * t) = b1v[j];
-      *reinterpret_cast<float2*>(bs + MLP_E + fc) = b2v;
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(rec + MLP_REC_B1 + 4 * (eb + 8 * j + 2 * t)) = b1v[j];
     }
     const float lr_row[2] = {ld_as_float<T>(gbase + SM::OFF_LR + slot * 32, g),
                              ld_as_float<T>(gbase + SM::OFF_LR + slot * 32, g + 8)};
@@ -359,6 +358,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
                      "r"(pack_bf16(x2[j][r].x, x2[j][r].y))
                      : "memory");
       }
+    if (SAVE) fence_proxy_async_smem();  // (X2 also leaves by a bulk copy)
     fail = __syncthreads_or(fail);  // B1: X2 tile and the refreshed W2 copy are visible; previous stage fully left
     if (fail) {
       failed = true;
@@ -383,6 +383,11 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
       mma_bf16(z2, a0[0].p[0], a0[1].p[0], a0[2].p[0], a0[3].p[0], bb[0], bb[1]);
       mma_bf16(z2, a1[0].p[0], a1[1].p[0], a1[2].p[0], a1[3].p[0], bb[2], bb[3]);
     }
+    if (SAVE) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        *reinterpret_cast<float2*>(rec + MLP_REC_Z2 + 4 * ((g + 8 * r) * HD + fc)) = pr(z2, r);
+    }
     // ---- S4. LN + L2 gradient of Z2 against V - K; G2p = lr o G2 to its operand tile
     F2 g2p[2];
     {
@@ -406,15 +411,23 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
            a0, a1, f0);
       xsel ^= 1;
       const float A[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)}, Bv[2] = {a0.y * (1.f / HD), a1.y * (1.f / HD)};
+      if (SAVE && warp == 0 && t < 2)
+        *reinterpret_cast<float4*>(rec + MLP_REC_STAT + 32 * (g + 8 * t)) =
+            t == 0 ? make_float4(mean[0], rstd[0], A[0], Bv[0]) : make_float4(mean[1], rstd[1], A[1], Bv[1]);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         g2p[r] = f2mul(f2fma(x[r], f2(-Bv[r]), f2sub(gg[r], f2(A[r]))), f2(rstd[r] * lr_row[r]));
         const uint32_t pk2 = pack_bf16(g2p[r].x, g2p[r].y);
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(tG2 + off_bf16(g + 8 * r, fc)), "r"(pk2) : "memory");
-        if (sv_g2p != nullptr) sv_g2p[((size_t)s * CS + g + 8 * r) * (HD / 2) + (fc >> 1)] = pk2;
       }
     }
+    if (SAVE) fence_proxy_async_smem();
     __syncthreads();  // B2: G2p tile visible
+    if (SAVE && tid == 0) {
+      bulk_store_1d(rec + MLP_REC_X2, tX2, 4 * TL);
+      bulk_store_1d(rec + MLP_REC_G2P, tG2, TL);
+      bulk_commit();
+    }
     // ---- S5. G1p = (G2p W2^T) o gelu'(Z1)  (columns eb..eb+31; W2 straight from registers)
     tmem_ld_8x4(tm_w2, w2[0]);
     tmem_ld_8x4(tm_w2 + 32u, w2[1]);
@@ -449,7 +462,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const Pk<1> pk1 = split_pack<1>(g1p[j][r].x, g1p[j][r].y);
-        if (sv_g1p != nullptr) sv_g1p[((size_t)s * CS + g + 8 * r) * (MLP_E / 2) + ((eb + 8 * j + 2 * t) >> 1)] = pk1.p[0];
+        if (SAVE) *reinterpret_cast<uint32_t*>(rec + MLP_REC_G1P + off_e(g + 8 * r, eb + 8 * j + 2 * t)) = pk1.p[0];
         gt1[j][r] = movm_t_np<1>(pk1);
       }
     {
@@ -520,6 +533,11 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
       ldsm_x2_t(bg, tG2 + off_bf16((lane & 7) + (((lane >> 3) & 1) << 3), fb));
       mma_bf16(zb2, am2[0].p[0], am2[1].p[0], am2[2].p[0], am2[3].p[0], bg[0], bg[1]);
     }
+    if (SAVE) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        *reinterpret_cast<float2*>(rec + MLP_REC_ZB2 + 4 * ((g + 8 * r) * HD + fc)) = pr(zb2, r);
+    }
     // ---- S10. out = Q + LN(Zb2)
     {
       const F2 zp[2] = {pr(zb2, 0), pr(zb2, 1)};
@@ -531,6 +549,9 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
       const float mean[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)};
       const float rstd[2] = {rsqrtf(fmaxf(a0.y * (1.f / HD) - mean[0] * mean[0], 0.f) + p.eps),
                              rsqrtf(fmaxf(a1.y * (1.f / HD) - mean[1] * mean[1], 0.f) + p.eps)};
+      if (SAVE && warp == 1 && t < 2)
+        *reinterpret_cast<float2*>(rec + MLP_REC_STAT + 32 * (g + 8 * t) + 16) =
+            t == 0 ? make_float2(mean[0], rstd[0]) : make_float2(mean[1], rstd[1]);
       const uint32_t so = base + SM::OFF_OUT + (n & 1) * TL;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -539,8 +560,9 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         st_pair<T>(so, g + 8 * r, fc, o.x, o.y);
       }
       fence_proxy_async_smem();
+      if (SAVE && tid == 0) bulk_wait_read<0>();  // the copies of X2 and G2p have left: their tiles may be rewritten
       __syncthreads();  // E
-      if (tid == 0) {
+      if (tid == 0 && !(SAVE && p.walk_only)) {
         tma_store_2d(&tm_o, 0, row_base + s * CS, so);
         bulk_commit();
         bulk_wait_read<1>();
@@ -610,19 +632,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     __syncthreads();
     if (tid == 0) *reinterpret_cast<volatile int*>(p.sched + 1 + stream) = chunk + 1;
   } else {
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int kt = 0; kt < 8; ++kt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int e = eb + 16 * mt + g + 8 * (i >> 1), c = 8 * kt + 2 * t + (i & 1);
-          st_from_float<T>(p.w1_out, (size_t)stream * HD * MLP_E + (size_t)c * MLP_E + e, w1t[mt][kt][i] * wscale);
-          st_from_float<T>(p.w2_out, (size_t)stream * HD * MLP_E + (size_t)e * HD + c, w2[mt][kt][i] * wscale);
-        }
-    if (bws != nullptr) {
-      float* const M1 = bws;
-      float* const M2 = bws + HD * MLP_E;
+    if (!(SAVE && p.walk_only)) {
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
@@ -630,18 +640,23 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int e = eb + 16 * mt + g + 8 * (i >> 1), c = 8 * kt + 2 * t + (i & 1);
-            M1[mlp_state_at(c, e, MLP_E)] = w1t[mt][kt][i] * wscale;
-            M2[mlp_state_at(e, c, HD)] = w2[mt][kt][i] * wscale;
+            st_from_float<T>(p.w1_out, (size_t)stream * HD * MLP_E + (size_t)c * MLP_E + e, w1t[mt][kt][i] * wscale);
+            st_from_float<T>(p.w2_out, (size_t)stream * HD * MLP_E + (size_t)e * HD + c, w2[mt][kt][i] * wscale);
           }
-      if (g == 0) {
-        float* const ho = bws + 4 * HD * MLP_E;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          *reinterpret_cast<float2*>(ho + MLP_HO_B1 + eb + 8 * j + 2 * t) = b1v[j];
-        *reinterpret_cast<float2*>(ho + MLP_HO_B2 + fc) = b2v;
-      }
     }
-    if (g == 0) {
+    if (SAVE) {  // masters as the backward takes them up
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int kt = 0; kt < 8; ++kt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int at = mlp_master_at(eb + 16 * mt + g + 8 * r, 8 * kt + 2 * t);
+            *reinterpret_cast<float2*>(bws + at) = pr(w1t[mt][kt], r);
+            *reinterpret_cast<float2*>(bws + HD * MLP_E + at) = pr(w2[mt][kt], r);
+          }
+    }
+    if (g == 0 && !(SAVE && p.walk_only)) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const size_t o = (size_t)stream * MLP_E + eb + 8 * j + 2 * t;
@@ -661,15 +676,16 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 }
 
 cudaError_t launch_mlp_fwd(const CUtensorMap* m, const MlpFwdParams& p, int nstreams, cudaStream_t st) {
-  auto kfn = ttt_mlp_fwd_kernel;
-  static DeviceValue resident;
+  const bool save = p.bwd_ws != nullptr;
+  auto kfn = save ? ttt_mlp_fwd_kernel<true> : ttt_mlp_fwd_kernel<false>;
+  static DeviceValue resident[2];
   int sms = 0, per_sm = 0;
-  cudaError_t e = resident.get(0, &per_sm, [&](int* n) {
+  cudaError_t e = resident[save].get(0, &per_sm, [&](int* n) {
     const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MlpSmem::DYN_BYTES);
     return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, MLP_THREADS, MlpSmem::DYN_BYTES);
   });
   if (e != cudaSuccess) return e;
-  if (p.sched == nullptr) {  // no workspace to park state in: one block per stream
+  if (!save) {  // no workspace to park state in: one block per stream
     kfn<<<nstreams, MLP_THREADS, MlpSmem::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], p);
     return cudaGetLastError();
   }
@@ -678,10 +694,10 @@ cudaError_t launch_mlp_fwd(const CUtensorMap* m, const MlpFwdParams& p, int nstr
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   MlpFwdParams pp = p;
   pp.nstreams = nstreams;
-  pp.CH = MLP_FWD_CHUNK;
-  pp.NCH = (p.NS + MLP_FWD_CHUNK - 1) / MLP_FWD_CHUNK;
   int grid = sms * per_sm;
-  if (grid > nstreams * pp.NCH) grid = nstreams * pp.NCH;
+  if (grid > nstreams) grid = nstreams;
+  pp.CH = mlp_chunk_stages(p.NS, nstreams, grid);
+  pp.NCH = (p.NS + pp.CH - 1) / pp.CH;
   if ((e = cudaMemsetAsync(pp.sched, 0, sizeof(int) * (size_t)(1 + nstreams), st)) != cudaSuccess) return e;
   void* args[] = {(void*)&m[0], (void*)&m[1], (void*)&m[2], (void*)&m[3], (void*)&pp};
   return cudaLaunchCooperativeKernel((const void*)kfn, dim3(grid), dim3(MLP_THREADS), args, MlpSmem::DYN_BYTES, st);
