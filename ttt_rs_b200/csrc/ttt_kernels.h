@@ -346,7 +346,7 @@ inline int mlp_chunk_stages(int NS, int nstreams, int blocks) {
   if (nstreams <= blocks) return NS;
   int best = NS;
   long long least = -1;
-  for (int ch = 8; ch <= 64; ch += 4) {
+  for (int ch = 8; ch <= 64; ++ch) {
     const long long nch = (NS + ch - 1) / ch, rounds = (nch * nstreams + blocks - 1) / blocks;
     const long long cost = rounds * (2 * (ch < NS ? ch : NS) + 3);
     if (least < 0 || cost < least) {

@@ -24,7 +24,7 @@
 //  * A warp also owns one token row of the 16 x 64 tiles for the two LayerNorms.
 // A stage is six barrier intervals (I1..I6 below).  Before, 25 phases passed every intermediate tile through shared
 // memory as bf16, undid the updates through registers and read dW from L2: 43 k cycles a stage; 192 streams of 128 stages
-// forward and backward 4.11 ms, now 2.68 ms.
+// forward and backward 4.12 ms, now 2.55 ms.
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
 #include "ttt_stage.cuh"
@@ -32,6 +32,7 @@
 namespace ttt {
 
 constexpr int MB_THREADS = 512;
+constexpr uint32_t ONES = 0x3f803f80u;  // a pair of bf16 ones
 constexpr int MB_E = 256;  // hidden width of the inner MLP (4 * head_dim)
 constexpr float GELU_C0 = 0.7978845608028654f, GELU_C1 = 0.044715f;
 typedef __nv_bfloat16 bf;
@@ -55,14 +56,14 @@ struct MlpBwdSmem {
   static constexpr uint32_t DB2 = DA1 + 16 * 24 * 2;  // float [64]
   static constexpr uint32_t LR = DB2 + HD * 4;      // float [2][16], then ell = te15 lr [2][16]
   static constexpr uint32_t TE = LR + 4 * CS * 4;   // float [16]
-  static constexpr uint32_t DLG = TE + CS * 4;      // float [8][16]
-  static constexpr uint32_t DLP = DLG + 8 * CS * 4; // float [16] sum over i of dEta te, then [16] the rest of dell
+  static constexpr uint32_t M1T = TE + CS * 4;      // bf16 [16][24]: -M1
+  static constexpr uint32_t DLP = M1T + 16 * 24 * 2;  // float [16] sum over i of dEta te, then [16] the rest of dell
   static constexpr uint32_t LN = DLP + 2 * CS * 4;  // float [2][64]: LayerNorm weight, bias
-  static constexpr uint32_t BAR = LN + 2 * HD * 4; // mbarriers: stage inputs, G1p, products; then item, tensor-memory base
-  static constexpr uint32_t TOTAL = BAR + 3 * 8 + 8;
+  static constexpr uint32_t BAR = LN + 2 * HD * 4; // mbarriers: stage inputs, late inputs, dW products, undone updates; then item, tensor-memory base
+  static constexpr uint32_t TOTAL = BAR + 4 * 8 + 8;
 };
 static_assert(MlpBwdSmem::TOTAL <= 227 * 1024, "shared-memory tiles exceed one SM");
-static_assert(MlpBwdSmem::DA1 % 16 == 0 && MlpBwdSmem::BAR % 8 == 0, "alignment");
+static_assert(MlpBwdSmem::DA1 % 16 == 0 && MlpBwdSmem::M1T % 16 == 0 && MlpBwdSmem::BAR % 8 == 0, "alignment");
 
 // ---- tcgen05 ---------------------------------------------------------------------------------------------------
 // operand descriptor of token tiles read MN-major: 64 contiguous elements (128 bytes, swizzled) x 8 tokens per atom, the
@@ -88,6 +89,9 @@ __device__ __forceinline__ void ldsm_x2_trans(uint32_t (&r)[2], uint32_t addr) {
 }
 __device__ __forceinline__ void mma4(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   mma_bf16(c, a[0], a[1], a[2], a[3], b0, b1);
+}
+__device__ __forceinline__ void stsm_x4(uint32_t addr, const uint32_t (&r)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts_f(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
@@ -141,6 +145,12 @@ __device__ __forceinline__ float warp_sum(float v) {
 // fragment (4 rows x 4 column pairs per half-warp) fall in distinct banks
 __device__ __forceinline__ uint32_t off_x(int row, int col) { return (uint32_t)(row * 256 + ((col ^ ((row & 3) << 3)) << 2)); }
 
+// float [16][16] partial sum of a causal matrix, stored by columns: even columns before odd ones, rows turned by 8 in every
+// other pair of them, so that neither the fragments' stores nor a column's load meet in a bank
+__device__ __forceinline__ uint32_t off_causal(int j, int i) {
+  return (uint32_t)((((j >> 1) + 8 * (j & 1)) * 16 + (i ^ (((j >> 2) & 1) << 3))) << 2);
+}
+
 // gelu(z), gelu'(z) and (D2) gelu''(z) of a pair from one tanh.  tanh(x) = 1 - 2 / (1 + e^{2x}) with the fast exponential and
 // division (relative error ~1e-6, as in the forward kernel)
 template <bool D2>
@@ -175,12 +185,13 @@ struct Place {
   __device__ __forceinline__ uint32_t bn_off() const {
     return (16 * warp + (lane & 7) + ((lane >> 4) << 3)) * 128 + ((((lane >> 3) & 1) ^ (lane & 7)) << 4);
   }
-  // pair (row g, this warp's hidden column 2 t) of a 16 x 256 tile; n-tile: ^ 16, row g + 8: + 1024
+  // ldmatrix / stmatrix address (x4) of this warp's 16 columns of a 16 x 256 tile: blocks (n-tile, row half) in the order of
+  // the accumulator registers; read transposed they are the B fragments of a contraction over the tokens
   __device__ __forceinline__ uint32_t e_off() const {
-    return (warp >> 2) * TILE_BF16_BYTES + g * 128 + (((2 * (warp & 3)) ^ g) << 4) + 4 * t;
+    return (warp >> 2) * TILE_BF16_BYTES + (lane & 15) * 128 + (((2 * (warp & 3) + (lane >> 4)) ^ (lane & 7)) << 4);
   }
-  // this warp's share of the masters: matrix warp / 4 (W1, W2, dW1, dW2), lane quarter warp % 4 = hidden features
-  // 32 (warp % 4) + lane and, 64 columns on, those + 128
+  // this warp's share of the masters between work items: matrix warp / 4 (W1, W2, dW1, dW2), lane quarter warp % 4 =
+  // hidden features 32 (warp % 4) + lane and, 64 columns on, those + 128
   __device__ __forceinline__ int mi() const { return warp >> 2; }
   __device__ __forceinline__ uint32_t tm(uint32_t tmem) const { return tmem + ((32u * (uint32_t)(warp & 3)) << 16) + 128u * (uint32_t)mi(); }
   __device__ __forceinline__ int rc() const { return 2 * lane; }  // row-wise steps: row = warp, columns rc, rc + 1
@@ -199,20 +210,21 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
   extern __shared__ __align__(1024) uint8_t mlp_bwd_smem[];
   const uint32_t base0 = smem_u32(mlp_bwd_smem);
   const int NS = p.NS;
-  const uint32_t barL = base0 + SM::BAR, barG = barL + 8, barM = barL + 16;
-  int* const s_item = reinterpret_cast<int*>(mlp_bwd_smem + SM::BAR + 24);
-  const uint32_t* const s_tmem = reinterpret_cast<const uint32_t*>(mlp_bwd_smem + SM::BAR + 28);
+  const uint32_t barL = base0 + SM::BAR, barG = barL + 8, barD = barL + 16, barU = barL + 24;
+  int* const s_item = reinterpret_cast<int*>(mlp_bwd_smem + SM::BAR + 32);
+  const uint32_t* const s_tmem = reinterpret_cast<const uint32_t*>(mlp_bwd_smem + SM::BAR + 36);
   if ((base0 & 1023u) != 0) {  // (the tiles need it; dynamic shared memory starts there when there is no static one)
     if (threadIdx.x == 0) report_timeout(p.status, 2, 0);
     return;
   }
   // Tensor memory, all 512 columns (shared memory keeps the block alone on its SM).  The warp that allocates frees it at
   // the end of the kernel; every way out of the item loop leads there.
-  if (threadIdx.x < 32) tmem_alloc(base0 + SM::BAR + 28, 512);
+  if (threadIdx.x < 32) tmem_alloc(base0 + SM::BAR + 36, 512);
   if (threadIdx.x == 32) {
     mbar_init(barL, 1);
     mbar_init(barG, 1);
-    mbar_init(barM, 1);
+    mbar_init(barD, 1);
+    mbar_init(barU, 1);
     fence_mbar_init();
     prefetch_tmap(&tm_q);
     prefetch_tmap(&tm_k);
@@ -362,66 +374,115 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
     }
     tmem_fence_before_sync();
     __syncthreads();
+    // bf16 copy of half a master (128 hidden features; this warp's 32) to its operand matrix
+    auto convert = [&](const Place& P, int mat, int half) {
+      const float sc = mat < 2 ? wscale : 1.f;
+      const uint32_t src = tmem + ((32u * (uint32_t)(P.warp & 3)) << 16) + 128 * mat + 64 * half;
+      const uint32_t dst = base0 + SM::W1 + mat * SM::WM + (128 * half + 32 * (P.warp & 3) + P.lane) * 128;
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        float v[8][4];
+        tmem_ld_8x4(src + 32 * cc, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const F2 x = f2mul(pr(v[2 * i + (j >> 1)], j & 1), f2(sc));
+            w[j] = pack_bf16(x.x, x.y);
+          }
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + (((4 * cc + i) ^ (P.lane & 7)) << 4)), "r"(w[0]),
+                       "r"(w[1]), "r"(w[2]), "r"(w[3])
+                       : "memory");
+        }
+      }
+    };
+    // What a stage needs before its first barrier and does not take from the stage after it; `b`: its input buffer.
+    //  * both LayerNorms, a row per warp: G2 and dZb2 as bf16 pairs
+    uint32_t g2_pair, dzb_pair;
+    auto rows_of = [&](int b) {
+      if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+      TTT_PLACE
+      const uint32_t in = base0 + SM::IN + b * 3 * TL;
+      const F2 gam = lds_f2(base0 + SM::LN + 4 * rc), bet = lds_f2(base0 + SM::LN + 4 * (HD + rc));
+      const F2 vv = ld_pair<T>(base0 + SM::V, warp, rc), kk = ld_pair<T>(in + TL, warp, rc), dd = ld_pair<T>(in + 2 * TL, warp, rc);
+      const F2 xh = f2mul(f2add(zz, f2(-st1.x)), f2(st1.y));
+      const F2 xb = f2mul(f2add(zzb, f2(-st2.x)), f2(st2.y)), tt = f2mul(dd, gam);
+      const F2 gy = f2sub(f2fma(gam, xh, bet), f2sub(vv, kk));
+      const F2 sums = warp_sum2(f2hsum(tt), f2hsum(f2mul(tt, xb)));
+      const F2 G = f2mul(f2fma(xh, f2(-st1.w), f2fma(gy, gam, f2(-st1.z))), f2(st1.y));
+      const F2 dzb = f2mul(f2fma(xb, f2(sums.y * (-1.f / HD)), f2add(tt, f2(sums.x * (-1.f / HD)))), f2(st2.y));
+      dgam = f2fma(dd, xb, dgam);
+      dbet = f2add(dbet, dd);
+      g2_pair = pack_bf16(G.x, G.y);
+      dzb_pair = pack_bf16(dzb.x, dzb.y);
+    };
+    //  * (one warp) the learning rates, A1 = Q K^T and -M1 = -eta o (1 + A1)
+    auto causal_first = [&](int s, int b) {
+      TTT_PLACE
+      float lr = 0.f;
+      if (lane < CS) lr = ld_as_float<T>(p.lr, row_base + (size_t)s * CS + lane);
+      if (!mbar_wait_bounded(barL, nload & 1)) failed = 1;
+      const uint32_t q = base0 + SM::IN + b * 3 * TL + P.a_off();
+      float at[2][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t ak[4], aq[4];
+        ldsm_x4(ak, (q + TL) ^ (ks << 5));
+        ldsm_x4(aq, q ^ (ks << 5));
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) mma4(at[nt], aq, ak[nt], ak[nt + 2]);  // (the blocks of an A fragment are those of a B fragment)
+      }
+      if (lane < CS) put_rates(b, lr);
+      __syncwarp();
+#pragma unroll
+      for (int jt = 0; jt < 2; ++jt)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int i = g + 8 * r, j = 8 * jt + 2 * t;
+          const F2 e = f2mul(lds_f2(base0 + SM::LR + 4 * (b * CS + j)), f2(-lds_f(base0 + SM::TE + 4 * i))), m = f2fma(pr(at[jt], r), e, e);
+          sts32(base0 + SM::M1T + 2 * (24 * i + j), pack_bf16(j <= i ? m.x : 0.f, j + 1 <= i ? m.y : 0.f));
+          if (j <= i) sts_f(base0 + SM::AD + 4 * (17 * i + j), at[jt][2 * r]);
+          if (j + 1 <= i) sts_f(base0 + SM::AD + 4 * (17 * i + j + 1), at[jt][2 * r + 1]);
+        }
+    };
+    //  * (warps 8..15) the bf16 copies of dW2 and W2, whose last readers are further back than those of dW1 and W1
+    auto second_layer_copies = [&]() {
+      TTT_PLACE
+      if (!mbar_wait_bounded(warp < 12 ? barD : barU, nmma & 1)) failed = 1;
+      tmem_fence_after_sync();
+      convert(P, warp < 12 ? 3 : 1, 0);
+      convert(P, warp < 12 ? 3 : 1, 1);
+    };
     if (threadIdx.x >> 5 == 15 && elect_one()) {
       tmem_fence_after_sync();
+      umma_commit_to(barD);
       if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
       undo_updates(buf);
-      umma_commit_to(barM);
+      umma_commit_to(barU);
     }
+    __syncwarp();
+    if (threadIdx.x >> 5 == 8) causal_first(s, buf);
+    if (threadIdx.x >= 256) second_layer_copies();
+    rows_of(buf);
 
     while (true) {
       // (addresses formed anew in every stage: kept across the loop they would push the tiles' values into local memory)
       uint32_t base = base0;
       asm volatile("" : "+r"(base));
       const uint32_t sAD = base + SM::AD, sDET = base + SM::DET, sDB2 = base + SM::DB2, sTE = base + SM::TE, sLN = base + SM::LN;
-      // ---- I1. The stage's operands: bf16 copies of the four masters; both LayerNorms, a row per warp
       const uint32_t tq = base + SM::IN + buf * 3 * TL, tk = tq + TL, tdo = tk + TL, tx2 = base + SM::X2 + buf * ET;
       const uint32_t sLR = base + SM::LR + buf * CS * 4, sELL = sLR + 2 * CS * 4;
-      if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+      // ---- I1. G2 and dZb2 (their tiles have been read by the products of the stage before), bf16 copies of W1 and dW1
       ++nload;
+      if (!mbar_wait_bounded(barD, nmma & 1) || !mbar_wait_bounded(barU, nmma & 1)) failed = 1;
+      ++nmma;
+      tmem_fence_after_sync();
       {
         TTT_PLACE
-        const uint32_t r_off = off_bf16(warp, rc);
-        const F2 gam = lds_f2(sLN + 4 * rc), bet = lds_f2(sLN + 4 * (HD + rc));
-        const F2 vv = ld_pair<T>(base + SM::V, warp, rc), kk = ld_pair<T>(tk, warp, rc), dd = ld_pair<T>(tdo, warp, rc);
-        const F2 xh = f2mul(f2add(zz, f2(-st1.x)), f2(st1.y));
-        const F2 xb = f2mul(f2add(zzb, f2(-st2.x)), f2(st2.y)), tt = f2mul(dd, gam);
-        const F2 gy = f2sub(f2fma(gam, xh, bet), f2sub(vv, kk));
-        const F2 sums = warp_sum2(f2hsum(tt), f2hsum(f2mul(tt, xb)));
-        const F2 G = f2mul(f2fma(xh, f2(-st1.w), f2fma(gy, gam, f2(-st1.z))), f2(st1.y));
-        const F2 dzb = f2mul(f2fma(xb, f2(sums.y * (-1.f / HD)), f2add(tt, f2(sums.x * (-1.f / HD)))), f2(st2.y));
-        dgam = f2fma(dd, xb, dgam);
-        dbet = f2add(dbet, dd);
-        // (the products of the stage before may still be reading the two tiles)
-        if (!mbar_wait_bounded(barM, nmma & 1)) failed = 1;
-        ++nmma;
-        tmem_fence_after_sync();
-        sts32(base + SM::G2 + r_off, pack_bf16(G.x, G.y));
-        sts32(base + SM::DZ2B + r_off, pack_bf16(dzb.x, dzb.y));
-      }
-      {
-        TTT_PLACE
-        const float sc = P.mi() < 2 ? wscale : 1.f;
-        const uint32_t dst = base + SM::W1 + P.mi() * SM::WM + (32 * (warp & 3) + lane) * 128;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            float v[8][4];
-            tmem_ld_8x4(P.tm(tmem) + 64 * h + 32 * cc, v);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t w[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const F2 x = f2mul(f2(v[2 * i + (j >> 1)][2 * (j & 1)], v[2 * i + (j >> 1)][2 * (j & 1) + 1]), f2(sc));
-                w[j] = pack_bf16(x.x, x.y);
-              }
-              asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + h * 128 * 128 + (((4 * cc + i) ^ (lane & 7)) << 4)),
-                           "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
-                           : "memory");
-            }
-          }
+        sts32(base + SM::G2 + off_bf16(warp, rc), g2_pair);
+        sts32(base + SM::DZ2B + off_bf16(warp, rc), dzb_pair);
+        convert(P, (warp >> 3) * 2, (warp >> 2) & 1);
       }
       tmem_fence_before_sync();
       failed = __syncthreads_or(failed);  // 1
@@ -436,57 +497,43 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       float dx[2][4];            // dX2 so far: dA2^T X2b - l o gl2
       {
         TTT_PLACE
-        const uint32_t a_off = P.a_off(), bn_off = P.bn_off(), e_st = P.e_off();
-        const float te_row[2] = {lds_f(sTE + 4 * g), lds_f(sTE + 4 * (g + 8))};
-        const float ell[2] = {lds_f(sELL + 4 * g), lds_f(sELL + 4 * (g + 8))};
-        const F2 lrc[2] = {lds_f2(sLR + 8 * t), lds_f2(sLR + 32 + 8 * t)};
-        float z1[2][4] = {}, zq[2][4] = {}, at[2][4] = {};
+        const uint32_t a_off = P.a_off(), bn_off = P.bn_off(), e_off = P.e_off();
+        float z1[2][4] = {}, zq[2][4] = {}, u1[2][4] = {};
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-          uint32_t ak[4], aq[4], bw[4];
+          uint32_t ak[4], aq[4], bw[4], bd[4];
           ldsm_x4(ak, (tk + a_off) ^ (ks << 5));
-          ldsm_x4(aq, (tq + a_off) ^ (ks << 5));
           ldsm_x4(bw, (base + SM::W1 + bn_off) ^ (ks << 5));
+          ldsm_x4(aq, (tq + a_off) ^ (ks << 5));
+          ldsm_x4(bd, (base + SM::DW1 + bn_off) ^ (ks << 5));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(z1[nt], ak, bw[2 * nt], bw[2 * nt + 1]);
 #pragma unroll
           for (int nt = 0; nt < 2; ++nt) {
-            mma4(z1[nt], ak, bw[2 * nt], bw[2 * nt + 1]);
             mma4(zq[nt], aq, bw[2 * nt], bw[2 * nt + 1]);
-            mma4(at[nt], aq, ak[nt], ak[nt + 2]);           // Q K^T (the blocks of an A fragment are those of a B fragment)
+            mma4(u1[nt], ak, bd[2 * nt], bd[2 * nt + 1]);  // K dW1
           }
         }
-        uint32_t x2[2][2], gd2[2][2];  // bf16 pairs
+        uint32_t gd2[2][2];  // gelu''(Z1), bf16 pairs
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             F2 d2;
-            const F2 x = gelu_pair<true>(f2add(pr(z1[nt], r), b1v[nt]), gd1[nt][r], d2);
-            x2[nt][r] = pack_bf16(x.x, x.y);
+            gelu_pair<true>(f2add(pr(z1[nt], r), b1v[nt]), gd1[nt][r], d2);
             gd2[nt][r] = pack_bf16(d2.x, d2.y);
             zq[nt][2 * r] += b1v[nt].x;
             zq[nt][2 * r + 1] += b1v[nt].y;
-          }
-        // -M1 = -eta o (1 + A1), as an A operand
-        uint32_t am1[4];
-#pragma unroll
-        for (int jt = 0; jt < 2; ++jt)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const int i = g + 8 * r, j = 8 * jt + 2 * t;
-            const F2 e = f2mul(lrc[jt], f2(-te_row[r])), m = f2fma(pr(at[jt], r), e, e);
-            am1[2 * jt + r] = pack_bf16(j <= i ? m.x : 0.f, j + 1 <= i ? m.y : 0.f);
-            if (warp == 0) {
-              if (j <= i) sts_f(sAD + 4 * (17 * i + j), at[jt][2 * r]);
-              if (j + 1 <= i) sts_f(sAD + 4 * (17 * i + j + 1), at[jt][2 * r + 1]);
-            }
+            u1[nt][2 * r] += db1v[nt].x;  // K dW1 + db1
+            u1[nt][2 * r + 1] += db1v[nt].y;
           }
         float h[2][4] = {}, dzw[2][4] = {}, gl2[2][4] = {}, dm[2][4] = {};
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
           uint32_t ag[4], az[4], bw[4], bd[4];
           ldsm_x4(ag, (base + SM::G2 + a_off) ^ (ks << 5));
-          ldsm_x4(az, (base + SM::DZ2B + a_off) ^ (ks << 5));
           ldsm_x4(bw, (base + SM::W2 + bn_off) ^ (ks << 5));
+          ldsm_x4(az, (base + SM::DZ2B + a_off) ^ (ks << 5));
           ldsm_x4(bd, (base + SM::DW2 + bn_off) ^ (ks << 5));
 #pragma unroll
           for (int nt = 0; nt < 2; ++nt) {
@@ -496,89 +543,96 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
             mma4(dm[nt], az, ag[nt], ag[nt + 2]);            // dZb2 G2^T = -dM2
           }
         }
-        uint32_t ad2[4];  // dA2 = dM2 o eta, as an A operand
+        // G1 = H o gelu'(Z1);  Zb1 = Q W1 + b1 - M1 G1;  the row sums of dell that are ready here: G1.(K dW1 + db1) + gl2.X2
+        uint32_t own[4], tb[4];  // a tile's own columns: as pairs, and as a B operand (contraction over the tokens)
+        {
+          uint32_t x2[4];
+          ldsm_x4(x2, tx2 + e_off);
+          float del[2] = {0.f, 0.f};
 #pragma unroll
-        for (int jt = 0; jt < 2; ++jt)
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const F2 g1 = f2mul(pr(h[nt], r), gd1[nt][r]);
+              own[2 * nt + r] = pack_bf16(g1.x, g1.y);
+              del[r] += f2hsum(f2fma(g1, pr(u1[nt], r), f2mul(pr(gl2[nt], r), unpack_bf16(x2[2 * nt + r]))));
+            }
+          stsm_x4(base + SM::G1 + e_off, own);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            del[r] = quad_sum(del[r]);
+            if (t == 0) sts_f(sDET + 4 * (16 * warp + g + 8 * r), del[r]);
+          }
+        }
+        __syncwarp();
+        {
+          uint32_t am1[4];
+          ldsm_x4_t(tb, base + SM::G1 + e_off);
+          ldsm_x4(am1, base + SM::M1T + (lane & 15) * 48 + (lane >> 4) * 16);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(zq[nt], am1, tb[2 * nt], tb[2 * nt + 1]);
+        }
+        // dA2 = dM2 o eta, as an A operand;  dZb2 W2^T + dA2 X2;  dX2 = dA2^T X2b - l o gl2 + ..
+        uint32_t ad2[4];
+#pragma unroll
+        for (int jt = 0; jt < 2; ++jt) {
+          const F2 lrc = lds_f2(sLR + 4 * (8 * jt + 2 * t));
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const int i = g + 8 * r, j = 8 * jt + 2 * t;
-            const F2 m = f2mul(pr(dm[jt], r), f2mul(lrc[jt], f2(-te_row[r])));
+            const F2 m = f2mul(pr(dm[jt], r), f2mul(lrc, f2(-lds_f(sTE + 4 * i))));
             ad2[2 * jt + r] = pack_bf16(j <= i ? m.x : 0.f, j + 1 <= i ? m.y : 0.f);
             if (warp == 1) {
               if (j <= i) sts_f(sAD + 4 * (17 * j + i + 1), -dm[jt][2 * r]);
               if (j + 1 <= i) sts_f(sAD + 4 * (17 * (j + 1) + i + 1), -dm[jt][2 * r + 1]);
             }
           }
-        uint32_t tb[2][2];  // a tile's own columns as a B operand (contraction over the tokens)
-        float del[2] = {0.f, 0.f};
-        // G1 = H o gelu'(Z1);  Zb1 = Q W1 + b1 - M1 G1
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const F2 g1 = f2mul(pr(h[nt], r), gd1[nt][r]);
-            const uint32_t v = pack_bf16(g1.x, g1.y);
-            sts32(base + SM::G1 + (e_st ^ (nt << 4)) + r * 1024, v);
-            tb[nt][r] = movm_t(v);
-            const F2 q = f2fma(g1, db1v[nt], f2mul(pr(gl2[nt], r), unpack_bf16(x2[nt][r])));
-            del[r] += f2hsum(q);
-          }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) mma4(zq[nt], am1, tb[nt][0], tb[nt][1]);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          del[r] = quad_sum(del[r]);
-          if (t == 0) sts_f(sDET + 4 * (16 * warp + g + 8 * r), del[r]);
         }
-        // dZb2 W2^T + dA2 X2
+        ldsm_x4_t(tb, tx2 + e_off);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) mma4(dzw[nt], ad2, tb[2 * nt], tb[2 * nt + 1]);
+        const float ell[2] = {lds_f(sELL + 4 * g), lds_f(sELL + 4 * (g + 8))};
+        // X2b = gelu(Zb1);  dZ1b = (dZb2 W2^T + dA2 X2) o gelu'(Zb1)
+        uint32_t own2[4];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
-          mma4(dzw[nt], ad2, movm_t(x2[nt][0]), movm_t(x2[nt][1]));
-        // X2b = gelu(Zb1);  dZ1b = (dZb2 W2^T + dA2 X2) o gelu'(Zb1);  dX2 = dA2^T X2b - l o gl2 + ..
-        const uint32_t ad2t[4] = {movm_t(ad2[0]), movm_t(ad2[2]), movm_t(ad2[1]), movm_t(ad2[3])};
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          uint32_t xb[2];
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             F2 d1, unused;
             const F2 x = gelu_pair<false>(pr(zq[nt], r), d1, unused), d = f2mul(pr(dzw[nt], r), d1);
-            const uint32_t v = pack_bf16(x.x, x.y), w = pack_bf16(d.x, d.y);
-            sts32(base + SM::X2B + (e_st ^ (nt << 4)) + r * 1024, v);
-            sts32(base + SM::DZ1B + (e_st ^ (nt << 4)) + r * 1024, w);
-            xb[r] = movm_t(v);
-            tb[nt][r] = movm_t(w);
+            own[2 * nt + r] = pack_bf16(x.x, x.y);
+            own2[2 * nt + r] = pack_bf16(d.x, d.y);
             dx[nt][2 * r] = -ell[r] * gl2[nt][2 * r];
             dx[nt][2 * r + 1] = -ell[r] * gl2[nt][2 * r + 1];
           }
-          mma4(dx[nt], ad2t, xb[0], xb[1]);
+        stsm_x4(base + SM::X2B + e_off, own);
+        stsm_x4(base + SM::DZ1B + e_off, own2);
+        __syncwarp();
+        {
+          const uint32_t ad2t[4] = {movm_t(ad2[0]), movm_t(ad2[2]), movm_t(ad2[1]), movm_t(ad2[3])};
+          ldsm_x4_t(tb, base + SM::X2B + e_off);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(dx[nt], ad2t, tb[2 * nt], tb[2 * nt + 1]);
         }
         // dG1 = -M1^T dZ1b - l o (K dW1 + db1);  dH = dG1 o gelu'(Z1)
-        const uint32_t am1t[4] = {movm_t(am1[0]), movm_t(am1[2]), movm_t(am1[1]), movm_t(am1[3])};
-        float u1[2][4] = {};  // K dW1
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          uint32_t ak[4], bd[4];
-          ldsm_x4(ak, (tk + a_off) ^ (ks << 5));
-          ldsm_x4(bd, (base + SM::DW1 + bn_off) ^ (ks << 5));
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) mma4(u1[nt], ak, bd[2 * nt], bd[2 * nt + 1]);
-        }
-        constexpr uint32_t ONES = 0x3f803f80u;
+        uint32_t am1t[4];
+        ldsm_x4_t(am1t, base + SM::M1T + ((lane & 7) + ((lane >> 4) << 3)) * 48 + ((lane >> 3) & 1) * 16);
+        ldsm_x4_t(tb, base + SM::DZ1B + e_off);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           float d[4] = {}, cs[4] = {};
-          mma4(d, am1t, tb[nt][0], tb[nt][1]);
-          mma_bf16(cs, ONES, ONES, ONES, ONES, tb[nt][0], tb[nt][1]);  // column sums
+          mma4(d, am1t, tb[2 * nt], tb[2 * nt + 1]);
+          mma_bf16(cs, ONES, ONES, ONES, ONES, tb[2 * nt], tb[2 * nt + 1]);  // column sums
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            const F2 dg = f2fma(f2add(pr(u1[nt], r), db1v[nt]), f2(-ell[r]), pr(d, r));
+            const F2 dg = f2fma(pr(u1[nt], r), f2(-ell[r]), pr(d, r));
             const F2 dh = f2mul(dg, gd1[nt][r]);
             dz1a[nt][r] = f2mul(f2mul(dg, pr(h[nt], r)), unpack_bf16(gd2[nt][r]));
-            sts32(base + SM::DH + (e_st ^ (nt << 4)) + r * 1024, pack_bf16(dh.x, dh.y));
+            own[2 * nt + r] = pack_bf16(dh.x, dh.y);
           }
           db1v[nt] = f2add(db1v[nt], f2(cs[0], cs[1]));
         }
+        stsm_x4(base + SM::DH + e_off, own);
       }
       __syncthreads();  // 2
 
@@ -629,9 +683,9 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 #pragma unroll
           for (int jt = 0; jt < 2; ++jt)
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {  // transposed, [j][i], rows of 16: the reader takes a column of the matrix
-              sts_f(dst + 4 * (16 * (8 * jt + 2 * t) + g + 8 * r), c[jt][2 * r]);
-              sts_f(dst + 4 * (16 * (8 * jt + 2 * t + 1) + g + 8 * r), c[jt][2 * r + 1]);
+            for (int r = 0; r < 2; ++r) {  // transposed: the reader takes a column of the matrix
+              sts_f(dst + off_causal(8 * jt + 2 * t, g + 8 * r), c[jt][2 * r]);
+              sts_f(dst + off_causal(8 * jt + 2 * t + 1, g + 8 * r), c[jt][2 * r + 1]);
             }
         }
         dell_row = lane < 16 ? lds_f(sDET + 4 * (16 * lane + warp)) : 0.f;  // row sums of the 16 warps (finished in I4)
@@ -653,14 +707,14 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 #pragma unroll
         for (int kq = 0; kq < 4; ++kq) dg2 = f2add(dg2, lds_f2(base + SM::PART + kq * 4096 + x_off));
         // lane i < 16: column j of the causal matrices
-        const uint32_t sM2 = base + SM::EXG + 3 * 1024 + 64 * warp;  // (each lane has read the partial sum there)
+        const uint32_t sM2 = base + SM::EXG + 3 * 1024 + 64 * ((warp >> 1) + 8 * (warp & 1));  // (the row's own partial sums, read by then)
         float m2 = 0.f, dlr = 0.f;
         if (lane < 16) {
           float a2 = 0.f, d1 = 0.f;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            a2 += lds_f(base + SM::EXD + q * 1024 + 4 * (16 * warp + lane));
-            d1 -= lds_f(base + SM::EXG + q * 1024 + 4 * (16 * warp + lane));
+            a2 += lds_f(base + SM::EXD + q * 1024 + off_causal(warp, lane));
+            d1 -= lds_f(base + SM::EXG + q * 1024 + off_causal(warp, lane));
           }
           const float te_i = lds_f(sTE + 4 * lane);
           float deta = 0.f, da1 = 0.f;
@@ -670,6 +724,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
             da1 = d1 * te_i * lr_j;
           }
           dlr = deta * te_i;
+          __syncwarp(0xffffu);
           sts_f(sM2 + 4 * lane, m2);
           sts_f(sDET + 4 * (17 * lane + warp), deta * lr_j);
           *reinterpret_cast<bf*>(mlp_bwd_smem + SM::DA1 + 2 * (24 * lane + warp)) = __float2bfloat16_rn(da1);
@@ -699,12 +754,15 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
         fence_proxy_async_smem();  // (G1p lands where the partial sums were)
       }
       __syncthreads();  // 4
-      if (s > s_lo && threadIdx.x == 0) issue_late(s - 1);
+      if (s > s_lo) {
+        if (threadIdx.x == 0) issue_late(s - 1);
+        load_own(s - 1);
+      }
 
       // ---- I5. dX2 += dZ2 W2^T;  dZ1 = dG1 o H o gelu''(Z1) + dX2 o gelu'(Z1)
       {
         TTT_PLACE
-        const uint32_t a_off = P.a_off(), bn_off = P.bn_off(), e_st = P.e_off();
+        const uint32_t a_off = P.a_off(), bn_off = P.bn_off(), e_off = P.e_off();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
           uint32_t az[4], bw[4];
@@ -713,117 +771,138 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 #pragma unroll
           for (int nt = 0; nt < 2; ++nt) mma4(dx[nt], az, bw[2 * nt], bw[2 * nt + 1]);
         }
-        constexpr uint32_t ONES = 0x3f803f80u;
+        uint32_t own[4], tb[4];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          uint32_t tb[2];
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const F2 d = f2fma(pr(dx[nt], r), gd1[nt][r], dz1a[nt][r]);
-            const uint32_t v = pack_bf16(d.x, d.y);
-            sts32(base + SM::DZ1 + (e_st ^ (nt << 4)) + r * 1024, v);
-            tb[r] = movm_t(v);
+            own[2 * nt + r] = pack_bf16(d.x, d.y);
           }
+        stsm_x4(base + SM::DZ1 + e_off, own);
+        fence_proxy_async_smem();  // every operand tile of the products below has been written by now
+        __syncwarp();
+        ldsm_x4_t(tb, base + SM::DZ1 + e_off);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
           float cs[4] = {};
-          mma_bf16(cs, ONES, ONES, ONES, ONES, tb[0], tb[1]);
+          mma_bf16(cs, ONES, ONES, ONES, ONES, tb[2 * nt], tb[2 * nt + 1]);
           db1v[nt] = f2add(db1v[nt], f2(cs[0], cs[1]));
         }
-        fence_proxy_async_smem();  // every operand tile of the products below has been written by now
       }
       __syncthreads();  // 5
 
-      // ---- I6. dW1 += Q^T dZ1b + K^T dZ1, dW2 += X2^T dZ2 + X2b^T dZb2 + dH^T G2, and W1, W2 one stage back: tcgen05, in
-      //      the background of dq = dZ1b W1^T + dA1 K, dk = dZ1 W1^T + dA1^T Q (warps 0..7, eight features each) and
-      //      gl1 = G1 dW1^T (warps 8..15)
-      if (threadIdx.x >> 5 == 15 && elect_one()) {
-        tmem_fence_after_sync();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t d1 = tmem + 256 + 64 * h, d2 = d1 + 128, o = h * 2 * TL;
-          umma_update(d1, base + SM::DZ1B + o, tq, UPD_IDESC);
-          umma_update(d1, base + SM::DZ1 + o, tk, UPD_IDESC);
-          umma_update(d2, tx2 + o, base + SM::DZ2, UPD_IDESC);
-          umma_update(d2, base + SM::X2B + o, base + SM::DZ2B, UPD_IDESC);
-          umma_update(d2, base + SM::DH + o, base + SM::G2, UPD_IDESC);
-        }
-      }
-      __syncwarp();
-      if (s > s_lo) load_own(s - 1);
+      // ---- I6. dW1 += Q^T dZ1b + K^T dZ1, dW2 += X2^T dZ2 + X2b^T dZb2 + dH^T G2, and W1, W2 one stage back: tcgen05.
+      //      Meanwhile warps 0..3: dq = dZ1b W1^T + dA1 K, dk = dZ1 W1^T + dA1^T Q (16 features each); warps 4..7: gl1 = G1 dW1^T,
+      //      db2; warps 8..15: the eta gradients, the next stage's rates, causal matrix and copies of W2, dW2; all: its LayerNorms
       const size_t r0 = (size_t)(row_base + s * CS) * HD;
-      {
+      if (threadIdx.x >> 5 == 15) {
+        if (elect_one()) {
+          tmem_fence_after_sync();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t d1 = tmem + 256 + 64 * h, d2 = d1 + 128, o = h * 2 * TL;
+            umma_update(d1, base + SM::DZ1B + o, tq, UPD_IDESC);
+            umma_update(d1, base + SM::DZ1 + o, tk, UPD_IDESC);
+            umma_update(d2, tx2 + o, base + SM::DZ2, UPD_IDESC);
+            umma_update(d2, base + SM::X2B + o, base + SM::DZ2B, UPD_IDESC);
+            umma_update(d2, base + SM::DH + o, base + SM::G2, UPD_IDESC);
+          }
+          umma_commit_to(barD);
+          if (s > s_lo) {
+            if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+            undo_updates(buf ^ 1);
+          }
+          umma_commit_to(barU);
+        }
+        __syncwarp();
+      }
+      if (threadIdx.x < 128) {
         TTT_PLACE
         const uint32_t a_off = P.a_off();
-        const int nt = warp & 7, col = 8 * nt + 2 * t;
-        const uint32_t b_off = lane * 128 + ((nt ^ (lane & 7)) << 4);
-        const uint32_t f_off = (lane & 15) * 128 + ((nt ^ (lane & 7)) << 4);  // the tile's 16 tokens as k, columns 8 nt.. as n
-        if (warp < 8) {
-          float aq[2][4] = {}, ak[2][4] = {};
+        const uint32_t b_off = (lane & 15) * 128 + (((2 * warp + (lane >> 4)) ^ (lane & 7)) << 4);  // 16 rows as k, columns 16 warp.. as n
+        float aq[2][4] = {}, ak[2][4] = {};
 #pragma unroll
-          for (int kp = 0; kp < 8; ++kp) {
-            uint32_t a0[4], a1[4], c0[4], c1[4], b[4];
-            const uint32_t o = (kp >> 1) * TL + a_off, x = (kp & 1) << 6;
-            ldsm_x4_t(b, base + SM::W1 + b_off + kp * 4096);
-            ldsm_x4(a0, (base + SM::DZ1B + o) ^ x);
-            ldsm_x4(a1, (base + SM::DZ1B + o) ^ (x + 32));
-            ldsm_x4(c0, (base + SM::DZ1 + o) ^ x);
-            ldsm_x4(c1, (base + SM::DZ1 + o) ^ (x + 32));
-            mma4(aq[0], a0, b[0], b[1]);
-            mma4(ak[0], c0, b[0], b[1]);
-            mma4(aq[1], a1, b[2], b[3]);
-            mma4(ak[1], c1, b[2], b[3]);
+        for (int kk = 0; kk < 16; ++kk) {
+          uint32_t a[4], c[4], b[4];
+          const uint32_t o = (kk >> 2) * TL + a_off, x = (kk & 3) << 5;
+          ldsm_x4_t(b, base + SM::W1 + b_off + kk * 2048);
+          ldsm_x4(a, (base + SM::DZ1B + o) ^ x);
+          ldsm_x4(c, (base + SM::DZ1 + o) ^ x);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            mma4(aq[nt], a, b[2 * nt], b[2 * nt + 1]);
+            mma4(ak[nt], c, b[2 * nt], b[2 * nt + 1]);
           }
-          uint32_t da[4], dat[4], bk[2], bq[2], bz[2], by[2];
-          ldsm_x4(da, base + SM::DA1 + (lane & 15) * 48 + (lane >> 4) * 16);                                // dA1
-          ldsm_x4_t(dat, base + SM::DA1 + ((lane & 7) + ((lane >> 4) << 3)) * 48 + ((lane >> 3) & 1) * 16);  // dA1^T
-          ldsm_x2_trans(bk, tk + f_off);
-          ldsm_x2_trans(bq, tq + f_off);
-          ldsm_x2_trans(bz, base + SM::DZ2B + f_off);
-          ldsm_x2_trans(by, base + SM::DZ2 + f_off);
-          mma4(aq[0], da, bk[0], bk[1]);
-          mma4(ak[0], dat, bq[0], bq[1]);
-          constexpr uint32_t ONES = 0x3f803f80u;
+        }
+        uint32_t da[4], dat[4], bk[4], bq[4];
+        ldsm_x4(da, base + SM::DA1 + (lane & 15) * 48 + (lane >> 4) * 16);                                // dA1
+        ldsm_x4_t(dat, base + SM::DA1 + ((lane & 7) + ((lane >> 4) << 3)) * 48 + ((lane >> 3) & 1) * 16);  // dA1^T
+        ldsm_x4_t(bk, tk + b_off);
+        ldsm_x4_t(bq, tq + b_off);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const int col = 16 * warp + 8 * nt + 2 * t;
+          mma4(aq[nt], da, bk[2 * nt], bk[2 * nt + 1]);
+          mma4(ak[nt], dat, bq[2 * nt], bq[2 * nt + 1]);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 o = f2add(pr(aq[nt], r), ld_pair<T>(tdo, g + 8 * r, col));
+            static_cast<uint32_t*>(p.d_q)[(r0 + (g + 8 * r) * HD + col) >> 1] = pack_bf16(o.x, o.y);
+            sts_f2(base + SM::EXD + off_x(g + 8 * r, col), pr(ak[nt], r));
+          }
+        }
+      } else if (threadIdx.x < 256) {
+        TTT_PLACE
+        const int np = warp & 3;
+        const uint32_t a_off = P.a_off();
+        const uint32_t b_off = (lane & 15) * 128 + (((2 * np + (lane >> 4)) ^ (lane & 7)) << 4);
+        float c[2][2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < 16; ++kk) {
+          uint32_t a[4], b[4];
+          ldsm_x4_t(b, base + SM::DW1 + b_off + kk * 2048);
+          ldsm_x4(a, (base + SM::G1 + (kk >> 2) * TL + a_off) ^ ((kk & 3) << 5));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(c[nt][kk & 1], a, b[2 * nt], b[2 * nt + 1]);
+        }
+        uint32_t bz[4], by[4];
+        ldsm_x4_t(bz, base + SM::DZ2B + b_off);
+        ldsm_x4_t(by, base + SM::DZ2 + b_off);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const int col = 16 * np + 8 * nt + 2 * t;
           float cs[4] = {}, ct[4] = {};
-          mma_bf16(cs, ONES, ONES, ONES, ONES, bz[0], bz[1]);
-          mma_bf16(ct, ONES, ONES, ONES, ONES, by[0], by[1]);
+          mma_bf16(cs, ONES, ONES, ONES, ONES, bz[2 * nt], bz[2 * nt + 1]);
+          mma_bf16(ct, ONES, ONES, ONES, ONES, by[2 * nt], by[2 * nt + 1]);
           if (g == 0) sts_f2(sDB2 + 4 * col, f2add(lds_f2(sDB2 + 4 * col), f2(cs[0] + ct[0], cs[1] + ct[1])));
 #pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const F2 o = f2add(f2add(pr(aq[0], r), pr(aq[1], r)), ld_pair<T>(tdo, g + 8 * r, col));
-            static_cast<uint32_t*>(p.d_q)[(r0 + (g + 8 * r) * HD + col) >> 1] = pack_bf16(o.x, o.y);
-            sts_f2(base + SM::EXD + off_x(g + 8 * r, col), f2add(pr(ak[0], r), pr(ak[1], r)));
-          }
-        } else {
-          float c[2][4] = {};
+          for (int r = 0; r < 2; ++r)
+            sts_f2(base + SM::EXG + off_x(g + 8 * r, col), f2mul(f2add(pr(c[nt][0], r), pr(c[nt][1], r)), f2(-lds_f(sELL + 4 * (g + 8 * r)))));
+        }
+      } else {
+        if (threadIdx.x >> 5 == 13) {
+          // dell[j] = -(gl1[j].K[j] + G1[j].db1 + gl2[j].X2[j] + G2[j].db2)
+          const int lane = threadIdx.x & 31;
+          float dell = 0.f, dte = 0.f, lr = 0.f;
+          if (lane < CS) {
+            dell = -lds_f(base + SM::DLP + 4 * (CS + lane));
+            lr = lds_f(sLR + 4 * lane);
 #pragma unroll
-          for (int kp = 0; kp < 8; ++kp) {
-            uint32_t a0[4], a1[4], b[4];
-            const uint32_t o = (kp >> 1) * TL + a_off, x = (kp & 1) << 6;
-            ldsm_x4_t(b, base + SM::DW1 + b_off + kp * 4096);
-            ldsm_x4(a0, (base + SM::G1 + o) ^ x);
-            ldsm_x4(a1, (base + SM::G1 + o) ^ (x + 32));
-            mma4(c[0], a0, b[0], b[1]);
-            mma4(c[1], a1, b[2], b[3]);
+            for (int j = 0; j < CS; ++j) dte += lds_f(sDET + 4 * (17 * lane + j));
+            st_from_float<T>(p.d_lr, row_base + (size_t)s * CS + lane, lds_f(base + SM::DLP + 4 * lane) + dell * te_last);
           }
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const F2 gl = f2add(pr(c[0], r), pr(c[1], r)), kk = ld_pair<T>(tk, g + 8 * r, col);
-            const float l = lds_f(sELL + 4 * (g + 8 * r)), d = quad_sum(f2hsum(f2mul(gl, kk)));
-            if (t == 0) sts_f(base + SM::DLG + 4 * (CS * nt + g + 8 * r), d);
-            sts_f2(base + SM::EXG + off_x(g + 8 * r, col), f2mul(gl, f2(-l)));
-          }
-          if (warp == 14 && s > s_lo && lane < CS) put_rates(buf ^ 1, ld_as_float<T>(p.lr, row_base + (size_t)(s - 1) * CS + lane));
-          if (warp == 15 && elect_one()) {
-            if (s > s_lo) {
-              if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
-              undo_updates(buf ^ 1);
-            }
-            umma_commit_to(barM);
-          }
-          __syncwarp();
+          const float sum = warp_sum(dell * lr);
+          if (lane < CS) p.part_te[(size_t)row_base + (size_t)s * CS + lane] = lane == CS - 1 ? dte + sum : dte;
+        }
+        if (s > s_lo) {
+          if (threadIdx.x >> 5 == 8) causal_first(s - 1, buf ^ 1);
+          second_layer_copies();
         }
       }
+      if (s > s_lo) rows_of(buf ^ 1);
       __syncthreads();  // 6
-      // ---- outputs of the stage: dk = (products) - l o gl1 - dT, dv = dT; the eta factors
+      // ---- outputs of the stage: dk = (products) - l o gl1 - dT, dv = dT
       {
         TTT_PLACE
         const uint32_t x_off = off_x(warp, rc);
@@ -832,29 +911,12 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
         static_cast<uint32_t*>(p.d_k)[at] = pack_bf16(dk.x, dk.y);
         static_cast<uint32_t*>(p.d_v)[at] = pack_bf16(dT.x, dT.y);
       }
-      if (threadIdx.x >> 5 == 13) {
-        const int lane = threadIdx.x & 31;
-        // dell[j] = -(gl1[j].K[j] + G1[j].db1 + gl2[j].X2[j] + G2[j].db2)
-        float dell = 0.f, dte = 0.f, lr = 0.f;
-        if (lane < CS) {
-          dell = lds_f(base + SM::DLP + 4 * (CS + lane));
-#pragma unroll
-          for (int w = 0; w < 8; ++w) dell += lds_f(base + SM::DLG + 4 * (CS * w + lane));
-          dell = -dell;
-          lr = lds_f(sLR + 4 * lane);
-#pragma unroll
-          for (int j = 0; j < CS; ++j) dte += lds_f(sDET + 4 * (17 * lane + j));
-          st_from_float<T>(p.d_lr, row_base + (size_t)s * CS + lane, lds_f(base + SM::DLP + 4 * lane) + dell * te_last);
-        }
-        const float sum = warp_sum(dell * lr);
-        if (lane < CS) p.part_te[(size_t)row_base + (size_t)s * CS + lane] = lane == CS - 1 ? dte + sum : dte;
-      }
       if (s == s_lo) break;
       --s;
       buf ^= 1;
     }
     if (!failed) {
-      if (!mbar_wait_bounded(barM, nmma & 1)) failed = 1;
+      if (!mbar_wait_bounded(barD, nmma & 1) || !mbar_wait_bounded(barU, nmma & 1)) failed = 1;
       ++nmma;
       tmem_fence_after_sync();
     }
@@ -928,7 +990,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
   }  // item loop
   if (failed && threadIdx.x == 0)  // copies and products in flight land before the block leaves
     for (int i = 0; i < 4096; ++i)
-      if (mbar_try_wait(barL, nload & 1) && mbar_try_wait(barG, nload & 1) && mbar_try_wait(barM, nmma & 1)) break;
+      if (mbar_try_wait(barL, nload & 1) && mbar_try_wait(barG, nload & 1) && mbar_try_wait(barU, nmma & 1)) break;
   tmem_fence_before_sync();
   __syncthreads();
   if (threadIdx.x < 32) tmem_dealloc(tmem, 512);
