@@ -182,12 +182,13 @@ __device__ __forceinline__ Pk<1> split_pack<1>(float x, float y) {
 template <>
 __device__ __forceinline__ Pk<3> split_pack<3>(float x, float y) {
   Pk<3> r;
-  r.p[0] = pack_bf16(x, y);
-  float rx = x - bf16_lo(r.p[0]), ry = y - bf16_hi(r.p[0]);
-  r.p[1] = pack_bf16(rx, ry);
-  rx -= bf16_lo(r.p[1]);
-  ry -= bf16_hi(r.p[1]);
-  r.p[2] = pack_bf16(rx, ry);
+  float2 v = make_float2(x, y);
+  const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    r.p[i] = pack_bf16(v.x, v.y);
+    if (i < 2) v = __ffma2_rn(make_float2(bf16_lo(r.p[i]), bf16_hi(r.p[i])), minus, v);  // the remainder, exact
+  }
   return r;
 }
 
@@ -236,6 +237,16 @@ template <int NP>
 __device__ __forceinline__ void mma_np2(float (&c0)[4], const Pk<NP> (&a0)[4], const Pk<NP> (&b0)[2], float (&c1)[4],
                                         const Pk<NP> (&a1)[4], const Pk<NP> (&b1)[2]) {
   mma_np_n<NP, 2>({&c0, &c1}, {&a0, &a1}, {&b0, &b1});
+}
+
+// two k-steps of two products (the joins of one accumulator follow one another, so the sums are those of two calls of mma_np2):
+// a product of the float32 planes waits for the one before it, and a lone warp on its scheduler has only its own others to
+// fill that
+template <int NP>
+__device__ __forceinline__ void mma_np2x2(float (&c0)[4], float (&c1)[4], const Pk<NP> (&a0)[4], const Pk<NP> (&b00)[2],
+                                          const Pk<NP> (&b01)[2], const Pk<NP> (&a1)[4], const Pk<NP> (&b10)[2],
+                                          const Pk<NP> (&b11)[2]) {
+  mma_np_n<NP, 4>({&c0, &c1, &c0, &c1}, {&a0, &a0, &a1, &a1}, {&b00, &b01, &b10, &b11});
 }
 
 template <int NP>

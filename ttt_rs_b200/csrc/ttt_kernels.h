@@ -388,6 +388,9 @@ cudaError_t launch_mlp_fwd(const CUtensorMap* maps, const MlpFwdParams& p, int n
 // maps: q, k, v, out, gp (saved lr-scaled LN gradient, [B*H*T, 64] of T)
 cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* maps, const LinFwdParams& p, int nstreams,
                               cudaStream_t st);
+// the form for streams that have an SM each (ttt_linear_fwd_roles.cu), chosen by launch_linear_fwd
+cudaError_t launch_linear_fwd_roles(int dtype, int seg, int mb, const CUtensorMap* maps, const LinFwdParams& p, int nstreams,
+                                    cudaStream_t st);
 // maps: q, k, v, d_out, d_q, d_k, d_v, gp
 cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, LinBwdParams& p, int nstreams,
                               cudaStream_t st);

@@ -455,7 +455,9 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
       F2 z1p[2][2];
       slab_pairs(z1, z1p);
       float sa[2], sb[2];
-      ln_l2_pieces<T, SEG>(z1p, mean1, rstd1, gam, bet, tk, tv, L, xh, gy, gx, sa, sb);
+      F2 btg[2][2];
+      beta_minus_target<T, SEG>(bet, tk, tv, L, btg);
+      ln_l2_pieces(z1p, mean1, rstd1, gam, btg, xh, gy, gx, sa, sb);
       g_from_pieces(gx, xh, A, Bv1, rstd1, G);
     }
     // ---- 5. Zbar = Zq - M' Gp   (am holds -M')

@@ -1,4 +1,5 @@
-// Fused TTT-Linear forward scan for sm_100a: one 4-warp CTA per (batch, head) stream walks all mini-batches.
+// Fused TTT-Linear forward scan for sm_100a: one 4-warp CTA per (batch, head) stream walks all mini-batches.  This is the form
+// for more streams than SMs; ttt_linear_fwd_roles.cu has the one for streams that have an SM each.
 //
 // What it computes is the reference's multi-stage forward kernel
 // (rust/fused/src/linear_fused_tile/forward/kernel.rs:92-176, stage body forward/stage.rs:29-208, semantics
@@ -296,7 +297,9 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? 3 : 1))
     {
       F2 xh[2][2], gy[2][2], gx[2][2];
       float sa[2], sb[2];
-      ln_l2_pieces<T, SEG>(z1p, mean, rstd, gam, bet, tk, tv, L, xh, gy, gx, sa, sb);
+      F2 btg[2][2];
+      beta_minus_target<T, SEG>(bet, tk, tv, L, btg);
+      ln_l2_pieces(z1p, mean, rstd, gam, btg, xh, gy, gx, sa, sb);
       float2 a0, a1;
       int f2_ = 0;
       xch_rows2<SEG, false>(&xch[xsel], L, sa[0], sb[0], sa[1], sb[1], a0, a1, f2_);
@@ -481,6 +484,14 @@ static cudaError_t launch_fwd_mb(int mb, const CUtensorMap* m, const LinFwdParam
 // mb: tokens per mini-batch, 16 or 8 (the maps' boxes then have 8 rows)
 cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* maps,
                               const LinFwdParams& p, int nstreams, cudaStream_t st) {
+  int sms = 0;
+  const cudaError_t e = device_sms(&sms);
+  if (e != cudaSuccess) return e;
+  // Streams that have an SM each: a stage's work on three groups of warps, where a lone group of four leaves the SM waiting for
+  // its chain (64 stages, us, this form / three groups: bf16 148 streams 72.4 / 62.3, f32 188 / 163).  From there on streams
+  // share SMs and fill one another's waits, and the three groups' registers let in one block only (192 streams: 86 / 120,
+  // f32 248 / 314).  A few stages cost the same either way.
+  if (nstreams <= sms) return launch_linear_fwd_roles(dtype, seg, mb, maps, p, nstreams, st);
   if (seg == 32) {
     if (dtype == 1) return launch_fwd_mb<__nv_bfloat16, 32>(mb, maps, p, nstreams, st);
     return launch_fwd_mb<float, 32>(mb, maps, p, nstreams, st);

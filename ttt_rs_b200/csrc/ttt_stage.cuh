@@ -22,6 +22,26 @@ struct Lane {
   }
 };
 
+// The barrier of an exchange: the whole CTA (BAR = 0), or the four warps of a group on named barrier BAR.
+template <int BAR>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (BAR == 0) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NTHREADS) : "memory");
+}
+template <int BAR>
+__device__ __forceinline__ int group_sync_or(int v) {
+  if constexpr (BAR == 0) {
+    return __syncthreads_or(v);
+  } else {
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbar.red.or.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(any)
+                 : "r"(v), "n"(BAR), "n"(NTHREADS)
+                 : "memory");
+    return (int)any;
+  }
+}
+
 // Exchange of up to four per-row partial sums across the four warps of the CTA.
 struct __align__(16) Xch4 {
   float4 v[CS][5];  // [row][warp] with the row padded to 80 bytes: the 8 rows a warp reads fall in distinct banks
@@ -66,7 +86,7 @@ __device__ __forceinline__ void xch_rows(Xch4* xb, const Lane& L, const float4 a
   }
 }
 // Two-value variant (same buffer type, half the shuffles).
-template <int SEG = 64, bool FLAG = true>
+template <int SEG = 64, bool FLAG = true, int BAR = 0>
 __device__ __forceinline__ void xch_rows2(Xch4* xb, const Lane& L, float a0x, float a0y, float a1x, float a1y,
                                           float2& o0, float2& o1, int& flag) {
   a0x = quad_sum(a0x); a0y = quad_sum(a0y); a1x = quad_sum(a1x); a1y = quad_sum(a1y);
@@ -76,8 +96,8 @@ __device__ __forceinline__ void xch_rows2(Xch4* xb, const Lane& L, float a0x, fl
     base[L.g * 6 + L.warp] = make_float2(a0x, a0y);
     base[(L.g + 8) * 6 + L.warp] = make_float2(a1x, a1y);
   }
-  if constexpr (FLAG) flag = __syncthreads_or(flag);
-  else __syncthreads();
+  if constexpr (FLAG) flag = group_sync_or<BAR>(flag);
+  else group_sync<BAR>();
   const float4 p = *reinterpret_cast<const float4*>(&base[L.g * 6]);
   const float4 q = *reinterpret_cast<const float4*>(&base[L.g * 6 + 2]);
   const float4 p2 = *reinterpret_cast<const float4*>(&base[(L.g + 8) * 6]);
@@ -96,7 +116,7 @@ __device__ __forceinline__ void xch_rows2(Xch4* xb, const Lane& L, float a0x, fl
 // LayerNorm row statistics of a slab: mean and 1/sqrt(var + eps) for rows g and g+8.
 // bf16 I/O uses one exchange (sum, sum of squares); float32 I/O uses the two-pass variance of the reference.
 // Slabs here are column pairs: F2 z[nt][r] = columns (nb + 8nt + 2t, +1) of row g + 8r.
-template <bool TWO_PASS, int SEG = 64, bool FLAG = true>
+template <bool TWO_PASS, int SEG = 64, bool FLAG = true, int BAR = 0>
 __device__ __forceinline__ void ln_row_stats(const F2 (&z)[2][2], Xch4* xch, int& xsel, const Lane& L, float eps,
                                              float (&mean)[2], float (&rstd)[2], int& flag) {
   constexpr float INV = 1.f / SEG;  // features per LayerNorm row
@@ -107,7 +127,7 @@ __device__ __forceinline__ void ln_row_stats(const F2 (&z)[2][2], Xch4* xch, int
     if constexpr (!TWO_PASS) s2[r] = f2hsum(f2fma(z[0][r], z[0][r], f2mul(z[1][r], z[1][r])));
   }
   float2 a0, a1;
-  xch_rows2<SEG, FLAG>(&xch[xsel], L, s1[0], s2[0], s1[1], s2[1], a0, a1, flag);
+  xch_rows2<SEG, FLAG, BAR>(&xch[xsel], L, s1[0], s2[0], s1[1], s2[1], a0, a1, flag);
   xsel ^= 1;
   mean[0] = a0.x * INV;
   mean[1] = a1.x * INV;
@@ -122,10 +142,10 @@ __device__ __forceinline__ void ln_row_stats(const F2 (&z)[2][2], Xch4* xch, int
       q2[r] = f2hsum(f2fma(d0, d0, f2mul(d1, d1)));
     }
     int f2_ = 0;
-    xch_rows2<SEG, false>(&xch[xsel], L, q2[0], 0.f, q2[1], 0.f, a0, a1, f2_);
+    xch_rows2<SEG, false, BAR>(&xch[xsel], L, q2[0], 0.f, q2[1], 0.f, a0, a1, f2_);
     xsel ^= 1;
-    rstd[0] = 1.0f / sqrtf(a0.x * INV + eps);
-    rstd[1] = 1.0f / sqrtf(a1.x * INV + eps);
+    rstd[0] = __frsqrt_rn(a0.x * INV + eps);
+    rstd[1] = __frsqrt_rn(a1.x * INV + eps);
   }
 }
 
@@ -151,21 +171,27 @@ __device__ __forceinline__ void bfrag_from_state(const float (&m)[8][4], int ks,
 
 // LN + L2 gradient pieces for one slab of Z1 given its row statistics.
 // Outputs x_hat, gy = gamma*x_hat + beta - (v - k), gx = gy*gamma and the per-thread partial row sums of gx, gx*x_hat.
-// gam / bet: the thread's column pairs, index nt.
+// gam / bet: the thread's column pairs, index nt; btg = beta - (v - k).
 template <typename T, int SEG>
-__device__ __forceinline__ void ln_l2_pieces(const F2 (&z1)[2][2], const float (&mean)[2], const float (&rstd)[2],
-                                             const F2 (&gam)[2], const F2 (&bet)[2], uint32_t tk, uint32_t tv,
-                                             const Lane& L, F2 (&xh)[2][2], F2 (&gy)[2][2], F2 (&gx)[2][2],
-                                             float (&sa)[2], float (&sb)[2]) {
-  F2 pa[2] = {f2(0.f), f2(0.f)}, pb[2] = {f2(0.f), f2(0.f)};
+__device__ __forceinline__ void beta_minus_target(const F2 (&bet)[2], uint32_t tk, uint32_t tv, const Lane& L, F2 (&btg)[2][2]) {
 #pragma unroll
   for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int row = L.g + 8 * r, col = L.nb + 8 * nt + 2 * L.t;
-      const F2 tg = f2sub(ld_io<T, SEG>(tv, row, col), ld_io<T, SEG>(tk, row, col));
+      btg[nt][r] = f2sub(bet[nt], f2sub(ld_io<T, SEG>(tv, row, col), ld_io<T, SEG>(tk, row, col)));
+    }
+}
+__device__ __forceinline__ void ln_l2_pieces(const F2 (&z1)[2][2], const float (&mean)[2], const float (&rstd)[2],
+                                             const F2 (&gam)[2], const F2 (&btg)[2][2], F2 (&xh)[2][2], F2 (&gy)[2][2],
+                                             F2 (&gx)[2][2], float (&sa)[2], float (&sb)[2]) {
+  F2 pa[2] = {f2(0.f), f2(0.f)}, pb[2] = {f2(0.f), f2(0.f)};
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
       const F2 x = f2mul(f2sub(z1[nt][r], f2(mean[r])), f2(rstd[r]));
-      const F2 y = f2fma(gam[nt], x, f2sub(bet[nt], tg));
+      const F2 y = f2fma(gam[nt], x, btg[nt][r]);
       const F2 gg = f2mul(y, gam[nt]);
       xh[nt][r] = x;
       gy[nt][r] = y;
@@ -198,13 +224,15 @@ __device__ __forceinline__ void g_from_pieces(const F2 (&gx)[2][2], const F2 (&x
 template <int NP, int SEG = 64>
 __device__ __forceinline__ void state_update_direct(float (&wt)[8][4], const Pk<NP> (&agt)[4], uint32_t k_planes,
                                                     int lane, int khalf = -1) {
+  typedef std::conditional_t<NP == 1, __nv_bfloat16, float> T;
 #pragma unroll
-  for (int kp = 0; kp < 4; ++kp) {
+  for (int kp = 0; kp < 4; kp += 2) {
     if (khalf >= 0 && (kp >> 1) != khalf) continue;
-    Pk<NP> bk[4];
-    ldsm_np<NP>(bk, k_planes + lane_off_io<std::conditional_t<NP == 1, __nv_bfloat16, float>, SEG>(lane, 16 * kp), TILE_BF16_BYTES, true);
-    const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]};
-    mma_np2<NP>(wt[2 * kp], agt, b0, wt[2 * kp + 1], agt, b1);
+    Pk<NP> bk[4], bl[4];
+    ldsm_np<NP>(bk, k_planes + lane_off_io<T, SEG>(lane, 16 * kp), TILE_BF16_BYTES, true);
+    ldsm_np<NP>(bl, k_planes + lane_off_io<T, SEG>(lane, 16 * kp + 16), TILE_BF16_BYTES, true);
+    const Pk<NP> b0[2] = {bk[0], bk[1]}, b1[2] = {bk[2], bk[3]}, b2[2] = {bl[0], bl[1]}, b3[2] = {bl[2], bl[3]};
+    mma_np_n<NP, 4>({&wt[2 * kp], &wt[2 * kp + 1], &wt[2 * kp + 2], &wt[2 * kp + 3]}, {&agt, &agt, &agt, &agt}, {&b0, &b1, &b2, &b3});
   }
 }
 template <int NP>
