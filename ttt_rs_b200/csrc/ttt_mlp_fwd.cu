@@ -72,13 +72,13 @@ __device__ __forceinline__ F2 gelu2(F2 z, F2* deriv) {
 // row sums of two values over the 8 warps (rows g and g+8); buffer float2[16][10] (rows padded to 80 bytes so that
 // the 8 rows a warp reads fall in distinct banks)
 __device__ __forceinline__ void xch8(float2* xb, const Lane& L, float a0x, float a0y, float a1x, float a1y, float2& o0,
-                                     float2& o1, int& flag) {
+                                     float2& o1) {
   a0x = quad_sum(a0x); a0y = quad_sum(a0y); a1x = quad_sum(a1x); a1y = quad_sum(a1y);
   if (L.t == 0) {
     xb[L.g * 10 + L.warp] = make_float2(a0x, a0y);
     xb[(L.g + 8) * 10 + L.warp] = make_float2(a1x, a1y);
   }
-  flag = __syncthreads_or(flag);
+  __syncthreads();
   float2 s0 = make_float2(0.f, 0.f), s1 = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -91,6 +91,9 @@ __device__ __forceinline__ void xch8(float2* xb, const Lane& L, float a0x, float
   o1 = s1;
 }
 
+__device__ __forceinline__ void stsm_x4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // offset of element (row, col) of a 16 x 256 operand tile stored as four [16][64] swizzled sub-tiles
 __device__ __forceinline__ uint32_t off_e(int row, int col) {
   return static_cast<uint32_t>((col >> 6) * TILE_BF16_BYTES) + off_bf16(row, col & 63);
@@ -185,12 +188,11 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int rn = 0; rn < 2; ++rn)
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(tW2 + (2 * warp + mt) * TL + off_bf16(g + 8 * rn, 8 * nt + 2 * t)),
-                       "r"(pack_bf16(w2[mt][nt][2 * rn] * wscale, w2[mt][nt][2 * rn + 1] * wscale))
-                       : "memory");
+      for (int nt = 0; nt < 8; nt += 2)  // four 8 x 8 blocks: (row half, column tile) = (0, nt), (1, nt), (0, nt + 1), (1, nt + 1)
+        stsm_x4(tW2 + (2 * warp + mt) * TL + off_bf16(lane & 15, 8 * (nt + (lane >> 4))),
+                pack_bf16(w2[mt][nt][0] * wscale, w2[mt][nt][1] * wscale), pack_bf16(w2[mt][nt][2] * wscale, w2[mt][nt][3] * wscale),
+                pack_bf16(w2[mt][nt + 1][0] * wscale, w2[mt][nt + 1][1] * wscale),
+                pack_bf16(w2[mt][nt + 1][2] * wscale, w2[mt][nt + 1][3] * wscale));
   };
 
   int xsel = 0;
@@ -354,10 +356,15 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         x2[j][r] = gelu2(pr(z1[j], r), &d1[j][r]);
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tX2 + off_e(g + 8 * r, eb + 8 * j + 2 * t)),
-                     "r"(pack_bf16(x2[j][r].x, x2[j][r].y))
-                     : "memory");
       }
+    const uint32_t own_off = off_e(lane & 15, eb + 8 * (lane >> 4));  // stmatrix address of this warp's 16 first columns
+    auto put_own = [&](uint32_t tile, const F2 (&x)[4][2]) {
+#pragma unroll
+      for (int j = 0; j < 4; j += 2)
+        stsm_x4((tile + own_off) ^ (16 * j), pack_bf16(x[j][0].x, x[j][0].y), pack_bf16(x[j][1].x, x[j][1].y),
+                pack_bf16(x[j + 1][0].x, x[j + 1][0].y), pack_bf16(x[j + 1][1].x, x[j + 1][1].y));
+    };
+    put_own(tX2, x2);
     if (SAVE) fence_proxy_async_smem();  // (X2 also leaves by a bulk copy)
     fail = __syncthreads_or(fail);  // B1: X2 tile and the refreshed W2 copy are visible; previous stage fully left
     if (fail) {
@@ -372,17 +379,24 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     const int m_ = lane >> 3, r_ = lane & 7;
     const uint32_t w2_lane = tW2 + (m_ >> 1) * TL + off_bf16(r_ + ((m_ & 1) << 3), fb);
     // ---- S3. Z2 = X2 W2 + b2 (columns fb..fb+7)
-    float z2[4] = {b2v.x, b2v.y, b2v.x, b2v.y};
+    // (four accumulators take turns: one would be a chain of 16 dependent products)
+    auto sum_over_hidden = [&](float (&z)[4], const uint32_t tile) {
+      float c[3][4] = {};
 #pragma unroll
-    for (int kp = 0; kp < 8; ++kp) {
-      Pk<1> a0[4], a1[4];
-      uint32_t bb[4];
-      ldsm_np<1>(a0, tX2 + (kp >> 1) * TL + lane_off_A(lane, (kp & 1) * 32), TL, false);
-      ldsm_np<1>(a1, tX2 + (kp >> 1) * TL + lane_off_A(lane, (kp & 1) * 32 + 16), TL, false);
-      ldsm_x4_t(bb, w2_lane + 2 * kp * TL);
-      mma_bf16(z2, a0[0].p[0], a0[1].p[0], a0[2].p[0], a0[3].p[0], bb[0], bb[1]);
-      mma_bf16(z2, a1[0].p[0], a1[1].p[0], a1[2].p[0], a1[3].p[0], bb[2], bb[3]);
-    }
+      for (int kp = 0; kp < 8; ++kp) {
+        Pk<1> a0[4], a1[4];
+        uint32_t bb[4];
+        ldsm_np<1>(a0, tile + (kp >> 1) * TL + lane_off_A(lane, (kp & 1) * 32), TL, false);
+        ldsm_np<1>(a1, tile + (kp >> 1) * TL + lane_off_A(lane, (kp & 1) * 32 + 16), TL, false);
+        ldsm_x4_t(bb, w2_lane + 2 * kp * TL);
+        mma_bf16((kp & 1) ? c[1] : z, a0[0].p[0], a0[1].p[0], a0[2].p[0], a0[3].p[0], bb[0], bb[1]);
+        mma_bf16((kp & 1) ? c[2] : c[0], a1[0].p[0], a1[1].p[0], a1[2].p[0], a1[3].p[0], bb[2], bb[3]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[i] = (z[i] + c[0][i]) + (c[1][i] + c[2][i]);
+    };
+    float z2[4] = {b2v.x, b2v.y, b2v.x, b2v.y};
+    sum_over_hidden(z2, tX2);
     if (SAVE) {
 #pragma unroll
       for (int r = 0; r < 2; ++r)
@@ -393,9 +407,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     {
       const F2 zp[2] = {pr(z2, 0), pr(z2, 1)};
       float2 a0, a1;
-      int f0 = 0;
       xch8(xchb + xsel * 160, L, f2hsum(zp[0]), f2hsum(f2mul(zp[0], zp[0])), f2hsum(zp[1]), f2hsum(f2mul(zp[1], zp[1])),
-           a0, a1, f0);
+           a0, a1);
       xsel ^= 1;
       const float mean[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)};
       const float rstd[2] = {rsqrtf(fmaxf(a0.y * (1.f / HD) - mean[0] * mean[0], 0.f) + p.eps),
@@ -408,7 +421,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         gg[r] = f2mul(f2fma(gam, x[r], f2sub(bet, tg)), gam);
       }
       xch8(xchb + xsel * 160, L, f2hsum(gg[0]), f2hsum(f2mul(gg[0], x[0])), f2hsum(gg[1]), f2hsum(f2mul(gg[1], x[1])),
-           a0, a1, f0);
+           a0, a1);
       xsel ^= 1;
       const float A[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)}, Bv[2] = {a0.y * (1.f / HD), a1.y * (1.f / HD)};
       if (SAVE && warp == 0 && t < 2)
@@ -481,10 +494,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         xb2[j][r] = gelu2(pr(zq[j], r), nullptr);
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(tXB2 + off_e(g + 8 * r, eb + 8 * j + 2 * t)),
-                     "r"(pack_bf16(xb2[j][r].x, xb2[j][r].y))
-                     : "memory");
       }
+    put_own(tXB2, xb2);
     float a2[2][4];
     {
       float a2p[2][4];
@@ -516,16 +527,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     }
     // ---- S9. Zb2 = Xb2 W2 + b2 - M2' G2p (columns fb..fb+7)
     float zb2[4] = {b2v.x, b2v.y, b2v.x, b2v.y};
-#pragma unroll
-    for (int kp = 0; kp < 8; ++kp) {
-      Pk<1> a0[4], a1[4];
-      uint32_t bb[4];
-      ldsm_np<1>(a0, tXB2 + (kp >> 1) * TL + lane_off_A(lane, (kp & 1) * 32), TL, false);
-      ldsm_np<1>(a1, tXB2 + (kp >> 1) * TL + lane_off_A(lane, (kp & 1) * 32 + 16), TL, false);
-      ldsm_x4_t(bb, w2_lane + 2 * kp * TL);
-      mma_bf16(zb2, a0[0].p[0], a0[1].p[0], a0[2].p[0], a0[3].p[0], bb[0], bb[1]);
-      mma_bf16(zb2, a1[0].p[0], a1[1].p[0], a1[2].p[0], a1[3].p[0], bb[2], bb[3]);
-    }
+    sum_over_hidden(zb2, tXB2);
     {
       Pk<1> am2[4];
       masked_operand(a2, am2);
@@ -542,9 +544,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     {
       const F2 zp[2] = {pr(zb2, 0), pr(zb2, 1)};
       float2 a0, a1;
-      int f0 = 0;
       xch8(xchb + xsel * 160, L, f2hsum(zp[0]), f2hsum(f2mul(zp[0], zp[0])), f2hsum(zp[1]), f2hsum(f2mul(zp[1], zp[1])),
-           a0, a1, f0);
+           a0, a1);
       xsel ^= 1;
       const float mean[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)};
       const float rstd[2] = {rsqrtf(fmaxf(a0.y * (1.f / HD) - mean[0] * mean[0], 0.f) + p.eps),
