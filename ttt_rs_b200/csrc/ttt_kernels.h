@@ -165,6 +165,7 @@ struct LayerEpiParams {
   const void* ln_b;
   void* y;                // [B,T,H*F]
   int row_groups;         // set by the launcher: rows of a tile that a CTA's threads work on at once
+  int tile_rows;          // set by the launcher: tokens of a tile
   int B, H, T;
   float eps;
 };
@@ -235,6 +236,7 @@ struct LayerEpiBwdParams {
   float* d_ln_b;
   float* partials;        // workspace (float32): [CTAs][2][H*F] partial sums
   int row_groups;         // set by the launcher: rows of a tile that a CTA's threads work on at once
+  int tile_rows;          // set by the launcher: tokens of a tile
   int B, H, T;
   float eps;
 };

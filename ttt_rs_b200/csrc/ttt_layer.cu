@@ -24,6 +24,8 @@ struct Vec8<__nv_bfloat16> {
   uint4 raw;
   __device__ __forceinline__ void load(const void* p) { raw = *reinterpret_cast<const uint4*>(p); }
   __device__ __forceinline__ void store(void* p) const { *reinterpret_cast<uint4*>(p) = raw; }
+  __device__ __forceinline__ void load_once(const void* p) { raw = __ldcs(reinterpret_cast<const uint4*>(p)); }
+  __device__ __forceinline__ void store_once(void* p) const { __stcs(reinterpret_cast<uint4*>(p), raw); }
   __device__ __forceinline__ void unpack(float (&f)[8]) const {
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
@@ -49,6 +51,14 @@ struct Vec8<float> {
   __device__ __forceinline__ void store(void* p) const {
     reinterpret_cast<float4*>(p)[0] = a;
     reinterpret_cast<float4*>(p)[1] = b;
+  }
+  __device__ __forceinline__ void load_once(const void* p) {
+    a = __ldcs(reinterpret_cast<const float4*>(p));
+    b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+  }
+  __device__ __forceinline__ void store_once(void* p) const {
+    __stcs(reinterpret_cast<float4*>(p), a);
+    __stcs(reinterpret_cast<float4*>(p) + 1, b);
   }
   __device__ __forceinline__ void unpack(float (&f)[8]) const {
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
@@ -231,11 +241,34 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
 // CTAs per SM: one fewer for float32 without a gate, which is at 0.9 of the memory rate with two (67 against 76 us at 768).
 // MAXCH: 16-byte chunks of one row per lane (rows of up to 32 * MAXCH chunks = 512 * MAXCH bytes).
 constexpr int EPI_THREADS = 384;
+// A CTA's tiles: tile `first + i * stride` of a batch of sequences cut into `per_b` tiles each, as (sequence, tile in it); stepped
+// without dividing (two 64-bit divisions per tile were a third of the instructions)
+struct TileWalk {
+  int b, t, per_b, step_b, step_t;
+  long left;  // tiles from this one to the last
+  __device__ __forceinline__ TileWalk(long first, long stride, long ntiles, int per_b_) : per_b(per_b_) {
+    b = (int)(first / per_b);
+    t = (int)(first - (long)b * per_b);
+    step_b = (int)(stride / per_b);
+    step_t = (int)(stride - (long)step_b * per_b);
+    left = ntiles - first;
+  }
+  __device__ __forceinline__ bool valid() const { return left > 0; }
+  __device__ __forceinline__ void step(long stride) {
+    left -= stride;
+    b += step_b;
+    t += step_t;
+    if (t >= per_b) {
+      t -= per_b;
+      ++b;
+    }
+  }
+};
 template <typename T, int MAXCH, int FD, bool GATE>
 __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_THREADS, (MAXCH == 16 ? 2 : 3) - (sizeof(T) == 4 && !GATE ? 1 : 0))
     ttt_layer_epilogue_kernel(const LayerEpiParams p) {
   constexpr int HD = FD;  // features per head in this instantiation
-  constexpr int TT = 64 / MAXCH;
+  const int TT = p.tile_rows;
   constexpr int EPC = 16 / sizeof(T);  // elements per 16-byte chunk
   constexpr int NPAIR = EPC / 2;
   extern __shared__ __align__(16) uint8_t epi_smem[];
@@ -258,9 +291,10 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_THREADS, (MAXCH == 16 
       v[1] = f2(__uint_as_float(raw.z), __uint_as_float(raw.w));
     }
   };
-  auto fetch = [&](long tile_id, int buf) {
-    if (tile_id < ntiles && my_grp < ngroups) {
-      const int b = (int)(tile_id / tiles_per_b), t0 = (int)(tile_id - (long)b * tiles_per_b) * TT;
+  TileWalk ahead(blockIdx.x, gridDim.x, ntiles, tiles_per_b), cur = ahead;
+  auto fetch = [&](int buf) {  // the next tile that is not on its way yet
+    if (ahead.valid() && my_grp < ngroups) {
+      const int b = ahead.b, t0 = ahead.t * TT;
       const int rows = min(TT, NT - t0);
       const uint32_t dst = smem_u32(epi_smem + buf * tile_bytes) + (uint32_t)(c_own * sizeof(T));
       const T* z = static_cast<const T*>(p.inner_out) + (((size_t)b * H + h_own) * NT + t0) * HD + f_own;
@@ -270,6 +304,7 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_THREADS, (MAXCH == 16 
                      : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+    ahead.step(gridDim.x);
   };
   F2 gam[NPAIR], bet[NPAIR];
 #pragma unroll
@@ -278,11 +313,11 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_THREADS, (MAXCH == 16 
     bet[k] = f2(ld_as_float<T>(p.ln_b, (size_t)c_own + 2 * k), ld_as_float<T>(p.ln_b, (size_t)c_own + 2 * k + 1));
   }
   int buf = 0;
-  fetch(blockIdx.x, 0);
-  for (long tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, buf ^= 1) {
-    const int b = (int)(tile_id / tiles_per_b), t0 = (int)(tile_id - (long)b * tiles_per_b) * TT;
+  fetch(0);
+  for (; cur.valid(); cur.step(gridDim.x), buf ^= 1) {
+    const int b = cur.b, t0 = cur.t * TT;
     const int rows = min(TT, NT - t0);
-    fetch(tile_id + gridDim.x, buf ^ 1);  // the other buffer was released by the barrier that ended the last tile
+    fetch(buf ^ 1);  // that buffer was released by the barrier that ended the last tile
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();  // this tile has landed for every thread
     const uint8_t* tile = epi_smem + buf * tile_bytes;
@@ -360,10 +395,10 @@ static int sm_count() {
 // Grid of the two prologue kernels: one warp per (batch, group of 256 / head_dim heads, token chunk), capped.  The chunk
 // is halved down to one group of PRO_TG tokens while the tasks leave schedulers without a second warp: a chunk is a chain
 // of loads and stores, and a short prompt's time is that chain (1 x 1001 tokens, 12 heads: 20.4 us with chunks of 32).
-static int prologue_grid(int B, int H, int T, int head_dim, int* tchunk) {
+static int prologue_grid(int B, int H, int T, int head_dim, int first_chunk, int per_sm, int* tchunk) {
   const int hpw = 256 / head_dim;
-  const long cap = (long)sm_count() * 8;
-  int ch = PRO_TCHUNK;
+  const long cap = (long)sm_count() * per_sm;
+  int ch = first_chunk;
   auto tasks = [&](int c) { return (long)B * ((H + hpw - 1) / hpw) * ((T + c - 1) / c); };
   while (ch > PRO_TG && tasks(ch) < (long)sm_count() * 8) ch /= 2;
   *tchunk = ch;
@@ -381,7 +416,7 @@ static void launch_pro_t(const LayerProParams& p, int grid, cudaStream_t st) {
 
 cudaError_t launch_layer_prologue(int dtype, int head_dim, const LayerProParams& p0, cudaStream_t st) {
   LayerProParams p = p0;
-  const int grid = prologue_grid(p.B, p.H, p.T, head_dim, &p.tchunk);
+  const int grid = prologue_grid(p.B, p.H, p.T, head_dim, PRO_TCHUNK, 8, &p.tchunk);
   if (head_dim == 32) {
     if (dtype == 1) launch_pro_t<__nv_bfloat16, 32>(p, grid, st);
     else launch_pro_t<float, 32>(p, grid, st);
@@ -397,11 +432,14 @@ static cudaError_t launch_epi_g(LayerEpiParams p, cudaStream_t st) {
   const int C = p.H * FD, nch = C / (16 / (int)sizeof(T));
   constexpr int TT = 64 / MAXCH, MAXT = MAXCH == 16 ? 512 : EPI_THREADS;
   auto kfn = ttt_layer_epilogue_kernel<T, MAXCH, FD, GATE>;
-  // as many row groups as fit a CTA and divide the rows of a tile evenly (65536 x 512, bf16: 39.8 us with 6 groups, 35.8 with 4)
+  // as many row groups as fit a CTA, a tile of a row per warp, of groups that divide its rows evenly (65536 x 512, bf16: 39.8 us
+  // with 6 groups of 16 rows, 35.8 with 4; 65536 x 768: 45.1 us with 12 warps for 16 rows, 43.5 for 12)
   p.row_groups = MAXT / nch < TT ? MAXT / nch : TT;
-  while (TT % p.row_groups) --p.row_groups;
+  p.tile_rows = (p.row_groups * nch + 31) / 32 < TT ? (p.row_groups * nch + 31) / 32 : TT;
+  if (p.row_groups > p.tile_rows) p.row_groups = p.tile_rows;
+  while (p.tile_rows % p.row_groups) --p.row_groups;
   const int threads = (p.row_groups * nch + 31) & ~31;
-  const size_t smem = 2 * (size_t)TT * C * sizeof(T) + TT * sizeof(float2);
+  const size_t smem = 2 * (size_t)p.tile_rows * C * sizeof(T) + p.tile_rows * sizeof(float2);
   static DeviceValue resident;
   int per_sm = 1;
   cudaError_t e = resident.get((uint32_t)C, &per_sm, [&](int* n) {
@@ -411,7 +449,7 @@ static cudaError_t launch_epi_g(LayerEpiParams p, cudaStream_t st) {
     return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, threads, smem);
   });
   if (e != cudaSuccess) return e;
-  const long ntiles = (long)p.B * ((p.T + TT - 1) / TT);
+  const long ntiles = (long)p.B * ((p.T + p.tile_rows - 1) / p.tile_rows);
   const long cap = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
   const int grid = (int)(ntiles < cap ? ntiles : cap);
   kfn<<<grid < 1 ? 1 : grid, threads, smem, st>>>(p);
@@ -468,8 +506,8 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
   const int hgroups = (H + HPW - 1) / HPW, tchunks = (NT + p.tchunk - 1) / p.tchunk;
   const long ntasks = (long)p.B * hgroups * tchunks;
   for (long task = (long)blockIdx.x * (PRO_THREADS / 32) + warp; task < ntasks; task += (long)gridDim.x * (PRO_THREADS / 32)) {
-    const int tc = (int)(task % tchunks);
-    const int hg = (int)((task / tchunks) % hgroups);
+    const int hg = (int)(task % hgroups);
+    const int tc = (int)((task / hgroups) % tchunks);
     const int b = (int)(task / ((long)tchunks * hgroups));
     const int h = HPW * hg + hq;
     if (h >= H) continue;
@@ -514,26 +552,35 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
             vk[u].pack(fk);
           }
           const size_t drow = ((size_t)b * NT + t) * p.ld_dst + col;
-          vq[u].store(static_cast<T*>(p.dq_dst) + drow);
-          vk[u].store(static_cast<T*>(p.dk_dst) + drow);
-          vv[u].store(static_cast<T*>(p.dv_dst) + drow);
+          vq[u].store_once(static_cast<T*>(p.dq_dst) + drow);
+          vk[u].store_once(static_cast<T*>(p.dk_dst) + drow);
+          vv[u].store_once(static_cast<T*>(p.dv_dst) + drow);
         }
       }
     }
   }
+  // logits' columns, four elements of a thread at a time (their loads in flight together)
   const float inv_c = (float)F / p.base_lr;
-  const long nlr = (long)p.B * NT * p.lr_cols;
-  for (long e = (long)blockIdx.x * PRO_THREADS + tid; e < nlr; e += (long)gridDim.x * PRO_THREADS) {
-    const int h = (int)(e % p.lr_cols);
-    const long row = e / p.lr_cols;  // b * T + t
-    float dz = 0.f;
-    if (h < H) {
-      const int t = (int)(row % NT), b = (int)(row / NT);
-      const size_t i = ((size_t)b * H + h) * NT + t;
-      const float lr = ld_as_float<T>(p.lr, i);
-      dz = ld_as_float<T>(p.dlr, i) * lr * (1.f - lr * inv_c);
+  const long nlr = (long)p.B * NT * p.lr_cols, step = (long)gridDim.x * PRO_THREADS;
+  for (long e0 = (long)blockIdx.x * PRO_THREADS + tid; e0 < nlr; e0 += 4 * step) {
+    float lr[4], dl[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long e = e0 + u * step, row = e / p.lr_cols;  // b * T + t
+      const int h = (int)(e % p.lr_cols);
+      lr[u] = dl[u] = 0.f;
+      if (e < nlr && h < H) {
+        const int t = (int)(row % NT), b = (int)(row / NT);
+        const size_t i = ((size_t)b * H + h) * NT + t;
+        lr[u] = ld_as_float<T>(p.lr, i);
+        dl[u] = ld_as_float<T>(p.dlr, i);
+      }
     }
-    st_from_float<T>(p.dlogits_dst, (size_t)row * p.ld_dlr + h, dz);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long e = e0 + u * step;
+      if (e < nlr) st_from_float<T>(p.dlogits_dst, (size_t)(e / p.lr_cols) * p.ld_dlr + (int)(e % p.lr_cols), dl[u] * lr[u] * (1.f - lr[u] * inv_c));
+    }
   }
 }
 
@@ -545,7 +592,7 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
 // shuffles (the mean; then the variance and both sums of dx together).  Column phase: a thread per 16-byte chunk of columns
 // and row group, which writes dz straight to [B,H,T,F] and keeps its columns' parameter sums in registers over all of the
 // CTA's tiles; the row groups meet in shared memory at the end and leave one [2][C] row of `partials` per CTA.
-// 65536 tokens x 768, bf16: 187 -> 86 us without a gate, 359 -> 208 us with one; float32 409 -> 104 us (the parameter sums
+// 65536 tokens x 768, bf16: 187 -> 86 -> 71 us without a gate (the last step: packed arithmetic, tiles of a row per warp, no divisions), 359 -> 208 us with one; float32 409 -> 104 us (the parameter sums
 // were a kernel of their own that read both operands again).  TT: with a gate (whose row phase is bound by tanh) half, so
 // that the tanh values that the column phase uses again fit beside two CTAs' tiles.
 constexpr int EPI_BWD_THREADS = 384;
@@ -553,7 +600,7 @@ template <typename T, int MAXCH, int FD, bool GATE>
 __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T) == 2 || MAXCH == 16) ? 2 : 3)
     ttt_layer_epilogue_bwd_kernel(const LayerEpiBwdParams p) {
   constexpr int HD = FD;  // features per head in this instantiation
-  constexpr int TT = (GATE ? 32 : 64) / MAXCH;
+  const int TT = p.tile_rows;
   constexpr int EPC = 16 / sizeof(T);
   constexpr int CPR = HD / EPC;
   extern __shared__ __align__(16) uint8_t epi_smem[];
@@ -570,10 +617,11 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
   const int my_ch = tid % nch, my_grp = tid / nch, c_own = my_ch * EPC;
   const int h_own = c_own / HD, f_own = c_own - h_own * HD;
 
-  // tile `tile_id`: the inner output to buffer `buf`, dy to buffer 2 + buf (both [TT][C])
-  auto fetch = [&](long tile_id, int buf) {
-    if (tile_id < ntiles) {
-      const int b = (int)(tile_id / tiles_per_b), t0 = (int)(tile_id - (long)b * tiles_per_b) * TT;
+  // the next tile that is not on its way yet: the inner output to buffer `buf`, dy to buffer 2 + buf (both [TT][C])
+  TileWalk ahead(blockIdx.x, gridDim.x, ntiles, tiles_per_b), cur = ahead;
+  auto fetch = [&](int buf) {
+    if (ahead.valid()) {
+      const int b = ahead.b, t0 = ahead.t * TT;
       const int rows = min(TT, NT - t0);
       if (my_grp < ngroups) {
         const uint32_t dst = smem_u32(epi_smem + buf * tile_bytes) + (uint32_t)(c_own * sizeof(T));
@@ -588,42 +636,48 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+    ahead.step(gridDim.x);
   };
-  auto chunk = [](const void* src, float (&f)[EPC]) {
+  constexpr int NPAIR = EPC / 2;
+  auto chunk = [](const void* src, F2 (&f)[NPAIR]) {
+    const uint4 v = *reinterpret_cast<const uint4*>(src);
     if constexpr (sizeof(T) == 2) {
-      Vec8<T> raw;
-      raw.load(static_cast<const T*>(src));
-      raw.unpack(f);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f[k] = f2(bf16_lo(w[k]), bf16_hi(w[k]));
     } else {
-      const float4 v = *reinterpret_cast<const float4*>(src);
-      f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+      f[0] = f2(__uint_as_float(v.x), __uint_as_float(v.y));
+      f[1] = f2(__uint_as_float(v.z), __uint_as_float(v.w));
     }
   };
-  auto gate_chunk = [&](size_t tok, int c0, float (&g)[EPC]) {  // (rows of the gate buffer are aligned to 8 bytes only)
+  auto gate_chunk = [&](size_t tok, int c0, F2 (&g)[NPAIR]) {  // (rows of the gate buffer are aligned to 8 bytes only)
     const uint2* src = reinterpret_cast<const uint2*>(static_cast<const T*>(p.gate) + tok * p.ld_gate + c0);
     const uint2 a = src[0], b = src[1];
     if constexpr (sizeof(T) == 2) {
-      g[0] = bf16_lo(a.x); g[1] = bf16_hi(a.x); g[2] = bf16_lo(a.y); g[3] = bf16_hi(a.y);
-      g[4] = bf16_lo(b.x); g[5] = bf16_hi(b.x); g[6] = bf16_lo(b.y); g[7] = bf16_hi(b.y);
+      const uint32_t w[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) g[k] = f2(bf16_lo(w[k]), bf16_hi(w[k]));
     } else {
-      g[0] = __uint_as_float(a.x); g[1] = __uint_as_float(a.y); g[2] = __uint_as_float(b.x); g[3] = __uint_as_float(b.y);
+      g[0] = f2(__uint_as_float(a.x), __uint_as_float(a.y));
+      g[1] = f2(__uint_as_float(b.x), __uint_as_float(b.y));
     }
   };
   auto gelu_tanh = [](float g) { return tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)); };
 
-  float ag[EPC], ab[EPC], gam_own[EPC], bet_own[EPC];
+  F2 ag[NPAIR], ab[NPAIR], gam_own[NPAIR], bet_own[NPAIR];
 #pragma unroll
-  for (int e = 0; e < EPC; ++e) {
-    ag[e] = ab[e] = 0.f;
-    gam_own[e] = ld_as_float<T>(p.ln_w, (size_t)(c_own + e));
-    bet_own[e] = GATE ? ld_as_float<T>(p.ln_b, (size_t)(c_own + e)) : 0.f;
+  for (int k = 0; k < NPAIR; ++k) {
+    const size_t c = (size_t)(c_own + 2 * k);
+    ag[k] = ab[k] = f2(0.f);
+    gam_own[k] = f2(ld_as_float<T>(p.ln_w, c), ld_as_float<T>(p.ln_w, c + 1));
+    bet_own[k] = GATE ? f2(ld_as_float<T>(p.ln_b, c), ld_as_float<T>(p.ln_b, c + 1)) : f2(0.f);
   }
   int buf = 0;
-  fetch(blockIdx.x, 0);
-  for (long tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, buf ^= 1) {
-    const int b = (int)(tile_id / tiles_per_b), t0 = (int)(tile_id - (long)b * tiles_per_b) * TT;
+  fetch(0);
+  for (; cur.valid(); cur.step(gridDim.x), buf ^= 1) {
+    const int b = cur.b, t0 = cur.t * TT;
     const int rows = min(TT, NT - t0);
-    fetch(tile_id + gridDim.x, buf ^ 1);
+    fetch(buf ^ 1);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
     const uint8_t* zt = epi_smem + buf * tile_bytes;
@@ -631,44 +685,48 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
     for (int r = warp; r < rows; r += nwarps) {
       const T* zr = reinterpret_cast<const T*>(zt) + (size_t)r * C;
       const T* yr = reinterpret_cast<const T*>(yt) + (size_t)r * C;
-      float s = 0.f;
+      F2 acc = f2(0.f);
 #pragma unroll
       for (int j = 0; j < MAXCH; ++j)
         if (j * 32 + lane < nch) {
-          float v[EPC];
+          F2 v[NPAIR];
           chunk(zr + (j * 32 + lane) * EPC, v);
 #pragma unroll
-          for (int e = 0; e < EPC; ++e) s += v[e];
+          for (int k = 0; k < NPAIR; ++k) acc = f2add(acc, v[k]);
         }
+      float s = f2hsum(acc);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       const float mean = s / C;
-      float q = 0.f, m1 = 0.f, m2 = 0.f;
+      F2 qq = f2(0.f), a1 = f2(0.f), a2 = f2(0.f);
 #pragma unroll
       for (int j = 0; j < MAXCH; ++j)
         if (j * 32 + lane < nch) {
           const int c0 = (j * 32 + lane) * EPC;
-          float v[EPC], dn[EPC], g[EPC];
+          F2 v[NPAIR], dn[NPAIR];
           chunk(zr + c0, v);
           chunk(yr + c0, dn);
-          float th[EPC];
           if constexpr (GATE) {
+            F2 g[NPAIR], th[NPAIR];
             gate_chunk((size_t)b * NT + t0 + r, c0, g);
 #pragma unroll
-            for (int e = 0; e < EPC; ++e) th[e] = gelu_tanh(g[e]);
+            for (int k = 0; k < NPAIR; ++k) {
+              th[k] = f2(gelu_tanh(g[k].x), gelu_tanh(g[k].y));
+              dn[k] = f2mul(dn[k], f2mul(f2mul(g[k], f2(0.5f)), f2add(th[k], f2(1.f))));
+            }
 #pragma unroll
-            for (int e = 0; e < EPC; e += 4)
-              *reinterpret_cast<float4*>(&th_tile[(size_t)r * C + c0 + e]) = make_float4(th[e], th[e + 1], th[e + 2], th[e + 3]);
+            for (int k = 0; k < NPAIR; k += 2)
+              *reinterpret_cast<float4*>(&th_tile[(size_t)r * C + c0 + 2 * k]) = make_float4(th[k].x, th[k].y, th[k + 1].x, th[k + 1].y);
           }
 #pragma unroll
-          for (int e = 0; e < EPC; ++e) {
-            if constexpr (GATE) dn[e] *= 0.5f * g[e] * (1.f + th[e]);
-            const float x = v[e] - mean, dx = dn[e] * gam[c0 + e];
-            q = fmaf(x, x, q);
-            m1 += dx;
-            m2 = fmaf(dx, x, m2);
+          for (int k = 0; k < NPAIR; ++k) {
+            const F2 x = f2sub(v[k], f2(mean)), dx = f2mul(dn[k], *reinterpret_cast<const F2*>(&gam[c0 + 2 * k]));
+            qq = f2fma(x, x, qq);
+            a1 = f2add(a1, dx);
+            a2 = f2fma(dx, x, a2);
           }
         }
+      float q = f2hsum(qq), m1 = f2hsum(a1), m2 = f2hsum(a2);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         q += __shfl_xor_sync(0xffffffffu, q, o);
@@ -684,48 +742,44 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
       for (int r = my_grp; r < rows; r += ngroups) {
         const float4 st = stat[r];
         const size_t tok = (size_t)b * NT + t0 + r;
-        float z[EPC], dn[EPC];
+        F2 z[NPAIR], dn[NPAIR];
         chunk(reinterpret_cast<const T*>(zt) + (size_t)r * C + c_own, z);
         chunk(reinterpret_cast<const T*>(yt) + (size_t)r * C + c_own, dn);
         if constexpr (GATE) {
-          float g[EPC], dg[EPC];
+          F2 g[NPAIR], dg[NPAIR];
           gate_chunk(tok, c_own, g);
-          float th[EPC];
 #pragma unroll
-          for (int e = 0; e < EPC; e += 4) {
-            const float4 v = *reinterpret_cast<const float4*>(&th_tile[(size_t)r * C + c_own + e]);
-            th[e] = v.x; th[e + 1] = v.y; th[e + 2] = v.z; th[e + 3] = v.w;
-          }
-#pragma unroll
-          for (int e = 0; e < EPC; ++e) {
-            const float g2 = g[e] * g[e];
-            const float dgelu = 0.5f * (1.f + th[e]) + 0.5f * g[e] * (1.f - th[e] * th[e]) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * g2);
-            dg[e] = dn[e] * (gam_own[e] * ((z[e] - st.x) * st.y) + bet_own[e]) * dgelu;
-            dn[e] *= 0.5f * g[e] * (1.f + th[e]);
+          for (int k = 0; k < NPAIR; ++k) {
+            const F2 th = *reinterpret_cast<const F2*>(&th_tile[(size_t)r * C + c_own + 2 * k]);
+            const F2 half = f2fma(th, f2(0.5f), f2(0.5f)), g2 = f2mul(g[k], g[k]);  // 0.5 (1 + tanh)
+            const F2 slope = f2fma(g2, f2(3.f * 0.044715f * 0.7978845608028654f), f2(0.7978845608028654f));
+            const F2 dgelu = f2fma(f2mul(f2mul(g[k], f2(0.5f)), f2fma(f2neg(th), th, f2(1.f))), slope, half);
+            const F2 n = f2fma(gam_own[k], f2mul(f2sub(z[k], f2(st.x)), f2(st.y)), bet_own[k]);
+            dg[k] = f2mul(f2mul(dn[k], n), dgelu);
+            dn[k] = f2mul(dn[k], f2mul(g[k], half));
           }
           uint2* dst = reinterpret_cast<uint2*>(static_cast<T*>(p.dgate) + tok * p.ld_dgate + c_own);
           if constexpr (sizeof(T) == 2) {
-            dst[0] = make_uint2(pack_bf16(dg[0], dg[1]), pack_bf16(dg[2], dg[3]));
-            dst[1] = make_uint2(pack_bf16(dg[4], dg[5]), pack_bf16(dg[6], dg[7]));
+            dst[0] = make_uint2(pack_bf16(dg[0].x, dg[0].y), pack_bf16(dg[1].x, dg[1].y));
+            dst[1] = make_uint2(pack_bf16(dg[2].x, dg[2].y), pack_bf16(dg[3].x, dg[3].y));
           } else {
-            dst[0] = make_uint2(__float_as_uint(dg[0]), __float_as_uint(dg[1]));
-            dst[1] = make_uint2(__float_as_uint(dg[2]), __float_as_uint(dg[3]));
+            dst[0] = make_uint2(__float_as_uint(dg[0].x), __float_as_uint(dg[0].y));
+            dst[1] = make_uint2(__float_as_uint(dg[1].x), __float_as_uint(dg[1].y));
           }
         }
 #pragma unroll
-        for (int e = 0; e < EPC; ++e) {
-          const float xh = (z[e] - st.x) * st.y;
-          ag[e] = fmaf(dn[e], xh, ag[e]);
-          ab[e] += dn[e];
-          z[e] = st.y * (dn[e] * gam_own[e] - st.z - xh * st.w);
+        for (int k = 0; k < NPAIR; ++k) {
+          const F2 xh = f2mul(f2sub(z[k], f2(st.x)), f2(st.y));
+          ag[k] = f2fma(dn[k], xh, ag[k]);
+          ab[k] = f2add(ab[k], dn[k]);
+          z[k] = f2mul(f2fma(xh, f2(-st.w), f2fma(dn[k], gam_own[k], f2(-st.z))), f2(st.y));
         }
-        if constexpr (sizeof(T) == 2) {
-          Vec8<T> o;
-          o.pack(z);
-          o.store(out + (size_t)r * HD);
-        } else {
-          *reinterpret_cast<float4*>(out + (size_t)r * HD) = make_float4(z[0], z[1], z[2], z[3]);
-        }
+        uint4 o;
+        if constexpr (sizeof(T) == 2)
+          o = make_uint4(pack_bf16(z[0].x, z[0].y), pack_bf16(z[1].x, z[1].y), pack_bf16(z[2].x, z[2].y), pack_bf16(z[3].x, z[3].y));
+        else
+          o = make_uint4(__float_as_uint(z[0].x), __float_as_uint(z[0].y), __float_as_uint(z[1].x), __float_as_uint(z[1].y));
+        *reinterpret_cast<uint4*>(out + (size_t)r * HD) = o;
       }
     }
     __syncthreads();  // done with this buffer before the next iteration refills it
@@ -736,9 +790,9 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
   float* red = reinterpret_cast<float*>(epi_smem);
   if (my_grp < ngroups) {
 #pragma unroll
-    for (int e = 0; e < EPC; ++e) {
-      red[(size_t)my_grp * 2 * C + c_own + e] = ag[e];
-      red[(size_t)my_grp * 2 * C + C + c_own + e] = ab[e];
+    for (int k = 0; k < NPAIR; ++k) {
+      *reinterpret_cast<F2*>(&red[(size_t)my_grp * 2 * C + c_own + 2 * k]) = ag[k];
+      *reinterpret_cast<F2*>(&red[(size_t)my_grp * 2 * C + C + c_own + 2 * k]) = ab[k];
     }
   }
   __syncthreads();
@@ -775,7 +829,9 @@ __global__ void __launch_bounds__(256) ttt_layer_epilogue_bwd_reduce_kernel(cons
 
 cudaError_t launch_layer_prologue_bwd(int dtype, int head_dim, const LayerProBwdParams& p0, cudaStream_t st) {
   LayerProBwdParams p = p0;
-  const int grid = prologue_grid(p.B, p.H, p.T, head_dim, &p.tchunk);
+  // as many blocks as are resident, each warp several short tasks: a task per warp was 1.7 rounds of them at 65536 tokens x 768
+  // (130 us; 107 with two blocks of eight warps per SM, head groups of the same tokens side by side and streaming stores)
+  const int grid = prologue_grid(p.B, p.H, p.T, head_dim, PRO_TG, 2, &p.tchunk);
   if (head_dim == 32) {
     if (dtype == 1) ttt_layer_prologue_bwd_kernel<__nv_bfloat16, 32><<<grid, PRO_THREADS, 0, st>>>(p);
     else ttt_layer_prologue_bwd_kernel<float, 32><<<grid, PRO_THREADS, 0, st>>>(p);
@@ -801,7 +857,11 @@ static cudaError_t launch_epi_bwd_g(LayerEpiBwdParams p, cudaStream_t st) {
   // as many row groups as fit a CTA, but no more than a tile has rows
   p.row_groups = MAXT / nch < TT ? MAXT / nch : TT;
   const int threads = (p.row_groups * nch + 31) & ~31;
-  const size_t smem = 4 * (size_t)TT * C * sizeof(T) + TT * sizeof(float4) + (size_t)(GATE ? TT + 1 : 1) * C * sizeof(float);
+  // a row of the tile per warp where the tile is not smaller than that (twelve warps of sixteen rows took two turns)
+  p.tile_rows = threads / 32 < TT ? threads / 32 : TT;
+  if (p.row_groups > p.tile_rows) p.row_groups = p.tile_rows;
+  const size_t smem = 4 * (size_t)p.tile_rows * C * sizeof(T) + p.tile_rows * sizeof(float4) +
+                      (size_t)(GATE ? p.tile_rows + 1 : 1) * C * sizeof(float);
   static DeviceValue resident;
   int per_sm = 1;
   cudaError_t e = resident.get((uint32_t)C, &per_sm, [&](int* n) {
@@ -811,7 +871,7 @@ static cudaError_t launch_epi_bwd_g(LayerEpiBwdParams p, cudaStream_t st) {
     return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, threads, smem);
   });
   if (e != cudaSuccess) return e;
-  const long ntiles = (long)p.B * ((p.T + TT - 1) / TT);
+  const long ntiles = (long)p.B * ((p.T + p.tile_rows - 1) / p.tile_rows);
   long grid = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
   if (grid > EPI_BWD_MAX_CTAS) grid = EPI_BWD_MAX_CTAS;
   if (grid > ntiles) grid = ntiles;
