@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <ATen/autocast_mode.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/torch.h>
 
@@ -590,6 +591,198 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- the outer layer, training -----------------------------------------------------------------------------------------
+// The whole layer as one node of the graph, for the lengths whose projections are a product of their own: the steps of the
+// Python composition (a node per step: its interpreter time is most of a training step of a few thousand tokens) with the
+// same kernels and roundings, forward and backward.  The projections' gradients, the gate's among them, are the columns of one
+// buffer, so the weights' and the input's are one product each.  5 x 192 tokens of 768 features, forward + backward: 1148 us
+// through the composition, 528 here.
+struct LayerDims {
+  ttt_dims d;
+  int64_t B, T, C, H, F, mb, M;
+  int64_t lr, N0, g, N;  // columns q | k | v | lr (and padding) up to N0 | gate from g (-1: none) up to N
+  int64_t K, rope, start, eps_scaled;
+  float theta, base_lr;
+};
+struct LayerFn : torch::autograd::Function<LayerFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& q, const Tensor& k, const Tensor& v,
+                               const Tensor& g, const Tensor& lrw, const Tensor& lrb, const Tensor& learnable,
+                               const Tensor& post_w, const Tensor& post_b, const Tensor& o, const Tensor& w0,
+                               const Tensor& b0, const Tensor& ln_w, const Tensor& ln_b, const Tensor& idx,
+                               const LayerDims& l) {
+    Dims m;
+    m.d = l.d;
+    m.B = l.B, m.H = l.H, m.T = l.T, m.F = l.F;
+    m.dt = x.scalar_type();
+    m.dev = x.device();
+    m.status = g_status[m.dev.index()];
+    c10::cuda::CUDAGuard guard(m.dev);
+    void* const st = m.stream();
+    auto must = [](int rc) {
+      if (rc != TTT_OK) throw_error(rc);
+    };
+    const bool gated = l.g >= 0, bf = m.dt == at::kBFloat16;
+    const Tensor x2 = x.reshape({l.M, l.C}).contiguous();
+    const Tensor lr2 = lrw.reshape({l.H, l.C});  // weights stacked in the order of the columns
+    std::vector<Tensor> rows{q, k, v, lr2};
+    if (l.N0 > l.lr + l.H) rows.push_back(at::zeros({l.N0 - l.lr - l.H, l.C}, m.opt()));
+    if (gated) rows.push_back(g);
+    const Tensor wcat = at::cat(rows, 0);
+    const Tensor te = at::add(idx, learnable);
+    // token_eta of one mini-batch, which is all that is read of it: by the projections' kernel, or here in float32
+    Tensor te16 = bf ? at::empty({16}, m.opt()) : at::clamp_min(te, 0.0);
+    Tensor s[4];
+    for (int i = 0; i < 3; ++i) s[i] = at::empty({l.B, l.H, l.T, l.F}, m.opt());
+    s[3] = at::empty({l.B, l.H, l.T}, m.opt());
+    const void* const ip = bf ? idx.const_data_ptr() : nullptr;
+    const void* const lp = bf ? learnable.const_data_ptr() : nullptr;
+    Tensor gate;
+    {
+      const Tensor proj = at::mm(x2, wcat.narrow(0, 0, l.N0).t());
+      const uint8_t* const p = static_cast<const uint8_t*>(proj.const_data_ptr());
+      const int64_t e = proj.element_size();
+      must(ttt_internal_layer_prologue(&l.d, p, p + e * l.C, p + e * 2 * l.C, l.N0, p + e * l.lr, l.N0, lrb.const_data_ptr(), nullptr,
+                                       nullptr, nullptr, nullptr, 0, (int)l.start, (int)l.rope, l.theta, l.base_lr, ip, lp,
+                                       bf ? te16.data_ptr() : nullptr, s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(),
+                                       s[3].data_ptr(), (int)l.T, st));
+    }
+    if (gated) gate = at::mm(x2, wcat.narrow(0, l.g, l.C).t());
+    LinIn in{{s[0], s[1], s[2], w0, b0, te16, s[3], ln_w, ln_b}};
+    LinOut lo;
+    must(linear_forward(m, in, true, lo));
+    const Tensor y = at::empty({l.M, l.C}, m.opt());
+    must(ttt_layer_epilogue(&l.d, lo.out.const_data_ptr(), gated ? gate.const_data_ptr() : nullptr, gated ? l.C : 0,
+                            post_w.const_data_ptr(), post_b.const_data_ptr(), 1e-6f, y.data_ptr(), st));
+    const Tensor out = at::mm(y, o.t()).view({l.B, l.T, l.C});
+    ctx->save_for_backward({x, wcat, te, lo.out, gate, post_w, post_b, y, o});
+    // kept as plain references, as the inner loop's own node keeps what it saves
+    ctx->saved_data["t"] = std::vector<Tensor>{s[0], s[1], s[2], w0, b0, te16, s[3], ln_w, ln_b, lo.wck, lo.bck};
+    ctx->saved_data["l"] = c10::IValue(std::string(reinterpret_cast<const char*>(&l), sizeof(l)));
+    ctx->saved_data["s"] = std::vector<std::vector<int64_t>>{lrw.sizes().vec(), lrb.sizes().vec()};
+    ctx->mark_non_differentiable({lo.w, lo.b});
+    ctx->set_materialize_grads(false);
+    return {out, lo.w, lo.b};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list go_) {
+    const variable_list sv = ctx->get_saved_variables();
+    const Tensor &x = sv[0], &wcat = sv[1], &te = sv[2], &inner_out = sv[3], &gate = sv[4], &post_w = sv[5], &post_b = sv[6],
+                 &y = sv[7], &o = sv[8];
+    const std::vector<Tensor> t = ctx->saved_data["t"].toTensorVector();
+    LayerDims l;
+    memcpy(&l, ctx->saved_data["l"].toStringRef().data(), sizeof(l));
+    const auto shapes = ctx->saved_data["s"].toList();
+    Dims m;
+    m.d = l.d;
+    m.B = l.B, m.H = l.H, m.T = l.T, m.F = l.F;
+    m.dt = x.scalar_type();
+    m.dev = x.device();
+    m.status = g_status[m.dev.index()];
+    c10::cuda::CUDAGuard guard(m.dev);
+    void* const st = m.stream();
+    auto must = [](int rc) {
+      if (rc != TTT_OK) throw_error(rc);
+    };
+    const Tensor go = (go_[0].defined() ? go_[0] : at::zeros_like(x)).reshape({l.M, l.C}).contiguous();
+    variable_list r(17);  // x q k v g lrw lrb learnable post_w post_b o w0 b0 ln_w ln_b idx dims
+    if (ctx->needs_input_grad(10)) r[10] = at::mm(go.t(), y);
+    const Tensor dy = at::mm(go, o);
+    // post norm and gate: the gate's gradient goes to its columns of the projections' gradient
+    const Tensor dproj = at::empty({l.M, l.N}, m.opt());
+    uint8_t* const dp = static_cast<uint8_t*>(dproj.data_ptr());
+    const int64_t e = dproj.element_size();
+    const bool gated = gate.defined();
+    const Tensor d_inner = at::empty({l.B, l.H, l.T, l.F}, m.opt()), dn = at::empty({2, l.C}, m.opt(at::kFloat));
+    {
+      const size_t wsb = ttt_layer_epilogue_backward_workspace_bytes(&l.d);
+      const Tensor ws = at::empty({(int64_t)wsb}, m.opt(at::kByte));
+      must(ttt_layer_epilogue_backward(&l.d, dy.const_data_ptr(), inner_out.const_data_ptr(), gated ? gate.const_data_ptr() : nullptr,
+                                       gated ? l.C : 0, post_w.const_data_ptr(), post_b.const_data_ptr(), 1e-6f, d_inner.data_ptr(),
+                                       gated ? dp + e * l.g : nullptr, gated ? l.N : 0, static_cast<float*>(dn.data_ptr()),
+                                       static_cast<float*>(dn.data_ptr()) + l.C, ws.data_ptr(), wsb, st));
+    }
+    const Tensor dnt = m.dt == at::kFloat ? dn : dn.to(m.dt);
+    r[8] = dnt.select(0, 0);
+    r[9] = dnt.select(0, 1);
+    LinIn in;
+    for (int i = 0; i < 9; ++i) in.t[i] = t[i];
+    Tensor gr[9];
+    must(linear_backward(m, in, t[9], t[10], d_inner, Tensor(), Tensor(), Tensor(), gr));
+    r[11] = gr[3];
+    r[12] = gr[4];
+    r[13] = gr[7];
+    r[14] = gr[8];
+    must(ttt_layer_prologue_backward(&l.d, gr[0].const_data_ptr(), gr[1].const_data_ptr(), gr[2].const_data_ptr(),
+                                     gr[6].const_data_ptr(), t[6].const_data_ptr(), (int)l.start, (int)l.rope, l.theta, l.base_lr,
+                                     dp, dp + e * l.C, dp + e * 2 * l.C, l.N, dp + e * l.lr, l.N, (int)(l.N0 - l.lr), st));
+    if (ctx->needs_input_grad(0)) r[0] = at::mm(dproj, wcat).view(x.sizes());
+    bool weights = false;
+    for (int i = 1; i <= 5; ++i) weights = weights || ctx->needs_input_grad(i);
+    if (weights) {
+      const Tensor dw = at::mm(dproj.t(), x.reshape({l.M, l.C}));
+      for (int i = 0; i < 3; ++i) r[1 + i] = dw.narrow(0, i * l.C, l.C);
+      if (gated) r[4] = dw.narrow(0, l.g, l.C);
+      r[5] = dw.narrow(0, l.lr, l.H).view(shapes.get(0).toIntVector());
+    }
+    if (ctx->needs_input_grad(6))
+      r[6] = at::sum(dproj.narrow(1, l.lr, l.H), {0}, false, at::kFloat).to(m.dt).view(shapes.get(1).toIntVector());
+    if (ctx->needs_input_grad(7)) {
+      const Tensor sum = at::sum(gr[5].view({l.T / l.mb, l.mb}), {0}, false, m.dt);
+      r[7] = at::where(at::ge(te, 0), sum, at::zeros({}, sum.options()));
+    }
+    return r;
+  }
+};
+// layer_train(x, q_proj, k_proj, v_proj, g_proj | None, lr weight, lr bias, learnable_token_idx, post norm weight, bias, o_proj,
+//             state weight, state bias, ln weight, ln bias, token_idx, heads, mini_batch, rope_mode, rope_theta, base_lr,
+//             checkpoint interval, eps_scaled, start_idx) -> (y, state weight, state bias), recorded for autograd | None
+PyObject* py_layer_train(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 24)) return nullptr;
+  Tensor t[16];
+  for (int i = 0; i < 16; ++i) {
+    if (i == 4 && args[i] == Py_None) continue;
+    NONE_IF(!THPVariable_Check(args[i]));
+    t[i] = THPVariable_Unpack(args[i]);
+    NONE_IF(t[i].unsafeGetTensorImpl()->is_python_dispatch());
+  }
+  LayerDims l;
+  l.H = as_int(args[16]), l.mb = as_int(args[17]), l.rope = as_int(args[18]);
+  l.theta = (float)PyFloat_AsDouble(args[19]), l.base_lr = (float)PyFloat_AsDouble(args[20]);
+  l.K = as_int(args[21]), l.eps_scaled = as_int(args[22]), l.start = as_int(args[23]);
+  if (PyErr_Occurred()) return nullptr;
+  const Tensor& x = t[0];
+  NONE_IF(at::autocast::is_autocast_enabled(at::kCUDA));
+  NONE_IF(!x.is_cuda() || x.layout() != c10::kStrided || x.dim() != 3 || l.H <= 0 || l.mb <= 0);
+  const c10::Device dev = x.device();
+  const at::ScalarType dt = x.scalar_type();
+  NONE_IF((dt != at::kBFloat16 && dt != at::kFloat) || dev.index() >= kMaxDevices || !g_status[dev.index()].defined());
+  l.B = x.size(0), l.T = x.size(1), l.C = x.size(2), l.F = l.C / l.H, l.M = l.B * l.T;
+  NONE_IF(l.M <= 0 || l.M > INT32_MAX || l.F * l.H != l.C || (l.F != 64 && l.F != 32) || l.C > 2048 || l.H > 64 || l.C % 8 != 0);
+  NONE_IF((l.mb != 16 && l.mb != 8) || l.T % l.mb != 0 || (l.F == 32 && l.H % 2 != 0));
+  for (int i : {1, 2, 3, 10}) NONE_IF(!is(t[i], dt, dev, {l.C, l.C}));
+  const bool gated = t[4].defined();
+  NONE_IF(gated && !is(t[4], dt, dev, {l.C, l.C}));
+  NONE_IF(t[5].numel() != l.H * l.C || t[5].size(0) != l.H || t[5].scalar_type() != dt || t[5].device() != dev || !t[5].is_contiguous());
+  NONE_IF(t[6].numel() != l.H || t[6].scalar_type() != dt || t[6].device() != dev || !t[6].is_contiguous());
+  for (int i : {7, 15}) NONE_IF(!is(t[i], dt, dev, {l.mb}));
+  for (int i : {8, 9}) NONE_IF(!is(t[i], dt, dev, {l.C}));
+  NONE_IF(!is(t[11], dt, dev, {l.B, l.H, l.F, l.F}) || !is(t[12], dt, dev, {l.B, l.H, l.F}));
+  for (int i : {13, 14}) NONE_IF(!is(t[i], dt, dev, {l.H, l.F}));
+  for (int i = 0; i < 16; ++i) NONE_IF(t[i].defined() && !on_16_bytes(t[i]));
+  // (those run projections and prologue in one launch: the composition)
+  NONE_IF(dt == at::kBFloat16 && l.T % 128 == 0 && l.F == 64 && l.rope != 2);
+  l.lr = 3 * l.C;
+  l.N0 = (l.lr + l.H + 7) & ~(int64_t)7;
+  l.g = gated ? l.N0 : -1;
+  l.N = l.N0 + (gated ? l.C : 0);
+  l.d = ttt_dims{(int32_t)l.B, (int32_t)l.H, (int32_t)l.T, (int32_t)l.F, (int32_t)l.mb, (int32_t)l.K, (float)l.eps_scaled * 1e-9f,
+                 dt == at::kBFloat16 ? TTT_BF16 : TTT_F32};
+  NONE_IF(ttt_linear_num_checkpoints(&l.d) < 0);
+  if (!gated) t[4] = at::empty({0});  // (a node's arguments are defined tensors)
+  return wrap(LayerFn::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11], t[12], t[13], t[14], t[15], l));
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST(set_status),
@@ -602,6 +795,7 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST(param_key),
                          FAST(stream_key),
                          FAST(layer_infer),
+                         FAST(layer_train),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

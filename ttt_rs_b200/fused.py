@@ -427,6 +427,12 @@ class TTTLinearState:
     bias: torch.Tensor    # [batch, heads, F]
 
 
+def _per_sequence(init: torch.Tensor, batch_size: int) -> torch.Tensor:
+    """One copy of `init` per sequence, with memory of its own (states are advanced in place); repeat() takes three times the
+    host time of this."""
+    return init.expand(batch_size, *init.shape).clone(memory_format=torch.contiguous_format)
+
+
 class TTTLinear(torch.nn.Module):
     """Parameter holder of the TTT-Linear inner model: weight_init [H,F,F] ~ N(0, 0.02), bias_init [H,F] = 0,
     per-head LayerNorm weight = 1 / bias = 0."""
@@ -443,8 +449,7 @@ class TTTLinear(torch.nn.Module):
         self.ln_bias = torch.nn.Parameter(torch.zeros(num_heads, head_dim, **kw))
 
     def init_state(self, batch_size: int) -> TTTLinearState:
-        return TTTLinearState(self.weight_init.unsqueeze(0).repeat(batch_size, 1, 1, 1),
-                              self.bias_init.unsqueeze(0).repeat(batch_size, 1, 1))
+        return TTTLinearState(_per_sequence(self.weight_init, batch_size), _per_sequence(self.bias_init, batch_size))
 
 
 class FusedTileMultiTTTLinear(torch.nn.Module):
@@ -691,8 +696,7 @@ class TTTMLP(torch.nn.Module):
         self.ln_bias = torch.nn.Parameter(torch.zeros(num_heads, head_dim, **kw))
 
     def init_state(self, batch_size: int) -> TTTMLPState:
-        r = lambda t: t.unsqueeze(0).repeat(batch_size, *([1] * t.dim()))  # noqa: E731
-        return TTTMLPState(r(self.w1_init), r(self.b1_init), r(self.w2_init), r(self.b2_init))
+        return TTTMLPState(*(_per_sequence(t, batch_size) for t in (self.w1_init, self.b1_init, self.w2_init, self.b2_init)))
 
 
 class FusedTTTMLP(torch.nn.Module):

@@ -574,11 +574,35 @@ class TTT(torch.nn.Module):
         return self._project(y, self.o_proj.detach())
 
 
+def _train_native(self, x, inner, state, start_idx):
+    """The whole layer as one native autograd node (None: not a case it takes, nothing was done)."""
+    c = self.config
+    if c.share_qk or type(inner) is not FusedTileMultiTTTLinear or not x.is_cuda:
+        return None
+    i = inner._modules["inner"]
+    if type(i) is not TTTLinear or i.mini_batch_size != c.mini_batch_size:
+        return None
+    P, I = self._parameters.get, i._parameters.get
+    r = _lib.host().layer_train(
+        x, P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj") if c.use_gate else None, P("learnable_ttt_lr_weight"),
+        P("learnable_ttt_lr_bias"), P("learnable_token_idx"), P("post_norm_weight"), P("post_norm_bias"), P("o_proj"),
+        state.weight, state.bias, I("ln_weight"), I("ln_bias"), self._buffers.get("token_idx"), c.num_heads,
+        c.mini_batch_size, _POS[c.pos_encoding], c.rope_theta, c.base_lr, i.checkpoint_interval, _eps_scaled(i.epsilon),
+        start_idx)
+    if r is None:
+        return None
+    y, state.weight, state.bias = r
+    return y
+
+
 def _train_forward(self, x, inner, state, start_idx):
     """Training path: the same kernels, each with its gradient kernel, joined by torch autograd.  Where the one-launch
     projections apply (bf16, no shared q / k) they run here as in inference; elsewhere the projection is a library
     product, and the gate's a product of its own, so that every column of the fused projection's gradient is written by
     exactly one kernel.  (65536 tokens of 768 features: one launch instead of product + prologue 300 -> 219 us.)"""
+    y = _train_native(self, x, inner, state, start_idx)
+    if y is not None:
+        return y
     c = self.config
     B, T, _ = x.shape
     H, hs = c.num_heads, c.hidden_size
