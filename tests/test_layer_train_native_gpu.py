@@ -12,10 +12,11 @@ def _step(m, inner, x, gy, leaves):
     return [y.detach(), state.weight, state.bias] + list(grads)
 
 
-def _setup(dtype, B, T, H, F, mb, pos, gate, K=4):
+def _setup(dtype, B, T, H, F, mb, pos, gate, taps=0, K=4):
     import ttt_rs_b200 as tb
     torch.manual_seed(T + H)
-    cfg = tb.TTTLayerConfig(hidden_size=F * H, num_heads=H, mini_batch_size=mb, pos_encoding=pos, use_gate=gate)
+    cfg = tb.TTTLayerConfig(hidden_size=F * H, num_heads=H, mini_batch_size=mb, pos_encoding=pos, use_gate=gate,
+                            **(dict(share_qk=True, conv_kernel_size=taps) if taps else {}))
     m = tb.TTT(cfg, device="cuda", dtype=dtype)
     inner = tb.new_inner(cfg, checkpoint_interval=K, device="cuda", dtype=dtype)
     with torch.no_grad():
@@ -26,14 +27,16 @@ def _setup(dtype, B, T, H, F, mb, pos, gate, K=4):
     return m, inner, x, gy
 
 
-@pytest.mark.parametrize("dtype,B,T,H,F,mb,pos,gate", [
-    (torch.bfloat16, 1, 16, 1, 64, 16, "rope", False), (torch.bfloat16, 2, 144, 3, 64, 16, "rope", True),
-    (torch.bfloat16, 3, 200, 5, 64, 8, "none", True), (torch.bfloat16, 2, 128, 4, 32, 16, "rope", True),
-    (torch.bfloat16, 1, 256, 2, 64, 16, "rope_global", False), (torch.float32, 2, 48, 3, 64, 16, "rope", True),
-    (torch.float32, 1, 128, 2, 64, 16, "rope", False), (torch.float32, 2, 24, 2, 32, 8, "rope", True)])
-def test_one_node_equals_the_composition(monkeypatch, dtype, B, T, H, F, mb, pos, gate):
+@pytest.mark.parametrize("dtype,B,T,H,F,mb,pos,gate,taps", [
+    (torch.bfloat16, 1, 16, 1, 64, 16, "rope", False, 0), (torch.bfloat16, 2, 144, 3, 64, 16, "rope", True, 0),
+    (torch.bfloat16, 3, 200, 5, 64, 8, "none", True, 0), (torch.bfloat16, 2, 128, 4, 32, 16, "rope", True, 0),
+    (torch.bfloat16, 1, 256, 2, 64, 16, "rope_global", False, 0), (torch.float32, 2, 48, 3, 64, 16, "rope", True, 0),
+    (torch.float32, 1, 128, 2, 64, 16, "rope", False, 0), (torch.float32, 2, 24, 2, 32, 8, "rope", True, 0),
+    (torch.bfloat16, 2, 144, 3, 64, 16, "rope", True, 4), (torch.bfloat16, 1, 128, 2, 64, 16, "none", False, 2),
+    (torch.float32, 2, 48, 2, 32, 16, "rope", True, 3)])
+def test_one_node_equals_the_composition(monkeypatch, dtype, B, T, H, F, mb, pos, gate, taps):
     from ttt_rs_b200 import layer as L
-    m, inner, x, gy = _setup(dtype, B, T, H, F, mb, pos, gate)
+    m, inner, x, gy = _setup(dtype, B, T, H, F, mb, pos, gate, taps)
     x.requires_grad_()
     leaves = [x] + list(m.parameters()) + list(inner.inner.parameters())
     used, native = [], L._train_native

@@ -600,7 +600,8 @@ PyObject* py_layer_infer(PyObject*, PyObject* const* args, Py_ssize_t n) {
 struct LayerDims {
   ttt_dims d;
   int64_t B, T, C, H, F, mb, M;
-  int64_t lr, N0, g, N;  // columns q | k | v | lr (and padding) up to N0 | gate from g (-1: none) up to N
+  int64_t v, lr, N0, g, N;  // columns q | k | v | lr (and padding) up to N0 | gate from g (-1: none) up to N
+  int64_t taps;             // shared q / k projection (v = C then): taps of its two convolutions; 0: projections of their own
   int64_t K, rope, start, eps_scaled;
   float theta, base_lr;
 };
@@ -608,8 +609,8 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& q, const Tensor& k, const Tensor& v,
                                const Tensor& g, const Tensor& lrw, const Tensor& lrb, const Tensor& learnable,
                                const Tensor& post_w, const Tensor& post_b, const Tensor& o, const Tensor& w0,
-                               const Tensor& b0, const Tensor& ln_w, const Tensor& ln_b, const Tensor& idx,
-                               const LayerDims& l) {
+                               const Tensor& b0, const Tensor& ln_w, const Tensor& ln_b, const Tensor& cqw, const Tensor& cqb,
+                               const Tensor& ckw, const Tensor& ckb, const Tensor& idx, const LayerDims& l) {
     Dims m;
     m.d = l.d;
     m.B = l.B, m.H = l.H, m.T = l.T, m.F = l.F;
@@ -624,7 +625,10 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     const bool gated = l.g >= 0, bf = m.dt == at::kBFloat16;
     const Tensor x2 = x.reshape({l.M, l.C}).contiguous();
     const Tensor lr2 = lrw.reshape({l.H, l.C});  // weights stacked in the order of the columns
-    std::vector<Tensor> rows{q, k, v, lr2};
+    std::vector<Tensor> rows{q};
+    if (!l.taps) rows.push_back(k);
+    rows.push_back(v);
+    rows.push_back(lr2);
     if (l.N0 > l.lr + l.H) rows.push_back(at::zeros({l.N0 - l.lr - l.H, l.C}, m.opt()));
     if (gated) rows.push_back(g);
     const Tensor wcat = at::cat(rows, 0);
@@ -636,16 +640,18 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     s[3] = at::empty({l.B, l.H, l.T}, m.opt());
     const void* const ip = bf ? idx.const_data_ptr() : nullptr;
     const void* const lp = bf ? learnable.const_data_ptr() : nullptr;
-    Tensor gate;
+    Tensor gate, proj = at::mm(x2, wcat.narrow(0, 0, l.N0).t());
     {
-      const Tensor proj = at::mm(x2, wcat.narrow(0, 0, l.N0).t());
       const uint8_t* const p = static_cast<const uint8_t*>(proj.const_data_ptr());
       const int64_t e = proj.element_size();
-      must(ttt_internal_layer_prologue(&l.d, p, p + e * l.C, p + e * 2 * l.C, l.N0, p + e * l.lr, l.N0, lrb.const_data_ptr(), nullptr,
-                                       nullptr, nullptr, nullptr, 0, (int)l.start, (int)l.rope, l.theta, l.base_lr, ip, lp,
-                                       bf ? te16.data_ptr() : nullptr, s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(),
-                                       s[3].data_ptr(), (int)l.T, st));
+      const bool cv = l.taps != 0;
+      must(ttt_internal_layer_prologue(&l.d, p, p + (cv ? 0 : e * l.C), p + e * l.v, l.N0, p + e * l.lr, l.N0, lrb.const_data_ptr(),
+                                       cv ? cqw.const_data_ptr() : nullptr, cv ? cqb.const_data_ptr() : nullptr,
+                                       cv ? ckw.const_data_ptr() : nullptr, cv ? ckb.const_data_ptr() : nullptr, (int)l.taps,
+                                       (int)l.start, (int)l.rope, l.theta, l.base_lr, ip, lp, bf ? te16.data_ptr() : nullptr,
+                                       s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(), s[3].data_ptr(), (int)l.T, st));
     }
+    if (!l.taps) proj = Tensor();  // (the convolutions' gradient reads it)
     if (gated) gate = at::mm(x2, wcat.narrow(0, l.g, l.C).t());
     LinIn in{{s[0], s[1], s[2], w0, b0, te16, s[3], ln_w, ln_b}};
     LinOut lo;
@@ -654,7 +660,7 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     must(ttt_layer_epilogue(&l.d, lo.out.const_data_ptr(), gated ? gate.const_data_ptr() : nullptr, gated ? l.C : 0,
                             post_w.const_data_ptr(), post_b.const_data_ptr(), 1e-6f, y.data_ptr(), st));
     const Tensor out = at::mm(y, o.t()).view({l.B, l.T, l.C});
-    ctx->save_for_backward({x, wcat, te, lo.out, gate, post_w, post_b, y, o});
+    ctx->save_for_backward({x, wcat, te, lo.out, gate, post_w, post_b, y, o, proj, cqw, ckw});
     // kept as plain references, as the inner loop's own node keeps what it saves
     ctx->saved_data["t"] = std::vector<Tensor>{s[0], s[1], s[2], w0, b0, te16, s[3], ln_w, ln_b, lo.wck, lo.bck};
     ctx->saved_data["l"] = c10::IValue(std::string(reinterpret_cast<const char*>(&l), sizeof(l)));
@@ -683,7 +689,7 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
       if (rc != TTT_OK) throw_error(rc);
     };
     const Tensor go = (go_[0].defined() ? go_[0] : at::zeros_like(x)).reshape({l.M, l.C}).contiguous();
-    variable_list r(17);  // x q k v g lrw lrb learnable post_w post_b o w0 b0 ln_w ln_b idx dims
+    variable_list r(21);  // x q k v g lrw lrb learnable post_w post_b o w0 b0 ln_w ln_b, four of the convolutions, idx dims
     if (ctx->needs_input_grad(10)) r[10] = at::mm(go.t(), y);
     const Tensor dy = at::mm(go, o);
     // post norm and gate: the gate's gradient goes to its columns of the projections' gradient
@@ -711,15 +717,49 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     r[12] = gr[4];
     r[13] = gr[7];
     r[14] = gr[8];
-    must(ttt_layer_prologue_backward(&l.d, gr[0].const_data_ptr(), gr[1].const_data_ptr(), gr[2].const_data_ptr(),
-                                     gr[6].const_data_ptr(), t[6].const_data_ptr(), (int)l.start, (int)l.rope, l.theta, l.base_lr,
-                                     dp, dp + e * l.C, dp + e * 2 * l.C, l.N, dp + e * l.lr, l.N, (int)(l.N0 - l.lr), st));
+    auto prologue_backward = [&](void* dq, void* dk, void* dv, int64_t ld) {
+      must(ttt_layer_prologue_backward(&l.d, gr[0].const_data_ptr(), gr[1].const_data_ptr(), gr[2].const_data_ptr(),
+                                       gr[6].const_data_ptr(), t[6].const_data_ptr(), (int)l.start, (int)l.rope, l.theta, l.base_lr,
+                                       dq, dk, dv, ld, dp + e * l.lr, l.N, (int)(l.N0 - l.lr), st));
+    };
+    if (!l.taps) {
+      prologue_backward(dp, dp + e * l.C, dp + e * l.v, l.N);
+    } else {
+      // through the two convolutions to their shared projection
+      const Tensor &proj = sv[9], d4 = at::empty({4, l.M, l.C}, m.opt());  // of q, k, v, and of the shared projection
+      uint8_t* const d0 = static_cast<uint8_t*>(d4.data_ptr());
+      const int64_t one = e * l.M * l.C;
+      prologue_backward(d0, d0 + one, d0 + 2 * one, l.C);
+      const Tensor gp = at::empty({2, 5, l.C}, m.opt(at::kFloat));  // four taps and the bias, of each
+      auto taps4 = [&](const Tensor& w) {  // [C][4], aligned to the end
+        const Tensor w2 = w.reshape({l.C, l.taps});
+        if (l.taps == 4) return w2;
+        Tensor w4 = at::zeros({l.C, 4}, w2.options());
+        w4.narrow(1, 4 - l.taps, l.taps).copy_(w2);
+        return w4;
+      };
+      const Tensor wq4 = taps4(sv[10]), wk4 = taps4(sv[11]);
+      const size_t wsb = ttt_layer_qk_conv_backward_workspace_bytes(&l.d);
+      const Tensor ws = at::empty({(int64_t)wsb}, m.opt(at::kByte));
+      must(ttt_layer_qk_conv_backward(&l.d, d0, d0 + one, proj.const_data_ptr(), l.N0, wq4.const_data_ptr(), wk4.const_data_ptr(),
+                                      d0 + 3 * one, static_cast<float*>(gp.data_ptr()), static_cast<float*>(gp.data_ptr()) + 5 * l.C,
+                                      ws.data_ptr(), wsb, st));
+      dproj.narrow(1, 0, l.C).copy_(d4.select(0, 3));
+      dproj.narrow(1, l.v, l.C).copy_(d4.select(0, 2));
+      const Tensor gpt = gp.to(m.dt);
+      for (int i = 0; i < 2; ++i) {
+        r[15 + 2 * i] = gpt.select(0, i).narrow(0, 4 - l.taps, l.taps).t().reshape(sv[10 + i].sizes());
+        r[16 + 2 * i] = gpt.select(0, i).select(0, 4);
+      }
+    }
     if (ctx->needs_input_grad(0)) r[0] = at::mm(dproj, wcat).view(x.sizes());
     bool weights = false;
     for (int i = 1; i <= 5; ++i) weights = weights || ctx->needs_input_grad(i);
     if (weights) {
       const Tensor dw = at::mm(dproj.t(), x.reshape({l.M, l.C}));
-      for (int i = 0; i < 3; ++i) r[1 + i] = dw.narrow(0, i * l.C, l.C);
+      r[1] = dw.narrow(0, 0, l.C);
+      if (!l.taps) r[2] = dw.narrow(0, l.C, l.C);
+      r[3] = dw.narrow(0, l.v, l.C);
       if (gated) r[4] = dw.narrow(0, l.g, l.C);
       r[5] = dw.narrow(0, l.lr, l.H).view(shapes.get(0).toIntVector());
     }
@@ -732,23 +772,25 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     return r;
   }
 };
-// layer_train(x, q_proj, k_proj, v_proj, g_proj | None, lr weight, lr bias, learnable_token_idx, post norm weight, bias, o_proj,
-//             state weight, state bias, ln weight, ln bias, token_idx, heads, mini_batch, rope_mode, rope_theta, base_lr,
+// layer_train(x, q_proj, k_proj | None, v_proj, g_proj | None, lr weight, lr bias, learnable_token_idx, post norm weight, bias,
+//             o_proj, state weight, state bias, ln weight, ln bias, conv q weight, bias, conv k weight, bias (with k_proj: four
+//             None), token_idx, heads, mini_batch, rope_mode, rope_theta, base_lr,
 //             checkpoint interval, eps_scaled, start_idx) -> (y, state weight, state bias), recorded for autograd | None
 PyObject* py_layer_train(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (!arity(n, 24)) return nullptr;
-  Tensor t[16];
-  for (int i = 0; i < 16; ++i) {
-    if (i == 4 && args[i] == Py_None) continue;
+  if (!arity(n, 28)) return nullptr;
+  Tensor t[20];
+  const bool shared = args[2] == Py_None;
+  for (int i = 0; i < 20; ++i) {
+    if (args[i] == Py_None && (i == 4 || (shared ? i == 2 : i >= 15 && i < 19))) continue;
     NONE_IF(!THPVariable_Check(args[i]));
     t[i] = THPVariable_Unpack(args[i]);
     NONE_IF(t[i].unsafeGetTensorImpl()->is_python_dispatch());
   }
   LayerDims l;
-  l.H = as_int(args[16]), l.mb = as_int(args[17]), l.rope = as_int(args[18]);
-  l.theta = (float)PyFloat_AsDouble(args[19]), l.base_lr = (float)PyFloat_AsDouble(args[20]);
-  l.K = as_int(args[21]), l.eps_scaled = as_int(args[22]), l.start = as_int(args[23]);
+  l.H = as_int(args[20]), l.mb = as_int(args[21]), l.rope = as_int(args[22]);
+  l.theta = (float)PyFloat_AsDouble(args[23]), l.base_lr = (float)PyFloat_AsDouble(args[24]);
+  l.K = as_int(args[25]), l.eps_scaled = as_int(args[26]), l.start = as_int(args[27]);
   if (PyErr_Occurred()) return nullptr;
   const Tensor& x = t[0];
   NONE_IF(at::autocast::is_autocast_enabled(at::kCUDA));
@@ -759,27 +801,37 @@ PyObject* py_layer_train(PyObject*, PyObject* const* args, Py_ssize_t n) {
   l.B = x.size(0), l.T = x.size(1), l.C = x.size(2), l.F = l.C / l.H, l.M = l.B * l.T;
   NONE_IF(l.M <= 0 || l.M > INT32_MAX || l.F * l.H != l.C || (l.F != 64 && l.F != 32) || l.C > 2048 || l.H > 64 || l.C % 8 != 0);
   NONE_IF((l.mb != 16 && l.mb != 8) || l.T % l.mb != 0 || (l.F == 32 && l.H % 2 != 0));
-  for (int i : {1, 2, 3, 10}) NONE_IF(!is(t[i], dt, dev, {l.C, l.C}));
+  for (int i : {1, 2, 3, 10}) NONE_IF(t[i].defined() && !is(t[i], dt, dev, {l.C, l.C}));
   const bool gated = t[4].defined();
   NONE_IF(gated && !is(t[4], dt, dev, {l.C, l.C}));
   NONE_IF(t[5].numel() != l.H * l.C || t[5].size(0) != l.H || t[5].scalar_type() != dt || t[5].device() != dev || !t[5].is_contiguous());
   NONE_IF(t[6].numel() != l.H || t[6].scalar_type() != dt || t[6].device() != dev || !t[6].is_contiguous());
-  for (int i : {7, 15}) NONE_IF(!is(t[i], dt, dev, {l.mb}));
+  for (int i : {7, 19}) NONE_IF(!is(t[i], dt, dev, {l.mb}));
   for (int i : {8, 9}) NONE_IF(!is(t[i], dt, dev, {l.C}));
   NONE_IF(!is(t[11], dt, dev, {l.B, l.H, l.F, l.F}) || !is(t[12], dt, dev, {l.B, l.H, l.F}));
   for (int i : {13, 14}) NONE_IF(!is(t[i], dt, dev, {l.H, l.F}));
-  for (int i = 0; i < 16; ++i) NONE_IF(t[i].defined() && !on_16_bytes(t[i]));
+  l.taps = 0;
+  if (shared) {
+    for (int i = 15; i < 19; ++i)
+      NONE_IF(t[i].dim() < 1 || t[i].size(0) != l.C || t[i].scalar_type() != dt || t[i].device() != dev || !t[i].is_contiguous());
+    l.taps = t[15].numel() / l.C;
+    NONE_IF(l.taps < 1 || l.taps > 4 || t[17].numel() != t[15].numel() || t[16].numel() != l.C || t[18].numel() != l.C);
+  }
+  for (int i = 0; i < 20; ++i) NONE_IF(t[i].defined() && !on_16_bytes(t[i]));
   // (those run projections and prologue in one launch: the composition)
-  NONE_IF(dt == at::kBFloat16 && l.T % 128 == 0 && l.F == 64 && l.rope != 2);
-  l.lr = 3 * l.C;
+  NONE_IF(!shared && dt == at::kBFloat16 && l.T % 128 == 0 && l.F == 64 && l.rope != 2);
+  l.v = shared ? l.C : 2 * l.C;
+  l.lr = l.v + l.C;
   l.N0 = (l.lr + l.H + 7) & ~(int64_t)7;
   l.g = gated ? l.N0 : -1;
   l.N = l.N0 + (gated ? l.C : 0);
   l.d = ttt_dims{(int32_t)l.B, (int32_t)l.H, (int32_t)l.T, (int32_t)l.F, (int32_t)l.mb, (int32_t)l.K, (float)l.eps_scaled * 1e-9f,
                  dt == at::kBFloat16 ? TTT_BF16 : TTT_F32};
   NONE_IF(ttt_linear_num_checkpoints(&l.d) < 0);
-  if (!gated) t[4] = at::empty({0});  // (a node's arguments are defined tensors)
-  return wrap(LayerFn::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11], t[12], t[13], t[14], t[15], l));
+  for (Tensor& u : t)
+    if (!u.defined()) u = at::empty({0});  // (a node's arguments are defined tensors)
+  return wrap(LayerFn::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11], t[12], t[13], t[14], t[15],
+                             t[16], t[17], t[18], t[19], l));
   END_HANDLE_TH_ERRORS
 }
 

@@ -577,16 +577,19 @@ class TTT(torch.nn.Module):
 def _train_native(self, x, inner, state, start_idx):
     """The whole layer as one native autograd node (None: not a case it takes, nothing was done)."""
     c = self.config
-    if c.share_qk or type(inner) is not FusedTileMultiTTTLinear or not x.is_cuda:
+    if type(inner) is not FusedTileMultiTTTLinear or not x.is_cuda:
         return None
     i = inner._modules["inner"]
     if type(i) is not TTTLinear or i.mini_batch_size != c.mini_batch_size:
         return None
     P, I = self._parameters.get, i._parameters.get
+    if (not c.share_qk and P("k_proj") is None) or (c.use_gate and P("g_proj") is None):
+        return None  # (a weight that is computed at every access)
+    conv = (P("q_conv_weight"), P("q_conv_bias"), P("k_conv_weight"), P("k_conv_bias")) if c.share_qk else _NO_CONV
     r = _lib.host().layer_train(
-        x, P("q_proj"), P("k_proj"), P("v_proj"), P("g_proj") if c.use_gate else None, P("learnable_ttt_lr_weight"),
+        x, P("q_proj"), None if c.share_qk else P("k_proj"), P("v_proj"), P("g_proj") if c.use_gate else None, P("learnable_ttt_lr_weight"),
         P("learnable_ttt_lr_bias"), P("learnable_token_idx"), P("post_norm_weight"), P("post_norm_bias"), P("o_proj"),
-        state.weight, state.bias, I("ln_weight"), I("ln_bias"), self._buffers.get("token_idx"), c.num_heads,
+        state.weight, state.bias, I("ln_weight"), I("ln_bias"), *conv, self._buffers.get("token_idx"), c.num_heads,
         c.mini_batch_size, _POS[c.pos_encoding], c.rope_theta, c.base_lr, i.checkpoint_interval, _eps_scaled(i.epsilon),
         start_idx)
     if r is None:
