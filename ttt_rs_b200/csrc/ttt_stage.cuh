@@ -144,8 +144,8 @@ __device__ __forceinline__ void ln_row_stats(const F2 (&z)[2][2], Xch4* xch, int
     int f2_ = 0;
     xch_rows2<SEG, false, BAR>(&xch[xsel], L, q2[0], 0.f, q2[1], 0.f, a0, a1, f2_);
     xsel ^= 1;
-    rstd[0] = __frsqrt_rn(a0.x * INV + eps);
-    rstd[1] = __frsqrt_rn(a1.x * INV + eps);
+    rstd[0] = 1.0f / sqrtf(a0.x * INV + eps);
+    rstd[1] = 1.0f / sqrtf(a1.x * INV + eps);
   }
 }
 
