@@ -17,7 +17,7 @@ CSRC = PKG / "csrc"
 LIB = PKG / "libttt_b200.so"
 PROBE_SRC = CSRC / "probe_chain_latency.cu"      # stand-alone measurement program (bench.py --workload chain-latency)
 PROBE_BIN = PKG / "build" / "probe_chain_latency"
-SOURCES = ["ttt_abi.cu", "ttt_linear_fwd.cu", "ttt_linear_fwd_roles.cu", "ttt_linear_bwd.cu", "ttt_mlp_fwd.cu", "ttt_layer.cu", "ttt_layer_small.cu", "ttt_linear_partial.cu", "ttt_mlp_bwd.cu", "ttt_gemm.cu"]
+SOURCES = ["ttt_abi.cu", "ttt_linear_fwd.cu", "ttt_linear_fwd_roles.cu", "ttt_linear_bwd.cu", "ttt_linear_bwd_f32.cu", "ttt_mlp_fwd.cu", "ttt_layer.cu", "ttt_layer_small.cu", "ttt_linear_partial.cu", "ttt_mlp_bwd.cu", "ttt_gemm.cu"]
 HOST_SRC = CSRC / "ttt_host.cpp"                 # native host path of the Python operator, linked against LIB
 HOST_LIB = PKG / "_host.so"
 HOST_TAG = PKG / "build" / "_host.tag"           # what HOST_LIB was built against

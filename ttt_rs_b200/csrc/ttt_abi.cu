@@ -579,6 +579,9 @@ int ttt_internal_linear_backward(const ttt_dims* d, const void* xq, const void* 
   p.d_w = grad_weight;
   p.d_b = grad_bias;
   p.d_lr = grad_ttt_lr_eta;
+  p.d_q = grad_xq;
+  p.d_k = grad_xk;
+  p.d_v = grad_xv;
   p.part_ln = ws + wl.off_ln;
   p.part_te = ws + wl.off_te;
   p.part_w = (outer_grad_packed != nullptr) ? ws + wl.off_w : nullptr;

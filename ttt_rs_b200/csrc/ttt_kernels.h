@@ -72,6 +72,7 @@ struct LinBwdParams {
   void* d_w;        // [B,H,F,F] element type T (per batch element), nullable
   void* d_b;        // [B,H,F], nullable
   void* d_lr;       // [B,H,T]
+  void *d_q, *d_k, *d_v;  // [B,H,T,F]: what the tensor maps of the gradients cover
   int* sched;       // workspace: [0] next work item, [1 + stream] chunks of the stream finished so far (zeroed per launch)
   float* handoff;   // workspace: [B*H][2*F*F + F] W^T, dW^T (register layout) and db handed from chunk to chunk
   int CH, NCH, nstreams;  // stages per chunk, chunks per stream, B*H (the launcher sets CH = NS, NCH = 1, sched = null
@@ -396,6 +397,7 @@ cudaError_t launch_linear_fwd_roles(int dtype, int seg, int mb, const CUtensorMa
 // maps: q, k, v, d_out, d_q, d_k, d_v, gp
 cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps, LinBwdParams& p, int nstreams,
                               cudaStream_t st);
+cudaError_t launch_linear_bwd_f32(int seg, int mb, const CUtensorMap* maps, LinBwdParams& p, int nstreams, cudaStream_t st);
 cudaError_t launch_linear_bwd_reduce(const ReduceParams& p, cudaStream_t st);
 
 }  // namespace ttt

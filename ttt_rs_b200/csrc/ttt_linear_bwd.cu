@@ -1,5 +1,5 @@
-// Fused TTT-Linear backward scan for sm_100a: one 4-warp CTA per (batch, head) stream walks the mini-batches in
-// reverse.
+// Fused TTT-Linear backward scan for sm_100a, bf16: one 4-warp CTA per (batch, head) stream walks the mini-batches in
+// reverse (float32: ttt_linear_bwd_f32.cu).
 //
 // What it computes is the reference's multi-stage backward kernel
 // (rust/fused/src/linear_fused_tile/backward/kernel.rs:254-429 with the stage body backward/stage.rs:42-1006 and the
@@ -32,9 +32,9 @@
 
 namespace ttt {
 
-template <typename T, int SEG>
+template <int SEG>
 struct BwdSmem {
-  using TF = TileFmt<T>;
+  using TF = TileFmt<__nv_bfloat16>;
   static constexpr int NP = TF::NP;
   static constexpr int NSLOT = 2;
   static constexpr uint32_t PLANES = NP * TILE_BF16_BYTES;  // one operand tile
@@ -61,8 +61,8 @@ struct BwdSmem {
 #define TTT_BWD_MINB_BF16 2  // resident blocks per SM the bf16 kernel is compiled for
 #endif
 
-template <typename T, int SEG, int MB>
-__global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 : 1))
+template <int SEG, int MB>
+__global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                           const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v,
@@ -71,8 +71,9 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
                           const __grid_constant__ CUtensorMap tm_dk,
                           const __grid_constant__ CUtensorMap tm_dv,
                           const __grid_constant__ CUtensorMap tm_g, const LinBwdParams p) {
+  using T = __nv_bfloat16;
   using TF = TileFmt<T>;
-  using SM = BwdSmem<T, SEG>;
+  using SM = BwdSmem<SEG>;
   constexpr int NP = TF::NP;
   constexpr uint32_t PL = TILE_BF16_BYTES;  // plane stride
   constexpr float INV_F = 1.f / SEG;        // features per head (LayerNorm row length)
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
   // Everything stage s needs, into slot n % NSLOT, and the output tiles of a stage from their staging buffers.  Issuing a copy
   // takes its thread some 100 cycles, on the way of the stage's next barrier whichever warp does it: they are spread over
   // the four warps, and a stage's stores share the next stage's first barrier (bf16, 64 stages: 146 -> 134 us at 12 streams,
-  // 291 -> 278 us at 384; float32: 453 -> 442 us at 96).  Pairs of 32-wide heads come as two 64-byte-swizzled boxes per tile
+  // 291 -> 278 us at 384).  Pairs of 32-wide heads come as two 64-byte-swizzled boxes per tile
   // (gathered by the threads they cost 162 us at 72 heads, 150 us this way).
   auto issue_loads = [&](int n, int s) {
     const int slot = n % SM::NSLOT;
@@ -364,19 +365,6 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
         if (s > s_lo) issue_loads(n + 1, s - 1);
       }
     };
-    if constexpr (NP == 3) {
-      if (!fail) {
-        split_tile_f32(tk, tid);
-        split_tile_f32(tq, tid);
-        split_tile_f32(tg, tid);
-      }
-      fail = __syncthreads_or(fail);
-      if (fail) {
-        failed = true;
-        if (tid == 0) report_timeout(p.status, 11, s);
-        break;
-      }
-    }
     // (SEG = 32: the pair's second head has its 16 values right after the first head's)
     const float lr_row[2] = {ld_as_float<T>(gsl + SM::OFF_LR, (SEG == 32 ? hsel * CS : 0) + g),
                              ld_as_float<T>(gsl + SM::OFF_LR, (SEG == 32 ? hsel * CS : 0) + g + 8)};
@@ -529,19 +517,16 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) pp[nt][i] = gl[nt][i] = dk[nt][i] = dgp[nt][i] = 0.f;
-    // (bf16: the B fragments of W^T read here serve step 13 as well -- there are registers for them now that the state
+    // (the B fragments of W^T read here serve step 13 as well -- there are registers for them now that the state
     // is parked in tensor memory)
-    constexpr bool KEEP_W = (NP == 1);
-    Pk<NP> bw_keep[KEEP_W ? 4 : 1][4];
+    Pk<NP> bw_keep[4][4];
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       Pk<NP> adz[4], bwt[4], ags[4], bdw[4];
       ldsm_np<NP>(adz, tDZ + lane_off_A(lane, 16 * ks), PL, false);
       ldsm_np<NP>(bwt, tW + ks * SM::PLANES + lane_off_B_kn(lane, nb), PL, true);
-      if constexpr (KEEP_W) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) bw_keep[ks][i] = bwt[i];
-      }
+      for (int i = 0; i < 4; ++i) bw_keep[ks][i] = bwt[i];
       ldsm_np<NP>(ags, pg + lane_off_A(lane, 16 * ks), PL, false);
       ldsm_np<NP>(bdw, tDW + ks * SM::PLANES + lane_off_B_kn(lane, nb), PL, true);
       if (SEG == 64 || (ks >> 1) == hsel) {
@@ -679,14 +664,9 @@ __global__ void __launch_bounds__(NTHREADS, (sizeof(T) == 2 ? TTT_BWD_MINB_BF16 
     // ---- 13. dk += dZ1 W^T ; dW^T += dZ1^T K ; bias gradient
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
-      Pk<NP> adz1[4], bwt[4];
+      Pk<NP> adz1[4];
+      const Pk<NP>(&bwt)[4] = bw_keep[ks];
       ldsm_np<NP>(adz1, tDZ1 + lane_off_A(lane, 16 * ks), PL, false);
-      if constexpr (KEEP_W) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) bwt[i] = bw_keep[ks][i];
-      } else {
-        ldsm_np<NP>(bwt, tW + ks * SM::PLANES + lane_off_B_kn(lane, nb), PL, true);
-      }
       const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
       mma_np2<NP>(dk[0], adz1, b0, dk[1], adz1, b1);
     }
@@ -891,11 +871,11 @@ __global__ void ttt_linear_bwd_fold_kernel(const ReduceParams p) {
   if (lane == 0) p.packed[(size_t)p.H * p.F * p.F + 3 * p.H * p.F + c] = acc;
 }
 
-template <typename T, int SEG, int MB>
+template <int SEG, int MB>
 static cudaError_t launch_bwd_t(const CUtensorMap* m, LinBwdParams& p, int nstreams,
                                 cudaStream_t st) {
-  using SM = BwdSmem<T, SEG>;
-  auto kfn = ttt_linear_bwd_kernel<T, SEG, MB>;
+  using SM = BwdSmem<SEG>;
+  auto kfn = ttt_linear_bwd_kernel<SEG, MB>;
   // Persistent grid: as many blocks as fit on the device at once, never more than there are work items.  The count
   // comes from the kernel's registers and shared memory: the occupancy calculator answers one block per SM for any
   // kernel that allocates tensor memory, whatever it allocates (which also rules out a cooperative launch of more).
@@ -937,21 +917,12 @@ static cudaError_t launch_bwd_t(const CUtensorMap* m, LinBwdParams& p, int nstre
   return cudaGetLastError();
 }
 
-template <typename T, int SEG>
-static cudaError_t launch_bwd_mb(int mb, const CUtensorMap* m, LinBwdParams& p,
-                                 int nstreams, cudaStream_t st) {
-  return mb == 8 ? launch_bwd_t<T, SEG, 8>(m, p, nstreams, st) : launch_bwd_t<T, SEG, 16>(m, p, nstreams, st);
-}
-
 // mb: tokens per mini-batch, 16 or 8 (the maps' boxes then have 8 rows)
 cudaError_t launch_linear_bwd(int dtype, int seg, int mb, const CUtensorMap* maps,
                               LinBwdParams& p, int nstreams, cudaStream_t st) {
-  if (seg == 32) {
-    if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 32>(mb, maps, p, nstreams, st);
-    return launch_bwd_mb<float, 32>(mb, maps, p, nstreams, st);
-  }
-  if (dtype == 1) return launch_bwd_mb<__nv_bfloat16, 64>(mb, maps, p, nstreams, st);
-  return launch_bwd_mb<float, 64>(mb, maps, p, nstreams, st);
+  if (dtype != 1) return launch_linear_bwd_f32(seg, mb, maps, p, nstreams, st);
+  if (seg == 32) return mb == 8 ? launch_bwd_t<32, 8>(maps, p, nstreams, st) : launch_bwd_t<32, 16>(maps, p, nstreams, st);
+  return mb == 8 ? launch_bwd_t<64, 8>(maps, p, nstreams, st) : launch_bwd_t<64, 16>(maps, p, nstreams, st);
 }
 
 cudaError_t launch_linear_bwd_reduce(const ReduceParams& p, cudaStream_t st) {

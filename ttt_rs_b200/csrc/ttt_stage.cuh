@@ -42,6 +42,20 @@ __device__ __forceinline__ int group_sync_or(int v) {
   }
 }
 
+// For blocks whose groups of warps have roles of their own and meet on mbarriers.
+__device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {  // one arrival for the warp's accesses before it
+  __syncwarp();
+  if (elect_one()) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_u4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 ld_u4(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+
 // Exchange of up to four per-row partial sums across the four warps of the CTA.
 struct __align__(16) Xch4 {
   float4 v[CS][5];  // [row][warp] with the row padded to 80 bytes: the 8 rows a warp reads fall in distinct banks
@@ -51,18 +65,19 @@ struct __align__(16) Xch4 {
 // (SEG = 64) or the warp pair that holds this thread's 32-wide head (SEG = 32: warps 0,1 / 2,3).
 // `flag` is OR-reduced over the CTA by the same barrier (used to spread a timed-out wait); with FLAG = false the
 // barrier is a plain one and `flag` is left alone (a barrier that reduces costs more than one that does not).
-template <int SEG = 64, bool FLAG = true>
+// (W4 = false: the fourth value is not used.)
+template <int SEG = 64, bool FLAG = true, int BAR = 0, bool W4 = true>
 __device__ __forceinline__ void xch_rows(Xch4* xb, const Lane& L, const float4 a0, const float4 a1, float4& o0,
                                          float4& o1, int& flag) {
   float4 p0, p1;
-  p0.x = quad_sum(a0.x); p0.y = quad_sum(a0.y); p0.z = quad_sum(a0.z); p0.w = quad_sum(a0.w);
-  p1.x = quad_sum(a1.x); p1.y = quad_sum(a1.y); p1.z = quad_sum(a1.z); p1.w = quad_sum(a1.w);
+  p0.x = quad_sum(a0.x); p0.y = quad_sum(a0.y); p0.z = quad_sum(a0.z); p0.w = W4 ? quad_sum(a0.w) : 0.f;
+  p1.x = quad_sum(a1.x); p1.y = quad_sum(a1.y); p1.z = quad_sum(a1.z); p1.w = W4 ? quad_sum(a1.w) : 0.f;
   if (L.t == 0) {
     xb->v[L.g][L.warp] = p0;
     xb->v[L.g + 8][L.warp] = p1;
   }
-  if constexpr (FLAG) flag = __syncthreads_or(flag);
-  else __syncthreads();
+  if constexpr (FLAG) flag = group_sync_or<BAR>(flag);
+  else group_sync<BAR>();
   const float4* r0 = &xb->v[L.g][0];
   const float4* r1 = &xb->v[L.g + 8][0];
   if constexpr (SEG == 64) {
