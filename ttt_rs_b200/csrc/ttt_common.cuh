@@ -138,6 +138,10 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
 }
+// the counterpart of ldsm_x4: the same lanes' addresses, the same fragments
+__device__ __forceinline__ void stsm_x4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // Transpose an 8x8 matrix of 16-bit values held one register per lane across the warp.
 __device__ __forceinline__ uint32_t movm_t(uint32_t a) {
   uint32_t d;

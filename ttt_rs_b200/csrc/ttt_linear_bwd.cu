@@ -389,13 +389,14 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     }
     // ---- 2. operand copies of W_s^T and dW^T (this warp's 16 rows) for the products that contract over n
 #pragma unroll
-    for (int kt = 0; kt < 8; ++kt)
-#pragma unroll
-      for (int rn = 0; rn < 2; ++rn) {
-        st_pair_planes<NP>(tW + warp * SM::PLANES, g + 8 * rn, 8 * kt + 2 * t, wt[kt][2 * rn] * wscale,
-                           wt[kt][2 * rn + 1] * wscale);
-        st_pair_planes<NP>(tDW + warp * SM::PLANES, g + 8 * rn, 8 * kt + 2 * t, dwt[kt][2 * rn], dwt[kt][2 * rn + 1]);
-      }
+    for (int ks = 0; ks < 4; ++ks) {
+      const float(&a)[4] = wt[2 * ks], (&b)[4] = wt[2 * ks + 1], (&c)[4] = dwt[2 * ks], (&d)[4] = dwt[2 * ks + 1];
+      const uint32_t o = warp * SM::PLANES + lane_off_A(lane, 16 * ks);
+      stsm_np<NP>(tW + o, split_pack<NP>(a[0] * wscale, a[1] * wscale), split_pack<NP>(a[2] * wscale, a[3] * wscale),
+                  split_pack<NP>(b[0] * wscale, b[1] * wscale), split_pack<NP>(b[2] * wscale, b[3] * wscale));
+      stsm_np<NP>(tDW + o, split_pack<NP>(c[0], c[1]), split_pack<NP>(c[2], c[3]), split_pack<NP>(d[0], d[1]),
+                  split_pack<NP>(d[2], d[3]));
+    }
     // ---- 3. Z1 = K W + b, Zq = Q W + b, KdW = K dW, Attn = Q K^T
     float z1[2][4], zq[2][4], kdw[2][4], at[2][4];
 #pragma unroll
@@ -468,13 +469,14 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     F2 dzb[2][2], dzsum[2];
     float dq[2][4];
     {
-      F2 xz[2][2], tt[2][2];
+      F2 xz[2][2], tt[2][2], dd[2][2];
+      ld_slab<T, SEG>(tdo, lane, nb, dd);
       F2 p1[2] = {f2(0.f), f2(0.f)}, p2[2] = {f2(0.f), f2(0.f)};
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const F2 d = ld_io<T, SEG>(tdo, g + 8 * r, nb + 8 * nt + 2 * t);
+          const F2 d = dd[nt][r];
           const F2 x = f2mul(f2sub(pr(zq[nt], r), f2(mean2[r])), f2(rstd2[r]));
           xz[nt][r] = x;
           dq[nt][2 * r] = d.x;
@@ -505,10 +507,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
       dzsum[1] = f2add(dzb[1][0], dzb[1][1]);
     }
     // ---- 8. dZbar to shared memory as an operand tile; the barrier also publishes tW / tDW
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) st_pair_planes<NP>(tDZ, g + 8 * r, nb + 8 * nt + 2 * t, dzb[nt][r].x, dzb[nt][r].y);
+    st_slab<T, 64>(tDZ, lane, nb, dzb);
     __syncthreads();
 
     // ---- 9. products that need dZbar
@@ -581,11 +580,13 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     float s1t[2], s2t[2];
     {
       F2 p1[2] = {f2(0.f), f2(0.f)}, p2[2] = {f2(0.f), f2(0.f)}, pdl[2] = {f2(0.f), f2(0.f)}, prt[2] = {f2(0.f), f2(0.f)};
+      F2 k[2][2];
+      ld_slab<T, SEG>(tk, lane, nb, k);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const F2 kk = ld_io<T, SEG>(tk, g + 8 * r, nb + 8 * nt + 2 * t);
+          const F2 kk = k[nt][r];
           const F2 glp = pr(gl[nt], r);
           // dL/dGp = -M'^T dZbar - te15 (K dW + db)
           const F2 dg = f2fma(f2add(pr(kdw[nt], r), dbias[nt]), f2(-te15), pr(dgp[nt], r));
@@ -655,10 +656,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
           dz1[nt][r] = f2fma(f2sub(dxh[nt][r], f2(D[r])), f2(rstd1[r]), f2mul(xh[nt][r], f2(S[r])));
     }
     // ---- 12. dZ1 to shared memory as an operand tile
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) st_pair_planes<NP>(tDZ1, g + 8 * r, nb + 8 * nt + 2 * t, dz1[nt][r].x, dz1[nt][r].y);
+    st_slab<T, 64>(tDZ1, lane, nb, dz1);
     if (elect_one()) bulk_wait_read<0>();  // the previous stage's output tiles have left the staging buffers
     __syncthreads();
     // ---- 13. dk += dZ1 W^T ; dW^T += dZ1^T K ; bias gradient
@@ -706,16 +704,15 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     // ---- 14. outputs: dq = d_out + ..., dk = -dT + ..., dv = dT
     {
       const uint32_t so_q = base + SM::OFF_OUT, so_k = so_q + TF::RAW_BYTES, so_v = so_k + TF::RAW_BYTES;
+      F2 dqq[2][2], dkk[2][2];
+      slab_pairs(dq, dqq);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const int row = g + 8 * r, col = nb + 8 * nt + 2 * t;
-          const F2 dkk = f2sub(pr(dk[nt], r), dT[nt][r]);
-          st_io<T, SEG>(so_q, row, col, dq[nt][2 * r], dq[nt][2 * r + 1]);
-          st_io<T, SEG>(so_k, row, col, dkk.x, dkk.y);
-          st_io<T, SEG>(so_v, row, col, dT[nt][r].x, dT[nt][r].y);
-        }
+        for (int r = 0; r < 2; ++r) dkk[nt][r] = f2sub(pr(dk[nt], r), dT[nt][r]);
+      st_slab<T, SEG>(so_q, lane, nb, dqq);
+      st_slab<T, SEG>(so_k, lane, nb, dkk);
+      st_slab<T, SEG>(so_v, lane, nb, dT);
       fence_proxy_async_smem();  // (stored behind the next stage's first barrier)
     }
   }

@@ -462,10 +462,8 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
       // ---- 5. the record: dZbar as an operand tile, W's copy, Z1, dGp' = -M'^T dZbar
       if (n >= NR && !mbar_wait_or_stop(b_rtaken + 8 * rb, ((n / NR) - 1) & 1, stop)) fail = 1;
       const uint32_t tDZ = rr + SM::R_DZ;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) st_pair_planes<NP>(tDZ, g + 8 * r, nb + 8 * nt + 2 * t, dzb[nt][r].x, dzb[nt][r].y);
+      stsm_np<NP>(tDZ + lane_off_A(lane, nb), split_pack<NP>(dzb[0][0].x, dzb[0][0].y), split_pack<NP>(dzb[0][1].x, dzb[0][1].y),
+                  split_pack<NP>(dzb[1][0].x, dzb[1][0].y), split_pack<NP>(dzb[1][1].x, dzb[1][1].y));
       __syncwarp();
       float dgp[2][4] = {};
       {
@@ -476,11 +474,12 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         mma_np2<NP>(dgp[0], amt, z0, dgp[1], amt, zz1);
       }
 #pragma unroll
-      for (int kt = 0; kt < 8; ++kt)
-#pragma unroll
-        for (int rn = 0; rn < 2; ++rn)
-          st_pair_planes<NP>(rr + SM::R_W + warp * SM::PLANES, g + 8 * rn, 8 * kt + 2 * t, wt[kt][2 * rn] * wscale,
-                             wt[kt][2 * rn + 1] * wscale);
+      for (int ks = 0; ks < 4; ++ks) {
+        const float(&a)[4] = wt[2 * ks], (&b)[4] = wt[2 * ks + 1];
+        stsm_np<NP>(rr + SM::R_W + warp * SM::PLANES + lane_off_A(lane, 16 * ks), split_pack<NP>(a[0] * wscale, a[1] * wscale),
+                    split_pack<NP>(a[2] * wscale, a[3] * wscale), split_pack<NP>(b[0] * wscale, b[1] * wscale),
+                    split_pack<NP>(b[2] * wscale, b[3] * wscale));
+      }
       {
         const F2 d0 = f2add(dzb[0][0], dzb[0][1]), d1 = f2add(dzb[1][0], dzb[1][1]);
         st_f4(rr + SM::R_SUM + tid * 16, d0.x, d0.y, d1.x, d1.y);
@@ -591,15 +590,7 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         if (ks == 0 && n >= ND && !mbar_wait_or_stop(b_dtaken + 8 * db, ((n / ND) - 1) & 1, stop)) fail = 1;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int rn = 0; rn < 2; ++rn)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const uint32_t a = rd + warp * SM::PLANES + off_bf16(g + 8 * rn, 16 * (ks + j) + 8 * e + 2 * t);
-#pragma unroll
-              for (int q = 0; q < NP; ++q)
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + q * PL), "r"(bd[j][rn][e].p[q]) : "memory");
-            }
+          stsm_np<NP>(rd + warp * SM::PLANES + lane_off_A(lane, 16 * (ks + j)), bd[j][0][0], bd[j][1][0], bd[j][0][1], bd[j][1][1]);
       }
       mbar_arrive_warp(b_dgiven + 8 * db);
       const float lr_row[2] = {ld_as_float<T>(gsl + SM::OFF_LR, (SEG == 32 ? hsel * CS : 0) + g),
@@ -715,14 +706,9 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         const Pk<NP> agt[4] = {gt[0][0], gt[1][0], gt[0][1], gt[1][1]};
         state_update_direct<NP, SEG>(dwt, agt, pk, lane, khalf);
         if (n >= NZ && !mbar_wait_or_stop(b_ztaken + 8 * zb, ((n / NZ) - 1) & 1, stop)) fail = 1;
+        stsm_np<NP>(rz + SM::Z_DZ1 + lane_off_A(lane, nb), pz[0][0], pz[0][1], pz[1][0], pz[1][1]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const uint32_t a = rz + SM::Z_DZ1 + off_bf16(g + 8 * r, nb + 8 * nt + 2 * t);
-#pragma unroll
-            for (int q = 0; q < NP; ++q) asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + q * PL), "r"(pz[nt][r].p[q]) : "memory");
-          }
           st_f4(rz + SM::Z_DT + (nt * NTHREADS + tid) * 16, dT[nt][0].x, dT[nt][0].y, dT[nt][1].x, dT[nt][1].y);
         }
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(rz + SM::Z_PS + tid * 4), "f"(pgb) : "memory");

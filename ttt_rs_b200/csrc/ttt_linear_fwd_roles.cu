@@ -311,15 +311,9 @@ __global__ void __launch_bounds__(ROLE_THREADS, 1)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const Pk<NP> pkd = split_pack<NP>(gp[nt][r].x, gp[nt][r].y);
-          if (save) {
-            if constexpr (NP == 1) {
-              asm volatile("st.shared.b32 [%0], %1;" ::"r"(sgt + off_bf16(g + 8 * r, nb + 8 * nt + 2 * t)), "r"(pkd.p[0]) : "memory");
-            } else {
-              st_pair<T>(sgt, g + 8 * r, nb + 8 * nt + 2 * t, gp[nt][r].x, gp[nt][r].y);
-            }
-          }
           gt[nt][r] = movm_t_np<NP>(pkd);
         }
+      if (save) st_slab<T, 64>(sgt, lane, nb, gp);
       // state update: W^T[nb.., :] -= te15 * Gp^T K ; b -= te15 * colsum(Gp)
       {
         const Pk<NP> agt[4] = {gt[0][0], gt[1][0], gt[0][1], gt[1][1]};
@@ -500,15 +494,16 @@ __global__ void __launch_bounds__(ROLE_THREADS, 1)
         if constexpr (MB == CS) sp[at0 + step] = make_float4(mean[1], rstd[1], 0.f, 0.f);
       }
       const uint32_t so = base + SM::OFF_OUT + par * TF::RAW_BYTES;
+      F2 oo[2][2];
+      ld_slab<T, SEG>(tq, lane, nb, oo);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const int row = g + 8 * r, col = nb + 8 * nt + 2 * t;
           const F2 x = f2mul(f2sub(zb[nt][r], f2(mean[r])), f2(rstd[r]));
-          const F2 o = f2add(ld_io<T, SEG>(tq, row, col), f2fma(gam[nt], x, bet[nt]));
-          st_io<T, SEG>(so, row, col, o.x, o.y);
+          oo[nt][r] = f2add(oo[nt][r], f2fma(gam[nt], x, bet[nt]));
         }
+      st_slab<T, SEG>(so, lane, nb, oo);
       mbar_arrive_warp(bar_empty + 8 * slot);
       fence_proxy_async_smem();  // (stored behind the next stage's exchange)
     }

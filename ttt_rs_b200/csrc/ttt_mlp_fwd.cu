@@ -91,9 +91,6 @@ __device__ __forceinline__ void xch8(float2* xb, const Lane& L, float a0x, float
   o1 = s1;
 }
 
-__device__ __forceinline__ void stsm_x4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 // offset of element (row, col) of a 16 x 256 operand tile stored as four [16][64] swizzled sub-tiles
 __device__ __forceinline__ uint32_t off_e(int row, int col) {
   return static_cast<uint32_t>((col >> 6) * TILE_BF16_BYTES) + off_bf16(row, col & 63);

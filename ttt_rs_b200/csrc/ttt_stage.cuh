@@ -189,13 +189,13 @@ __device__ __forceinline__ void bfrag_from_state(const float (&m)[8][4], int ks,
 // gam / bet: the thread's column pairs, index nt; btg = beta - (v - k).
 template <typename T, int SEG>
 __device__ __forceinline__ void beta_minus_target(const F2 (&bet)[2], uint32_t tk, uint32_t tv, const Lane& L, F2 (&btg)[2][2]) {
+  F2 k[2][2], v[2][2];
+  ld_slab<T, SEG>(tk, L.lane, L.nb, k);
+  ld_slab<T, SEG>(tv, L.lane, L.nb, v);
 #pragma unroll
   for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int row = L.g + 8 * r, col = L.nb + 8 * nt + 2 * L.t;
-      btg[nt][r] = f2sub(bet[nt], f2sub(ld_io<T, SEG>(tv, row, col), ld_io<T, SEG>(tk, row, col)));
-    }
+    for (int r = 0; r < 2; ++r) btg[nt][r] = f2sub(bet[nt], f2sub(v[nt][r], k[nt][r]));
 }
 __device__ __forceinline__ void ln_l2_pieces(const F2 (&z1)[2][2], const float (&mean)[2], const float (&rstd)[2],
                                              const F2 (&gam)[2], const F2 (&btg)[2][2], F2 (&xh)[2][2], F2 (&gy)[2][2],

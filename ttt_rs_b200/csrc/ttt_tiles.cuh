@@ -152,6 +152,41 @@ __device__ __forceinline__ uint32_t lane_off_io(int lane, int kc) {
   if constexpr (sizeof(T) == 2 && SEG == 32) return off_io<T, SEG>((lane & 7) + (((lane >> 3) & 1) << 3), kc + ((lane >> 4) << 3));
   else return lane_off_A(lane, kc);
 }
+// A warp's 16 x 16 slab of a tile, columns nb..nb+15, as column pairs x[nt][r]: in bf16 the four pairs of a thread are the four
+// 8 x 8 blocks of one ldmatrix / stmatrix, in place of an access each with an address of its own.
+template <typename T, int SEG>
+__device__ __forceinline__ void ld_slab(uint32_t tile, int lane, int nb, float2 (&x)[2][2]) {
+  if constexpr (sizeof(T) == 2) {
+    uint32_t v[4];
+    ldsm_x4(v, tile + lane_off_io<T, SEG>(lane, nb));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i >> 1][i & 1] = make_float2(bf16_lo(v[i]), bf16_hi(v[i]));
+  } else {
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) x[nt][r] = ld_io<T, SEG>(tile, (lane >> 2) + 8 * r, nb + 8 * nt + 2 * (lane & 3));
+  }
+}
+template <typename T, int SEG>
+__device__ __forceinline__ void st_slab(uint32_t tile, int lane, int nb, const float2 (&x)[2][2]) {
+  if constexpr (sizeof(T) == 2) {
+    stsm_x4(tile + lane_off_io<T, SEG>(lane, nb), pack_bf16(x[0][0].x, x[0][0].y), pack_bf16(x[0][1].x, x[0][1].y),
+            pack_bf16(x[1][0].x, x[1][0].y), pack_bf16(x[1][1].x, x[1][1].y));
+  } else {
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) st_io<T, SEG>(tile, (lane >> 2) + 8 * r, nb + 8 * nt + 2 * (lane & 3), x[nt][r].x, x[nt][r].y);
+  }
+}
+// Operand planes of a 16 x 16 block whose fragments are b[nt][r] (rows 8r.., columns 8nt.. of it): `at` is the address of
+// the planes plus lane_off_A of the block's first column.
+template <int NP>
+__device__ __forceinline__ void stsm_np(uint32_t at, const Pk<NP>& b00, const Pk<NP>& b01, const Pk<NP>& b10, const Pk<NP>& b11) {
+#pragma unroll
+  for (int p = 0; p < NP; ++p) stsm_x4(at + p * TILE_BF16_BYTES, b00.p[p], b01.p[p], b10.p[p], b11.p[p]);
+}
 // `stream` (SEG = 32: pair) and first token of the tile; `seq` tokens per stream
 template <typename T, int SEG>
 __device__ __forceinline__ void tma_load_io(uint32_t tile, const CUtensorMap* tm, int stream, int t0, int seq, uint32_t bar) {
