@@ -43,3 +43,34 @@ def test_chunks_equal_one_piece_and_the_oracle(F, mb, NS, K):
         else:  # sums over the streams, in an order of each launch's own: a few hundred additions of 2^-24 each
             a, b = whole[k].double(), lo[k].double() + hi[k].double()
             assert ((a - b).norm() / b.norm()).item() < 1e-5, k
+
+
+@pytest.mark.gpu
+def test_a_handoff_that_never_comes_ends_the_launch():
+    """The first item numbers are skipped, so the chain group of every block waits for a hand-off that nothing publishes: its
+    bounded wait ends the other groups' waits, the launch returns, and the next one gives the earlier gradients."""
+    import ttt_rs_b200 as tb
+    from ttt_rs_b200 import _lib
+    dev = torch.device("cuda:0")
+    B, H = 40, 4
+    t = O.make_inputs(B, H, 32 * 16, 64, 16, seed=3, dtype=torch.float32)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 128, 16)
+    outs, saved = tb.TttTileMultiKernel.forward_launch(tb.TttInputs(*[t[k].to(dev).contiguous() for k in IN]), cfg)
+    go = tb.TttOutputs(t["grad_output"].to(dev), None, None)
+    good = tb.TttTileMultiKernel.backward_launch(saved, go, cfg)
+    tb.check_status()
+    lib = _lib.load()
+    try:
+        lib.ttt_b200_debug_handoff(2000, B * H)
+        bad = tb.TttTileMultiKernel.backward_launch(saved, go, cfg)
+        torch.cuda.synchronize()
+    finally:
+        lib.ttt_b200_debug_handoff(0, 0)
+    words = bad.status.cpu().tolist()
+    assert words[0] == _lib.TTT_ERR_TIMEOUT and words[1] == 15 and words[3] == 15, words
+    with pytest.raises(tb.TttError):
+        tb.check_status()
+    again = tb.TttTileMultiKernel.backward_launch(saved, go, cfg)
+    tb.check_status()
+    for n in IN:
+        assert torch.equal(getattr(again, n), getattr(good, n)), n
