@@ -682,7 +682,8 @@ def roofline_of(w, res, name):
     ms, fwd_ms, bwd_ms = res["ms"], res["fwd_ms"], res["bwd_ms"]
     total_b, fb, bb = algorithmic_bytes(w, True, w["backward"])
     if w["backward"]:
-        dom_ms, dom_bytes, dom_name = bwd_ms, bb, ("ttt_mlp_bwd_kernel" if mlp else "ttt_linear_bwd_kernel")
+        dom_ms, dom_bytes, dom_name = bwd_ms, bb, ("ttt_mlp_bwd_kernel" if mlp else "ttt_linear_bwd_kernel" if w["dtype"] == "bf16"
+                                          else "ttt_linear_bwd_f32_kernel")
     else:
         dom_ms, dom_bytes, dom_name = fwd_ms, fb, ("ttt_mlp_fwd_kernel" if mlp else "ttt_linear_fwd_kernel")
     achieved = dom_bytes / (dom_ms * 1e-3) / 1e9

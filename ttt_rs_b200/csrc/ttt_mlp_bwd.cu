@@ -24,7 +24,7 @@
 //  * A warp also owns one token row of the 16 x 64 tiles for the two LayerNorms.
 // A stage is six barrier intervals (I1..I6 below).  Before, 25 phases passed every intermediate tile through shared
 // memory as bf16, undid the updates through registers and read dW from L2: 43 k cycles a stage; 192 streams of 128 stages
-// forward and backward 4.12 ms, now 2.55 ms.
+// forward and backward 4.12 ms, now 2.52 ms.
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
 #include "ttt_stage.cuh"
