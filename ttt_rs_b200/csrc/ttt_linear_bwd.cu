@@ -387,17 +387,9 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
         bias[2 * nt + 1] = b2.y;
       }
     }
-    // ---- 2. operand copies of W_s^T and dW^T (this warp's 16 rows) for the products that contract over n
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      const float(&a)[4] = wt[2 * ks], (&b)[4] = wt[2 * ks + 1], (&c)[4] = dwt[2 * ks], (&d)[4] = dwt[2 * ks + 1];
-      const uint32_t o = warp * SM::PLANES + lane_off_A(lane, 16 * ks);
-      stsm_np<NP>(tW + o, split_pack<NP>(a[0] * wscale, a[1] * wscale), split_pack<NP>(a[2] * wscale, a[3] * wscale),
-                  split_pack<NP>(b[0] * wscale, b[1] * wscale), split_pack<NP>(b[2] * wscale, b[3] * wscale));
-      stsm_np<NP>(tDW + o, split_pack<NP>(c[0], c[1]), split_pack<NP>(c[2], c[3]), split_pack<NP>(d[0], d[1]),
-                  split_pack<NP>(d[2], d[3]));
-    }
-    // ---- 3. Z1 = K W + b, Zq = Q W + b, KdW = K dW, Attn = Q K^T
+    // ---- 2/3. Z1 = K W + b, Zq = Q W + b, KdW = K dW, Attn = Q K^T; the fragments of What_s^T and dW^T (this warp's 16 rows) also
+    // go to shared memory, for the products that contract over n (scaling the copy of W instead of those products' sums
+    // took a conversion and a multiplication more per element: 64 stages, 12 streams 132 -> 126 us, 384 271 -> 261)
     float z1[2][4], zq[2][4], kdw[2][4], at[2][4];
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
@@ -408,6 +400,9 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
       Pk<NP> bw[2][2], bdw[2][2], ak[4], aq[4];
       bfrag_from_state<NP>(wt, ks, bw);
       bfrag_from_state<NP>(dwt, ks, bdw);
+      const uint32_t o = warp * SM::PLANES + lane_off_A(lane, 16 * ks);
+      stsm_np<NP>(tW + o, bw[0][0], bw[1][0], bw[0][1], bw[1][1]);
+      stsm_np<NP>(tDW + o, bdw[0][0], bdw[1][0], bdw[0][1], bdw[1][1]);
       ldsm_np<NP>(ak, pk + lane_off_io<T, SEG>(lane, 16 * ks), PL, false);
       ldsm_np<NP>(aq, pq + lane_off_io<T, SEG>(lane, 16 * ks), PL, false);
 #pragma unroll
@@ -423,13 +418,8 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     }
     tmem_st_8x4(tm_w, wt);  // W_s^T: next used by the stage below (dW^T is unchanged so far: nothing to store)
     // products were taken with What: Z = wscale * acc + b
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        z1[nt][i] = fmaf(z1[nt][i], wscale, bias[2 * nt + (i & 1)]);
-        zq[nt][i] = fmaf(zq[nt][i], wscale, bias[2 * nt + (i & 1)]);
-      }
+    scale_add(z1, wscale, bias);
+    scale_add(zq, wscale, bias);
     // ---- 4. LN + L2 pieces of Z1 from the saved row statistics
     float mean1[2], rstd1[2], Bv1[2], mean2[2], rstd2[2];
     F2 xh[2][2], gy[2][2], gx[2][2], G[2][2];
@@ -511,11 +501,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     __syncthreads();
 
     // ---- 9. products that need dZbar
-    float pp[2][4], gl[2][4], dk[2][4], dgp[2][4];
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) pp[nt][i] = gl[nt][i] = dk[nt][i] = dgp[nt][i] = 0.f;
+    float pp[2][4] = {}, gl[2][4] = {}, dk[2][4] = {}, dgp[2][4] = {}, xw[2][4] = {};
     // (the B fragments of W^T read here serve step 13 as well -- there are registers for them now that the state
     // is parked in tensor memory)
     Pk<NP> bw_keep[4][4];
@@ -534,15 +520,16 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
         const Pk<NP> b0[2] = {ags[0], ags[2]}, b1[2] = {ags[1], ags[3]};
         mma_np2<NP>(pp[0], adz, b0, pp[1], adz, b1);
       }
-      {  // dq += dZbar W^T (columns nb..nb+15)
+      {  // dZbar What^T (columns nb..nb+15)
         const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
-        mma_np2<NP>(dq[0], adz, b0, dq[1], adz, b1);
+        mma_np2<NP>(xw[0], adz, b0, xw[1], adz, b1);
       }
       {  // Gl' = Gp dW^T (columns nb..nb+15)
         const Pk<NP> b0[2] = {bdw[0], bdw[1]}, b1[2] = {bdw[2], bdw[3]};
         mma_np2<NP>(gl[0], ags, b0, gl[1], ags, b1);
       }
     }
+    add_scaled(dq, wscale, xw);
     // dM' = -tril(P');  dA = dM' o te[i];  d te[i] = sum_j dM'[i,j] (1 + Attn[i,j])
     float dte_row[2];
     Pk<NP> ada[4];
@@ -660,13 +647,14 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     if (elect_one()) bulk_wait_read<0>();  // the previous stage's output tiles have left the staging buffers
     __syncthreads();
     // ---- 13. dk += dZ1 W^T ; dW^T += dZ1^T K ; bias gradient
+    float xk[2][4] = {};
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       Pk<NP> adz1[4];
       const Pk<NP>(&bwt)[4] = bw_keep[ks];
       ldsm_np<NP>(adz1, tDZ1 + lane_off_A(lane, 16 * ks), PL, false);
       const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
-      mma_np2<NP>(dk[0], adz1, b0, dk[1], adz1, b1);
+      mma_np2<NP>(xk[0], adz1, b0, xk[1], adz1, b1);
     }
     // dW^T += dZbar^T Q, then dW^T += dZ1^T K: both here (the dZbar tile and this stage's Q tile are still in place), so
     // that dW^T is in registers for this one stretch of the stage
@@ -703,6 +691,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     }
     // ---- 14. outputs: dq = d_out + ..., dk = -dT + ..., dv = dT
     {
+      add_scaled(dk, wscale, xk);
       const uint32_t so_q = base + SM::OFF_OUT, so_k = so_q + TF::RAW_BYTES, so_v = so_k + TF::RAW_BYTES;
       F2 dqq[2][2], dkk[2][2];
       slab_pairs(dq, dqq);

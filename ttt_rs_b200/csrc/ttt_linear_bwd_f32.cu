@@ -10,7 +10,7 @@
 //   chain   (warps 4..7): K dW, the second derivative, dZ1, dW += dZbar^T Q + dZ1^T K, the bias gradient;
 //   output  (warps 8..11): dq, dk, dv and the token_eta terms from the copies of W, dW, dZbar and dZ1 that the others leave;
 //   prepare (warps 12..15): split of float32 tiles into bf16 planes and Q K^T (three warps), the copies (one lane).
-// 64 stages, us, in one group / in four: 96 streams 419 / 321, 12 streams 411 / 298, 192 streams 617 / 565, 384 1134 / 1011.
+// 64 stages, us, in one group / in four: 96 streams 419 / 309, 12 streams 411 / 296, 192 streams 617 / 552, 384 1134 / 997.
 // The chain group is what the others wait for (9.0 k of 9.3 k cycles a stage, 550 mma.sync per scheduler among them).  The
 // same split of a bf16 stage is slower than the one group from 12 streams (138 / 132 us) to 1024 (1185 / 667): its products
 // take a sixth, and four programs of 25 KB together miss in the instruction cache (3.4 of 12.7 stalled warps).
@@ -44,7 +44,7 @@ struct BwdRoleSmem {
   static constexpr uint32_t OFF_REC = OFF_LR + 128;          // int4: stream, stage, chunk, flags
   static constexpr uint32_t SLOT = OFF_STAT + (NH == 2 ? 2048 : 1024);
   static_assert(OFF_REC + 16 <= SLOT && SLOT % 1024 == 0, "");
-  // recover's record: W copy, dZbar tile, Z1, dGp' and the rows' sum of dZbar as the threads hold them
+  // recover's record: copy of What, dZbar tile, Z1, dGp' and the rows' sum of dZbar as the threads hold them
   static constexpr uint32_t R_W = 0, R_DZ = 4 * PLANES, R_Z1 = R_DZ + PLANES, R_DG = R_Z1 + NTHREADS * 32,
                             R_SUM = R_DG + NTHREADS * 32, R_LN = R_SUM + NTHREADS * 16, R_BYTES = R_LN + 1024;
   // chain's record: dZ1 tile, dT and a partial sum as the threads hold them
@@ -382,26 +382,26 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         const Pk<NP> ngt[4] = {neg_pk<NP>(agt[0]), neg_pk<NP>(agt[1]), neg_pk<NP>(agt[2]), neg_pk<NP>(agt[3])};
         state_update_direct<NP, SEG>(wt, ngt, pk, lane, khalf);
       }
-      // ---- 2. Z1 = K W + b, Zq = Q W + b  (products with What: Z = wscale * acc + b)
+      // ---- 2. Z1 = K W + b, Zq = Q W + b  (products with What: Z = wscale * acc + b); the fragments of What also go to the record
+      // (whose last readers are past it by now: the slot this stage came in was theirs)
+      if (n >= NR && !mbar_wait_or_stop(b_rtaken + 8 * rb, ((n / NR) - 1) & 1, stop)) fail = 1;
       float z1[2][4] = {}, zq[2][4] = {};
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         Pk<NP> bw[2][2], ak[4], aq[4];
         bfrag_from_state<NP>(wt, ks, bw);
+        stsm_np<NP>(rr + SM::R_W + warp * SM::PLANES + lane_off_A(lane, 16 * ks), bw[0][0], bw[1][0], bw[0][1], bw[1][1]);
         ldsm_np<NP>(ak, pk + lane_off_io<T, SEG>(lane, 16 * ks), PL, false);
         ldsm_np<NP>(aq, pq + lane_off_io<T, SEG>(lane, 16 * ks), PL, false);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) mma_np2<NP>(z1[nt], ak, bw[nt], zq[nt], aq, bw[nt]);
       }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        const float2 b2 = *reinterpret_cast<const float2*>(gsl + SM::OFF_BS + (nb + 8 * nt + 2 * t) * 4);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float b = (i & 1) ? b2.y : b2.x;
-          z1[nt][i] = fmaf(z1[nt][i], wscale, b);
-          zq[nt][i] = fmaf(zq[nt][i], wscale, b);
-        }
+      {
+        const float2 b0 = *reinterpret_cast<const float2*>(gsl + SM::OFF_BS + (nb + 2 * t) * 4);
+        const float2 b1 = *reinterpret_cast<const float2*>(gsl + SM::OFF_BS + (nb + 8 + 2 * t) * 4);
+        const float bias[4] = {b0.x, b0.y, b1.x, b1.y};
+        scale_add(z1, wscale, bias);
+        scale_add(zq, wscale, bias);
       }
       // ---- 3. Zbar = Zq - M' Gp   (am holds -M')
       Pk<NP> am[4];
@@ -459,8 +459,7 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
           for (int r = 0; r < 2; ++r)
             dzb[nt][r] = f2mul(f2fma(xz[nt][r], f2(-c2[r]), f2sub(tt[nt][r], f2(c1[r]))), f2(rstd2[r]));
       }
-      // ---- 5. the record: dZbar as an operand tile, W's copy, Z1, dGp' = -M'^T dZbar
-      if (n >= NR && !mbar_wait_or_stop(b_rtaken + 8 * rb, ((n / NR) - 1) & 1, stop)) fail = 1;
+      // ---- 5. the rest of the record: dZbar as an operand tile, Z1, dGp' = -M'^T dZbar
       const uint32_t tDZ = rr + SM::R_DZ;
       stsm_np<NP>(tDZ + lane_off_A(lane, nb), split_pack<NP>(dzb[0][0].x, dzb[0][0].y), split_pack<NP>(dzb[0][1].x, dzb[0][1].y),
                   split_pack<NP>(dzb[1][0].x, dzb[1][0].y), split_pack<NP>(dzb[1][1].x, dzb[1][1].y));
@@ -472,13 +471,6 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         const Pk<NP> amt[4] = {movm_t_np<NP>(am[0]), movm_t_np<NP>(am[2]), movm_t_np<NP>(am[1]), movm_t_np<NP>(am[3])};
         const Pk<NP> z0[2] = {bdz[0], bdz[1]}, zz1[2] = {bdz[2], bdz[3]};
         mma_np2<NP>(dgp[0], amt, z0, dgp[1], amt, zz1);
-      }
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const float(&a)[4] = wt[2 * ks], (&b)[4] = wt[2 * ks + 1];
-        stsm_np<NP>(rr + SM::R_W + warp * SM::PLANES + lane_off_A(lane, 16 * ks), split_pack<NP>(a[0] * wscale, a[1] * wscale),
-                    split_pack<NP>(a[2] * wscale, a[3] * wscale), split_pack<NP>(b[0] * wscale, b[1] * wscale),
-                    split_pack<NP>(b[2] * wscale, b[3] * wscale));
       }
       {
         const F2 d0 = f2add(dzb[0][0], dzb[0][1]), d1 = f2add(dzb[1][0], dzb[1][1]);
@@ -809,7 +801,7 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
       if (!mbar_wait_or_stop(b_rgiven + 8 * rb, (n / NR) & 1, stop)) fail = 1;
       // ---- 1. P' = dZbar Gp^T (over the head's own columns), dq = d_out + dZbar W^T
       const uint32_t tDZ = rr + SM::R_DZ, tW = rr + SM::R_W;
-      float pp[2][4] = {}, dq[2][4], dk[2][4] = {}, gl[2][4] = {};
+      float pp[2][4] = {}, dq[2][4], dk[2][4] = {}, gl[2][4] = {}, xw[2][4] = {};
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -831,8 +823,9 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
           mma_np2<NP>(pp[0], adz, b0, pp[1], adz, b1);
         }
         const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
-        mma_np2<NP>(dq[0], adz, b0, dq[1], adz, b1);
+        mma_np2<NP>(xw[0], adz, b0, xw[1], adz, b1);
       }
+      add_scaled(dq, wscale, xw);
       // ---- 2. Gl' = Gp dW^T
       if (!mbar_wait_or_stop(b_dgiven + 8 * db, (n / ND) & 1, stop)) fail = 1;
 #pragma unroll
@@ -891,6 +884,7 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
       }
       mbar_arrive_warp(b_empty + 8 * slot);
       // ---- 4. dk += dZ1 W^T;  dk = -dT + ..., dv = dT
+      float xk[2][4] = {};
       if (!mbar_wait_or_stop(b_zgiven + 8 * zb, (n / NZ) & 1, stop)) fail = 1;
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
@@ -898,8 +892,9 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         ldsm_np<NP>(adz1, rz + SM::Z_DZ1 + lane_off_A(lane, 16 * ks), PL, false);
         ldsm_np<NP>(bwt, tW + ks * SM::PLANES + lane_off_B_kn(lane, nb), PL, true);
         const Pk<NP> b0[2] = {bwt[0], bwt[1]}, b1[2] = {bwt[2], bwt[3]};
-        mma_np2<NP>(dk[0], adz1, b0, dk[1], adz1, b1);
+        mma_np2<NP>(xk[0], adz1, b0, xk[1], adz1, b1);
       }
+      add_scaled(dk, wscale, xk);
       mbar_arrive_warp(b_rtaken + 8 * rb);
       F2 dT[2][2];
 #pragma unroll

@@ -173,6 +173,28 @@ __device__ __forceinline__ void slab_pairs(const float (&c)[2][4], F2 (&z)[2][2]
   }
 }
 
+// c = c * s + b (column pairs of b), and c += s * x, on the accumulator registers of a 16x16 slab
+__device__ __forceinline__ void scale_add(float (&c)[2][4], float s, const float (&b)[4]) {
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const F2 z = f2fma(pr(c[nt], r), f2(s), f2(b[2 * nt], b[2 * nt + 1]));
+      c[nt][2 * r] = z.x;
+      c[nt][2 * r + 1] = z.y;
+    }
+}
+__device__ __forceinline__ void add_scaled(float (&c)[2][4], float s, const float (&x)[2][4]) {
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const F2 z = f2fma(pr(x[nt], r), f2(s), pr(c[nt], r));
+      c[nt][2 * r] = z.x;
+      c[nt][2 * r + 1] = z.y;
+    }
+}
+
 // B fragments of a 64x64 matrix held transposed in accumulator registers (m[kt][2*rn+e] = M[k=8kt+2t+e][n=nb+g+8rn]),
 // for products X[16 x 64(k)] . M[:, nb..nb+15]:  k-step ks, n-tile nt.
 template <int NP>
