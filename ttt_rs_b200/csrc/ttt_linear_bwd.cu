@@ -389,8 +389,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
     }
     // ---- 2/3. Z1 = K W + b, Zq = Q W + b, KdW = K dW, Attn = Q K^T; the fragments of What_s^T and dW^T (this warp's 16 rows) also
     // go to shared memory, for the products that contract over n (scaling the copy of W instead of those products' sums
-    // took a conversion and a multiplication more per element: 64 stages, 12 streams 132 -> 126 us, 384 271 -> 261; the two row
-    // sums formed from products and sums at hand instead of another pass over K and dL/dG, below: 126 -> 124, 1024 636 -> 630)
+    // took a conversion and a multiplication more per element: 64 stages, 12 streams 132 -> 126 us, 384 271 -> 261)
     float z1[2][4], zq[2][4], kdw[2][4], at[2][4];
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
@@ -564,38 +563,40 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
       mma_np2<NP>(dgp[0], amt, z0, dgp[1], amt, zz1);  // dGp = -M'^T dZbar
     }
     // ---- 10. gradient reaching Gp, the lr / token_eta terms, and the first pair of second-derivative sums
-    F2 v[2][2];
-    float s1t[2], s2t[2], ug[2];
+    F2 u[2][2], v[2][2];
+    float s1t[2], s2t[2];
     {
-      F2 p1[2] = {f2(0.f), f2(0.f)}, p2[2] = {f2(0.f), f2(0.f)}, pdl[2] = {f2(0.f), f2(0.f)}, prt = f2(0.f);
+      F2 p1[2] = {f2(0.f), f2(0.f)}, p2[2] = {f2(0.f), f2(0.f)}, pdl[2] = {f2(0.f), f2(0.f)}, prt[2] = {f2(0.f), f2(0.f)};
+      F2 k[2][2];
+      ld_slab<T, SEG>(tk, lane, nb, k);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
+          const F2 kk = k[nt][r];
           const F2 glp = pr(gl[nt], r);
           // dL/dGp = -M'^T dZbar - te15 (K dW + db)
-          const F2 dup = f2add(pr(kdw[nt], r), dbias[nt]);
-          const F2 dg = f2fma(dup, f2(-te15), pr(dgp[nt], r));
+          const F2 dg = f2fma(f2add(pr(kdw[nt], r), dbias[nt]), f2(-te15), pr(dgp[nt], r));
           const F2 dkn = f2fma(glp, f2(-te15), pr(dk[nt], r));
           dk[nt][2 * r] = dkn.x;
           dk[nt][2 * r + 1] = dkn.y;
-          prt = f2fma(f2mul(G[nt][r], f2(lr_row[r])), dup, prt);  // (the sum of K o (Gp dW^T) is that of Gp o (K dW))
+          prt[r] = f2fma(kk, glp, f2fma(f2mul(G[nt][r], f2(lr_row[r])), dbias[nt], prt[r]));
           pdl[r] = f2fma(dg, G[nt][r], pdl[r]);
           const F2 uu = f2mul(dg, f2(lr_row[r]));  // dL/dG
           const F2 vv = f2mul(uu, f2(-rstd1[r]));
+          u[nt][r] = uu;
           v[nt][r] = vv;
           p1[r] = f2add(p1[r], vv);
           p2[r] = f2fma(vv, xh[nt][r], p2[r]);
         }
       float4 o0, o1;
       int f2_ = 0;
-      xch_rows<SEG, false>(&xch[xsel], L, make_float4(f2hsum(p1[0]), f2hsum(p2[0]), f2hsum(pdl[0]), f2hsum(prt)),
-                    make_float4(f2hsum(p1[1]), f2hsum(p2[1]), f2hsum(pdl[1]), 0.f), o0, o1, f2_);
+      xch_rows<SEG, false>(&xch[xsel], L, make_float4(f2hsum(p1[0]), f2hsum(p2[0]), f2hsum(pdl[0]), f2hsum(prt[0])),
+                    make_float4(f2hsum(p1[1]), f2hsum(p2[1]), f2hsum(pdl[1]), f2hsum(prt[1])), o0, o1, f2_);
       xsel ^= 1;
       s1t[0] = o0.x * INV_F; s2t[0] = o0.y * INV_F;
       s1t[1] = o1.x * INV_F; s2t[1] = o1.y * INV_F;
-      ug[0] = lr_row[0] * o0.z; ug[1] = lr_row[1] * o1.z;  // row sums of dL/dG o G
-      const float rt_all = col_sum(o0.w);  // sum over the mini-batch (a thread's two rows came as one)
+      const float rt_all = col_sum(o0.w + o1.w);  // sum over the 16 rows
       // (every warp holds these row values; warp 2 writes them, of a pair of heads the first warp of each)
       if ((SEG == 32 ? (warp & 1) == 0 : warp == 2) && t == 0) {
         // per (batch, head) stream of the caller's tensors: the pair's heads are streams 2 * stream and 2 * stream + 1
@@ -628,13 +629,13 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
           dxh[nt][r] = dx;
           dT[nt][r] = f2neg(dy);
           pd[r] = f2add(pd[r], dx);
-          ps[r] = f2fma(dx, x, ps[r]);
+          ps[r] = f2fma(f2fma(dx, x, f2mul(u[nt][r], G[nt][r])), f2(-rstd1[r]), ps[r]);
         }
       float2 a0, a1;
       int f2_ = 0;
       xch_rows2<SEG, false>(&xch[xsel], L, f2hsum(pd[0]), f2hsum(ps[0]), f2hsum(pd[1]), f2hsum(ps[1]), a0, a1, f2_);
       xsel ^= 1;
-      const float D[2] = {a0.x * INV_F, a1.x * INV_F}, S[2] = {-rstd1[0] * INV_F * (a0.y + ug[0]), -rstd1[1] * INV_F * (a1.y + ug[1])};
+      const float D[2] = {a0.x * INV_F, a1.x * INV_F}, S[2] = {a0.y * INV_F, a1.y * INV_F};
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll

@@ -10,7 +10,7 @@
 //   chain   (warps 4..7): K dW, the second derivative, dZ1, dW += dZbar^T Q + dZ1^T K, the bias gradient;
 //   output  (warps 8..11): dq, dk, dv and the token_eta terms from the copies of W, dW, dZbar and dZ1 that the others leave;
 //   prepare (warps 12..15): split of float32 tiles into bf16 planes and Q K^T (three warps), the copies (one lane).
-// 64 stages, us, in one group / in four: 96 streams 419 / 309, 12 streams 411 / 296, 192 streams 617 / 549, 384 1134 / 989.
+// 64 stages, us, in one group / in four: 96 streams 419 / 309, 12 streams 411 / 296, 192 streams 617 / 552, 384 1134 / 997.
 // The chain group is what the others wait for (9.0 k of 9.3 k cycles a stage, 550 mma.sync per scheduler among them).  The
 // same split of a bf16 stage is slower than the one group from 12 streams (138 / 132 us) to 1024 (1185 / 667): its products
 // take a sixth, and four programs of 25 KB together miss in the instruction cache (3.4 of 12.7 stalled warps).
@@ -620,9 +620,8 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             // dL/dGp = -M'^T dZbar - te15 (K dW + db)
-            const F2 dup = f2add(pr(kdw[nt], r), dbias[nt]);
-            const F2 dg = f2fma(dup, f2(-te15), dgp[r]);
-            pg_ = f2fma(f2mul(G[nt][r], f2(lr_row[r])), dup, pg_);  // (the sum of K o (Gp dW^T) is that of Gp o (K dW))
+            const F2 dg = f2fma(f2add(pr(kdw[nt], r), dbias[nt]), f2(-te15), dgp[r]);
+            pg_ = f2fma(f2mul(G[nt][r], f2(lr_row[r])), dbias[nt], pg_);
             pdl[r] = f2fma(dg, G[nt][r], pdl[r]);
             const F2 uu = f2mul(dg, f2(lr_row[r]));  // dL/dG
             const F2 vv = f2mul(uu, f2(-rstd1[r]));
@@ -867,7 +866,22 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         mma_np2<NP>(dq[0], ada, k0, dq[1], ada, k1);
         mma_np2<NP>(dk[0], adat, q0, dk[1], adat, q1);
       }
-      add_scaled(dk, -te15, gl);
+      float prt;
+      {
+        F2 ps[2] = {f2(0.f), f2(0.f)};
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const F2 kk = ld_io<T, SEG>(tk, g + 8 * r, nb + 8 * nt + 2 * t);
+            const F2 glp = pr(gl[nt], r);
+            const F2 dkn = f2fma(glp, f2(-te15), pr(dk[nt], r));
+            dk[nt][2 * r] = dkn.x;
+            dk[nt][2 * r + 1] = dkn.y;
+            ps[r] = f2fma(kk, glp, ps[r]);
+          }
+        prt = f2hsum(f2add(ps[0], ps[1]));
+      }
       mbar_arrive_warp(b_empty + 8 * slot);
       // ---- 4. dk += dZ1 W^T;  dk = -dT + ..., dv = dT
       float xk[2][4] = {};
@@ -889,11 +903,10 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
         dT[nt][0] = f2(v.x, v.y);
         dT[nt][1] = f2(v.z, v.w);
       }
-      float prt;
       {
         float pgb;
         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(pgb) : "r"(rz + SM::Z_PS + tid * 4) : "memory");
-        prt = col_sum(quad_sum(pgb));  // over the mini-batch and this warp's columns
+        prt = col_sum(quad_sum(prt + pgb));  // over the mini-batch and this warp's columns
       }
       mbar_arrive_warp(b_ztaken + 8 * zb);
       float* const oxb = ox + 4 * (n & 1);
