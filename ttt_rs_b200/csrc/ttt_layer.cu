@@ -685,20 +685,21 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
     for (int r = warp; r < rows; r += nwarps) {
       const T* zr = reinterpret_cast<const T*>(zt) + (size_t)r * C;
       const T* yr = reinterpret_cast<const T*>(yt) + (size_t)r * C;
-      F2 acc = f2(0.f);
+      // (row sums in the order of the columns: a learning-rate position's gradient is a difference of large sums and shows their last
+      // bits)
+      float s = 0.f;
 #pragma unroll
       for (int j = 0; j < MAXCH; ++j)
         if (j * 32 + lane < nch) {
           F2 v[NPAIR];
           chunk(zr + (j * 32 + lane) * EPC, v);
 #pragma unroll
-          for (int k = 0; k < NPAIR; ++k) acc = f2add(acc, v[k]);
+          for (int k = 0; k < NPAIR; ++k) s = s + v[k].x + v[k].y;
         }
-      float s = f2hsum(acc);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       const float mean = s / C;
-      F2 qq = f2(0.f), a1 = f2(0.f), a2 = f2(0.f);
+      float q = 0.f, m1 = 0.f, m2 = 0.f;
 #pragma unroll
       for (int j = 0; j < MAXCH; ++j)
         if (j * 32 + lane < nch) {
@@ -721,12 +722,11 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
 #pragma unroll
           for (int k = 0; k < NPAIR; ++k) {
             const F2 x = f2sub(v[k], f2(mean)), dx = f2mul(dn[k], *reinterpret_cast<const F2*>(&gam[c0 + 2 * k]));
-            qq = f2fma(x, x, qq);
-            a1 = f2add(a1, dx);
-            a2 = f2fma(dx, x, a2);
+            q = fmaf(x.y, x.y, fmaf(x.x, x.x, q));
+            m1 = m1 + dx.x + dx.y;
+            m2 = fmaf(dx.y, x.y, fmaf(dx.x, x.x, m2));
           }
         }
-      float q = f2hsum(qq), m1 = f2hsum(a1), m2 = f2hsum(a2);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         q += __shfl_xor_sync(0xffffffffu, q, o);
