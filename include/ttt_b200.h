@@ -194,7 +194,7 @@ int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const voi
  *   (per batch element); grad_ttt_lr_eta [B,H,T]; float32 grad_token_eta [T] (per stage position, summed over B, H),
  *   float32 grad_ln_weight / grad_ln_bias [H,F] (summed over B).  All written, never accumulated into.
  * `workspace`: ttt_mlp_backward_workspace_bytes(d) bytes, 16-byte aligned (the float32 state and state gradients, a
- * hand-off record and one record per mini-batch of every stream: about B*H*(259 KB + 27.5 KB per mini-batch), plus the
+ * hand-off record and one record per mini-batch of every stream: about B*H*(259 KB + 27.1 KB per mini-batch), plus the
  * scheduler words).  The kernel is persistent: blocks take (stream, chunk of mini-batches) work items and hand a stream's
  * state to one another through the workspace; it is launched cooperatively (all blocks co-resident), one block per SM, and
  * every hand-off wait is bounded.  A block allocates the SM's whole tensor memory (512 columns) for the float32 state while

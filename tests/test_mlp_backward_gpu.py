@@ -157,3 +157,29 @@ def test_mlp_backward_is_bitwise_reproducible(from_forward):
     for k in runs[0]:
         assert torch.equal(runs[0][k], runs[1][k]), f"{k} differs between two runs"
     assert all(bool(torch.isfinite(v.float()).all()) for v in runs[0].values())
+
+
+@pytest.mark.gpu
+def test_rows_off_their_centre():
+    """Z2 and Zb2 rows whose mean is about 100 times their standard deviation: the gradients differentiate both LayerNorms with
+    variances summed about the mean.  From E[z^2] - mean^2 in float32 the variance would be off by up to 100^2 2^-22 = 2.4e-3,
+    a bias of every row (grad_w1 of this case: 1.1e-2 off in 2-norm, against 3.7e-3).  The other errors are those of centred
+    rows, bf16 operands (largest here: 4.3e-3), plus 2.4e-3 through the forward's own inner gradients: 7e-3 holds both."""
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    t = _case(1, 8, 256, 5)
+    g = torch.Generator().manual_seed(6)
+    t["b2"] = (2.0 + 0.01 * torch.randn(1, 8, 64, generator=g)).to(torch.bfloat16)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 128, 1)
+    d = {k: v.to(dev) for k, v in t.items()}
+    want = O.ttt_mlp_backward_autograd(*[d[k].double() for k in MLP_IN], d["grad_output"].double())
+    st = tb.TTTMLPState(d["w1"], d["b1"], d["w2"], d["b2"])
+    got = tb.fused_ttt_mlp_backward(d["xq"], d["xk"], d["xv"], st, d["token_eta"], d["ttt_lr_eta"], d["ln_weight"],
+                                    d["ln_bias"], d["grad_output"], cfg)
+    torch.cuda.synchronize()
+    tb.check_mlp_status(got)
+    for k in ("grad_xq", "grad_xk", "grad_xv", "grad_w1", "grad_b1", "grad_w2", "grad_b2", "grad_ttt_lr_eta",
+              "grad_ln_weight", "grad_ln_bias"):
+        err = ((got[k].double() - want[k]).norm() / want[k].norm()).item()
+        print(f"{k}: {err:.2e}")
+        assert err < 7e-3, f"{k}: {err}"

@@ -339,9 +339,9 @@ constexpr int MLP_HO_B1 = 0, MLP_HO_B2 = 256, MLP_HO_DB1 = 320, MLP_HO_DB2 = 576
 __host__ __device__ inline int mlp_master_at(int e, int f) { return ((((e >> 5) * 16 + (f >> 2)) * 32 + (e & 31)) << 2) + (f & 3); }
 // A stage's record, in bytes.  X2 [16][256] and G1p [16][256] (four tiles of 64 columns) and G2p [16][64]: bf16, in the
 // swizzled form that shared memory holds them in (off_bf16); float32: Z2, Zb2 [16][64], b1 [256] at the start of the stage, and
-// per token (8 floats) mean and 1 / std of Z2, the two row means of its LayerNorm gradient, mean and 1 / std of Zb2
+// per token the means of Z2 and of Zb2
 constexpr int MLP_REC_X2 = 0, MLP_REC_G1P = 8192, MLP_REC_G2P = 16384, MLP_REC_Z2 = 18432, MLP_REC_ZB2 = 22528,
-              MLP_REC_B1 = 26624, MLP_REC_STAT = 27648, MLP_REC_BYTES = 28160;
+              MLP_REC_B1 = 26624, MLP_REC_MEAN = 27648, MLP_REC_BYTES = 27776;
 // Stages per work item of the persistent launches: a stream that has a block to itself is one item; otherwise the length
 // for which the busiest block has least to do, a hand-over of a stream counted as one stage and a half (the backward: 512 KB
 // through L2 against a stage of 4 us)

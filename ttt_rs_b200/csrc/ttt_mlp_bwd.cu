@@ -8,7 +8,7 @@
 // How: the stage-by-stage analytic backward (reverse walk over the mini-batches carrying dW1, db1, dW2, db2; GELU and
 // LayerNorm second derivatives).  The forward kernel leaves one record per stage (MlpStage: X2, the lr-scaled inner
 // gradients G1p and G2p, Z2, Zb2, b1): W1_s = W1_{s+1} + te15 K^T G1p, W2_s = W2_{s+1} + te15 X2^T G2p undo the stage's
-// update, and both LayerNorms of the stage are differentiated straight from the saved Z2 and Zb2.
+// update, and both LayerNorms of the stage are differentiated straight from the saved Z2 and Zb2, with statistics of two passes.
 //
 // Where things live, and who does what:
 //  * The float32 masters of W1^T, W2, dW1^T, dW2 fill the SM's tensor memory, each as [256 hidden][64 features] = two
@@ -100,6 +100,11 @@ __device__ __forceinline__ float lds_f(uint32_t a) {
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ uint32_t lds_u(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
 __device__ __forceinline__ F2 lds_f2(uint32_t a) {
   F2 v;
   asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
@@ -110,11 +115,6 @@ __device__ __forceinline__ void sts_f2(uint32_t a, F2 v) { asm volatile("st.shar
 __device__ __forceinline__ F2 ldg_now2(const void* p) {
   F2 v;
   asm volatile("ld.global.cg.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ldg_now4(const void* p) {
-  float4 v;
-  asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ F2 unpack_bf16(uint32_t v) { return make_float2(bf16_lo(v), bf16_hi(v)); }
@@ -212,7 +212,6 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
   const int NS = p.NS;
   const uint32_t barL = base0 + SM::BAR, barG = barL + 8, barD = barL + 16, barU = barL + 24;
   int* const s_item = reinterpret_cast<int*>(mlp_bwd_smem + SM::BAR + 32);
-  const uint32_t* const s_tmem = reinterpret_cast<const uint32_t*>(mlp_bwd_smem + SM::BAR + 36);
   if ((base0 & 1023u) != 0) {  // (the tiles need it; dynamic shared memory starts there when there is no static one)
     if (threadIdx.x == 0) report_timeout(p.status, 2, 0);
     return;
@@ -234,12 +233,10 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
   tmem_fence_before_sync();
   __syncthreads();
   tmem_fence_after_sync();
-  const uint32_t tmem = *s_tmem;
-  const float te_last = ld_as_float<T>(p.token_eta, CS - 1);
-  // the masters of W1, W2 are carried divided by wscale = -te15, so that a stage's update accumulates directly (te15 = 0:
-  // they never move)
-  const bool w_moves = te_last != 0.f;
-  const float wscale = w_moves ? -te_last : 1.f;
+  const auto tmem = [&]() { return lds_u(base0 + SM::BAR + 36); };  // (read where it is used, like te15: a register less across the stage loop)
+  const auto te15 = [&]() { return lds_f(base0 + SM::TE + 4 * (CS - 1)); };
+  // the masters of W1, W2 are carried divided by -te15, so that a stage's update accumulates directly (te15 = 0: they never
+  // move)
   if (threadIdx.x < CS) sts_f(base0 + SM::TE + 4 * threadIdx.x, ld_as_float<T>(p.token_eta, threadIdx.x));
 
   const int nitems = p.nstreams * p.NCH;
@@ -302,39 +299,37 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       const int tid = threadIdx.x;
       const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
       if (tid < 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_G1P + 128 * tid));
-      else if (tid < 64 + 76) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_Z2 + 128 * (tid - 64)));
+      else if (tid < 64 + (MLP_REC_BYTES - MLP_REC_Z2) / 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_Z2 + 128 * (tid - 64)));
     };
-    // what a thread reads of a stage by itself: its pair of Z2 and Zb2 and the row's statistics, its hidden columns of b1
-    F2 zz, zzb, b1v[2], st2;
-    float4 st1;
-    auto load_first = [&](int s) {
+    // what a thread reads of a stage by itself: its pair of Z2 and Zb2 and the row's means, its hidden columns of b1
+    F2 zz, zzb, b1v[2], means;
+    float ln_row;  // Z2's row, lanes 8 i ..: the two means of its LayerNorm gradient, 1 / std, mean
+    auto load_z2 = [&](int s) {
       TTT_PLACE
-      const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
-      zz = ldg_now2(rec + MLP_REC_Z2 + 8 * tid);
-      st1 = ldg_now4(rec + MLP_REC_STAT + 32 * warp);
+      zz = ldg_now2(rec0 + (size_t)s * MLP_REC_BYTES + MLP_REC_Z2 + 8 * tid);
     };
     auto load_own = [&](int s) {
-      load_first(s);
+      load_z2(s);
       TTT_PLACE
       const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
       zzb = ldg_now2(rec + MLP_REC_ZB2 + 8 * tid);
+      means = ldg_now2(rec + MLP_REC_MEAN + 8 * warp);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) b1v[nt] = ldg_now2(rec + MLP_REC_B1 + 8 * (8 * warp + 4 * nt + t));
-      st2 = ldg_now2(rec + MLP_REC_STAT + 32 * warp + 16);
     };
     auto put_rates = [&](int buf, float lr) {  // 16 lanes
       const int lane = threadIdx.x & 31;
       sts_f(base0 + SM::LR + buf * CS * 4 + 4 * lane, lr);
-      sts_f(base0 + SM::LR + (2 + buf) * CS * 4 + 4 * lane, te_last * lr);
+      sts_f(base0 + SM::LR + (2 + buf) * CS * 4 + 4 * lane, te15() * lr);
     };
     // W1_s, W2_s from W1_{s+1}, W2_{s+1} (inputs of stage s in buffer `buf`): one thread
     auto undo_updates = [&](int buf) {
-      if (!w_moves) return;
-      const uint32_t k = base0 + SM::IN + buf * 3 * TL + TL;
+      if (te15() == 0.f) return;
+      const uint32_t k = base0 + SM::IN + buf * 3 * TL + TL, tm = tmem();
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        umma_update(tmem + 64 * h, base0 + SM::G1P + h * 2 * TL, k, UPD_IDESC | UPD_NEGATE);
-        umma_update(tmem + 128 + 64 * h, base0 + SM::X2 + buf * ET + h * 2 * TL, base0 + SM::G2P, UPD_IDESC | UPD_NEGATE);
+        umma_update(tm + 64 * h, base0 + SM::G1P + h * 2 * TL, k, UPD_IDESC | UPD_NEGATE);
+        umma_update(tm + 128 + 64 * h, base0 + SM::X2 + buf * ET + h * 2 * TL, base0 + SM::G2P, UPD_IDESC | UPD_NEGATE);
       }
     };
 
@@ -363,7 +358,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
             if (P.mi() < 2 || !fresh) f = __ldcg(src + ((h * 4 + (warp & 3)) * 16 + cc * 8 + j) * 32);
             v[j][0] = f.x; v[j][1] = f.y; v[j][2] = f.z; v[j][3] = f.w;
           }
-          tmem_st_8x4(P.tm(tmem) + 64 * h + 32 * cc, v);
+          tmem_st_8x4(P.tm(tmem()) + 64 * h + 32 * cc, v);
         }
       tmem_wait_st();
       if (tid < 2 * HD) sts_f(base0 + SM::LN + 4 * tid, ld_as_float<T>(tid < HD ? p.ln_g : p.ln_b, (size_t)head * HD + (tid & (HD - 1))));
@@ -376,8 +371,8 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
     __syncthreads();
     // bf16 copy of half a master (128 hidden features; this warp's 32) to its operand matrix
     auto convert = [&](const Place& P, int mat, int half) {
-      const float sc = mat < 2 ? wscale : 1.f;
-      const uint32_t src = tmem + ((32u * (uint32_t)(P.warp & 3)) << 16) + 128 * mat + 64 * half;
+      const float te = te15(), sc = mat < 2 && te != 0.f ? -te : 1.f;
+      const uint32_t src = tmem() + ((32u * (uint32_t)(P.warp & 3)) << 16) + 128 * mat + 64 * half;
       const uint32_t dst = base0 + SM::W1 + mat * SM::WM + (128 * half + 32 * (P.warp & 3) + P.lane) * 128;
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
@@ -398,20 +393,30 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       }
     };
     // What a stage needs before its first barrier and does not take from the stage after it; `b`: its input buffer.
-    //  * both LayerNorms, a row per warp: G2 and dZb2 as bf16 pairs
+    //  * both LayerNorms, a row per warp: G2 and dZb2 as bf16 pairs.  Variances are sums of squared deviations: with the forward's
+    //    E[z^2] - mean^2, rows whose mean is 100 standard deviations had gradients 2e-2 off (8e-3 this way; 1.3 % of the kernel's time)
     uint32_t g2_pair, dzb_pair;
+    F2 rstds;
+    auto row_stats = [&]() {
+      const F2 xc = f2add(zz, f2(-means.x)), bc = f2add(zzb, f2(-means.y));
+      const F2 var = f2mul(warp_sum2(f2hsum(f2mul(xc, xc)), f2hsum(f2mul(bc, bc))), f2(1.f / HD));
+      rstds = f2(rsqrtf(var.x + p.eps), rsqrtf(var.y + p.eps));
+    };
     auto rows_of = [&](int b) {
       if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
       TTT_PLACE
       const uint32_t in = base0 + SM::IN + b * 3 * TL;
       const F2 gam = lds_f2(base0 + SM::LN + 4 * rc), bet = lds_f2(base0 + SM::LN + 4 * (HD + rc));
       const F2 vv = ld_pair<T>(base0 + SM::V, warp, rc), kk = ld_pair<T>(in + TL, warp, rc), dd = ld_pair<T>(in + 2 * TL, warp, rc);
-      const F2 xh = f2mul(f2add(zz, f2(-st1.x)), f2(st1.y));
-      const F2 xb = f2mul(f2add(zzb, f2(-st2.x)), f2(st2.y)), tt = f2mul(dd, gam);
-      const F2 gy = f2sub(f2fma(gam, xh, bet), f2sub(vv, kk));
-      const F2 sums = warp_sum2(f2hsum(tt), f2hsum(f2mul(tt, xb)));
-      const F2 G = f2mul(f2fma(xh, f2(-st1.w), f2fma(gy, gam, f2(-st1.z))), f2(st1.y));
-      const F2 dzb = f2mul(f2fma(xb, f2(sums.y * (-1.f / HD)), f2add(tt, f2(sums.x * (-1.f / HD)))), f2(st2.y));
+      const F2 xh = f2mul(f2add(zz, f2(-means.x)), f2(rstds.x)), xb = f2mul(f2add(zzb, f2(-means.y)), f2(rstds.y));
+      const F2 gxh = f2mul(f2sub(f2fma(gam, xh, bet), f2sub(vv, kk)), gam), tt = f2mul(dd, gam);
+      const float m = warp_sum4_spread(f2hsum(gxh), f2hsum(f2mul(gxh, xh)), f2hsum(tt), f2hsum(f2mul(tt, xb))) * (1.f / HD);
+      float mi[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mi[i] = __shfl_sync(0xffffffffu, m, 8 * i);
+      const F2 G = f2mul(f2fma(xh, f2(-mi[1]), f2add(gxh, f2(-mi[0]))), f2(rstds.x));
+      const F2 dzb = f2mul(f2fma(xb, f2(-mi[3]), f2add(tt, f2(-mi[2]))), f2(rstds.y));
+      ln_row = lane < 16 ? m : lane < 24 ? rstds.x : means.x;
       dgam = f2fma(dd, xb, dgam);
       dbet = f2add(dbet, dd);
       g2_pair = pack_bf16(G.x, G.y);
@@ -464,6 +469,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
     __syncwarp();
     if (threadIdx.x >> 5 == 8) causal_first(s, buf);
     if (threadIdx.x >= 256) second_layer_copies();
+    row_stats();
     rows_of(buf);
 
     while (true) {
@@ -639,7 +645,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       // ---- I3. Contractions over the hidden features that the chain waits for: dH W2 - l o (X2 dW2) (four partial sums), and
       //      the causal matrices A2 = X2b X2^T, dZ1b G1^T (eight warps, a quarter of one of them each)
       float dell_row;
-      load_first(s);  // Z2's LayerNorm once more, for I4
+      load_z2(s);  // Z2's LayerNorm once more, for I4
       {
         TTT_PLACE
         const uint32_t a_off = P.a_off();
@@ -700,8 +706,8 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
         const F2 bet = lds_f2(sLN + 4 * (HD + rc)), vk = f2sub(ld_pair<T>(base + SM::V, warp, rc), ld_pair<T>(tk, warp, rc));
         const float lr_j = lds_f(sLR + 4 * warp), ell_j = lds_f(sELL + 4 * warp);
         const F2 db2v = lds_f2(sDB2 + 4 * rc), gam = lds_f2(sLN + 4 * rc);
-        const float rs = st1.y, sg = st1.z, sgx = st1.w;
-        const F2 xh = f2mul(f2add(zz, f2(-st1.x)), f2(rs)), gy = f2sub(f2fma(gam, xh, bet), vk);  // its output minus the target
+        const float rs = __shfl_sync(0xffffffffu, ln_row, 16), sg = __shfl_sync(0xffffffffu, ln_row, 0), sgx = __shfl_sync(0xffffffffu, ln_row, 8);
+        const F2 xh = f2mul(f2add(zz, f2(-__shfl_sync(0xffffffffu, ln_row, 24))), f2(rs)), gy = f2sub(f2fma(gam, xh, bet), vk);  // its output minus the target
         const F2 gxh = f2mul(gy, gam), G = f2mul(f2fma(xh, f2(-sgx), f2add(gxh, f2(-sg))), f2(rs));
         F2 dg2 = f2mul(db2v, f2(-ell_j));
 #pragma unroll
@@ -801,7 +807,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
           tmem_fence_after_sync();
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint32_t d1 = tmem + 256 + 64 * h, d2 = d1 + 128, o = h * 2 * TL;
+            const uint32_t d1 = tmem() + 256 + 64 * h, d2 = d1 + 128, o = h * 2 * TL;
             umma_update(d1, base + SM::DZ1B + o, tq, UPD_IDESC);
             umma_update(d1, base + SM::DZ1 + o, tk, UPD_IDESC);
             umma_update(d2, tx2 + o, base + SM::DZ2, UPD_IDESC);
@@ -817,6 +823,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
         }
         __syncwarp();
       }
+      if (s > s_lo) row_stats();
       if (threadIdx.x < 128) {
         TTT_PLACE
         const uint32_t a_off = P.a_off();
@@ -890,7 +897,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
             lr = lds_f(sLR + 4 * lane);
 #pragma unroll
             for (int j = 0; j < CS; ++j) dte += lds_f(sDET + 4 * (17 * lane + j));
-            st_from_float<T>(p.d_lr, row_base + (size_t)s * CS + lane, lds_f(base + SM::DLP + 4 * lane) + dell * te_last);
+            st_from_float<T>(p.d_lr, row_base + (size_t)s * CS + lane, lds_f(base + SM::DLP + 4 * lane) + dell * te15());
           }
           const float sum = warp_sum(dell * lr);
           if (lane < CS) p.part_te[(size_t)row_base + (size_t)s * CS + lane] = lane == CS - 1 ? dte + sum : dte;
@@ -939,7 +946,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           float v[8][4];
-          tmem_ld_8x4(P.tm(tmem) + 64 * h + 32 * cc, v);
+          tmem_ld_8x4(P.tm(tmem()) + 64 * h + 32 * cc, v);
           const int e = 128 * h + 32 * (warp & 3) + lane;
           if (!last) {
             float4* dst = reinterpret_cast<float4*>(ws + P.mi() * HD * MB_E) + lane;
@@ -993,7 +1000,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       if (mbar_try_wait(barL, nload & 1) && mbar_try_wait(barG, nload & 1) && mbar_try_wait(barU, nmma & 1)) break;
   tmem_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x < 32) tmem_dealloc(tmem, 512);
+  if (threadIdx.x < 32) tmem_dealloc(tmem(), 512);
 }
 
 // grad_token_eta[t] = sum over streams, grad_ln_weight / grad_ln_bias [h][f] = sum over the batch; fixed order.  Block =

@@ -421,9 +421,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
            a0, a1);
       xsel ^= 1;
       const float A[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)}, Bv[2] = {a0.y * (1.f / HD), a1.y * (1.f / HD)};
-      if (SAVE && warp == 0 && t < 2)
-        *reinterpret_cast<float4*>(rec + MLP_REC_STAT + 32 * (g + 8 * t)) =
-            t == 0 ? make_float4(mean[0], rstd[0], A[0], Bv[0]) : make_float4(mean[1], rstd[1], A[1], Bv[1]);
+      if (SAVE && warp == 0 && t < 2) *reinterpret_cast<float*>(rec + MLP_REC_MEAN + 8 * (g + 8 * t)) = t == 0 ? mean[0] : mean[1];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         g2p[r] = f2mul(f2fma(x[r], f2(-Bv[r]), f2sub(gg[r], f2(A[r]))), f2(rstd[r] * lr_row[r]));
@@ -547,9 +545,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
       const float mean[2] = {a0.x * (1.f / HD), a1.x * (1.f / HD)};
       const float rstd[2] = {rsqrtf(fmaxf(a0.y * (1.f / HD) - mean[0] * mean[0], 0.f) + p.eps),
                              rsqrtf(fmaxf(a1.y * (1.f / HD) - mean[1] * mean[1], 0.f) + p.eps)};
-      if (SAVE && warp == 1 && t < 2)
-        *reinterpret_cast<float2*>(rec + MLP_REC_STAT + 32 * (g + 8 * t) + 16) =
-            t == 0 ? make_float2(mean[0], rstd[0]) : make_float2(mean[1], rstd[1]);
+      if (SAVE && warp == 1 && t < 2) *reinterpret_cast<float*>(rec + MLP_REC_MEAN + 8 * (g + 8 * t) + 4) = t == 0 ? mean[0] : mean[1];
       const uint32_t so = base + SM::OFF_OUT + (n & 1) * TL;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
