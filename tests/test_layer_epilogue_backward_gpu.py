@@ -32,3 +32,12 @@ def test_epilogue_gradients(dtype, B, H, T, F, gate):
     for a, r in zip(got, want):
         assert torch.isfinite(a).all()
         assert (a.float() - r).norm() <= tol * r.norm() + 1e-6
+
+
+@pytest.mark.parametrize("gate", [False, True])
+@pytest.mark.parametrize("dtype,H,F", [
+    (torch.bfloat16, 1, 32), (torch.bfloat16, 4, 32), (torch.bfloat16, 5, 32), (torch.bfloat16, 7, 64), (torch.bfloat16, 18, 32),
+    (torch.bfloat16, 19, 32), (torch.bfloat16, 23, 32), (torch.bfloat16, 24, 32), (torch.float32, 7, 64), (torch.float32, 13, 64)])
+def test_tile_rules(dtype, H, F, gate):
+    """The widths on both sides of each line of the rule for groups, rows and threads, on a tile and a ragged rest."""
+    test_epilogue_gradients(dtype, 2, H, 29, F, gate)

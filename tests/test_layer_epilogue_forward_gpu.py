@@ -25,3 +25,12 @@ def test_epilogue(dtype, B, H, T, F, gate):
         want = want * torch.nn.functional.gelu(g[:, :C].float(), approximate="tanh").reshape(B, T, C)
     tol = 1e-2 if dtype == torch.bfloat16 else 1e-5
     assert (y.float() - want).norm() <= tol * want.norm()
+
+
+@pytest.mark.parametrize("gate", [False, True])
+@pytest.mark.parametrize("dtype,H,F", [
+    (torch.bfloat16, 1, 32), (torch.bfloat16, 4, 32), (torch.bfloat16, 5, 32), (torch.bfloat16, 7, 64), (torch.bfloat16, 18, 32),
+    (torch.bfloat16, 19, 32), (torch.bfloat16, 23, 32), (torch.bfloat16, 24, 32), (torch.float32, 7, 64), (torch.float32, 13, 64)])
+def test_tile_rules(dtype, H, F, gate):
+    """The widths on both sides of each line of the rule for groups, rows and threads, on a tile and a ragged rest."""
+    test_epilogue(dtype, 2, H, 29, F, gate)

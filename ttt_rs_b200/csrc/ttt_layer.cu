@@ -432,13 +432,21 @@ static cudaError_t launch_epi_g(LayerEpiParams p, cudaStream_t st) {
   const int C = p.H * FD, nch = C / (16 / (int)sizeof(T));
   constexpr int TT = 64 / MAXCH, MAXT = MAXCH == 16 ? 512 : EPI_THREADS;
   auto kfn = ttt_layer_epilogue_kernel<T, MAXCH, FD, GATE>;
-  // as many row groups as fit a CTA, a tile of a row per warp, of groups that divide its rows evenly (65536 x 512, bf16: 39.8 us
-  // with 6 groups of 16 rows, 35.8 with 4; 65536 x 768: 45.1 us with 12 warps for 16 rows, 43.5 for 12)
+  // Row groups g, rows of a tile, threads.  128 MB of input, bf16 / bf16 gated, us (g, rows, threads):
+  //   up to 72 chunks (four groups use the threads that a row per warp wants): 448 features (4, 16, 224) 72 / 140, (1, 11, 64)
+  //     78 / 166, (6, 12, 384) 78 / 154; 64 features (4, 16, 32) 227 / 302, (4, 4, 32) 246 / 320, (16, 16, 128) 244 / 319
+  //   up to 95: two groups, 640 features (2, 12, 160) 64 / 132, (4, 16, 320) 69 / 141; 704 (2, 12, 192) 62 / 138, (1, 11, 96) 65 / 153
+  //   more: whole blocks of a warp per row, 768 features (4, 12, 384) 59 / 124, (4, 16, 384) 63 / 125; float32, 448 features
+  //     (3, 12, 384) 48 / 91, (1, 11, 128) 54 / 114
+  // Rows of more than 512 bytes x 4 (TT < 16): as many groups as fit, a row per warp.
   p.row_groups = MAXT / nch < TT ? MAXT / nch : TT;
-  p.tile_rows = (p.row_groups * nch + 31) / 32 < TT ? (p.row_groups * nch + 31) / 32 : TT;
-  if (p.row_groups > p.tile_rows) p.row_groups = p.tile_rows;
-  while (p.tile_rows % p.row_groups) --p.row_groups;
-  const int threads = (p.row_groups * nch + 31) & ~31;
+  int threads = (p.row_groups * nch + 31) & ~31;
+  p.tile_rows = threads / 32 < TT ? threads / 32 : TT;
+  if (TT == 16) {
+    p.row_groups = nch <= 72 ? 4 : nch < 96 ? 2 : MAXT / nch;
+    p.tile_rows = nch <= 72 ? 16 : 12;
+    threads = nch < 96 ? (p.row_groups * nch + 31) & ~31 : MAXT;
+  }
   const size_t smem = 2 * (size_t)p.tile_rows * C * sizeof(T) + p.tile_rows * sizeof(float2);
   static DeviceValue resident;
   int per_sm = 1;
@@ -854,11 +862,14 @@ static cudaError_t launch_epi_bwd_g(LayerEpiBwdParams p, cudaStream_t st) {
   const int C = p.H * FD, nch = C / (16 / (int)sizeof(T));
   constexpr int TT = (GATE ? 32 : 64) / MAXCH, MAXT = MAXCH == 16 ? 512 : EPI_BWD_THREADS;
   auto kfn = ttt_layer_epilogue_bwd_kernel<T, MAXCH, FD, GATE>;
-  // as many row groups as fit a CTA, but no more than a tile has rows
+  // as many row groups as fit a CTA, but no more than a tile has rows, and with a gate a warp for each of them (the row phase is
+  // bound by tanh; 128 MB of bf16 input: 64 features 1397 us with 64 threads for 8 rows, 872 with 256)
   p.row_groups = MAXT / nch < TT ? MAXT / nch : TT;
-  const int threads = (p.row_groups * nch + 31) & ~31;
-  // a row of the tile per warp where the tile is not smaller than that (twelve warps of sixteen rows took two turns)
-  p.tile_rows = threads / 32 < TT ? threads / 32 : TT;
+  int threads = (p.row_groups * nch + 31) & ~31;
+  if (GATE && threads < 32 * TT) threads = 32 * TT;
+  // a row of the tile per warp where the tile is not smaller than that (twelve warps of sixteen rows took two turns), unless a
+  // row has so few chunks that the column phase would run on a part of the block (64 features: 552 us with 4 rows, 445 with 16)
+  p.tile_rows = threads / 32 < TT && nch > 16 ? threads / 32 : TT;
   if (p.row_groups > p.tile_rows) p.row_groups = p.tile_rows;
   const size_t smem = 4 * (size_t)p.tile_rows * C * sizeof(T) + p.tile_rows * sizeof(float4) +
                       (size_t)(GATE ? p.tile_rows + 1 : 1) * C * sizeof(float);
