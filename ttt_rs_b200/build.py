@@ -7,6 +7,7 @@
 from __future__ import annotations
 
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -25,6 +26,19 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
 ]
+# Kernels whose groups of warps split the launch's registers among themselves (setmaxnreg): registers per thread that the
+# splits add up to.  With fewer at launch a group would wait for registers that do not exist.
+REGISTER_SPLITS = {"ttt_linear_bwd_f32.cu": ("ttt_linear_bwd_f32_kernel", 128)}
+
+
+def check_register_split(src: str, log: str) -> None:
+    """Raises unless every instantiation of `src`'s splitting kernel has exactly its registers in ptxas's report `log`."""
+    if src not in REGISTER_SPLITS:
+        return
+    kernel, want = REGISTER_SPLITS[src]
+    used = [int(n) for name, n in re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", log, re.S) if kernel in name]
+    if not used or any(n != want for n in used):
+        raise RuntimeError(f"{src}: {kernel} must be built with {want} registers per thread, ptxas reports {used}")
 
 
 def find_nvcc() -> str:
@@ -113,6 +127,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         log.append(f"== {src}\n{out}")
         if pr.returncode != 0:
             raise RuntimeError(f"nvcc failed on {src}:\n{out}")
+        check_register_split(src, out)
     cmd = [nvcc, "-shared", "-o", str(LIB), *objs]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:

@@ -956,7 +956,8 @@ static cudaError_t launch_t(const CUtensorMap* m, LinBwdParams& p, int nstreams,
   static DeviceValue ready;
   int bytes = 0, sms = 0;
   cudaError_t e = ready.get(0, &bytes, [&](int* n) {
-    // the groups' shares of the registers add up to those of the launch
+    // the groups' shares of the registers add up to those of the launch (the build fails otherwise; a library built in another
+    // way must not wait for registers that do not exist)
     cudaFuncAttributes fa;
     const cudaError_t a = cudaFuncGetAttributes(&fa, kfn);
     if (a != cudaSuccess) return a;
