@@ -58,7 +58,6 @@ namespace ttt {
 constexpr int GEMM_BM = 128, GEMM_BN = 256, GEMM_BK = 64;
 constexpr uint32_t GEMM_A_BYTES = GEMM_BM * GEMM_BK * 2;  // 16 KB: the A tile of a stage
 constexpr uint32_t GEMM_B_BYTES = GEMM_BN * GEMM_BK * 2;  // 32 KB: the B tile of a stage
-constexpr uint32_t GEMM_STAGE_BYTES = GEMM_A_BYTES + GEMM_B_BYTES;
 constexpr uint32_t GEMM_STG_BYTES = GEMM_BM * 64 * 2;     // 16 KB: one [128][64] bf16 staging tile of the epilogue
 constexpr int GEMM_THREADS = 192;
 

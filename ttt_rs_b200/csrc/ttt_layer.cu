@@ -610,7 +610,6 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_BWD_THREADS, (sizeof(T
   constexpr int HD = FD;  // features per head in this instantiation
   const int TT = p.tile_rows;
   constexpr int EPC = 16 / sizeof(T);
-  constexpr int CPR = HD / EPC;
   extern __shared__ __align__(16) uint8_t epi_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int H = p.H, NT = p.T, C = H * HD;

@@ -84,14 +84,8 @@ __device__ __forceinline__ void umma_commit_to(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void ldsm_x2_trans(uint32_t (&r)[2], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-}
 __device__ __forceinline__ void mma4(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   mma_bf16(c, a[0], a[1], a[2], a[3], b0, b1);
-}
-__device__ __forceinline__ void stsm_x4(uint32_t addr, const uint32_t (&r)[4]) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts_f(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
@@ -563,7 +557,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
               own[2 * nt + r] = pack_bf16(g1.x, g1.y);
               del[r] += f2hsum(f2fma(g1, pr(u1[nt], r), f2mul(pr(gl2[nt], r), unpack_bf16(x2[2 * nt + r]))));
             }
-          stsm_x4(base + SM::G1 + e_off, own);
+          stsm_x4(base + SM::G1 + e_off, own[0], own[1], own[2], own[3]);
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             del[r] = quad_sum(del[r]);
@@ -611,8 +605,8 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
             dx[nt][2 * r] = -ell[r] * gl2[nt][2 * r];
             dx[nt][2 * r + 1] = -ell[r] * gl2[nt][2 * r + 1];
           }
-        stsm_x4(base + SM::X2B + e_off, own);
-        stsm_x4(base + SM::DZ1B + e_off, own2);
+        stsm_x4(base + SM::X2B + e_off, own[0], own[1], own[2], own[3]);
+        stsm_x4(base + SM::DZ1B + e_off, own2[0], own2[1], own2[2], own2[3]);
         __syncwarp();
         {
           const uint32_t ad2t[4] = {movm_t(ad2[0]), movm_t(ad2[2]), movm_t(ad2[1]), movm_t(ad2[3])};
@@ -638,7 +632,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
           }
           db1v[nt] = f2add(db1v[nt], f2(cs[0], cs[1]));
         }
-        stsm_x4(base + SM::DH + e_off, own);
+        stsm_x4(base + SM::DH + e_off, own[0], own[1], own[2], own[3]);
       }
       __syncthreads();  // 2
 
@@ -785,7 +779,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
             const F2 d = f2fma(pr(dx[nt], r), gd1[nt][r], dz1a[nt][r]);
             own[2 * nt + r] = pack_bf16(d.x, d.y);
           }
-        stsm_x4(base + SM::DZ1 + e_off, own);
+        stsm_x4(base + SM::DZ1 + e_off, own[0], own[1], own[2], own[3]);
         fence_proxy_async_smem();  // every operand tile of the products below has been written by now
         __syncwarp();
         ldsm_x4_t(tb, base + SM::DZ1 + e_off);

@@ -574,8 +574,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     tmem_st_8x4(tm_w1 + 32u, w1t[1]);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      // float32 column sums, like the reference; the backward's reverse walk subtracts the sums of the bf16 operand
-      // values instead, which moves the recovered biases by rounding noise only (~1e-3 of one stage's step)
+      // float32 column sums, like the reference
       const F2 cs = f2add(g1p[j][0], g1p[j][1]);
       b1v[j] = f2fma(f2(col_sum(cs.x), col_sum(cs.y)), f2(-te15), b1v[j]);
     }

@@ -62,15 +62,6 @@ __device__ __forceinline__ void st_pair<float>(uint32_t tile, int row, int col, 
   asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(tile + off_f32(row, col)), "f"(x), "f"(y) : "memory");
 }
 
-// Write an element pair into operand planes (bf16 planes at `planes`, plane stride 2048).
-template <int NP>
-__device__ __forceinline__ void st_pair_planes(uint32_t planes, int row, int col, float x, float y) {
-  const Pk<NP> v = split_pack<NP>(x, y);
-  const uint32_t a = planes + off_bf16(row, col);
-#pragma unroll
-  for (int p = 0; p < NP; ++p) asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + p * TILE_BF16_BYTES), "r"(v.p[p]) : "memory");
-}
-
 // f32 only: split a raw float tile into its three bf16 operand planes. All 128 threads take part.
 __device__ __forceinline__ void split_tile_f32(uint32_t tile, int tid) {
   const int row = tid >> 3, c0 = (tid & 7) << 3;
