@@ -183,3 +183,46 @@ def test_rows_off_their_centre():
         err = ((got[k].double() - want[k]).norm() / want[k].norm()).item()
         print(f"{k}: {err:.2e}")
         assert err < 7e-3, f"{k}: {err}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("from_forward", (False, True))
+@pytest.mark.parametrize("B,H,NS,te_scale,bound", ((1, 3, 9, 0.0, 1e-2), (1, 3, 24, 0.7, 1e-2), (1, 4, 512, 1.0, 2e-2)))
+def test_step_scales_and_many_stages(B, H, NS, te_scale, bound, from_forward):
+    """The masters of W1, W2 are carried divided by -token_eta[15] and undone stage by stage: token_eta[15] = 0 (nothing moves and
+    nothing is undone), a token_eta[15] that is no power of two (bf16(0.7 / 16): the division rounds), and 512 stages.
+    bf16 operands give gradients 2e-3 to 4e-3 off (2-norm; 1e-2 is the bf16 tolerance of these tests' L2 errors); over 512 stages
+    the state's own rounding comes back through the chain, up to 1e-2 (grad_b1).  Where the undone state has drifted longest, in
+    the first four stages, the gradients of the tokens are held to the bound of a short sequence."""
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    t = _case(B, H, NS * 16, 200 + NS)
+    te = t["token_eta"].float().view(-1, 16)
+    if te_scale == 0.0:
+        te[:, 15] = 0.0
+    else:
+        te = te * te_scale
+    t["token_eta"] = te.reshape(-1).to(torch.bfloat16)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 128, 1)
+    d = {k: v.to(dev) for k, v in t.items()}
+    st = tb.TTTMLPState(d["w1"], d["b1"], d["w2"], d["b2"])
+    ws = None
+    if from_forward:
+        ws = tb.mlp_backward_workspace(d["xq"], cfg)
+        tb.fused_ttt_mlp_forward(d["xq"], d["xk"], d["xv"], st, d["token_eta"], d["ttt_lr_eta"], d["ln_weight"],
+                                 d["ln_bias"], cfg, backward_workspace=ws)
+    g = tb.fused_ttt_mlp_backward(d["xq"], d["xk"], d["xv"], st, d["token_eta"], d["ttt_lr_eta"], d["ln_weight"],
+                                  d["ln_bias"], d["grad_output"], cfg, workspace_from_forward=ws)
+    torch.cuda.synchronize()
+    tb.check_mlp_status(g)
+    want = O.ttt_mlp_backward_autograd(*[d[k].double() for k in MLP_IN], d["grad_output"].double())
+    for k in ("grad_xq", "grad_xk", "grad_xv", "grad_w1", "grad_b1", "grad_w2", "grad_b2", "grad_ttt_lr_eta",
+              "grad_ln_weight", "grad_ln_bias"):
+        err = ((g[k].double() - want[k]).norm() / want[k].norm()).item()
+        print(f"{k}: {err:.2e}")
+        assert err < bound, f"{k}: {err}"
+    for k in ("grad_xq", "grad_xk", "grad_xv"):
+        a, b = g[k][:, :, :64].double(), want[k][:, :, :64]
+        err = ((a - b).norm() / b.norm()).item()
+        print(f"{k}, first stages: {err:.2e}")
+        assert err < 1e-2, f"{k}, first stages: {err}"
