@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
 // its rows asynchronously to a [TT][H*F] tile in shared memory.  Row phase: a warp per row takes mean and variance (two
 // sweeps over registers).  Column phase: a thread per 16-byte chunk of columns and row group, its weights and biases in
 // registers, applies the norm and the optional gate and stores to [B,T,H*F].  Bound by shared-memory and issue slots before
-// memory: 65536 tokens, bf16: 55.6 -> 49.3 us at 768 features, 118 -> 93 us at 2048; gated 289 -> 233 us, float32 gated
-// 678 -> 327 us at 2048 (a warp that also wrote its row read 4 to 16 KB of weights and biases for it from shared memory).
+// memory: 65536 tokens, bf16: 55.6 -> 49.3 -> 45 us at 768 features (the last with tiles of a row per warp), 118 -> 93 us at
+// 2048; gated 289 -> 233 us, float32 gated 678 -> 327 us at 2048 (a warp that also wrote its row read 4 to 16 KB of weights and
+// biases for it from shared memory).
 // CTAs per SM: one fewer for float32 without a gate, which is at 0.9 of the memory rate with two (67 against 76 us at 768).
 // MAXCH: 16-byte chunks of one row per lane (rows of up to 32 * MAXCH chunks = 512 * MAXCH bytes).
 constexpr int EPI_THREADS = 384;
@@ -600,8 +601,9 @@ __global__ void __launch_bounds__(PRO_THREADS, sizeof(T) == 2 ? 3 : 1) ttt_layer
 // shuffles (the mean; then the variance and both sums of dx together).  Column phase: a thread per 16-byte chunk of columns
 // and row group, which writes dz straight to [B,H,T,F] and keeps its columns' parameter sums in registers over all of the
 // CTA's tiles; the row groups meet in shared memory at the end and leave one [2][C] row of `partials` per CTA.
-// 65536 tokens x 768, bf16: 187 -> 86 -> 71 us without a gate (the last step: packed arithmetic, tiles of a row per warp, no divisions), 359 -> 208 us with one; float32 409 -> 104 us (the parameter sums
-// were a kernel of their own that read both operands again).  TT: with a gate (whose row phase is bound by tanh) half, so
+// 65536 tokens x 768, bf16: 187 -> 86 -> 72 us without a gate (the last step: packed arithmetic, tiles of a row per warp, no
+// divisions), 359 -> 208 us with one; float32 409 -> 104 us (the parameter sums were a kernel of their own that read both
+// operands again).  TT: with a gate (whose row phase is bound by tanh) half, so
 // that the tanh values that the column phase uses again fit beside two CTAs' tiles.
 constexpr int EPI_BWD_THREADS = 384;
 template <typename T, int MAXCH, int FD, bool GATE>

@@ -10,7 +10,7 @@
 //   chain   (warps 4..7): K dW, the second derivative, dZ1, dW += dZbar^T Q + dZ1^T K, the bias gradient;
 //   output  (warps 8..11): dq, dk, dv and the token_eta terms from the copies of W, dW, dZbar and dZ1 that the others leave;
 //   prepare (warps 12..15): split of float32 tiles into bf16 planes and Q K^T (three warps), the copies (one lane).
-// 64 stages, us, in one group / in four: 96 streams 419 / 309, 12 streams 411 / 296, 192 streams 617 / 552, 384 1134 / 997.
+// 64 stages, us, in one group / in four: 96 streams 419 / 309, 12 streams 411 / 297, 192 streams 617 / 537, 384 1134 / 995.
 // The chain group is what the others wait for (9.0 k of 9.3 k cycles a stage, 550 mma.sync per scheduler among them).  The
 // same split of a bf16 stage is slower than the one group from 12 streams (138 / 132 us) to 1024 (1185 / 667): its products
 // take a sixth, and four programs of 25 KB together miss in the instruction cache (3.4 of 12.7 stalled warps).

@@ -483,9 +483,9 @@ cudaError_t launch_linear_fwd(int dtype, int seg, int mb, const CUtensorMap* map
   const cudaError_t e = device_sms(&sms);
   if (e != cudaSuccess) return e;
   // Streams that have an SM each: a stage's work on three groups of warps, where a lone group of four leaves the SM waiting for
-  // its chain (64 stages, us, this form / three groups: bf16 148 streams 72.4 / 62.3, f32 188 / 163).  From there on streams
-  // share SMs and fill one another's waits, and the three groups' registers let in one block only (192 streams: 86 / 120,
-  // f32 248 / 314).  A few stages cost the same either way.
+  // its chain (64 stages, inference, us, this form / three groups: bf16 148 streams 68.4 / 60.1, f32 186 / 163).  From there on
+  // streams share SMs and fill one another's waits, and the three groups' registers let in one block only (192 streams: 82 / 116,
+  // f32 244 / 319).  A few stages cost the same either way.
   if (nstreams <= sms) return launch_linear_fwd_roles(dtype, seg, mb, maps, p, nstreams, st);
   if (seg == 32) {
     if (dtype == 1) return launch_fwd_mb<__nv_bfloat16, 32>(mb, maps, p, nstreams, st);

@@ -4,8 +4,9 @@
 //
 // Of a stage only W -> Z1 -> LayerNorm gradient -> W is a chain from one stage to the next; the output of the stage (its
 // second product with W, the causal matrix, the second LayerNorm) hangs off it.  With one stream on an SM nothing else
-// fills the chain's waits, and a group that does all of it adds the rest to every stage (64 stages, 12 to 148 streams: bf16
-// heads of 64 71-73 us in one group, 60-62 in three; pairs of 32-wide heads 81 and 60-62; f32 188 and 160-170).  So:
+// fills the chain's waits, and a group that does all of it adds the rest to every stage (64 stages, 12 to 148 streams, one group
+// and three, inference: bf16 heads of 64 68 us and 58-60; pairs of 32-wide heads 74 and 61-62; f32 185 and 152-163; saving
+// state for the backward: 73-74 and 66; 81-83 and 66-68; 191-193 and 163-171).  So:
 //   chain  (warps 0..3): W^T in its accumulator registers; publishes the stage's W as operand fragments and the bias, forms
 //          Z1, its LayerNorm gradient Gp, publishes Gp as operand fragments, updates W and the bias, saves what the backward reads;
 //   output (warps 4..7): Zq = Q W + b from the published fragments, Zbar = Zq - M' Gp, the LayerNorm and the output tile --

@@ -24,7 +24,11 @@
 //  * A warp also owns one token row of the 16 x 64 tiles for the two LayerNorms.
 // A stage is six barrier intervals (I1..I6 below).  Before, 25 phases passed every intermediate tile through shared
 // memory as bf16, undid the updates through registers and read dW from L2: 43 k cycles a stage; 192 streams of 128 stages
-// forward and backward 4.12 ms, now 2.52 ms.
+// forward and backward 4.11 ms, now 2.53 ms.
+// What the tensor cores' accumulation does to the masters: undone over 112 / 470 stages they are 7e-6 / 3e-5 (2-norm) off the
+// forward's own state there (terms summed from zero and added in registers: W1 4e-6 / 2e-5, W2 6e-6 / 3e-5); the bf16 copies that
+// the products read are 1.7e-3 off.  Gradients against float64: 128 stages 0.74 to 1.01 times the errors of the sums in
+// registers, 512 stages 0.81 to 0.99 (264 streams).
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
 #include "ttt_stage.cuh"
