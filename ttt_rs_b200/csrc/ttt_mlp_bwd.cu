@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
     };
     // What a stage needs before its first barrier and does not take from the stage after it; `b`: its input buffer.
     //  * both LayerNorms, a row per warp: G2 and dZb2 as bf16 pairs.  Variances are sums of squared deviations: with the forward's
-    //    E[z^2] - mean^2, rows whose mean is 100 standard deviations had gradients 2e-2 off (8e-3 this way; 1.3 % of the kernel's time)
+    //    E[z^2] - mean^2, rows whose mean is 100 standard deviations had state gradients 3e-2 to 4e-2 off (5e-3 to 7e-3 this way; 1.3 % of the time)
     uint32_t g2_pair, dzb_pair;
     F2 rstds;
     auto row_stats = [&]() {
