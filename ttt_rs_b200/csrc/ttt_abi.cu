@@ -654,7 +654,7 @@ int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const voi
   ttt::MlpFwdParams p;
   p.w1 = w1; p.b1 = b1; p.w2 = w2; p.b2 = b2;
   p.token_eta = token_eta; p.lr = ttt_lr_eta; p.ln_g = ln_weight; p.ln_b = ln_bias;
-  p.w1_out = w1_out; p.b1_out = b1_out; p.w2_out = w2_out; p.b2_out = b2_out;
+  p.out = output; p.w1_out = w1_out; p.b1_out = b1_out; p.w2_out = w2_out; p.b2_out = b2_out;
   p.status = static_cast<uint32_t*>(status);
   p.bwd_ws = static_cast<float*>(backward_workspace);
   p.bwd_ws_stride = wl.stride_floats;

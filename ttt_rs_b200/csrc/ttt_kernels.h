@@ -111,6 +111,7 @@ struct MlpFwdParams {
   const void* lr;         // [B,H,T]
   const void* ln_g;       // [H,F]
   const void* ln_b;       // [H,F]
+  void* out;              // [B,H,T,F]
   void* w1_out;
   void* b1_out;
   void* w2_out;

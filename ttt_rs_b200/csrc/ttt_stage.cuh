@@ -288,4 +288,23 @@ __device__ __forceinline__ void report_timeout(uint32_t* status, uint32_t where,
   }
 }
 
+// ---- rank-16 updates of a state in tensor memory by tcgen05 (TTT-MLP) ----------------------------------------------
+// operand descriptor of token tiles read MN-major: 64 contiguous elements (128 bytes, swizzled) x 8 tokens per atom, the
+// other 8 tokens 1024 bytes on, the next 64 elements (A: M = 128) one tile on
+__device__ __forceinline__ uint64_t token_desc(uint32_t tile) {
+  return (uint64_t)((tile >> 4) & 0x3fff) | ((uint64_t)(TILE_BF16_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
+}
+// D[128 x 64] (float32) += (-)A . B over 16 tokens; A and B bf16, MN-major
+constexpr uint32_t UPD_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t UPD_NEGATE = 1u << 13;
+__device__ __forceinline__ void umma_update(uint32_t d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 1, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+               "l"(token_desc(a_tile)), "l"(token_desc(b_tile)), "r"(idesc)
+               : "memory");
+}
+__device__ __forceinline__ void umma_commit_to(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 }  // namespace ttt
