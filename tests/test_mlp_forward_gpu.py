@@ -45,3 +45,38 @@ def test_mlp_rejects_float32():
         tb.fused_ttt_mlp_forward(d["xq"], d["xk"], d["xv"], tb.TTTMLPState(d["w1"], d["b1"], d["w2"], d["b2"]),
                                  d["token_eta"], d["ttt_lr_eta"], d["ln_weight"], d["ln_bias"],
                                  tb.FusedTttConfig.new(16, 64, 1e-6, 256, 1))
+
+
+@pytest.mark.parametrize("B,H,NS,eta", [(1, 1, 2, "plain"), (2, 1, 3, "zero"), (1, 3, 4, "thirds"), (3, 1, 5, "zero"), (21, 8, 9, "thirds")])
+def test_mlp_forward_at_the_edges_of_its_rings(B, H, NS, eta):
+    """Fewer stages than slots of inputs, just as many, one and two more (every ring and parity of the kernel wraps), streams in
+    chunks handed from block to block (168 of them), an update coefficient of zero (the state stays) and one that is no power
+    of two.  Saving state for the backward changes nothing in the results of a stream in one piece; a chunk ends with float32
+    biases added up once more, which moves bf16 results by roundings."""
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    t = O.make_inputs(B, H, NS * 16, 64, 16, seed=900 + NS, dtype=torch.bfloat16, inner="mlp", with_grad_output=False)
+    g = torch.Generator().manual_seed(NS)
+    for k, at, scale in (("ln_weight", 1.0, 0.1), ("ln_bias", 0.0, 0.1), ("b1", 0.0, 0.05), ("b2", 0.0, 0.05)):
+        t[k] = (at + scale * torch.randn(t[k].shape, generator=g)).to(torch.bfloat16)
+    if eta == "zero":
+        t["token_eta"].view(-1, 16)[:, 15] = 0.0
+    elif eta == "thirds":
+        t["token_eta"] = (t["token_eta"].float() / 3).to(torch.bfloat16)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 256, 1)
+    d = {k: t[k].to(dev) for k in NAMES}
+    st = tb.TTTMLPState(d["w1"], d["b1"], d["w2"], d["b2"])
+    args = (d["xq"], d["xk"], d["xv"], st, d["token_eta"], d["ttt_lr_eta"], d["ln_weight"], d["ln_bias"], cfg)
+    out, new = tb.fused_ttt_mlp_forward(*args)
+    saved, kept = tb.fused_ttt_mlp_forward(*args, backward_workspace=tb.mlp_backward_workspace(d["xq"], cfg))
+    torch.cuda.synchronize()
+    tb.TttTileMultiKernel.check_status()
+    ref = O.ttt_mlp_forward(*[t[k].double() for k in NAMES], mini_batch=16, eps=1e-6)
+    for o, s in ((out, new), (saved, kept)):
+        assert_close(o, ref["output"], 2e-2, "output", max_bad_frac=3.6e-4)  # the fractions of the test above
+        for k in ("w1", "b1", "w2", "b2"):
+            assert_close(getattr(s, k), ref[k], 2e-2, "final " + k, max_bad_frac=1.3e-3)
+    if B * H <= 128:  # no more streams than blocks: one piece each
+        assert torch.equal(out, saved) and all(torch.equal(getattr(new, k), getattr(kept, k)) for k in ("w1", "b1", "w2", "b2"))
+    if eta == "zero":
+        assert all(torch.equal(getattr(new, k), d[k]) for k in ("w1", "b1", "w2", "b2"))

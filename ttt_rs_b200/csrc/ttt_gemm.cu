@@ -81,28 +81,6 @@ struct GemmSmem {
   static constexpr uint32_t DYN_BYTES = TOTAL + 1024;
 };
 
-// shared-memory matrix descriptor for a K-major bf16 tile of 128-byte rows with 128-byte swizzle: start address >> 4,
-// stride between 8-row groups = 1024 bytes, descriptor version 1 (sm_100), layout type 2 (SWIZZLE_128B)
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-         (2ull << 61);
-}
-// instruction descriptor, kind::f16: D float32 (bit 4), A and B bf16 (bits 7, 10), both K-major, N >> 3 at bit 17,
-// M >> 4 at bit 24
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {  // N: a multiple of 16, 16..256, at M = 128
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // cta_group::2 forms: issued by the leader CTA of a pair; `bar` of the commit may be a mapa address in the peer.
 __device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {

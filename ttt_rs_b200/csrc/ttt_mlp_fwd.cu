@@ -9,20 +9,26 @@
 //     out = Q + LN(Zb2);   W1 -= te15 K^T G1p;  b1 -= te15 colsum(G1p);  W2 -= te15 X2^T G2p;  b2 -= te15 colsum(G2p)
 //
 // What bounds it: the chain W -> Z1 -> X2 -> Z2 -> G2 -> G1 -> W from one stage to the next on one SM (the state and its
-// copies fill it), and the instructions of a stage: 16 warps issue them, 4 096 tanh twice, ~1 000 mma.sync.  So:
+// copies fill it): 6.1 k cycles a stage, 5.0 k with nothing beside it, of them 1.2 k round trips of three dependent tcgen05
+// products and their commits, the rest instructions of two warps a scheduler at seven cycles each.  So:
 //  * Only that chain is the first group's work (warps 0..7).  The second group (warps 8..15) forms the stage's output from
-//    what the chain publishes in shared memory -- bf16 copies of W1 and W2, X2, G1p, G2p -- about half a stage behind.
+//    what the chain publishes in shared and tensor memory, about half a stage behind.
 //  * Warp w of either group owns hidden features e in [32w, 32w+32) of every 16 x 256 tile, in mma accumulator layout, from Z1
-//    to G1p and from Zb1 to Xb2.  Sums over all hidden features (Z2, Zb2) are formed by each warp over its own 32 straight from
-//    registers; the eight partial tiles meet in shared memory, where a half-warp adds up a token's row and has the whole row for
+//    to G1p and from Zb1 to Xb2.  Products of tokens with the state over its 64 columns (Q W1, K W1, G2p W2^T) are tcgen05.mma
+//    with hidden features as lanes, two halves of 128.
+//  * Sums over all hidden features (Z2, Zb2) are formed by each warp over its own 32 by mma.sync; the eight partial tiles meet
+//    in shared memory, where a half-warp adds up a token's row and has the whole row for
 //    its LayerNorm: two barriers of the group a stage in the chain, where column owners exchanging row sums needed six.
 //  * A2 = Xb2 X2^T meets the same way, two of its rows per warp; each warp then forms a column tile of M2' G2p.
-//  * A1 and M1' of the next stage are formed by one warp of the second group in turn while it would wait.
+//  * A1 and M1' of the next stage are formed by one warp of the second group in turn.
 //  * The float32 masters of W1^T[e][k] and W2[e][n] are tensor-memory accumulators of 128 hidden features x 64; both rank-16
-//    updates are tcgen05.mma into them (operands: the token tiles, tokens the contraction), and each warp of the chain reads its
-//    32 rows back and refreshes their bf16 copies in shared memory, the operand of every product with the state.
-// One group of eight warps with the masters in registers: 9.2 k cycles a stage, 48 streams of 31 stages 150 us, forward +
-// backward of 192 streams of 128 stages 2 528 us; this form 6.8 k, 115 and 2 284 us.
+//    updates are tcgen05.mma into them (operands: the token tiles, tokens the contraction).  Each warp of the chain reads its 32
+//    rows back and refreshes their bf16 copies: in tensor memory, the A operand of the products with the state, and W2's in
+//    shared memory.  (With the copies in shared memory only, a product of 128 x 16 read 4 KB of them at the 128 bytes a cycle that
+//    everything else there needs too: 119 against 106 us.)
+// 48 streams of 31 stages / forward + backward of 192 streams of 128 stages: one group of eight warps with the masters in
+// registers 150 / 2 528 us; two groups, products with the state by mma.sync 115 / 2 284; by tcgen05 106 / 2 243.  Not better: two groups
+// of sixteen warps 121 / 2 355; K_next W1_next taken as K_next W1 plus a product with G1p, which takes W1's refresh off the chain, 111 / 2 284.
 //
 // Scheduling.  One CTA fills an SM, so a launch of one CTA per stream runs in whole
 // waves: 192 streams on 148 SMs cost two stream-times.  When the caller passes the backward's workspace (training),
@@ -42,34 +48,37 @@ constexpr int MLP_NST = 3;
 
 struct MlpSmem {
   static constexpr uint32_t TILE = TILE_BF16_BYTES, ET = 4 * TILE;    // [16][64] bf16; [16 tok][256 e] = four of them
-  static constexpr uint32_t SLOT = 3 * TILE;                          // q, k, v
+  static constexpr uint32_t SLOT = 3 * TILE;                          // q, k, v; in odd stages k, q, v
   static constexpr uint32_t WC = MLP_E * HD * 2;                      // [256 e][64] bf16, 128-byte rows, swizzled
   static constexpr uint32_t PART = 8 * 4096;                          // float [8 warps][16][64]
-  static constexpr uint32_t OFF_W1 = MLP_NST * SLOT;                  // copy of W1^T
-  static constexpr uint32_t OFF_W2 = OFF_W1 + WC;                     // two copies of W2 (stage parity)
+  static constexpr uint32_t OFF_W2 = MLP_NST * SLOT;                  // two copies of W2 (stage parity)
   static constexpr uint32_t OFF_X2 = OFF_W2 + 2 * WC;                 // two X2, then two G1p
   static constexpr uint32_t OFF_G1 = OFF_X2 + 2 * ET;
   static constexpr uint32_t OFF_G2 = OFF_G1 + 2 * ET;                 // two G2p
   static constexpr uint32_t OFF_PC = OFF_G2 + 2 * TILE;               // partials of Z2
-  static constexpr uint32_t OFF_PO = OFF_PC + PART;                   // partials of Zb2
-  static constexpr uint32_t OFF_B1 = OFF_PO + PART;                   // float [256]
+  static constexpr uint32_t OFF_PO = OFF_PC + PART;                   // partials of Zb2, and M2' G2p
+  static constexpr uint32_t OFF_M1 = OFF_PO + PART + 4096;                   // two [16][16] in tile form (the first columns of a [16][64]): -M1' / wscale
+  static constexpr uint32_t OFF_B1 = OFF_M1 + 2 * TILE;               // float [2][256] (stage parity)
   static constexpr uint32_t B2 = 8 * HD * 4;                          // b2 / wscale as shares of the eight warps of the chain
-  static constexpr uint32_t OFF_B2 = OFF_B1 + MLP_E * 4;              // float [2][8][64] (stage parity)
-  static constexpr uint32_t OFF_M1 = OFF_B2 + 2 * B2;                 // two bf16 [16][24]: -M1', then -M2' (stage parity)
-  static constexpr uint32_t OFF_A2 = OFF_M1 + 2 * 16 * 24 * 2;        // float [8 warps][3][8][8]: partials of A2 (its lower blocks)
+  static constexpr uint32_t OFF_B2 = OFF_B1 + 2 * MLP_E * 4;              // float [2][8][64] (stage parity)
+  static constexpr uint32_t OFF_M2 = OFF_B2 + 2 * B2;                 // bf16 [16][24]: -M2'
+  static constexpr uint32_t OFF_A2 = OFF_M2 + 16 * 24 * 2;            // float [8 warps][3][8][8]: partials of A2 (its lower blocks)
   static constexpr uint32_t OFF_LR = OFF_A2 + 8 * 768;                // MLP_NST x 32 bytes
-  // mbarriers: full [MLP_NST], published [2], done [2], state, read, updates of W1, W2; then item, failure flag, tensor-memory base
+  // mbarriers: full [MLP_NST], published [2], done [2], state, partials read; products: Zb1 [2], Z1, G1, updates of W1, W2; M1';
+  // then item, failure flag, tensor-memory base
   static constexpr uint32_t OFF_BAR = OFF_LR + MLP_NST * 32;
-  static constexpr uint32_t OFF_WORDS = OFF_BAR + (MLP_NST + 8) * 8;
+  static constexpr uint32_t OFF_WORDS = OFF_BAR + (MLP_NST + 13) * 8;
   static constexpr uint32_t TOTAL = OFF_WORDS + 16;
 };
 static_assert(MlpSmem::TOTAL <= 227 * 1024, "shared-memory tiles exceed one SM");
-static_assert(MlpSmem::OFF_M1 % 16 == 0 && MlpSmem::OFF_LR % 16 == 0 && MlpSmem::OFF_BAR % 8 == 0, "alignment");
+static_assert(MlpSmem::OFF_M1 % 1024 == 0 && MlpSmem::OFF_M2 % 16 == 0 && MlpSmem::OFF_LR % 16 == 0 && MlpSmem::OFF_BAR % 8 == 0, "alignment");
 
-// tanh-approximated GELU of a column pair and (DERIV) its derivative times sc.  tanh(x) = 1 - 2 / (1 + e^{2x}) (relative error
-// ~1e-6; the hardware tanh.approx is only good to ~5e-4, which shows after a few dozen chained stages).  The two quotients share
-// one reciprocal, 1/a = b / (ab): the special-function unit, which a stage's 8 192 tanh keep busy for a thousand cycles, is
-// asked three times instead of four.  Exponents stop at 2^60, where tanh is 1, so that the product stays finite.
+// tanh-approximated GELU of a pair and (DERIV) its derivative times sc, from q = 1 / (1 + e^{2u}), tanh(u) = 1 - 2q (relative
+// error ~1e-6; the hardware tanh.approx is only good to ~5e-4, which shows after a few dozen chained stages):
+//     gelu = z (1 - q),   gelu' = (1 - q) (1 + 2 z q u'),   u = c0 z (1 + c1 z^2).
+// The pair's quotients share one reciprocal, 1/a = b / (ab): three calls of the special-function unit instead of four.
+// Exponents stop at 2^60, where tanh is 1, so that the product stays finite; the 2^-60 that q keeps there is taken off, or its
+// product with z^3 would show in gelu' of a z in the millions.
 __device__ __forceinline__ float ex2_approx(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -86,15 +95,9 @@ __device__ __forceinline__ F2 gelu2(F2 z, F2& deriv, float sc) {
   const F2 z2 = f2mul(z, z);
   const F2 a = f2mul(z, f2fma(z2, f2(L2E2 * C0 * C1), f2(L2E2 * C0)));
   const F2 d = f2add(f2(ex2_approx(fminf(a.x, 60.f)), ex2_approx(fminf(a.y, 60.f))), f2(1.f));
-  const F2 th = f2fma(f2mul(f2(rcp_approx(d.x * d.y)), f2(d.y, d.x)), f2(-2.f), f2(1.f));
-  const F2 hz = f2mul(z, f2(0.5f));
-  if constexpr (DERIV) {
-    // sc (0.5 z (1 - t^2) c0 (1 + 3 c1 z^2) + 0.5 (1 + t))
-    const F2 sech2 = f2fma(f2neg(th), th, f2(1.f));
-    const F2 poly = f2fma(z2, f2(sc * (3.f * C0 * C1)), f2(sc * C0));
-    deriv = f2fma(f2mul(hz, sech2), poly, f2fma(th, f2(0.5f * sc), f2(0.5f * sc)));
-  }
-  return f2fma(hz, th, hz);
+  const F2 nq = f2fma(f2(rcp_approx(-(d.x * d.y))), f2(d.y, d.x), f2(0x1p-60f)), y = f2mul(z, nq);
+  if constexpr (DERIV) deriv = f2mul(f2fma(nq, f2(sc), f2(sc)), f2fma(y, f2fma(z2, f2(-6.f * C0 * C1), f2(-2.f * C0)), f2(1.f)));
+  return f2add(z, y);
 }
 
 namespace {
@@ -126,16 +129,73 @@ __device__ __forceinline__ uint32_t lds_word(uint32_t a) {
 __device__ __forceinline__ void sts_word(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ F2 bf_pair(uint32_t v) { return make_float2(bf16_lo(v), bf16_hi(v)); }
 // four columns of a token's row summed over the eight warps' partial tiles (addresses: see `part_row`)
+template <int N>
 __device__ __forceinline__ void sum_partials(uint32_t a, F2 (&z)[2]) {
-  float4 v[8];
+  float4 v[N];
 #pragma unroll
-  for (int w = 0; w < 8; ++w) v[w] = lds_f4(a + 4096 * w);
+  for (int w = 0; w < N; ++w) v[w] = lds_f4(a + 4096 * w);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    F2 x[8];
+    F2 x[N];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) x[w] = h ? f2(v[w].z, v[w].w) : f2(v[w].x, v[w].y);
+    for (int w = 0; w < N; ++w) x[w] = h ? f2(v[w].z, v[w].w) : f2(v[w].x, v[w].y);
     z[h] = f2add(f2add(f2add(x[0], x[1]), f2add(x[2], x[3])), f2add(f2add(x[4], x[5]), f2add(x[6], x[7])));
+    if constexpr (N == 9) z[h] = f2add(z[h], x[8]);
+  }
+}
+// An accumulator of sixteen tokens (columns) for this warp's 32 hidden features (lanes), in mma accumulator layout:
+// z[mt][nt][2r + c] is hidden feature 16 mt + 8 r + g, token 8 nt + 2 t + c.
+__device__ __forceinline__ void tmem_ld_tokens(uint32_t taddr, float (&z)[2][2][4]) {
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(z[mt][0][0]), "=f"(z[mt][0][1]), "=f"(z[mt][0][2]), "=f"(z[mt][0][3]), "=f"(z[mt][1][0]), "=f"(z[mt][1][1]), "=f"(z[mt][1][2]), "=f"(z[mt][1][3])
+                 : "r"(taddr + (16u << 16) * mt));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(z[i >> 3][(i >> 2) & 1][i & 3]));  // (not used before the wait)
+}
+__device__ __forceinline__ void tmem_st_16(uint32_t taddr, const uint32_t (&w)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]), "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]),
+               "r"(w[15]), "r"(taddr)
+               : "memory");
+}
+// D[128 x N] (float32) += A . B over 16 of the contraction; A bf16 in tensor memory (a pair of the contraction per word), B K-major
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d), "r"(a),
+               "l"(b), "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void stsm_x4_t(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// A warp's share of X W2 + b2 over its 32 hidden features, all in units of wscale, times sc, to its partial tile: x2f the A
+// fragments of X, w2 the warp's rows of the copy, sh its share of b2.  Four column tiles at a time, their loads ahead of the
+// products: with all eight accumulators live the registers left serialised every ldmatrix with its products.
+__device__ __forceinline__ void share_of_hidden_sum(const uint32_t (&a)[2][4], uint32_t w2, uint32_t sh, uint32_t part, float sc) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t b[4][4];
+    float z[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ldsm_x4_t(b[i], (w2 + 16 * 128 * (i >> 1)) ^ ((4 * h + 2 * (i & 1)) << 4));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const F2 v = lds_pair(sh + 32 * (4 * h + j));
+      z[j][0] = z[j][2] = v.x;
+      z[j][1] = z[j][3] = v.y;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        mma_bf16(z[j], a[c][0], a[c][1], a[c][2], a[c][3], b[2 * c + (j >> 1)][2 * (j & 1)], b[2 * c + (j >> 1)][2 * (j & 1) + 1]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sts_pair(part ^ ((4 * h + j) << 5), f2mul(pr(z[j], 0), f2(sc)));
+      sts_pair((part ^ ((4 * h + j) << 5)) + 8 * 256, f2mul(pr(z[j], 1), f2(sc)));
+    }
   }
 }
 // sums of two values over the sixteen lanes that share a row
@@ -163,7 +223,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     return;
   }
   const uint32_t bar_full = base + SM::OFF_BAR, bar_pub = bar_full + 8 * MLP_NST, bar_done = bar_pub + 16,
-                 bar_state = bar_done + 16, bar_read = bar_state + 8, bar_w1 = bar_read + 8, bar_w2 = bar_w1 + 8;
+                 bar_state = bar_done + 16, bar_parts = bar_state + 8, bar_zq = bar_parts + 8, bar_z = bar_zq + 16, bar_h = bar_z + 8,
+                 bar_w1 = bar_h + 8, bar_w2 = bar_w1 + 8, bar_m1 = bar_w2 + 8;
   const uint32_t w_item = base + SM::OFF_WORDS, w_fail = w_item + 4, w_tmem = w_item + 8;
 
   const bool output_group = __shfl_sync(0xffffffffu, threadIdx.x >> 8, 0) != 0;
@@ -172,23 +233,27 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   const int NS = p.NS, CH = SAVE ? p.CH : NS, NCH = SAVE ? p.NCH : 1;
   const int nitems = SAVE ? p.nstreams * NCH : (int)gridDim.x;
 
-  if (threadIdx.x < 32) tmem_alloc(w_tmem, 256);
+  if (threadIdx.x < 32) tmem_alloc(w_tmem, 512);
   if (threadIdx.x == MLP_GROUP) {
     prefetch_tmap(&tm_q);
     prefetch_tmap(&tm_k);
     prefetch_tmap(&tm_v);
     for (int i = 0; i < MLP_NST; ++i) mbar_init(bar_full + 8 * i, 1);
     for (int i = 0; i < 6; ++i) mbar_init(bar_pub + 8 * i, 8);
-    mbar_init(bar_w1, 2);
-    mbar_init(bar_w2, 2);
+    for (int i = 0; i < 6; ++i) mbar_init(bar_zq + 8 * i, 2);  // (a commit for each half of the hidden features)
+    mbar_init(bar_m1, 1);
     fence_mbar_init();
     sts_word(w_fail, 0u);
   }
   tmem_fence_before_sync();
   __syncthreads();
   tmem_fence_after_sync();
-  // tensor memory: W1^T, W2, each as two accumulators of 128 hidden features (lanes) x 64 columns
+  // Tensor memory, hidden features as lanes, two halves of 128.  Masters W1^T and W2 [half][64 columns]; products with columns of
+  // tokens [half][Zb1 of even stages, Z1 (then G1), Zb1 of odd stages]; bf16 copies of W1^T and W2 [half][32 columns].
   const uint32_t tmem = lds_word(w_tmem);
+  constexpr uint32_t TM_Z = 256, TM_W1B = 352, TM_W2B = 416;
+  const uint32_t tm_lane = (32u * (uint32_t)(warp & 3)) << 16;  // this warp's lanes: hidden features 32 warp .. of half warp / 4
+  const int half = warp >> 2;
 
   const float te15 = ld_as_float<T>(p.token_eta, CS - 1);
   // both states are carried divided by wscale = -te15, so that their rank-16 updates accumulate directly by mma
@@ -199,7 +264,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   // chunks of k-step or column pair i: ^ (i << 5); the next chunk's blocks: ^ (1 << 4).
   const uint32_t tl = lane_off_A(lane, 0);
   const uint32_t own = (warp >> 1) * TL + (tl ^ ((warp & 1) << 6));  // this warp's 32 columns of a 16 x 256 tile
-  const uint32_t wrow = warp * 32 * 128 + tl;                        // this warp's 32 rows of a copy of W1^T or W2
+  const uint32_t wrow = warp * 32 * 128 + tl;                        // this warp's 32 rows of a copy of W2
   // partial sums: a fragment's pairs (rows g, g + 8; column tile nt: ^ (nt << 5)) and a row owner's four columns
   const uint32_t part_frag = warp * 4096 + g * 256 + ((8 * t) ^ ((g & 3) << 5));
   const int row = 2 * warp + (lane >> 4), c4 = 4 * (lane & 15);
@@ -266,32 +331,51 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 
     if (!output_group) {
       // ============================== chain ==============================
-      // warp w reads back lanes 32 (w % 4) .. of accumulator w / 4: the masters' rows e = 32 w + lane
-      const uint32_t tm_own = tmem + ((32u * (uint32_t)(warp & 3)) << 16) + 64u * (uint32_t)(warp >> 2);
-      const int e_own = 32 * warp + lane, b1_col = 32 * warp + 8 * (g >> 1) + 2 * t + (g & 1);
-      // bf16 copy of 32 columns of this warp's rows of a master
-      auto put_copy = [&](uint32_t copy, int cc, const float (&v)[8][4]) {
+      const uint32_t tm_own = tmem + tm_lane + 64u * half;
+      const int e_own = 32 * warp + lane, b1_col = 32 * warp + 8 * t + g;
+      // bf16 copies of 32 columns of this warp's rows of a master: in tensor memory, the A operand of products with the state, and
+      // of W2 in shared memory too
+      auto put_copy = [&](int mat, uint32_t buf, int cc, const float (&v)[8][4]) {
+        uint32_t w[16];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          st_u4(copy + e_own * 128 + (((4 * cc + i) ^ (lane & 7)) << 4), pack_bf16(v[2 * i][0], v[2 * i][1]), pack_bf16(v[2 * i][2], v[2 * i][3]),
-                pack_bf16(v[2 * i + 1][0], v[2 * i + 1][1]), pack_bf16(v[2 * i + 1][2], v[2 * i + 1][3]));
+        for (int i = 0; i < 16; ++i) w[i] = pack_bf16(v[i >> 1][2 * (i & 1)], v[i >> 1][2 * (i & 1) + 1]);
+        tmem_st_16(tmem + tm_lane + (mat == 0 ? TM_W1B : TM_W2B) + 32 * half + 16 * cc, w);
+        if (mat == 1) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            st_u4(base + SM::OFF_W2 + buf * SM::WC + e_own * 128 + (((4 * cc + i) ^ (lane & 7)) << 4), w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+        }
       };
-      auto refresh = [&](uint32_t copy, int mat) {
+      auto refresh = [&](int mat, uint32_t buf) {
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           float v[8][4];
           tmem_ld_8x4(tm_own + 128 * mat + 32 * cc, v);
-          put_copy(copy, cc, v);
+          put_copy(mat, buf, cc, v);
         }
       };
-      // the rank-16 update of this half's 128 hidden features: one thread of warps 0 and 4
-      auto issue_update = [&](int mat, uint32_t a_tile, uint32_t b_tile, uint32_t bar) {
-        if ((warp & 3) == 0 && elect_one()) {
-          tmem_fence_after_sync();
-          if (w_moves) umma_update(tmem + 128 * mat + 16 * warp, a_tile + (warp >> 1) * TL, b_tile, UPD_IDESC);
-          umma_commit_to(bar);
+      // Products of this half's 128 hidden features, issued by one thread of its i-th warp (four of them keep it for 400 cycles).
+      auto issue = [&](int i, uint32_t bar, auto&& products) {
+        if ((warp & 3) == i) {
+          if (elect_one()) {
+            tmem_fence_after_sync();
+            products();
+            umma_commit_to(bar);
+          }
+          __syncwarp();
         }
-        __syncwarp();
+      };
+      auto half_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(3 + half) : "memory"); };
+      // [Q; K] W1 / wscale of the n'th stage
+      auto issue_first = [&](uint32_t n, int s) {
+        const uint32_t slot = n % MLP_NST;
+        if ((warp & 3) == 0) wait_for(bar_full + 8 * slot, (n / MLP_NST) & 1, 21, s);
+        issue(0, bar_z, [&]() {
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16_ts(tmem + TM_Z + 48 * half + 16 * (n & 1), tmem + TM_W1B + 32 * half + 8 * ks, umma_desc_sw128(base + slot * SM::SLOT + 32 * ks),
+                         umma_idesc_bf16(128, 32), ks != 0);
+        });
       };
       float b1c;  // b1[b1_col]
       {
@@ -322,12 +406,12 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
               }
             }
             tmem_st_8x4(tm_own + 128 * mat + 32 * cc, v);
-            put_copy(base + (mat == 0 ? SM::OFF_W1 : SM::OFF_W2 + (n & 1) * SM::WC), cc, v);
+            put_copy(mat, n & 1, cc, v);
           }
         const float* const ho = bws + 4 * HD * MLP_E;
         const bool first = !SAVE || chunk == 0;
         b1c = first ? ld_as_float<T>(p.b1, (size_t)stream * MLP_E + b1_col) : __ldcg(ho + MLP_HO_B1 + b1_col);
-        sts_word(base + SM::OFF_B1 + 4 * b1_col, __float_as_uint(b1c));
+        sts_word(base + SM::OFF_B1 + (n & 1) * MLP_E * 4 + 4 * b1_col, __float_as_uint(b1c));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // b2: the first warp's share
           const int c = lane + 32 * h;
@@ -337,67 +421,46 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         tmem_wait_st();
         tmem_fence_before_sync();
         mbar_arrive_warp(bar_state);
+        half_sync();
+        issue_first(n, s_lo);
       }
 
       for (int s = s_lo; s <= s_hi; ++s, ++n) {
         const uint32_t slot = n % MLP_NST, par = n & 1;
-        const uint32_t tq = base + slot * SM::SLOT, tk = tq + TL, tv = tk + TL;
+        const uint32_t tk = base + slot * SM::SLOT + (par ^ 1) * TL, tv = base + slot * SM::SLOT + 2 * TL;
         const uint32_t w2c = base + SM::OFF_W2 + par * SM::WC, tx2 = base + SM::OFF_X2 + par * SM::ET,
                        tg1 = base + SM::OFF_G1 + par * SM::ET, tg2 = base + SM::OFF_G2 + par * TL;
         uint8_t* const rec = SAVE ? rec0 + (size_t)s * MLP_REC_BYTES : nullptr;  // the backward's record of the stage
         if (SAVE) *reinterpret_cast<float*>(rec + MLP_REC_B1 + 4 * b1_col) = b1c;
         const uint32_t sh = base + SM::OFF_B2 + par * SM::B2 + warp * HD * 4;  // this warp's share of b2
         wait_for(bar_full + 8 * slot, (n / MLP_NST) & 1, 21, s);
+        wait_for(bar_z, n & 1, 24, s);
+        tmem_fence_after_sync();
         // ---- C1. Z1 = K W1 + b1 (this warp's hidden features), X2 = gelu(Z1), D1 = wscale gelu'(Z1)
-        F2 d1[4][2];
-        uint32_t x2[4][2];
+        F2 d1[4][2];         // [i][nt]: hidden feature 8 i + g, tokens 8 nt + 2 t, + 1
         {
-          float z1[4][4] = {};
+          float z1[2][2][4];
+          uint32_t x2[4][2];
+          tmem_ld_tokens(tmem + tm_lane + TM_Z + 48 * half + 16, z1);
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            uint32_t ak[4], b[2][4];
-            ldsm_x4(ak, tk + (tl ^ (ks << 5)));
-            ldsm_x4(b[0], (base + SM::OFF_W1 + wrow) ^ (ks << 5));
-            ldsm_x4(b[1], (base + SM::OFF_W1 + wrow + 16 * 128) ^ (ks << 5));
+          for (int i = 0; i < 4; ++i) {
+            const F2 b1 = f2(__uint_as_float(lds_word(base + SM::OFF_B1 + par * MLP_E * 4 + 4 * (32 * warp + 8 * i + g))));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) mma_bf16(z1[j], ak[0], ak[1], ak[2], ak[3], b[j >> 1][j & 1], b[j >> 1][2 + (j & 1)]);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const F2 b1 = lds_pair(base + SM::OFF_B1 + 4 * (32 * warp + 8 * j + 2 * t));
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const F2 x = gelu2<true>(f2fma(pr(z1[j], r), f2(wscale), b1), d1[j][r], wscale);
-              x2[j][r] = pack_bf16(x.x, x.y);
+            for (int nt = 0; nt < 2; ++nt) {
+              const F2 x = gelu2<true>(f2fma(pr(z1[i >> 1][nt], i & 1), f2(wscale), b1), d1[i][nt], wscale);
+              x2[i][nt] = pack_bf16(x.x, x.y);
             }
           }
+          stsm_x4_t(tx2 + own, x2[0][0], x2[0][1], x2[1][0], x2[1][1]);
+          stsm_x4_t((tx2 + own) ^ 32u, x2[2][0], x2[2][1], x2[3][0], x2[3][1]);
         }
-        stsm_x4(tx2 + own, x2[0][0], x2[0][1], x2[1][0], x2[1][1]);
-        stsm_x4((tx2 + own) ^ 32u, x2[2][0], x2[2][1], x2[3][0], x2[3][1]);
-        // ---- C2. this warp's share of (X2 W2 + b2) / wscale (all 64 columns, its own 32 hidden features)
+        // ---- C2. this warp's share of Z2 = X2 W2 + b2 (all 64 columns, its own 32 hidden features)
         {
-          float z[8][4];
-#pragma unroll
-          for (int nt = 0; nt < 8; ++nt) {
-            const F2 b = lds_pair(sh + 4 * (8 * nt + 2 * t));
-            z[nt][0] = z[nt][2] = b.x;
-            z[nt][1] = z[nt][3] = b.y;
-          }
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int nt = 0; nt < 8; nt += 2) {
-              uint32_t b[4];
-              ldsm_x4_t(b, (w2c + wrow + 16 * 128 * c) ^ (nt << 4));
-              mma_bf16(z[nt], x2[2 * c][0], x2[2 * c][1], x2[2 * c + 1][0], x2[2 * c + 1][1], b[0], b[1]);
-              mma_bf16(z[nt + 1], x2[2 * c][0], x2[2 * c][1], x2[2 * c + 1][0], x2[2 * c + 1][1], b[2], b[3]);
-            }
-          const uint32_t pf = base + SM::OFF_PC + part_frag;
-#pragma unroll
-          for (int nt = 0; nt < 8; ++nt) {
-            sts_pair(pf ^ (nt << 5), pr(z[nt], 0));
-            sts_pair((pf ^ (nt << 5)) + 8 * 256, pr(z[nt], 1));
-          }
+          uint32_t a[2][4];
+          __syncwarp();
+          ldsm_x4(a[0], tx2 + own);
+          ldsm_x4(a[1], (tx2 + own) ^ 32u);
+          share_of_hidden_sum(a, w2c + wrow, sh + 8 * t, base + SM::OFF_PC + part_frag, wscale);
         }
         F2 btg[2];  // beta - (v - k)
         {
@@ -412,9 +475,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         F2 gp[2];
         {
           F2 z[2], x[2], gg[2];
-          sum_partials(base + SM::OFF_PC + part_row, z);
-          z[0] = f2mul(z[0], f2(wscale));
-          z[1] = f2mul(z[1], f2(wscale));
+          sum_partials<8>(base + SM::OFF_PC + part_row, z);
           if (SAVE) *reinterpret_cast<float4*>(rec + MLP_REC_Z2 + 4 * (row * HD + c4)) = make_float4(z[0].x, z[0].y, z[1].x, z[1].y);
           const F2 s1 = row_sum2(f2hsum(f2add(z[0], z[1])), f2hsum(f2fma(z[0], z[0], f2mul(z[1], z[1]))));
           const float mean = s1.x * (1.f / HD), rstd = rsqrtf(fmaxf(s1.y * (1.f / HD) - mean * mean, 0.f) + p.eps);
@@ -433,50 +494,52 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         fence_proxy_async_smem();  // (X2 and G2p are read by tcgen05.mma and, SAVE, leave by bulk copies)
         tmem_fence_before_sync();
         mlp_group_sync<1>();  // G2p
-        issue_update(1, tx2, tg2, bar_w2);
+        issue(0, bar_h, [&]() {
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16_ts(tmem + TM_Z + 48 * half + 16, tmem + TM_W2B + 32 * half + 8 * ks, umma_desc_sw128(tg2 + 32 * ks), umma_idesc_bf16(128, 16), ks != 0);
+        });
+        issue(1, bar_w2, [&]() {
+          if (w_moves) umma_update(tmem + 128 + 64 * half, tx2 + half * 2 * TL, tg2, UPD_IDESC);
+        });
         // ---- C4. G1p = (G2p W2^T) o gelu'(Z1)
-        F2 cs1[4];  // float32 column sums of G1p over rows g, g + 8
+        wait_for(bar_h, n & 1, 24, s);
+        tmem_fence_after_sync();
+        float cs1[4];  // float32 sums over this thread's tokens
         {
-          float h[4][4] = {};
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            uint32_t ag[4], b[2][4];
-            ldsm_x4(ag, tg2 + (tl ^ (ks << 5)));
-            ldsm_x4(b[0], (w2c + wrow) ^ (ks << 5));
-            ldsm_x4(b[1], (w2c + wrow + 16 * 128) ^ (ks << 5));
-#pragma unroll
-            for (int j = 0; j < 4; ++j) mma_bf16(h[j], ag[0], ag[1], ag[2], ag[3], b[j >> 1][j & 1], b[j >> 1][2 + (j & 1)]);
-          }
+          float h[2][2][4];
+          tmem_ld_tokens(tmem + tm_lane + TM_Z + 48 * half + 16, h);
           uint32_t gp[4][2];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const F2 a = f2mul(pr(h[j], 0), d1[j][0]), b = f2mul(pr(h[j], 1), d1[j][1]);
-            gp[j][0] = pack_bf16(a.x, a.y);
-            gp[j][1] = pack_bf16(b.x, b.y);
-            cs1[j] = f2add(a, b);
+          for (int i = 0; i < 4; ++i) {
+            const F2 a = f2mul(pr(h[i >> 1][0], i & 1), d1[i][0]), b = f2mul(pr(h[i >> 1][1], i & 1), d1[i][1]);
+            gp[i][0] = pack_bf16(a.x, a.y);
+            gp[i][1] = pack_bf16(b.x, b.y);
+            cs1[i] = f2hsum(f2add(a, b));
           }
-          stsm_x4(tg1 + own, gp[0][0], gp[0][1], gp[1][0], gp[1][1]);
-          stsm_x4((tg1 + own) ^ 32u, gp[2][0], gp[2][1], gp[3][0], gp[3][1]);
+          stsm_x4_t(tg1 + own, gp[0][0], gp[0][1], gp[1][0], gp[1][1]);
+          stsm_x4_t((tg1 + own) ^ 32u, gp[2][0], gp[2][1], gp[3][0], gp[3][1]);
         }
         fence_proxy_async_smem();
+        tmem_fence_before_sync();
         mbar_arrive_warp(bar_pub + 8 * par);  // X2, G2p, G1p of the stage
-        asm volatile("bar.sync %0, 128;" ::"r"(3 + (warp >> 2)) : "memory");  // G1p of the half's hidden features
-        issue_update(0, tg1, tk, bar_w1);
+        half_sync();  // G1p of the half's hidden features
+        issue(0, bar_w1, [&]() {
+          if (w_moves) umma_update(tmem + 64 * half, tg1 + half * 2 * TL, tk, UPD_IDESC);
+        });
+        if ((warp & 3) == 2) wait_for(bar_m1, n & 1, 24, s);
+        issue(2, bar_zq + 8 * par, [&]() {  // Zb1 = Q W1 - M1' G1p
+          umma_bf16(tmem + TM_Z + 48 * half + 32 * par, token_desc(tg1 + half * 2 * TL), umma_desc_sw128(base + SM::OFF_M1 + par * TL), umma_idesc_bf16(128, 16) | (1u << 15), 1u);
+        });
         // ---- C5. under the updates: float32 column sums (like the reference) of G2p and G1p; then the next stage's copies
         const bool more = s < s_hi;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
           gp[h] = f2add(gp[h], f2(__shfl_xor_sync(0xffffffffu, gp[h].x, 16), __shfl_xor_sync(0xffffffffu, gp[h].y, 16)));
-        {  // lanes of a column pair take one column each
-          F2 a[2];
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const F2 send = lane & 16 ? cs1[i] : cs1[2 + i];
-            a[i] = f2add(lane & 16 ? cs1[2 + i] : cs1[i], f2(__shfl_xor_sync(0xffffffffu, send.x, 16), __shfl_xor_sync(0xffffffffu, send.y, 16)));
-          }
-          const F2 send = lane & 8 ? a[0] : a[1];
-          const F2 b = f2add(lane & 8 ? a[1] : a[0], f2(__shfl_xor_sync(0xffffffffu, send.x, 8), __shfl_xor_sync(0xffffffffu, send.y, 8)));
-          const float c = (lane & 4 ? b.y : b.x) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b.x : b.y, 4);
+        {  // lanes of a quad take one hidden feature each
+          const float a0 = (t & 2 ? cs1[2] : cs1[0]) + __shfl_xor_sync(0xffffffffu, t & 2 ? cs1[0] : cs1[2], 2);
+          const float a1 = (t & 2 ? cs1[3] : cs1[1]) + __shfl_xor_sync(0xffffffffu, t & 2 ? cs1[1] : cs1[3], 2);
+          const float c = (t & 1 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, t & 1 ? a0 : a1, 1);
           b1c = fmaf(c, -te15, b1c);
         }
         if (n > 0) wait_for(bar_done + 8 * (par ^ 1), ((n - 1) >> 1) & 1, 25, s);  // the output group is done with the stage before
@@ -489,15 +552,16 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         }
         wait_for(bar_w2, n & 1, 23, s);
         tmem_fence_after_sync();
-        if (more) {
-          refresh(base + SM::OFF_W2 + (par ^ 1) * SM::WC, 1);
-          wait_for(bar_read, n & 1, 24, s);  // the output group has read W1 and b1 of this stage
-        }
+        if (more) refresh(1, par ^ 1);
         wait_for(bar_w1, n & 1, 23, s);
         tmem_fence_after_sync();
         if (more) {
-          refresh(base + SM::OFF_W1, 0);
-          sts_word(base + SM::OFF_B1 + 4 * b1_col, __float_as_uint(b1c));
+          refresh(0, 0);
+          sts_word(base + SM::OFF_B1 + (par ^ 1) * MLP_E * 4 + 4 * b1_col, __float_as_uint(b1c));
+          tmem_wait_st();
+          tmem_fence_before_sync();
+          half_sync();
+          issue_first(n + 1, s + 1);
           mbar_arrive_warp(bar_state);
         }
         // (stage ends)
@@ -549,9 +613,10 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
       // ============================== output ==============================
       const float te_row[2] = {ld_as_float<T>(p.token_eta, g), ld_as_float<T>(p.token_eta, g + 8)};
       const float te_two = ld_as_float<T>(p.token_eta, 2 * warp + (lane >> 4));
-      // -M1' = -te (1 + tril(Q K^T)) of the n'th stage, as bf16 rows
+      const float m1_row[2] = {-te_row[0] / wscale, -te_row[1] / wscale};
+      // -M1' / wscale = -te (1 + tril(Q K^T)) / wscale of the n'th stage, the K-major operand of a product over its tokens
       auto form_m1 = [&](uint32_t n, int s) {
-        const uint32_t slot = n % MLP_NST, tq = base + slot * SM::SLOT, tk = tq + TL;
+        const uint32_t slot = n % MLP_NST, tq = base + slot * SM::SLOT + (n & 1) * TL, tk = base + slot * SM::SLOT + ((n & 1) ^ 1) * TL;
         wait_for(bar_full + 8 * slot, (n / MLP_NST) & 1, 26, s);
         float at[2][4] = {};
 #pragma unroll
@@ -567,63 +632,44 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const int i = g + 8 * r, jj = 8 * jt + 2 * t;
-            const F2 m = f2fma(pr(at[jt], r), f2(-te_row[r]), f2(-te_row[r]));
-            sts_word(base + SM::OFF_M1 + (n & 1) * 768 + 2 * (24 * i + jj), pack_bf16(jj <= i ? m.x : 0.f, jj + 1 <= i ? m.y : 0.f));
+            const F2 m = f2fma(pr(at[jt], r), f2(m1_row[r]), f2(m1_row[r]));
+            sts_word(base + SM::OFF_M1 + (n & 1) * TL + off_bf16(i, jj), pack_bf16(jj <= i ? m.x : 0.f, jj + 1 <= i ? m.y : 0.f));
           }
+        fence_proxy_async_smem();
+        mbar_arrive_warp(bar_m1);
       };
-      // stage s, the n'th of this block, into its ring slot
-      auto issue_loads = [&](uint32_t n, int s) {
-        const uint32_t slot = n % MLP_NST, bar = bar_full + 8 * slot, tq = base + slot * SM::SLOT;
-        mbar_expect_tx(bar, 3 * TL + CS * 2);
-        const int r0 = row_base + s * CS;
-        tma_load_2d(tq + TL, &tm_k, 0, r0, bar);
-        tma_load_2d(tq, &tm_q, 0, r0, bar);
-        tma_load_2d(tq + 2 * TL, &tm_v, 0, r0, bar);
-        bulk_load_1d(base + SM::OFF_LR + slot * 32, static_cast<const uint8_t*>(p.lr) + (size_t)r0 * 2, CS * 2, bar);
-      };
-      uint32_t asked = n + (s_lo < s_hi ? 2 : 1);  // stages whose loads have been issued
-      if (warp == 2) {
+      // stage s, the n'th of this block, into its ring slot: four copies by a warp each (a copy costs its thread a hundred cycles)
+      auto issue_load = [&](uint32_t n, int s, int which) {
         if (elect_one()) {
-          issue_loads(n, s_lo);
-          if (s_lo < s_hi) issue_loads(n + 1, s_lo + 1);
+          const uint32_t slot = n % MLP_NST, bar = bar_full + 8 * slot, to = base + slot * SM::SLOT;
+          const int r0 = row_base + s * CS;
+          if (which == 0) {
+            mbar_expect_tx(bar, 3 * TL + CS * 2);
+            tma_load_2d(to + ((n & 1) ^ 1) * TL, &tm_k, 0, r0, bar);
+          } else if (which == 1) {
+            tma_load_2d(to + (n & 1) * TL, &tm_q, 0, r0, bar);
+          } else if (which == 2) {
+            tma_load_2d(to + 2 * TL, &tm_v, 0, r0, bar);
+          } else {
+            bulk_load_1d(base + SM::OFF_LR + slot * 32, static_cast<const uint8_t*>(p.lr) + (size_t)r0 * 2, CS * 2, bar);
+          }
         }
         __syncwarp();
+      };
+      uint32_t asked = n + (s_lo < s_hi ? 2 : 1);  // stages whose loads have been issued
+      if (warp >= 2 && warp < 6) {
+        issue_load(n, s_lo, warp - 2);
+        if (s_lo < s_hi) issue_load(n + 1, s_lo + 1, warp - 2);
       }
       if (warp == 0) form_m1(n, s_lo);
-      mlp_group_sync<2>();
       for (int s = s_lo; s <= s_hi; ++s, ++n) {
-        const uint32_t slot = n % MLP_NST, par = n & 1, tq = base + slot * SM::SLOT;
+        const uint32_t slot = n % MLP_NST, par = n & 1, tq = base + slot * SM::SLOT + par * TL;
         const uint32_t w2c = base + SM::OFF_W2 + par * SM::WC, tx2 = base + SM::OFF_X2 + par * SM::ET,
                        tg1 = base + SM::OFF_G1 + par * SM::ET, tg2 = base + SM::OFF_G2 + par * TL;
         uint8_t* const rec = SAVE ? rec0 + (size_t)s * MLP_REC_BYTES : nullptr;
-        // ---- O1. Q W1 + b1 (this warp's hidden features)
         wait_for(bar_full + 8 * slot, (n / MLP_NST) & 1, 26, s);
         wait_for(bar_state, n & 1, 27, s);
-        float zq[4][4] = {};
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          uint32_t aq[4], b[2][4];
-          ldsm_x4(aq, tq + (tl ^ (ks << 5)));
-          ldsm_x4(b[0], (base + SM::OFF_W1 + wrow) ^ (ks << 5));
-          ldsm_x4(b[1], (base + SM::OFF_W1 + wrow + 16 * 128) ^ (ks << 5));
-#pragma unroll
-          for (int j = 0; j < 4; ++j) mma_bf16(zq[j], aq[0], aq[1], aq[2], aq[3], b[j >> 1][j & 1], b[j >> 1][2 + (j & 1)]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const F2 b1 = lds_pair(base + SM::OFF_B1 + 4 * (32 * warp + 8 * j + 2 * t));
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const F2 z = f2fma(pr(zq[j], r), f2(wscale), b1);
-            zq[j][2 * r] = z.x;
-            zq[j][2 * r + 1] = z.y;
-          }
-        }
-        mbar_arrive_warp(bar_read);
-        uint32_t am[4];
-        ldsm_x4(am, base + SM::OFF_M1 + par * 768 + (lane & 15) * 48 + ((lane >> 4) << 4));
-        if (s < s_hi && warp == (int)((n + 1) & 7)) form_m1(n + 1, s + 1);
-        // ---- O2. Zb1 = Q W1 + b1 - M1' G1p;  Xb2 = gelu(Zb1)
+        // ---- O1. Zb1 = Q W1 + b1 - M1' G1p;  Xb2 = gelu(Zb1)
         wait_for(bar_pub + 8 * par, (n >> 1) & 1, 28, s);
         if (SAVE && warp == 1) {  // the stage's operands to its record
           if (elect_one()) {
@@ -634,23 +680,25 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
           }
           __syncwarp();
         }
-        uint32_t xb[4][2];
+        wait_for(bar_zq + 8 * par, (n >> 1) & 1, 28, s);
+        tmem_fence_after_sync();
+        uint32_t xb[4][2];  // token 8 nt + g, hidden features 8 i + 2 t, + 1
+        {
+          float zq[2][2][4];
+          tmem_ld_tokens(tmem + tm_lane + TM_Z + 48 * half + 32 * par, zq);
+          tmem_fence_before_sync();
 #pragma unroll
-        for (int j = 0; j < 4; j += 2) {
-          uint32_t b[4];
-          ldsm_x4_t(b, (tg1 + own) ^ (j << 4));
-          mma_bf16(zq[j], am[0], am[1], am[2], am[3], b[0], b[1]);
-          mma_bf16(zq[j + 1], am[0], am[1], am[2], am[3], b[2], b[3]);
-        }
+          for (int i = 0; i < 4; ++i) {
+            const F2 b1 = f2(__uint_as_float(lds_word(base + SM::OFF_B1 + par * MLP_E * 4 + 4 * (32 * warp + 8 * i + g))));
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            F2 unused;
-            const F2 x = gelu2<false>(pr(zq[j], r), unused, 1.f);
-            xb[j][r] = pack_bf16(x.x, x.y);
+            for (int nt = 0; nt < 2; ++nt) {
+              F2 unused;
+              const F2 x = gelu2<false>(f2fma(pr(zq[i >> 1][nt], i & 1), f2(wscale), b1), unused, 1.f);
+              xb[i][nt] = movm_t(pack_bf16(x.x, x.y));
+            }
           }
-        // ---- O3. this warp's share of A2 = Xb2 X2^T and of (Xb2 W2 + b2) / wscale: its 32 hidden features
+        }
+        // ---- O2. this warp's share of A2 = Xb2 X2^T and of (Xb2 W2 + b2) / wscale: its 32 hidden features
         {
           float a2[2][4] = {};
 #pragma unroll
@@ -665,27 +713,17 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
           sts_pair(to + 256, pr(a2[0], 1));
           sts_pair(to + 512, pr(a2[1], 1));
         }
-        float z[8][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const F2 b = lds_pair(base + SM::OFF_B2 + par * SM::B2 + 4 * (warp * HD + 8 * nt + 2 * t));
-          z[nt][0] = z[nt][2] = b.x;
-          z[nt][1] = z[nt][3] = b.y;
+        if (n > 0) wait_for(bar_parts, (n - 1) & 1, 29, s);  // the partials of the stage before have been read
+        {
+          const uint32_t a[2][4] = {{xb[0][0], xb[0][1], xb[1][0], xb[1][1]}, {xb[2][0], xb[2][1], xb[3][0], xb[3][1]}};
+          share_of_hidden_sum(a, w2c + wrow, base + SM::OFF_B2 + par * SM::B2 + warp * HD * 4 + 8 * t, base + SM::OFF_PO + part_frag, wscale);
         }
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int nt = 0; nt < 8; nt += 2) {
-            uint32_t b[4];
-            ldsm_x4_t(b, (w2c + wrow + 16 * 128 * c) ^ (nt << 4));
-            mma_bf16(z[nt], xb[2 * c][0], xb[2 * c][1], xb[2 * c + 1][0], xb[2 * c + 1][1], b[0], b[1]);
-            mma_bf16(z[nt + 1], xb[2 * c][0], xb[2 * c][1], xb[2 * c + 1][0], xb[2 * c + 1][1], b[2], b[3]);
-          }
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) z[nt][i] *= wscale;
-        mlp_group_sync<2>();  // the partials of A2; those of the stage before's Zb2 have been read
+        mlp_group_sync<2>();  // the partials of A2
+        // the slot of the stage before, which everyone has left (the chain has published this one), takes the stage after next
+        if (s + 2 <= s_hi) {
+          if (warp >= 2 && warp < 6 && lds_word(w_fail) == 0u) issue_load(n + 2, s + 2, warp - 2);
+          asked = n + 3;
+        }
         {  // -M2' = -te (1 + tril(A2)), two rows per warp
           const int i = 2 * warp + (lane >> 4), j = lane & 15;
           float a = 0.f;
@@ -696,35 +734,25 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             a = fmaf(a, -te_two, -te_two);
           }
           const float hi = __shfl_down_sync(0xffffffffu, a, 1);
-          if ((lane & 1) == 0) sts_word(base + SM::OFF_M1 + par * 768 + 2 * (24 * i + j), pack_bf16(a, hi));
-        }
-        // the slot of the stage before, which everyone has left (the chain has published this one), takes the stage after next
-        if (warp == 2 && s + 2 <= s_hi && __shfl_sync(0xffffffffu, lds_word(w_fail), 0) == 0u) {
-          if (elect_one()) issue_loads(n + 2, s + 2);
-          asked = n + 3;
-          __syncwarp();
+          if ((lane & 1) == 0) sts_word(base + SM::OFF_M2 + 2 * (24 * i + j), pack_bf16(a, hi));
         }
         mlp_group_sync<2>();  // -M2'
-        {  // M2' G2p: column tile `warp` goes into this warp's partial
-          uint32_t b[4];
-          ldsm_x4(am, base + SM::OFF_M1 + par * 768 + (lane & 15) * 48 + ((lane >> 4) << 4));
+        {  // M2' G2p, a column tile per warp: the ninth partial
+          uint32_t am[4], b[4];
+          float z[4] = {};
+          ldsm_x4(am, base + SM::OFF_M2 + (lane & 15) * 48 + ((lane >> 4) << 4));
           ldsm_x4_t(b, tg2 + (tl ^ ((warp & 6) << 4)));
-          const uint32_t b0 = warp & 1 ? b[2] : b[0], b1 = warp & 1 ? b[3] : b[1];
-#pragma unroll
-          for (int nt = 0; nt < 8; ++nt)
-            if (nt == warp) mma_bf16(z[nt], am[0], am[1], am[2], am[3], b0, b1);
-        }
-        const uint32_t pf = base + SM::OFF_PO + part_frag;
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          sts_pair(pf ^ (nt << 5), pr(z[nt], 0));
-          sts_pair((pf ^ (nt << 5)) + 8 * 256, pr(z[nt], 1));
+          mma_bf16(z, am[0], am[1], am[2], am[3], warp & 1 ? b[2] : b[0], warp & 1 ? b[3] : b[1]);
+          const uint32_t to = base + SM::OFF_PO + 8 * 4096 + g * 256 + ((32 * warp + 8 * t) ^ ((g & 3) << 5));
+          sts_pair(to, pr(z, 0));
+          sts_pair(to + 8 * 256, pr(z, 1));
         }
         const uint2 qv = lds_u2(tq + tile_row);
         mlp_group_sync<2>();  // the partials of Zb2
-        // ---- O4. out = Q + LN(Zb2), a row per half-warp
+        // ---- O3. out = Q + LN(Zb2), a row per half-warp
         F2 zb[2], o[2];
-        sum_partials(base + SM::OFF_PO + part_row, zb);
+        sum_partials<9>(base + SM::OFF_PO + part_row, zb);
+        mbar_arrive_warp(bar_parts);
         if (SAVE) *reinterpret_cast<float4*>(rec + MLP_REC_ZB2 + 4 * (row * HD + c4)) = make_float4(zb[0].x, zb[0].y, zb[1].x, zb[1].y);
         if (SAVE && warp == 1) {  // the bulk copies have left
           if (elect_one()) bulk_wait_read<0>();
@@ -740,6 +768,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
           *reinterpret_cast<uint2*>(static_cast<uint8_t*>(p.out) + ((size_t)(row_base + s * CS + row) * HD + c4) * 2) =
               make_uint2(pack_bf16(o[0].x, o[0].y), pack_bf16(o[1].x, o[1].y));
         }
+        if (s < s_hi && warp == (int)((n + 1) & 7)) form_m1(n + 1, s + 1);  // (one warp)
       }
       if (warp == 2 && lds_word(w_fail) != 0u) {  // copies that are on their way land before the block leaves
         for (uint32_t i = 1; i <= MLP_NST && i <= asked; ++i) mbar_wait_bounded(bar_full + 8 * ((asked - i) % MLP_NST), ((asked - i) / MLP_NST) & 1);
@@ -750,7 +779,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   }  // work items
   tmem_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x < 32) tmem_dealloc(lds_word(w_tmem), 256);
+  if (threadIdx.x < 32) tmem_dealloc(lds_word(w_tmem), 512);
   if (SAVE) bulk_wait_all<0>();
 }
 
