@@ -24,7 +24,7 @@
 //  * A warp also owns one token row of the 16 x 64 tiles for the two LayerNorms.
 // A stage is six barrier intervals (I1..I6 below).  Before, 25 phases passed every intermediate tile through shared
 // memory as bf16, undid the updates through registers and read dW from L2: 43 k cycles a stage; 192 streams of 128 stages
-// forward and backward 4.11 ms, now 2.53 ms.
+// forward and backward 4.11 ms, now 2.21 ms (2.53 before the forward's two groups).
 // What the tensor cores' accumulation does to the masters: undone over 112 / 470 stages they are 7e-6 / 3e-5 (2-norm) off the
 // forward's own state there (terms summed from zero and added in registers: W1 4e-6 / 2e-5, W2 6e-6 / 3e-5); the bf16 copies that
 // the products read are 1.7e-3 off.  Gradients against float64: 128 stages 0.74 to 1.01 times the errors of the sums in
@@ -38,7 +38,6 @@ namespace ttt {
 constexpr int MB_THREADS = 512;
 constexpr uint32_t ONES = 0x3f803f80u;  // a pair of bf16 ones
 constexpr int MB_E = 256;  // hidden width of the inner MLP (4 * head_dim)
-constexpr float GELU_C0 = 0.7978845608028654f, GELU_C1 = 0.044715f;
 typedef __nv_bfloat16 bf;
 
 // Shared memory: offsets from a 1024-byte aligned base.  Token tiles are [16][64] bf16 with the 128-byte swizzle; the
@@ -128,23 +127,6 @@ __device__ __forceinline__ uint32_t off_x(int row, int col) { return (uint32_t)(
 // other pair of them, so that neither the fragments' stores nor a column's load meet in a bank
 __device__ __forceinline__ uint32_t off_causal(int j, int i) {
   return (uint32_t)((((j >> 1) + 8 * (j & 1)) * 16 + (i ^ (((j >> 2) & 1) << 3))) << 2);
-}
-
-// gelu(z), gelu'(z) and (D2) gelu''(z) of a pair from one tanh.  tanh(x) = 1 - 2 / (1 + e^{2x}) with the fast exponential and
-// division (relative error ~1e-6, as in the forward kernel)
-template <bool D2>
-__device__ __forceinline__ F2 gelu_pair(F2 z, F2& d1, F2& d2) {
-  const F2 z2 = f2mul(z, z);
-  const F2 inner = f2mul(f2mul(z, f2(GELU_C0)), f2fma(z2, f2(GELU_C1), f2(1.f)));
-  const F2 th = f2(1.f - __fdividef(2.f, 1.f + __expf(2.f * inner.x)), 1.f - __fdividef(2.f, 1.f + __expf(2.f * inner.y)));
-  const F2 hz = f2mul(z, f2(0.5f)), sech2 = f2fma(f2neg(th), th, f2(1.f));
-  const F2 du = f2fma(z2, f2(3.f * GELU_C0 * GELU_C1), f2(GELU_C0)), hs = f2mul(hz, sech2);
-  d1 = f2fma(hs, du, f2fma(th, f2(0.5f), f2(0.5f)));
-  if constexpr (D2) {
-    const F2 e = f2fma(f2mul(f2mul(th, du), du), f2(-2.f), f2mul(z, f2(6.f * GELU_C0 * GELU_C1)));
-    d2 = f2fma(sech2, du, f2mul(hs, e));
-  }
-  return f2fma(hz, th, hz);
 }
 
 // The thread's place, read anew in every interval of a stage: what follows from it (a dozen addresses) is then formed where
@@ -257,16 +239,25 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
         break;
       }
     }
+    // one thread of each of five warps (a copy costs its thread a hundred cycles)
     auto issue_inputs = [&](int s, int buf) {
+      const int which = threadIdx.x >> 5;
+      if ((threadIdx.x & 31) != 0 || which > 4) return;
       const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
       const int r0 = row_base + s * CS;
       const uint32_t in = base0 + SM::IN + buf * 3 * TL;
-      mbar_expect_tx(barL, 4 * TL + ET);
-      tma_load_2d(in, &tm_q, 0, r0, barL);
-      tma_load_2d(in + TL, &tm_k, 0, r0, barL);
-      tma_load_2d(in + 2 * TL, &tm_do, 0, r0, barL);
-      bulk_load_1d(base0 + SM::X2 + buf * ET, rec + MLP_REC_X2, ET, barL);
-      bulk_load_1d(base0 + SM::G2P, rec + MLP_REC_G2P, TL, barL);
+      if (which == 0) {
+        mbar_expect_tx(barL, 4 * TL + ET);
+        tma_load_2d(in, &tm_q, 0, r0, barL);
+      } else if (which == 1) {
+        tma_load_2d(in + TL, &tm_k, 0, r0, barL);
+      } else if (which == 2) {
+        tma_load_2d(in + 2 * TL, &tm_do, 0, r0, barL);
+      } else if (which == 3) {
+        bulk_load_1d(base0 + SM::X2 + buf * ET, rec + MLP_REC_X2, ET, barL);
+      } else {
+        bulk_load_1d(base0 + SM::G2P, rec + MLP_REC_G2P, TL, barL);
+      }
     };
     auto issue_late = [&](int s) {  // what is read until I4: V, and G1p where the partial sums of I3 are
       mbar_expect_tx(barG, ET + TL);
@@ -279,6 +270,11 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       const uint8_t* rec = rec0 + (size_t)s * MLP_REC_BYTES;
       if (tid < 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_G1P + 128 * tid));
       else if (tid < 64 + (MLP_REC_BYTES - MLP_REC_Z2) / 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + MLP_REC_Z2 + 128 * (tid - 64)));
+    };
+    // (asked together: an answer takes a hundred cycles)
+    auto wait_both = [&](uint32_t a, uint32_t b, uint32_t parity) {
+      const uint32_t there = mbar_try_wait(a, parity) & mbar_try_wait(b, parity);
+      return there || (mbar_wait_bounded(a, parity) && mbar_wait_bounded(b, parity));
     };
     // what a thread reads of a stage by itself: its pair of Z2 and Zb2 and the row's means, its hidden columns of b1
     F2 zz, zzb, b1v[2], means;
@@ -315,10 +311,8 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
     // ---- item begins: masters into tensor memory, gradients carried from the later chunk, the inputs of its last stage
     int s = s_hi;
     uint32_t buf = nload & 1;
-    if (threadIdx.x == 0) {
-      issue_inputs(s, buf);
-      issue_late(s);
-    }
+    issue_inputs(s, buf);
+    if (threadIdx.x == 0) issue_late(s);
     load_own(s);
     if (threadIdx.x < CS) put_rates(buf, ld_as_float<T>(p.lr, row_base + (size_t)s * CS + threadIdx.x));
     const bool fresh = rank == 0;  // the gradients w.r.t. the final state are zero
@@ -357,14 +351,21 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       for (int cc = 0; cc < 2; ++cc) {
         float v[8][4];
         tmem_ld_8x4(src + 32 * cc, v);
+        if (mat < 2) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const F2 x = f2mul(pr(v[i], j), f2(sc));
+              v[i][2 * j] = x.x;
+              v[i][2 * j + 1] = x.y;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint32_t w[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const F2 x = f2mul(pr(v[2 * i + (j >> 1)], j & 1), f2(sc));
-            w[j] = pack_bf16(x.x, x.y);
-          }
+          for (int j = 0; j < 4; ++j) w[j] = pack_bf16(v[2 * i + (j >> 1)][2 * (j & 1)], v[2 * i + (j >> 1)][2 * (j & 1) + 1]);
           asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + (((4 * cc + i) ^ (P.lane & 7)) << 4)), "r"(w[0]),
                        "r"(w[1]), "r"(w[2]), "r"(w[3])
                        : "memory");
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       rstds = f2(rsqrtf(var.x + p.eps), rsqrtf(var.y + p.eps));
     };
     auto rows_of = [&](int b) {
-      if (!mbar_wait_bounded(barL, nload & 1) || !mbar_wait_bounded(barG, nload & 1)) failed = 1;
+      if (!wait_both(barL, barG, nload & 1)) failed = 1;
       TTT_PLACE
       const uint32_t in = base0 + SM::IN + b * 3 * TL;
       const F2 gam = lds_f2(base0 + SM::LN + 4 * rc), bet = lds_f2(base0 + SM::LN + 4 * (HD + rc));
@@ -460,7 +461,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       const uint32_t sLR = base + SM::LR + buf * CS * 4, sELL = sLR + 2 * CS * 4;
       // ---- I1. G2 and dZb2 (their tiles have been read by the products of the stage before), bf16 copies of W1 and dW1
       ++nload;
-      if (!mbar_wait_bounded(barD, nmma & 1) || !mbar_wait_bounded(barU, nmma & 1)) failed = 1;
+      if (!wait_both(barD, barU, nmma & 1)) failed = 1;
       ++nmma;
       tmem_fence_after_sync();
       {
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       failed = __syncthreads_or(failed);  // 1
       if (failed) break;
       if (s > s_lo) {
-        if (threadIdx.x == 0) issue_inputs(s - 1, buf ^ 1);
+        issue_inputs(s - 1, buf ^ 1);
         prefetch_record(s - 1);
       }
 
@@ -505,7 +506,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             F2 d2;
-            gelu_pair<true>(f2add(pr(z1[nt], r), b1v[nt]), gd1[nt][r], d2);
+            gelu_pair<2>(f2add(pr(z1[nt], r), b1v[nt]), gd1[nt][r], d2);
             gd2[nt][r] = pack_bf16(d2.x, d2.y);
             zq[nt][2 * r] += b1v[nt].x;
             zq[nt][2 * r + 1] += b1v[nt].y;
@@ -584,7 +585,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             F2 d1, unused;
-            const F2 x = gelu_pair<false>(pr(zq[nt], r), d1, unused), d = f2mul(pr(dzw[nt], r), d1);
+            const F2 x = gelu_pair<1>(pr(zq[nt], r), d1, unused), d = f2mul(pr(dzw[nt], r), d1);
             own[2 * nt + r] = pack_bf16(x.x, x.y);
             own2[2 * nt + r] = pack_bf16(d.x, d.y);
             dx[nt][2 * r] = -ell[r] * gl2[nt][2 * r];
@@ -778,8 +779,11 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
       __syncthreads();  // 5
 
       // ---- I6. dW1 += Q^T dZ1b + K^T dZ1, dW2 += X2^T dZ2 + X2b^T dZb2 + dH^T G2, and W1, W2 one stage back: tcgen05.
-      //      Meanwhile warps 0..3: dq = dZ1b W1^T + dA1 K, dk = dZ1 W1^T + dA1^T Q (16 features each); warps 4..7: gl1 = G1 dW1^T,
-      //      db2; warps 8..15: the eta gradients, the next stage's rates, causal matrix and copies of W2, dW2; all: its LayerNorms
+      //      Meanwhile, 16 features of a product each: warps 0..3 dq = dZ1b W1^T + dA1 K, 4..7 dk = dZ1 W1^T + dA1^T Q and db2, 8..11
+      //      gl1 = G1 dW1^T, then the copy of dW2; 12..15 the eta gradients, the next stage's rates and causal matrix, the copy of W2.
+      //      All: the next stage's LayerNorms, warps 12..15 while they would wait for the products.  (dq and dk on the same four
+      //      warps, the copies' eight warps with their LayerNorms last, one product's loads at a time: 192 streams of 128 stages 1 670 us,
+      //      1 614 this way and with GELU's derivatives from one quotient.)
       const size_t r0 = (size_t)(row_base + s * CS) * HD;
       if (threadIdx.x >> 5 == 15) {
         if (elect_one()) {
@@ -803,68 +807,62 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
         __syncwarp();
       }
       if (s > s_lo) row_stats();
-      if (threadIdx.x < 128) {
+      if (threadIdx.x < 384) {
         TTT_PLACE
+        const int np = warp & 3, what = warp >> 2;  // dq, dk, gl1
         const uint32_t a_off = P.a_off();
-        const uint32_t b_off = (lane & 15) * 128 + (((2 * warp + (lane >> 4)) ^ (lane & 7)) << 4);  // 16 rows as k, columns 16 warp.. as n
-        float aq[2][4] = {}, ak[2][4] = {};
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-          uint32_t a[4], c[4], b[4];
-          const uint32_t o = (kk >> 2) * TL + a_off, x = (kk & 3) << 5;
-          ldsm_x4_t(b, base + SM::W1 + b_off + kk * 2048);
-          ldsm_x4(a, (base + SM::DZ1B + o) ^ x);
-          ldsm_x4(c, (base + SM::DZ1 + o) ^ x);
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            mma4(aq[nt], a, b[2 * nt], b[2 * nt + 1]);
-            mma4(ak[nt], c, b[2 * nt], b[2 * nt + 1]);
-          }
-        }
-        uint32_t da[4], dat[4], bk[4], bq[4];
-        ldsm_x4(da, base + SM::DA1 + (lane & 15) * 48 + (lane >> 4) * 16);                                // dA1
-        ldsm_x4_t(dat, base + SM::DA1 + ((lane & 7) + ((lane >> 4) << 3)) * 48 + ((lane >> 3) & 1) * 16);  // dA1^T
-        ldsm_x4_t(bk, tk + b_off);
-        ldsm_x4_t(bq, tq + b_off);
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const int col = 16 * warp + 8 * nt + 2 * t;
-          mma4(aq[nt], da, bk[2 * nt], bk[2 * nt + 1]);
-          mma4(ak[nt], dat, bq[2 * nt], bq[2 * nt + 1]);
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const F2 o = f2add(pr(aq[nt], r), ld_pair<T>(tdo, g + 8 * r, col));
-            static_cast<uint32_t*>(p.d_q)[(r0 + (g + 8 * r) * HD + col) >> 1] = pack_bf16(o.x, o.y);
-            sts_f2(base + SM::EXD + off_x(g + 8 * r, col), pr(ak[nt], r));
-          }
-        }
-      } else if (threadIdx.x < 256) {
-        TTT_PLACE
-        const int np = warp & 3;
-        const uint32_t a_off = P.a_off();
-        const uint32_t b_off = (lane & 15) * 128 + (((2 * np + (lane >> 4)) ^ (lane & 7)) << 4);
+        const uint32_t b_off = (lane & 15) * 128 + (((2 * np + (lane >> 4)) ^ (lane & 7)) << 4);  // 16 rows as k, columns 16 np.. as n
+        const uint32_t ta = base + (what == 0 ? SM::DZ1B : what == 1 ? SM::DZ1 : SM::G1) + a_off, tb = base + (what < 2 ? SM::W1 : SM::DW1) + b_off;
         float c[2][2][4] = {};
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-          uint32_t a[4], b[4];
-          ldsm_x4_t(b, base + SM::DW1 + b_off + kk * 2048);
-          ldsm_x4(a, (base + SM::G1 + (kk >> 2) * TL + a_off) ^ ((kk & 3) << 5));
+        for (int k4 = 0; k4 < 4; ++k4) {
+          uint32_t a[4][4], b[4][4];
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) mma4(c[nt][kk & 1], a, b[2 * nt], b[2 * nt + 1]);
+          for (int i = 0; i < 4; ++i) {
+            ldsm_x4_t(b[i], tb + (4 * k4 + i) * 2048);
+            ldsm_x4(a[i], (ta + k4 * TL) ^ (i << 5));
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) mma4(c[nt][i & 1], a[i], b[i][2 * nt], b[i][2 * nt + 1]);
         }
-        uint32_t bz[4], by[4];
-        ldsm_x4_t(bz, base + SM::DZ2B + b_off);
-        ldsm_x4_t(by, base + SM::DZ2 + b_off);
+        if (what < 2) {
+          uint32_t d[4], b[4];
+          if (what == 0) ldsm_x4(d, base + SM::DA1 + (lane & 15) * 48 + (lane >> 4) * 16);                                  // dA1
+          else ldsm_x4_t(d, base + SM::DA1 + ((lane & 7) + ((lane >> 4) << 3)) * 48 + ((lane >> 3) & 1) * 16);  // dA1^T
+          ldsm_x4_t(b, (what == 0 ? tk : tq) + b_off);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma4(c[nt][0], d, b[2 * nt], b[2 * nt + 1]);
+        }
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const int col = 16 * np + 8 * nt + 2 * t;
-          float cs[4] = {}, ct[4] = {};
-          mma_bf16(cs, ONES, ONES, ONES, ONES, bz[2 * nt], bz[2 * nt + 1]);
-          mma_bf16(ct, ONES, ONES, ONES, ONES, by[2 * nt], by[2 * nt + 1]);
-          if (g == 0) sts_f2(sDB2 + 4 * col, f2add(lds_f2(sDB2 + 4 * col), f2(cs[0] + ct[0], cs[1] + ct[1])));
 #pragma unroll
-          for (int r = 0; r < 2; ++r)
-            sts_f2(base + SM::EXG + off_x(g + 8 * r, col), f2mul(f2add(pr(c[nt][0], r), pr(c[nt][1], r)), f2(-lds_f(sELL + 4 * (g + 8 * r)))));
+          for (int r = 0; r < 2; ++r) {
+            const F2 o = f2add(pr(c[nt][0], r), pr(c[nt][1], r));
+            if (what == 0) {
+              const F2 q = f2add(o, ld_pair<T>(tdo, g + 8 * r, col));
+              static_cast<uint32_t*>(p.d_q)[(r0 + (g + 8 * r) * HD + col) >> 1] = pack_bf16(q.x, q.y);
+            } else if (what == 1) {
+              sts_f2(base + SM::EXD + off_x(g + 8 * r, col), o);
+            } else {
+              sts_f2(base + SM::EXG + off_x(g + 8 * r, col), f2mul(o, f2(-lds_f(sELL + 4 * (g + 8 * r)))));
+            }
+          }
+        }
+        if (what == 1) {
+          uint32_t bz[4], by[4];
+          ldsm_x4_t(bz, base + SM::DZ2B + b_off);
+          ldsm_x4_t(by, base + SM::DZ2 + b_off);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            const int col = 16 * np + 8 * nt + 2 * t;
+            float cs[4] = {}, ct[4] = {};
+            mma_bf16(cs, ONES, ONES, ONES, ONES, bz[2 * nt], bz[2 * nt + 1]);
+            mma_bf16(ct, ONES, ONES, ONES, ONES, by[2 * nt], by[2 * nt + 1]);
+            if (g == 0) sts_f2(sDB2 + 4 * col, f2add(lds_f2(sDB2 + 4 * col), f2(cs[0] + ct[0], cs[1] + ct[1])));
+          }
         }
       } else {
         if (threadIdx.x >> 5 == 13) {
@@ -882,11 +880,14 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
           if (lane < CS) p.part_te[(size_t)row_base + (size_t)s * CS + lane] = lane == CS - 1 ? dte + sum : dte;
         }
         if (s > s_lo) {
-          if (threadIdx.x >> 5 == 8) causal_first(s - 1, buf ^ 1);
-          second_layer_copies();
+          if (threadIdx.x >> 5 == 12) causal_first(s - 1, buf ^ 1);
+          rows_of(buf ^ 1);
         }
       }
-      if (s > s_lo) rows_of(buf ^ 1);
+      if (s > s_lo) {
+        if (threadIdx.x >= 256) second_layer_copies();
+        if (threadIdx.x < 384) rows_of(buf ^ 1);
+      }
       __syncthreads();  // 6
       // ---- outputs of the stage: dk = (products) - l o gl1 - dT, dv = dT
       {

@@ -73,33 +73,6 @@ struct MlpSmem {
 static_assert(MlpSmem::TOTAL <= 227 * 1024, "shared-memory tiles exceed one SM");
 static_assert(MlpSmem::OFF_M1 % 1024 == 0 && MlpSmem::OFF_M2 % 16 == 0 && MlpSmem::OFF_LR % 16 == 0 && MlpSmem::OFF_BAR % 8 == 0, "alignment");
 
-// tanh-approximated GELU of a pair and (DERIV) its derivative times sc, from q = 1 / (1 + e^{2u}), tanh(u) = 1 - 2q (relative
-// error ~1e-6; the hardware tanh.approx is only good to ~5e-4, which shows after a few dozen chained stages):
-//     gelu = z (1 - q),   gelu' = (1 - q) (1 + 2 z q u'),   u = c0 z (1 + c1 z^2).
-// The pair's quotients share one reciprocal, 1/a = b / (ab): three calls of the special-function unit instead of four.
-// Exponents stop at 2^60, where tanh is 1, so that the product stays finite; the 2^-60 that q keeps there is taken off, or its
-// product with z^3 would show in gelu' of a z in the millions.
-__device__ __forceinline__ float ex2_approx(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-template <bool DERIV>
-__device__ __forceinline__ F2 gelu2(F2 z, F2& deriv, float sc) {
-  constexpr float C0 = 0.7978845608028654f, C1 = 0.044715f, L2E2 = 2.f * 1.4426950408889634f;
-  const F2 z2 = f2mul(z, z);
-  const F2 a = f2mul(z, f2fma(z2, f2(L2E2 * C0 * C1), f2(L2E2 * C0)));
-  const F2 d = f2add(f2(ex2_approx(fminf(a.x, 60.f)), ex2_approx(fminf(a.y, 60.f))), f2(1.f));
-  const F2 nq = f2fma(f2(rcp_approx(-(d.x * d.y))), f2(d.y, d.x), f2(0x1p-60f)), y = f2mul(z, nq);
-  if constexpr (DERIV) deriv = f2mul(f2fma(nq, f2(sc), f2(sc)), f2fma(y, f2fma(z2, f2(-6.f * C0 * C1), f2(-2.f * C0)), f2(1.f)));
-  return f2add(z, y);
-}
-
 namespace {
 template <int BAR>
 __device__ __forceinline__ void mlp_group_sync() {
@@ -447,7 +420,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             const F2 b1 = f2(__uint_as_float(lds_word(base + SM::OFF_B1 + par * MLP_E * 4 + 4 * (32 * warp + 8 * i + g))));
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-              const F2 x = gelu2<true>(f2fma(pr(z1[i >> 1][nt], i & 1), f2(wscale), b1), d1[i][nt], wscale);
+              F2 unused;
+              const F2 x = gelu_pair<1>(f2fma(pr(z1[i >> 1][nt], i & 1), f2(wscale), b1), d1[i][nt], unused, wscale);
               x2[i][nt] = pack_bf16(x.x, x.y);
             }
           }
@@ -693,7 +667,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
               F2 unused;
-              const F2 x = gelu2<false>(f2fma(pr(zq[i >> 1][nt], i & 1), f2(wscale), b1), unused, 1.f);
+              const F2 x = gelu_pair<0>(f2fma(pr(zq[i >> 1][nt], i & 1), f2(wscale), b1), unused, unused);
               xb[i][nt] = movm_t(pack_bf16(x.x, x.y));
             }
           }

@@ -288,6 +288,43 @@ __device__ __forceinline__ void report_timeout(uint32_t* status, uint32_t where,
   }
 }
 
+// ---- TTT-MLP: tanh-approximated GELU -------------------------------------------------------------------------------
+// gelu(z), (D > 0) gelu'(z) times sc and (D > 1) gelu''(z) of a pair, from q = 1 / (1 + e^{2u}), tanh(u) = 1 - 2q (relative error
+// ~1e-6; the hardware tanh.approx is only good to ~5e-4, which shows after a few dozen chained stages):
+//     u = c0 z (1 + c1 z^2), m = -2 u':   gelu = z (1 - q),   gelu' = (1 - q) (1 - z q m),
+//     gelu'' = q (1 - q) (-4 m - 4 c0 - z m^2 (1 - 2q))      (z u'' = -m - 2 c0)
+// The pair's quotients share one reciprocal, 1/a = b / (ab): three calls of the special-function unit instead of four.
+// Exponents stop at 2^60, where tanh is 1, so that the product stays finite; the 2^-60 that q keeps there is taken off, or its
+// product with z^3 would show in gelu' of a z in the millions.
+__device__ __forceinline__ float ex2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+template <int D>
+__device__ __forceinline__ F2 gelu_pair(F2 z, F2& d1, F2& d2, float sc = 1.f) {
+  constexpr float C0 = 0.7978845608028654f, C1 = 0.044715f, L2E2 = 2.f * 1.4426950408889634f;
+  const F2 z2 = f2mul(z, z);
+  const F2 a = f2mul(z, f2fma(z2, f2(L2E2 * C0 * C1), f2(L2E2 * C0)));
+  const F2 d = f2add(f2(ex2_approx(fminf(a.x, 60.f)), ex2_approx(fminf(a.y, 60.f))), f2(1.f));
+  const F2 nq = f2fma(f2(rcp_approx(-(d.x * d.y))), f2(d.y, d.x), f2(0x1p-60f)), y = f2mul(z, nq);  // -q, -z q
+  if constexpr (D > 0) {
+    const F2 m = f2fma(z2, f2(-6.f * C0 * C1), f2(-2.f * C0));
+    d1 = f2mul(f2fma(nq, f2(sc), f2(sc)), f2fma(y, m, f2(1.f)));
+    if constexpr (D > 1) {
+      const F2 p = f2add(nq, f2(1.f));
+      const F2 b = f2fma(f2mul(f2mul(z, m), m), f2add(p, nq), f2fma(m, f2(4.f), f2(4.f * C0)));
+      d2 = f2mul(f2mul(nq, p), b);
+    }
+  }
+  return f2add(z, y);
+}
+
 // ---- rank-16 updates of a state in tensor memory by tcgen05 (TTT-MLP) ----------------------------------------------
 // operand descriptor of token tiles read MN-major: 64 contiguous elements (128 bytes, swizzled) x 8 tokens per atom, the
 // other 8 tokens 1024 bytes on, the next 64 elements (A: M = 128) one tile on
