@@ -47,10 +47,10 @@ def test_mlp_rejects_float32():
                                  tb.FusedTttConfig.new(16, 64, 1e-6, 256, 1))
 
 
-@pytest.mark.parametrize("B,H,NS,eta", [(1, 1, 2, "plain"), (2, 1, 3, "zero"), (1, 3, 4, "thirds"), (3, 1, 5, "zero"), (21, 8, 9, "thirds")])
+@pytest.mark.parametrize("B,H,NS,eta", [(1, 1, 2, "plain"), (2, 1, 3, "zero"), (1, 3, 4, "thirds"), (3, 1, 5, "zero"), (21, 8, 24, "thirds")])
 def test_mlp_forward_at_the_edges_of_its_rings(B, H, NS, eta):
     """Fewer stages than slots of inputs, just as many, one and two more (every ring and parity of the kernel wraps), streams in
-    chunks handed from block to block (168 of them), an update coefficient of zero (the state stays) and one that is no power
+    chunks handed from block to block (168 of them, in training and in inference), an update coefficient of zero (the state stays) and one that is no power
     of two.  Saving state for the backward changes nothing in the results of a stream in one piece; a chunk ends with float32
     biases added up once more, which moves bf16 results by roundings."""
     import ttt_rs_b200 as tb

@@ -622,11 +622,12 @@ int ttt_internal_linear_backward(const ttt_dims* d, const void* xq, const void* 
   return TTT_OK;
 }
 
-int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* w1, const void* b1,
-                    const void* w2, const void* b2, const void* token_eta, const void* ttt_lr_eta,
-                    const void* ln_weight, const void* ln_bias, void* output, void* w1_out, void* b1_out, void* w2_out,
-                    void* b2_out, void* backward_workspace, size_t backward_workspace_bytes, void* status,
-                    void* stream) {
+// ttt_mlp_forward, with a scratch buffer in place of a workspace if there is one (inference)
+static int mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* w1, const void* b1,
+                       const void* w2, const void* b2, const void* token_eta, const void* ttt_lr_eta,
+                       const void* ln_weight, const void* ln_bias, void* output, void* w1_out, void* b1_out, void* w2_out,
+                       void* b2_out, void* backward_workspace, size_t backward_workspace_bytes, void* scratch,
+                       size_t scratch_bytes, void* status, void* stream) {
   int rc = check_dims(d);
   if (rc != TTT_OK) return rc;
   if (d->dtype != TTT_BF16) return fail(TTT_ERR_UNSUPPORTED, "the TTT-MLP kernel is built for bf16 only");
@@ -658,17 +659,41 @@ int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const voi
   p.status = static_cast<uint32_t*>(status);
   p.bwd_ws = static_cast<float*>(backward_workspace);
   p.bwd_ws_stride = wl.stride_floats;
+  p.records = 1;
   p.walk_only = 0;
   // with a workspace the launch is persistent and uses the workspace's scheduler words (the backward re-zeroes them)
   p.sched = backward_workspace != nullptr ? reinterpret_cast<int*>(static_cast<float*>(backward_workspace) + wl.off_sched)
                                           : nullptr;
   p.nstreams = d->batch * d->heads;
   p.CH = p.NCH = 0;
+  const size_t need = scratch != nullptr ? ttt::mlp_fwd_scratch_floats(d->seq_len / d->mini_batch, p.nstreams) : 0;
+  if (backward_workspace == nullptr && need != 0 && scratch_bytes / sizeof(float) >= need)
+    ttt::mlp_fwd_use_scratch(p, static_cast<float*>(scratch), p.nstreams);
   p.handoff_polls = g_handoff_polls.load();
   p.H = d->heads; p.T = d->seq_len; p.NS = d->seq_len / d->mini_batch; p.eps = d->epsilon;
   cudaError_t e = ttt::launch_mlp_fwd(maps, p, d->batch * d->heads, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "MLP forward launch failed: %s", cudaGetErrorString(e));
   return TTT_OK;
+}
+
+int ttt_mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* w1, const void* b1,
+                    const void* w2, const void* b2, const void* token_eta, const void* ttt_lr_eta,
+                    const void* ln_weight, const void* ln_bias, void* output, void* w1_out, void* b1_out, void* w2_out,
+                    void* b2_out, void* backward_workspace, size_t backward_workspace_bytes, void* status,
+                    void* stream) {
+  return mlp_forward(d, xq, xk, xv, w1, b1, w2, b2, token_eta, ttt_lr_eta, ln_weight, ln_bias, output, w1_out, b1_out, w2_out,
+                     b2_out, backward_workspace, backward_workspace_bytes, nullptr, 0, status, stream);
+}
+
+size_t ttt_internal_mlp_infer_scratch_bytes(const ttt_dims* d) {
+  return check_dims(d) == TTT_OK ? sizeof(float) * ttt::mlp_fwd_scratch_floats(d->seq_len / d->mini_batch, d->batch * d->heads) : 0;
+}
+int ttt_internal_mlp_infer(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* w1, const void* b1,
+                           const void* w2, const void* b2, const void* token_eta, const void* ttt_lr_eta,
+                           const void* ln_weight, const void* ln_bias, void* output, void* w1_out, void* b1_out, void* w2_out,
+                           void* b2_out, void* scratch, size_t scratch_bytes, void* status, void* stream) {
+  return mlp_forward(d, xq, xk, xv, w1, b1, w2, b2, token_eta, ttt_lr_eta, ln_weight, ln_bias, output, w1_out, b1_out, w2_out,
+                     b2_out, nullptr, 0, scratch, scratch_bytes, status, stream);
 }
 
 }  // extern "C"
@@ -1174,6 +1199,7 @@ extern "C" int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, cons
     f.status = static_cast<uint32_t*>(status);
     f.bwd_ws = ws;
     f.bwd_ws_stride = l.stride_floats;
+    f.records = 1;
     f.walk_only = 1;
     f.sched = reinterpret_cast<int*>(ws + l.off_sched);
     f.handoff_polls = g_handoff_polls.load();

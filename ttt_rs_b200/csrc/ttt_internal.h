@@ -27,6 +27,14 @@ int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, const void* xk,
                               void* grad_ln_weight, void* grad_ln_bias, int reduced_dtype, void* workspace,
                               size_t workspace_bytes, int workspace_from_forward, void* status, void* stream);
 
+// ttt_mlp_forward without a backward to follow.  scratch (16-byte aligned; null: none): memory to park streams' states in,
+// with which more streams than SMs need not run in whole waves; bytes 0: not used for these dims on the current device.
+size_t ttt_internal_mlp_infer_scratch_bytes(const ttt_dims* d);
+int ttt_internal_mlp_infer(const ttt_dims* d, const void* xq, const void* xk, const void* xv, const void* w1, const void* b1,
+                           const void* w2, const void* b2, const void* token_eta, const void* ttt_lr_eta,
+                           const void* ln_weight, const void* ln_bias, void* output, void* w1_out, void* b1_out, void* w2_out,
+                           void* b2_out, void* scratch, size_t scratch_bytes, void* status, void* stream);
+
 // Inference forward over the first `d->seq_len` tokens (whole mini-batches) of sequences whose rows are `seq_pitch` tokens
 // apart in xq, xk, xv, output and `lr_pitch` elements apart in ttt_lr_eta; token_eta: the first mini-batch's.
 int ttt_internal_linear_infer(const ttt_dims* d, int seq_pitch, int lr_pitch, const void* xq, const void* xk,

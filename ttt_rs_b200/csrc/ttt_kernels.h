@@ -117,8 +117,9 @@ struct MlpFwdParams {
   void* w2_out;
   void* b2_out;
   uint32_t* status;
-  float* bwd_ws;         // optional: the backward's workspace; the forward then leaves there the final state and a record
-  size_t bwd_ws_stride;  // of every stage
+  float* bwd_ws;         // optional: a block per stream to park its state in between work items
+  size_t bwd_ws_stride;
+  int records;           // it is the backward's workspace: the final state and a record of every stage are left there
   int walk_only;         // only that: no output and no final state for the caller
   int* sched;            // with bwd_ws (null otherwise): [1 + B*H] work-item counter and per-stream count of finished chunks (the
                          // persistent launch; zeroed by the launcher)
@@ -386,6 +387,9 @@ cudaError_t launch_gemm_bf16_tn(const CUtensorMap* maps, const GemmParams& p, bo
 
 // bf16 only.  maps: q, k, v, out.
 cudaError_t launch_mlp_fwd(const CUtensorMap* maps, const MlpFwdParams& p, int nstreams, cudaStream_t st);
+// scratch of an inference call (current device), 0: none is used
+size_t mlp_fwd_scratch_floats(int NS, int nstreams);
+void mlp_fwd_use_scratch(MlpFwdParams& p, float* scratch, int nstreams);
 
 // dtype: 0 = float32, 1 = bfloat16.  seg: features per head, 64 or 32 (two heads per tile).  mb: tokens per
 // mini-batch, 16 or 8 (the tile maps then have boxes of 8 rows).

@@ -31,10 +31,12 @@
 // of sixteen warps 121 / 2 355; K_next W1_next taken as K_next W1 plus a product with G1p, which takes W1's refresh off the chain, 111 / 2 284.
 //
 // Scheduling.  One CTA fills an SM, so a launch of one CTA per stream runs in whole
-// waves: 192 streams on 148 SMs cost two stream-times.  When the caller passes the backward's workspace (training),
-// the kernel is launched persistently instead: blocks take work items (stream, chunk of stages: mlp_chunk_stages), first
-// chunks of all streams first, and a chunk hands the state to the next one through the stream's workspace block (which
-// is where the final state goes anyway) behind a per-stream counter -- the scheme of the TTT-Linear backward.
+// waves: 192 streams on 148 SMs cost two stream-times.  When there is memory to park a stream's state in -- the backward's
+// workspace in training (where the final state goes anyway), a scratch buffer of the host path in inference with more
+// streams than SMs -- blocks take work items (stream, chunk of stages: mlp_chunk_stages) instead, first
+// chunks of all streams first, and a chunk hands the state to the next one through the stream's block of that memory
+// behind a per-stream counter -- the scheme of the TTT-Linear backward.  Inference: 192 streams of 128 stages
+// 818 -> 581 us, 384 of 64 stages 633 -> 610, 300 of 32 stages 325 -> 293.
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
 #include "ttt_stage.cuh"
@@ -180,8 +182,9 @@ __device__ __forceinline__ F2 row_sum2(float a, float b) {
 }
 }  // namespace
 
-// SAVE: persistent, with the backward's workspace (the tests of a record pointer in the stage loop cost inference 1.5 %)
-template <bool SAVE>
+// CHUNKS: work items of several stages; SAVE: into the backward's workspace, with its records (the tests of a record pointer in
+// the stage loop cost inference 1.5 %)
+template <bool SAVE, bool CHUNKS>
 __global__ void __launch_bounds__(MLP_THREADS, 1)
     ttt_mlp_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, const MlpFwdParams p) {
@@ -203,8 +206,10 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   const bool output_group = __shfl_sync(0xffffffffu, threadIdx.x >> 8, 0) != 0;
   const int tid = threadIdx.x & (MLP_GROUP - 1), lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int NS = p.NS, CH = SAVE ? p.CH : NS, NCH = SAVE ? p.NCH : 1;
-  const int nitems = SAVE ? p.nstreams * NCH : (int)gridDim.x;
+  static_assert(CHUNKS || !SAVE, "the backward's workspace comes with chunks");
+  constexpr size_t HANDOFF = (SAVE ? 4 : 2) * HD * MLP_E;  // biases, in floats, behind the masters
+  const int NS = p.NS, CH = CHUNKS ? p.CH : NS, NCH = CHUNKS ? p.NCH : 1;
+  const int nitems = CHUNKS ? p.nstreams * NCH : (int)gridDim.x;
 
   if (threadIdx.x < 32) tmem_alloc(w_tmem, 512);
   if (threadIdx.x == MLP_GROUP) {
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   for (int round = 0;; ++round) {
     // ---- next work item: (stream, chunk); one block per stream and a single chunk when not persistent
     int item;
-    if constexpr (SAVE) {
+    if constexpr (CHUNKS) {
       if (threadIdx.x == 0) sts_word(w_item, (uint32_t)atomicAdd(&p.sched[0], 1));
       __syncthreads();
       item = (int)lds_word(w_item);
@@ -269,15 +274,15 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
       item = (round == 0) ? (int)blockIdx.x : nitems;
     }
     if (item >= nitems) break;
-    const int chunk = SAVE ? item / p.nstreams : 0, stream = SAVE ? item - chunk * p.nstreams : item;
+    const int chunk = CHUNKS ? item / p.nstreams : 0, stream = CHUNKS ? item - chunk * p.nstreams : item;
     const int head = stream % p.H, row_base = stream * p.T;
     const int s_lo = chunk * CH, s_hi = min(s_lo + CH, NS) - 1;
-    // Optional: the backward's per-stream workspace block (layout in ttt_kernels.h).  The lr-scaled inner gradients of
+    // The stream's block of the workspace or scratch buffer (layout in ttt_kernels.h).  SAVE: the lr-scaled inner gradients of
     // every stage (the bf16 operands of the state updates) and the final state go there, so that the backward can
     // start its reverse walk at once.
-    float* const bws = SAVE ? p.bwd_ws + (size_t)stream * p.bwd_ws_stride : nullptr;
-    uint8_t* const rec0 = SAVE ? reinterpret_cast<uint8_t*>(bws + 4 * HD * MLP_E + MLP_BWD_HANDOFF_FLOATS) : nullptr;
-    if (SAVE && chunk > 0) {
+    float* const bws = CHUNKS ? p.bwd_ws + (size_t)stream * p.bwd_ws_stride : nullptr;
+    uint8_t* const rec0 = SAVE ? reinterpret_cast<uint8_t*>(bws + HANDOFF + MLP_BWD_HANDOFF_FLOATS) : nullptr;
+    if (CHUNKS && chunk > 0) {
       // wait (bounded) until the previous chunk of this stream has parked its state in the workspace block
       int ok = 1;
       if (threadIdx.x == 0) {
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {
             float v[8][4];
-            if (SAVE && chunk > 0) {
+            if (CHUNKS && chunk > 0) {
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const float4 a = __ldcg(parked + mat * (HD * MLP_E / 4) + (8 * cc + i) * 32);
@@ -381,8 +386,8 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
             tmem_st_8x4(tm_own + 128 * mat + 32 * cc, v);
             put_copy(mat, n & 1, cc, v);
           }
-        const float* const ho = bws + 4 * HD * MLP_E;
-        const bool first = !SAVE || chunk == 0;
+        const float* const ho = bws + HANDOFF;
+        const bool first = !CHUNKS || chunk == 0;
         b1c = first ? ld_as_float<T>(p.b1, (size_t)stream * MLP_E + b1_col) : __ldcg(ho + MLP_HO_B1 + b1_col);
         sts_word(base + SM::OFF_B1 + (n & 1) * MLP_E * 4 + 4 * b1_col, __float_as_uint(b1c));
 #pragma unroll
@@ -543,15 +548,15 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 
       // ---- the item's state: float32 masters and biases
       mlp_group_sync<1>();  // (the shares of b2)
-      float* const ho = bws + 4 * HD * MLP_E;
-      const bool park = SAVE && chunk < NCH - 1, results = !park && !(SAVE && p.walk_only);
+      float* const ho = bws + HANDOFF;
+      const bool park = CHUNKS && chunk < NCH - 1, results = !park && !(SAVE && p.walk_only);
 #pragma unroll
       for (int mat = 0; mat < 2; ++mat)
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           float v[8][4];
           tmem_ld_8x4(tm_own + 128 * mat + 32 * cc, v);
-          if (SAVE) {  // for the next chunk of this stream, or as the backward takes them up
+          if (SAVE || park) {  // for the next chunk of this stream, or as the backward takes them up
             float4* const to = reinterpret_cast<float4*>(bws + mat * HD * MLP_E) + warp * 16 * 32 + lane;
 #pragma unroll
             for (int i = 0; i < 8; ++i) to[(8 * cc + i) * 32] = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
@@ -758,20 +763,19 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 }
 
 cudaError_t launch_mlp_fwd(const CUtensorMap* m, const MlpFwdParams& p, int nstreams, cudaStream_t st) {
-  const bool save = p.bwd_ws != nullptr;
-  auto kfn = save ? ttt_mlp_fwd_kernel<true> : ttt_mlp_fwd_kernel<false>;
-  static DeviceValue resident[2];
+  const bool chunks = p.bwd_ws != nullptr, save = chunks && p.records;
+  auto kfn = save ? ttt_mlp_fwd_kernel<true, true> : chunks ? ttt_mlp_fwd_kernel<false, true> : ttt_mlp_fwd_kernel<false, false>;
+  static DeviceValue resident[3];
   int sms = 0, per_sm = 0;
-  cudaError_t e = resident[save].get(0, &per_sm, [&](int* n) {
+  cudaError_t e = resident[save ? 2 : chunks].get(0, &per_sm, [&](int* n) {
     const cudaError_t a = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MlpSmem::TOTAL);
     return a != cudaSuccess ? a : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kfn, MLP_THREADS, MlpSmem::TOTAL);
   });
   if (e != cudaSuccess) return e;
-  if (!save) {  // no workspace to park state in: one block per stream
+  if (!chunks) {  // nothing to park state in: one block per stream
     kfn<<<nstreams, MLP_THREADS, MlpSmem::TOTAL, st>>>(m[0], m[1], m[2], p);
     return cudaGetLastError();
   }
-  // persistent: as many blocks as are co-resident (they wait on one another's hand-offs), never more than items
   if ((e = device_sms(&sms)) != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
   MlpFwdParams pp = p;
@@ -781,7 +785,26 @@ cudaError_t launch_mlp_fwd(const CUtensorMap* m, const MlpFwdParams& p, int nstr
   pp.CH = mlp_chunk_stages(p.NS, nstreams, grid);
   pp.NCH = (p.NS + pp.CH - 1) / pp.CH;
   if ((e = cudaMemsetAsync(pp.sched, 0, sizeof(int) * (size_t)(1 + nstreams), st)) != cudaSuccess) return e;
+  if (!save) {  // (an item waits only for one of smaller index, which a block holds that runs or has run)
+    kfn<<<grid, MLP_THREADS, MlpSmem::TOTAL, st>>>(m[0], m[1], m[2], pp);
+    return cudaGetLastError();
+  }
+  // as many blocks as are co-resident, never more than streams
   void* args[] = {(void*)&m[0], (void*)&m[1], (void*)&m[2], (void*)&pp};
   return cudaLaunchCooperativeKernel((const void*)kfn, dim3(grid), dim3(MLP_THREADS), args, MlpSmem::TOTAL, st);
+}
+// Floats per stream, and whether the scheme above gains anything (one CTA per SM): no more streams than SMs, or chunks of less
+// than the whole sequence would cost more than the waves they even out, and no scratch is used.
+constexpr size_t MLP_PARK_FLOATS = 2 * HD * MLP_E + MLP_BWD_HANDOFF_FLOATS;
+size_t mlp_fwd_scratch_floats(int NS, int nstreams) {
+  int sms = 0;
+  if (device_sms(&sms) != cudaSuccess || nstreams <= sms || mlp_chunk_stages(NS, nstreams, sms) >= NS) return 0;
+  return MLP_PARK_FLOATS * (size_t)nstreams + (size_t)((1 + nstreams + 3) & ~3);
+}
+void mlp_fwd_use_scratch(MlpFwdParams& p, float* scratch, int nstreams) {
+  p.bwd_ws = scratch;
+  p.bwd_ws_stride = MLP_PARK_FLOATS;
+  p.records = 0;
+  p.sched = reinterpret_cast<int*>(scratch + MLP_PARK_FLOATS * (size_t)nstreams);
 }
 }  // namespace ttt
