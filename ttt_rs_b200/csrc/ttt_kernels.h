@@ -335,7 +335,9 @@ struct MlpBwdParams {
 // (order: mlp_master_at; W1 and W2 divided by -token_eta[15], as the kernels carry them, unless that is zero), the hand-off
 // record between work items, then one record per stage, written by the forward.
 constexpr int MLP_BWD_HANDOFF_FLOATS = 2 * 256 + 4 * 64;
-constexpr int MLP_HO_B1 = 0, MLP_HO_B2 = 256, MLP_HO_DB1 = 320, MLP_HO_DB2 = 576, MLP_HO_DG = 640;  // DG: weight, bias [2][64]
+constexpr int MLP_HO_B1 = 0, MLP_HO_B2 = 256;                             // the forward's: b1, eight shares of b2 [8][64]
+constexpr int MLP_HO_DB1 = 320, MLP_HO_DB2 = 576, MLP_HO_DG = 640;        // the backward's, once the forward is done; DG: weight, bias [2][64]
+static_assert(MLP_HO_B2 + 8 * 64 <= MLP_BWD_HANDOFF_FLOATS && MLP_HO_DG + 2 * 64 <= MLP_BWD_HANDOFF_FLOATS, "hand-off record");
 // element (hidden feature e, feature f) of a master, as a float index: 16-byte pieces of 32 consecutive hidden features
 // (the lanes of a warp) side by side
 __host__ __device__ inline int mlp_master_at(int e, int f) { return ((((e >> 5) * 16 + (f >> 2)) * 32 + (e & 31)) << 2) + (f & 3); }

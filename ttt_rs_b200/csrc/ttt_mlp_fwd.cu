@@ -391,10 +391,12 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         b1c = first ? ld_as_float<T>(p.b1, (size_t)stream * MLP_E + b1_col) : __ldcg(ho + MLP_HO_B1 + b1_col);
         sts_word(base + SM::OFF_B1 + (n & 1) * MLP_E * 4 + 4 * b1_col, __float_as_uint(b1c));
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {  // b2: the first warp's share
+        for (int h = 0; h < 2; ++h) {  // b2: at first all of it the first warp's share
           const int c = lane + 32 * h;
-          const float b = first ? ld_as_float<T>(p.b2, (size_t)stream * HD + c) : __ldcg(ho + MLP_HO_B2 + c);
-          sts_word(base + SM::OFF_B2 + (n & 1) * SM::B2 + 4 * (warp * HD + c), warp == 0 ? __float_as_uint(b * winv) : 0u);
+          float b = 0.f;
+          if (!first) b = __ldcg(ho + MLP_HO_B2 + warp * HD + c);
+          else if (warp == 0) b = ld_as_float<T>(p.b2, (size_t)stream * HD + c) * winv;
+          sts_word(base + SM::OFF_B2 + (n & 1) * SM::B2 + 4 * (warp * HD + c), __float_as_uint(b));
         }
         tmem_wait_st();
         tmem_fence_before_sync();
@@ -575,12 +577,17 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         }
       if (park) ho[MLP_HO_B1 + b1_col] = b1c;
       if (results) st_from_float<T>(p.b1_out, (size_t)stream * MLP_E + b1_col, b1c);
-      if (tid < HD) {
+      // (the shares as they are: a stream's results are the same bits whether it runs in chunks or not)
+      if (park) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          ho[MLP_HO_B2 + tid + MLP_GROUP * h] = __uint_as_float(lds_word(base + SM::OFF_B2 + (n & 1) * SM::B2 + 4 * (tid + MLP_GROUP * h)));
+      }
+      if (results && tid < HD) {
         float b = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) b += __uint_as_float(lds_word(base + SM::OFF_B2 + (n & 1) * SM::B2 + 4 * (w * HD + tid)));
-        if (park) ho[MLP_HO_B2 + tid] = b * wscale;
-        if (results) st_from_float<T>(p.b2_out, (size_t)stream * HD + tid, b * wscale);
+        st_from_float<T>(p.b2_out, (size_t)stream * HD + tid, b * wscale);
       }
       if (park) {
         __threadfence();
