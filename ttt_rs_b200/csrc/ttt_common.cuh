@@ -432,6 +432,14 @@ struct TokenEtaElement {
 // pdl_wait, so that at most one kernel is unfinished when a later one starts.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Both, for a kernel that reads nothing before: only its launch and what it sets up for itself overlap the kernel before it.  (The
+// products, the prologue, the epilogue and the three-group scan of a layer: 1 x 1001 tokens x 768 107 -> 97 us, 4 x 43 tokens x 1024
+// 57 -> 47, a token of 51 sequences as graphs replay it 35.8 -> 27.0.)  Only where it does not matter which SMs the kernel before
+// leaves first: blocks that several to an SM are to be spread evenly fill those (ttt_linear_fwd.cu).
+__device__ __forceinline__ void pdl_join() {
+  pdl_wait();
+  pdl_go();
+}
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchAttribute at;

@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers are initialised and both hold their tensor memory
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_join();  // (barriers, tensor memory and descriptors are there)
 
   if (warp == 0) {
     // ---------------- TMA producer: one ring over all the tiles of this CTA
@@ -534,8 +535,7 @@ static cudaError_t launch_gemm_t(const CUtensorMap* m, const GemmParams& p, cuda
   if (e != cudaSuccess) return e;
   const long ntiles = (long)((p.N + GEMM_BN - 1) / GEMM_BN) * ((p.M + GEMM_BM - 1) / GEMM_BM);
   const int grid = (int)(ntiles < sms ? ntiles : sms);  // persistent: one CTA per SM walks the tiles
-  kfn<<<grid, GEMM_THREADS, SM::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
-  return cudaGetLastError();
+  return launch_dependent(kfn, grid, GEMM_THREADS, SM::DYN_BYTES, st, m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
 }
 
 // pair form: clusters of two CTAs, as many as can be resident (a cluster waits on nothing outside itself)
@@ -544,7 +544,7 @@ static cudaError_t launch_gemm_pair_t(const CUtensorMap* m, const GemmParams& p,
   using SM = GemmSmem<FUSED, true>;
   auto kfn = ttt_gemm_bf16_tn_kernel<FUSED, true>;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -570,6 +570,9 @@ static cudaError_t launch_gemm_pair_t(const CUtensorMap* m, const GemmParams& p,
   const long ntiles = (long)((p.N + GEMM_BN - 1) / GEMM_BN) * ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM));
   if (nclusters > ntiles) nclusters = (int)ntiles;
   cfg.gridDim = dim3(2 * nclusters);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (as launch_dependent)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kfn, m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
 }
 

@@ -89,8 +89,6 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
   const bool rope = p.rope_mode != 0;
   const bool rope_wrap = p.rope_mode == 1;
   const float log2_theta = log2f(p.rope_theta);
-  TokenEtaElement te;
-  if (sizeof(T) == 2 && blockIdx.x == 0) te.load(p.te, tid);
   if (rope && rope_wrap) {
     for (int e = tid; e < p.pos_mod * 32; e += PRO_THREADS) {
       const int pos = e >> 5, i = e & 31;
@@ -100,7 +98,12 @@ __global__ void __launch_bounds__(PRO_THREADS, (CONV || sizeof(T) == 4) ? 1 : 3)
       rope_tab[pos][i] = make_float2(c, s);
     }
   }
-  if (sizeof(T) == 2 && blockIdx.x == 0) te.store(p.te, tid);
+  pdl_join();
+  if (sizeof(T) == 2 && blockIdx.x == 0) {
+    TokenEtaElement te;
+    te.load(p.te, tid);
+    te.store(p.te, tid);
+  }
   __syncthreads();
 
   const int hq = lane / SUBS, sub = lane % SUBS;
@@ -292,6 +295,7 @@ __global__ void __launch_bounds__(MAXCH == 16 ? 512 : EPI_THREADS, (MAXCH == 16 
       v[1] = f2(__uint_as_float(raw.z), __uint_as_float(raw.w));
     }
   };
+  pdl_join();
   TileWalk ahead(blockIdx.x, gridDim.x, ntiles, tiles_per_b), cur = ahead;
   auto fetch = [&](int buf) {  // the next tile that is not on its way yet
     if (ahead.valid() && my_grp < ngroups) {
@@ -408,24 +412,17 @@ static int prologue_grid(int B, int H, int T, int head_dim, int first_chunk, int
 }
 
 template <typename T, int FD>
-static void launch_pro_t(const LayerProParams& p, int grid, cudaStream_t st) {
+static cudaError_t launch_pro_t(const LayerProParams& p, int grid, cudaStream_t st) {
   if (p.conv_q_w != nullptr)
-    ttt_layer_prologue_kernel<T, true, FD><<<grid, PRO_THREADS, 0, st>>>(p);
-  else
-    ttt_layer_prologue_kernel<T, false, FD><<<grid, PRO_THREADS, 0, st>>>(p);
+    return launch_dependent(ttt_layer_prologue_kernel<T, true, FD>, grid, PRO_THREADS, 0, st, p);
+  return launch_dependent(ttt_layer_prologue_kernel<T, false, FD>, grid, PRO_THREADS, 0, st, p);
 }
 
 cudaError_t launch_layer_prologue(int dtype, int head_dim, const LayerProParams& p0, cudaStream_t st) {
   LayerProParams p = p0;
   const int grid = prologue_grid(p.B, p.H, p.T, head_dim, PRO_TCHUNK, 8, &p.tchunk);
-  if (head_dim == 32) {
-    if (dtype == 1) launch_pro_t<__nv_bfloat16, 32>(p, grid, st);
-    else launch_pro_t<float, 32>(p, grid, st);
-  } else {
-    if (dtype == 1) launch_pro_t<__nv_bfloat16, 64>(p, grid, st);
-    else launch_pro_t<float, 64>(p, grid, st);
-  }
-  return cudaGetLastError();
+  if (head_dim == 32) return dtype == 1 ? launch_pro_t<__nv_bfloat16, 32>(p, grid, st) : launch_pro_t<float, 32>(p, grid, st);
+  return dtype == 1 ? launch_pro_t<__nv_bfloat16, 64>(p, grid, st) : launch_pro_t<float, 64>(p, grid, st);
 }
 
 template <typename T, int MAXCH, int FD, bool GATE>
@@ -461,8 +458,7 @@ static cudaError_t launch_epi_g(LayerEpiParams p, cudaStream_t st) {
   const long ntiles = (long)p.B * ((p.T + p.tile_rows - 1) / p.tile_rows);
   const long cap = (long)sm_count() * (per_sm < 1 ? 1 : per_sm);
   const int grid = (int)(ntiles < cap ? ntiles : cap);
-  kfn<<<grid < 1 ? 1 : grid, threads, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(kfn, grid < 1 ? 1 : grid, threads, smem, st, p);
 }
 template <typename T, int MAXCH, int FD>
 static cudaError_t launch_epi_t(const LayerEpiParams& p, cudaStream_t st) {

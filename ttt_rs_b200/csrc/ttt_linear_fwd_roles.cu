@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(ROLE_THREADS, 1)
       asm volatile("st.shared.b32 [%0], %1;" ::"r"(base + SM::OFF_LR + e), "r"(0u) : "memory");
   }
   __syncthreads();
+  pdl_join();
 
   const float te_row[2] = {ld_as_float<T>(p.token_eta, g), MB == CS ? ld_as_float<T>(p.token_eta, g + 8) : 0.f};
   const float te15 = ld_as_float<T>(p.token_eta, MB - 1);
@@ -528,8 +529,8 @@ static cudaError_t launch_t(const CUtensorMap* m, const LinFwdParams& p, int nst
     return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, *n);
   });
   if (e != cudaSuccess) return e;
-  kfn<<<nstreams, ROLE_THREADS, SM::DYN_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], p);
-  return cudaGetLastError();
+  // (one block to an SM at most, so it does not matter which SMs the kernel before leaves first)
+  return launch_dependent(kfn, nstreams, ROLE_THREADS, SM::DYN_BYTES, st, m[0], m[1], m[2], m[3], m[4], p);
 }
 template <typename T, int SEG>
 static cudaError_t launch_mb(int mb, const CUtensorMap* m, const LinFwdParams& p, int nstreams, cudaStream_t st) {
