@@ -23,7 +23,8 @@ def test_every_kernel_that_may_begin_early_waits():
                 launched |= set(re.findall(r"kfn = [^;]*?\b(ttt_\w+_kernel)\b", text)) - {"ttt_layer_epilogue_bwd_kernel"}
     assert launched <= set(waiting), launched - set(waiting)
     joined = {n for n, k in waiting.items() if "pdl_join()" in k}
-    assert joined == {"ttt_gemm_bf16_tn_kernel", "ttt_layer_prologue_kernel", "ttt_layer_epilogue_kernel", "ttt_linear_fwd_roles_kernel"}
+    assert joined == {"ttt_gemm_bf16_tn_kernel", "ttt_layer_prologue_kernel", "ttt_layer_epilogue_kernel", "ttt_linear_fwd_roles_kernel",
+                      "ttt_linear_bwd_reduce_kernel", "ttt_mlp_bwd_reduce_kernel"}
     for n in joined:  # what the kernel before may still write is never read as read-only data
         assert not re.search(r"\b(?:ldg4|__ldg)\(|ld\.global\.nc", waiting[n]), n
 

@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
   if (warp == 0) tmem_alloc(smem_u32(&s_tmem), 64);
   tmem_fence_before_sync();
   __syncthreads();
+  if (p.sched == nullptr) pdl_go();  // every stream alone on an SM: the reduction may come (it waits); beside more, its blocks cost 0.1 %
   tmem_fence_after_sync();
   const uint32_t tm_w = s_tmem + ((32u * (uint32_t)warp) << 16), tm_dw = tm_w + 32u;
 
@@ -796,6 +797,7 @@ __global__ void __launch_bounds__(NTHREADS, TTT_BWD_MINB_BF16)
 template <int F>
 __global__ void __launch_bounds__(256) ttt_linear_bwd_reduce_kernel(const ReduceParams p) {
   __shared__ float part[8][32];
+  pdl_join();
   // H heads of F features as the caller counts them; the partials of the LayerNorm gradients are in the kernel's
   // 64-wide tiles, which hold NP = 64 / F heads side by side
   constexpr int NP = HD / F;
@@ -915,8 +917,8 @@ cudaError_t launch_linear_bwd_reduce(const ReduceParams& p, cudaStream_t st) {
   const int total = p.T + 2 * p.H * p.F + (p.packed != nullptr ? p.H * (p.F * p.F + p.F) : 0);
   int blocks = (total + 31) / 32;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  if (p.F == 32) ttt_linear_bwd_reduce_kernel<32><<<blocks, 256, 0, st>>>(p);
-  else ttt_linear_bwd_reduce_kernel<64><<<blocks, 256, 0, st>>>(p);
+  const cudaError_t e = launch_dependent(p.F == 32 ? ttt_linear_bwd_reduce_kernel<32> : ttt_linear_bwd_reduce_kernel<64>, blocks, 256, 0, st, p);
+  if (e != cudaSuccess) return e;
   if (p.packed != nullptr) ttt_linear_bwd_fold_kernel<<<1, p.mb * 32, 0, st>>>(p);
   return cudaGetLastError();
 }

@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(BR_THREADS, 1)
     fence_proxy_async_smem();
   }
   __syncthreads();
+  pdl_go();  // (the reduction waits)
 
   const float te_row[2] = {ld_as_float<T>(p.token_eta, g), MB == CS ? ld_as_float<T>(p.token_eta, g + 8) : 0.f};
   const float te15 = ld_as_float<T>(p.token_eta, MB - 1);

@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
   tmem_fence_before_sync();
   __syncthreads();
   tmem_fence_after_sync();
+  pdl_go();  // (the reduction waits)
   const auto tmem = [&]() { return lds_u(base0 + SM::BAR + 36); };  // (read where it is used, like te15: a register less across the stage loop)
   const auto te15 = [&]() { return lds_f(base0 + SM::TE + 4 * (CS - 1)); };
   // the masters of W1, W2 are carried divided by -te15, so that a stage's update accumulates directly (te15 = 0: they never
@@ -989,6 +990,7 @@ __global__ void __launch_bounds__(MB_THREADS, 1)
 __global__ void __launch_bounds__(256) ttt_mlp_bwd_reduce_kernel(const float* part_te, const float* part_ln, int B, int H,
                                                                  int T, int bf16, void* dte, void* dg, void* db) {
   __shared__ float part[8][32];
+  pdl_join();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane, n_ln = 2 * H * HD;
   float acc = 0.f;
@@ -1039,9 +1041,8 @@ cudaError_t launch_mlp_bwd(const CUtensorMap* m, const MlpBwdParams& p0, int B, 
   e = cudaLaunchCooperativeKernel((const void*)ttt_mlp_bwd_kernel, dim3(grid), dim3(MB_THREADS), args, MlpBwdSmem::TOTAL, st);
   if (e != cudaSuccess) return e;
   const int n = p.T + 2 * p.H * HD;
-  ttt_mlp_bwd_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(p.part_te, p.part_ln, B, p.H, p.T, p.reduced_bf16,
-                                                         p.d_token_eta, p.d_ln_g, p.d_ln_b);
-  return cudaGetLastError();
+  return launch_dependent(ttt_mlp_bwd_reduce_kernel, (n + 31) / 32, 256, 0, st, (const float*)p.part_te, (const float*)p.part_ln, B, p.H, p.T, (int)p.reduced_bf16,
+                          p.d_token_eta, p.d_ln_g, p.d_ln_b);
 }
 
 }  // namespace ttt
