@@ -289,13 +289,14 @@ __device__ __forceinline__ void report_timeout(uint32_t* status, uint32_t where,
 }
 
 // ---- TTT-MLP: tanh-approximated GELU -------------------------------------------------------------------------------
-// gelu(z), (D > 0) gelu'(z) times sc and (D > 1) gelu''(z) of a pair, from q = 1 / (1 + e^{2u}), tanh(u) = 1 - 2q (relative error
-// ~1e-6; the hardware tanh.approx is only good to ~5e-4, which shows after a few dozen chained stages):
-//     u = c0 z (1 + c1 z^2), m = -2 u':   gelu = z (1 - q),   gelu' = (1 - q) (1 - z q m),
-//     gelu'' = q (1 - q) (-4 m - 4 c0 - z m^2 (1 - 2q))      (z u'' = -m - 2 c0)
-// The pair's quotients share one reciprocal, 1/a = b / (ab): three calls of the special-function unit instead of four.
-// Exponents stop at 2^60, where tanh is 1, so that the product stays finite; the 2^-60 that q keeps there is taken off, or its
-// product with z^3 would show in gelu' of a z in the millions.
+// gelu(z), (D > 0) gelu'(z) times sc and (D > 1) gelu''(z) of a pair, through p = (1 + tanh u) / 2 = 1 / (1 + e^{-2u}) (the hardware
+// tanh.approx is only good to ~5e-4, which shows after a few dozen chained stages):
+//     u = c0 z (1 + c1 z^2), m = 2 u', q = 1 - p:   gelu = z p,   gelu' = p + z p q m,
+//     gelu'' = p q (4 m - 4 c0 - z (p - q) m^2)      (z u'' = m - 2 c0)
+// With e = e^{-2|u|} the smaller of p and q is s = e / (1 + e), to its relative accuracy, and the larger l = 1 - s: far out s is
+// exactly 0 and l exactly 1.  (The residue of 2^-24 that 1 - q leaves for a small p is multiplied by z^3 in gelu' and by z^5 in gelu''.)
+// Each element has a reciprocal of its own: a value depends on no other token or feature.  Errors of gelu, gelu', gelu'' against
+// float64, root mean square over z ~ N(0, 2^2): 4.2e-8, 3.0e-8, 4.2e-8 (from tanh = 1 - 2 / (1 + e^{2u}): 6.4e-8, 1.9e-7, 8.3e-7).
 __device__ __forceinline__ float ex2_approx(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -311,18 +312,18 @@ __device__ __forceinline__ F2 gelu_pair(F2 z, F2& d1, F2& d2, float sc = 1.f) {
   constexpr float C0 = 0.7978845608028654f, C1 = 0.044715f, L2E2 = 2.f * 1.4426950408889634f;
   const F2 z2 = f2mul(z, z);
   const F2 a = f2mul(z, f2fma(z2, f2(L2E2 * C0 * C1), f2(L2E2 * C0)));
-  const F2 d = f2add(f2(ex2_approx(fminf(a.x, 60.f)), ex2_approx(fminf(a.y, 60.f))), f2(1.f));
-  const F2 nq = f2fma(f2(rcp_approx(-(d.x * d.y))), f2(d.y, d.x), f2(0x1p-60f)), y = f2mul(z, nq);  // -q, -z q
+  const F2 e = f2(ex2_approx(-fabsf(a.x)), ex2_approx(-fabsf(a.y))), d = f2add(e, f2(1.f));
+  const F2 s = f2mul(e, f2(rcp_approx(d.x), rcp_approx(d.y))), l = f2sub(f2(1.f), s);
+  const F2 p = f2(z.x > 0.f ? l.x : s.x, z.y > 0.f ? l.y : s.y);
   if constexpr (D > 0) {
-    const F2 m = f2fma(z2, f2(-6.f * C0 * C1), f2(-2.f * C0));
-    d1 = f2mul(f2fma(nq, f2(sc), f2(sc)), f2fma(y, m, f2(1.f)));
+    const F2 t = f2mul(l, s), m = f2fma(z2, f2(6.f * C0 * C1), f2(2.f * C0));
+    d1 = f2mul(f2fma(f2mul(z, t), m, p), f2(sc));
     if constexpr (D > 1) {
-      const F2 p = f2add(nq, f2(1.f));
-      const F2 b = f2fma(f2mul(f2mul(z, m), m), f2add(p, nq), f2fma(m, f2(4.f), f2(4.f * C0)));
-      d2 = f2mul(f2mul(nq, p), b);
+      const F2 y = f2mul(f2(fabsf(z.x), fabsf(z.y)), f2sub(l, s));
+      d2 = f2fma(f2mul(t, m), f2fma(f2neg(y), m, f2(4.f)), f2mul(t, f2(-4.f * C0)));
     }
   }
-  return f2add(z, y);
+  return f2mul(z, p);
 }
 
 // ---- rank-16 updates of a state in tensor memory by tcgen05 (TTT-MLP) ----------------------------------------------
