@@ -66,10 +66,10 @@ struct MlpSmem {
   static constexpr uint32_t OFF_M2 = OFF_B2 + 2 * B2;                 // bf16 [16][24]: -M2'
   static constexpr uint32_t OFF_A2 = OFF_M2 + 16 * 24 * 2;            // float [8 warps][3][8][8]: partials of A2 (its lower blocks)
   static constexpr uint32_t OFF_LR = OFF_A2 + 8 * 768;                // MLP_NST x 32 bytes
-  // mbarriers: full [MLP_NST], published [2], done [2], state, partials read; products: Zb1 [2], Z1, G1, updates of W1, W2; M1';
+  // mbarriers: full [MLP_NST], published [2], done [2], partials read; products: Zb1 [2], Z1, G1, updates of W1, W2; M1';
   // then item, failure flag, tensor-memory base
   static constexpr uint32_t OFF_BAR = OFF_LR + MLP_NST * 32;
-  static constexpr uint32_t OFF_WORDS = OFF_BAR + (MLP_NST + 13) * 8;
+  static constexpr uint32_t OFF_WORDS = OFF_BAR + (MLP_NST + 12) * 8;
   static constexpr uint32_t TOTAL = OFF_WORDS + 16;
 };
 static_assert(MlpSmem::TOTAL <= 227 * 1024, "shared-memory tiles exceed one SM");
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     return;
   }
   const uint32_t bar_full = base + SM::OFF_BAR, bar_pub = bar_full + 8 * MLP_NST, bar_done = bar_pub + 16,
-                 bar_state = bar_done + 16, bar_parts = bar_state + 8, bar_zq = bar_parts + 8, bar_z = bar_zq + 16, bar_h = bar_z + 8,
+                 bar_parts = bar_done + 16, bar_zq = bar_parts + 8, bar_z = bar_zq + 16, bar_h = bar_z + 8,
                  bar_w1 = bar_h + 8, bar_w2 = bar_w1 + 8, bar_m1 = bar_w2 + 8;
   const uint32_t w_item = base + SM::OFF_WORDS, w_fail = w_item + 4, w_tmem = w_item + 8;
 
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     prefetch_tmap(&tm_k);
     prefetch_tmap(&tm_v);
     for (int i = 0; i < MLP_NST; ++i) mbar_init(bar_full + 8 * i, 1);
-    for (int i = 0; i < 6; ++i) mbar_init(bar_pub + 8 * i, 8);
+    for (int i = 0; i < 5; ++i) mbar_init(bar_pub + 8 * i, 8);
     for (int i = 0; i < 6; ++i) mbar_init(bar_zq + 8 * i, 2);  // (a commit for each half of the hidden features)
     mbar_init(bar_m1, 1);
     fence_mbar_init();
@@ -400,7 +400,6 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         }
         tmem_wait_st();
         tmem_fence_before_sync();
-        mbar_arrive_warp(bar_state);
         half_sync();
         issue_first(n, s_lo);
       }
@@ -503,7 +502,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
         }
         fence_proxy_async_smem();
         tmem_fence_before_sync();
-        mbar_arrive_warp(bar_pub + 8 * par);  // X2, G2p, G1p of the stage
+        mbar_arrive_warp(bar_pub + 8 * par);  // X2, G2p, G1p of the stage, and the copies and biases that it began with
         half_sync();  // G1p of the half's hidden features
         issue(0, bar_w1, [&]() {
           if (w_moves) umma_update(tmem + 64 * half, tg1 + half * 2 * TL, tk, UPD_IDESC);
@@ -543,7 +542,6 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
           tmem_fence_before_sync();
           half_sync();
           issue_first(n + 1, s + 1);
-          mbar_arrive_warp(bar_state);
         }
         // (stage ends)
       }
@@ -654,7 +652,6 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
                        tg1 = base + SM::OFF_G1 + par * SM::ET, tg2 = base + SM::OFF_G2 + par * TL;
         uint8_t* const rec = SAVE ? rec0 + (size_t)s * MLP_REC_BYTES : nullptr;
         wait_for(bar_full + 8 * slot, (n / MLP_NST) & 1, 26, s);
-        wait_for(bar_state, n & 1, 27, s);
         // ---- O1. Zb1 = Q W1 + b1 - M1' G1p;  Xb2 = gelu(Zb1)
         wait_for(bar_pub + 8 * par, (n >> 1) & 1, 28, s);
         if (SAVE && warp == 1) {  // the stage's operands to its record
