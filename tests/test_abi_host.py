@@ -110,6 +110,30 @@ def test_null_and_misaligned_pointers_are_rejected(lib):
     assert lib.ttt_linear_forward(None, *([fake] * 14), None, None) == _lib.TTT_ERR_NULL
 
 
+def test_mlp_backward_refuses_what_its_copies_cannot_take(lib):
+    """Rates off a 16-byte boundary (the walk copies sixteen at a time; a workspace that the forward filled needs no walk), token
+    gradients off a pair's boundary."""
+    d = _dims()
+    p = C.c_void_p(0x1000)
+
+    def backward(from_forward=0, workspace=p, **at):
+        names = ("xq", "xk", "xv", "w1", "b1", "w2", "b2", "token_eta", "ttt_lr_eta", "ln_weight", "ln_bias", "grad_output", "grad_xq",
+                 "grad_xk", "grad_xv", "grad_w1", "grad_b1", "grad_w2", "grad_b2", "grad_ttt_lr_eta", "grad_token_eta", "grad_ln_weight",
+                 "grad_ln_bias")
+        return lib.ttt_mlp_backward(C.byref(d), *[C.c_void_p(at.get(n, 0x1000)) for n in names], workspace, 0, from_forward, None, None)
+
+    assert backward() == _lib.TTT_ERR_WORKSPACE  # (all that follows is refused before this)
+    for off in (2, 8):
+        assert backward(ttt_lr_eta=0x1000 + off) == _lib.TTT_ERR_ALIGN
+        assert "ttt_lr_eta" in _lib.last_error()
+    assert backward(from_forward=1, ttt_lr_eta=0x1002) == _lib.TTT_ERR_WORKSPACE
+    for name in ("grad_xq", "grad_xk", "grad_xv"):
+        assert backward(**{name: 0x1002}) == _lib.TTT_ERR_ALIGN
+        assert name in _lib.last_error()
+        assert backward(**{name: 0x1004}) == _lib.TTT_ERR_WORKSPACE
+    assert backward(w2=0x1002) == _lib.TTT_ERR_WORKSPACE  # (read at any address)
+
+
 def test_config_epsilon_scaling_matches_reference():
     # (1e-6f32 / 1e-9f32) as u32 == 1000 (rust/fused/src/lib.rs:298-311)
     cfg = ttt_rs_b200.FusedTttConfig.new(16, 64, 1e-6, 64)

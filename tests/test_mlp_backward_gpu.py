@@ -226,3 +226,28 @@ def test_step_scales_and_many_stages(B, H, NS, te_scale, bound, from_forward):
         err = ((a - b).norm() / b.norm()).item()
         print(f"{k}, first stages: {err:.2e}")
         assert err < 1e-2, f"{k}, first stages: {err}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", (1, 4))
+def test_walk_takes_a_second_layer_at_any_address(offset):
+    """w2 sliced out of a flat buffer, 2 or 8 bytes past a 16-byte boundary: the same gradients, bit for bit."""
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    t = _case(1, 3, 48, 91)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 128, 1)
+    d = {k: v.to(dev) for k, v in t.items()}
+    flat = torch.zeros(d["w2"].numel() + 8, dtype=torch.bfloat16, device=dev)
+    sliced = flat[offset:offset + d["w2"].numel()].view_as(d["w2"])
+    sliced.copy_(d["w2"])
+    assert sliced.data_ptr() % 16 == 2 * offset
+    got = []
+    for w2 in (d["w2"], sliced):
+        g = tb.fused_ttt_mlp_backward(d["xq"], d["xk"], d["xv"], tb.TTTMLPState(d["w1"], d["b1"], w2, d["b2"]), d["token_eta"],
+                                      d["ttt_lr_eta"], d["ln_weight"], d["ln_bias"], d["grad_output"], cfg)
+        torch.cuda.synchronize()
+        tb.check_mlp_status(g)
+        got.append(g)
+    for k in got[0]:
+        if k.startswith("grad_"):
+            assert torch.equal(got[0][k], got[1][k]), k

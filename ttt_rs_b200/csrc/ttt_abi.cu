@@ -1180,6 +1180,12 @@ extern "C" int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, cons
                            {"grad_ln_bias", grad_ln_bias}};
   for (const NamedPtr& np : ptrs)
     if (np.p == nullptr) return fail(TTT_ERR_NULL, "%s is null", np.name);
+  // Addresses that the tensor maps do not check and the kernels move in more than one element: the walk's copies of the rates, pairs
+  // of a token's gradients.  (A w2 that is no multiple of 16 bytes the walk reads element by element.)
+  if (workspace_from_forward == 0 && (reinterpret_cast<uintptr_t>(ttt_lr_eta) & 15u) != 0)
+    return fail(TTT_ERR_ALIGN, "ttt_lr_eta is not 16-byte aligned");
+  for (const NamedPtr& np : {NamedPtr{"grad_xq", grad_xq}, NamedPtr{"grad_xk", grad_xk}, NamedPtr{"grad_xv", grad_xv}})
+    if ((reinterpret_cast<uintptr_t>(np.p) & 3u) != 0) return fail(TTT_ERR_ALIGN, "%s is not 4-byte aligned", np.name);
   const MlpWsLayout l = mlp_ws_layout(d);
   if (workspace == nullptr || workspace_bytes < l.total_bytes)
     return fail(TTT_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", l.total_bytes, workspace_bytes);

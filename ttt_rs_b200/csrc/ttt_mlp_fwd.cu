@@ -374,6 +374,10 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 v[i >> 2][i & 3] = ld_as_float<T>(p.w1, (size_t)stream * HD * MLP_E + (size_t)(32 * cc + i) * MLP_E + e_own) * winv;
+            } else if (SAVE && (reinterpret_cast<uintptr_t>(p.w2) & 15) != 0) {  // (the backward's own walk takes any address)
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                v[i >> 2][i & 3] = ld_as_float<T>(p.w2, (size_t)stream * HD * MLP_E + (size_t)e_own * HD + 32 * cc + i) * winv;
             } else {
               const uint4* const src = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.w2) + ((size_t)stream * HD * MLP_E + (size_t)e_own * HD + 32 * cc) * 2);
 #pragma unroll
