@@ -152,3 +152,16 @@ def test_a_warp_held_up_anywhere_finds_its_phase(held):
     for at in range(len(warps[held])):
         wrong = _simulate(warps, held, at)
         assert wrong is None, f"held before its operation {at}, {warps[held][at]}: {wrong}"
+
+
+def test_products_end_before_tensor_memory_is_freed():
+    """When a wait ran out nobody waits for the products behind it: on the way out every warp that issues products commits them once
+    more, and the warp that frees tensor memory waits for all those commits."""
+    text = re.sub(r"//.*", "", SRC.read_text())
+    issuing = {int(i) for i in re.findall(r"\bissue\((\d),", text)}
+    out = text[text.index("if (lds_word(w_fail) != 0u) break;"):text.index("tmem_dealloc(")]
+    commit = re.search(r"if \(!output_group && \(warp & 3\) < (\d)\) \{\s*if \(elect_one\(\)\) umma_commit_to\((\w+)\);", out)
+    assert commit and issuing == set(range(int(commit[1]))), issuing
+    wait = re.search(rf"if \(threadIdx\.x < 32\) mbar_wait_bounded\({commit[2]}, 0\);", out)
+    assert wait and commit.end() < wait.start()
+    assert re.search(rf"mbar_init\({commit[2]}, {2 * len(issuing)}\);", text)  # (both halves of the hidden features)

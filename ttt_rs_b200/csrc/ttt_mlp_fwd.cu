@@ -66,10 +66,10 @@ struct MlpSmem {
   static constexpr uint32_t OFF_M2 = OFF_B2 + 2 * B2;                 // bf16 [16][24]: -M2'
   static constexpr uint32_t OFF_A2 = OFF_M2 + 16 * 24 * 2;            // float [8 warps][3][8][8]: partials of A2 (its lower blocks)
   static constexpr uint32_t OFF_LR = OFF_A2 + 8 * 768;                // MLP_NST x 32 bytes
-  // mbarriers: full [MLP_NST], published [2], done [2], partials read; products: Zb1 [2], Z1, G1, updates of W1, W2; M1';
+  // mbarriers: full [MLP_NST], published [2], done [2], partials read; products: Zb1 [2], Z1, G1, updates of W1, W2; M1'; end;
   // then item, failure flag, tensor-memory base
   static constexpr uint32_t OFF_BAR = OFF_LR + MLP_NST * 32;
-  static constexpr uint32_t OFF_WORDS = OFF_BAR + (MLP_NST + 12) * 8;
+  static constexpr uint32_t OFF_WORDS = OFF_BAR + (MLP_NST + 13) * 8;
   static constexpr uint32_t TOTAL = OFF_WORDS + 16;
 };
 static_assert(MlpSmem::TOTAL <= 227 * 1024, "shared-memory tiles exceed one SM");
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
   }
   const uint32_t bar_full = base + SM::OFF_BAR, bar_pub = bar_full + 8 * MLP_NST, bar_done = bar_pub + 16,
                  bar_parts = bar_done + 16, bar_zq = bar_parts + 8, bar_z = bar_zq + 16, bar_h = bar_z + 8,
-                 bar_w1 = bar_h + 8, bar_w2 = bar_w1 + 8, bar_m1 = bar_w2 + 8;
+                 bar_w1 = bar_h + 8, bar_w2 = bar_w1 + 8, bar_m1 = bar_w2 + 8, bar_end = bar_m1 + 8;
   const uint32_t w_item = base + SM::OFF_WORDS, w_fail = w_item + 4, w_tmem = w_item + 8;
 
   const bool output_group = __shfl_sync(0xffffffffu, threadIdx.x >> 8, 0) != 0;
@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     for (int i = 0; i < 5; ++i) mbar_init(bar_pub + 8 * i, 8);
     for (int i = 0; i < 6; ++i) mbar_init(bar_zq + 8 * i, 2);  // (a commit for each half of the hidden features)
     mbar_init(bar_m1, 1);
+    mbar_init(bar_end, 6);  // (the warps that issue products: three of each half)
     fence_mbar_init();
     sts_word(w_fail, 0u);
   }
@@ -764,6 +765,13 @@ __global__ void __launch_bounds__(MLP_THREADS, 1)
     __syncthreads();  // the item is left by both groups
     if (lds_word(w_fail) != 0u) break;
   }  // work items
+  if (lds_word(w_fail) != 0u) {  // products that nobody waited for end before tensor memory and the block's memory are given back
+    if (!output_group && (warp & 3) < 3) {
+      if (elect_one()) umma_commit_to(bar_end);
+      __syncwarp();
+    }
+    if (threadIdx.x < 32) mbar_wait_bounded(bar_end, 0);
+  }
   tmem_fence_before_sync();
   __syncthreads();
   if (threadIdx.x < 32) tmem_dealloc(lds_word(w_tmem), 512);
