@@ -81,3 +81,35 @@ def test_mlp_forward_at_the_edges_of_its_rings(B, H, NS, eta):
     assert torch.equal(part, out[:2])
     if eta == "zero":
         assert all(torch.equal(getattr(new, k), d[k]) for k in ("w1", "b1", "w2", "b2"))
+
+
+def test_more_streams_than_sms_without_memory_for_their_chunks():
+    """The allocator has room for the results of 192 streams and not for the 26 MB that their states would be parked in: the call
+    runs in whole waves, to the same bits."""
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    t = O.make_inputs(24, 8, 24 * 16, 64, 16, seed=41, dtype=torch.bfloat16, inner="mlp", with_grad_output=False)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 256, 1)
+    d = {k: t[k].to(dev) for k in NAMES}
+    args = (d["xq"], d["xk"], d["xv"], tb.TTTMLPState(d["w1"], d["b1"], d["w2"], d["b2"]), d["token_eta"], d["ttt_lr_eta"],
+            d["ln_weight"], d["ln_bias"], cfg)
+    torch.cuda.empty_cache()
+    before = torch.cuda.memory_reserved()
+    out, new = tb.fused_ttt_mlp_forward(*args)
+    torch.cuda.synchronize()
+    want = [x.cpu() for x in (out, new.w1, new.b1, new.w2, new.b2)]
+    took = torch.cuda.memory_reserved() - before
+    del out, new
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    failed = torch.cuda.memory_stats()["num_ooms"]
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + took - (16 << 20)) / total)
+        out, new = tb.fused_ttt_mlp_forward(*args)
+        torch.cuda.synchronize()
+        assert torch.cuda.memory_stats()["num_ooms"] == failed + 1
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    tb.TttTileMultiKernel.check_status()
+    for a, b in zip(want, (out, new.w1, new.b1, new.w2, new.b2)):
+        assert torch.equal(a, b.cpu())

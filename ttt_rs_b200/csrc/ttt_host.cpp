@@ -187,9 +187,15 @@ int mlp_forward(const Dims& m, const MlpIn& in, const Tensor& ws, Tensor (&o)[5]
   o[0] = at::empty({m.B, m.H, m.T, m.F}, m.opt());
   for (int i = 0; i < 4; ++i) o[1 + i] = at::empty(in.t[3 + i].sizes(), m.opt());
   if (!ws.defined()) {
-    const size_t bytes = ttt_internal_mlp_infer_scratch_bytes(&m.d);
+    size_t bytes = ttt_internal_mlp_infer_scratch_bytes(&m.d);
     Tensor scratch;
-    if (bytes != 0) scratch = at::empty({(int64_t)bytes}, m.opt(at::kByte));
+    if (bytes != 0) {
+      try {
+        scratch = at::empty({(int64_t)bytes}, m.opt(at::kByte));
+      } catch (const c10::OutOfMemoryError&) {  // whole waves need none
+        bytes = 0;
+      }
+    }
     return ttt_internal_mlp_infer(&m.d, in.p(0), in.p(1), in.p(2), in.p(3), in.p(4), in.p(5), in.p(6), in.p(7), in.p(8),
                                   in.p(9), in.p(10), o[0].data_ptr(), o[1].data_ptr(), o[2].data_ptr(), o[3].data_ptr(),
                                   o[4].data_ptr(), bytes != 0 ? scratch.data_ptr() : nullptr, bytes, m.status.data_ptr(),
