@@ -646,9 +646,9 @@ static int mlp_forward(const ttt_dims* d, const void* xq, const void* xk, const 
   rc = check_ptrs(ptrs, sizeof(ptrs) / sizeof(ptrs[0]));
   if (rc != TTT_OK) return rc;
   const int64_t rows = (int64_t)d->batch * d->heads * d->seq_len;
-  CUtensorMap maps[4];
-  const void* bases[4] = {xq, xk, xv, output};
-  for (int i = 0; i < 4; ++i) {
+  CUtensorMap maps[3];
+  const void* bases[3] = {xq, xk, xv};
+  for (int i = 0; i < 3; ++i) {
     rc = make_tile_map(&maps[i], bases[i], rows, d->dtype);
     if (rc != TTT_OK) return rc;
   }
@@ -1210,7 +1210,7 @@ extern "C" int ttt_internal_mlp_backward(const ttt_dims* d, const void* xq, cons
     f.sched = reinterpret_cast<int*>(ws + l.off_sched);
     f.handoff_polls = g_handoff_polls.load();
     f.H = d->heads; f.T = d->seq_len; f.NS = d->seq_len / d->mini_batch; f.eps = d->epsilon;
-    const cudaError_t e = ttt::launch_mlp_fwd(maps, f, d->batch * d->heads, st);  // (the output's map is not used)
+    const cudaError_t e = ttt::launch_mlp_fwd(maps, f, d->batch * d->heads, st);
     if (e != cudaSuccess) return fail(TTT_ERR_CUDA, "MLP forward walk launch failed: %s", cudaGetErrorString(e));
   }
   ttt::MlpBwdParams p;

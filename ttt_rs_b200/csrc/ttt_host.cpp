@@ -203,8 +203,7 @@ int mlp_forward(const Dims& m, const MlpIn& in, const Tensor& ws, Tensor (&o)[5]
   }
   return ttt_mlp_forward(&m.d, in.p(0), in.p(1), in.p(2), in.p(3), in.p(4), in.p(5), in.p(6), in.p(7), in.p(8), in.p(9),
                          in.p(10), o[0].data_ptr(), o[1].data_ptr(), o[2].data_ptr(), o[3].data_ptr(), o[4].data_ptr(),
-                         ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
-                         m.status.data_ptr(), m.stream());
+                         ws.data_ptr(), (size_t)ws.numel(), m.status.data_ptr(), m.stream());
 }
 // gradients in the order of the inputs; `from_forward`: ws was filled by the forward on the same inputs
 int mlp_backward(const Dims& m, const MlpIn& in, const Tensor& go, const Tensor& ws, bool from_forward, Tensor (&g)[11]) {

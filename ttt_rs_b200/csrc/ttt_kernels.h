@@ -387,7 +387,7 @@ struct GemmParams {
 };
 cudaError_t launch_gemm_bf16_tn(const CUtensorMap* maps, const GemmParams& p, bool fused, bool pair, cudaStream_t st);
 
-// bf16 only.  maps: q, k, v, out.
+// bf16 only.  maps: q, k, v.
 cudaError_t launch_mlp_fwd(const CUtensorMap* maps, const MlpFwdParams& p, int nstreams, cudaStream_t st);
 // scratch of an inference call (current device), 0: none is used
 size_t mlp_fwd_scratch_floats(int NS, int nstreams);
