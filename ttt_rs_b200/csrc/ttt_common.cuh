@@ -429,7 +429,8 @@ struct TokenEtaElement {
 // A kernel launched with launch_dependent may begin while the kernel before it on the stream drains: its launch and
 // prologue (and loads of data that neither the kernel before nor an unfinished one writes) are off the chain.
 // pdl_wait: everything before on the stream is complete and visible.  pdl_go: the next kernel may begin; called after
-// pdl_wait, so that at most one kernel is unfinished when a later one starts.
+// pdl_wait, or by a kernel that is only ever launched behind everything before it (the scans of the backwards), so that at most
+// one kernel is unfinished when a later one starts.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Both, for a kernel that reads nothing before: only its launch and what it sets up for itself overlap the kernel before it.  (The
