@@ -113,3 +113,27 @@ def test_more_streams_than_sms_without_memory_for_their_chunks():
     tb.TttTileMultiKernel.check_status()
     for a, b in zip(want, (out, new.w1, new.b1, new.w2, new.b2)):
         assert torch.equal(a, b.cpu())
+
+
+@pytest.mark.parametrize("NS", (25, 35))
+def test_chunks_of_odd_length_with_a_short_one_at_the_end(NS):
+    """168 streams of 25 or 35 stages on 148 SMs run in chunks of 9, the last of 7 or 8: chunks begin at either parity of the rings.
+    The same bits as eight and sixteen streams alone, which run in one piece."""
+    import ttt_rs_b200 as tb
+    dev = torch.device("cuda:0")
+    t = O.make_inputs(21, 8, NS * 16, 64, 16, seed=60 + NS, dtype=torch.bfloat16, inner="mlp", with_grad_output=False)
+    cfg = tb.FusedTttConfig.new(16, 64, 1e-6, 256, 1)
+    d = {k: t[k].to(dev) for k in NAMES}
+
+    def run(lo, hi):
+        a = {k: v[lo:hi].contiguous() if v.dim() > 1 and v.size(0) == 21 else v for k, v in d.items()}
+        st = tb.TTTMLPState(a["w1"], a["b1"], a["w2"], a["b2"])
+        out, new = tb.fused_ttt_mlp_forward(a["xq"], a["xk"], a["xv"], st, a["token_eta"], a["ttt_lr_eta"], a["ln_weight"], a["ln_bias"], cfg)
+        return out, new.w1, new.b1, new.w2, new.b2
+
+    whole = run(0, 21)
+    for lo, hi in ((0, 1), (19, 21)):
+        for a, b in zip(whole, run(lo, hi)):
+            assert torch.equal(a[lo:hi], b)
+    torch.cuda.synchronize()
+    tb.TttTileMultiKernel.check_status()
