@@ -9,8 +9,9 @@
 //     out = Q + LN(Zb2);   W1 -= te15 K^T G1p;  b1 -= te15 colsum(G1p);  W2 -= te15 X2^T G2p;  b2 -= te15 colsum(G2p)
 //
 // What bounds it: the chain W -> Z1 -> X2 -> Z2 -> G2 -> G1 -> W from one stage to the next on one SM (the state and its
-// copies fill it): 6.1 k cycles a stage, 5.0 k with nothing beside it, of them 1.2 k round trips of three dependent tcgen05
-// products and their commits, the rest instructions of two warps a scheduler at seven cycles each.  So:
+// copies fill it): 6.3 k cycles a stage, 5.0 k with nothing beside it, of them 1.2 k round trips of three dependent tcgen05
+// products and their commits, the rest instructions of two warps a scheduler at seven cycles each (the 5.0 k and what follows: of a
+// GELU that was 0.15 k cycles a stage shorter).  So:
 //  * Only that chain is the first group's work (warps 0..7).  The second group (warps 8..15) forms the stage's output from
 //    what the chain publishes in shared and tensor memory, about half a stage behind.
 //  * Warp w of either group owns hidden features e in [32w, 32w+32) of every 16 x 256 tile, in mma accumulator layout, from Z1
@@ -29,6 +30,8 @@
 // 48 streams of 31 stages / forward + backward of 192 streams of 128 stages: one group of eight warps with the masters in
 // registers 150 / 2 528 us; two groups, products with the state by mma.sync 115 / 2 284; by tcgen05 106 / 2 243.  Not better: two groups
 // of sixteen warps 121 / 2 355; K_next W1_next taken as K_next W1 plus a product with G1p, which takes W1's refresh off the chain, 111 / 2 284.
+// Now 108.6 / 2 207 (with the backward's last interval on twelve warps, and a reciprocal for every element of GELU: one that two shared
+// was 106.1 / 2 188 and lost the negative tail of the derivatives).
 //
 // Scheduling.  One CTA fills an SM, so a launch of one CTA per stream runs in whole
 // waves: 192 streams on 148 SMs cost two stream-times.  When there is memory to park a stream's state in -- the backward's
@@ -36,7 +39,7 @@
 // streams than SMs -- blocks take work items (stream, chunk of stages: mlp_chunk_stages) instead, first
 // chunks of all streams first, and a chunk hands the state to the next one through the stream's block of that memory
 // behind a per-stream counter -- the scheme of the TTT-Linear backward.  Inference: 192 streams of 128 stages
-// 818 -> 581 us, 384 of 64 stages 633 -> 610, 300 of 32 stages 325 -> 293.
+// 836 -> 591 us, 384 of 64 stages 640 -> 623, 300 of 32 stages 332 -> 296.
 #include "ttt_kernels.h"
 #include "ttt_common.cuh"
 #include "ttt_stage.cuh"
